@@ -53,7 +53,7 @@ enum {
 #define SDDMM_FLAG_W_TRANSPOSED  0x8u /* W is given K-major, W_t[t*M + r] */
 #define SDDMM_FLAG_KERNEL_GATHER 0x10u /* force the planless gather kernel */
 #define SDDMM_FLAG_KERNEL_PANEL  0x20u /* force the TMA-staged row-panel kernel */
-#define SDDMM_FLAG_KERNEL_RING   0x40u /* force the shared-memory gather-ring kernels (K = 32, 64, 128, 256, 512 or 1024) */
+#define SDDMM_FLAG_KERNEL_RING   0x40u /* force the row path (no dense cells, no column tiles): the shared-memory rings for K = 256, 512 or 1024, the gather kernel for K = 32, 64 or 128 */
 
 #define SDDMM_FLAG_OPERANDS_BF16 0x100u /* W and H point to bfloat16 arrays (row-major, 2 bytes per element; K = 256, 512,
                                           1024 or 2048); products and sums stay fp32.  Opt-in, outside the fp32 tolerance
@@ -173,8 +173,11 @@ SDDMM_API int sddmm_fused_execute(sddmm_plan_t p, const float *W, const float *H
  * uploads between them are not counted. */
 SDDMM_API int sddmm_last_kernel_ms(sddmm_plan_t p, float *ms);
 
-/* Which kernels the last sddmm_execute() on this plan launched: "ring", "ring_small",
- * "panel", "gather", "dense_tc+ring_small", ... (static storage).  The reference has one
+/* Which path the last sddmm_execute() on this plan took (static storage): "ring" (K = 256, 512,
+ * 1024), "ring_small" (K = 32, 64, 128), "panel" (any other K, or fewer than 65,536 nonzeros), "htile",
+ * "dense_tc+ring_small", ... by default; "ring", "ring_small", "panel" or "gather" when forced by a flag.
+ * The names stand for classes of K and size, not for kernel functions: by default the row classes run on the
+ * gather kernel, and on the rings where H is far larger than L2.  The reference has one
  * kernel, comp_kernel_COO (HiPC18/src/kernel.h:2), and nothing to report. */
 SDDMM_API const char *sddmm_last_kernel_name(sddmm_plan_t p);
 

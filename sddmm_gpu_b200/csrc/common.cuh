@@ -83,11 +83,13 @@ struct PanelConfig {
 // Chooses panel height / item budget / CTA shape for a given K and hint.
 PanelConfig choose_panel_config(int K, int panel_rows_hint, int sm_count, size_t smem_optin);
 
-// Planless kernel: every sub-warp group gathers its W row and H row from global
-// memory.  rows/cols/P in the same (input) order.
-cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const float *sval,
-                          const float *W, const float *H, float *P, int64_t nnz, int K,
-                          int sm_count, cudaStream_t stream);
+// Gather kernel (sddmm_gather.cu): any K % 4 == 0, no plan data needed; the default path.  perm as in launch_panel.
+cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
+                          const float *W, const float *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream);
+// The same over operands stored in bfloat16 (rows of 2K bytes): K = 256 or 512.
+bool gather_bf16_supports(int K);
+cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
+                               const void *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream);
 
 // Row-panel kernel: persistent CTAs walk the work items; the W rows an item
 // touches (item_rows lists them) are staged into shared memory with bulk
@@ -111,9 +113,12 @@ cudaError_t launch_upload_rows(const float *mapped_host, float *dev, const int32
 
 // Ring kernel: H rows gathered by bulk asynchronous copies (TMA) into per-warp
 // shared-memory rings, work handed out dynamically through *work_counter (one
-// device word, zeroed by the launcher).  K must satisfy ring_supports(K)
-// (32, 64, 128, 256, 512, 1024).
+// device word, zeroed by the launcher).  K = 256, 512 or 1024.
 bool ring_supports(int K);
+// K that SDDMM_FLAG_KERNEL_RING takes.
+inline bool rows_path_supports(int K) { return K == 32 || K == 64 || K == 128 || K == 256 || K == 512 || K == 1024; }
+// Whether the ring kernel is the faster one for an H of N rows (see sddmm_ring.cu).
+bool ring_preferred(int64_t N, int K);
 // cols_hinted: bit 31 of every column index marks a hub column (see build_hub_column_hints).
 cudaError_t launch_ring(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t nnz, int K, bool cols_hinted, int sm_count,
@@ -154,12 +159,6 @@ cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const
                                   int64_t n_dense_rows, const int32_t *dense_cols, int64_t n_dense_cols, const float *sval,
                                   const float *W, const float *H, float *P, int64_t M, int64_t N, int K, int sm_count,
                                   int *dev_status, cudaStream_t stream);
-
-// Ring kernel for short rows (K = 32, 64, 128): the same per-warp rings filled with
-// 16-byte cp.async copies; reached through launch_ring.
-cudaError_t launch_ring_small(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
-                              const float *W, const float *H, float *P, int64_t nnz, int K, bool cols_hinted,
-                              int sm_count, unsigned long long *work_counter, cudaStream_t stream);
 
 // SpMM / fused SDDMM->SpMM over the plan's rows (spmm.cu).  A task is a run of whole rows
 // [row_a, row_b) (slot < 0), or the nonzeros [j0, j1) of the long row row_a, summed into scratch slot `slot`.

@@ -31,6 +31,37 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float acc)
     return acc;
 }
 
+// 16 bytes as two 64-bit words: the operands of the packed FMA (two fp32 per word).
+struct u64x2 {
+    unsigned long long a, b;
+};
+__device__ __forceinline__ u64x2 ldg_u64x2(const void *p)
+{
+    u64x2 r;
+    asm volatile("ld.global.nc.v2.u64 {%0, %1}, [%2];" : "=l"(r.a), "=l"(r.b) : "l"(p));
+    return r;
+}
+// d.lo = a.lo * b.lo + c.lo, d.hi likewise: two fp32 FMAs in one instruction
+__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float fold2(unsigned long long a)
+{
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return x + y;
+}
+// two bfloat16 (the lower one first) as two fp32
+__device__ __forceinline__ unsigned long long widen_bf16x2(unsigned x)
+{
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(x << 16), "r"(x & 0xffff0000u));
+    return d;
+}
+
 // Transposed butterfly over a group of L lanes holding B accumulators each
 // (B <= L, both powers of two).  On return acc[0] of lane `lig` (lane in group)
 // holds the complete sum of accumulator j = lig / (L/B); every lane of that

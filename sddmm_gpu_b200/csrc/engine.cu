@@ -104,8 +104,6 @@ void free_plan_memory(sddmm_plan_s *p)
     cudaFree(p->d_item_rows);
     cudaFree(p->d_cols_hint);
     p->dense.release();
-    cudaFree(p->d_items_s);
-    cudaFree(p->d_item_rows_s);
     cudaFree(p->d_used_rows);
     cudaFree(p->d_used_cols);
     p->row_groups.release();
@@ -138,15 +136,6 @@ cudaError_t ensure_pipeline(sddmm_handle_s *h)
     return e;
 }
 
-// The gather kernel for ring-supported K.
-cudaError_t launch_rows_gather(sddmm_handle_s *h, const int32_t *rows, const int32_t *cols, const int32_t *perm,
-                               const float *sval, const float *W, const float *H, float *P, int64_t nnz, int K,
-                               bool cols_hinted, cudaStream_t stream)
-{
-    return launch_ring(rows, cols, perm, sval, W, H, P, nnz, K, cols_hinted, h->sm_count, h->d_work_counter, h->d_status,
-                       stream);
-}
-
 // After a synchronising point: turn the device status word into a status code.
 int check_device_status(sddmm_handle_s *h)
 {
@@ -159,7 +148,72 @@ int check_device_status(sddmm_handle_s *h)
     return SDDMM_OK;
 }
 
+// What sddmm_last_kernel_name reports for a call on the row path: the class of its K and size.  The names are part of the
+// interface and outlived the kernels they were taken from; "panel" by default means K outside the list of
+// SDDMM_FLAG_KERNEL_RING or fewer than 65,536 nonzeros.
+const char *rows_class_name(const sddmm_plan_s *p, bool panel, bool ring)
+{
+    if (panel || !rows_path_supports(p->K) || (!ring && p->nnz < 65536)) return "panel";
+    return p->K <= 128 ? "ring_small" : "ring";
+}
+
+// Work items of the row-panel kernel, built when the kernel is forced or their number is asked for.
+cudaError_t ensure_items(sddmm_plan_s *p)
+{
+    if (p->n_items >= 0) return cudaSuccess;
+    const bool tiled = p->d_perm != nullptr;
+    int64_t n = 0;
+    cudaError_t e = build_work_items(tiled ? p->d_rows_t : p->d_rows, tiled ? p->d_cols_t : p->d_cols, p->nnz, p->cfg.panel_rows,
+                                     p->col_tile, p->cfg.item_nnz, &p->d_items, &n, &p->d_item_rows, &p->n_item_rows, p->h->stream);
+    if (e != cudaSuccess) return e;
+    p->n_items = n;
+    p->device_bytes += (int64_t)(sizeof(WorkItem) * (size_t)n + sizeof(int32_t) * (size_t)p->n_item_rows);
+    return cudaSuccess;
+}
+
+// Hub-column marks for the ring kernel, when H is too large to live in L2 as a whole.
+cudaError_t ensure_hints(sddmm_plan_s *p)
+{
+    if (p->hints_built) return cudaSuccess;
+    const int64_t row_bytes = (int64_t)p->K * 4;
+    if (p->nnz > 0 && rows_path_supports(p->K) && p->hub_budget > 0 && p->N * row_bytes > p->hub_budget) {
+        cudaError_t e = dev_alloc(p, &p->d_cols_hint, (size_t)p->nnz);
+        int thr = 0;
+        if (e == cudaSuccess)
+            e = build_hub_column_hints(p->d_perm ? p->d_cols_t : p->d_cols, p->nnz, p->N, row_bytes, p->hub_budget, p->d_cols_hint,
+                                       &p->n_hub_cols, &thr, p->h->stream);
+        if (e != cudaSuccess) return e;
+    }
+    p->hints_built = true;
+    return cudaSuccess;
+}
+
 }  // namespace
+
+namespace sddmm {
+
+cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
+                        const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
+                        cudaStream_t stream)
+{
+    sddmm_handle_s *h = p->h;
+    rows += first;
+    if (perm) {
+        perm += first;
+    } else {
+        P += first;
+        if (sval) sval += first;
+    }
+    if (ring_supports(p->K) && (force_ring || ring_preferred(p->N, p->K))) {
+        // the marks are in the plan's processing order: not for the dense-cell remainder
+        const bool hinted = p->d_cols_hint && cols == (p->d_perm ? p->d_cols_t : p->d_cols);
+        return launch_ring(rows, (hinted ? p->d_cols_hint : cols) + first, perm, sval, W, H, P, count, p->K, hinted, h->sm_count,
+                           h->d_work_counter, h->d_status, stream);
+    }
+    return launch_gather(rows, cols + first, perm, sval, W, H, P, count, p->K, h->sm_count, stream);
+}
+
+}  // namespace sddmm
 
 extern "C" {
 
@@ -357,18 +411,12 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     p->col_tile = (int)ct;
     p->n_col_tiles = (int)((N + ct - 1) / ct);
     if (p->n_col_tiles < 1) p->n_col_tiles = 1;
-    const int32_t *rows_p = p->d_rows, *cols_p = p->d_cols;
     if (p->n_col_tiles > 1 && nnz > 0) {
         PLAN_TRY(dev_alloc(p, &p->d_perm, (size_t)nnz));
         PLAN_TRY(dev_alloc(p, &p->d_rows_t, (size_t)nnz));
         PLAN_TRY(dev_alloc(p, &p->d_cols_t, (size_t)nnz));
         PLAN_TRY(build_tiled_order(p->d_rows, p->d_cols, nnz, N, p->col_tile, p->d_perm, p->d_rows_t, p->d_cols_t, s));
-        rows_p = p->d_rows_t;
-        cols_p = p->d_cols_t;
     }
-    PLAN_TRY(build_work_items(rows_p, cols_p, nnz, p->cfg.panel_rows, p->col_tile, p->cfg.item_nnz, &p->d_items,
-                              &p->n_items, &p->d_item_rows, &p->n_item_rows, s));
-    p->device_bytes += (int64_t)(sizeof(WorkItem) * (size_t)p->n_items + sizeof(int32_t) * (size_t)p->n_item_rows);
     // Locally dense matrices (many nonzeros per row): cells that are at least a
     // quarter full go to the dense-cell kernel, if they hold half of S or more
     // (below that the second launch and the permuted remainder cost more than they save).
@@ -378,28 +426,18 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         const bool enabled = !(env && std::atoi(env) == 0);
         if (enabled && p->n_col_tiles == 1 && p->n_nonempty_rows > 0 && nnz / p->n_nonempty_rows >= 32) {
             PLAN_TRY(build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, nnz, M, N, 0.25f, 0.5f, &p->dense, s));
-            if (p->dense.n_cells > 0 && p->dense.n_sparse > 0 && !ring_supports(K)) {
-                PLAN_TRY(build_work_items(p->dense.rows_s, p->dense.cols_s, p->dense.n_sparse, p->cfg.panel_rows,
-                                          p->col_tile, p->cfg.item_nnz, &p->d_items_s, &p->n_items_s, &p->d_item_rows_s,
-                                          &p->n_item_rows_s, s));
-            }
             if (p->dense.n_cells > 0)
                 p->device_bytes += (int64_t)(sizeof(DenseCell) * p->dense.n_cells + 6 * p->dense.n_dense_nnz +
                                              12 * p->dense.n_sparse);
         }
     }
-    // Hub-column marks for the ring kernel, when H is too large to live in L2 as a
-    // whole.  SDDMM_L2_HUB_MB overrides the share of L2 set aside for hub rows (0 = off).
-    if (ring_supports(K) && nnz > 0) {
+    // Hub-column marks are for the ring kernel: now if it will run by default, else if it is forced.
+    // SDDMM_L2_HUB_MB overrides the share of L2 set aside for hub rows (0 = off).
+    {
         int64_t budget_mb = 64;  // best of a 16..128 MB sweep on the scale-22 R-MAT matrix at K = 256
         if (const char *env = std::getenv("SDDMM_L2_HUB_MB")) budget_mb = std::atoll(env);
-        const int64_t row_bytes = (int64_t)K * 4;
-        if (budget_mb > 0 && N * row_bytes > budget_mb * (1ll << 20)) {
-            PLAN_TRY(dev_alloc(p, &p->d_cols_hint, (size_t)nnz));
-            int thr = 0;
-            PLAN_TRY(build_hub_column_hints(cols_p, nnz, N, row_bytes, budget_mb * (1ll << 20), p->d_cols_hint,
-                                            &p->n_hub_cols, &thr, s));
-        }
+        p->hub_budget = budget_mb > 0 ? budget_mb * (1ll << 20) : 0;
+        if (ring_preferred(N, K)) PLAN_TRY(ensure_hints(p));
     }
     // Few columns and many nonzeros per column (a bag-of-words matrix): H is a handful of shared-memory tiles, and
     // the column-tile kernel reads every H row of a nonzero from shared memory.  Worth it when a CTA's share of
@@ -425,7 +463,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     // last row of every chunk -- rows are sorted, so a chunk needs one contiguous
     // block of W rows, and W rows between two chunks that no nonzero touches are
     // never uploaded.
-    if (ring_supports(K) && p->n_col_tiles == 1 && p->dense.n_cells == 0 && nnz >= (1 << 20)) {
+    if (p->n_col_tiles == 1 && p->dense.n_cells == 0 && nnz >= (1 << 20)) {
         int64_t chunks = (int64_t)sizeof(float) * M * K / (128ll << 20);
         if (chunks > SDDMM_PIPE_MAX_CHUNKS) chunks = SDDMM_PIPE_MAX_CHUNKS;
         if (chunks >= 2) {
@@ -493,9 +531,8 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     const bool tiled_out = (flags & SDDMM_FLAG_TILED_ORDER) != 0;
     const uint32_t forced = flags & (SDDMM_FLAG_KERNEL_GATHER | SDDMM_FLAG_KERNEL_PANEL | SDDMM_FLAG_KERNEL_RING);
     if (forced & (forced - 1)) return SDDMM_INVALID_ARG;  // at most one kernel may be forced
-    if ((flags & SDDMM_FLAG_KERNEL_RING) && !ring_supports(p->K)) return SDDMM_K_UNSUPPORTED;
-    // tiny inputs are launch-bound: the panel kernel needs no counter reset and starts faster
-    const bool use_ring = (flags & SDDMM_FLAG_KERNEL_RING) || (!forced && ring_supports(p->K) && p->nnz >= 65536);
+    const bool use_ring = (flags & SDDMM_FLAG_KERNEL_RING) != 0, use_panel = (flags & SDDMM_FLAG_KERNEL_PANEL) != 0;
+    if (use_ring && !rows_path_supports(p->K)) return SDDMM_K_UNSUPPORTED;
     if (use_gather && tiled_out && p->d_perm) return SDDMM_INVALID_ARG;
     CUDA_TRY(h, cudaSetDevice(h->device));
     cudaStream_t s = h->stream;
@@ -518,13 +555,19 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             return SDDMM_INVALID_ARG;
         }
         const bool tiled = p->d_perm != nullptr;
-        const int32_t *rows_p = tiled ? p->d_rows_t : p->d_rows;
-        const int32_t *cols_p = p->d_cols_hint ? p->d_cols_hint : (tiled ? p->d_cols_t : p->d_cols);
+        const int32_t *rows_p = tiled ? p->d_rows_t : p->d_rows, *cols_p = tiled ? p->d_cols_t : p->d_cols;
+        const int32_t *perm_p = tiled ? p->d_perm : nullptr;
+        // rows of half the bytes: the same line between the two kernels as for fp32 rows of K / 2
+        const bool gather = gather_bf16_supports(p->K) && !(flags & SDDMM_FLAG_KERNEL_RING) && !ring_preferred(p->N / 2, p->K);
+        if (!gather) CUDA_TRY(h, ensure_hints(p));
         p->last_kernel = "ring (bf16 operands)";
         p->last_h2d_bytes = p->last_d2h_bytes = 0;
         CUDA_TRY(h, cudaEventRecord(h->ev0, s));
-        LAUNCH_TRY(h, launch_ring_bf16(rows_p, cols_p, tiled ? p->d_perm : nullptr, Sval, W, H, P, p->nnz, p->K,
-                                       p->d_cols_hint != nullptr, h->sm_count, h->d_work_counter, h->d_status, s));
+        if (gather)
+            LAUNCH_TRY(h, launch_gather_bf16(rows_p, cols_p, perm_p, Sval, W, H, P, p->nnz, p->K, h->sm_count, s));
+        else
+            LAUNCH_TRY(h, launch_ring_bf16(rows_p, p->d_cols_hint ? p->d_cols_hint : cols_p, perm_p, Sval, W, H, P, p->nnz, p->K,
+                                           p->d_cols_hint != nullptr, h->sm_count, h->d_work_counter, h->d_status, s));
         CUDA_TRY(h, cudaEventRecord(h->ev1, s));
         if (flags & SDDMM_FLAG_ASYNC) {
             p->last_ms = -1.f;
@@ -542,7 +585,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     // W in host memory and a plain ring-kernel plan: upload W (and S) chunk by chunk
     // and let every chunk's kernel and download run behind the later uploads
     const bool w_t = (flags & SDDMM_FLAG_W_TRANSPOSED) != 0, h_t = (flags & SDDMM_FLAG_H_TRANSPOSED) != 0;
-    const bool pipelined = h->pipeline && p->n_pipe > 0 && !w_dev && use_ring && !tiled_out && !p->d_perm &&
+    const bool pipelined = h->pipeline && p->n_pipe > 0 && !w_dev && !use_gather && !use_panel && !tiled_out && !p->d_perm &&
                            p->dense.n_cells == 0 && !w_t && !h_t;
     // page-locked, mapped host arrays are read row by row by the GPU: only the rows a nonzero touches travel
     const float *W_mapped = (pipelined && h->sparse_upload) ? mapped_host_ptr(W) : nullptr;
@@ -608,11 +651,13 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         h->last_error = "W and H must be 16-byte aligned on the device";
         return SDDMM_INVALID_ARG;
     }
-    const char *ring_name = p->K <= 128 ? "ring_small" : "ring";
+    if (use_panel) CUDA_TRY(h, ensure_items(p));
+    if (use_ring && ring_supports(p->K)) CUDA_TRY(h, ensure_hints(p));
     if (pipelined) {
-        p->last_kernel = p->K <= 128 ? "ring_small (pipelined chunks)" : "ring (pipelined chunks)";
+        p->last_kernel = !rows_path_supports(p->K) ? "panel (pipelined chunks)"
+                         : p->K <= 128             ? "ring_small (pipelined chunks)"
+                                                   : "ring (pipelined chunks)";
         CUDA_TRY(h, ensure_pipeline(h));
-        const int32_t *cols_p = p->d_cols_hint ? p->d_cols_hint : p->d_cols;
         for (int i = 0; i < p->n_pipe; ++i) {
             const int64_t n0 = p->pipe_nnz[i], cnt = p->pipe_nnz[i + 1] - n0;
             const int64_t r0 = p->pipe_w_begin[i], r1 = p->pipe_w_end[i];
@@ -630,8 +675,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             CUDA_TRY(h, cudaEventRecord(h->pipe_uploaded[i], s));
             CUDA_TRY(h, cudaStreamWaitEvent(h->pipe_compute, h->pipe_uploaded[i], 0));
             CUDA_TRY(h, cudaEventRecord(h->pipe_started[i], h->pipe_compute));
-            LAUNCH_TRY(h, launch_rows_gather(h, p->d_rows + n0, cols_p + n0, nullptr, dS ? dS + n0 : nullptr, dW, dH, dP + n0,
-                                             cnt, p->K, p->d_cols_hint != nullptr, h->pipe_compute));
+            LAUNCH_TRY(h, launch_rows(p, p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, n0, cnt, use_ring, h->pipe_compute));
             CUDA_TRY(h, cudaEventRecord(h->pipe_computed[i], h->pipe_compute));
             if (!p_dev) {
                 CUDA_TRY(h, cudaStreamWaitEvent(h->pipe_download, h->pipe_computed[i], 0));
@@ -657,15 +701,11 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (!forced && !tiled_out && p->dense.n_cells > 0) {
         // locally dense plan: dense cells as small dense products, the rest gathered
         {
-            static const char *const names[3][3] = {
-                {"dense_fma", "dense_fma+ring", "dense_fma+panel"},
-                {"dense_mma_sync", "dense_mma_sync+ring", "dense_mma_sync+panel"},
-                {"dense_tc", "dense_tc+ring", "dense_tc+panel"}};
-            const int rest = p->dense.n_sparse == 0 ? 0 : (ring_supports(p->K) ? 1 : 2);
-            p->last_kernel = names[h->dense_mode][rest];
-            if (rest == 1 && p->K <= 128)
-                p->last_kernel = h->dense_mode == 2 ? "dense_tc+ring_small"
-                                                    : (h->dense_mode == 1 ? "dense_mma_sync+ring_small" : "dense_fma+ring_small");
+            static const char *const names[3][4] = {
+                {"dense_fma", "dense_fma+panel", "dense_fma+ring_small", "dense_fma+ring"},
+                {"dense_mma_sync", "dense_mma_sync+panel", "dense_mma_sync+ring_small", "dense_mma_sync+ring"},
+                {"dense_tc", "dense_tc+panel", "dense_tc+ring_small", "dense_tc+ring"}};
+            p->last_kernel = names[h->dense_mode][p->dense.n_sparse == 0 ? 0 : !rows_path_supports(p->K) ? 1 : p->K <= 128 ? 2 : 3];
         }
         if (h->dense_mode == 2)
             LAUNCH_TRY(h, launch_dense_cells_tc(p->dense.cells, p->dense.n_cells, p->dense.idx, p->dense.rc, p->dense.row_mask,
@@ -677,17 +717,12 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
                                            p->dense.row_base, p->dense.dense_rows, p->dense.n_dense_rows,
                                            p->dense.dense_cols, p->dense.n_dense_cols, dS, dW, dH, dP, p->M, p->N, p->K,
                                            h->dense_mode == 1, h->sm_count, s));
-        if (p->dense.n_sparse > 0) {
-            if (ring_supports(p->K))
-                LAUNCH_TRY(h, launch_rows_gather(h, p->dense.rows_s, p->dense.cols_s, p->dense.perm_s, dS, dW, dH, dP,
-                                                 p->dense.n_sparse, p->K, false, s));
-            else
-                LAUNCH_TRY(h, launch_panel(p->d_items_s, p->n_items_s, p->d_item_rows_s, p->dense.rows_s, p->dense.cols_s,
-                                         p->dense.perm_s, dS, dW, dH, dP, p->K, p->cfg, h->sm_count, h->d_status, s));
-        }
+        if (p->dense.n_sparse > 0)
+            LAUNCH_TRY(h, launch_rows(p, p->dense.rows_s, p->dense.cols_s, p->dense.perm_s, dS, dW, dH, dP, 0, p->dense.n_sparse,
+                                      false, s));
     } else if (use_gather) {
         p->last_kernel = "gather";
-        LAUNCH_TRY(h, launch_gather(p->d_rows, p->d_cols, dS, dW, dH, dP, p->nnz, p->K, h->sm_count, s));
+        LAUNCH_TRY(h, launch_gather(p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, p->nnz, p->K, h->sm_count, s));
     } else {
         const bool tiled = p->d_perm != nullptr;
         const int32_t *rows_p = tiled ? p->d_rows_t : p->d_rows;
@@ -702,16 +737,15 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             return SDDMM_INVALID_ARG;
         }
         const bool use_htile = p->d_ht_off && !forced && !tiled && ((reinterpret_cast<uintptr_t>(dW) | reinterpret_cast<uintptr_t>(dH)) & 15u) == 0;
-        p->last_kernel = use_htile ? "htile" : use_ring ? ring_name : "panel";
+        p->last_kernel = use_htile ? "htile" : rows_class_name(p, use_panel, use_ring);
         if (use_htile)
             LAUNCH_TRY(h, launch_htile(p->d_ht_rows, p->d_ht_cols, p->d_ht_perm, dS, dW, dH, dP, p->nnz, p->N, p->K, p->ht_col_tile,
                                        p->d_ht_off, p->ht_n_tiles, h->sm_count, h->d_status, s));
-        else if (use_ring)
-            LAUNCH_TRY(h, launch_rows_gather(h, rows_p, p->d_cols_hint ? p->d_cols_hint : cols_p, perm, dS, dW, dH, dP, p->nnz,
-                                             p->K, p->d_cols_hint != nullptr, s));
-        else
+        else if (use_panel)
             LAUNCH_TRY(h, launch_panel(p->d_items, p->n_items, p->d_item_rows, rows_p, cols_p, perm, dS, dW, dH, dP, p->K,
                                      p->cfg, h->sm_count, h->d_status, s));
+        else
+            LAUNCH_TRY(h, launch_rows(p, rows_p, cols_p, perm, dS, dW, dH, dP, 0, p->nnz, use_ring, s));
     }
     CUDA_TRY(h, cudaEventRecord(h->ev1, s));
     if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dP, nbytes, cudaMemcpyDeviceToHost, s));
@@ -1107,7 +1141,7 @@ int sddmm_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const int32_t
         CUDA_TRY(h, cudaMalloc(&tmp.p[5], sizeof(float) * nnz));
         dp = (float *)tmp.p[5];
     }
-    CUDA_TRY(h, launch_gather((const int32_t *)dr, (const int32_t *)dc, (const float *)ds, (const float *)dw,
+    CUDA_TRY(h, launch_gather((const int32_t *)dr, (const int32_t *)dc, nullptr, (const float *)ds, (const float *)dw,
                               (const float *)dh, dp, nnz, K, h->sm_count, s));
     if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dp, sizeof(float) * nnz, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
@@ -1128,6 +1162,9 @@ int sddmm_selftest_wait_timeout(sddmm_handle_t h)
 int sddmm_plan_get_info(sddmm_plan_t p, sddmm_plan_info *info)
 {
     if (!p || !info) return SDDMM_INVALID_ARG;
+    CUDA_TRY(p->h, cudaSetDevice(p->h->device));
+    CUDA_TRY(p->h, ensure_items(p));
+    CUDA_TRY(p->h, ensure_hints(p));
     info->M = p->M; info->N = p->N; info->nnz = p->nnz; info->K = p->K;
     info->panel_rows = p->cfg.panel_rows;
     info->col_tile = p->col_tile;

@@ -55,20 +55,18 @@ struct sddmm_plan_s {
     // pattern, tiled order (only when n_col_tiles > 1)
     int32_t *d_rows_t = nullptr, *d_cols_t = nullptr, *d_perm = nullptr;
     int64_t *d_row_ptr = nullptr;
-    WorkItem *d_items = nullptr;
-    int64_t n_items = 0;
+    WorkItem *d_items = nullptr;     // row-panel kernel; built when it is first asked for (ensure_items)
+    int64_t n_items = -1;
     int32_t *d_item_rows = nullptr;  // distinct rows of every item, concatenated
-    int32_t *d_cols_hint = nullptr;  // processing-order columns with hub marks (ring kernel), or null
+    int32_t *d_cols_hint = nullptr;  // processing-order columns with hub marks (ring kernel), or null (ensure_hints)
+    int64_t hub_budget = 0;          // bytes of H rows to keep in L2 (0 = no marks)
+    bool hints_built = false;
     // column-tile kernel (few columns, many nonzeros per column): its own tiled order and tile offsets
     int32_t *d_ht_rows = nullptr, *d_ht_cols = nullptr, *d_ht_perm = nullptr;
     int64_t *d_ht_off = nullptr;
     int ht_col_tile = 0, ht_n_tiles = 0;
     // dense cells + row-sorted remainder (single-tile plans of locally dense matrices)
     DensePlan dense;
-    WorkItem *d_items_s = nullptr;
-    int64_t n_items_s = 0;
-    int32_t *d_item_rows_s = nullptr;
-    int64_t n_item_rows_s = 0;
     int64_t n_hub_cols = 0;
     int64_t n_item_rows = 0;
     int64_t n_nonempty_rows = 0, n_nonempty_cols = -1;
@@ -103,3 +101,11 @@ struct sddmm_plan_s {
     int64_t n_spmr_tasks = -1, n_spmr_long = 0;
 };
 
+
+namespace sddmm {
+// SDDMM over nonzeros in the plan's processing order, [first, first + count): the ring kernel when it is the faster one
+// for this plan (or forced), else the gather kernel.
+cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
+                        const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
+                        cudaStream_t stream);
+}  // namespace sddmm

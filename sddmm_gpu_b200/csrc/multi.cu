@@ -467,11 +467,10 @@ int sddmm_dist_execute(sddmm_dist_plan_t p, const float *W_local, float *H, cons
         }
         const int64_t o0 = p->tile_off[(size_t)i], cnt = p->tile_off[(size_t)i + 1] - o0;
         if (cnt <= 0) continue;
-        const int32_t *cols_p = q->d_cols_hint ? q->d_cols_hint : q->d_cols_t;
         cudaError_t e;
-        if (ring_supports(p->K)) {
-            e = launch_ring(q->d_rows_t + o0, cols_p + o0, q->d_perm + o0, Sval_local, W_local, H, P_local, cnt, p->K,
-                                q->d_cols_hint != nullptr, h->sm_count, h->d_work_counter, h->d_status, s);
+        if (rows_path_supports(p->K)) {
+            e = launch_rows(const_cast<sddmm_plan_s *>(q), q->d_rows_t, q->d_cols_t, q->d_perm, Sval_local, W_local, H, P_local, o0,
+                            cnt, false, s);
             if (e != cudaSuccess) return fail_cuda_m(h, e, "launching the gather kernel of an H chunk");
             ++h->n_launches;
         } else {

@@ -1,0 +1,324 @@
+// Gather kernel: the SDDMM of any K that is a multiple of 4, with or without a plan.
+//
+// The 32 lanes of a warp are sets of L lanes; a set takes a run of consecutive nonzeros and works on one nonzero at a
+// time: lane l of the set holds the 16-byte pieces l, l + L, ... (F of them) of the W row and of the H row, so one
+// load instruction of a set covers L * 16 consecutive bytes of one row.  H rows are loaded straight into registers, B
+// nonzeros ahead of their use; the W row stays in registers until the row of S changes.  Rows, columns and S values of
+// a step (8 nonzeros per set) are loaded one step ahead, one nonzero per lane, and spread by shuffles; the 8 partial
+// sums of a lane are reduced by one transposed butterfly, after which lane l stores nonzero l of the set.
+//
+// What bounds it.  Every nonzero brings one row of H from L2 (or L1, or DRAM) to its SM: 4K bytes, 16.7 TB/s at most
+// over all SMs (a bare copy loop).  Latency is hidden by warps, not by a pipeline inside the warp: few registers per
+// thread and many resident warps (24 to 48 per SM, __launch_bounds__ below) move more bytes than deeper batches with
+// fewer warps (K = 128, 16.1 M nonzeros of an R-MAT matrix: 0.53 ms at 40 warps with one nonzero in flight per set,
+// 0.59 ms at 24 warps with two, 0.64 ms at 16 warps with four).  No shared memory: all of it is L1, which serves the
+// hub columns of a power-law matrix, and nothing is issued beyond the load, the packed FMAs (two per instruction) and
+// 1/8 of a butterfly -- 9 warp instructions per nonzero at K = 128 where the shared-memory ring needed 34.  Grids are
+// not persistent: a warp's share is 16 or 32 nonzeros per set, the hardware's block scheduler evens out the rest, and
+// there is no work counter to clear before the launch.
+//
+// Measured against the shared-memory ring and panel kernels (R-MAT, 16.1 M nonzeros, 1 M x 1 M, and 4.1 M nonzeros,
+// 300 K x 250 K; us before -> after):  K = 32: 250 -> 185, K = 64: 480 -> 296, K = 128: 832 -> 540, K = 256: 1250 ->
+// 1146;  K = 100: 590 -> 135, K = 192: 752 -> 187, K = 300: 1233 -> 283, K = 512: 599 -> 522, K = 768: 2775 -> 820.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "common.cuh"
+#include "device_utils.cuh"
+
+namespace sddmm {
+
+using namespace dev;
+
+namespace {
+
+constexpr int GA_TPB = 256;
+
+// L lanes per nonzero, F 16-byte pieces per lane, B nonzeros of a set in flight, RB nonzeros per reduction, CTAS
+// resident blocks per SM asked of the compiler.  EXACT: the L * F pieces are the row (no predicate on the last one).
+// PF: the W rows of the next step are prefetched into L1.  BF16: W and H hold bfloat16 (a piece is 8 values).
+template <int L_, int F_, int B_, int RB_, bool EXACT_, bool PF_, int CTAS_, bool BF16_ = false>
+struct GatherShape {
+    static constexpr int L = L_, F = F_, B = B_, RB = RB_, CTAS = CTAS_;
+    static constexpr bool EXACT = EXACT_, PF = PF_, BF16 = BF16_;
+    static constexpr int NB = L < 8 ? L : 8;  // nonzeros of a set per step
+    static constexpr int G = 32 / L;          // sets of a warp
+    static_assert(NB % RB == 0 && RB % B == 0 && RB <= L, "step geometry");
+};
+
+// A lane's share of the W row: fp32 pairs, widened once per row when the operands are bfloat16.
+template <class S>
+struct WShare {
+    u64x2 v[S::F * (S::BF16 ? 2 : 1)];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int i = 0; i < S::F * (S::BF16 ? 2 : 1); ++i) v[i] = u64x2{0, 0};
+    }
+    __device__ __forceinline__ void load(const char *wp, bool last_ok)
+    {
+#pragma unroll
+        for (int f = 0; f < S::F; ++f) {
+            if (f < S::F - 1 || last_ok) {
+                const u64x2 t = ldg_u64x2(wp + f * S::L * 16);
+                if constexpr (S::BF16) {
+                    v[2 * f] = u64x2{widen_bf16x2((unsigned)t.a), widen_bf16x2((unsigned)(t.a >> 32))};
+                    v[2 * f + 1] = u64x2{widen_bf16x2((unsigned)t.b), widen_bf16x2((unsigned)(t.b >> 32))};
+                } else {
+                    v[f] = t;
+                }
+            }
+        }
+    }
+    __device__ __forceinline__ float dot(const u64x2 (&h)[S::F]) const
+    {
+        unsigned long long a0 = 0, a1 = 0;  // two fp32 sums each
+#pragma unroll
+        for (int f = 0; f < S::F; ++f) {
+            if constexpr (S::BF16) {
+                a0 = ffma2(v[2 * f].a, widen_bf16x2((unsigned)h[f].a), a0);
+                a1 = ffma2(v[2 * f].b, widen_bf16x2((unsigned)(h[f].a >> 32)), a1);
+                a0 = ffma2(v[2 * f + 1].a, widen_bf16x2((unsigned)h[f].b), a0);
+                a1 = ffma2(v[2 * f + 1].b, widen_bf16x2((unsigned)(h[f].b >> 32)), a1);
+            } else {
+                a0 = ffma2(v[f].a, h[f].a, a0);
+                a1 = ffma2(v[f].b, h[f].b, a1);
+            }
+        }
+        return fold2(a0) + fold2(a1);
+    }
+};
+
+// pieces: 16-byte pieces of a row.  run_len: nonzeros of a set, a multiple of S::NB.  perm (HAS_PERM): the result of
+// nonzero j goes to P[perm[j]] and is scaled by sval[perm[j]].
+template <class S, bool HAS_PERM>
+__global__ void __launch_bounds__(GA_TPB, S::CTAS)
+sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
+                    const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
+                    float *__restrict__ P, unsigned nnz, int pieces, unsigned run_len)
+{
+    constexpr int L = S::L, F = S::F, B = S::B, RB = S::RB, NB = S::NB, G = S::G;
+    const int lane = threadIdx.x & 31, lig = lane & (L - 1), set = lane / L;
+    const unsigned warp0 = ((blockIdx.x * GA_TPB + threadIdx.x) >> 5) * (G * run_len);  // first nonzero of this warp
+    if (warp0 >= nnz) return;
+    const unsigned row_bytes = (unsigned)pieces * 16u;
+    const char *H_lane = H + lig * 16, *W_lane = W + lig * 16;
+    const bool last_ok = S::EXACT || lig + (F - 1) * L < pieces;
+    unsigned setmask = 0;  // lane 0 of every set
+#pragma unroll
+    for (int g = 0; g < G; ++g) setmask |= 1u << (g * L);
+
+    WShare<S> w;
+    w.clear();
+    const int il = lig & (NB - 1);  // lanes >= NB of a set mirror a nonzero
+    unsigned j = warp0 + set * run_len + il;
+    auto at = [&](unsigned x) { return x < nnz ? x : nnz - 1; };  // past the end the last nonzero is read again, never stored
+    int r, c, dst = 0;
+    float s = 1.f;
+    {
+        const unsigned a = at(j);
+        r = __ldg(rows + a);
+        c = __ldg(cols + a);
+        if (HAS_PERM) dst = __ldg(perm + a);
+        else if (sval) s = __ldg(sval + a);
+    }
+    int cur = -1;  // row of the set's nonzero before this step
+#pragma unroll 1
+    for (unsigned step = run_len / NB; step > 0; --step) {
+        int rn = 0, cn = 0, dn = 0;
+        float sn = 1.f;
+        if (step > 1) {
+            const unsigned a = at(j + NB);
+            rn = __ldg(rows + a);
+            cn = __ldg(cols + a);
+            if (HAS_PERM) dn = __ldg(perm + a);
+            else if (sval) sn = __ldg(sval + a);
+        }
+        int before = __shfl_up_sync(FULL, r, 1, L);
+        if (lig == 0) before = cur;
+        const unsigned changed = __ballot_sync(FULL, r != before && lig < NB);
+        cur = __shfl_sync(FULL, r, NB - 1, L);
+        if (S::PF && step > 1) {
+            int b2 = __shfl_up_sync(FULL, rn, 1, L);
+            if (lig == 0) b2 = cur;
+            if (rn != b2 && lig < NB) {
+                const char *wp = W + (size_t)(unsigned)rn * row_bytes;
+                for (unsigned o = 0; o < row_bytes; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(wp + o));
+            }
+        }
+        float res = 0.f;
+#pragma unroll
+        for (int h0 = 0; h0 < NB; h0 += RB) {
+            float acc[RB];
+#pragma unroll
+            for (int b = 0; b < RB; b += B) {
+                u64x2 h[B][F];
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    const unsigned cj = (unsigned)__shfl_sync(FULL, c, h0 + b + i, L);
+                    const char *hp = H_lane + (size_t)cj * row_bytes;
+#pragma unroll
+                    for (int f = 0; f < F; ++f)
+                        h[i][f] = (f < F - 1 || last_ok) ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
+                }
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    const int x = h0 + b + i;
+                    if (changed & (setmask << x)) {  // uniform over the warp: nonzero x of some set opens a row
+                        const unsigned rj = (unsigned)__shfl_sync(FULL, r, x, L);
+                        if ((changed >> (set * L + x)) & 1u) w.load(W_lane + (size_t)rj * row_bytes, last_ok);
+                    }
+                    acc[b + i] = w.dot(h[i]);
+                }
+            }
+            reduce_transposed<L, RB>(acc, lig);
+            // the sum of nonzero h0 + q of the set is in its lanes q (L / RB) and following
+            const float t = RB == L ? acc[0] : __shfl_sync(FULL, acc[0], (lig & (RB - 1)) * (L / RB), L);
+            if (RB == NB || il / RB == h0 / RB) res = t;
+        }
+        if (lig < NB && j < nnz) {
+            if (HAS_PERM) {
+                if (sval) res *= __ldg(sval + dst);
+                P[dst] = res;
+            } else {
+                P[j] = res * s;
+            }
+        }
+        j += NB;
+        r = rn;
+        c = cn;
+        s = sn;
+        dst = dn;
+    }
+}
+
+// Rows of more than 256 pieces (K > 1024): a warp per nonzero, both rows in passes of 32 pieces, W through L1.
+template <bool HAS_PERM>
+__global__ void __launch_bounds__(GA_TPB)
+sddmm_gather_long_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
+                         const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
+                         float *__restrict__ P, unsigned nnz, int pieces)
+{
+    constexpr int U = 4;
+    const int lane = threadIdx.x & 31;
+    const unsigned j = (blockIdx.x * GA_TPB + threadIdx.x) >> 5;
+    if (j >= nnz) return;
+    const char *wp = W + (size_t)(unsigned)__ldg(rows + j) * pieces * 16 + lane * 16;
+    const char *hp = H + (size_t)(unsigned)__ldg(cols + j) * pieces * 16 + lane * 16;
+    unsigned long long a0 = 0, a1 = 0;
+    for (int q = lane; q < pieces; q += 32 * U) {
+        u64x2 h[U], w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = q + 32 * u < pieces;
+            h[u] = in ? ldg_u64x2(hp + 512 * u) : u64x2{0, 0};
+            w[u] = in ? ldg_u64x2(wp + 512 * u) : u64x2{0, 0};
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            a0 = ffma2(w[u].a, h[u].a, a0);
+            a1 = ffma2(w[u].b, h[u].b, a1);
+        }
+        hp += 512 * U;
+        wp += 512 * U;
+    }
+    float a = fold2(a0) + fold2(a1);
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
+    if (lane == 0) {
+        const unsigned dst = HAS_PERM ? (unsigned)__ldg(perm + j) : j;
+        if (sval) a *= __ldg(sval + dst);
+        P[dst] = a;
+    }
+}
+
+template <class S, bool HAS_PERM>
+cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
+                           const void *H, float *P, unsigned nnz, int pieces, int sm_count, cudaStream_t stream)
+{
+    // A set's share: 16 nonzeros (32 when a warp is one or two sets), less when the warps would not fill the SMs.
+    constexpr unsigned most = S::L >= 16 ? 32 : 16;
+    const unsigned resident = (unsigned)sm_count * S::CTAS * (GA_TPB / 32) * S::G;  // sets
+    unsigned run = nnz / resident / S::NB * S::NB;
+    run = run < (unsigned)S::NB ? (unsigned)S::NB : run > most ? most : run;
+    const unsigned per_block = run * S::G * (GA_TPB / 32);
+    const unsigned blocks = (unsigned)(((uint64_t)nnz + per_block - 1) / per_block);
+    sddmm_gather_kernel<S, HAS_PERM><<<blocks, GA_TPB, 0, stream>>>(rows, cols, perm, sval, static_cast<const char *>(W),
+                                                                    static_cast<const char *>(H), P, nnz, pieces, run);
+    return cudaGetLastError();
+}
+
+template <class S>
+cudaError_t launch_shape(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
+                         const void *H, float *P, unsigned nnz, int pieces, int sm_count, cudaStream_t stream)
+{
+    return perm ? launch_shape_p<S, true>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, stream)
+                : launch_shape_p<S, false>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, stream);
+}
+
+}  // namespace
+
+// The shape for a row of K floats: the smallest L * F that covers its K / 4 pieces, L small enough that a set's lanes
+// are busy and large enough that F pieces of W and B * F of H stay in few registers.  Every line is the best of a sweep
+// over (L, B, RB, prefetch, resident blocks) at a K of its range on the matrices named at the top of this file.
+cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const float *W,
+                          const float *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream)
+{
+    constexpr int64_t SLICE = 1ll << 30;  // the kernels count nonzeros in 32 bits
+    for (int64_t j0 = 0; j0 < nnz; j0 += SLICE) {
+        const unsigned n = (unsigned)(nnz - j0 < SLICE ? nnz - j0 : SLICE);
+        const int32_t *r = rows + j0, *c = cols + j0, *p = perm ? perm + j0 : nullptr;
+        const float *s = sval && !perm ? sval + j0 : sval;
+        float *out = perm ? P : P + j0;
+        const int q = K / 4;
+        cudaError_t e;
+#define GA_GO(L, F, B, RB, EXACT, PF, CTAS) \
+    e = launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS>>(r, c, p, s, W, H, out, n, q, sm_count, stream)
+        if (q <= 4) GA_GO(4, 1, 4, 4, false, false, 6);
+        else if (q < 8) GA_GO(8, 1, 4, 4, false, false, 6);
+        else if (q == 8) GA_GO(8, 1, 4, 4, true, false, 6);
+        else if (q <= 12) GA_GO(4, 3, 2, 4, false, true, 4);
+        else if (q < 16) GA_GO(8, 2, 4, 4, false, true, 4);
+        else if (q == 16) GA_GO(8, 2, 4, 4, true, true, 4);
+        else if (q <= 24) GA_GO(8, 3, 2, 8, false, true, 4);
+        else if (q < 32) GA_GO(16, 2, 2, 8, false, true, 5);
+        else if (q == 32) GA_GO(16, 2, 2, 8, true, false, 5);
+        else if (q <= 48) GA_GO(16, 3, 2, 8, false, true, 4);
+        else if (q < 64) GA_GO(16, 4, 1, 8, false, true, 4);
+        else if (q == 64) GA_GO(32, 2, 2, 8, true, false, 5);
+        else if (q <= 80) GA_GO(16, 5, 1, 8, false, true, 4);
+        else if (q <= 96) GA_GO(16, 6, 1, 8, false, false, 4);
+        else if (q < 128) GA_GO(32, 4, 2, 8, false, true, 3);
+        else if (q == 128) GA_GO(32, 4, 2, 8, true, true, 3);
+        else if (q <= 160) GA_GO(32, 5, 1, 8, false, false, 4);
+        else if (q <= 192) GA_GO(32, 6, 1, 8, false, false, 4);
+        else if (q <= 256) GA_GO(32, 8, 1, 8, false, false, 3);
+        else {
+            const unsigned blocks = (n + GA_TPB / 32 - 1) / (GA_TPB / 32);
+            if (p) sddmm_gather_long_kernel<true><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q);
+            else sddmm_gather_long_kernel<false><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q);
+            e = cudaGetLastError();
+        }
+#undef GA_GO
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// bfloat16 rows of 2K bytes; a bfloat16 is the upper half of an fp32, so widening is a shift or a mask.
+bool gather_bf16_supports(int K) { return K == 256 || K == 512; }
+
+cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
+                               const void *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream)
+{
+    if (nnz == 0) return cudaSuccess;
+    if (nnz > INT32_MAX) return cudaErrorInvalidValue;  // plans hold fewer
+    const unsigned n = (unsigned)nnz;
+    switch (K) {
+    case 256: return launch_shape<GatherShape<16, 2, 2, 8, true, false, 4, true>>(rows, cols, perm, sval, W, H, P, n, 32, sm_count, stream);
+    case 512: return launch_shape<GatherShape<32, 2, 2, 8, true, false, 4, true>>(rows, cols, perm, sval, W, H, P, n, 64, sm_count, stream);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace sddmm

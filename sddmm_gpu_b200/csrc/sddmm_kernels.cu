@@ -1,12 +1,12 @@
-// SDDMM compute kernels for sm_100a.
+// Row-panel kernel for sm_100a (SDDMM_FLAG_KERNEL_PANEL; the default path is the gather kernel of sddmm_gather.cu).
 //
 //   P[i] = dot(W[row_i, :], H[col_i, :]) [* S.val_i]      (fp32, K % 4 == 0)
 //
-// They replace comp_kernel_COO of the reference (HiPC18/src/kernel.h:2-52): one
+// It replaces comp_kernel_COO of the reference (HiPC18/src/kernel.h:2-52): one
 // launch per call instead of n_col_tiles x K/k_slice launches, no read-modify-write
 // of the result, 64-bit offsets, any K that is a multiple of 4.
 //
-// Work decomposition shared by both kernels.  A group of L lanes (L = 1..32, a
+// Work decomposition.  A group of L lanes (L = 1..32, a
 // power of two, L*4 floats cover min(K,128) floats) owns one nonzero at a time and
 // processes B nonzeros per step, so a warp retires NB = B * (32/L) consecutive
 // nonzeros per step.  All 128-bit H loads of a step are issued before the first
@@ -208,30 +208,7 @@ __device__ __forceinline__ void warp_stream(const int32_t *__restrict__ rows, co
 }
 
 // ---------------------------------------------------------------------------
-// Kernel A: planless gather.  Warps stride over the nonzeros; W rows come from
-// global memory through L1 (row-sorted input makes consecutive nonzeros share them).
-// ---------------------------------------------------------------------------
-template <int L, int C, int B>
-__global__ void __launch_bounds__(256)
-sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols,
-                    const float *__restrict__ sval, const float *__restrict__ W,
-                    const float *__restrict__ H, float *__restrict__ P, int64_t nnz, int K4)
-{
-    using S = Shape<L, C, B>;
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    auto store = [&](int64_t off, int n_valid, float res) {
-        if (lane < n_valid) {
-            if (sval) res *= __ldcs(sval + off + lane);
-            __stcs(P + off + lane, res);
-        }
-    };
-    warp_stream<L, C, B, false, int64_t>(rows, cols, 0, W, H, 0, nnz, warp, n_warps, K4, lane, store);
-}
-
-// ---------------------------------------------------------------------------
-// Kernel B: row-panel kernel.
+// Row-panel kernel.
 //
 // Persistent CTAs walk the work items (item = blockIdx.x, + gridDim.x, ...).
 // One producer warp stages the W rows an item touches into one of two
@@ -357,22 +334,6 @@ sddmm_panel_kernel(const WorkItem *__restrict__ items, int64_t n_items,
     }
 }
 
-template <int L, int C, int B>
-cudaError_t launch_gather_t(const int32_t *rows, const int32_t *cols, const float *sval, const float *W,
-                            const float *H, float *P, int64_t nnz, int K, int sm_count,
-                            cudaStream_t stream)
-{
-    using S = Shape<L, C, B>;
-    const int threads = 256;
-    const int64_t steps = (nnz + S::NB - 1) / S::NB;
-    int64_t blocks = (steps + (threads / 32) - 1) / (threads / 32);
-    const int64_t cap = (int64_t)sm_count * 8;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    sddmm_gather_kernel<L, C, B><<<(unsigned)blocks, threads, 0, stream>>>(rows, cols, sval, W, H, P, nnz, K / 4);
-    return cudaGetLastError();
-}
-
 constexpr int PANEL_WARPS = 15;  // consumer warps; with the producer warp 16 warps = 4 per SM sub-partition, 128 registers each
 
 template <int L, int C, int B>
@@ -412,16 +373,6 @@ cudaError_t launch_panel_t(const WorkItem *items, int64_t n_items, const int32_t
         else if ((K) <= 512) { CALL(32, 4, 2); }       \
         else { CALL(32, 8, 1); }                       \
     } while (0)
-
-cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const float *sval, const float *W,
-                          const float *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream)
-{
-    if (nnz == 0) return cudaSuccess;
-#define CALL(L, C, B) return launch_gather_t<L, C, B>(rows, cols, sval, W, H, P, nnz, K, sm_count, stream)
-    SDDMM_DISPATCH_K(K, CALL);
-#undef CALL
-    return cudaSuccess;
-}
 
 cudaError_t launch_panel(const WorkItem *items, int64_t n_items, const int32_t *item_rows, const int32_t *rows,
                          const int32_t *cols, const int32_t *perm, const float *sval, const float *W, const float *H, float *P,

@@ -27,8 +27,9 @@
 // memory, L1/L2) only when the row changes -- one group ahead, right after the
 // previous group's FMAs.
 //
-// Used for K = 256, 512 and 1024 (C = 2, 4, 8); K = 32, 64 and 128 are served by
-// the cp.async ring of sddmm_ring_small.cu through the same launcher.
+// Used for K = 256, 512 and 1024 (C = 2, 4, 8) when H is far larger than L2 (ring_preferred): there most gathers
+// come from DRAM, whose latency the deep rings hide better than the gather kernel's resident warps, and the copies
+// carry the plan's hub-column hints.  Everything else is the gather kernel's (sddmm_gather.cu).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -367,7 +368,12 @@ cudaError_t launch_ring_t(const int32_t *rows, const int32_t *cols, const int32_
 
 }  // namespace
 
-bool ring_supports(int K) { return K == 32 || K == 64 || K == 128 || K == 256 || K == 512 || K == 1024; }
+bool ring_supports(int K) { return K == 256 || K == 512 || K == 1024; }
+
+// The line between the two kernels, by the size of H (R-MAT matrices, ms on the gather kernel / on the rings):
+// K = 256: 0.27 GB 0.28 / 0.37, 1.1 GB 1.15 / 1.25, 2.6 GB 1.95 / 1.90, 4.3 GB 8.7 / 8.3;
+// K = 512: 0.5 GB 0.52 / 0.60, 1.1 GB 1.27 / 1.31, 2.1 GB 2.40 / 2.28;  K = 1024: 4.3 GB 6.2 / 5.0.
+bool ring_preferred(int64_t N, int K) { return ring_supports(K) && N * K * 4 >= (3ll << 29); }
 
 cudaError_t launch_ring(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t nnz, int K, bool cols_hinted, int sm_count,
@@ -375,10 +381,6 @@ cudaError_t launch_ring(const int32_t *rows, const int32_t *cols, const int32_t 
 {
     if (nnz == 0) return cudaSuccess;
     switch (K) {
-    case 32:
-    case 64:
-    case 128:  // rows up to 512 bytes: the cp.async ring (measured faster than one bulk copy per row there)
-        return launch_ring_small(rows, cols, perm, sval, W, H, P, nnz, K, cols_hinted, sm_count, work_counter, stream);
     case 256: return launch_ring_t<2>(rows, cols, perm, sval, W, H, P, nnz, cols_hinted, sm_count, work_counter, dev_status, stream);
     case 512: return launch_ring_t<4>(rows, cols, perm, sval, W, H, P, nnz, cols_hinted, sm_count, work_counter, dev_status, stream);
     case 1024: return launch_ring_t<8>(rows, cols, perm, sval, W, H, P, nnz, cols_hinted, sm_count, work_counter, dev_status, stream);
