@@ -157,6 +157,12 @@ def _ptr(a):
     """Address of a numpy array / torch tensor / int / None."""
     if a is None:
         return None
+    try:  # a torch tensor, the case of every call in a loop
+        if a.is_contiguous():
+            return a.data_ptr()
+        raise ValueError("tensor must be contiguous")
+    except AttributeError:
+        pass
     if isinstance(a, int):
         return a
     if isinstance(a, np.ndarray):
@@ -175,6 +181,16 @@ CUDA_STREAM_LEGACY = 0x1  # cudaStreamLegacy: the handle that names the legacy d
 
 def _is_cuda_tensor(a):
     return hasattr(a, "is_cuda") and a.is_cuda
+
+
+def _torch_stream_getter():
+    """device -> cudaStream_t of torch's current stream, as cheaply as this torch allows."""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw or (lambda device: torch.cuda.current_stream(device).cuda_stream)
+
+
+_torch_stream = None
 
 
 class Handle:
@@ -197,15 +213,25 @@ class Handle:
             raise SddmmError(st)
         self.device = device
         self._explicit_stream = False
+        self._stream = None  # what sddmm_set_stream was last given (None: the handle's own stream)
 
     def _follow_torch_stream(self, *args):
         """Launch on torch's current stream when a CUDA tensor is among the arguments
         (and the caller has not chosen a stream)."""
-        if self._explicit_stream or not any(_is_cuda_tensor(a) for a in args):
+        global _torch_stream
+        if self._explicit_stream:
             return
-        import torch
-        s = torch.cuda.current_stream(self.device).cuda_stream
-        self._check(lib().sddmm_set_stream(self._h, s if s else CUDA_STREAM_LEGACY))
+        for a in args:
+            if getattr(a, "is_cuda", False):
+                break
+        else:
+            return
+        if _torch_stream is None:
+            _torch_stream = _torch_stream_getter()
+        s = _torch_stream(self.device) or CUDA_STREAM_LEGACY
+        if s != self._stream:  # the engine still points at the stream of the call before otherwise
+            self._check(lib().sddmm_set_stream(self._h, s))
+            self._stream = s
 
     def close(self):
         if self._h:
@@ -232,6 +258,7 @@ class Handle:
     def set_stream(self, cuda_stream):
         """cuda_stream: integer cudaStream_t (e.g. torch.cuda.current_stream().cuda_stream) or None."""
         self._check(lib().sddmm_set_stream(self._h, cuda_stream))
+        self._stream = cuda_stream
         self._explicit_stream = cuda_stream is not None
 
     def kernel_launches(self):

@@ -84,12 +84,14 @@ struct PanelConfig {
 PanelConfig choose_panel_config(int K, int panel_rows_hint, int sm_count, size_t smem_optin);
 
 // Gather kernel (sddmm_gather.cu): any K % 4 == 0, no plan data needed; the default path.  perm as in launch_panel.
+// clock: two device words that receive the kernel's start and end (clock_begin / clock_end), or null.
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
-                          const float *W, const float *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream);
+                          const float *W, const float *H, float *P, int64_t nnz, int K, int sm_count,
+                          unsigned long long *clock, cudaStream_t stream);
 // The same over operands stored in bfloat16 (rows of 2K bytes): K = 256 or 512.
 bool gather_bf16_supports(int K);
 cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                               const void *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream);
+                               const void *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream);
 
 // Row-panel kernel: persistent CTAs walk the work items; the W rows an item
 // touches (item_rows lists them) are staged into shared memory with bulk

@@ -136,13 +136,75 @@ cudaError_t ensure_pipeline(sddmm_handle_s *h)
     return e;
 }
 
+// ---- kernel time of synchronous calls (sddmm_last_kernel_ms) ----
+
+// Brings the last call's kernel time into p->last_ms.
+cudaError_t resolve_ms(sddmm_plan_s *p)
+{
+    sddmm_handle_s *h = p->h;
+    cudaError_t e = cudaSuccess;
+    if (p->ms_state == sddmm_plan_s::MS_IN_EVENTS) {
+        e = cudaEventElapsedTime(&p->last_ms, h->ev_begin[p->ev_pair], h->ev_end[p->ev_pair]);
+    } else if (p->ms_state == sddmm_plan_s::MS_IN_CLOCK) {
+        unsigned long long t[2] = {0, 0};
+        e = cudaMemcpyAsync(t, h->d_clocks + 2 * p->clock, sizeof(t), cudaMemcpyDeviceToHost, h->own_stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->own_stream);
+        p->last_ms = t[1] > t[0] ? (float)((double)(t[1] - t[0]) * 1e-6) : 0.f;
+    }
+    p->ms_state = sddmm_plan_s::MS_KNOWN;
+    return e;
+}
+
+// Times the kernels of one call: by the kernel's own clock when the call is one launch of a kernel that has one
+// (clock() is then non-null and is passed to it), else by an event pair.  Nothing for an asynchronous call.
+struct CallTimer {
+    sddmm_plan_s *p;
+    bool async;
+    unsigned long long *clk = nullptr;
+    int pair = -1;
+    CallTimer(sddmm_plan_s *plan, bool is_async) : p(plan), async(is_async)
+    {
+        p->last_ms = -1.f;
+        p->ms_state = sddmm_plan_s::MS_KNOWN;
+    }
+    cudaError_t begin(bool kernel_has_clock, cudaStream_t s)
+    {
+        if (async) return cudaSuccess;
+        sddmm_handle_s *h = p->h;
+        if (kernel_has_clock && p->clock < 0 && !h->free_clocks.empty()) {
+            p->clock = h->free_clocks.back();
+            h->free_clocks.pop_back();
+        }
+        if (kernel_has_clock && p->clock >= 0) {
+            clk = h->d_clocks + 2 * p->clock;
+            return cudaSuccess;
+        }
+        pair = h->next_pair;
+        h->next_pair = (pair + 1) % SDDMM_EVENT_PAIRS;
+        sddmm_plan_s *before = h->ev_owner[pair];
+        if (before && before != p && before->ms_state == sddmm_plan_s::MS_IN_EVENTS && before->ev_pair == pair) {
+            cudaError_t e = resolve_ms(before);
+            if (e != cudaSuccess) return e;
+        }
+        h->ev_owner[pair] = p;
+        return cudaEventRecord(h->ev_begin[pair], s);
+    }
+    cudaError_t end(cudaStream_t s) { return pair >= 0 ? cudaEventRecord(p->h->ev_end[pair], s) : cudaSuccess; }
+    // after the synchronisation
+    void done()
+    {
+        p->ms_state = clk ? sddmm_plan_s::MS_IN_CLOCK : sddmm_plan_s::MS_IN_EVENTS;
+        p->ev_pair = pair;
+    }
+};
+
 // After a synchronising point: turn the device status word into a status code.
 int check_device_status(sddmm_handle_s *h)
 {
-    if (*h->h_status != DEV_OK) {
+    volatile int *status = h->h_status;
+    if (*status != DEV_OK) {
         h->last_error = "a bounded device-side wait (mbarrier) gave up";
-        *h->h_status = DEV_OK;
-        cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream);
+        *status = DEV_OK;
         return SDDMM_DEVICE_TIMEOUT;
     }
     return SDDMM_OK;
@@ -194,7 +256,7 @@ namespace sddmm {
 
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
-                        cudaStream_t stream)
+                        unsigned long long *clock, cudaStream_t stream)
 {
     sddmm_handle_s *h = p->h;
     rows += first;
@@ -210,7 +272,7 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
         return launch_ring(rows, (hinted ? p->d_cols_hint : cols) + first, perm, sval, W, H, P, count, p->K, hinted, h->sm_count,
                            h->d_work_counter, h->d_status, stream);
     }
-    return launch_gather(rows, cols + first, perm, sval, W, H, P, count, p->K, h->sm_count, stream);
+    return launch_gather(rows, cols + first, perm, sval, W, H, P, count, p->K, h->sm_count, clock, stream);
 }
 
 }  // namespace sddmm
@@ -261,18 +323,23 @@ int sddmm_create(sddmm_handle_t *out, int device)
         h->smem_optin = prop.sharedMemPerBlockOptin;
         e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking);
     }
-    if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
-    if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_status, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(h->d_status, 0, sizeof(int));
+    for (int i = 0; i < SDDMM_EVENT_PAIRS && e == cudaSuccess; ++i) {
+        e = cudaEventCreate(&h->ev_begin[i]);
+        if (e == cudaSuccess) e = cudaEventCreate(&h->ev_end[i]);
+    }
+    if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_clocks, 2 * sizeof(unsigned long long) * N_KERNEL_CLOCKS);
+    if (e == cudaSuccess) e = cudaMemset(h->d_clocks, 0, 2 * sizeof(unsigned long long) * N_KERNEL_CLOCKS);
     if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_work_counter, sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaHostAlloc((void **)&h->h_status, sizeof(int), cudaHostAllocDefault);
+    if (e == cudaSuccess) e = cudaHostAlloc((void **)&h->h_status, sizeof(int), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&h->d_status, h->h_status, 0);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         sddmm_destroy(h);
         return SDDMM_CUDA_ERROR;
     }
     *h->h_status = DEV_OK;
+    h->free_clocks.reserve(N_KERNEL_CLOCKS);
+    for (int i = N_KERNEL_CLOCKS - 1; i >= 0; --i) h->free_clocks.push_back(i);
     h->stream = h->own_stream;
     if (const char *env = std::getenv("SDDMM_DENSE_TENSOR")) {
         const int v = std::atoi(env);
@@ -294,9 +361,9 @@ int sddmm_destroy(sddmm_handle_t h)
     if (!h) return SDDMM_OK;
     cudaSetDevice(h->device);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
-    if (h->ev0) cudaEventDestroy(h->ev0);
-    if (h->ev1) cudaEventDestroy(h->ev1);
-    if (h->d_status) cudaFree(h->d_status);
+    for (cudaEvent_t e : h->ev_begin) if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : h->ev_end) if (e) cudaEventDestroy(e);
+    if (h->d_clocks) cudaFree(h->d_clocks);
     if (h->d_work_counter) cudaFree(h->d_work_counter);
     if (h->h_status) cudaFreeHost(h->h_status);
     if (h->pipe_compute) cudaStreamDestroy(h->pipe_compute);
@@ -516,6 +583,8 @@ int sddmm_destroy_plan(sddmm_plan_t p)
     cudaSetDevice(p->h->device);
     cudaStreamSynchronize(p->h->stream);
     free_plan_memory(p);
+    if (p->clock >= 0) p->h->free_clocks.push_back(p->clock);
+    for (sddmm_plan_s *&owner : p->h->ev_owner) if (owner == p) owner = nullptr;
     (void)cudaGetLastError();
     delete p;
     return SDDMM_OK;
@@ -525,7 +594,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
 {
     if (!p) return SDDMM_INVALID_ARG;
     sddmm_handle_s *h = p->h;
-    if (p->nnz == 0) { p->last_ms = 0.f; return SDDMM_OK; }
+    if (p->nnz == 0) { p->last_ms = 0.f; p->ms_state = sddmm_plan_s::MS_KNOWN; return SDDMM_OK; }
     if (!W || !H || !P) return SDDMM_INVALID_ARG;
     const bool use_gather = (flags & SDDMM_FLAG_KERNEL_GATHER) != 0;
     const bool tiled_out = (flags & SDDMM_FLAG_TILED_ORDER) != 0;
@@ -540,7 +609,8 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     const bool w_dev = is_device_ptr(W), h_dev = is_device_ptr(H), p_dev = is_device_ptr(P);
     const bool s_dev = Sval ? is_device_ptr(Sval) : true;
     const bool all_dev = w_dev && h_dev && p_dev && s_dev;
-    if ((flags & SDDMM_FLAG_ASYNC) && !all_dev) return SDDMM_INVALID_ARG;
+    const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
+    if (async && !all_dev) return SDDMM_INVALID_ARG;
 
     if (flags & SDDMM_FLAG_OPERANDS_BF16) {
         // W and H hold bfloat16: the TMA rings over rows of 2K bytes, products and sums in fp32.  Opt-in and
@@ -562,20 +632,17 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         if (!gather) CUDA_TRY(h, ensure_hints(p));
         p->last_kernel = "ring (bf16 operands)";
         p->last_h2d_bytes = p->last_d2h_bytes = 0;
-        CUDA_TRY(h, cudaEventRecord(h->ev0, s));
+        CallTimer timer(p, async);
+        CUDA_TRY(h, timer.begin(gather, s));
         if (gather)
-            LAUNCH_TRY(h, launch_gather_bf16(rows_p, cols_p, perm_p, Sval, W, H, P, p->nnz, p->K, h->sm_count, s));
+            LAUNCH_TRY(h, launch_gather_bf16(rows_p, cols_p, perm_p, Sval, W, H, P, p->nnz, p->K, h->sm_count, timer.clk, s));
         else
             LAUNCH_TRY(h, launch_ring_bf16(rows_p, p->d_cols_hint ? p->d_cols_hint : cols_p, perm_p, Sval, W, H, P, p->nnz, p->K,
                                            p->d_cols_hint != nullptr, h->sm_count, h->d_work_counter, h->d_status, s));
-        CUDA_TRY(h, cudaEventRecord(h->ev1, s));
-        if (flags & SDDMM_FLAG_ASYNC) {
-            p->last_ms = -1.f;
-            return SDDMM_OK;
-        }
-        CUDA_TRY(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CUDA_TRY(h, timer.end(s));
+        if (async) return SDDMM_OK;
         CUDA_TRY(h, cudaStreamSynchronize(s));
-        CUDA_TRY(h, cudaEventElapsedTime(&p->last_ms, h->ev0, h->ev1));
+        timer.done();
         return check_device_status(h);
     }
     const float *dW = W, *dH = H, *dS = Sval;
@@ -675,7 +742,8 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             CUDA_TRY(h, cudaEventRecord(h->pipe_uploaded[i], s));
             CUDA_TRY(h, cudaStreamWaitEvent(h->pipe_compute, h->pipe_uploaded[i], 0));
             CUDA_TRY(h, cudaEventRecord(h->pipe_started[i], h->pipe_compute));
-            LAUNCH_TRY(h, launch_rows(p, p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, n0, cnt, use_ring, h->pipe_compute));
+            LAUNCH_TRY(h, launch_rows(p, p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, n0, cnt, use_ring, nullptr,
+                                      h->pipe_compute));
             CUDA_TRY(h, cudaEventRecord(h->pipe_computed[i], h->pipe_compute));
             if (!p_dev) {
                 CUDA_TRY(h, cudaStreamWaitEvent(h->pipe_download, h->pipe_computed[i], 0));
@@ -687,8 +755,8 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         cudaStream_t last = p_dev ? h->pipe_compute : h->pipe_download;
         CUDA_TRY(h, cudaEventRecord(h->pipe_joined, last));
         CUDA_TRY(h, cudaStreamWaitEvent(s, h->pipe_joined, 0));
-        CUDA_TRY(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
         CUDA_TRY(h, cudaStreamSynchronize(s));
+        p->ms_state = sddmm_plan_s::MS_KNOWN;
         p->last_ms = 0.f;  // kernel time only: the chunks' kernels, not the waits for uploads between them
         for (int i = 0; i < p->n_pipe; ++i) {
             float ms = 0.f;
@@ -697,8 +765,14 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         }
         return check_device_status(h);
     }
-    CUDA_TRY(h, cudaEventRecord(h->ev0, s));
-    if (!forced && !tiled_out && p->dense.n_cells > 0) {
+    const bool use_dense = !forced && !tiled_out && p->dense.n_cells > 0;
+    const bool use_htile = p->d_ht_off && !forced && !p->d_perm;
+    // a call that is one gather launch is timed by the kernel itself, everything else by events
+    const bool one_gather = !use_dense && !use_htile && !use_panel &&
+                            !(ring_supports(p->K) && (use_ring || (!use_gather && ring_preferred(p->N, p->K))));
+    CallTimer timer(p, async);
+    CUDA_TRY(h, timer.begin(one_gather, s));
+    if (use_dense) {
         // locally dense plan: dense cells as small dense products, the rest gathered
         {
             static const char *const names[3][4] = {
@@ -719,10 +793,10 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
                                            h->dense_mode == 1, h->sm_count, s));
         if (p->dense.n_sparse > 0)
             LAUNCH_TRY(h, launch_rows(p, p->dense.rows_s, p->dense.cols_s, p->dense.perm_s, dS, dW, dH, dP, 0, p->dense.n_sparse,
-                                      false, s));
+                                      false, nullptr, s));
     } else if (use_gather) {
         p->last_kernel = "gather";
-        LAUNCH_TRY(h, launch_gather(p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, p->nnz, p->K, h->sm_count, s));
+        LAUNCH_TRY(h, launch_gather(p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, p->nnz, p->K, h->sm_count, timer.clk, s));
     } else {
         const bool tiled = p->d_perm != nullptr;
         const int32_t *rows_p = tiled ? p->d_rows_t : p->d_rows;
@@ -736,7 +810,6 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             h->last_error = "SDDMM_FLAG_TILED_ORDER with S values is not supported on a multi-tile plan";
             return SDDMM_INVALID_ARG;
         }
-        const bool use_htile = p->d_ht_off && !forced && !tiled && ((reinterpret_cast<uintptr_t>(dW) | reinterpret_cast<uintptr_t>(dH)) & 15u) == 0;
         p->last_kernel = use_htile ? "htile" : rows_class_name(p, use_panel, use_ring);
         if (use_htile)
             LAUNCH_TRY(h, launch_htile(p->d_ht_rows, p->d_ht_cols, p->d_ht_perm, dS, dW, dH, dP, p->nnz, p->N, p->K, p->ht_col_tile,
@@ -745,17 +818,13 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             LAUNCH_TRY(h, launch_panel(p->d_items, p->n_items, p->d_item_rows, rows_p, cols_p, perm, dS, dW, dH, dP, p->K,
                                      p->cfg, h->sm_count, h->d_status, s));
         else
-            LAUNCH_TRY(h, launch_rows(p, rows_p, cols_p, perm, dS, dW, dH, dP, 0, p->nnz, use_ring, s));
+            LAUNCH_TRY(h, launch_rows(p, rows_p, cols_p, perm, dS, dW, dH, dP, 0, p->nnz, use_ring, timer.clk, s));
     }
-    CUDA_TRY(h, cudaEventRecord(h->ev1, s));
+    CUDA_TRY(h, timer.end(s));
     if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dP, nbytes, cudaMemcpyDeviceToHost, s));
-    if (flags & SDDMM_FLAG_ASYNC) {
-        p->last_ms = -1.f;
-        return SDDMM_OK;
-    }
-    CUDA_TRY(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (async) return SDDMM_OK;
     CUDA_TRY(h, cudaStreamSynchronize(s));
-    CUDA_TRY(h, cudaEventElapsedTime(&p->last_ms, h->ev0, h->ev1));
+    timer.done();
     return check_device_status(h);
 }
 
@@ -883,7 +952,6 @@ int sddmm_sync(sddmm_handle_t h)
 {
     if (!h) return SDDMM_INVALID_ARG;
     CUDA_TRY(h, cudaSetDevice(h->device));
-    CUDA_TRY(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     return check_device_status(h);
 }
@@ -1045,7 +1113,9 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
         h->last_error = "W, H and Y must be 16-byte aligned on the device";
         return SDDMM_INVALID_ARG;
     }
-    CUDA_TRY(h, cudaEventRecord(h->ev0, s));
+    const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
+    CallTimer timer(p, async);
+    CUDA_TRY(h, timer.begin(false, s));
     if (p->M > 0 && ring) {
         LAUNCH_TRY(h, launch_spmm_ring(fused, p->d_spmr_tasks, p->n_spmr_tasks, p->row_groups.pcols, p->row_groups.pidx,
                                        p->row_groups.grow, dV, dW, dH, dP, dY, p->d_spmr_scratch, p->K, h->d_work_counter,
@@ -1055,17 +1125,13 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
         LAUNCH_TRY(h, launch_spmm(fused, p->d_spmm_tasks, p->n_spmm_tasks, p->d_spmm_long, p->n_spmm_long, p->d_row_ptr, p->d_cols,
                                   dV, dW, dH, dP, dY, p->d_spmm_scratch, p->K, h->d_work_counter, h->sm_count, s));
     }
-    CUDA_TRY(h, cudaEventRecord(h->ev1, s));
+    CUDA_TRY(h, timer.end(s));
     p->last_kernel = ring ? (fused ? "fused_sddmm_spmm_ring" : "spmm_ring") : (fused ? "fused_sddmm_spmm" : "spmm");
     if (!y_dev) CUDA_TRY(h, cudaMemcpyAsync(Y, dY, sizeof(float) * mk, cudaMemcpyDeviceToHost, s));
     if (P_out && !p_dev) CUDA_TRY(h, cudaMemcpyAsync(P_out, dP, sizeof(float) * nz, cudaMemcpyDeviceToHost, s));
-    if (flags & SDDMM_FLAG_ASYNC) {
-        p->last_ms = -1.f;
-        return SDDMM_OK;
-    }
-    CUDA_TRY(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (async) return SDDMM_OK;
     CUDA_TRY(h, cudaStreamSynchronize(s));
-    CUDA_TRY(h, cudaEventElapsedTime(&p->last_ms, h->ev0, h->ev1));
+    timer.done();
     return check_device_status(h);
 }
 
@@ -1101,6 +1167,7 @@ int sddmm_selftest_optin_cache(void)
 int sddmm_last_kernel_ms(sddmm_plan_t p, float *ms)
 {
     if (!p || !ms) return SDDMM_INVALID_ARG;
+    CUDA_TRY(p->h, resolve_ms(p));
     *ms = p->last_ms;
     return SDDMM_OK;
 }
@@ -1142,7 +1209,7 @@ int sddmm_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const int32_t
         dp = (float *)tmp.p[5];
     }
     CUDA_TRY(h, launch_gather((const int32_t *)dr, (const int32_t *)dc, nullptr, (const float *)ds, (const float *)dw,
-                              (const float *)dh, dp, nnz, K, h->sm_count, s));
+                              (const float *)dh, dp, nnz, K, h->sm_count, nullptr, s));
     if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dp, sizeof(float) * nnz, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
     return SDDMM_OK;
@@ -1154,7 +1221,6 @@ int sddmm_selftest_wait_timeout(sddmm_handle_t h)
     CUDA_TRY(h, cudaSetDevice(h->device));
     cudaStream_t s = h->stream;
     CUDA_TRY(h, launch_wait_timeout_probe(h->d_status, s));
-    CUDA_TRY(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
     return check_device_status(h);
 }

@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include "binning.cuh"
 #include "common.cuh"
@@ -15,16 +16,25 @@ using namespace sddmm;
 // Host-operand pipeline: S is cut into at most this many chunks of consecutive nonzeros.
 #define SDDMM_PIPE_MAX_CHUNKS 16
 
+#define SDDMM_EVENT_PAIRS 8
+
 struct sddmm_handle_s {
     int device = 0;
     int sm_count = 0;
     size_t smem_optin = 0;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    int *d_status = nullptr;  // device status word of bounded waits
+    // event pairs around the kernels of synchronous calls that no kernel clock times, taken in turn; a plan's time is
+    // read from its pair when it is asked for, or before another plan takes the pair
+    cudaEvent_t ev_begin[SDDMM_EVENT_PAIRS] = {}, ev_end[SDDMM_EVENT_PAIRS] = {};
+    sddmm_plan_s *ev_owner[SDDMM_EVENT_PAIRS] = {};
+    int next_pair = 0;
+    int *h_status = nullptr;  // status word of bounded waits, in mapped host memory
+    int *d_status = nullptr;  // its device address
     unsigned long long *d_work_counter = nullptr;  // dynamic work distribution of the ring kernel
-    int *h_status = nullptr;  // pinned mirror
+    // kernel clocks (two words each) of plans whose last synchronous call was a single gather launch
+    unsigned long long *d_clocks = nullptr;
+    std::vector<int> free_clocks;
     std::string last_error;
     // dense cells: 0 = fp32 FMA, 1 = 3xTF32 on mma.sync, 2 = 3xTF32 on tcgen05 / tensor memory (SDDMM_DENSE_TENSOR)
     int dense_mode = 2;
@@ -75,6 +85,9 @@ struct sddmm_plan_s {
     float *d_Wt = nullptr, *d_Ht = nullptr;  // device copies of K-major host operands, before their transposition
     int64_t device_bytes = 0;
     float plan_ms = 0.f, last_ms = -1.f;
+    int clock = -1;              // index of this plan's kernel clock in the handle's array
+    enum { MS_KNOWN, MS_IN_CLOCK, MS_IN_EVENTS } ms_state = MS_KNOWN;  // where the last call's kernel time is
+    int ev_pair = -1;
     // chunks of the host-operand pipeline (0 = not pipelined): nonzeros
     // [pipe_nnz[i], pipe_nnz[i+1]) touch the rows pipe_row_first[i] .. pipe_row_last[i] of W
     int n_pipe = 0;
@@ -103,9 +116,11 @@ struct sddmm_plan_s {
 
 
 namespace sddmm {
+constexpr int N_KERNEL_CLOCKS = 1024;
+
 // SDDMM over nonzeros in the plan's processing order, [first, first + count): the ring kernel when it is the faster one
 // for this plan (or forced), else the gather kernel.
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
-                        cudaStream_t stream);
+                        unsigned long long *clock, cudaStream_t stream);
 }  // namespace sddmm

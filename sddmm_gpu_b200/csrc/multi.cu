@@ -470,7 +470,7 @@ int sddmm_dist_execute(sddmm_dist_plan_t p, const float *W_local, float *H, cons
         cudaError_t e;
         if (rows_path_supports(p->K)) {
             e = launch_rows(const_cast<sddmm_plan_s *>(q), q->d_rows_t, q->d_cols_t, q->d_perm, Sval_local, W_local, H, P_local, o0,
-                            cnt, false, s);
+                            cnt, false, nullptr, s);
             if (e != cudaSuccess) return fail_cuda_m(h, e, "launching the gather kernel of an H chunk");
             ++h->n_launches;
         } else {
@@ -480,14 +480,12 @@ int sddmm_dist_execute(sddmm_dist_plan_t p, const float *W_local, float *H, cons
     }
     CU_TRY(h, cudaEventRecord(c->ev_end, s));
     if (exec_flags & SDDMM_FLAG_ASYNC) return SDDMM_OK;
-    CU_TRY(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
     CU_TRY(h, cudaStreamSynchronize(s));
     CU_TRY(h, cudaEventElapsedTime(&p->t_total, c->ev_begin, c->ev_end));
     CU_TRY(h, cudaEventElapsedTime(&p->t_bcast, c->ev_begin, c->ev_bcast_end));
-    if (*h->h_status != DEV_OK) {
+    if (*reinterpret_cast<volatile int *>(h->h_status) != DEV_OK) {
         h->last_error = "a bounded device-side wait (mbarrier) gave up";
         *h->h_status = DEV_OK;
-        cudaMemsetAsync(h->d_status, 0, sizeof(int), s);
         return SDDMM_DEVICE_TIMEOUT;
     }
     return SDDMM_OK;

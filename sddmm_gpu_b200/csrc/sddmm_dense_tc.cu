@@ -487,7 +487,7 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-    if (!ok && lane == 0) atomicExch(dev_status, (int)DEV_MBARRIER_TIMEOUT);
+    if (!ok && lane == 0) report_timeout(dev_status);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == MMA_WARP)

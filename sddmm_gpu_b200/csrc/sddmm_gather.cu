@@ -95,8 +95,9 @@ template <class S, bool HAS_PERM>
 __global__ void __launch_bounds__(GA_TPB, S::CTAS)
 sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
                     const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
-                    float *__restrict__ P, unsigned nnz, int pieces, unsigned run_len)
+                    float *__restrict__ P, unsigned nnz, int pieces, unsigned run_len, unsigned long long *clock)
 {
+    clock_begin(clock);
     constexpr int L = S::L, F = S::F, B = S::B, RB = S::RB, NB = S::NB, G = S::G;
     const int lane = threadIdx.x & 31, lig = lane & (L - 1), set = lane / L;
     const unsigned warp0 = ((blockIdx.x * GA_TPB + threadIdx.x) >> 5) * (G * run_len);  // first nonzero of this warp
@@ -190,6 +191,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
         s = sn;
         dst = dn;
     }
+    clock_end(clock);
 }
 
 // Rows of more than 256 pieces (K > 1024): a warp per nonzero, both rows in passes of 32 pieces, W through L1.
@@ -197,8 +199,9 @@ template <bool HAS_PERM>
 __global__ void __launch_bounds__(GA_TPB)
 sddmm_gather_long_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
                          const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
-                         float *__restrict__ P, unsigned nnz, int pieces)
+                         float *__restrict__ P, unsigned nnz, int pieces, unsigned long long *clock)
 {
+    clock_begin(clock);
     constexpr int U = 4;
     const int lane = threadIdx.x & 31;
     const unsigned j = (blockIdx.x * GA_TPB + threadIdx.x) >> 5;
@@ -230,12 +233,15 @@ sddmm_gather_long_kernel(const int32_t *__restrict__ rows, const int32_t *__rest
         if (sval) a *= __ldg(sval + dst);
         P[dst] = a;
     }
+    clock_end(clock);
 }
 
 template <class S, bool HAS_PERM>
 cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                           const void *H, float *P, unsigned nnz, int pieces, int sm_count, cudaStream_t stream)
+                           const void *H, float *P, unsigned nnz, int pieces, int sm_count, unsigned long long *clock, cudaStream_t stream)
 {
+    // only the last piece of a lane is predicated: the ones before it have to lie inside the row
+    if (pieces > S::L * S::F || pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
     // A set's share: 16 nonzeros (32 when a warp is one or two sets), less when the warps would not fill the SMs.
     constexpr unsigned most = S::L >= 16 ? 32 : 16;
     const unsigned resident = (unsigned)sm_count * S::CTAS * (GA_TPB / 32) * S::G;  // sets
@@ -244,25 +250,25 @@ cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32
     const unsigned per_block = run * S::G * (GA_TPB / 32);
     const unsigned blocks = (unsigned)(((uint64_t)nnz + per_block - 1) / per_block);
     sddmm_gather_kernel<S, HAS_PERM><<<blocks, GA_TPB, 0, stream>>>(rows, cols, perm, sval, static_cast<const char *>(W),
-                                                                    static_cast<const char *>(H), P, nnz, pieces, run);
+                                                                    static_cast<const char *>(H), P, nnz, pieces, run, clock);
     return cudaGetLastError();
 }
 
 template <class S>
 cudaError_t launch_shape(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                         const void *H, float *P, unsigned nnz, int pieces, int sm_count, cudaStream_t stream)
+                         const void *H, float *P, unsigned nnz, int pieces, int sm_count, unsigned long long *clock, cudaStream_t stream)
 {
-    return perm ? launch_shape_p<S, true>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, stream)
-                : launch_shape_p<S, false>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, stream);
+    return perm ? launch_shape_p<S, true>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, clock, stream)
+                : launch_shape_p<S, false>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, clock, stream);
 }
 
 }  // namespace
 
-// The shape for a row of K floats: the smallest L * F that covers its K / 4 pieces, L small enough that a set's lanes
+// The shape for a row of K floats: L * (F - 1) < K / 4 <= L * F, L small enough that a set's lanes
 // are busy and large enough that F pieces of W and B * F of H stay in few registers.  Every line is the best of a sweep
 // over (L, B, RB, prefetch, resident blocks) at a K of its range on the matrices named at the top of this file.
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const float *W,
-                          const float *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream)
+                          const float *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream)
 {
     constexpr int64_t SLICE = 1ll << 30;  // the kernels count nonzeros in 32 bits
     for (int64_t j0 = 0; j0 < nnz; j0 += SLICE) {
@@ -273,7 +279,7 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
         const int q = K / 4;
         cudaError_t e;
 #define GA_GO(L, F, B, RB, EXACT, PF, CTAS) \
-    e = launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS>>(r, c, p, s, W, H, out, n, q, sm_count, stream)
+    e = launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS>>(r, c, p, s, W, H, out, n, q, sm_count, clock, stream)
         if (q <= 4) GA_GO(4, 1, 4, 4, false, false, 6);
         else if (q < 8) GA_GO(8, 1, 4, 4, false, false, 6);
         else if (q == 8) GA_GO(8, 1, 4, 4, true, false, 6);
@@ -292,11 +298,12 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
         else if (q == 128) GA_GO(32, 4, 2, 8, true, true, 3);
         else if (q <= 160) GA_GO(32, 5, 1, 8, false, false, 4);
         else if (q <= 192) GA_GO(32, 6, 1, 8, false, false, 4);
+        else if (q <= 224) GA_GO(32, 7, 1, 8, false, false, 3);
         else if (q <= 256) GA_GO(32, 8, 1, 8, false, false, 3);
         else {
             const unsigned blocks = (n + GA_TPB / 32 - 1) / (GA_TPB / 32);
-            if (p) sddmm_gather_long_kernel<true><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q);
-            else sddmm_gather_long_kernel<false><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q);
+            if (p) sddmm_gather_long_kernel<true><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock);
+            else sddmm_gather_long_kernel<false><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock);
             e = cudaGetLastError();
         }
 #undef GA_GO
@@ -309,14 +316,14 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
 bool gather_bf16_supports(int K) { return K == 256 || K == 512; }
 
 cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                               const void *H, float *P, int64_t nnz, int K, int sm_count, cudaStream_t stream)
+                               const void *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream)
 {
     if (nnz == 0) return cudaSuccess;
     if (nnz > INT32_MAX) return cudaErrorInvalidValue;  // plans hold fewer
     const unsigned n = (unsigned)nnz;
     switch (K) {
-    case 256: return launch_shape<GatherShape<16, 2, 2, 8, true, false, 4, true>>(rows, cols, perm, sval, W, H, P, n, 32, sm_count, stream);
-    case 512: return launch_shape<GatherShape<32, 2, 2, 8, true, false, 4, true>>(rows, cols, perm, sval, W, H, P, n, 64, sm_count, stream);
+    case 256: return launch_shape<GatherShape<16, 2, 2, 8, true, false, 4, true>>(rows, cols, perm, sval, W, H, P, n, 32, sm_count, clock, stream);
+    case 512: return launch_shape<GatherShape<32, 2, 2, 8, true, false, 4, true>>(rows, cols, perm, sval, W, H, P, n, 64, sm_count, clock, stream);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -78,7 +78,7 @@ sddmm_htile_kernel(const int32_t *__restrict__ rows_t, const int32_t *__restrict
         if (!__syncthreads_and(ok)) {
             // a copy that did not arrive within the budget: report, give it one more budget to land (the
             // shared memory must not be released under a copy in flight) and leave
-            if (tid == 0) atomicExch(dev_status, (int)DEV_MBARRIER_TIMEOUT);
+            if (tid == 0) report_timeout(dev_status);
             if (!ok) mbar_wait_bounded(&bar, phase);
             return;
         }

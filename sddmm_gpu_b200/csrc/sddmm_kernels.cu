@@ -292,7 +292,7 @@ sddmm_panel_kernel(const WorkItem *__restrict__ items, int64_t n_items,
         // before leaving, make sure every copy this warp issued has landed: the
         // consumers wait for them anyway, except on the abort path
         if (timed_out) {
-            if (lane == 0) { *abort_flag = 1; atomicExch(dev_status, (int)DEV_MBARRIER_TIMEOUT); }
+            if (lane == 0) { *abort_flag = 1; report_timeout(dev_status); }
         }
     } else {
         // ---- consumer warps ----
@@ -321,7 +321,7 @@ sddmm_panel_kernel(const WorkItem *__restrict__ items, int64_t n_items,
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm->empty[b]);
         }
-        if (timed_out && lane == 0) { *abort_flag = 1; atomicExch(dev_status, (int)DEV_MBARRIER_TIMEOUT); }
+        if (timed_out && lane == 0) { *abort_flag = 1; report_timeout(dev_status); }
     }
     // Copies may only still be in flight on the abort path (otherwise every
     // issued panel was waited for by the consumers).  Give them a bounded chance
@@ -426,7 +426,7 @@ __global__ void wait_timeout_probe_kernel(int *dev_status)
         done = mbar_try_wait(&bar, 0);
         if (!done) __nanosleep(256);
     }
-    if (!done && threadIdx.x == 0) atomicExch(dev_status, (int)DEV_MBARRIER_TIMEOUT);
+    if (!done && threadIdx.x == 0) report_timeout(dev_status);
 }
 }  // namespace
 

@@ -304,7 +304,7 @@ sddmm_ring_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ 
         }
     }
     if (timed_out) {
-        if (lane == 0) atomicExch(dev_status, (int)DEV_MBARRIER_TIMEOUT);
+        if (lane == 0) report_timeout(dev_status);
         // copies issued but not consumed may still be landing in this warp's ring:
         // give each a bounded chance before the CTA's shared memory is released
         while (in_flight > 0) {

@@ -220,7 +220,7 @@ spmm_ring_kernel(const SpmmTask *__restrict__ tasks, int64_t n_tasks, const int3
             for (int64_t r = prev_row + 1; r < task.row_b; ++r) zero_row(r);
     }
     if (timed_out) {
-        if (lane == 0) atomicExch(dev_status, (int)DEV_MBARRIER_TIMEOUT);
+        if (lane == 0) report_timeout(dev_status);
         // copies issued but not read may still be landing in this warp's ring
         for (unsigned i = 0; i < in_flight && i < (unsigned)NG; ++i) {
             (void)mbar_wait_bounded(&bars[s_cons], (phase >> s_cons) & 1u);

@@ -1,0 +1,63 @@
+"""The gather kernel (csrc/sddmm_gather.cu) at the edges of its lane shapes, and the timing of small calls.
+
+Tolerance: tests/helpers.py (1e-4 of max(|ref|, sum of magnitudes) per nonzero, against the CPU oracle)."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import assert_parity, random_coo
+from sddmm_gpu_b200 import api
+
+pytestmark = pytest.mark.gpu
+
+# the first and last K of every lane shape, exact widths, and the long-row form (K > 1024)
+EDGES = [4, 16, 20, 28, 32, 36, 48, 52, 60, 64, 68, 96, 100, 124, 128, 132, 192, 196, 252, 256, 260, 320, 324, 384, 388, 508,
+         512, 516, 640, 644, 768, 772, 896, 900, 1024, 1028, 1536, 4096]
+
+
+@pytest.mark.parametrize("K", EDGES)
+def test_gather_shapes(engine, K):
+    rng = np.random.default_rng(K)
+    M, N = 97, 131
+    # one nonzero; less than a step; a partial step behind full ones; one row; rows that change at every nonzero
+    for nnz, hub in ((1, None), (7, None), (1031, None), (2000, 40)):
+        rows, cols = random_coo(rng, M, N, nnz, empty_rows=[0, 3, M - 1], hub_row=hub)
+        if rows.size == 0:
+            continue
+        vals = rng.standard_normal(rows.shape[0]).astype(np.float32)
+        W = rng.standard_normal((M, K)).astype(np.float32)
+        H = rng.standard_normal((N, K)).astype(np.float32)
+        for col_tile in (0, 50):   # 50: the nonzeros in tiled order, results through the permutation
+            plan = engine.plan_coo(M, N, rows, cols, K, 0, col_tile)
+            for sv in (vals, None):
+                P = np.full(rows.shape[0], np.nan, np.float32)
+                plan.execute(W, H, P, sv)
+                assert_parity(P, rows, cols, W, H, sv)
+            plan.close()
+        P = np.full(rows.shape[0], np.nan, np.float32)
+        engine.sddmm_coo(M, N, rows, cols, W, H, K, P, vals)
+        assert_parity(P, rows, cols, W, H, vals)
+
+
+def test_kernel_time_of_small_calls(engine):
+    # timed by the kernel's own clock; each plan keeps its own time, also when calls of other plans lie between, and an
+    # asynchronous call has none
+    rng = np.random.default_rng(1)
+    plans = []
+    for nnz in (500, 60000):
+        rows, cols = random_coo(rng, 400, 300, nnz)
+        t = [torch.from_numpy(a).cuda() for a in (rows, cols)]
+        ops = [torch.randn(n, 64, device="cuda") for n in (400, 300)]
+        plans.append((engine.plan_coo(400, 300, *t, 64), ops, torch.zeros(rows.shape[0], device="cuda")))
+    for _ in range(3):
+        for plan, (W, H), P in plans:
+            plan.execute(W, H, P)
+    times = [plan.last_kernel_ms() for plan, _, _ in plans]
+    assert all(0 < t < 1.0 for t in times)
+    assert times == [plan.last_kernel_ms() for plan, _, _ in plans]
+    plan, (W, H), P = plans[0]
+    plan.execute(W, H, P, None, api.FLAG_ASYNC)
+    assert plan.last_kernel_ms() == -1.0
+    assert plans[1][0].last_kernel_ms() == times[1]
+    for plan, _, _ in plans:
+        plan.close()
