@@ -106,12 +106,6 @@ void free_plan_memory(sddmm_plan_s *p)
     p->dense.release();
     cudaFree(p->d_used_rows);
     cudaFree(p->d_used_cols);
-    p->row_groups.release();
-    cudaFree(p->d_spmr_tasks);
-    cudaFree(p->d_spmr_long);
-    cudaFree(p->d_spmr_scratch);
-    cudaFree(p->d_spmm_tasks);
-    cudaFree(p->d_spmm_long);
     cudaFree(p->d_spmm_scratch);
     cudaFree(p->d_Wt);
     cudaFree(p->d_Ht);
@@ -1000,73 +994,6 @@ int sddmm_check_result(sddmm_plan_t p, const float *W, const float *H, const flo
 
 namespace {
 
-// Tasks of the SpMM kernels, built once per plan from the row pointer (host side: one pass over M + 1 offsets).
-int ensure_spmm_tasks(sddmm_plan_s *p)
-{
-    if (p->n_spmm_tasks >= 0) return SDDMM_OK;
-    sddmm_handle_s *h = p->h;
-    std::vector<int64_t> rp;
-    std::vector<SpmmTask> tasks;
-    std::vector<SpmmLongRow> long_rows;
-    try {
-        rp.resize((size_t)p->M + 1);
-    } catch (const std::bad_alloc &) {
-        return SDDMM_OUT_OF_MEMORY;
-    }
-    CUDA_TRY(h, cudaMemcpyAsync(rp.data(), p->d_row_ptr, sizeof(int64_t) * rp.size(), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    int64_t slots = 0;
-    try {
-        build_spmm_tasks(rp.data(), p->M, tasks, long_rows, &slots);
-    } catch (const std::bad_alloc &) {
-        return SDDMM_OUT_OF_MEMORY;
-    }
-    CUDA_TRY(h, dev_alloc(p, &p->d_spmm_tasks, tasks.size()));
-    CUDA_TRY(h, dev_alloc(p, &p->d_spmm_long, long_rows.size()));
-    CUDA_TRY(h, dev_alloc(p, &p->d_spmm_scratch, (size_t)slots * p->K));
-    if (!tasks.empty())
-        CUDA_TRY(h, cudaMemcpyAsync(p->d_spmm_tasks, tasks.data(), sizeof(SpmmTask) * tasks.size(), cudaMemcpyHostToDevice, h->stream));
-    if (!long_rows.empty())
-        CUDA_TRY(h, cudaMemcpyAsync(p->d_spmm_long, long_rows.data(), sizeof(SpmmLongRow) * long_rows.size(),
-                                    cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    p->n_spmm_tasks = (int64_t)tasks.size();
-    p->n_spmm_long = (int64_t)long_rows.size();
-    p->n_spmm_slots = slots;
-    return SDDMM_OK;
-}
-
-// The ring form's plan data: row groups (device), tasks over groups (host from the groups' row offsets).
-int ensure_spmm_ring(sddmm_plan_s *p)
-{
-    if (p->n_spmr_tasks >= 0) return SDDMM_OK;
-    sddmm_handle_s *h = p->h;
-    std::vector<int64_t> gstart;
-    std::vector<SpmmTask> tasks;
-    std::vector<SpmmLongRow> long_rows;
-    int64_t slots = 0;
-    try {
-        CUDA_TRY(h, build_row_groups(p->d_rows, p->d_cols, p->d_row_ptr, p->nnz, p->M, spmm_ring_group_slots(p->K), &p->row_groups,
-                                     &gstart, h->stream));
-        build_spmm_tasks(gstart.data(), p->M, tasks, long_rows, &slots, /*groups per task*/ 256);
-    } catch (const std::bad_alloc &) {
-        return SDDMM_OUT_OF_MEMORY;
-    }
-    p->device_bytes += (int64_t)(p->row_groups.n_groups * (8 * p->row_groups.B + 4));
-    CUDA_TRY(h, dev_alloc(p, &p->d_spmr_tasks, tasks.size()));
-    CUDA_TRY(h, dev_alloc(p, &p->d_spmr_long, long_rows.size()));
-    CUDA_TRY(h, dev_alloc(p, &p->d_spmr_scratch, (size_t)slots * p->K));
-    if (!tasks.empty())
-        CUDA_TRY(h, cudaMemcpyAsync(p->d_spmr_tasks, tasks.data(), sizeof(SpmmTask) * tasks.size(), cudaMemcpyHostToDevice, h->stream));
-    if (!long_rows.empty())
-        CUDA_TRY(h, cudaMemcpyAsync(p->d_spmr_long, long_rows.data(), sizeof(SpmmLongRow) * long_rows.size(),
-                                    cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    p->n_spmr_tasks = (int64_t)tasks.size();
-    p->n_spmr_long = (int64_t)long_rows.size();
-    return SDDMM_OK;
-}
-
 // Y = P H (fused: P = S o (W H^T) on the fly).  Host arrays are staged for the call.
 int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const float *pval, float *P_out, float *Y,
              uint32_t flags)
@@ -1076,11 +1003,11 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     if (!H || !Y || (fused && !W)) return SDDMM_INVALID_ARG;
     if (flags & ~(uint32_t)SDDMM_FLAG_ASYNC) return SDDMM_INVALID_ARG;
     CUDA_TRY(h, cudaSetDevice(h->device));
-    // long rows on the shared-memory rings (SDDMM_SPMM_RING=0: the register-staged kernel for every K)
-    bool ring = spmm_ring_supports(p->K) && p->nnz >= 65536;
+    // the class that sddmm_last_kernel_name reports (SDDMM_SPMM_RING=0: never the long-row one)
+    bool ring = ring_supports(p->K) && p->nnz >= 65536;
     if (const char *env = std::getenv("SDDMM_SPMM_RING")) ring = ring && std::atoi(env) != 0;
-    int st = ring ? ensure_spmm_ring(p) : ensure_spmm_tasks(p);
-    if (st != SDDMM_OK) return st;
+    if (!p->d_spmm_scratch && p->nnz > 0)
+        CUDA_TRY(h, dev_alloc(p, &p->d_spmm_scratch, spmm_scratch_floats(p->nnz, p->K, h->sm_count)));
     cudaStream_t s = h->stream;
     struct Tmp {
         void *p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -1115,16 +1042,10 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     }
     const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
     CallTimer timer(p, async);
-    CUDA_TRY(h, timer.begin(false, s));
-    if (p->M > 0 && ring) {
-        LAUNCH_TRY(h, launch_spmm_ring(fused, p->d_spmr_tasks, p->n_spmr_tasks, p->row_groups.pcols, p->row_groups.pidx,
-                                       p->row_groups.grow, dV, dW, dH, dP, dY, p->d_spmr_scratch, p->K, h->d_work_counter,
-                                       h->d_status, h->sm_count, s));
-        LAUNCH_TRY(h, launch_spmm_fixup(p->d_spmr_long, p->n_spmr_long, p->d_spmr_scratch, dY, p->K, s));
-    } else if (p->M > 0) {
-        LAUNCH_TRY(h, launch_spmm(fused, p->d_spmm_tasks, p->n_spmm_tasks, p->d_spmm_long, p->n_spmm_long, p->d_row_ptr, p->d_cols,
-                                  dV, dW, dH, dP, dY, p->d_spmm_scratch, p->K, h->d_work_counter, h->sm_count, s));
-    }
+    CUDA_TRY(h, timer.begin(p->M > 0, s));
+    SpmmCall call{p->d_rows, p->d_cols, p->d_row_ptr, dV, fused ? dW : nullptr, dH, dP, dY, p->d_spmm_scratch, p->M, p->nnz, p->K,
+                  timer.clk};
+    CUDA_TRY(h, launch_spmm(call, h->sm_count, &h->n_launches, s));
     CUDA_TRY(h, timer.end(s));
     p->last_kernel = ring ? (fused ? "fused_sddmm_spmm_ring" : "spmm_ring") : (fused ? "fused_sddmm_spmm" : "spmm");
     if (!y_dev) CUDA_TRY(h, cudaMemcpyAsync(Y, dY, sizeof(float) * mk, cudaMemcpyDeviceToHost, s));

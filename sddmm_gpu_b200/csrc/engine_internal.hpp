@@ -101,17 +101,7 @@ struct sddmm_plan_s {
     int64_t n_used_rows = 0, n_used_cols = 0;
     int64_t last_h2d_bytes = 0, last_d2h_bytes = 0;  // moved by the last sddmm_execute
     const char *last_kernel = "none";                // kernels the last sddmm_execute launched
-    // SpMM / fused SDDMM->SpMM over the plan's rows (built on first use): tasks, long-row table, scratch
-    SpmmTask *d_spmm_tasks = nullptr;
-    SpmmLongRow *d_spmm_long = nullptr;
-    float *d_spmm_scratch = nullptr;
-    int64_t n_spmm_tasks = -1, n_spmm_long = 0, n_spmm_slots = 0;
-    // the same for the ring form (K = 256, 512, 1024): padded row groups and tasks counted in groups
-    RowGroups row_groups;
-    SpmmTask *d_spmr_tasks = nullptr;
-    SpmmLongRow *d_spmr_long = nullptr;
-    float *d_spmr_scratch = nullptr;
-    int64_t n_spmr_tasks = -1, n_spmr_long = 0;
+    float *d_spmm_scratch = nullptr;  // partial rows of SpMM / fused SDDMM->SpMM, allocated on first use
 };
 
 

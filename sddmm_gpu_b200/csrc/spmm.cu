@@ -11,23 +11,22 @@
 //     p_i     = Pval[i]                                    (SpMM; 1 when Pval is NULL)
 //             = (sum_t W[r, t] H[col_i, t]) * Sval[i]      (fused; Sval NULL = 1)
 //
-// Shape.  Like the SDDMM gather kernels this is an integer-indexed gather bound by
-// HBM / L2, not a GEMM: per nonzero one row of H (4K bytes) comes in, once, and is
-// used twice in the fused form (for the dot product and for the update of Y).  A
-// warp owns whole rows of S: all 32 lanes work on one nonzero, lane l holding the
-// float4 pieces l, l + 32, ... of the H row, of the W row (fused) and of the Y row,
-// so the dot product is one 5-step butterfly and the update needs no exchange at
-// all; four nonzeros are in flight per warp (two at K > 512), indices one step ahead.
-// Rows are dealt out as TASKS built once per plan on the host from the row pointer:
-// runs of consecutive whole rows holding about 1024 nonzeros, and -- for rows longer
-// than that -- pieces of one row whose partial sums go to a scratch slot each and are
-// added up in a fixed order by a second, tiny kernel.  No atomics on Y: the result
-// does not depend on scheduling.
+// Shape.  The lane sets of the gather kernel (sddmm_gather.cu): a set of L lanes takes a RUN of consecutive nonzeros, one
+// at a time, lane l holding the 16-byte pieces l, l + L, ... of the H row, of the Y row being summed and (fused) of the
+// W row; B nonzeros of H are in flight per set.  When the row of S changes the set stores the finished row of Y and
+// starts the next one.  Runs are equal shares of the nonzeros whatever the rows look like, so a power-law matrix
+// loads every warp alike, and nothing is built per plan.  A row that crosses a run boundary leaves partial rows in
+// scratch -- tail[q]: run q's part of the row that goes on in run q + 1, head[q]: run q's part of a row that
+// began before it and ends in it -- and spmm_fixup_kernel adds them in run order: no atomics on Y, the result does
+// not depend on scheduling.  Rows of S without nonzeros are zeroed by blocks of their own at the end of the grid.
+//
+// What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero through L2; used twice in the fused form), hidden
+// by resident warps.  Measured on R-MAT matrices against the row-task and shared-memory-ring kernels this replaces
+// (us): SPMM_MEASURED
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
-#include <vector>
 
 #include "common.cuh"
 #include "device_utils.cuh"
@@ -38,226 +37,318 @@ using namespace dev;
 
 namespace {
 
-constexpr int SPMM_TASK_NNZ = 1024;  // nonzeros a task aims for; longer rows are cut into pieces of this size
-constexpr int SPMM_WARPS = 8;        // warps per CTA
+constexpr int SP_TPB = 256;
+constexpr int SP_NB = 8;         // nonzeros of a set per index step (4 when a set is 4 lanes)
+constexpr int SP_MAX_RUN = 1024;  // bounds the scratch of partial rows
 
-// F = float4 pieces per lane (K <= 128 F floats ... K4 <= 32 F); FUSED: p_i from W and H
-template <int F, bool FUSED>
-__global__ void __launch_bounds__(SPMM_WARPS * 32)
-spmm_rows_kernel(const SpmmTask *__restrict__ tasks, int64_t n_tasks, const int64_t *__restrict__ row_ptr,
-                 const int32_t *__restrict__ cols, const float *__restrict__ pval, const float *__restrict__ W,
-                 const float *__restrict__ H, float *__restrict__ P_out, float *__restrict__ Y, float *__restrict__ scratch,
-                 int K4, unsigned long long *work_counter)
+template <int L_, int F_, int B_, bool EXACT_, int CTAS_>
+struct SpmmShape {
+    static constexpr int L = L_, F = F_, B = B_, CTAS = CTAS_;
+    static constexpr bool EXACT = EXACT_;
+    static constexpr int NB = L < SP_NB ? L : SP_NB, G = 32 / L;
+    static_assert(NB % B == 0, "step geometry");
+};
+
+__device__ __forceinline__ void stg_u64x2(char *p, u64x2 v)
 {
-    // nonzeros in flight per warp.  Four (two for the longest rows): eight were measured slower at K = 256
-    // (19.6 ms against 16.2 ms on the scale-22 R-MAT matrix) -- the registers they take cost a resident CTA
-    constexpr int U = F >= 8 ? 2 : 4;
+    asm volatile("st.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v.a), "l"(v.b) : "memory");
+}
+__device__ __forceinline__ unsigned long long pair_of(float x)
+{
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+    return d;
+}
+
+template <class S, bool FUSED>
+__global__ void __launch_bounds__(SP_TPB, S::CTAS)
+spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const float *__restrict__ val,
+            const char *__restrict__ W, const char *__restrict__ H, float *__restrict__ P_out, char *__restrict__ Y,
+            char *__restrict__ scratch, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces,
+            unsigned run_len, unsigned gather_blocks, unsigned long long *clock)
+{
+    constexpr int L = S::L, F = S::F, B = S::B, NB = S::NB, G = S::G;
+    clock_begin(clock);
     const int lane = threadIdx.x & 31;
-    const float4 *H4 = reinterpret_cast<const float4 *>(H);
-    bool qv[F];
+    const size_t row_bytes = (size_t)pieces * 16;
+    if (blockIdx.x >= gather_blocks) {
+        // 32 rows of S per warp: those without nonzeros are written as zeros
+        const int64_t r0 = ((int64_t)(blockIdx.x - gather_blocks) * (SP_TPB / 32) + (threadIdx.x >> 5)) * 32;
+        const int64_t r = r0 + lane;
+        unsigned empty = __ballot_sync(FULL, r < M && row_ptr[r] == row_ptr[r + 1]);
+        while (empty) {
+            char *out = Y + (size_t)(r0 + __ffs(empty) - 1) * row_bytes;
+            empty &= empty - 1;
+            for (int q = lane; q < pieces; q += 32) stg_u64x2(out + q * 16, u64x2{0, 0});
+        }
+        clock_end(clock);
+        return;
+    }
+    const int lig = lane & (L - 1), set = lane / L;
+    const unsigned warp = (blockIdx.x * SP_TPB + threadIdx.x) >> 5;
+    const unsigned run = warp * G + set;
+    if (warp * G * run_len >= nnz) return;
+    const unsigned j0 = run * run_len;
+    const char *H_lane = H + lig * 16, *W_lane = W + lig * 16;
+    const bool last_ok = S::EXACT || lig + (F - 1) * L < pieces;
+    unsigned setmask = 0;
 #pragma unroll
-    for (int c = 0; c < F; ++c) qv[c] = lane + 32 * c < K4;
+    for (int g = 0; g < G; ++g) setmask |= 1u << (g * L);
 
-    // One row (or a piece of one): nonzeros [j0, j1) of row r; the sum goes to out (K floats).
-    auto run_row = [&](int64_t j0, int64_t j1, int r, float *out) {
-        float4 y[F], w[F];
+    u64x2 y[F], w[F];
 #pragma unroll
-        for (int c = 0; c < F; ++c) {
-            y[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-            w[c] = y[c];
-            if (FUSED && qv[c]) w[c] = __ldg(reinterpret_cast<const float4 *>(W) + (int64_t)r * K4 + lane + 32 * c);
-        }
-        // lanes 0..U-1 hold the columns of the step's U nonzeros
-        auto load_cols = [&](int64_t j) { return (lane < U && j + lane < j1) ? __ldcs(cols + j + lane) : 0; };
-        int cnext = j0 < j1 ? load_cols(j0) : 0;
-        for (int64_t j = j0; j < j1; j += U) {
-            const int cmine = cnext;
-            cnext = load_cols(j + U);
-            float4 h[U][F];
+    for (int f = 0; f < F; ++f) y[f] = w[f] = u64x2{0, 0};
+    auto load_w = [&](unsigned r) {
+        const char *wp = W_lane + r * row_bytes;
 #pragma unroll
-            for (int i = 0; i < U; ++i) {
-                const int ci = __shfl_sync(FULL, cmine, i);
-                const bool live = j + i < j1;
-#pragma unroll
-                for (int c = 0; c < F; ++c)
-                    h[i][c] = (live && qv[c]) ? ld_h(H4 + (int64_t)ci * K4 + lane + 32 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            float p[U];
-            if (FUSED) {
-#pragma unroll
-                for (int i = 0; i < U; ++i) {
-                    float a = 0.f;
-#pragma unroll
-                    for (int c = 0; c < F; ++c) a = dot4(w[c], h[i][c], a);
-                    p[i] = a;
-                }
-#pragma unroll
-                for (int off = 16; off >= 1; off >>= 1) {
-#pragma unroll
-                    for (int i = 0; i < U; ++i) p[i] += __shfl_xor_sync(FULL, p[i], off);
-                }
-                if (pval) {
-                    const float s = (lane < U && j + lane < j1) ? __ldcs(pval + j + lane) : 0.f;
-#pragma unroll
-                    for (int i = 0; i < U; ++i) p[i] *= __shfl_sync(FULL, s, i);
-                }
-                if (P_out) {
-                    float mine = p[0];
-#pragma unroll
-                    for (int i = 1; i < U; ++i) mine = lane == i ? p[i] : mine;
-                    if (lane < U && j + lane < j1) __stcs(P_out + j + lane, mine);
-                }
-            } else {
-                const float s = pval ? ((lane < U && j + lane < j1) ? __ldcs(pval + j + lane) : 0.f) : 1.f;
-#pragma unroll
-                for (int i = 0; i < U; ++i) p[i] = pval ? __shfl_sync(FULL, s, i) : 1.f;
-            }
-            // the nonzeros are added in their input order (dead ones carry h = 0)
-#pragma unroll
-            for (int i = 0; i < U; ++i) {
-#pragma unroll
-                for (int c = 0; c < F; ++c) {
-                    y[c].x = fmaf(p[i], h[i][c].x, y[c].x);
-                    y[c].y = fmaf(p[i], h[i][c].y, y[c].y);
-                    y[c].z = fmaf(p[i], h[i][c].z, y[c].z);
-                    y[c].w = fmaf(p[i], h[i][c].w, y[c].w);
-                }
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < F; ++c)
-            if (qv[c]) reinterpret_cast<float4 *>(out)[lane + 32 * c] = y[c];
+        for (int f = 0; f < F; ++f)
+            if (f < F - 1 || last_ok) w[f] = ldg_u64x2(wp + f * L * 16);
     };
-
-    for (;;) {
-        unsigned long long t = 0;
-        if (lane == 0) t = atomicAdd(work_counter, 1ull);
-        t = __shfl_sync(FULL, t, 0);
-        if ((int64_t)t >= n_tasks) break;
-        const SpmmTask task = tasks[t];
-        if (task.slot >= 0) {
-            run_row(task.j0, task.j1, task.row_a, scratch + (int64_t)task.slot * K4 * 4);
-        } else {
-            for (int r = task.row_a; r < task.row_b; ++r)
-                run_row(row_ptr[r], row_ptr[r + 1], r, Y + (int64_t)r * K4 * 4);
+    auto flush = [&](char *out) {
+        out += lig * 16;
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            if (f < F - 1 || last_ok) stg_u64x2(out + f * L * 16, y[f]);
+            y[f] = u64x2{0, 0};
         }
+    };
+    const int il = lig & (NB - 1);
+    unsigned j = j0 + il;
+    auto at = [&](unsigned x) { return x < nnz ? x : nnz - 1; };
+    int cur = __ldg(rows + at(j0));                                // row being summed
+    bool head = j0 > 0 && __ldg(rows + at(j0 - 1)) == cur;         // it began in an earlier run
+    if (FUSED) load_w((unsigned)cur);
+    int r, c;
+    float s = 1.f;
+    {
+        const unsigned a = at(j);
+        r = __ldg(rows + a);
+        c = __ldg(cols + a);
+        if (val) s = __ldg(val + a);
     }
+    int last = cur;  // row of the nonzero before this step
+#pragma unroll 1
+    for (unsigned step = run_len / NB; step > 0; --step) {
+        int rn = 0, cn = 0;
+        float sn = 1.f;
+        if (step > 1) {
+            const unsigned a = at(j + NB);
+            rn = __ldg(rows + a);
+            cn = __ldg(cols + a);
+            if (val) sn = __ldg(val + a);
+        }
+        int before = __shfl_up_sync(FULL, r, 1, L);
+        if (lig == 0) before = last;
+        const unsigned changed = __ballot_sync(FULL, r != before && lig < NB);
+        const unsigned valid = __ballot_sync(FULL, j < nnz && lig < NB);
+        last = __shfl_sync(FULL, r, NB - 1, L);
+        float p_mine = 0.f;
+#pragma unroll
+        for (int b = 0; b < NB; b += B) {
+            u64x2 h[B][F];
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                const unsigned cj = (unsigned)__shfl_sync(FULL, c, b + i, L);
+                const bool ok = (valid >> (set * L + b + i)) & 1u;  // past the end: nothing is added
+                const char *hp = H_lane + cj * row_bytes;
+#pragma unroll
+                for (int f = 0; f < F; ++f)
+                    h[i][f] = ok && (f < F - 1 || last_ok) ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
+            }
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                const int x = b + i;
+                if (changed & (setmask << x)) {  // uniform over the warp: some set goes on to another row
+                    const int rj = __shfl_sync(FULL, r, x, L);
+                    if ((changed >> (set * L + x)) & 1u) {
+                        flush(head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
+                        head = false;
+                        cur = rj;
+                        if (FUSED) load_w((unsigned)rj);
+                    }
+                }
+                float p = __shfl_sync(FULL, s, x, L);
+                if (FUSED) {
+                    unsigned long long a0 = 0, a1 = 0;
+#pragma unroll
+                    for (int f = 0; f < F; ++f) {
+                        a0 = ffma2(w[f].a, h[i][f].a, a0);
+                        a1 = ffma2(w[f].b, h[i][f].b, a1);
+                    }
+                    float a = fold2(a0) + fold2(a1);
+#pragma unroll
+                    for (int off = L / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
+                    p *= a;
+                    if (il == x) p_mine = p;
+                }
+                const unsigned long long pp = pair_of(p);
+#pragma unroll
+                for (int f = 0; f < F; ++f) {
+                    y[f].a = ffma2(pp, h[i][f].a, y[f].a);
+                    y[f].b = ffma2(pp, h[i][f].b, y[f].b);
+                }
+            }
+        }
+        if (FUSED && P_out && lig < NB && j < nnz) P_out[j] = p_mine;
+        j += NB;
+        r = rn;
+        c = cn;
+        s = sn;
+    }
+    if (j0 < nnz) {
+        const unsigned end = j0 + run_len;
+        const bool goes_on = end < nnz && __ldg(rows + end) == cur;
+        flush(goes_on ? scratch + (size_t)(2 * run + 1) * row_bytes
+                      : head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
+    }
+    clock_end(clock);
 }
 
-// Y[row] = sum of the row's scratch slots, in slot order.
+// Rows that cross a run boundary: Y[row] = tail[first run] + ... + tail[last run - 1] + head[last run].  A warp per
+// boundary; the one at the end of the row's first run does the row.  A row of many runs is shared by the block's warps.
 __global__ void __launch_bounds__(256)
-spmm_fixup_kernel(const SpmmLongRow *__restrict__ long_rows, int64_t n_long, const float *__restrict__ scratch,
-                  float *__restrict__ Y, int K)
+spmm_fixup_kernel(const int32_t *__restrict__ rows, const int64_t *__restrict__ row_ptr, const char *__restrict__ scratch,
+                  char *__restrict__ Y, unsigned nnz, unsigned n_runs, int pieces, unsigned run_len, unsigned long long *clock)
 {
-    for (int64_t i = blockIdx.x; i < n_long; i += gridDim.x) {
-        const SpmmLongRow lr = long_rows[i];
-        for (int t = threadIdx.x; t < K; t += blockDim.x) {
-            float s = 0.f;
-            for (int k = 0; k < lr.n_slots; ++k) s += scratch[((int64_t)lr.first_slot + k) * K + t];
-            Y[(int64_t)lr.row * K + t] = s;
+    constexpr unsigned ALONE = 64;  // partial rows a warp adds by itself
+    __shared__ unsigned many[8];    // first run of a row with more, per warp (or none)
+    __shared__ float4 part[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t row_bytes = (size_t)pieces * 16;
+    auto partial = [&](unsigned q, unsigned last, int piece) {  // run q's part of a row that ends in run `last`
+        return __ldcs(reinterpret_cast<const float4 *>(scratch + (size_t)(2 * q + (q < last ? 1 : 0)) * row_bytes) + piece);
+    };
+    auto add = [](float4 &a, float4 b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
+    auto sum = [&](unsigned q0, unsigned q1, unsigned last, int piece) {  // runs [q0, q1), in order
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        unsigned q = q0;
+        for (; q + 8 <= q1; q += 8) {
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = partial(q + u, last, piece);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) add(acc, v[u]);
+        }
+        for (; q < q1; ++q) add(acc, partial(q, last, piece));
+        return acc;
+    };
+    const unsigned q = blockIdx.x * 8 + warp;
+    unsigned row = 0, last = 0;
+    bool mine = false;
+    if (q + 1 < n_runs) {
+        const unsigned edge = (q + 1) * run_len;
+        const int r = rows[edge];
+        if (rows[edge - 1] == r && row_ptr[r] >= (int64_t)q * run_len) {
+            mine = true;
+            row = (unsigned)r;
+            last = (unsigned)((row_ptr[r + 1] - 1) / run_len);
         }
     }
+    const bool shared_row = mine && last - q + 1 > ALONE;
+    if (lane == 0) many[warp] = shared_row ? q : 0xffffffffu;
+    if (mine && !shared_row) {
+        for (int p = lane; p < pieces; p += 32)
+            reinterpret_cast<float4 *>(Y + (size_t)row * row_bytes)[p] = sum(q, last + 1, last, p);
+    }
+    if (!__syncthreads_or(shared_row)) {
+        clock_end(clock);
+        return;
+    }
+    for (int k = 0; k < 8; ++k) {
+        const unsigned f = many[k];
+        if (f == 0xffffffffu) continue;
+        const int r = rows[(f + 1) * run_len];
+        const unsigned l = (unsigned)((row_ptr[r + 1] - 1) / run_len), n = l - f + 1;
+        const unsigned a = f + (unsigned)((uint64_t)n * warp / 8), b = f + (unsigned)((uint64_t)n * (warp + 1) / 8);
+        for (int p0 = 0; p0 < pieces; p0 += 32) {
+            const int p = p0 + lane;
+            if (p < pieces) part[warp][lane] = sum(a, b, l, p);
+            __syncthreads();
+            if (warp == 0 && p < pieces) {
+                float4 acc = part[0][lane];
+                for (int w = 1; w < 8; ++w) add(acc, part[w][lane]);
+                reinterpret_cast<float4 *>(Y + (size_t)r * row_bytes)[p] = acc;
+            }
+            __syncthreads();
+        }
+    }
+    clock_end(clock);
 }
 
-template <int F>
-cudaError_t launch_rows(bool fused, const SpmmTask *tasks, int64_t n_tasks, const int64_t *row_ptr, const int32_t *cols,
-                        const float *pval, const float *W, const float *H, float *P_out, float *Y, float *scratch, int K4,
-                        unsigned long long *work_counter, int sm_count, cudaStream_t stream)
+template <class S>
+unsigned run_length(int64_t nnz, int sm_count)
 {
-    int64_t blocks = (n_tasks + SPMM_WARPS - 1) / SPMM_WARPS;
-    const int64_t cap = (int64_t)sm_count * 8;  // more than can be resident: the tasks are handed out by a counter
-    if (blocks > cap) blocks = cap;
-    if (fused)
-        spmm_rows_kernel<F, true><<<(unsigned)blocks, SPMM_WARPS * 32, 0, stream>>>(tasks, n_tasks, row_ptr, cols, pval, W, H,
-                                                                                   P_out, Y, scratch, K4, work_counter);
-    else
-        spmm_rows_kernel<F, false><<<(unsigned)blocks, SPMM_WARPS * 32, 0, stream>>>(tasks, n_tasks, row_ptr, cols, pval, W, H,
-                                                                                    P_out, Y, scratch, K4, work_counter);
+    // eight waves of resident sets even out the last one; long runs leave fewer partial rows
+    const int64_t sets = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G * 8;
+    int64_t run = nnz / sets / S::NB * S::NB;
+    if (run < 2 * S::NB) run = 2 * S::NB;
+    if (run > SP_MAX_RUN) run = SP_MAX_RUN;
+    return (unsigned)run;
+}
+
+template <class S>
+cudaError_t launch_shape(const SpmmCall &a, int sm_count, int64_t *n_launches, cudaStream_t stream)
+{
+    const int pieces = a.K / 4;
+    if (pieces > S::L * S::F || pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
+    const unsigned run = run_length<S>(a.nnz, sm_count), n_runs = (unsigned)((a.nnz + run - 1) / run);
+    const unsigned sets_per_block = SP_TPB / 32 * S::G;
+    const unsigned gather_blocks = (n_runs + sets_per_block - 1) / sets_per_block;
+    const unsigned zero_blocks = (unsigned)((a.M + SP_TPB - 1) / SP_TPB);
+    auto kern = a.W ? spmm_kernel<S, true> : spmm_kernel<S, false>;
+    kern<<<gather_blocks + zero_blocks, SP_TPB, 0, stream>>>(
+        a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H), a.P_out,
+        reinterpret_cast<char *>(a.Y), reinterpret_cast<char *>(a.scratch), a.row_ptr, (unsigned)a.nnz, a.M, pieces, run,
+        gather_blocks, a.clock);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    ++*n_launches;
+    if (n_runs < 2) return e;
+    ++*n_launches;
+    spmm_fixup_kernel<<<(n_runs - 1 + 7) / 8, 256, 0, stream>>>(a.rows, a.row_ptr, reinterpret_cast<const char *>(a.scratch),
+                                                               reinterpret_cast<char *>(a.Y), (unsigned)a.nnz, n_runs, pieces, run,
+                                                               a.clock);
     return cudaGetLastError();
+}
+
+// Calls f with the shape for K; the table of sddmm_gather.cu with registers left for the Y row.
+template <class Fn>
+auto with_shape(int K, Fn f)
+{
+    const int q = K / 4;
+    if (q <= 4) return f(SpmmShape<4, 1, 4, false, 4>());
+    if (q <= 8) return f(SpmmShape<8, 1, 4, false, 4>());
+    if (q <= 12) return f(SpmmShape<4, 3, 2, false, 4>());
+    if (q < 16) return f(SpmmShape<8, 2, 4, false, 4>());
+    if (q == 16) return f(SpmmShape<8, 2, 4, true, 4>());
+    if (q <= 24) return f(SpmmShape<8, 3, 2, false, 4>());
+    if (q < 32) return f(SpmmShape<16, 2, 4, false, 4>());
+    if (q == 32) return f(SpmmShape<16, 2, 4, true, 4>());
+    if (q <= 48) return f(SpmmShape<16, 3, 2, false, 3>());
+    if (q < 64) return f(SpmmShape<32, 2, 4, false, 3>());
+    if (q == 64) return f(SpmmShape<32, 2, 4, true, 3>());
+    if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3>());
+    if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3>());
+    if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3>());
+    if (q <= 192) return f(SpmmShape<32, 6, 1, false, 2>());
+    if (q <= 224) return f(SpmmShape<32, 7, 1, false, 2>());
+    return f(SpmmShape<32, 8, 1, false, 2>());
 }
 
 }  // namespace
 
-void build_spmm_tasks(const int64_t *row_ptr_host, int64_t M, std::vector<SpmmTask> &tasks, std::vector<SpmmLongRow> &long_rows,
-                      int64_t *n_slots, int64_t budget)
-{
-    if (budget <= 0) budget = SPMM_TASK_NNZ;
-    tasks.clear();
-    long_rows.clear();
-    int64_t slots = 0;
-    int64_t r = 0;
-    while (r < M) {
-        const int64_t n = row_ptr_host[r + 1] - row_ptr_host[r];
-        if (n > budget) {
-            // a long row: pieces of `budget` units, one scratch slot each
-            SpmmLongRow lr;
-            lr.row = (int32_t)r;
-            lr.first_slot = (int32_t)slots;
-            lr.n_slots = 0;
-            for (int64_t j = row_ptr_host[r]; j < row_ptr_host[r + 1]; j += budget) {
-                SpmmTask t;
-                t.j0 = j;
-                t.j1 = std::min<int64_t>(j + budget, row_ptr_host[r + 1]);
-                t.row_a = (int32_t)r;
-                t.row_b = (int32_t)r + 1;
-                t.slot = (int32_t)slots++;
-                t.pad = 0;
-                tasks.push_back(t);
-                ++lr.n_slots;
-            }
-            long_rows.push_back(lr);
-            ++r;
-            continue;
-        }
-        // a run of whole rows: until the next row would pass the budget (empty rows ride along; at most
-        // 4096 rows per task so that long stretches of empty rows are shared out too)
-        int64_t e = r, acc = 0;
-        while (e < M && e - r < 4096) {
-            const int64_t ne = row_ptr_host[e + 1] - row_ptr_host[e];
-            if (ne > budget || (acc > 0 && acc + ne > budget)) break;
-            acc += ne;
-            ++e;
-        }
-        SpmmTask t;
-        t.j0 = row_ptr_host[r];
-        t.j1 = row_ptr_host[e];
-        t.row_a = (int32_t)r;
-        t.row_b = (int32_t)e;
-        t.slot = -1;
-        t.pad = 0;
-        tasks.push_back(t);
-        r = e;
-    }
-    *n_slots = slots;
-}
-
 bool spmm_supports(int K) { return K > 0 && K % 4 == 0 && K <= 1024; }
 
-cudaError_t launch_spmm(bool fused, const SpmmTask *tasks, int64_t n_tasks, const SpmmLongRow *long_rows, int64_t n_long,
-                        const int64_t *row_ptr, const int32_t *cols, const float *pval, const float *W, const float *H,
-                        float *P_out, float *Y, float *scratch, int K, unsigned long long *work_counter, int sm_count,
-                        cudaStream_t stream)
+size_t spmm_scratch_floats(int64_t nnz, int K, int sm_count)
 {
-    if (n_tasks == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(work_counter, 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
-    const int K4 = K / 4;
-    const int F = (K4 + 31) / 32;
-    if (F <= 1) e = launch_rows<1>(fused, tasks, n_tasks, row_ptr, cols, pval, W, H, P_out, Y, scratch, K4, work_counter, sm_count, stream);
-    else if (F <= 2) e = launch_rows<2>(fused, tasks, n_tasks, row_ptr, cols, pval, W, H, P_out, Y, scratch, K4, work_counter, sm_count, stream);
-    else if (F <= 4) e = launch_rows<4>(fused, tasks, n_tasks, row_ptr, cols, pval, W, H, P_out, Y, scratch, K4, work_counter, sm_count, stream);
-    else if (F <= 8) e = launch_rows<8>(fused, tasks, n_tasks, row_ptr, cols, pval, W, H, P_out, Y, scratch, K4, work_counter, sm_count, stream);
-    else return cudaErrorInvalidValue;
-    if (e != cudaSuccess) return e;
-    return launch_spmm_fixup(long_rows, n_long, scratch, Y, K, stream);
+    const unsigned run = with_shape(K, [&](auto s) { return run_length<decltype(s)>(nnz, sm_count); });
+    return (size_t)((nnz + run - 1) / run) * 2 * (size_t)K;
 }
 
-cudaError_t launch_spmm_fixup(const SpmmLongRow *long_rows, int64_t n_long, const float *scratch, float *Y, int K,
-                              cudaStream_t stream)
+cudaError_t launch_spmm(const SpmmCall &a, int sm_count, int64_t *n_launches, cudaStream_t stream)
 {
-    if (n_long <= 0) return cudaSuccess;
-    spmm_fixup_kernel<<<(unsigned)std::min<int64_t>(n_long, 4096), 256, 0, stream>>>(long_rows, n_long, scratch, Y, K);
-    return cudaGetLastError();
+    if (a.M == 0) return cudaSuccess;
+    return with_shape(a.K, [&](auto s) { return launch_shape<decltype(s)>(a, sm_count, n_launches, stream); });
 }
 
 }  // namespace sddmm
