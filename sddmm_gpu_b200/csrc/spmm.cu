@@ -22,7 +22,9 @@
 //
 // What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero through L2; used twice in the fused form), hidden
 // by resident warps.  Measured on R-MAT matrices against the row-task and shared-memory-ring kernels this replaces
-// (us): SPMM_MEASURED
+// (us): SpMM, 6.0 M nonzeros, 250 K x 250 K: K = 64 755 -> 136;  0.67 M nonzeros: K = 64 379 -> 31;  fused, 16.1 M
+// nonzeros, 1 M x 1 M: K = 256 2970 -> 1735;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.
+// At K = 64 the gather kernel alone runs at 14.2 TB/s of gathered bytes.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -39,12 +41,20 @@ namespace {
 
 constexpr int SP_TPB = 256;
 constexpr int SP_NB = 8;         // nonzeros of a set per index step (4 when a set is 4 lanes)
+constexpr int SP_WAVES = 6;
 constexpr int SP_MAX_RUN = 1024;  // bounds the scratch of partial rows
 
-template <int L_, int F_, int B_, bool EXACT_, int CTAS_>
+// What a run tells the fix-up (run_row): the row that goes on in the next run, RUN_MIDDLE added when it also began before
+// this run, or RUN_ENDS.
+constexpr int RUN_ENDS = 0x7fffffff, RUN_MIDDLE = (int)0x80000000;
+
+// L lanes per nonzero, F pieces per lane, B nonzeros of a set in flight, CTAS resident blocks asked of the compiler.  PF: the
+// W rows of the next step are prefetched into L1.  JOINT: the B dot products are reduced together (fewer shuffles, more
+// registers).
+template <int L_, int F_, int B_, bool EXACT_, int CTAS_, bool FUSED_ = false, bool PF_ = false, bool JOINT_ = true>
 struct SpmmShape {
     static constexpr int L = L_, F = F_, B = B_, CTAS = CTAS_;
-    static constexpr bool EXACT = EXACT_;
+    static constexpr bool EXACT = EXACT_, FUSED = FUSED_, PF = PF_, JOINT = JOINT_;
     static constexpr int NB = L < SP_NB ? L : SP_NB, G = 32 / L;
     static_assert(NB % B == 0, "step geometry");
 };
@@ -60,14 +70,15 @@ __device__ __forceinline__ unsigned long long pair_of(float x)
     return d;
 }
 
-template <class S, bool FUSED>
+template <class S>
 __global__ void __launch_bounds__(SP_TPB, S::CTAS)
 spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const float *__restrict__ val,
             const char *__restrict__ W, const char *__restrict__ H, float *__restrict__ P_out, char *__restrict__ Y,
-            char *__restrict__ scratch, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces,
+            char *__restrict__ scratch, int *__restrict__ run_row, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces,
             unsigned run_len, unsigned gather_blocks, unsigned long long *clock)
 {
     constexpr int L = S::L, F = S::F, B = S::B, NB = S::NB, G = S::G;
+    constexpr bool FUSED = S::FUSED;
     clock_begin(clock);
     const int lane = threadIdx.x & 31;
     const size_t row_bytes = (size_t)pieces * 16;
@@ -142,6 +153,15 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         const unsigned changed = __ballot_sync(FULL, r != before && lig < NB);
         const unsigned valid = __ballot_sync(FULL, j < nnz && lig < NB);
         last = __shfl_sync(FULL, r, NB - 1, L);
+        if (FUSED && S::PF && step > 1) {
+            // the W rows that the next step opens, into L1
+            int b2 = __shfl_up_sync(FULL, rn, 1, L);
+            if (lig == 0) b2 = last;
+            if (rn != b2 && lig < NB) {
+                const char *wp = W + (unsigned)rn * row_bytes;
+                for (unsigned o = 0; o < row_bytes; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(wp + o));
+            }
+        }
         float p_mine = 0.f;
 #pragma unroll
         for (int b = 0; b < NB; b += B) {
@@ -155,20 +175,49 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                 for (int f = 0; f < F; ++f)
                     h[i][f] = ok && (f < F - 1 || last_ok) ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
             }
+            float p[B];  // the nonzeros' weights, the same in all lanes of the set
+            if (FUSED && S::JOINT) {
+                // all B products first, so that their reductions overlap: one transposed butterfly, then B broadcasts
+                float acc[B];
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    const int x = b + i;
+                    if (changed & (setmask << x)) {  // uniform over the warp: some set goes on to another row
+                        const int rj = __shfl_sync(FULL, r, x, L);
+                        if ((changed >> (set * L + x)) & 1u) load_w((unsigned)rj);
+                    }
+                    unsigned long long a0 = 0, a1 = 0;
+#pragma unroll
+                    for (int f = 0; f < F; ++f) {
+                        a0 = ffma2(w[f].a, h[i][f].a, a0);
+                        a1 = ffma2(w[f].b, h[i][f].b, a1);
+                    }
+                    acc[i] = fold2(a0) + fold2(a1);
+                }
+                reduce_transposed<L, B>(acc, lig);
+#pragma unroll
+                for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, acc[0], i * (L / B), L) * __shfl_sync(FULL, s, b + i, L);
+#pragma unroll
+                for (int i = 0; i < B; ++i)
+                    if (il == b + i) p_mine = p[i];
+            } else if (FUSED) {
+            } else {
+#pragma unroll
+                for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, s, b + i, L);
+            }
 #pragma unroll
             for (int i = 0; i < B; ++i) {
                 const int x = b + i;
-                if (changed & (setmask << x)) {  // uniform over the warp: some set goes on to another row
+                if (changed & (setmask << x)) {
                     const int rj = __shfl_sync(FULL, r, x, L);
                     if ((changed >> (set * L + x)) & 1u) {
                         flush(head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
                         head = false;
                         cur = rj;
-                        if (FUSED) load_w((unsigned)rj);
+                        if (FUSED && !S::JOINT) load_w((unsigned)rj);
                     }
                 }
-                float p = __shfl_sync(FULL, s, x, L);
-                if (FUSED) {
+                if (FUSED && !S::JOINT) {
                     unsigned long long a0 = 0, a1 = 0;
 #pragma unroll
                     for (int f = 0; f < F; ++f) {
@@ -178,10 +227,10 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                     float a = fold2(a0) + fold2(a1);
 #pragma unroll
                     for (int off = L / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
-                    p *= a;
-                    if (il == x) p_mine = p;
+                    p[i] = a * __shfl_sync(FULL, s, x, L);
+                    if (il == x) p_mine = p[i];
                 }
-                const unsigned long long pp = pair_of(p);
+                const unsigned long long pp = pair_of(p[i]);
 #pragma unroll
                 for (int f = 0; f < F; ++f) {
                     y[f].a = ffma2(pp, h[i][f].a, y[f].a);
@@ -198,22 +247,27 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     if (j0 < nnz) {
         const unsigned end = j0 + run_len;
         const bool goes_on = end < nnz && __ldg(rows + end) == cur;
+        if (lig == 0) run_row[run] = goes_on ? cur | (head ? RUN_MIDDLE : 0) : RUN_ENDS;
         flush(goes_on ? scratch + (size_t)(2 * run + 1) * row_bytes
                       : head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
     }
     clock_end(clock);
 }
 
-// Rows that cross a run boundary: Y[row] = tail[first run] + ... + tail[last run - 1] + head[last run].  A warp per
-// boundary; the one at the end of the row's first run does the row.  A row of many runs is shared by the block's warps.
+// Rows that cross a run boundary: Y[row] = tail[first run] + ... + tail[last run - 1] + head[last run].  A set of
+// lanes (1 << log_set, as many as a row has pieces, 32 at most) per run; the row's first run does the row.  Most rows
+// cross one boundary: two loads of run_row, two partial rows, one store.  A row of many runs is left to its whole block.
 __global__ void __launch_bounds__(256)
-spmm_fixup_kernel(const int32_t *__restrict__ rows, const int64_t *__restrict__ row_ptr, const char *__restrict__ scratch,
-                  char *__restrict__ Y, unsigned nnz, unsigned n_runs, int pieces, unsigned run_len, unsigned long long *clock)
+spmm_fixup_kernel(const int *__restrict__ run_row, const int64_t *__restrict__ row_ptr, const char *__restrict__ scratch,
+                  char *__restrict__ Y, unsigned n_runs, int pieces, int log_set, unsigned run_len, unsigned long long *clock)
 {
-    constexpr unsigned ALONE = 64;  // partial rows a warp adds by itself
-    __shared__ unsigned many[8];    // first run of a row with more, per warp (or none)
-    __shared__ float4 part[8][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr unsigned ALONE = 16;  // partial rows a set adds by itself
+    __shared__ unsigned many[256];  // first runs of the rows with more
+    __shared__ unsigned n_many;
+    __shared__ float4 part[256];
+    const int tid = threadIdx.x;
+    if (tid == 0) n_many = 0;
+    __syncthreads();
     const size_t row_bytes = (size_t)pieces * 16;
     auto partial = [&](unsigned q, unsigned last, int piece) {  // run q's part of a row that ends in run `last`
         return __ldcs(reinterpret_cast<const float4 *>(scratch + (size_t)(2 * q + (q < last ? 1 : 0)) * row_bytes) + piece);
@@ -232,45 +286,40 @@ spmm_fixup_kernel(const int32_t *__restrict__ rows, const int64_t *__restrict__ 
         for (; q < q1; ++q) add(acc, partial(q, last, piece));
         return acc;
     };
-    const unsigned q = blockIdx.x * 8 + warp;
-    unsigned row = 0, last = 0;
-    bool mine = false;
+    auto last_run = [&](int row) { return (unsigned)((row_ptr[row + 1] - 1) / run_len); };
+    const unsigned q = (blockIdx.x * 256 + tid) >> log_set;
+    const int lig = tid & ((1 << log_set) - 1);
     if (q + 1 < n_runs) {
-        const unsigned edge = (q + 1) * run_len;
-        const int r = rows[edge];
-        if (rows[edge - 1] == r && row_ptr[r] >= (int64_t)q * run_len) {
-            mine = true;
-            row = (unsigned)r;
-            last = (unsigned)((row_ptr[r + 1] - 1) / run_len);
-        }
-    }
-    const bool shared_row = mine && last - q + 1 > ALONE;
-    if (lane == 0) many[warp] = shared_row ? q : 0xffffffffu;
-    if (mine && !shared_row) {
-        for (int p = lane; p < pieces; p += 32)
-            reinterpret_cast<float4 *>(Y + (size_t)row * row_bytes)[p] = sum(q, last + 1, last, p);
-    }
-    if (!__syncthreads_or(shared_row)) {
-        clock_end(clock);
-        return;
-    }
-    for (int k = 0; k < 8; ++k) {
-        const unsigned f = many[k];
-        if (f == 0xffffffffu) continue;
-        const int r = rows[(f + 1) * run_len];
-        const unsigned l = (unsigned)((row_ptr[r + 1] - 1) / run_len), n = l - f + 1;
-        const unsigned a = f + (unsigned)((uint64_t)n * warp / 8), b = f + (unsigned)((uint64_t)n * (warp + 1) / 8);
-        for (int p0 = 0; p0 < pieces; p0 += 32) {
-            const int p = p0 + lane;
-            if (p < pieces) part[warp][lane] = sum(a, b, l, p);
-            __syncthreads();
-            if (warp == 0 && p < pieces) {
-                float4 acc = part[0][lane];
-                for (int w = 1; w < 8; ++w) add(acc, part[w][lane]);
-                reinterpret_cast<float4 *>(Y + (size_t)r * row_bytes)[p] = acc;
+        const int m0 = __ldg(run_row + q), m1 = __ldg(run_row + q + 1);
+        if (m0 >= 0 && m0 != RUN_ENDS) {
+            const unsigned last = m1 >= 0 ? q + 1 : last_run(m0);
+            if (last - q < ALONE) {
+                for (int p = lig; p < pieces; p += 1 << log_set)
+                    reinterpret_cast<float4 *>(Y + (size_t)m0 * row_bytes)[p] = sum(q, last + 1, last, p);
+            } else if (lig == 0) {
+                many[atomicAdd(&n_many, 1u)] = q;  // (the order of the rows does not matter, each is summed alone)
             }
-            __syncthreads();
         }
+    }
+    __syncthreads();
+    const unsigned n = n_many;
+    // a row of many runs: pieces across the threads, its runs in equal shares over the groups of threads
+    const int width = pieces < 32 ? 1 << log_set : (pieces + 31) / 32 * 32, groups = 256 / width;
+    const int piece = tid % width, group = tid / width;
+    for (unsigned k = 0; k < n; ++k) {
+        const unsigned f = many[k];
+        const int row = run_row[f];
+        const unsigned l = last_run(row), cnt = l - f + 1;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (group < groups && piece < pieces)
+            acc = sum(f + (unsigned)((uint64_t)cnt * group / groups), f + (unsigned)((uint64_t)cnt * (group + 1) / groups), l, piece);
+        part[tid] = acc;
+        __syncthreads();
+        if (group == 0 && piece < pieces) {
+            for (int g = 1; g < groups; ++g) add(acc, part[g * width + piece]);
+            reinterpret_cast<float4 *>(Y + (size_t)row * row_bytes)[piece] = acc;
+        }
+        __syncthreads();
     }
     clock_end(clock);
 }
@@ -278,8 +327,8 @@ spmm_fixup_kernel(const int32_t *__restrict__ rows, const int64_t *__restrict__ 
 template <class S>
 unsigned run_length(int64_t nnz, int sm_count)
 {
-    // eight waves of resident sets even out the last one; long runs leave fewer partial rows
-    const int64_t sets = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G * 8;
+    // a few waves of resident sets even out the last one; long runs leave fewer partial rows
+    const int64_t sets = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G * SP_WAVES;
     int64_t run = nnz / sets / S::NB * S::NB;
     if (run < 2 * S::NB) run = 2 * S::NB;
     if (run > SP_MAX_RUN) run = SP_MAX_RUN;
@@ -295,27 +344,49 @@ cudaError_t launch_shape(const SpmmCall &a, int sm_count, int64_t *n_launches, c
     const unsigned sets_per_block = SP_TPB / 32 * S::G;
     const unsigned gather_blocks = (n_runs + sets_per_block - 1) / sets_per_block;
     const unsigned zero_blocks = (unsigned)((a.M + SP_TPB - 1) / SP_TPB);
-    auto kern = a.W ? spmm_kernel<S, true> : spmm_kernel<S, false>;
-    kern<<<gather_blocks + zero_blocks, SP_TPB, 0, stream>>>(
-        a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H), a.P_out,
-        reinterpret_cast<char *>(a.Y), reinterpret_cast<char *>(a.scratch), a.row_ptr, (unsigned)a.nnz, a.M, pieces, run,
-        gather_blocks, a.clock);
+    char *const scratch = reinterpret_cast<char *>(a.scratch), *const Y = reinterpret_cast<char *>(a.Y);
+    int *const run_row = reinterpret_cast<int *>(a.scratch + (size_t)n_runs * 2 * a.K);
+    spmm_kernel<S><<<gather_blocks + zero_blocks, SP_TPB, 0, stream>>>(
+        a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H), a.P_out, Y, scratch,
+        run_row, a.row_ptr, (unsigned)a.nnz, a.M, pieces, run, gather_blocks, a.clock);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     ++*n_launches;
     if (n_runs < 2) return e;
     ++*n_launches;
-    spmm_fixup_kernel<<<(n_runs - 1 + 7) / 8, 256, 0, stream>>>(a.rows, a.row_ptr, reinterpret_cast<const char *>(a.scratch),
-                                                               reinterpret_cast<char *>(a.Y), (unsigned)a.nnz, n_runs, pieces, run,
-                                                               a.clock);
+    int log_set = 0;
+    while (log_set < 5 && (1 << log_set) < pieces) ++log_set;
+    const unsigned per_block = 256u >> log_set;
+    spmm_fixup_kernel<<<(n_runs - 1 + per_block - 1) / per_block, 256, 0, stream>>>(run_row, a.row_ptr, scratch, Y, n_runs, pieces,
+                                                                                  log_set, run, a.clock);
     return cudaGetLastError();
 }
 
-// Calls f with the shape for K; the table of sddmm_gather.cu with registers left for the Y row.
+// Calls f with the shape for K (L * (F - 1) < K / 4 <= L * F).  The fused form holds the W row as well and wants fewer
+// nonzeros in flight; every line is the best of a sweep over (L, B, prefetch, joint reduction, resident blocks).
 template <class Fn>
-auto with_shape(int K, Fn f)
+auto with_shape(int K, bool fused, Fn f)
 {
     const int q = K / 4;
+    if (fused) {
+        if (q <= 4) return f(SpmmShape<4, 1, 2, false, 4, true, true, false>());
+        if (q <= 8) return f(SpmmShape<8, 1, 2, false, 4, true, true, false>());
+        if (q <= 12) return f(SpmmShape<4, 3, 2, false, 4, true, true, false>());
+        if (q < 16) return f(SpmmShape<8, 2, 2, false, 4, true, true, false>());
+        if (q == 16) return f(SpmmShape<8, 2, 2, true, 4, true, true, false>());
+        if (q <= 24) return f(SpmmShape<8, 3, 2, false, 3, true, true, false>());
+        if (q < 32) return f(SpmmShape<16, 2, 2, false, 4, true, true, false>());
+        if (q == 32) return f(SpmmShape<16, 2, 2, true, 4, true, true, false>());
+        if (q <= 48) return f(SpmmShape<16, 3, 2, false, 3, true, true, false>());
+        if (q < 64) return f(SpmmShape<32, 2, 2, false, 4, true, true, true>());
+        if (q == 64) return f(SpmmShape<32, 2, 2, true, 4, true, true, true>());
+        if (q <= 96) return f(SpmmShape<32, 3, 1, false, 4, true, false, false>());
+        if (q <= 128) return f(SpmmShape<32, 4, 1, false, 3, true, false, false>());
+        if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3, true, false, false>());
+        if (q <= 192) return f(SpmmShape<32, 6, 1, false, 2, true, false, false>());
+        if (q <= 224) return f(SpmmShape<32, 7, 1, false, 2, true, false, false>());
+        return f(SpmmShape<32, 8, 1, false, 2, true, false, false>());
+    }
     if (q <= 4) return f(SpmmShape<4, 1, 4, false, 4>());
     if (q <= 8) return f(SpmmShape<8, 1, 4, false, 4>());
     if (q <= 12) return f(SpmmShape<4, 3, 2, false, 4>());
@@ -324,13 +395,13 @@ auto with_shape(int K, Fn f)
     if (q <= 24) return f(SpmmShape<8, 3, 2, false, 4>());
     if (q < 32) return f(SpmmShape<16, 2, 4, false, 4>());
     if (q == 32) return f(SpmmShape<16, 2, 4, true, 4>());
-    if (q <= 48) return f(SpmmShape<16, 3, 2, false, 3>());
-    if (q < 64) return f(SpmmShape<32, 2, 4, false, 3>());
-    if (q == 64) return f(SpmmShape<32, 2, 4, true, 3>());
+    if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4>());
+    if (q < 64) return f(SpmmShape<32, 2, 2, false, 5>());
+    if (q == 64) return f(SpmmShape<32, 2, 2, true, 5>());
     if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3>());
     if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3>());
     if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3>());
-    if (q <= 192) return f(SpmmShape<32, 6, 1, false, 2>());
+    if (q <= 192) return f(SpmmShape<32, 6, 1, false, 3>());
     if (q <= 224) return f(SpmmShape<32, 7, 1, false, 2>());
     return f(SpmmShape<32, 8, 1, false, 2>());
 }
@@ -341,14 +412,16 @@ bool spmm_supports(int K) { return K > 0 && K % 4 == 0 && K <= 1024; }
 
 size_t spmm_scratch_floats(int64_t nnz, int K, int sm_count)
 {
-    const unsigned run = with_shape(K, [&](auto s) { return run_length<decltype(s)>(nnz, sm_count); });
-    return (size_t)((nnz + run - 1) / run) * 2 * (size_t)K;
+    // enough for either form
+    auto run_of = [&](bool fused) { return with_shape(K, fused, [&](auto s) { return run_length<decltype(s)>(nnz, sm_count); }); };
+    const unsigned run = std::min(run_of(false), run_of(true));
+    return (size_t)((nnz + run - 1) / run) * (2 * (size_t)K + 1);  // two partial rows and one word per run
 }
 
 cudaError_t launch_spmm(const SpmmCall &a, int sm_count, int64_t *n_launches, cudaStream_t stream)
 {
     if (a.M == 0) return cudaSuccess;
-    return with_shape(a.K, [&](auto s) { return launch_shape<decltype(s)>(a, sm_count, n_launches, stream); });
+    return with_shape(a.K, a.W != nullptr, [&](auto s) { return launch_shape<decltype(s)>(a, sm_count, n_launches, stream); });
 }
 
 }  // namespace sddmm

@@ -1,0 +1,49 @@
+"""SpMM and the fused form at the run boundaries of csrc/spmm.cu: rows that end exactly where a run ends, that cross one
+boundary, that span a few runs (added by one set of lanes) and hundreds (added by a whole block), stretches of empty rows,
+and every lane shape's first and last K.
+
+Tolerance: as tests/test_gpu_spmm.py (1e-4 of the sum of magnitudes per entry of Y, against float64)."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-4
+
+
+def _rows_of_lengths(rng, lengths, N):
+    rows = np.repeat(np.arange(len(lengths)), lengths)
+    cols = np.concatenate([np.sort(rng.choice(N, n, replace=False)) for n in lengths]) if rows.size else rows
+    return rows.astype(np.int32), cols.astype(np.int32)
+
+
+@pytest.mark.parametrize("K", [4, 16, 20, 32, 36, 48, 52, 64, 68, 96, 100, 128, 132, 192, 196, 256, 260, 384, 388, 512, 516, 640,
+                               644, 768, 772, 896, 900, 1024])
+def test_run_boundaries(engine, K):
+    rng = np.random.default_rng(K)
+    N = 6000
+    # runs are 16 nonzeros at this size for most shapes (8 for K <= 16 and 36 <= K <= 48)
+    lengths = [16, 16, 0, 0, 32, 8, 8, 15, 2, 1, 1, 1, 0, 70, 250, 5000, 3, 0, 0, 0, 16, 129, 6000, 0]
+    rows, cols = _rows_of_lengths(rng, lengths, N)
+    M = len(lengths)
+    vals = rng.standard_normal(rows.shape[0]).astype(np.float32)
+    W = rng.standard_normal((M, K)).astype(np.float32)
+    H = rng.standard_normal((N, K)).astype(np.float32)
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    for pv in (vals, None):
+        Y = np.full((M, K), np.nan, np.float32)
+        plan.spmm(H, Y, pv)
+        ref, A = oracle.cpu.spmm_f64(rows, cols, H, M, pv)
+        assert np.all(np.abs(Y - ref) <= TOL * np.maximum(np.abs(ref), A) + 1e-30)
+    Y, Y2, P = np.full((M, K), np.nan, np.float32), np.full((M, K), np.nan, np.float32), np.full(rows.shape[0], np.nan, np.float32)
+    plan.fused(W, H, Y, vals, P)
+    P64, A_p = oracle.cpu.sddmm_coo_f64(rows, cols, W, H, vals)
+    assert np.all(np.abs(P - P64) <= TOL * np.maximum(np.abs(P64), A_p))
+    ref, A = oracle.cpu.spmm_f64(rows, cols, H, M, P64.astype(np.float32))
+    _, A_from_p = oracle.cpu.spmm_f64(rows, cols, H, M, A_p)   # an error of 1e-4 A_p in p moves Y by up to that times |H|
+    assert np.all(np.abs(Y - ref) <= TOL * (np.maximum(np.abs(ref), A) + A_from_p) + 1e-30)
+    plan.fused(W, H, Y2, vals)
+    assert np.array_equal(Y, Y2)
+    plan.close()
