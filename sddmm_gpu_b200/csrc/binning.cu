@@ -4,6 +4,7 @@
 // Scans, selections and the stable tile sort use CUB device primitives; the
 // passes that are specific to this engine are the kernels below.
 #include "binning.cuh"
+#include "device_utils.cuh"
 
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
@@ -15,18 +16,35 @@
 
 namespace sddmm {
 
+DevicePool *&current_pool()
+{
+    static thread_local DevicePool *pool = nullptr;
+    return pool;
+}
+cudaError_t pool_alloc(void **ptr, size_t bytes)
+{
+    if (DevicePool *p = current_pool()) return p->alloc(ptr, bytes);
+    return cudaMalloc(ptr, bytes);
+}
+void pool_free(void *ptr)
+{
+    if (!ptr) return;
+    if (DevicePool *p = current_pool()) p->free(ptr, true);
+    else cudaFree(ptr);
+}
+
 cudaError_t Scratch::reserve(size_t n)
 {
     if (n <= bytes) return cudaSuccess;
     release();
-    cudaError_t e = cudaMalloc(&ptr, n);
+    cudaError_t e = pool_alloc(&ptr, n);
     if (e == cudaSuccess) bytes = n;
     else ptr = nullptr;
     return e;
 }
 void Scratch::release()
 {
-    if (ptr) cudaFree(ptr);
+    pool_free(ptr);
     ptr = nullptr;
     bytes = 0;
 }
@@ -42,33 +60,66 @@ inline unsigned grid_for(int64_t n, int64_t cap = 148 * 32)
     return (unsigned)b;
 }
 
-__global__ void validate_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, int64_t nnz,
-                                int64_t M, int64_t N, unsigned long long *out /* [2] */)
+// One pass over the indices for everything a plan has to know before it decides anything: the first unsorted and the
+// first out-of-range nonzero and the number of rows that hold one.  words[0..3] are kept by the handle in their initial
+// state (ULLONG_MAX, ULLONG_MAX, 0, 0) between calls: the last block takes them out, resets them and writes the result
+// and the time since block 0 began to mapped host memory, so that one launch and one wait are the whole plan of an
+// ordinary matrix.  VEC: both arrays are 16-byte aligned.
+template <bool VEC>
+__global__ void __launch_bounds__(TPB)
+plan_scan_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, int64_t nnz, int64_t M, int64_t N,
+                 unsigned long long *words, unsigned long long *out /* [4], mapped */)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) words[4] = dev::globaltimer_ns();
     unsigned long long bad_sort = ULLONG_MAX, bad_range = ULLONG_MAX;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
-        const int r = rows[i], c = cols[i];
+    unsigned heads = 0;
+    auto visit = [&](int64_t i, int before, int r, int c) {
         if (r < 0 || r >= M || c < 0 || c >= N) bad_range = min(bad_range, (unsigned long long)i);
-        if (i > 0 && rows[i - 1] > r) bad_sort = min(bad_sort, (unsigned long long)i);
+        if (i > 0 && before > r) bad_sort = min(bad_sort, (unsigned long long)i);
+        heads += (i == 0 || before != r) ? 1 : 0;
+    };
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    if (VEC) {
+        for (int64_t q = t0; q < nnz / 4; q += step) {
+            const int4 r = __ldg(reinterpret_cast<const int4 *>(rows) + q), c = __ldg(reinterpret_cast<const int4 *>(cols) + q);
+            const int before = q > 0 ? __ldg(rows + 4 * q - 1) : 0;
+            visit(4 * q, before, r.x, c.x);
+            visit(4 * q + 1, r.x, r.y, c.y);
+            visit(4 * q + 2, r.y, r.z, c.z);
+            visit(4 * q + 3, r.z, r.w, c.w);
+        }
     }
-    if (bad_sort != ULLONG_MAX) atomicMin(&out[0], bad_sort);
-    if (bad_range != ULLONG_MAX) atomicMin(&out[1], bad_range);
+    for (int64_t i = (VEC ? nnz / 4 * 4 : 0) + t0; i < nnz; i += step) visit(i, i > 0 ? __ldg(rows + i - 1) : 0, __ldg(rows + i), __ldg(cols + i));
+    if (bad_sort != ULLONG_MAX) atomicMin(&words[0], bad_sort);
+    if (bad_range != ULLONG_MAX) atomicMin(&words[1], bad_range);
+    __shared__ unsigned block_heads;
+    if (threadIdx.x == 0) block_heads = 0;
+    __syncthreads();
+    heads = __reduce_add_sync(0xffffffffu, heads);
+    if ((threadIdx.x & 31) == 0 && heads) atomicAdd(&block_heads, heads);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (block_heads) atomicAdd(&words[2], (unsigned long long)block_heads);
+    __threadfence();
+    if (atomicAdd(&words[3], 1ull) + 1 < gridDim.x) return;
+    __threadfence();
+    out[0] = atomicExch(&words[0], ULLONG_MAX);
+    out[1] = atomicExch(&words[1], ULLONG_MAX);
+    out[2] = atomicExch(&words[2], 0ull);
+    words[3] = 0;
+    const unsigned long long now = dev::globaltimer_ns();
+    out[3] = now - min(now, *reinterpret_cast<volatile unsigned long long *>(&words[4]));
+    __threadfence_system();
 }
 
 // One thread per boundary i in [0, nnz]: rows (rows[i-1], rows[i]] start at i.
-__global__ void row_ptr_kernel(const int32_t *__restrict__ rows, int64_t nnz, int64_t M,
-                               int64_t *__restrict__ row_ptr, unsigned long long *nonempty)
+__global__ void row_ptr_kernel(const int32_t *__restrict__ rows, int64_t nnz, int64_t M, int64_t *__restrict__ row_ptr)
 {
-    unsigned long long heads = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= nnz; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t prev = (i == 0) ? -1 : rows[i - 1];
         const int64_t cur = (i == nnz) ? M : rows[i];
         for (int64_t r = prev + 1; r <= cur; ++r) row_ptr[r] = i;
-        if (i < nnz && cur != prev) heads++;
     }
-    // block-level sum, one atomic per warp
-    for (int o = 16; o; o >>= 1) heads += __shfl_xor_sync(0xffffffffu, heads, o);
-    if ((threadIdx.x & 31) == 0 && heads) atomicAdd(nonempty, heads);
 }
 
 __global__ void mark_cols_kernel(const int32_t *__restrict__ cols, int64_t nnz, unsigned char *mark)
@@ -205,28 +256,25 @@ __global__ void set_list_begin_kernel(WorkItem *items, int64_t n_items, const in
 
 }  // namespace
 
-cudaError_t validate_coo(const int32_t *d_rows, const int32_t *d_cols, int64_t nnz, int64_t M, int64_t N,
-                         ValidationResult *host_out, cudaStream_t stream)
+cudaError_t init_plan_words(unsigned long long *words)
 {
-    unsigned long long init[2] = {ULLONG_MAX, ULLONG_MAX}, res[2];
-    Scratch s;
-    CK(s.reserve(sizeof(init)));
-    CK(cudaMemcpyAsync(s.ptr, init, sizeof(init), cudaMemcpyHostToDevice, stream));
-    if (nnz > 0)
-        validate_kernel<<<grid_for(nnz), TPB, 0, stream>>>(d_rows, d_cols, nnz, M, N, (unsigned long long *)s.ptr);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(res, s.ptr, sizeof(res), cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
-    host_out->first_unsorted = res[0] == ULLONG_MAX ? LLONG_MAX : (long long)res[0];
-    host_out->first_out_of_range = res[1] == ULLONG_MAX ? LLONG_MAX : (long long)res[1];
-    return cudaSuccess;
+    const unsigned long long init[PLAN_WORDS] = {ULLONG_MAX, ULLONG_MAX, 0, 0, 0};
+    return cudaMemcpy(words, init, sizeof(init), cudaMemcpyHostToDevice);
 }
 
-cudaError_t build_row_ptr(const int32_t *d_rows, int64_t nnz, int64_t M, int64_t *d_row_ptr,
-                          unsigned long long *d_nonempty, cudaStream_t stream)
+cudaError_t scan_coo(const int32_t *d_rows, const int32_t *d_cols, int64_t nnz, int64_t M, int64_t N, unsigned long long *words,
+                     unsigned long long *out_mapped, cudaStream_t stream)
 {
-    CK(cudaMemsetAsync(d_nonempty, 0, sizeof(unsigned long long), stream));
-    row_ptr_kernel<<<grid_for(nnz + 1), TPB, 0, stream>>>(d_rows, nnz, M, d_row_ptr, d_nonempty);
+    const bool vec = (((uintptr_t)d_rows | (uintptr_t)d_cols) & 15u) == 0;
+    const unsigned grid = grid_for((nnz + 3) / 4, 148 * 8);
+    if (vec) plan_scan_kernel<true><<<grid, TPB, 0, stream>>>(d_rows, d_cols, nnz, M, N, words, out_mapped);
+    else plan_scan_kernel<false><<<grid, TPB, 0, stream>>>(d_rows, d_cols, nnz, M, N, words, out_mapped);
+    return cudaGetLastError();
+}
+
+cudaError_t build_row_ptr(const int32_t *d_rows, int64_t nnz, int64_t M, int64_t *d_row_ptr, cudaStream_t stream)
+{
+    row_ptr_kernel<<<grid_for(nnz + 1), TPB, 0, stream>>>(d_rows, nnz, M, d_row_ptr);
     return cudaGetLastError();
 }
 
@@ -278,7 +326,7 @@ cudaError_t select_flagged_ids(const unsigned char *flag, int64_t n, int32_t **d
     CK(cudaMemcpyAsync(&n_sel, d_n_sel, sizeof(int), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     if (n_sel > 0) {
-        CK(cudaMalloc((void **)d_list, sizeof(int32_t) * (size_t)n_sel));
+        CK(pool_alloc(d_list, (size_t)n_sel));
         CK(cudaMemcpyAsync(*d_list, ids, sizeof(int32_t) * (size_t)n_sel, cudaMemcpyDeviceToDevice, stream));
         CK(cudaStreamSynchronize(stream));
     }
@@ -364,6 +412,42 @@ cudaError_t sort_coo(int32_t *d_a, int32_t *d_b, float *d_v, int64_t nnz, bool t
     CK(cudaMemcpyAsync(d_b, b_s, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, stream));
     CK(cudaMemcpyAsync(d_v, v_s, sizeof(float) * n, cudaMemcpyDeviceToDevice, stream));
     return cudaStreamSynchronize(stream);
+}
+
+namespace {
+__global__ void pick_kernel(const int32_t *__restrict__ a, PickAt at, int n, unsigned long long *out /* mapped */)
+{
+    const int i = threadIdx.x;
+    if (i < n) out[i] = (unsigned long long)a[at.v[i]];
+    __threadfence_system();
+}
+// number of entries of the ascending list that are smaller than at.v[i]
+__global__ void rank_kernel(const int32_t *__restrict__ list, int64_t n_list, PickAt at, int n, unsigned long long *out)
+{
+    const int i = threadIdx.x;
+    if (i < n) {
+        int64_t lo = 0, hi = n_list;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (list[mid] < at.v[i]) lo = mid + 1;
+            else hi = mid;
+        }
+        out[i] = (unsigned long long)lo;
+    }
+    __threadfence_system();
+}
+}  // namespace
+
+cudaError_t pick_values(const int32_t *d_array, const PickAt &at, int n, unsigned long long *out_mapped, cudaStream_t stream)
+{
+    pick_kernel<<<1, PICK_MAX, 0, stream>>>(d_array, at, n, out_mapped);
+    return cudaGetLastError();
+}
+cudaError_t rank_values(const int32_t *d_list, int64_t n_list, const PickAt &at, int n, unsigned long long *out_mapped,
+                        cudaStream_t stream)
+{
+    rank_kernel<<<1, PICK_MAX, 0, stream>>>(d_list, n_list, at, n, out_mapped);
+    return cudaGetLastError();
 }
 
 cudaError_t build_used_row_list(const int64_t *d_row_ptr, int64_t M, int32_t **d_list, int64_t *n_list,
@@ -464,7 +548,7 @@ cudaError_t build_work_items(const int32_t *d_rows_p, const int32_t *d_cols_p, i
 
     // 4. the items
     WorkItem *items = nullptr;
-    CK(cudaMalloc(&items, sizeof(WorkItem) * (size_t)total));
+    CK(pool_alloc(&items, (size_t)total));
     fill_items_kernel<<<grid_for(total), TPB, 0, stream>>>(run_start, item_off, n_runs, total, d_rows_p, items);
     cudaError_t e = cudaGetLastError();
 
@@ -490,7 +574,7 @@ cudaError_t build_work_items(const int32_t *d_rows_p, const int32_t *d_cols_p, i
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(&n_list, list_off + total, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
-        CK(cudaMalloc(&item_rows, sizeof(int32_t) * (size_t)(n_list > 0 ? n_list : 1)));
+        CK(pool_alloc(&item_rows, (size_t)(n_list > 0 ? n_list : 1)));
         auto head_flags = thrust::make_transform_iterator(counting, ItemRowHead{d_rows_p, (const unsigned char *)flags.ptr});
         tb = 0;
         CK(cub::DeviceSelect::Flagged(nullptr, tb, d_rows_p, head_flags, item_rows, d_n_sel, n, stream));
@@ -500,8 +584,8 @@ cudaError_t build_work_items(const int32_t *d_rows_p, const int32_t *d_cols_p, i
     };
     if (e == cudaSuccess) e = body();
     if (e != cudaSuccess) {
-        cudaFree(items);
-        if (item_rows) cudaFree(item_rows);
+        pool_free(items);
+        pool_free(item_rows);
         return e;
     }
     *d_items = items;
@@ -612,6 +696,44 @@ __global__ void dense_line_ids_kernel(const int32_t *__restrict__ flag, const in
             vid[i] = -1;
         }
     }
+}
+
+// An upper bound of the nonzeros that dense cells can hold, without sorting anything: those in (nearly) full rows and
+// columns, and those in cells of the regular grid with min_count or more of the others.  A block per panel of 128 rows,
+// the panel's cell counts in shared memory; one atomic per run of nonzeros in one cell.
+__global__ void __launch_bounds__(512)
+dense_bound_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int64_t *__restrict__ row_ptr,
+                   const int32_t *__restrict__ col_deg, int64_t M, int n_cell_cols, int64_t min_row_deg, int64_t min_col_deg,
+                   int min_count, unsigned long long *bound)
+{
+    extern __shared__ int cell_count[];
+    const int64_t r0 = (int64_t)blockIdx.x * DENSE_CELL_ROWS, r1 = min(M, r0 + DENSE_CELL_ROWS);
+    const int64_t j0 = row_ptr[r0], j1 = row_ptr[r1];
+    if (j0 == j1) return;
+    for (int i = threadIdx.x; i < n_cell_cols; i += blockDim.x) cell_count[i] = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    unsigned total = 0;
+    for (int64_t jb = j0 + (threadIdx.x & ~31); jb < j1; jb += blockDim.x) {
+        const int64_t j = jb + lane;
+        int cell = -1;
+        if (j < j1) {
+            const int r = rows[j], c = cols[j];
+            if (row_ptr[r + 1] - row_ptr[r] >= min_row_deg || col_deg[c] >= min_col_deg) ++total;
+            else cell = c / DENSE_CELL_COLS;
+        }
+        const int before = __shfl_up_sync(0xffffffffu, cell, 1);
+        const unsigned head = __ballot_sync(0xffffffffu, lane == 0 || cell != before);
+        if (((head >> lane) & 1u) && cell >= 0) {
+            const unsigned above = lane == 31 ? 0u : head >> (lane + 1);
+            atomicAdd(&cell_count[cell], above ? __ffs(above) : 32 - lane);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_cell_cols; i += blockDim.x)
+        if (cell_count[i] >= min_count) total += cell_count[i];
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (lane == 0 && total) atomicAdd(bound, (unsigned long long)total);
 }
 
 struct CellGeometry {
@@ -737,8 +859,8 @@ struct NotDense {
 
 void DensePlan::release()
 {
-    cudaFree(cells); cudaFree(idx); cudaFree(rc); cudaFree(rows_s); cudaFree(cols_s); cudaFree(perm_s);
-    cudaFree(dense_rows); cudaFree(dense_cols); cudaFree(row_mask); cudaFree(row_base);
+    pool_free(cells); pool_free(idx); pool_free(rc); pool_free(rows_s); pool_free(cols_s); pool_free(perm_s);
+    pool_free(dense_rows); pool_free(dense_cols); pool_free(row_mask); pool_free(row_base);
     cells = nullptr; idx = nullptr; rc = nullptr; rows_s = cols_s = perm_s = nullptr;
     dense_rows = dense_cols = nullptr;
     row_mask = nullptr; row_base = nullptr;
@@ -767,6 +889,24 @@ cudaError_t build_dense_cells(const int32_t *d_rows, const int32_t *d_cols, cons
     col_degree_kernel<<<grid_for(nnz), TPB, 0, stream>>>(d_cols, nnz, col_deg);
     const int64_t min_row_deg = std::max<int64_t>(N / 4, 4 * DENSE_CELL_COLS);
     const int64_t min_col_deg = std::max<int64_t>(M / 4, 4 * DENSE_CELL_ROWS);
+    // most matrices that get here have no dense cells: find out before the sort
+    const int64_t n_cell_cols = (N + DENSE_CELL_COLS - 1) / DENSE_CELL_COLS;
+    if (n_cell_cols * 4 <= (200 << 10)) {
+        static SmemOptinCache optin;
+        const size_t smem = (size_t)n_cell_cols * 4;
+        if (smem > (48 << 10)) CK(optin_dynamic_smem(dense_bound_kernel, smem, optin));
+        Scratch bound;
+        CK(bound.reserve(sizeof(unsigned long long)));
+        CK(cudaMemsetAsync(bound.ptr, 0, sizeof(unsigned long long), stream));
+        dense_bound_kernel<<<(unsigned)((M + DENSE_CELL_ROWS - 1) / DENSE_CELL_ROWS), 512, smem, stream>>>(
+            d_rows, d_cols, d_row_ptr, col_deg, M, (int)n_cell_cols, min_row_deg, min_col_deg, min_count,
+            (unsigned long long *)bound.ptr);
+        CK(cudaGetLastError());
+        unsigned long long most = 0;
+        CK(cudaMemcpyAsync(&most, bound.ptr, sizeof(most), cudaMemcpyDeviceToHost, stream));
+        CK(cudaStreamSynchronize(stream));
+        if ((double)most < (double)min_share * (double)nnz) return cudaSuccess;
+    }
     dense_line_flags_kernel<<<grid_for(std::max(M, N) + 1), TPB, 0, stream>>>(d_row_ptr, M, min_row_deg, col_deg, N,
                                                                            min_col_deg, row_flag, col_flag);
     CK(cudaGetLastError());
@@ -781,8 +921,8 @@ cudaError_t build_dense_cells(const int32_t *d_rows, const int32_t *d_cols, cons
     CK(cudaMemcpyAsync(&n_dr, row_rank + M, sizeof(int), cudaMemcpyDeviceToHost, stream));
     CK(cudaMemcpyAsync(&n_dcol, col_rank + N, sizeof(int), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    CK(cudaMalloc(&out->dense_rows, sizeof(int32_t) * (size_t)(n_dr > 0 ? n_dr : 1)));
-    CK(cudaMalloc(&out->dense_cols, sizeof(int32_t) * (size_t)(n_dcol > 0 ? n_dcol : 1)));
+    CK(pool_alloc(&out->dense_rows, (size_t)(n_dr > 0 ? n_dr : 1)));
+    CK(pool_alloc(&out->dense_cols, (size_t)(n_dcol > 0 ? n_dcol : 1)));
     dense_line_ids_kernel<<<grid_for(M), TPB, 0, stream>>>(row_flag, row_rank, M, row_vid, out->dense_rows);
     dense_line_ids_kernel<<<grid_for(N), TPB, 0, stream>>>(col_flag, col_rank, N, col_vid, out->dense_cols);
     CK(cudaGetLastError());
@@ -852,9 +992,9 @@ cudaError_t build_dense_cells(const int32_t *d_rows, const int32_t *d_cols, cons
 
     // 4. the dense arrays and the remainder
     auto body = [&]() -> cudaError_t {
-        CK(cudaMalloc(&out->cells, sizeof(DenseCell) * (size_t)n_dense_cells));
-        CK(cudaMalloc(&out->idx, sizeof(int32_t) * (size_t)n_dense_nnz));
-        CK(cudaMalloc(&out->rc, sizeof(uint16_t) * (size_t)n_dense_nnz));
+        CK(pool_alloc(&out->cells, (size_t)n_dense_cells));
+        CK(pool_alloc(&out->idx, (size_t)n_dense_nnz));
+        CK(pool_alloc(&out->rc, (size_t)n_dense_nnz));
         Scratch flags;
         CK(flags.reserve((size_t)nnz));
         CK(cudaMemsetAsync(flags.ptr, 0, (size_t)nnz, stream));
@@ -865,8 +1005,8 @@ cudaError_t build_dense_cells(const int32_t *d_rows, const int32_t *d_cols, cons
         // row-mask form of the cells that allow it
         {
             const size_t lines_n = (size_t)n_dense_cells * DENSE_CELL_ROWS;
-            CK(cudaMalloc(&out->row_mask, sizeof(unsigned long long) * lines_n));
-            CK(cudaMalloc(&out->row_base, sizeof(int32_t) * lines_n));
+            CK(pool_alloc(&out->row_mask, lines_n));
+            CK(pool_alloc(&out->row_base, lines_n));
             CK(cudaMemsetAsync(out->row_mask, 0, sizeof(unsigned long long) * lines_n, stream));
             CK(cudaMemsetAsync(out->row_base, 0x7f, sizeof(int32_t) * lines_n, stream));
             Scratch cnt;
@@ -882,9 +1022,9 @@ cudaError_t build_dense_cells(const int32_t *d_rows, const int32_t *d_cols, cons
         }
         const int64_t n_sparse = nnz - n_dense_nnz;
         if (n_sparse > 0) {
-            CK(cudaMalloc(&out->perm_s, sizeof(int32_t) * (size_t)n_sparse));
-            CK(cudaMalloc(&out->rows_s, sizeof(int32_t) * (size_t)n_sparse));
-            CK(cudaMalloc(&out->cols_s, sizeof(int32_t) * (size_t)n_sparse));
+            CK(pool_alloc(&out->perm_s, (size_t)n_sparse));
+            CK(pool_alloc(&out->rows_s, (size_t)n_sparse));
+            CK(pool_alloc(&out->cols_s, (size_t)n_sparse));
             tb = 0;
             CK(cub::DeviceSelect::If(nullptr, tb, counting, out->perm_s, d_n_sel, n, NotDense{(unsigned char *)flags.ptr}, stream));
             CK(tmp.reserve(tb));

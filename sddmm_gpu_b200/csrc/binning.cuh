@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "pool.hpp"
 
 namespace sddmm {
 
@@ -20,18 +21,26 @@ struct Scratch {
     ~Scratch() { release(); }
 };
 
-// First offending nonzero index per class, or INT64_MAX when clean.
-struct ValidationResult {
-    long long first_unsorted;
-    long long first_out_of_range;
-};
-cudaError_t validate_coo(const int32_t *d_rows, const int32_t *d_cols, int64_t nnz, int64_t M,
-                         int64_t N, ValidationResult *host_out, cudaStream_t stream);
+// First look at the indices (see plan_scan_kernel): out_mapped[0] / [1] = first unsorted / out-of-range nonzero or
+// ULLONG_MAX, [2] = rows with at least one nonzero, [3] = the kernel's time in ns.  words: PLAN_WORDS device words that
+// init_plan_words has set up once.
+constexpr int PLAN_WORDS = 5;
+cudaError_t init_plan_words(unsigned long long *words);
+cudaError_t scan_coo(const int32_t *d_rows, const int32_t *d_cols, int64_t nnz, int64_t M, int64_t N, unsigned long long *words,
+                     unsigned long long *out_mapped, cudaStream_t stream);
 
-// row_ptr[r] = first nonzero of row r (M + 1 entries, empty rows repeat);
-// *d_nonempty receives the number of rows with at least one nonzero.
-cudaError_t build_row_ptr(const int32_t *d_rows, int64_t nnz, int64_t M, int64_t *d_row_ptr,
-                          unsigned long long *d_nonempty, cudaStream_t stream);
+// row_ptr[r] = first nonzero of row r (M + 1 entries, empty rows repeat).
+cudaError_t build_row_ptr(const int32_t *d_rows, int64_t nnz, int64_t M, int64_t *d_row_ptr, cudaStream_t stream);
+
+// A few entries of a device array (at.v = positions), or their ranks in an ascending list (at.v = values), to mapped host
+// memory.
+constexpr int PICK_MAX = 64;
+struct PickAt {
+    int64_t v[PICK_MAX];
+};
+cudaError_t pick_values(const int32_t *d_array, const PickAt &at, int n, unsigned long long *out_mapped, cudaStream_t stream);
+cudaError_t rank_values(const int32_t *d_list, int64_t n_list, const PickAt &at, int n, unsigned long long *out_mapped,
+                        cudaStream_t stream);
 
 // Number of distinct columns (marks a byte per column, then counts).
 cudaError_t count_distinct_cols(const int32_t *d_cols, int64_t nnz, int64_t N, int64_t *host_out,

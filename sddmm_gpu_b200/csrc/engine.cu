@@ -5,6 +5,7 @@
 // assert(), and there is exactly one kernel launch per execute.
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -83,36 +84,47 @@ template <class T>
 cudaError_t dev_alloc(sddmm_plan_s *p, T **ptr, size_t count)
 {
     size_t bytes = sizeof(T) * (count ? count : 1);
-    cudaError_t e = cudaMalloc((void **)ptr, bytes);
+    cudaError_t e = pool_alloc((void **)ptr, bytes);
     if (e == cudaSuccess) p->device_bytes += (int64_t)bytes;
     return e;
 }
 
+// Device copies that live for one call.
+struct CallTmp {
+    void *p[6] = {};
+    ~CallTmp() { for (void *q : p) pool_free(q); }
+};
+
+// What destroying a plan has to wait for: everything enqueued since the last wait, on whatever stream.
+void mark_pending(sddmm_plan_s *p, bool async, cudaStream_t s)
+{
+    p->pending = true;
+    if (!async) return;
+    if (p->async_pending && p->async_stream != s) p->async_mixed = true;
+    p->async_pending = true;
+    p->async_stream = s;
+}
+void waited_for(sddmm_plan_s *p, cudaStream_t s)
+{
+    if (p->async_mixed || (p->async_pending && p->async_stream != s)) return;
+    p->pending = p->async_pending = false;
+}
+
+// Gives the plan's memory back to the handle's pool.  Work that was enqueued and not waited for may still use it: wait
+// for the device then, as cudaFree would.
 void free_plan_memory(sddmm_plan_s *p)
 {
-    if (p->owns_rows) cudaFree(p->d_rows);
-    if (p->owns_cols) cudaFree(p->d_cols);
-    cudaFree(p->d_rows_t);
-    cudaFree(p->d_cols_t);
-    cudaFree(p->d_perm);
-    cudaFree(p->d_ht_rows);
-    cudaFree(p->d_ht_cols);
-    cudaFree(p->d_ht_perm);
-    cudaFree(p->d_ht_off);
-    cudaFree(p->d_row_ptr);
-    cudaFree(p->d_items);
-    cudaFree(p->d_item_rows);
-    cudaFree(p->d_cols_hint);
+    sddmm_handle_s *h = p->h;
+    PoolScope scope(h->pool, h->stream);
+    if (p->pending) cudaDeviceSynchronize();
+    if (p->owns_rows) pool_free(p->d_rows);
+    if (p->owns_cols) pool_free(p->d_cols);
+    for (void *q : {(void *)p->d_rows_t, (void *)p->d_cols_t, (void *)p->d_perm, (void *)p->d_ht_rows, (void *)p->d_ht_cols,
+                    (void *)p->d_ht_perm, (void *)p->d_ht_off, (void *)p->d_row_ptr, (void *)p->d_items, (void *)p->d_item_rows,
+                    (void *)p->d_cols_hint, (void *)p->d_used_rows, (void *)p->d_used_cols, (void *)p->d_spmm_scratch,
+                    (void *)p->d_Wt, (void *)p->d_Ht, (void *)p->d_W, (void *)p->d_H, (void *)p->d_S, (void *)p->d_P})
+        pool_free(q);
     p->dense.release();
-    cudaFree(p->d_used_rows);
-    cudaFree(p->d_used_cols);
-    cudaFree(p->d_spmm_scratch);
-    cudaFree(p->d_Wt);
-    cudaFree(p->d_Ht);
-    cudaFree(p->d_W);
-    cudaFree(p->d_H);
-    cudaFree(p->d_S);
-    cudaFree(p->d_P);
 }
 
 // Streams and events of the host-operand pipeline, created on first use.
@@ -213,6 +225,70 @@ const char *rows_class_name(const sddmm_plan_s *p, bool panel, bool ring)
     return p->K <= 128 ? "ring_small" : "ring";
 }
 
+// Row pointer over all rows (empty rows included).
+cudaError_t ensure_row_ptr(sddmm_plan_s *p)
+{
+    if (p->d_row_ptr) return cudaSuccess;
+    cudaError_t e = dev_alloc(p, &p->d_row_ptr, (size_t)p->M + 1);
+    if (e == cudaSuccess) e = build_row_ptr(p->d_rows, p->nnz, p->M, p->d_row_ptr, p->h->stream);
+    return e;
+}
+
+// The rows of W (0) or H (1) that are read at all.
+cudaError_t ensure_used_rows(sddmm_plan_s *p)
+{
+    if (p->d_used_rows || p->nnz == 0) return cudaSuccess;
+    cudaError_t e = ensure_row_ptr(p);
+    if (e == cudaSuccess) e = build_used_row_list(p->d_row_ptr, p->M, &p->d_used_rows, &p->n_used_rows, p->h->stream);
+    p->device_bytes += (int64_t)sizeof(int32_t) * p->n_used_rows;
+    return e;
+}
+cudaError_t ensure_used_cols(sddmm_plan_s *p)
+{
+    if (p->d_used_cols || p->nnz == 0) return cudaSuccess;
+    cudaError_t e = build_used_col_list(p->d_cols, p->nnz, p->N, &p->d_used_cols, &p->n_used_cols, p->h->stream);
+    p->device_bytes += (int64_t)sizeof(int32_t) * p->n_used_cols;
+    return e;
+}
+
+// Host-operand pipeline (sddmm_execute with W in host memory): S is cut into chunks of consecutive nonzeros, about 128 MB
+// of W rows each.  Rows are sorted, so a chunk needs one contiguous block of W rows, and W rows between two chunks
+// that no nonzero touches are never uploaded.  Here: the first and last row of every chunk and the used-row list.
+cudaError_t ensure_pipe(sddmm_plan_s *p)
+{
+    if (p->pipe_ready) return cudaSuccess;
+    sddmm_handle_s *h = p->h;
+    const int chunks = p->n_pipe;
+    cudaError_t e = ensure_used_rows(p);
+    if (e == cudaSuccess) e = ensure_used_cols(p);
+    PickAt at{};
+    for (int i = 0; i < chunks; ++i) {
+        p->pipe_nnz[i] = (p->nnz * i / chunks) & ~(int64_t)31;
+        at.v[2 * i] = p->pipe_nnz[i];
+        if (i > 0) at.v[2 * i - 1] = p->pipe_nnz[i] - 1;
+    }
+    p->pipe_nnz[chunks] = p->nnz;
+    at.v[2 * chunks - 1] = p->nnz - 1;
+    if (e == cudaSuccess) e = pick_values(p->d_rows, at, 2 * chunks, h->d_words, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return e;
+    int64_t next_row = 0;  // first row of W no earlier chunk uploads
+    for (int i = 0; i < chunks; ++i) {
+        const int64_t first = (int64_t)h->h_words[2 * i], r1 = (int64_t)h->h_words[2 * i + 1] + 1;
+        p->pipe_w_begin[i] = first > next_row ? first : next_row;
+        p->pipe_w_end[i] = r1 > p->pipe_w_begin[i] ? r1 : p->pipe_w_begin[i];
+        at.v[i] = p->pipe_w_begin[i];
+        if (r1 > next_row) next_row = r1;
+    }
+    e = rank_values(p->d_used_rows, p->n_used_rows, at, chunks, h->d_words, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return e;
+    for (int i = 0; i < chunks; ++i) p->pipe_list_begin[i] = (int64_t)h->h_words[i];
+    p->pipe_list_begin[chunks] = p->n_used_rows;
+    p->pipe_ready = true;
+    return cudaSuccess;
+}
+
 // Work items of the row-panel kernel, built when the kernel is forced or their number is asked for.
 cudaError_t ensure_items(sddmm_plan_s *p)
 {
@@ -253,6 +329,7 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
                         unsigned long long *clock, cudaStream_t stream)
 {
     sddmm_handle_s *h = p->h;
+    p->pending = true;  // (sddmm_execute clears it again when it waits)
     rows += first;
     if (perm) {
         perm += first;
@@ -324,14 +401,20 @@ int sddmm_create(sddmm_handle_t *out, int device)
     if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_clocks, 2 * sizeof(unsigned long long) * N_KERNEL_CLOCKS);
     if (e == cudaSuccess) e = cudaMemset(h->d_clocks, 0, 2 * sizeof(unsigned long long) * N_KERNEL_CLOCKS);
     if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_work_counter, sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaHostAlloc((void **)&h->h_status, sizeof(int), cudaHostAllocMapped);
+    // mapped host memory: the status word, and at 64 bytes the words that plan-time kernels answer in
+    if (e == cudaSuccess) e = cudaHostAlloc((void **)&h->h_status, 64 + sizeof(unsigned long long) * PICK_MAX, cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&h->d_status, h->h_status, 0);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_plan_words, sizeof(unsigned long long) * PLAN_WORDS);
+    if (e == cudaSuccess) e = init_plan_words(h->d_plan_words);
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreate(&h->ev_plan[i]);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         sddmm_destroy(h);
         return SDDMM_CUDA_ERROR;
     }
     *h->h_status = DEV_OK;
+    h->h_words = reinterpret_cast<volatile unsigned long long *>(h->h_status + 16);
+    h->d_words = reinterpret_cast<unsigned long long *>(h->d_status + 16);
     h->free_clocks.reserve(N_KERNEL_CLOCKS);
     for (int i = N_KERNEL_CLOCKS - 1; i >= 0; --i) h->free_clocks.push_back(i);
     h->stream = h->own_stream;
@@ -358,6 +441,9 @@ int sddmm_destroy(sddmm_handle_t h)
     for (cudaEvent_t e : h->ev_begin) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : h->ev_end) if (e) cudaEventDestroy(e);
     if (h->d_clocks) cudaFree(h->d_clocks);
+    if (h->d_plan_words) cudaFree(h->d_plan_words);
+    for (cudaEvent_t e : h->ev_plan) if (e) cudaEventDestroy(e);
+    h->pool.release();
     if (h->d_work_counter) cudaFree(h->d_work_counter);
     if (h->h_status) cudaFreeHost(h->h_status);
     if (h->pipe_compute) cudaStreamDestroy(h->pipe_compute);
@@ -398,19 +484,17 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     p->h = h;
     p->M = M; p->N = N; p->nnz = nnz; p->K = K;
     cudaStream_t s = h->stream;
-    cudaEvent_t t0 = nullptr, t1 = nullptr;
+    PoolScope scope(h->pool, s);
 
-#define PLAN_TRY(expr)                                 \
-    do {                                               \
-        cudaError_t _e = (expr);                       \
-        if (_e != cudaSuccess) {                       \
-            int _st = fail_cuda(h, _e, #expr);         \
-            free_plan_memory(p);                       \
-            delete p;                                  \
-            if (t0) cudaEventDestroy(t0);              \
-            if (t1) cudaEventDestroy(t1);              \
-            return _st;                                \
-        }                                              \
+    auto drop = [&](int st) {
+        free_plan_memory(p);
+        delete p;
+        return st;
+    };
+#define PLAN_TRY(expr)                                                      \
+    do {                                                                    \
+        cudaError_t _e = (expr);                                            \
+        if (_e != cudaSuccess) return drop(fail_cuda(h, _e, #expr));        \
     } while (0)
 
     const bool dev_idx = (flags & SDDMM_PLAN_DEVICE_INDICES) != 0;
@@ -433,38 +517,27 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
             PLAN_TRY(cudaMemcpyAsync(p->d_cols, cols, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, s));
         }
     }
-    PLAN_TRY(cudaEventCreate(&t0));
-    PLAN_TRY(cudaEventCreate(&t1));
-    PLAN_TRY(cudaEventRecord(t0, s));
-
-    if (!(flags & SDDMM_PLAN_SKIP_VALIDATION)) {
-        ValidationResult vr;
-        PLAN_TRY(validate_coo(p->d_rows, p->d_cols, nnz, M, N, &vr, s));
-        if (vr.first_out_of_range != LLONG_MAX || vr.first_unsorted != LLONG_MAX) {
-            char buf[160];
-            const bool oob = vr.first_out_of_range != LLONG_MAX;
-            snprintf(buf, sizeof(buf), "%s at nonzero %lld", oob ? "index out of range" : "rows not sorted",
-                     oob ? vr.first_out_of_range : vr.first_unsorted);
-            h->last_error = buf;
-            free_plan_memory(p);
-            delete p;
-            cudaEventDestroy(t0);
-            cudaEventDestroy(t1);
-            return oob ? SDDMM_INDEX_OUT_OF_RANGE : SDDMM_UNSORTED_INPUT;
-        }
-    }
-
-    // row pointer over all rows (empty rows included)
-    PLAN_TRY(dev_alloc(p, &p->d_row_ptr, (size_t)M + 1));
-    {
-        Scratch cnt;
-        PLAN_TRY(cnt.reserve(sizeof(unsigned long long)));
-        PLAN_TRY(build_row_ptr(p->d_rows, nnz, M, p->d_row_ptr, (unsigned long long *)cnt.ptr, s));
-        unsigned long long ne = 0;
-        PLAN_TRY(cudaMemcpyAsync(&ne, cnt.ptr, sizeof(ne), cudaMemcpyDeviceToHost, s));
+    if (nnz > 0) {
+        PLAN_TRY(scan_coo(p->d_rows, p->d_cols, nnz, M, N, h->d_plan_words, h->d_words, s));
         PLAN_TRY(cudaStreamSynchronize(s));
-        p->n_nonempty_rows = (int64_t)ne;
+        const unsigned long long unsorted = h->h_words[0], oob = h->h_words[1];
+        if (!(flags & SDDMM_PLAN_SKIP_VALIDATION) && (unsorted != ULLONG_MAX || oob != ULLONG_MAX)) {
+            char buf[160];
+            snprintf(buf, sizeof(buf), "%s at nonzero %llu", oob != ULLONG_MAX ? "index out of range" : "rows not sorted",
+                     oob != ULLONG_MAX ? oob : unsorted);
+            h->last_error = buf;
+            return drop(oob != ULLONG_MAX ? SDDMM_INDEX_OUT_OF_RANGE : SDDMM_UNSORTED_INPUT);
+        }
+        p->n_nonempty_rows = (int64_t)h->h_words[2];
+        p->plan_ms = (float)((double)h->h_words[3] * 1e-6);
     }
+    // everything after the first look is timed by events, and only if there is anything
+    bool more = false;
+    auto begin_more = [&]() -> cudaError_t {
+        if (more) return cudaSuccess;
+        more = true;
+        return cudaEventRecord(h->ev_plan[0], s);
+    };
 
     // column tiles: a hint >= N (or <= 0) means one tile, the identity order
     p->cfg = choose_panel_config(K, panel_rows_hint, h->sm_count, h->smem_optin);
@@ -473,6 +546,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     p->n_col_tiles = (int)((N + ct - 1) / ct);
     if (p->n_col_tiles < 1) p->n_col_tiles = 1;
     if (p->n_col_tiles > 1 && nnz > 0) {
+        PLAN_TRY(begin_more());
         PLAN_TRY(dev_alloc(p, &p->d_perm, (size_t)nnz));
         PLAN_TRY(dev_alloc(p, &p->d_rows_t, (size_t)nnz));
         PLAN_TRY(dev_alloc(p, &p->d_cols_t, (size_t)nnz));
@@ -486,6 +560,8 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         const char *env = std::getenv("SDDMM_DENSE_CELLS");
         const bool enabled = !(env && std::atoi(env) == 0);
         if (enabled && p->n_col_tiles == 1 && p->n_nonempty_rows > 0 && nnz / p->n_nonempty_rows >= 32) {
+            PLAN_TRY(begin_more());
+            PLAN_TRY(ensure_row_ptr(p));
             PLAN_TRY(build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, nnz, M, N, 0.25f, 0.5f, &p->dense, s));
             if (p->dense.n_cells > 0)
                 p->device_bytes += (int64_t)(sizeof(DenseCell) * p->dense.n_cells + 6 * p->dense.n_dense_nnz +
@@ -498,7 +574,10 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         int64_t budget_mb = 64;  // best of a 16..128 MB sweep on the scale-22 R-MAT matrix at K = 256
         if (const char *env = std::getenv("SDDMM_L2_HUB_MB")) budget_mb = std::atoll(env);
         p->hub_budget = budget_mb > 0 ? budget_mb * (1ll << 20) : 0;
-        if (ring_preferred(N, K)) PLAN_TRY(ensure_hints(p));
+        if (ring_preferred(N, K)) {
+            PLAN_TRY(begin_more());
+            PLAN_TRY(ensure_hints(p));
+        }
     }
     // Few columns and many nonzeros per column (a bag-of-words matrix): H is a handful of shared-memory tiles, and
     // the column-tile kernel reads every H row of a nonzero from shared memory.  Worth it when a CTA's share of
@@ -509,6 +588,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         const int64_t n_tiles = tc > 0 ? (N + tc - 1) / tc : 0;
         if (!(env && std::atoi(env) == 0) && tc > 0 && p->n_col_tiles == 1 && p->dense.n_cells == 0 && n_tiles >= 1 &&
             n_tiles <= 64 && nnz >= 65536 && nnz / h->sm_count >= 8 * (int64_t)tc) {
+            PLAN_TRY(begin_more());
             PLAN_TRY(dev_alloc(p, &p->d_ht_perm, (size_t)nnz));
             PLAN_TRY(dev_alloc(p, &p->d_ht_rows, (size_t)nnz));
             PLAN_TRY(dev_alloc(p, &p->d_ht_cols, (size_t)nnz));
@@ -519,54 +599,20 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
             p->ht_n_tiles = (int)n_tiles;
         }
     }
-    // Host-operand pipeline (sddmm_execute with W in host memory): cut S into chunks
-    // of consecutive nonzeros, about 128 MB of W rows each, and note the first and
-    // last row of every chunk -- rows are sorted, so a chunk needs one contiguous
-    // block of W rows, and W rows between two chunks that no nonzero touches are
-    // never uploaded.
+    // chunks of the host-operand pipeline; what they need is built by the first call with host operands
     if (p->n_col_tiles == 1 && p->dense.n_cells == 0 && nnz >= (1 << 20)) {
-        int64_t chunks = (int64_t)sizeof(float) * M * K / (128ll << 20);
-        if (chunks > SDDMM_PIPE_MAX_CHUNKS) chunks = SDDMM_PIPE_MAX_CHUNKS;
-        if (chunks >= 2) {
-            for (int i = 0; i < chunks; ++i) p->pipe_nnz[i] = (nnz * i / chunks) & ~(int64_t)31;
-            p->pipe_nnz[chunks] = nnz;
-            for (int i = 0; i < chunks; ++i) {
-                PLAN_TRY(cudaMemcpyAsync(&p->pipe_row_first[i], p->d_rows + p->pipe_nnz[i], sizeof(int32_t),
-                                         cudaMemcpyDeviceToHost, s));
-                PLAN_TRY(cudaMemcpyAsync(&p->pipe_row_last[i], p->d_rows + p->pipe_nnz[i + 1] - 1, sizeof(int32_t),
-                                         cudaMemcpyDeviceToHost, s));
-            }
-            p->n_pipe = (int)chunks;
-            // the rows of W and H that are read at all, for the row upload from mapped host memory
-            PLAN_TRY(build_used_row_list(p->d_row_ptr, M, &p->d_used_rows, &p->n_used_rows, s));
-            PLAN_TRY(build_used_col_list(p->d_cols, nnz, N, &p->d_used_cols, &p->n_used_cols, s));
-            p->device_bytes += (int64_t)sizeof(int32_t) * (p->n_used_rows + p->n_used_cols);
-            std::vector<int32_t> used;
-            try {
-                used.resize((size_t)p->n_used_rows);
-            } catch (const std::bad_alloc &) {
-                PLAN_TRY(cudaErrorMemoryAllocation);
-            }
-            PLAN_TRY(cudaMemcpyAsync(used.data(), p->d_used_rows, sizeof(int32_t) * used.size(), cudaMemcpyDeviceToHost, s));
-            PLAN_TRY(cudaStreamSynchronize(s));  // also completes the copies of the chunks' first and last rows
-            int64_t next_row = 0;  // first row of W no earlier chunk uploads
-            for (int i = 0; i < chunks; ++i) {
-                const int64_t r0 = p->pipe_row_first[i] > next_row ? p->pipe_row_first[i] : next_row;
-                const int64_t r1 = (int64_t)p->pipe_row_last[i] + 1;
-                p->pipe_w_begin[i] = r0;
-                p->pipe_w_end[i] = r1 > r0 ? r1 : r0;
-                p->pipe_list_begin[i] = std::lower_bound(used.begin(), used.end(), (int32_t)r0) - used.begin();
-                if (r1 > next_row) next_row = r1;
-            }
-            p->pipe_list_begin[chunks] = (int64_t)used.size();
-        }
+        const int64_t chunks = std::min<int64_t>((int64_t)sizeof(float) * M * K / (128ll << 20), SDDMM_PIPE_MAX_CHUNKS);
+        if (chunks >= 2) p->n_pipe = (int)chunks;
     }
-    PLAN_TRY(cudaEventRecord(t1, s));
-    PLAN_TRY(cudaEventSynchronize(t1));
-    PLAN_TRY(cudaEventElapsedTime(&p->plan_ms, t0, t1));
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
+    if (more) {
+        PLAN_TRY(cudaEventRecord(h->ev_plan[1], s));
+        PLAN_TRY(cudaEventSynchronize(h->ev_plan[1]));
+        float ms = 0.f;
+        PLAN_TRY(cudaEventElapsedTime(&ms, h->ev_plan[0], h->ev_plan[1]));
+        p->plan_ms += ms;
+    }
 #undef PLAN_TRY
+    h->pool.settle(s);
     *out = p;
     return SDDMM_OK;
 }
@@ -575,7 +621,6 @@ int sddmm_destroy_plan(sddmm_plan_t p)
 {
     if (!p) return SDDMM_OK;
     cudaSetDevice(p->h->device);
-    cudaStreamSynchronize(p->h->stream);
     free_plan_memory(p);
     if (p->clock >= 0) p->h->free_clocks.push_back(p->clock);
     for (sddmm_plan_s *&owner : p->h->ev_owner) if (owner == p) owner = nullptr;
@@ -599,12 +644,14 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (use_gather && tiled_out && p->d_perm) return SDDMM_INVALID_ARG;
     CUDA_TRY(h, cudaSetDevice(h->device));
     cudaStream_t s = h->stream;
+    PoolScope scope(h->pool, s);
 
     const bool w_dev = is_device_ptr(W), h_dev = is_device_ptr(H), p_dev = is_device_ptr(P);
     const bool s_dev = Sval ? is_device_ptr(Sval) : true;
     const bool all_dev = w_dev && h_dev && p_dev && s_dev;
     const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
     if (async && !all_dev) return SDDMM_INVALID_ARG;
+    mark_pending(p, async, s);
 
     if (flags & SDDMM_FLAG_OPERANDS_BF16) {
         // W and H hold bfloat16: the TMA rings over rows of 2K bytes, products and sums in fp32.  Opt-in and
@@ -636,6 +683,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         CUDA_TRY(h, timer.end(s));
         if (async) return SDDMM_OK;
         CUDA_TRY(h, cudaStreamSynchronize(s));
+        waited_for(p, s);
         timer.done();
         return check_device_status(h);
     }
@@ -648,6 +696,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     const bool w_t = (flags & SDDMM_FLAG_W_TRANSPOSED) != 0, h_t = (flags & SDDMM_FLAG_H_TRANSPOSED) != 0;
     const bool pipelined = h->pipeline && p->n_pipe > 0 && !w_dev && !use_gather && !use_panel && !tiled_out && !p->d_perm &&
                            p->dense.n_cells == 0 && !w_t && !h_t;
+    if (pipelined) CUDA_TRY(h, ensure_pipe(p));
     // page-locked, mapped host arrays are read row by row by the GPU: only the rows a nonzero touches travel
     const float *W_mapped = (pipelined && h->sparse_upload) ? mapped_host_ptr(W) : nullptr;
     const float *H_mapped = (pipelined && h->sparse_upload && !h_dev) ? mapped_host_ptr(H) : nullptr;
@@ -750,6 +799,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         CUDA_TRY(h, cudaEventRecord(h->pipe_joined, last));
         CUDA_TRY(h, cudaStreamWaitEvent(s, h->pipe_joined, 0));
         CUDA_TRY(h, cudaStreamSynchronize(s));
+        waited_for(p, s);
         p->ms_state = sddmm_plan_s::MS_KNOWN;
         p->last_ms = 0.f;  // kernel time only: the chunks' kernels, not the waits for uploads between them
         for (int i = 0; i < p->n_pipe; ++i) {
@@ -818,6 +868,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dP, nbytes, cudaMemcpyDeviceToHost, s));
     if (async) return SDDMM_OK;
     CUDA_TRY(h, cudaStreamSynchronize(s));
+    waited_for(p, s);
     timer.done();
     return check_device_status(h);
 }
@@ -829,28 +880,26 @@ int sddmm_coo_sort_rows_gpu(sddmm_handle_t h, int64_t *M, int64_t *N, int64_t nn
     if (nnz > 0) {
         CUDA_TRY(h, cudaSetDevice(h->device));
         cudaStream_t s = h->stream;
+        PoolScope scope(h->pool, s);
         const bool idx_dev = is_device_ptr(rows), val_dev = is_device_ptr(vals);
         if (idx_dev != is_device_ptr(cols)) {
             h->last_error = "sddmm_coo_sort_rows_gpu: rows and cols must both be host or both be device arrays";
             return SDDMM_INVALID_ARG;
         }
-        struct Tmp {
-            void *p[3] = {nullptr, nullptr, nullptr};
-            ~Tmp() { for (void *q : p) if (q) cudaFree(q); }
-        } tmp;
+        CallTmp tmp;
         const size_t bytes = 4 * (size_t)nnz;
         int32_t *d_rows = rows, *d_cols = cols;
         float *d_vals = vals;
         if (!idx_dev) {
-            CUDA_TRY(h, cudaMalloc(&tmp.p[0], bytes));
-            CUDA_TRY(h, cudaMalloc(&tmp.p[1], bytes));
+            CUDA_TRY(h, pool_alloc(&tmp.p[0], bytes));
+            CUDA_TRY(h, pool_alloc(&tmp.p[1], bytes));
             d_rows = (int32_t *)tmp.p[0];
             d_cols = (int32_t *)tmp.p[1];
             CUDA_TRY(h, cudaMemcpyAsync(d_rows, rows, bytes, cudaMemcpyHostToDevice, s));
             CUDA_TRY(h, cudaMemcpyAsync(d_cols, cols, bytes, cudaMemcpyHostToDevice, s));
         }
         if (!val_dev) {
-            CUDA_TRY(h, cudaMalloc(&tmp.p[2], bytes));
+            CUDA_TRY(h, pool_alloc(&tmp.p[2], bytes));
             d_vals = (float *)tmp.p[2];
             CUDA_TRY(h, cudaMemcpyAsync(d_vals, vals, bytes, cudaMemcpyHostToDevice, s));
         }
@@ -864,7 +913,7 @@ int sddmm_coo_sort_rows_gpu(sddmm_handle_t h, int64_t *M, int64_t *N, int64_t nn
             CUDA_TRY(h, cudaMemcpyAsync(cols, new_cols, bytes, cudaMemcpyDeviceToHost, s));
         } else if (transpose) {
             // device arrays: exchange the contents of rows and cols through a scratch copy
-            CUDA_TRY(h, cudaMalloc(&tmp.p[0], bytes));
+            CUDA_TRY(h, pool_alloc(&tmp.p[0], bytes));
             CUDA_TRY(h, cudaMemcpyAsync(tmp.p[0], rows, bytes, cudaMemcpyDeviceToDevice, s));
             CUDA_TRY(h, cudaMemcpyAsync(rows, cols, bytes, cudaMemcpyDeviceToDevice, s));
             CUDA_TRY(h, cudaMemcpyAsync(cols, tmp.p[0], bytes, cudaMemcpyDeviceToDevice, s));
@@ -884,18 +933,13 @@ int sddmm_plan_used_lines(sddmm_plan_t p, int which, const int32_t **d_ids, int6
     *n = 0;
     if (p->nnz == 0) return SDDMM_OK;
     CUDA_TRY(h, cudaSetDevice(h->device));
+    PoolScope scope(h->pool, h->stream);
     if (which == 0) {
-        if (!p->d_used_rows) {
-            CUDA_TRY(h, build_used_row_list(p->d_row_ptr, p->M, &p->d_used_rows, &p->n_used_rows, h->stream));
-            p->device_bytes += (int64_t)sizeof(int32_t) * p->n_used_rows;
-        }
+        CUDA_TRY(h, ensure_used_rows(p));
         *d_ids = p->d_used_rows;
         *n = p->n_used_rows;
     } else {
-        if (!p->d_used_cols) {
-            CUDA_TRY(h, build_used_col_list(p->d_cols, p->nnz, p->N, &p->d_used_cols, &p->n_used_cols, h->stream));
-            p->device_bytes += (int64_t)sizeof(int32_t) * p->n_used_cols;
-        }
+        CUDA_TRY(h, ensure_used_cols(p));
         *d_ids = p->d_used_cols;
         *n = p->n_used_cols;
     }
@@ -961,14 +1005,12 @@ int sddmm_check_result(sddmm_plan_t p, const float *W, const float *H, const flo
     if (p->nnz == 0) return SDDMM_OK;
     if (!W || !H || !P) return SDDMM_INVALID_ARG;
     CUDA_TRY(h, cudaSetDevice(h->device));
+    PoolScope scope(h->pool, h->stream);
     // host arrays are staged for this call only
-    struct Tmp {
-        void *p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-        ~Tmp() { for (void *q : p) if (q) cudaFree(q); }
-    } tmp;
+    CallTmp tmp;
     auto stage = [&](int slot, const float *src, size_t count, const float **dst) -> cudaError_t {
         if (!src || is_device_ptr(src)) { *dst = src; return cudaSuccess; }
-        cudaError_t e = cudaMalloc(&tmp.p[slot], sizeof(float) * (count ? count : 1));
+        cudaError_t e = pool_alloc(&tmp.p[slot], sizeof(float) * (count ? count : 1));
         if (e != cudaSuccess) return e;
         *dst = (const float *)tmp.p[slot];
         return cudaMemcpyAsync(tmp.p[slot], src, sizeof(float) * count, cudaMemcpyHostToDevice, h->stream);
@@ -979,7 +1021,7 @@ int sddmm_check_result(sddmm_plan_t p, const float *W, const float *H, const flo
     CUDA_TRY(h, stage(2, Sval, (size_t)p->nnz, &dS));
     CUDA_TRY(h, stage(3, P, (size_t)p->nnz, &dP));
     CheckResult host{};
-    CUDA_TRY(h, cudaMalloc(&tmp.p[4], sizeof(CheckResult)));
+    CUDA_TRY(h, pool_alloc(&tmp.p[4], sizeof(CheckResult)));
     CheckResult *d_out = (CheckResult *)tmp.p[4];
     cudaError_t e = launch_check_result(p->d_rows, p->d_cols, dS, dW, dH, dP, p->nnz, p->K, stride, tol, d_out, h->sm_count,
                                         h->stream);
@@ -1003,19 +1045,17 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     if (!H || !Y || (fused && !W)) return SDDMM_INVALID_ARG;
     if (flags & ~(uint32_t)SDDMM_FLAG_ASYNC) return SDDMM_INVALID_ARG;
     CUDA_TRY(h, cudaSetDevice(h->device));
+    PoolScope scope(h->pool, h->stream);
     // the class that sddmm_last_kernel_name reports (SDDMM_SPMM_RING=0: never the long-row one)
     bool ring = ring_supports(p->K) && p->nnz >= 65536;
     if (const char *env = std::getenv("SDDMM_SPMM_RING")) ring = ring && std::atoi(env) != 0;
     if (!p->d_spmm_scratch && p->nnz > 0)
         CUDA_TRY(h, dev_alloc(p, &p->d_spmm_scratch, spmm_scratch_floats(p->nnz, p->K, h->sm_count)));
     cudaStream_t s = h->stream;
-    struct Tmp {
-        void *p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-        ~Tmp() { for (void *q : p) if (q) cudaFree(q); }
-    } tmp;
+    CallTmp tmp;
     auto stage_in = [&](int slot, const float *src, size_t count, const float **dst) -> cudaError_t {
         if (!src || is_device_ptr(src)) { *dst = src; return cudaSuccess; }
-        cudaError_t e = cudaMalloc(&tmp.p[slot], sizeof(float) * (count ? count : 1));
+        cudaError_t e = pool_alloc(&tmp.p[slot], sizeof(float) * (count ? count : 1));
         if (e != cudaSuccess) return e;
         *dst = (const float *)tmp.p[slot];
         return cudaMemcpyAsync(tmp.p[slot], src, sizeof(float) * count, cudaMemcpyHostToDevice, s);
@@ -1029,11 +1069,11 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     const bool y_dev = is_device_ptr(Y), p_dev = P_out ? is_device_ptr(P_out) : true;
     if ((flags & SDDMM_FLAG_ASYNC) && (!y_dev || !p_dev || tmp.p[0] || tmp.p[1] || tmp.p[2])) return SDDMM_INVALID_ARG;
     if (!y_dev) {
-        CUDA_TRY(h, cudaMalloc(&tmp.p[3], sizeof(float) * (mk ? mk : 1)));
+        CUDA_TRY(h, pool_alloc(&tmp.p[3], sizeof(float) * (mk ? mk : 1)));
         dY = (float *)tmp.p[3];
     }
     if (P_out && !p_dev) {
-        CUDA_TRY(h, cudaMalloc(&tmp.p[4], sizeof(float) * (nz ? nz : 1)));
+        CUDA_TRY(h, pool_alloc(&tmp.p[4], sizeof(float) * (nz ? nz : 1)));
         dP = (float *)tmp.p[4];
     }
     if ((((uintptr_t)dW | (uintptr_t)dH | (uintptr_t)dY) & 15u) != 0) {
@@ -1042,6 +1082,8 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     }
     const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
     CallTimer timer(p, async);
+    mark_pending(p, async, s);
+    CUDA_TRY(h, ensure_row_ptr(p));
     CUDA_TRY(h, timer.begin(p->M > 0, s));
     SpmmCall call{p->d_rows, p->d_cols, p->d_row_ptr, dV, fused ? dW : nullptr, dH, dP, dY, p->d_spmm_scratch, p->M, p->nnz, p->K,
                   timer.clk};
@@ -1052,6 +1094,7 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     if (P_out && !p_dev) CUDA_TRY(h, cudaMemcpyAsync(P_out, dP, sizeof(float) * nz, cudaMemcpyDeviceToHost, s));
     if (async) return SDDMM_OK;
     CUDA_TRY(h, cudaStreamSynchronize(s));
+    waited_for(p, s);
     timer.done();
     return check_device_status(h);
 }
@@ -1104,15 +1147,13 @@ int sddmm_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const int32_t
     if (!rows || !cols || !W || !H || !P) return SDDMM_INVALID_ARG;
     CUDA_TRY(h, cudaSetDevice(h->device));
     cudaStream_t s = h->stream;
+    PoolScope scope(h->pool, s);
     // Everything that is not already on the device is staged for this call only,
     // as the reference does (sddmm.cu:38-73,147-150).
-    struct Tmp {
-        void *p[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-        ~Tmp() { for (void *q : p) if (q) cudaFree(q); }
-    } tmp;
+    CallTmp tmp;
     auto stage = [&](int slot, const void *src, size_t bytes, const void **dst) -> cudaError_t {
         if (is_device_ptr(src)) { *dst = src; return cudaSuccess; }
-        cudaError_t e = cudaMalloc(&tmp.p[slot], bytes);
+        cudaError_t e = pool_alloc(&tmp.p[slot], bytes);
         if (e != cudaSuccess) return e;
         *dst = tmp.p[slot];
         return cudaMemcpyAsync(tmp.p[slot], src, bytes, cudaMemcpyHostToDevice, s);
@@ -1126,7 +1167,7 @@ int sddmm_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const int32_t
     float *dp = P;
     const bool p_dev = is_device_ptr(P);
     if (!p_dev) {
-        CUDA_TRY(h, cudaMalloc(&tmp.p[5], sizeof(float) * nnz));
+        CUDA_TRY(h, pool_alloc(&tmp.p[5], sizeof(float) * nnz));
         dp = (float *)tmp.p[5];
     }
     CUDA_TRY(h, launch_gather((const int32_t *)dr, (const int32_t *)dc, nullptr, (const float *)ds, (const float *)dw,
@@ -1150,6 +1191,7 @@ int sddmm_plan_get_info(sddmm_plan_t p, sddmm_plan_info *info)
 {
     if (!p || !info) return SDDMM_INVALID_ARG;
     CUDA_TRY(p->h, cudaSetDevice(p->h->device));
+    PoolScope scope(p->h->pool, p->h->stream);
     CUDA_TRY(p->h, ensure_items(p));
     CUDA_TRY(p->h, ensure_hints(p));
     info->M = p->M; info->N = p->N; info->nnz = p->nnz; info->K = p->K;
@@ -1173,6 +1215,7 @@ int sddmm_plan_count_cols(sddmm_plan_t p, int64_t *out)
     sddmm_handle_s *h = p->h;
     if (p->n_nonempty_cols < 0) {
         CUDA_TRY(h, cudaSetDevice(h->device));
+        PoolScope scope(h->pool, h->stream);
         int64_t c = 0;
         CUDA_TRY(h, count_distinct_cols(p->d_cols, p->nnz, p->N, &c, h->stream));
         p->n_nonempty_cols = c;
@@ -1186,6 +1229,8 @@ int sddmm_plan_export_row_ptr(sddmm_plan_t p, int64_t *row_ptr)
     if (!p || !row_ptr) return SDDMM_INVALID_ARG;
     sddmm_handle_s *h = p->h;
     CUDA_TRY(h, cudaSetDevice(h->device));
+    PoolScope scope(h->pool, h->stream);
+    CUDA_TRY(h, ensure_row_ptr(p));
     CUDA_TRY(h, cudaMemcpyAsync(row_ptr, p->d_row_ptr, sizeof(int64_t) * (size_t)(p->M + 1), cudaMemcpyDeviceToHost,
                                 h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -1199,6 +1244,7 @@ int sddmm_plan_export_tiling(sddmm_plan_t p, int panel_rows, int col_tile, int32
     if (!p || panel_rows <= 0 || col_tile <= 0) return SDDMM_INVALID_ARG;
     sddmm_handle_s *h = p->h;
     CUDA_TRY(h, cudaSetDevice(h->device));
+    PoolScope scope(h->pool, h->stream);
     TilingTables t{t_rows, t_cols, tiled_ind, lastIdx_tile, lastIdx_block_tile, active_row, n_actv_row, max_active_row};
     CUDA_TRY(h, export_reference_tiling(p->d_rows, p->d_cols, p->nnz, p->M, p->N, panel_rows, col_tile, t, h->stream));
     return SDDMM_OK;

@@ -9,6 +9,7 @@
 
 #include "binning.cuh"
 #include "common.cuh"
+#include "pool.hpp"
 #include "sddmm_b200.h"
 
 using namespace sddmm;
@@ -34,6 +35,11 @@ struct sddmm_handle_s {
     unsigned long long *d_work_counter = nullptr;  // dynamic work distribution of the ring kernel
     // kernel clocks (two words each) of plans whose last synchronous call was a single gather launch
     unsigned long long *d_clocks = nullptr;
+    unsigned long long *d_plan_words = nullptr;                          // of scan_coo
+    volatile unsigned long long *h_words = nullptr;                      // mapped: what plan-time kernels answer
+    unsigned long long *d_words = nullptr;                               // its device address
+    cudaEvent_t ev_plan[2] = {};
+    DevicePool pool;  // memory given back by plans and calls
     std::vector<int> free_clocks;
     std::string last_error;
     // dense cells: 0 = fp32 FMA, 1 = 3xTF32 on mma.sync, 2 = 3xTF32 on tcgen05 / tensor memory (SDDMM_DENSE_TENSOR)
@@ -85,14 +91,17 @@ struct sddmm_plan_s {
     float *d_Wt = nullptr, *d_Ht = nullptr;  // device copies of K-major host operands, before their transposition
     int64_t device_bytes = 0;
     float plan_ms = 0.f, last_ms = -1.f;
+    // work was enqueued that nothing has waited for yet; asynchronous calls: on which stream, on several
+    bool pending = false, async_pending = false, async_mixed = false;
+    cudaStream_t async_stream = nullptr;
     int clock = -1;              // index of this plan's kernel clock in the handle's array
     enum { MS_KNOWN, MS_IN_CLOCK, MS_IN_EVENTS } ms_state = MS_KNOWN;  // where the last call's kernel time is
     int ev_pair = -1;
     // chunks of the host-operand pipeline (0 = not pipelined): nonzeros
-    // [pipe_nnz[i], pipe_nnz[i+1]) touch the rows pipe_row_first[i] .. pipe_row_last[i] of W
+    // [pipe_nnz[i], pipe_nnz[i+1]); filled by ensure_pipe
     int n_pipe = 0;
+    bool pipe_ready = false;
     int64_t pipe_nnz[SDDMM_PIPE_MAX_CHUNKS + 1] = {};
-    int32_t pipe_row_first[SDDMM_PIPE_MAX_CHUNKS] = {}, pipe_row_last[SDDMM_PIPE_MAX_CHUNKS] = {};
     // rows of W chunk i uploads: [pipe_w_begin[i], pipe_w_end[i]) (empty when an earlier chunk brought them),
     // = entries [pipe_list_begin[i], pipe_list_begin[i+1]) of the used-row list
     int64_t pipe_w_begin[SDDMM_PIPE_MAX_CHUNKS] = {}, pipe_w_end[SDDMM_PIPE_MAX_CHUNKS] = {};

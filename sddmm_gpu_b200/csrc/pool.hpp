@@ -1,0 +1,116 @@
+// Device memory that plans and calls give back is kept by the handle for the next ones: cudaMalloc and cudaFree of a few
+// megabytes cost up to 1.5 ms a pair and wait for the whole device, more than planning a small matrix.
+//
+// The pool belongs to one handle and is used by one host thread at a time, like the handle.  It keeps at most LIMIT bytes
+// that nobody uses; more go back to CUDA at once, all of it when the handle is destroyed or an allocation fails.  A
+// block given back while work on a stream may still touch it carries that stream and is handed out again only to work
+// on the same stream, until settle() says that the stream has been waited for.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <map>
+#include <unordered_map>
+
+namespace sddmm {
+
+class DevicePool {
+public:
+    static constexpr size_t LIMIT = 2ull << 30;
+    cudaStream_t stream = nullptr;  // the stream of the current call
+
+    ~DevicePool() { release(); }
+    cudaError_t alloc(void **ptr, size_t bytes)
+    {
+        const size_t n = rounded(bytes);
+        // a quarter more than asked for at most, so that a small request does not take a large block away
+        for (auto it = free_.lower_bound(n); it != free_.end() && it->first <= n + n / 4; ++it) {
+            if (it->second.busy && it->second.stream != stream) continue;
+            *ptr = it->second.ptr;
+            kept_ -= it->first;
+            free_.erase(it);
+            return cudaSuccess;
+        }
+        cudaError_t e = cudaMalloc(ptr, n);
+        if (e == cudaErrorMemoryAllocation && kept_ > 0) {
+            (void)cudaGetLastError();
+            release();
+            e = cudaMalloc(ptr, n);
+        }
+        if (e != cudaSuccess) {
+            *ptr = nullptr;
+            return e;
+        }
+        size_.emplace(*ptr, n);
+        return cudaSuccess;
+    }
+    // busy: work enqueued on the current stream may still use the block
+    void free(void *ptr, bool busy)
+    {
+        if (!ptr) return;
+        auto it = size_.find(ptr);
+        if (it == size_.end() || kept_ + it->second > LIMIT) {
+            if (it != size_.end()) size_.erase(it);
+            cudaFree(ptr);  // waits for the device
+            return;
+        }
+        kept_ += it->second;
+        free_.emplace(it->second, Block{ptr, stream, busy});
+    }
+    // the stream has been waited for: what was given back on it is idle
+    void settle(cudaStream_t s)
+    {
+        for (auto &f : free_)
+            if (f.second.stream == s) f.second.busy = false;
+    }
+    void release()
+    {
+        for (auto &f : free_) {
+            size_.erase(f.second.ptr);
+            cudaFree(f.second.ptr);
+        }
+        free_.clear();
+        kept_ = 0;
+    }
+
+private:
+    struct Block {
+        void *ptr;
+        cudaStream_t stream;
+        bool busy;
+    };
+    std::multimap<size_t, Block> free_;
+    std::unordered_map<void *, size_t> size_;  // every block taken from CUDA and not given back to it
+    size_t kept_ = 0;
+
+    // sizes with three bits of mantissa, so that similar requests share blocks
+    static size_t rounded(size_t n)
+    {
+        if (n <= 4096) return 4096;
+        size_t step = 512;
+        while (step * 16 < n) step *= 2;
+        return (n + step - 1) / step * step;
+    }
+};
+
+// The pool that pool_alloc / pool_free use on this thread while a PoolScope lives; without one they are cudaMalloc / cudaFree.
+DevicePool *&current_pool();
+struct PoolScope {
+    DevicePool *before;
+    PoolScope(DevicePool &p, cudaStream_t s) : before(current_pool())
+    {
+        current_pool() = &p;
+        p.stream = s;
+    }
+    ~PoolScope() { current_pool() = before; }
+};
+cudaError_t pool_alloc(void **ptr, size_t bytes);
+void pool_free(void *ptr);  // after the last use on the call's stream has been enqueued
+
+template <class T>
+cudaError_t pool_alloc(T **ptr, size_t count)
+{
+    return pool_alloc(reinterpret_cast<void **>(ptr), sizeof(T) * (count ? count : 1));
+}
+
+}  // namespace sddmm
