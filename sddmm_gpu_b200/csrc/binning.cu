@@ -815,33 +815,51 @@ __global__ void fill_dense_kernel(const unsigned long long *__restrict__ keys_s,
         }
     }
 }
-// Row masks and first-nonzero indices of every dense cell (one CTA per cell, grid-stride), and whether
-// the cell qualifies for the row-mask form: inside every row the list entries (input order) must have
-// consecutive input indices and ascending columns.
+// Row masks and run positions of every dense cell (one CTA per cell, grid-stride), and whether the cell qualifies for
+// the row-mask form: inside every row the list entries (input order) have ascending columns and their input indices are
+// consecutive but for one gap at most.  row_mask arrives zeroed.
 __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const int32_t *__restrict__ idx,
-                                      const uint16_t *__restrict__ rc, unsigned long long *row_mask, int32_t *row_base,
-                                      unsigned long long *n_mask_cells)
+                                      const uint16_t *__restrict__ rc, unsigned long long *row_mask, int2 *row_base,
+                                      uint8_t *row_split, unsigned long long *n_mask_cells)
 {
     __shared__ int bad;
+    __shared__ int gaps[DENSE_CELL_ROWS], first[DENSE_CELL_ROWS], split[DENSE_CELL_ROWS], second[DENSE_CELL_ROWS];
     for (int64_t cell = blockIdx.x; cell < n_cells; cell += gridDim.x) {
         if (threadIdx.x == 0) bad = 0;
+        for (int r = threadIdx.x; r < DENSE_CELL_ROWS; r += blockDim.x) {
+            gaps[r] = first[r] = second[r] = 0;
+            split[r] = DENSE_CELL_COLS;
+        }
         __syncthreads();
         const DenseCell dc = cells[cell];
         const int32_t *ci = idx + dc.offset;
         const uint16_t *cr = rc + dc.offset;
         unsigned long long *mk = row_mask + cell * DENSE_CELL_ROWS;
-        int32_t *bs = row_base + cell * DENSE_CELL_ROWS;
         for (int t = threadIdx.x; t < dc.count; t += blockDim.x) {
             const unsigned code = cr[t];
             const int r = code >> 8, c = code & 255u;
             atomicOr(mk + r, 1ull << c);
-            atomicMin(bs + r, ci[t]);
-            if (t > 0) {
-                const unsigned prev = cr[t - 1];
-                if ((prev >> 8) == (unsigned)r && (ci[t] != ci[t - 1] + 1 || (int)(prev & 255u) >= c)) bad = 1;
+            const unsigned prev = t > 0 ? cr[t - 1] : 0u;
+            if (t == 0 || (prev >> 8) != (unsigned)r) {
+                first[r] = ci[t];
+            } else {
+                if ((int)(prev & 255u) >= c) bad = 1;
+                if (ci[t] != ci[t - 1] + 1) {
+                    if (atomicAdd(&gaps[r], 1) > 0) bad = 1;
+                    split[r] = c;
+                    second[r] = ci[t];
+                }
             }
         }
+        __threadfence_block();
         __syncthreads();
+        for (int r = threadIdx.x; r < DENSE_CELL_ROWS; r += blockDim.x) {
+            const unsigned long long m = atomicOr(mk + r, 0ull);
+            const int s = split[r];
+            const int before = s < DENSE_CELL_COLS ? __popcll(m & ((1ull << s) - 1ull)) : 0;
+            row_base[cell * DENSE_CELL_ROWS + r] = make_int2(first[r], second[r] - before);
+            row_split[cell * DENSE_CELL_ROWS + r] = (uint8_t)s;
+        }
         if (threadIdx.x == 0 && !bad) {
             cells[cell].cls = dc.cls | 0x100;
             atomicAdd(n_mask_cells, 1ull);
@@ -860,10 +878,10 @@ struct NotDense {
 void DensePlan::release()
 {
     pool_free(cells); pool_free(idx); pool_free(rc); pool_free(rows_s); pool_free(cols_s); pool_free(perm_s);
-    pool_free(dense_rows); pool_free(dense_cols); pool_free(row_mask); pool_free(row_base);
+    pool_free(dense_rows); pool_free(dense_cols); pool_free(row_mask); pool_free(row_base); pool_free(row_split);
     cells = nullptr; idx = nullptr; rc = nullptr; rows_s = cols_s = perm_s = nullptr;
     dense_rows = dense_cols = nullptr;
-    row_mask = nullptr; row_base = nullptr;
+    row_mask = nullptr; row_base = nullptr; row_split = nullptr;
     n_cells = n_dense_nnz = n_sparse = n_dense_rows = n_dense_cols = n_mask_cells = 0;
 }
 
@@ -1007,13 +1025,14 @@ cudaError_t build_dense_cells(const int32_t *d_rows, const int32_t *d_cols, cons
             const size_t lines_n = (size_t)n_dense_cells * DENSE_CELL_ROWS;
             CK(pool_alloc(&out->row_mask, lines_n));
             CK(pool_alloc(&out->row_base, lines_n));
+            CK(pool_alloc(&out->row_split, lines_n));
             CK(cudaMemsetAsync(out->row_mask, 0, sizeof(unsigned long long) * lines_n, stream));
-            CK(cudaMemsetAsync(out->row_base, 0x7f, sizeof(int32_t) * lines_n, stream));
             Scratch cnt;
             CK(cnt.reserve(sizeof(unsigned long long)));
             CK(cudaMemsetAsync(cnt.ptr, 0, sizeof(unsigned long long), stream));
             cell_row_masks_kernel<<<grid_for((int64_t)n_dense_cells * TPB), TPB, 0, stream>>>(
-                out->cells, n_dense_cells, out->idx, out->rc, out->row_mask, out->row_base, (unsigned long long *)cnt.ptr);
+                out->cells, n_dense_cells, out->idx, out->rc, out->row_mask, out->row_base,
+                out->row_split, (unsigned long long *)cnt.ptr);
             CK(cudaGetLastError());
             unsigned long long n_mask = 0;
             CK(cudaMemcpyAsync(&n_mask, cnt.ptr, sizeof(n_mask), cudaMemcpyDeviceToHost, stream));

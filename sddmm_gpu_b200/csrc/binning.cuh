@@ -96,12 +96,15 @@ struct DensePlan {
     int64_t n_cells = 0;
     int32_t *idx = nullptr;       // input index of every dense-cell nonzero, grouped by cell, row-major inside
     uint16_t *rc = nullptr;       // (row - row0) << 8 | (col - col0)
-    // Row-mask form of a cell (DenseCell::cls bit 8 set): per cell row a 64-bit column mask and the
-    // input index of the row's first nonzero inside the cell.  Valid for cells in which the nonzeros of
-    // every row are consecutive in the input with ascending columns (any (row, col)-sorted input, for
-    // cells over a contiguous column range); such a cell's nonzeros need no per-nonzero list.
+    // Row-mask form of a cell (DenseCell::cls bit 8 set): per cell row a 64-bit column mask and the input positions of
+    // its nonzeros as at most two runs: the nonzero in column c sits at popc(mask below c) past row_base.x, or past
+    // row_base.y from column row_split on (64: one run).  Valid for cells in which the nonzeros of every row have
+    // ascending columns and at most one gap in their input positions: cells of the regular grid (the gap is a nonzero
+    // that went to a compacted full column) and cells of compacted columns (the gap is the band between them) of a
+    // (row, col)-sorted input; such a cell's nonzeros need no per-nonzero list.
     unsigned long long *row_mask = nullptr;  // [n_cells][DENSE_CELL_ROWS]
-    int32_t *row_base = nullptr;             // [n_cells][DENSE_CELL_ROWS]
+    int2 *row_base = nullptr;                // [n_cells][DENSE_CELL_ROWS]
+    uint8_t *row_split = nullptr;            // [n_cells][DENSE_CELL_ROWS]
     int64_t n_mask_cells = 0;
     int64_t n_dense_nnz = 0;
     int32_t *rows_s = nullptr, *cols_s = nullptr, *perm_s = nullptr;  // remainder: indices and input positions

@@ -13,34 +13,37 @@ template <int NT = 256>
 __device__ __forceinline__ void pick_block(const float *Ct, int stride, const DenseCell &dc, bool masked, int64_t cell,
                                            int tid, const int32_t *__restrict__ idx, const uint16_t *__restrict__ rc,
                                            const unsigned long long *__restrict__ row_mask,
-                                           const int32_t *__restrict__ row_base, const float *__restrict__ sval,
+                                           const int2 *__restrict__ row_base, const uint8_t *__restrict__ row_split, const float *__restrict__ sval,
                                            float *__restrict__ P)
 {
     if (masked) {
-        // Row r of the cell holds the columns of mask[r]; its nonzeros are consecutive in the input from
-        // base[r] on, in column order, so the one in column c sits at base[r] + popc(mask[r] below bit c).
-        // A warp takes four rows at a time, lane l the columns l and l + 32: the S loads and the P stores of
-        // a row are one or two contiguous runs.
+        // Row r of the cell holds the columns of mask[r]; in column order its nonzeros are one or two runs of
+        // consecutive input positions: the one in column c sits at popc(mask[r] below bit c) past base[r].x, or past
+        // base[r].y from column split[r] on.  A warp takes four rows at a time, lane l the columns l and l + 32: the S
+        // loads and the P stores of a row are a few contiguous runs.
         const unsigned long long *cm = row_mask + cell * DENSE_CELL_ROWS;
-        const int32_t *cb = row_base + cell * DENSE_CELL_ROWS;
+        const int2 *cb = row_base + cell * DENSE_CELL_ROWS;
+        const uint8_t *cs = row_split + cell * DENSE_CELL_ROWS;
         const int lane = tid & 31, warp = tid >> 5;
         const unsigned below = (1u << lane) - 1u;
         for (int r0 = warp * 4; r0 < DENSE_CELL_ROWS; r0 += NT / 8) {
             unsigned lo[4], hi[4];
-            int32_t base[4];
+            int2 base[4];
+            int split[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const unsigned long long m = __ldg(cm + r0 + u);
                 lo[u] = (unsigned)m;
                 hi[u] = (unsigned)(m >> 32);
                 base[u] = __ldg(cb + r0 + u);
+                split[u] = __ldg(cs + r0 + u);
             }
             float s_lo[4], s_hi[4];
             int32_t p_lo[4], p_hi[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                p_lo[u] = base[u] + __popc(lo[u] & below);
-                p_hi[u] = base[u] + __popc(lo[u]) + __popc(hi[u] & below);
+                p_lo[u] = (lane < split[u] ? base[u].x : base[u].y) + __popc(lo[u] & below);
+                p_hi[u] = (lane + 32 < split[u] ? base[u].x : base[u].y) + __popc(lo[u]) + __popc(hi[u] & below);
                 s_lo[u] = s_hi[u] = 1.f;
                 if (sval) {
                     if ((lo[u] >> lane) & 1u) s_lo[u] = __ldcs(sval + p_lo[u]);

@@ -564,7 +564,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
             PLAN_TRY(ensure_row_ptr(p));
             PLAN_TRY(build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, nnz, M, N, 0.25f, 0.5f, &p->dense, s));
             if (p->dense.n_cells > 0)
-                p->device_bytes += (int64_t)(sizeof(DenseCell) * p->dense.n_cells + 6 * p->dense.n_dense_nnz +
+                p->device_bytes += (int64_t)(sizeof(DenseCell) * p->dense.n_cells + 6 * p->dense.n_dense_nnz + 17 * DENSE_CELL_ROWS * p->dense.n_cells +
                                              12 * p->dense.n_sparse);
         }
     }
@@ -827,12 +827,12 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         }
         if (h->dense_mode == 2)
             LAUNCH_TRY(h, launch_dense_cells_tc(p->dense.cells, p->dense.n_cells, p->dense.idx, p->dense.rc, p->dense.row_mask,
-                                              p->dense.row_base, p->dense.dense_rows, p->dense.n_dense_rows,
+                                              p->dense.row_base, p->dense.row_split, p->dense.dense_rows, p->dense.n_dense_rows,
                                               p->dense.dense_cols, p->dense.n_dense_cols, dS, dW, dH, dP, p->M, p->N, p->K,
                                               h->sm_count, h->d_status, s));
         else
             LAUNCH_TRY(h, launch_dense_cells(p->dense.cells, p->dense.n_cells, p->dense.idx, p->dense.rc, p->dense.row_mask,
-                                           p->dense.row_base, p->dense.dense_rows, p->dense.n_dense_rows,
+                                           p->dense.row_base, p->dense.row_split, p->dense.dense_rows, p->dense.n_dense_rows,
                                            p->dense.dense_cols, p->dense.n_dense_cols, dS, dW, dH, dP, p->M, p->N, p->K,
                                            h->dense_mode == 1, h->sm_count, s));
         if (p->dense.n_sparse > 0)

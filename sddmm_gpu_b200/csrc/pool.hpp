@@ -49,13 +49,23 @@ public:
     {
         if (!ptr) return;
         auto it = size_.find(ptr);
-        if (it == size_.end() || kept_ + it->second > LIMIT) {
+        if (it == size_.end() || it->second > LIMIT / 2) {
             if (it != size_.end()) size_.erase(it);
             cudaFree(ptr);  // waits for the device
             return;
         }
+        // the blocks that have been idle longest make room
+        while (kept_ + it->second > LIMIT) {
+            auto old = free_.begin();
+            for (auto f = free_.begin(); f != free_.end(); ++f)
+                if (f->second.since < old->second.since) old = f;
+            kept_ -= old->first;
+            size_.erase(old->second.ptr);
+            cudaFree(old->second.ptr);
+            free_.erase(old);
+        }
         kept_ += it->second;
-        free_.emplace(it->second, Block{ptr, stream, busy});
+        free_.emplace(it->second, Block{ptr, stream, busy, ++clock_});
     }
     // the stream has been waited for: what was given back on it is idle
     void settle(cudaStream_t s)
@@ -78,10 +88,12 @@ private:
         void *ptr;
         cudaStream_t stream;
         bool busy;
+        unsigned long long since;
     };
     std::multimap<size_t, Block> free_;
     std::unordered_map<void *, size_t> size_;  // every block taken from CUDA and not given back to it
     size_t kept_ = 0;
+    unsigned long long clock_ = 0;
 
     // sizes with three bits of mantissa, so that similar requests share blocks
     static size_t rounded(size_t n)

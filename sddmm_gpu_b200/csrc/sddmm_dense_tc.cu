@@ -83,7 +83,8 @@ constexpr int B_STAGE_BYTES = 2 * B_TILE_BYTES;               // head and tail t
 constexpr int RUNS_SMEM_BYTES = 2 * A_BUF_BYTES + STAGES * B_STAGE_BYTES + CT_BYTES;  // 215,040 bytes
 struct __align__(16) MetaSlot {
     unsigned long long mask[DENSE_CELL_ROWS];  // columns held by each cell row
-    int32_t base[DENSE_CELL_ROWS];             // input index of each cell row's first nonzero
+    int2 base[DENSE_CELL_ROWS];                // input position of the nonzero in column c, less the nonzeros below c: .x,
+    uint8_t split[DENSE_CELL_ROWS];            // and .y from this column on
     int32_t cls;                               // DenseCell::cls (class, row-mask flag)
     int32_t pad[3];
 };
@@ -150,7 +151,7 @@ template <bool RUNS>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, const int32_t *__restrict__ idx,
                       const uint16_t *__restrict__ rc, const unsigned long long *__restrict__ row_mask,
-                      const int32_t *__restrict__ row_base, const int32_t *__restrict__ dense_rows, int64_t n_dense_rows,
+                      const int2 *__restrict__ row_base, const uint8_t *__restrict__ row_split, const int32_t *__restrict__ dense_rows, int64_t n_dense_rows,
                       const int32_t *__restrict__ dense_cols, int64_t n_dense_cols, const float *__restrict__ sval,
                       const float *__restrict__ W, const float *__restrict__ H, float *__restrict__ P, int64_t M,
                       int64_t N, int K, int *dev_status)
@@ -374,20 +375,21 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
         const int quarter = warp & 3, cgroup = ew >> 2;
         const int row = quarter * 32 + lane;
         const unsigned below = (1u << lane) - 1u;
-        // metadata of cell i of this CTA -> ring slot i % META_SLOTS, by 16-byte cp.async (97 threads take part)
+        // metadata of cell i of this CTA -> ring slot i % META_SLOTS, by 16-byte cp.async (137 threads take part)
         auto fetch_meta = [&](int i) {
             if (i < my_cells) {
                 const int64_t c = cell_of(i);
                 MetaSlot &m = meta[i % META_SLOTS];
                 if (et < 64) cp_async16_zfill(&m.mask[et * 2], row_mask + c * DR + et * 2, 16);
-                else if (et < 96) cp_async16_zfill(&m.base[(et - 64) * 4], row_base + c * DR + (et - 64) * 4, 16);
-                else if (et == 96)
+                else if (et < 128) cp_async16_zfill(&m.base[(et - 64) * 2], row_base + c * DR + (et - 64) * 2, 16);
+                else if (et < 136) cp_async16_zfill(&m.split[(et - 128) * 16], row_split + c * DR + (et - 128) * 16, 16);
+                else if (et == 136)
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&m.cls)), "l"(&cells[c].cls) : "memory");
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
         // S values of this warp's rows of cell i (row-mask form): lane l takes the columns l and l + 32 of a row; the
-        // nonzero in column c sits at base + popc(mask below bit c)
+        // nonzero in column c sits at popc(mask below bit c) past one of the row's two bases
         auto load_s = [&](int i, float (&s_lo)[8], float (&s_hi)[8]) {
             const MetaSlot &m = meta[i % META_SLOTS];
             const bool on = i < my_cells && (m.cls & 0x100) != 0 && sval != nullptr;
@@ -397,9 +399,10 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
                 if (on) {
                     const unsigned long long mk = m.mask[ew * 8 + u];
                     const unsigned lo = (unsigned)mk, hi = (unsigned)(mk >> 32);
-                    const int32_t bs = m.base[ew * 8 + u];
-                    if ((lo >> lane) & 1u) s_lo[u] = __ldg(sval + bs + __popc(lo & below));
-                    if ((hi >> lane) & 1u) s_hi[u] = __ldg(sval + bs + __popc(lo) + __popc(hi & below));
+                    const int2 bs = m.base[ew * 8 + u];
+                    const int split = m.split[ew * 8 + u];
+                    if ((lo >> lane) & 1u) s_lo[u] = __ldg(sval + (lane < split ? bs.x : bs.y) + __popc(lo & below));
+                    if ((hi >> lane) & 1u) s_hi[u] = __ldg(sval + (lane + 32 < split ? bs.x : bs.y) + __popc(lo) + __popc(hi & below));
                 }
             }
         };
@@ -448,10 +451,11 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
                 for (int u = 0; u < 8; ++u) {
                     const unsigned long long mk = m.mask[ew * 8 + u];
                     const unsigned lo = (unsigned)mk, hi = (unsigned)(mk >> 32);
-                    const int32_t bs = m.base[ew * 8 + u];
+                    const int2 bs = m.base[ew * 8 + u];
+                    const int split = m.split[ew * 8 + u];
                     const float *cr = Ct + (ew * 8 + u) * CT_STRIDE;
-                    if ((lo >> lane) & 1u) P[bs + __popc(lo & below)] = cr[lane] * s_lo[u];
-                    if ((hi >> lane) & 1u) P[bs + __popc(lo) + __popc(hi & below)] = cr[lane + 32] * s_hi[u];
+                    if ((lo >> lane) & 1u) P[(lane < split ? bs.x : bs.y) + __popc(lo & below)] = cr[lane] * s_lo[u];
+                    if ((hi >> lane) & 1u) P[(lane + 32 < split ? bs.x : bs.y) + __popc(lo) + __popc(hi & below)] = cr[lane + 32] * s_hi[u];
                 }
             } else {
                 // per-nonzero lists, eight nonzeros per thread and trip, the loads of a trip grouped by dependency
@@ -497,7 +501,7 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
 }  // namespace
 
 cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const int32_t *idx, const uint16_t *rc,
-                                  const unsigned long long *row_mask, const int32_t *row_base, const int32_t *dense_rows,
+                                  const unsigned long long *row_mask, const int2 *row_base, const uint8_t *row_split, const int32_t *dense_rows,
                                   int64_t n_dense_rows, const int32_t *dense_cols, int64_t n_dense_cols, const float *sval,
                                   const float *W, const float *H, float *P, int64_t M, int64_t N, int K, int sm_count,
                                   int *dev_status, cudaStream_t stream)
@@ -519,7 +523,7 @@ cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const
         cudaError_t e = optin_dynamic_smem(sddmm_dense_tc_kernel<true>, RUNS_SMEM_BYTES, optin_runs);
         if (e != cudaSuccess) return e;
         sddmm_dense_tc_kernel<true><<<(unsigned)blocks, TC_THREADS, RUNS_SMEM_BYTES, stream>>>(
-            cells, n_cells, idx, rc, row_mask, row_base, dense_rows, n_dense_rows, dense_cols, n_dense_cols, sval, W, H, P, M,
+            cells, n_cells, idx, rc, row_mask, row_base, row_split, dense_rows, n_dense_rows, dense_cols, n_dense_cols, sval, W, H, P, M,
             N, K, dev_status);
         return cudaGetLastError();
     }
@@ -529,7 +533,7 @@ cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const
         if (e != cudaSuccess) return e;
     }
     sddmm_dense_tc_kernel<false><<<(unsigned)blocks, TC_THREADS, TC_SMEM_BYTES, stream>>>(
-        cells, n_cells, idx, rc, row_mask, row_base, dense_rows, n_dense_rows, dense_cols, n_dense_cols, sval, W, H, P, M, N,
+        cells, n_cells, idx, rc, row_mask, row_base, row_split, dense_rows, n_dense_rows, dense_cols, n_dense_cols, sval, W, H, P, M, N,
         K, dev_status);
     return cudaGetLastError();
 }
