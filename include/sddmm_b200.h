@@ -174,7 +174,7 @@ SDDMM_API int sddmm_fused_execute(sddmm_plan_t p, const float *W, const float *H
 SDDMM_API int sddmm_last_kernel_ms(sddmm_plan_t p, float *ms);
 
 /* Which path the last sddmm_execute() on this plan took (static storage): "ring" (K = 256, 512,
- * 1024), "ring_small" (K = 32, 64, 128), "panel" (any other K, or fewer than 65,536 nonzeros), "htile",
+ * 1024), "ring_small" (K = 32, 64, 128), "panel" (any other K, or fewer than 65,536 nonzeros), "htile" (K = 128, 256, 512 and few columns),
  * "dense_tc+ring_small", ... by default; "ring", "ring_small", "panel" or "gather" when forced by a flag.
  * The names stand for classes of K and size, not for kernel functions: by default the row classes run on the
  * gather kernel, and on the rings where H is far larger than L2.  The reference has one

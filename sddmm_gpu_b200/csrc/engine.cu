@@ -119,8 +119,7 @@ void free_plan_memory(sddmm_plan_s *p)
     if (p->pending) cudaDeviceSynchronize();
     if (p->owns_rows) pool_free(p->d_rows);
     if (p->owns_cols) pool_free(p->d_cols);
-    for (void *q : {(void *)p->d_rows_t, (void *)p->d_cols_t, (void *)p->d_perm, (void *)p->d_ht_rows, (void *)p->d_ht_cols,
-                    (void *)p->d_ht_perm, (void *)p->d_ht_off, (void *)p->d_row_ptr, (void *)p->d_items, (void *)p->d_item_rows,
+    for (void *q : {(void *)p->d_rows_t, (void *)p->d_cols_t, (void *)p->d_perm, (void *)p->d_row_ptr, (void *)p->d_items, (void *)p->d_item_rows,
                     (void *)p->d_cols_hint, (void *)p->d_used_rows, (void *)p->d_used_cols, (void *)p->d_spmm_scratch,
                     (void *)p->d_Wt, (void *)p->d_Ht, (void *)p->d_W, (void *)p->d_H, (void *)p->d_S, (void *)p->d_P})
         pool_free(q);
@@ -222,6 +221,11 @@ int check_device_status(sddmm_handle_s *h)
 const char *rows_class_name(const sddmm_plan_s *p, bool panel, bool ring)
 {
     if (panel || !rows_path_supports(p->K) || (!ring && p->nnz < 65536)) return "panel";
+    if (!ring && p->n_col_tiles == 1 && (p->K == 128 || p->K == 256 || p->K == 512)) {
+        // few columns and many nonzeros per column: H is at most 64 blocks of 192 KB, a block has 8 nonzeros per row and SM
+        const int64_t block = 196608 / (p->K * 4);
+        if ((p->N + block - 1) / block <= 64 && p->nnz / p->h->sm_count >= 8 * block) return "htile";
+    }
     return p->K <= 128 ? "ring_small" : "ring";
 }
 
@@ -579,26 +583,6 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
             PLAN_TRY(ensure_hints(p));
         }
     }
-    // Few columns and many nonzeros per column (a bag-of-words matrix): H is a handful of shared-memory tiles, and
-    // the column-tile kernel reads every H row of a nonzero from shared memory.  Worth it when a CTA's share of
-    // the nonzeros is several times the rows of the tiles it has to load.  SDDMM_HTILE=0 switches it off.
-    {
-        const char *env = std::getenv("SDDMM_HTILE");
-        const int tc = htile_cols(K);
-        const int64_t n_tiles = tc > 0 ? (N + tc - 1) / tc : 0;
-        if (!(env && std::atoi(env) == 0) && tc > 0 && p->n_col_tiles == 1 && p->dense.n_cells == 0 && n_tiles >= 1 &&
-            n_tiles <= 64 && nnz >= 65536 && nnz / h->sm_count >= 8 * (int64_t)tc) {
-            PLAN_TRY(begin_more());
-            PLAN_TRY(dev_alloc(p, &p->d_ht_perm, (size_t)nnz));
-            PLAN_TRY(dev_alloc(p, &p->d_ht_rows, (size_t)nnz));
-            PLAN_TRY(dev_alloc(p, &p->d_ht_cols, (size_t)nnz));
-            PLAN_TRY(dev_alloc(p, &p->d_ht_off, (size_t)n_tiles + 1));
-            PLAN_TRY(build_tiled_order(p->d_rows, p->d_cols, nnz, N, tc, p->d_ht_perm, p->d_ht_rows, p->d_ht_cols, s));
-            PLAN_TRY(build_htile_offsets(p->d_ht_cols, nnz, tc, (int)n_tiles, p->d_ht_off, s));
-            p->ht_col_tile = tc;
-            p->ht_n_tiles = (int)n_tiles;
-        }
-    }
     // chunks of the host-operand pipeline; what they need is built by the first call with host operands
     if (p->n_col_tiles == 1 && p->dense.n_cells == 0 && nnz >= (1 << 20)) {
         const int64_t chunks = std::min<int64_t>((int64_t)sizeof(float) * M * K / (128ll << 20), SDDMM_PIPE_MAX_CHUNKS);
@@ -810,9 +794,8 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         return check_device_status(h);
     }
     const bool use_dense = !forced && !tiled_out && p->dense.n_cells > 0;
-    const bool use_htile = p->d_ht_off && !forced && !p->d_perm;
     // a call that is one gather launch is timed by the kernel itself, everything else by events
-    const bool one_gather = !use_dense && !use_htile && !use_panel &&
+    const bool one_gather = !use_dense && !use_panel &&
                             !(ring_supports(p->K) && (use_ring || (!use_gather && ring_preferred(p->N, p->K))));
     CallTimer timer(p, async);
     CUDA_TRY(h, timer.begin(one_gather, s));
@@ -854,11 +837,8 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             h->last_error = "SDDMM_FLAG_TILED_ORDER with S values is not supported on a multi-tile plan";
             return SDDMM_INVALID_ARG;
         }
-        p->last_kernel = use_htile ? "htile" : rows_class_name(p, use_panel, use_ring);
-        if (use_htile)
-            LAUNCH_TRY(h, launch_htile(p->d_ht_rows, p->d_ht_cols, p->d_ht_perm, dS, dW, dH, dP, p->nnz, p->N, p->K, p->ht_col_tile,
-                                       p->d_ht_off, p->ht_n_tiles, h->sm_count, h->d_status, s));
-        else if (use_panel)
+        p->last_kernel = rows_class_name(p, use_panel, use_ring);
+        if (use_panel)
             LAUNCH_TRY(h, launch_panel(p->d_items, p->n_items, p->d_item_rows, rows_p, cols_p, perm, dS, dW, dH, dP, p->K,
                                      p->cfg, h->sm_count, h->d_status, s));
         else

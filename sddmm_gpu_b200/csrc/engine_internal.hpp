@@ -77,10 +77,6 @@ struct sddmm_plan_s {
     int32_t *d_cols_hint = nullptr;  // processing-order columns with hub marks (ring kernel), or null (ensure_hints)
     int64_t hub_budget = 0;          // bytes of H rows to keep in L2 (0 = no marks)
     bool hints_built = false;
-    // column-tile kernel (few columns, many nonzeros per column): its own tiled order and tile offsets
-    int32_t *d_ht_rows = nullptr, *d_ht_cols = nullptr, *d_ht_perm = nullptr;
-    int64_t *d_ht_off = nullptr;
-    int ht_col_tile = 0, ht_n_tiles = 0;
     // dense cells + row-sorted remainder (single-tile plans of locally dense matrices)
     DensePlan dense;
     int64_t n_hub_cols = 0;
