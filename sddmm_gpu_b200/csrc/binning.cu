@@ -820,12 +820,15 @@ __global__ void fill_dense_kernel(const unsigned long long *__restrict__ keys_s,
 // consecutive but for one gap at most.  row_mask arrives zeroed.
 __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const int32_t *__restrict__ idx,
                                       const uint16_t *__restrict__ rc, unsigned long long *row_mask, int2 *row_base,
-                                      uint8_t *row_split, unsigned long long *n_mask_cells)
+                                      uint32_t *row_span, unsigned long long *n_mask_cells)
 {
-    __shared__ int bad;
+    __shared__ int bad, forms;
     __shared__ int gaps[DENSE_CELL_ROWS], first[DENSE_CELL_ROWS], split[DENSE_CELL_ROWS], second[DENSE_CELL_ROWS];
     for (int64_t cell = blockIdx.x; cell < n_cells; cell += gridDim.x) {
-        if (threadIdx.x == 0) bad = 0;
+        if (threadIdx.x == 0) {
+            bad = 0;
+            forms = CELL_RUNS;
+        }
         for (int r = threadIdx.x; r < DENSE_CELL_ROWS; r += blockDim.x) {
             gaps[r] = first[r] = second[r] = 0;
             split[r] = DENSE_CELL_COLS;
@@ -858,10 +861,13 @@ __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const i
             const int s = split[r];
             const int before = s < DENSE_CELL_COLS ? __popcll(m & ((1ull << s) - 1ull)) : 0;
             row_base[cell * DENSE_CELL_ROWS + r] = make_int2(first[r], second[r] - before);
-            row_split[cell * DENSE_CELL_ROWS + r] = (uint8_t)s;
+            const int c0 = m ? __ffsll(m) - 1 : 0, n = __popcll(m);
+            row_span[cell * DENSE_CELL_ROWS + r] = (uint32_t)c0 | (uint32_t)n << 8 | (uint32_t)s << 16;
+            if (s < DENSE_CELL_COLS || (m && (m >> c0) != (n < 64 ? (1ull << n) - 1ull : ~0ull))) forms = 0;
         }
+        __syncthreads();
         if (threadIdx.x == 0 && !bad) {
-            cells[cell].cls = dc.cls | 0x100;
+            cells[cell].cls = dc.cls | CELL_MASKED | forms;
             atomicAdd(n_mask_cells, 1ull);
         }
         __syncthreads();
@@ -878,10 +884,10 @@ struct NotDense {
 void DensePlan::release()
 {
     pool_free(cells); pool_free(idx); pool_free(rc); pool_free(rows_s); pool_free(cols_s); pool_free(perm_s);
-    pool_free(dense_rows); pool_free(dense_cols); pool_free(row_mask); pool_free(row_base); pool_free(row_split);
+    pool_free(dense_rows); pool_free(dense_cols); pool_free(row_mask); pool_free(row_base); pool_free(row_span);
     cells = nullptr; idx = nullptr; rc = nullptr; rows_s = cols_s = perm_s = nullptr;
     dense_rows = dense_cols = nullptr;
-    row_mask = nullptr; row_base = nullptr; row_split = nullptr;
+    row_mask = nullptr; row_base = nullptr; row_span = nullptr;
     n_cells = n_dense_nnz = n_sparse = n_dense_rows = n_dense_cols = n_mask_cells = 0;
 }
 
@@ -1025,14 +1031,14 @@ cudaError_t build_dense_cells(const int32_t *d_rows, const int32_t *d_cols, cons
             const size_t lines_n = (size_t)n_dense_cells * DENSE_CELL_ROWS;
             CK(pool_alloc(&out->row_mask, lines_n));
             CK(pool_alloc(&out->row_base, lines_n));
-            CK(pool_alloc(&out->row_split, lines_n));
+            CK(pool_alloc(&out->row_span, lines_n));
             CK(cudaMemsetAsync(out->row_mask, 0, sizeof(unsigned long long) * lines_n, stream));
             Scratch cnt;
             CK(cnt.reserve(sizeof(unsigned long long)));
             CK(cudaMemsetAsync(cnt.ptr, 0, sizeof(unsigned long long), stream));
             cell_row_masks_kernel<<<grid_for((int64_t)n_dense_cells * TPB), TPB, 0, stream>>>(
                 out->cells, n_dense_cells, out->idx, out->rc, out->row_mask, out->row_base,
-                out->row_split, (unsigned long long *)cnt.ptr);
+                out->row_span, (unsigned long long *)cnt.ptr);
             CK(cudaGetLastError());
             unsigned long long n_mask = 0;
             CK(cudaMemcpyAsync(&n_mask, cnt.ptr, sizeof(n_mask), cudaMemcpyDeviceToHost, stream));

@@ -31,6 +31,9 @@ struct WorkItem {
 // plain matrix coordinates.
 constexpr int DENSE_CELL_ROWS = 128;
 constexpr int DENSE_CELL_COLS = 64;
+// Forms of a cell in DenseCell::cls, above the class: CELL_MASKED = the row-mask form (see DensePlan); CELL_RUNS = of those, a
+// cell in which every row is one run of columns at consecutive input positions.
+constexpr int CELL_MASKED = 0x100, CELL_RUNS = 0x200;
 struct DenseCell {
     int64_t offset;
     int32_t row0, col0;
@@ -139,14 +142,14 @@ cudaError_t launch_ring_bf16(const int32_t *rows, const int32_t *cols, const int
 // Cells whose cls has bit 8 set are in row-mask form (row_mask / row_base, see DensePlan) and
 // do not read idx / rc.
 cudaError_t launch_dense_cells(const DenseCell *cells, int64_t n_cells, const int32_t *idx, const uint16_t *rc,
-                               const unsigned long long *row_mask, const int2 *row_base, const uint8_t *row_split, const int32_t *dense_rows, int64_t n_dense_rows, const int32_t *dense_cols,
+                               const unsigned long long *row_mask, const int2 *row_base, const uint32_t *row_span, const int32_t *dense_rows, int64_t n_dense_rows, const int32_t *dense_cols,
                                int64_t n_dense_cols, const float *sval, const float *W, const float *H, float *P,
                                int64_t M, int64_t N, int K, bool tensor, int sm_count, cudaStream_t stream);
 
 // The same dense cells on tcgen05: MMAs issued by one thread from shared-memory descriptors, accumulator in
 // tensor memory (3xTF32).  dev_status receives DEV_MBARRIER_TIMEOUT if a bounded wait gives up.
 cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const int32_t *idx, const uint16_t *rc,
-                                  const unsigned long long *row_mask, const int2 *row_base, const uint8_t *row_split, const int32_t *dense_rows,
+                                  const unsigned long long *row_mask, const int2 *row_base, const uint32_t *row_span, const int32_t *dense_rows,
                                   int64_t n_dense_rows, const int32_t *dense_cols, int64_t n_dense_cols, const float *sval,
                                   const float *W, const float *H, float *P, int64_t M, int64_t N, int K, int sm_count,
                                   int *dev_status, cudaStream_t stream);

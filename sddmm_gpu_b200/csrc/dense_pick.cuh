@@ -13,17 +13,17 @@ template <int NT = 256>
 __device__ __forceinline__ void pick_block(const float *Ct, int stride, const DenseCell &dc, bool masked, int64_t cell,
                                            int tid, const int32_t *__restrict__ idx, const uint16_t *__restrict__ rc,
                                            const unsigned long long *__restrict__ row_mask,
-                                           const int2 *__restrict__ row_base, const uint8_t *__restrict__ row_split, const float *__restrict__ sval,
+                                           const int2 *__restrict__ row_base, const uint32_t *__restrict__ row_span, const float *__restrict__ sval,
                                            float *__restrict__ P)
 {
     if (masked) {
         // Row r of the cell holds the columns of mask[r]; in column order its nonzeros are one or two runs of
         // consecutive input positions: the one in column c sits at popc(mask[r] below bit c) past base[r].x, or past
-        // base[r].y from column split[r] on.  A warp takes four rows at a time, lane l the columns l and l + 32: the S
+        // base[r].y from column span[r] >> 16 on.  A warp takes four rows at a time, lane l the columns l and l + 32: the S
         // loads and the P stores of a row are a few contiguous runs.
         const unsigned long long *cm = row_mask + cell * DENSE_CELL_ROWS;
         const int2 *cb = row_base + cell * DENSE_CELL_ROWS;
-        const uint8_t *cs = row_split + cell * DENSE_CELL_ROWS;
+        const uint32_t *cs = row_span + cell * DENSE_CELL_ROWS;
         const int lane = tid & 31, warp = tid >> 5;
         const unsigned below = (1u << lane) - 1u;
         for (int r0 = warp * 4; r0 < DENSE_CELL_ROWS; r0 += NT / 8) {
@@ -36,7 +36,7 @@ __device__ __forceinline__ void pick_block(const float *Ct, int stride, const De
                 lo[u] = (unsigned)m;
                 hi[u] = (unsigned)(m >> 32);
                 base[u] = __ldg(cb + r0 + u);
-                split[u] = __ldg(cs + r0 + u);
+                split[u] = (int)(__ldg(cs + r0 + u) >> 16);
             }
             float s_lo[4], s_hi[4];
             int32_t p_lo[4], p_hi[4];

@@ -810,12 +810,12 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         }
         if (h->dense_mode == 2)
             LAUNCH_TRY(h, launch_dense_cells_tc(p->dense.cells, p->dense.n_cells, p->dense.idx, p->dense.rc, p->dense.row_mask,
-                                              p->dense.row_base, p->dense.row_split, p->dense.dense_rows, p->dense.n_dense_rows,
+                                              p->dense.row_base, p->dense.row_span, p->dense.dense_rows, p->dense.n_dense_rows,
                                               p->dense.dense_cols, p->dense.n_dense_cols, dS, dW, dH, dP, p->M, p->N, p->K,
                                               h->sm_count, h->d_status, s));
         else
             LAUNCH_TRY(h, launch_dense_cells(p->dense.cells, p->dense.n_cells, p->dense.idx, p->dense.rc, p->dense.row_mask,
-                                           p->dense.row_base, p->dense.row_split, p->dense.dense_rows, p->dense.n_dense_rows,
+                                           p->dense.row_base, p->dense.row_span, p->dense.dense_rows, p->dense.n_dense_rows,
                                            p->dense.dense_cols, p->dense.n_dense_cols, dS, dW, dH, dP, p->M, p->N, p->K,
                                            h->dense_mode == 1, h->sm_count, s));
         if (p->dense.n_sparse > 0)

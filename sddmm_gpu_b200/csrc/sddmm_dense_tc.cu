@@ -84,7 +84,7 @@ constexpr int RUNS_SMEM_BYTES = 2 * A_BUF_BYTES + STAGES * B_STAGE_BYTES + CT_BY
 struct __align__(16) MetaSlot {
     unsigned long long mask[DENSE_CELL_ROWS];  // columns held by each cell row
     int2 base[DENSE_CELL_ROWS];                // input position of the nonzero in column c, less the nonzeros below c: .x,
-    uint8_t split[DENSE_CELL_ROWS];            // and .y from this column on
+    uint32_t span[DENSE_CELL_ROWS];            // and .y from column span >> 16 on; first column and number of columns below
     int32_t cls;                               // DenseCell::cls (class, row-mask flag)
     int32_t pad[3];
 };
@@ -151,7 +151,7 @@ template <bool RUNS>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, const int32_t *__restrict__ idx,
                       const uint16_t *__restrict__ rc, const unsigned long long *__restrict__ row_mask,
-                      const int2 *__restrict__ row_base, const uint8_t *__restrict__ row_split, const int32_t *__restrict__ dense_rows, int64_t n_dense_rows,
+                      const int2 *__restrict__ row_base, const uint32_t *__restrict__ row_span, const int32_t *__restrict__ dense_rows, int64_t n_dense_rows,
                       const int32_t *__restrict__ dense_cols, int64_t n_dense_cols, const float *__restrict__ sval,
                       const float *__restrict__ W, const float *__restrict__ H, float *__restrict__ P, int64_t M,
                       int64_t N, int K, int *dev_status)
@@ -375,15 +375,15 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
         const int quarter = warp & 3, cgroup = ew >> 2;
         const int row = quarter * 32 + lane;
         const unsigned below = (1u << lane) - 1u;
-        // metadata of cell i of this CTA -> ring slot i % META_SLOTS, by 16-byte cp.async (137 threads take part)
+        // metadata of cell i of this CTA -> ring slot i % META_SLOTS, by 16-byte cp.async (161 threads take part)
         auto fetch_meta = [&](int i) {
             if (i < my_cells) {
                 const int64_t c = cell_of(i);
                 MetaSlot &m = meta[i % META_SLOTS];
                 if (et < 64) cp_async16_zfill(&m.mask[et * 2], row_mask + c * DR + et * 2, 16);
                 else if (et < 128) cp_async16_zfill(&m.base[(et - 64) * 2], row_base + c * DR + (et - 64) * 2, 16);
-                else if (et < 136) cp_async16_zfill(&m.split[(et - 128) * 16], row_split + c * DR + (et - 128) * 16, 16);
-                else if (et == 136)
+                else if (et < 160) cp_async16_zfill(&m.span[(et - 128) * 4], row_span + c * DR + (et - 128) * 4, 16);
+                else if (et == 160)
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&m.cls)), "l"(&cells[c].cls) : "memory");
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
@@ -392,15 +392,26 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
         // nonzero in column c sits at popc(mask below bit c) past one of the row's two bases
         auto load_s = [&](int i, float (&s_lo)[8], float (&s_hi)[8]) {
             const MetaSlot &m = meta[i % META_SLOTS];
-            const bool on = i < my_cells && (m.cls & 0x100) != 0 && sval != nullptr;
+            const int cls = i < my_cells && sval != nullptr ? m.cls : 0;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                s_lo[u] = s_hi[u] = 1.f;
-                if (on) {
+            for (int u = 0; u < 8; ++u) s_lo[u] = s_hi[u] = 1.f;
+            if (cls & CELL_RUNS) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const uint32_t span = m.span[ew * 8 + u];
+                    const int d = lane - (int)(span & 255u);
+                    const unsigned n = (span >> 8) & 255u;
+                    const float *sp = sval + (m.base[ew * 8 + u].x + d);
+                    if ((unsigned)d < n) s_lo[u] = __ldg(sp);
+                    if ((unsigned)(d + 32) < n) s_hi[u] = __ldg(sp + 32);
+                }
+            } else if (cls & CELL_MASKED) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
                     const unsigned long long mk = m.mask[ew * 8 + u];
                     const unsigned lo = (unsigned)mk, hi = (unsigned)(mk >> 32);
                     const int2 bs = m.base[ew * 8 + u];
-                    const int split = m.split[ew * 8 + u];
+                    const int split = (int)(m.span[ew * 8 + u] >> 16);
                     if ((lo >> lane) & 1u) s_lo[u] = __ldg(sval + (lane < split ? bs.x : bs.y) + __popc(lo & below));
                     if ((hi >> lane) & 1u) s_hi[u] = __ldg(sval + (lane + 32 < split ? bs.x : bs.y) + __popc(lo) + __popc(hi & below));
                 }
@@ -416,7 +427,7 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
         for (int i = 0; i < my_cells; ++i) {
             const int64_t cell = cell_of(i);
             const MetaSlot &m = meta[i % META_SLOTS];
-            const bool masked = (m.cls & 0x100) != 0;
+            const int cls = m.cls;
             // two cells ahead: metadata; one cell ahead: S values -- neither depends on the product
             fetch_meta(i + 2);
             float n_lo[8], n_hi[8];
@@ -446,13 +457,26 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
                                                                         __uint_as_float(v[c + 2]), __uint_as_float(v[c + 3]));
             }
             epilogue_sync();  // the block is parked
-            if (masked) {
+            // The index arithmetic of the general masks is nearly half of the epilogue's instructions: runs of columns,
+            // nearly all cells of a band and of global lines, do without.
+            if (cls & CELL_RUNS) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const uint32_t span = m.span[ew * 8 + u];
+                    const int d = lane - (int)(span & 255u);
+                    const unsigned n = (span >> 8) & 255u;
+                    float *pp = P + (m.base[ew * 8 + u].x + d);
+                    const float *cr = Ct + (ew * 8 + u) * CT_STRIDE + lane;
+                    if ((unsigned)d < n) pp[0] = cr[0] * s_lo[u];
+                    if ((unsigned)(d + 32) < n) pp[32] = cr[32] * s_hi[u];
+                }
+            } else if (cls & CELL_MASKED) {
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const unsigned long long mk = m.mask[ew * 8 + u];
                     const unsigned lo = (unsigned)mk, hi = (unsigned)(mk >> 32);
                     const int2 bs = m.base[ew * 8 + u];
-                    const int split = m.split[ew * 8 + u];
+                    const int split = (int)(m.span[ew * 8 + u] >> 16);
                     const float *cr = Ct + (ew * 8 + u) * CT_STRIDE;
                     if ((lo >> lane) & 1u) P[(lane < split ? bs.x : bs.y) + __popc(lo & below)] = cr[lane] * s_lo[u];
                     if ((hi >> lane) & 1u) P[(lane + 32 < split ? bs.x : bs.y) + __popc(lo) + __popc(hi & below)] = cr[lane + 32] * s_hi[u];
@@ -501,7 +525,7 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
 }  // namespace
 
 cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const int32_t *idx, const uint16_t *rc,
-                                  const unsigned long long *row_mask, const int2 *row_base, const uint8_t *row_split, const int32_t *dense_rows,
+                                  const unsigned long long *row_mask, const int2 *row_base, const uint32_t *row_span, const int32_t *dense_rows,
                                   int64_t n_dense_rows, const int32_t *dense_cols, int64_t n_dense_cols, const float *sval,
                                   const float *W, const float *H, float *P, int64_t M, int64_t N, int K, int sm_count,
                                   int *dev_status, cudaStream_t stream)
@@ -523,7 +547,7 @@ cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const
         cudaError_t e = optin_dynamic_smem(sddmm_dense_tc_kernel<true>, RUNS_SMEM_BYTES, optin_runs);
         if (e != cudaSuccess) return e;
         sddmm_dense_tc_kernel<true><<<(unsigned)blocks, TC_THREADS, RUNS_SMEM_BYTES, stream>>>(
-            cells, n_cells, idx, rc, row_mask, row_base, row_split, dense_rows, n_dense_rows, dense_cols, n_dense_cols, sval, W, H, P, M,
+            cells, n_cells, idx, rc, row_mask, row_base, row_span, dense_rows, n_dense_rows, dense_cols, n_dense_cols, sval, W, H, P, M,
             N, K, dev_status);
         return cudaGetLastError();
     }
@@ -533,7 +557,7 @@ cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const
         if (e != cudaSuccess) return e;
     }
     sddmm_dense_tc_kernel<false><<<(unsigned)blocks, TC_THREADS, TC_SMEM_BYTES, stream>>>(
-        cells, n_cells, idx, rc, row_mask, row_base, row_split, dense_rows, n_dense_rows, dense_cols, n_dense_cols, sval, W, H, P, M, N,
+        cells, n_cells, idx, rc, row_mask, row_base, row_span, dense_rows, n_dense_rows, dense_cols, n_dense_cols, sval, W, H, P, M, N,
         K, dev_status);
     return cudaGetLastError();
 }
