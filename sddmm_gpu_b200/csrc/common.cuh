@@ -91,7 +91,7 @@ PanelConfig choose_panel_config(int K, int panel_rows_hint, int sm_count, size_t
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                           const float *W, const float *H, float *P, int64_t nnz, int K, int sm_count,
                           unsigned long long *clock, cudaStream_t stream);
-// The same over operands stored in bfloat16 (rows of 2K bytes): K = 256 or 512.
+// The same over operands stored in bfloat16 (rows of 2K bytes): K = 256, 512 or 1024.
 bool gather_bf16_supports(int K);
 cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
                                const void *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream);

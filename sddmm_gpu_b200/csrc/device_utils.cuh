@@ -54,12 +54,14 @@ __device__ __forceinline__ float fold2(unsigned long long a)
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
     return x + y;
 }
-// two bfloat16 (the lower one first) as two fp32
-__device__ __forceinline__ unsigned long long widen_bf16x2(unsigned x)
+// a0 += lower(x) * lower(y), a1 += upper(x) * upper(y): two bfloat16 per word, the product exact and the sum in fp32
+// (mixed-precision FMA of sm_100; widening with a shift, a mask and an fp32 FMA takes three times the instructions)
+__device__ __forceinline__ void fma_bf16x2(unsigned x, unsigned y, float &a0, float &a1)
 {
-    unsigned long long d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(x << 16), "r"(x & 0xffff0000u));
-    return d;
+    asm("{\n\t.reg .b16 xl, xh, yl, yh;\n\tmov.b32 {xl, xh}, %2;\n\tmov.b32 {yl, yh}, %3;\n\t"
+        "fma.rn.f32.bf16 %0, xl, yl, %0;\n\tfma.rn.f32.bf16 %1, xh, yh, %1;\n\t}"
+        : "+f"(a0), "+f"(a1)
+        : "r"(x), "r"(y));
 }
 
 // Transposed butterfly over a group of L lanes holding B accumulators each

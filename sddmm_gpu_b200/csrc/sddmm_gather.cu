@@ -46,46 +46,42 @@ struct GatherShape {
     static_assert(NB % RB == 0 && RB % B == 0 && RB <= L, "step geometry");
 };
 
-// A lane's share of the W row: fp32 pairs, widened once per row when the operands are bfloat16.
+// A lane's share of the W row.
 template <class S>
 struct WShare {
-    u64x2 v[S::F * (S::BF16 ? 2 : 1)];
+    u64x2 v[S::F];
     __device__ __forceinline__ void clear()
     {
 #pragma unroll
-        for (int i = 0; i < S::F * (S::BF16 ? 2 : 1); ++i) v[i] = u64x2{0, 0};
+        for (int f = 0; f < S::F; ++f) v[f] = u64x2{0, 0};
     }
     __device__ __forceinline__ void load(const char *wp, bool last_ok)
     {
 #pragma unroll
-        for (int f = 0; f < S::F; ++f) {
-            if (f < S::F - 1 || last_ok) {
-                const u64x2 t = ldg_u64x2(wp + f * S::L * 16);
-                if constexpr (S::BF16) {
-                    v[2 * f] = u64x2{widen_bf16x2((unsigned)t.a), widen_bf16x2((unsigned)(t.a >> 32))};
-                    v[2 * f + 1] = u64x2{widen_bf16x2((unsigned)t.b), widen_bf16x2((unsigned)(t.b >> 32))};
-                } else {
-                    v[f] = t;
-                }
-            }
-        }
+        for (int f = 0; f < S::F; ++f)
+            if (f < S::F - 1 || last_ok) v[f] = ldg_u64x2(wp + f * S::L * 16);
     }
     __device__ __forceinline__ float dot(const u64x2 (&h)[S::F]) const
     {
-        unsigned long long a0 = 0, a1 = 0;  // two fp32 sums each
+        if constexpr (S::BF16) {
+            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
-        for (int f = 0; f < S::F; ++f) {
-            if constexpr (S::BF16) {
-                a0 = ffma2(v[2 * f].a, widen_bf16x2((unsigned)h[f].a), a0);
-                a1 = ffma2(v[2 * f].b, widen_bf16x2((unsigned)(h[f].a >> 32)), a1);
-                a0 = ffma2(v[2 * f + 1].a, widen_bf16x2((unsigned)h[f].b), a0);
-                a1 = ffma2(v[2 * f + 1].b, widen_bf16x2((unsigned)(h[f].b >> 32)), a1);
-            } else {
+            for (int f = 0; f < S::F; ++f) {
+                fma_bf16x2((unsigned)v[f].a, (unsigned)h[f].a, s0, s1);
+                fma_bf16x2((unsigned)(v[f].a >> 32), (unsigned)(h[f].a >> 32), s2, s3);
+                fma_bf16x2((unsigned)v[f].b, (unsigned)h[f].b, s0, s1);
+                fma_bf16x2((unsigned)(v[f].b >> 32), (unsigned)(h[f].b >> 32), s2, s3);
+            }
+            return (s0 + s1) + (s2 + s3);
+        } else {
+            unsigned long long a0 = 0, a1 = 0;  // two fp32 sums each
+#pragma unroll
+            for (int f = 0; f < S::F; ++f) {
                 a0 = ffma2(v[f].a, h[f].a, a0);
                 a1 = ffma2(v[f].b, h[f].b, a1);
             }
+            return fold2(a0) + fold2(a1);
         }
-        return fold2(a0) + fold2(a1);
     }
 };
 
@@ -312,8 +308,9 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
     return cudaSuccess;
 }
 
-// bfloat16 rows of 2K bytes; a bfloat16 is the upper half of an fp32, so widening is a shift or a mask.
-bool gather_bf16_supports(int K) { return K == 256 || K == 512; }
+// bfloat16 rows of 2K bytes.  16.1 M nonzeros, 1 M x 1 M, K = 256: 677 us widening to fp32 first, 569 us with the
+// mixed-precision FMA (fewer registers: five resident blocks instead of four); K = 512: 1378 -> 1190.
+bool gather_bf16_supports(int K) { return K == 256 || K == 512 || K == 1024; }
 
 cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
                                const void *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream)
@@ -321,11 +318,15 @@ cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const i
     if (nnz == 0) return cudaSuccess;
     if (nnz > INT32_MAX) return cudaErrorInvalidValue;  // plans hold fewer
     const unsigned n = (unsigned)nnz;
+#define GA_GO(L, F, B, PF, CTAS) \
+    return launch_shape<GatherShape<L, F, B, 8, true, PF, CTAS, true>>(rows, cols, perm, sval, W, H, P, n, K / 8, sm_count, clock, stream)
     switch (K) {
-    case 256: return launch_shape<GatherShape<16, 2, 2, 8, true, false, 4, true>>(rows, cols, perm, sval, W, H, P, n, 32, sm_count, clock, stream);
-    case 512: return launch_shape<GatherShape<32, 2, 2, 8, true, false, 4, true>>(rows, cols, perm, sval, W, H, P, n, 64, sm_count, clock, stream);
+    case 256: GA_GO(16, 2, 2, false, 5);
+    case 512: GA_GO(16, 4, 1, true, 4);
+    case 1024: GA_GO(32, 4, 2, true, 3);
     default: return cudaErrorInvalidValue;
     }
+#undef GA_GO
 }
 
 }  // namespace sddmm

@@ -78,8 +78,7 @@ struct RingShape {
 };
 
 // A 16-byte piece of a row: four fp32 values, or eight bfloat16 values (operand storage
-// in bfloat16, products and sums in fp32: a bfloat16 is the upper half of an fp32, so
-// widening is a shift or a mask).
+// in bfloat16, products and sums in fp32 by the mixed-precision FMA).
 template <bool BF16>
 struct Piece {
     using T = float4;
@@ -88,17 +87,14 @@ struct Piece {
 template <>
 struct Piece<true> {
     using T = uint4;
-    static __device__ __forceinline__ float dot2(unsigned a, unsigned b, float acc)
-    {
-        acc = fmaf(__uint_as_float(a << 16), __uint_as_float(b << 16), acc);
-        return fmaf(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u), acc);
-    }
     static __device__ __forceinline__ float dot(T a, T b, float acc)
     {
-        acc = dot2(a.x, b.x, acc);
-        acc = dot2(a.y, b.y, acc);
-        acc = dot2(a.z, b.z, acc);
-        return dot2(a.w, b.w, acc);
+        float lo = acc, hi = 0.f;
+        fma_bf16x2(a.x, b.x, lo, hi);
+        fma_bf16x2(a.y, b.y, lo, hi);
+        fma_bf16x2(a.z, b.z, lo, hi);
+        fma_bf16x2(a.w, b.w, lo, hi);
+        return lo + hi;
     }
 };
 
