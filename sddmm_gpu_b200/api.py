@@ -330,18 +330,27 @@ class Plan:
             pass
 
     def execute(self, W, H, P, Sval=None, flags=0):
-        self.handle._follow_torch_stream(W, H, P, Sval)
-        self.handle._check(lib().sddmm_execute(self._p, _ptr(W), _ptr(H), _ptr(Sval), _ptr(P), flags))
+        h = self.handle
+        h._follow_torch_stream(W, H, P, Sval)
+        st = _lib.sddmm_execute(self._p, _ptr(W), _ptr(H), _ptr(Sval), _ptr(P), flags)
+        if st:
+            h._check(st)
 
     def spmm(self, H, Y, Pval=None, flags=0):
         """Y = P H on the plan's pattern (sddmm_spmm_execute); Pval None = all ones."""
-        self.handle._follow_torch_stream(H, Y, Pval)
-        self.handle._check(lib().sddmm_spmm_execute(self._p, _ptr(Pval), _ptr(H), _ptr(Y), flags))
+        h = self.handle
+        h._follow_torch_stream(H, Y, Pval)
+        st = _lib.sddmm_spmm_execute(self._p, _ptr(Pval), _ptr(H), _ptr(Y), flags)
+        if st:
+            h._check(st)
 
     def fused(self, W, H, Y, Sval=None, P_out=None, flags=0):
         """Y = (S o (W H^T)) H without writing P (sddmm_fused_execute); P_out, if given, receives P."""
-        self.handle._follow_torch_stream(W, H, Y, Sval, P_out)
-        self.handle._check(lib().sddmm_fused_execute(self._p, _ptr(W), _ptr(H), _ptr(Sval), _ptr(P_out), _ptr(Y), flags))
+        h = self.handle
+        h._follow_torch_stream(W, H, Y, Sval, P_out)
+        st = _lib.sddmm_fused_execute(self._p, _ptr(W), _ptr(H), _ptr(Sval), _ptr(P_out), _ptr(Y), flags)
+        if st:
+            h._check(st)
 
     def last_kernel_name(self):
         return lib().sddmm_last_kernel_name(self._p).decode()

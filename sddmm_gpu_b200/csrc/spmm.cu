@@ -23,7 +23,7 @@
 // What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero through L2; used twice in the fused form), hidden
 // by resident warps.  Measured on R-MAT matrices against the row-task and shared-memory-ring kernels this replaces
 // (us): SpMM, 6.0 M nonzeros, 250 K x 250 K: K = 64 755 -> 136;  0.67 M nonzeros: K = 64 379 -> 31;  fused, 16.1 M
-// nonzeros, 1 M x 1 M: K = 256 2970 -> 1735;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.
+// nonzeros, 1 M x 1 M: K = 256 2970 -> 1675;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.
 // At K = 64 the gather kernel alone runs at 14.2 TB/s of gathered bytes.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -41,7 +41,6 @@ namespace {
 
 constexpr int SP_TPB = 256;
 constexpr int SP_NB = 8;         // nonzeros of a set per index step (4 when a set is 4 lanes)
-constexpr int SP_WAVES = 6;
 constexpr int SP_MAX_RUN = 1024;  // bounds the scratch of partial rows
 
 // What a run tells the fix-up (run_row): the row that goes on in the next run, RUN_MIDDLE added when it also began before
@@ -61,7 +60,7 @@ struct SpmmShape {
 
 __device__ __forceinline__ void stg_u64x2(char *p, u64x2 v)
 {
-    asm volatile("st.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v.a), "l"(v.b) : "memory");
+    asm volatile("st.global.cs.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v.a), "l"(v.b) : "memory");
 }
 __device__ __forceinline__ unsigned long long pair_of(float x)
 {
@@ -81,7 +80,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     constexpr bool FUSED = S::FUSED;
     clock_begin(clock);
     const int lane = threadIdx.x & 31;
-    const size_t row_bytes = (size_t)pieces * 16;
+    const unsigned row_bytes = (unsigned)pieces * 16u;
     if (blockIdx.x >= gather_blocks) {
         // 32 rows of S per warp: those without nonzeros are written as zeros
         const int64_t r0 = ((int64_t)(blockIdx.x - gather_blocks) * (SP_TPB / 32) + (threadIdx.x >> 5)) * 32;
@@ -110,7 +109,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 #pragma unroll
     for (int f = 0; f < F; ++f) y[f] = w[f] = u64x2{0, 0};
     auto load_w = [&](unsigned r) {
-        const char *wp = W_lane + r * row_bytes;
+        const char *wp = W_lane + (size_t)r * row_bytes;
 #pragma unroll
         for (int f = 0; f < F; ++f)
             if (f < F - 1 || last_ok) w[f] = ldg_u64x2(wp + f * L * 16);
@@ -151,30 +150,37 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         int before = __shfl_up_sync(FULL, r, 1, L);
         if (lig == 0) before = last;
         const unsigned changed = __ballot_sync(FULL, r != before && lig < NB);
-        const unsigned valid = __ballot_sync(FULL, j < nnz && lig < NB);
+        const bool full = __all_sync(FULL, j < nnz);
         last = __shfl_sync(FULL, r, NB - 1, L);
         if (FUSED && S::PF && step > 1) {
             // the W rows that the next step opens, into L1
             int b2 = __shfl_up_sync(FULL, rn, 1, L);
             if (lig == 0) b2 = last;
             if (rn != b2 && lig < NB) {
-                const char *wp = W + (unsigned)rn * row_bytes;
+                const char *wp = W + (size_t)(unsigned)rn * row_bytes;
                 for (unsigned o = 0; o < row_bytes; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(wp + o));
             }
         }
         float p_mine = 0.f;
-#pragma unroll
-        for (int b = 0; b < NB; b += B) {
-            u64x2 h[B][F];
+        auto load_h = [&](int b, u64x2 (&h)[B][F]) {
 #pragma unroll
             for (int i = 0; i < B; ++i) {
                 const unsigned cj = (unsigned)__shfl_sync(FULL, c, b + i, L);
-                const bool ok = (valid >> (set * L + b + i)) & 1u;  // past the end: nothing is added
-                const char *hp = H_lane + cj * row_bytes;
+                const char *hp = H_lane + (size_t)cj * row_bytes;
+                if (full) {
 #pragma unroll
-                for (int f = 0; f < F; ++f)
-                    h[i][f] = ok && (f < F - 1 || last_ok) ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
+                    for (int f = 0; f < F; ++f) h[i][f] = f < F - 1 || last_ok ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
+                } else {  // the end of the matrix: nothing is added past it
+                    const bool ok = j - il + b + i < nnz;
+#pragma unroll
+                    for (int f = 0; f < F; ++f) h[i][f] = ok && (f < F - 1 || last_ok) ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
+                }
             }
+        };
+#pragma unroll
+        for (int b = 0; b < NB; b += B) {
+            u64x2 h[B][F];
+            load_h(b, h);
             float p[B];  // the nonzeros' weights, the same in all lanes of the set
             if (FUSED && S::JOINT) {
                 // all B products first, so that their reductions overlap: one transposed butterfly, then B broadcasts
@@ -327,9 +333,14 @@ spmm_fixup_kernel(const int *__restrict__ run_row, const int64_t *__restrict__ r
 template <class S>
 unsigned run_length(int64_t nnz, int sm_count)
 {
-    // a few waves of resident sets even out the last one; long runs leave fewer partial rows
-    const int64_t sets = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G * SP_WAVES;
-    int64_t run = nnz / sets / S::NB * S::NB;
+    // Waves of resident sets against the cost of a run's start and its two partial rows.  Six waves; down to three where
+    // runs would be shorter than 56 nonzeros, up to twelve where they would be longer than 160 (us at 12 / 6 / 3 waves:
+    // fused 16.1 M nonzeros K = 256 1704 / 1775 / 1878; fused 0.9 M K = 256 144 / 130 / 125; SpMM 6 M K = 256 391 / 375).
+    const int64_t wave = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G;
+    int64_t run = nnz / (6 * wave);
+    if (run < 56) run = std::min<int64_t>(56, nnz / (3 * wave));
+    if (run > 160) run = std::max<int64_t>(160, nnz / (12 * wave));
+    run = run / S::NB * S::NB;
     if (run < 2 * S::NB) run = 2 * S::NB;
     if (run > SP_MAX_RUN) run = SP_MAX_RUN;
     return (unsigned)run;
@@ -375,13 +386,13 @@ auto with_shape(int K, bool fused, Fn f)
         if (q < 16) return f(SpmmShape<8, 2, 2, false, 4, true, true, false>());
         if (q == 16) return f(SpmmShape<8, 2, 2, true, 4, true, true, false>());
         if (q <= 24) return f(SpmmShape<8, 3, 2, false, 3, true, true, false>());
-        if (q < 32) return f(SpmmShape<16, 2, 2, false, 4, true, true, false>());
-        if (q == 32) return f(SpmmShape<16, 2, 2, true, 4, true, true, false>());
-        if (q <= 48) return f(SpmmShape<16, 3, 2, false, 3, true, true, false>());
+        if (q < 32) return f(SpmmShape<8, 4, 1, false, 3, true, true, false>());
+        if (q == 32) return f(SpmmShape<8, 4, 1, true, 4, true, false, false>());
+        if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4, true, true, false>());
         if (q < 64) return f(SpmmShape<32, 2, 2, false, 4, true, true, true>());
         if (q == 64) return f(SpmmShape<32, 2, 2, true, 4, true, true, true>());
         if (q <= 96) return f(SpmmShape<32, 3, 1, false, 4, true, false, false>());
-        if (q <= 128) return f(SpmmShape<32, 4, 1, false, 3, true, false, false>());
+        if (q <= 128) return f(SpmmShape<32, 4, 1, false, 4, true, false, false>());
         if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3, true, false, false>());
         if (q <= 192) return f(SpmmShape<32, 6, 1, false, 2, true, false, false>());
         if (q <= 224) return f(SpmmShape<32, 7, 1, false, 2, true, false, false>());
