@@ -119,10 +119,10 @@ SDDMM_API int sddmm_destroy_plan(sddmm_plan_t p);
  * sddmm_GPU (HiPC18/src/sddmm.cu:53,71-73,93-119) and the kernel comp_kernel_COO
  * (HiPC18/src/kernel.h:2-52) -- one launch, no K-slicing.
  *
- *   W, H, P : host or device pointers (detected); host buffers are copied
+ *   W, H, P : host or device pointers (detected); host buffers go
  *             through plan-owned device staging inside the call.  With W in
- *             host memory and a large matrix (256 MB of W or more, a million
- *             nonzeros or more, ring-kernel K, single column tile) the call is
+ *             host memory and a large matrix (64 MB of W or more, 131,072
+ *             nonzeros or more, single column tile, no dense cells) the call is
  *             pipelined: H first, then W rows and S values in up to 16 chunks of
  *             consecutive nonzeros, every chunk's kernel and the download of
  *             its part of P running behind the uploads of the later chunks on
@@ -130,12 +130,15 @@ SDDMM_API int sddmm_destroy_plan(sddmm_plan_t p);
  *             chunks are not uploaded.  Results are bit-identical to the
  *             unpipelined call (SDDMM_PIPELINE=0 in the environment at
  *             sddmm_create() switches the pipeline off).  Pinned host buffers
- *             are needed for the copies to overlap.  In a pipelined call, W
- *             and H buffers that are page-locked and mapped (cudaHostAlloc,
- *             cudaHostRegister) are not copied whole: a kernel reads, over
- *             PCIe, exactly the rows of W and H that some nonzero touches (the
- *             reference uploads both arrays whole, sddmm.cu:71-73);
- *             SDDMM_SPARSE_UPLOAD=0 at sddmm_create() keeps cudaMemcpy.
+ *             are needed for the copies to overlap.  W, H and S that are
+ *             page-locked and mapped (cudaHostAlloc, cudaHostRegister) are read
+ *             by a kernel over PCIe instead of being copied one by one, and of W
+ *             and H only the rows that some nonzero touches (the reference
+ *             uploads both arrays whole, sddmm.cu:71-73) -- unless rows are
+ *             shorter than 128 bytes, or nearly all rows of an array of 4 MB or
+ *             more are used.  A mapped P of up to 256 KB is written by the
+ *             kernel itself.  SDDMM_SPARSE_UPLOAD=0 at sddmm_create() keeps
+ *             cudaMemcpy.
  *   Sval    : NULL -> the unscaled dot product, as sddmm_CPU_COO and the
  *             reference kernel store it (sddmm.cu:192, kernel.h:48);
  *             else P[i] *= Sval[i], as sddmm_CPU_CSR does (sddmm.cu:171).

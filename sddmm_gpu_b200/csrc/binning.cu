@@ -421,21 +421,6 @@ __global__ void pick_kernel(const int32_t *__restrict__ a, PickAt at, int n, uns
     if (i < n) out[i] = (unsigned long long)a[at.v[i]];
     __threadfence_system();
 }
-// number of entries of the ascending list that are smaller than at.v[i]
-__global__ void rank_kernel(const int32_t *__restrict__ list, int64_t n_list, PickAt at, int n, unsigned long long *out)
-{
-    const int i = threadIdx.x;
-    if (i < n) {
-        int64_t lo = 0, hi = n_list;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (list[mid] < at.v[i]) lo = mid + 1;
-            else hi = mid;
-        }
-        out[i] = (unsigned long long)lo;
-    }
-    __threadfence_system();
-}
 }  // namespace
 
 cudaError_t pick_values(const int32_t *d_array, const PickAt &at, int n, unsigned long long *out_mapped, cudaStream_t stream)
@@ -443,10 +428,10 @@ cudaError_t pick_values(const int32_t *d_array, const PickAt &at, int n, unsigne
     pick_kernel<<<1, PICK_MAX, 0, stream>>>(d_array, at, n, out_mapped);
     return cudaGetLastError();
 }
-cudaError_t rank_values(const int32_t *d_list, int64_t n_list, const PickAt &at, int n, unsigned long long *out_mapped,
-                        cudaStream_t stream)
+cudaError_t mark_used_cols(const int32_t *d_cols, int64_t nnz, int64_t N, unsigned char *d_used, cudaStream_t stream)
 {
-    rank_kernel<<<1, PICK_MAX, 0, stream>>>(d_list, n_list, at, n, out_mapped);
+    CK(cudaMemsetAsync(d_used, 0, (size_t)N, stream));
+    mark_cols_kernel<<<grid_for(nnz), TPB, 0, stream>>>(d_cols, nnz, d_used);
     return cudaGetLastError();
 }
 

@@ -32,15 +32,15 @@ cudaError_t scan_coo(const int32_t *d_rows, const int32_t *d_cols, int64_t nnz, 
 // row_ptr[r] = first nonzero of row r (M + 1 entries, empty rows repeat).
 cudaError_t build_row_ptr(const int32_t *d_rows, int64_t nnz, int64_t M, int64_t *d_row_ptr, cudaStream_t stream);
 
-// A few entries of a device array (at.v = positions), or their ranks in an ascending list (at.v = values), to mapped host
-// memory.
+// d_used[c] = 1 for the columns that hold a nonzero, 0 for the others.
+cudaError_t mark_used_cols(const int32_t *d_cols, int64_t nnz, int64_t N, unsigned char *d_used, cudaStream_t stream);
+
+// A few entries of a device array (at.v = positions) to mapped host memory.
 constexpr int PICK_MAX = 64;
 struct PickAt {
     int64_t v[PICK_MAX];
 };
 cudaError_t pick_values(const int32_t *d_array, const PickAt &at, int n, unsigned long long *out_mapped, cudaStream_t stream);
-cudaError_t rank_values(const int32_t *d_list, int64_t n_list, const PickAt &at, int n, unsigned long long *out_mapped,
-                        cudaStream_t stream);
 
 // Number of distinct columns (marks a byte per column, then counts).
 cudaError_t count_distinct_cols(const int32_t *d_cols, int64_t nnz, int64_t N, int64_t *host_out,

@@ -111,6 +111,20 @@ cudaError_t launch_panel(const WorkItem *items, int64_t n_items, const int32_t *
 // dst[r*K + t] = src[t*n + r]: a K-major operand (K x n) into the row-major layout (n x K) the kernels read.
 cudaError_t launch_transpose_operand(const float *src_kmajor, float *dst_rowmajor, int64_t n, int K, cudaStream_t stream);
 
+// Rows [begin, end) of a row-major array in mapped, page-locked host memory that are to be copied to the same rows of a
+// device array: those marked in col_used, those with a nonzero in row_ptr, or all of them (both null).  16-byte aligned.
+struct UploadRows {
+    const char *src = nullptr;
+    char *dst = nullptr;
+    const unsigned char *col_used = nullptr;
+    const int64_t *row_ptr = nullptr;
+    int64_t begin = 0, end = 0;
+    int row_bytes = 16;
+};
+// Two such ranges and s_count floats (both addresses 16-byte aligned) in one launch; the GPU reads the host memory.
+cudaError_t launch_upload_operands(const UploadRows &a, const UploadRows &b, const float *s_src, float *s_dst, int64_t s_count,
+                                   int n_ctas, cudaStream_t stream);
+
 // Copies the listed rows (K floats each) of a row-major array in mapped, page-locked
 // host memory to the same rows of a device array; the GPU reads the host memory.
 cudaError_t launch_upload_rows(const float *mapped_host, float *dev, const int32_t *d_row_list, int64_t n_rows, int K,

@@ -61,7 +61,7 @@ bool is_device_ptr(const void *p)
 
 // Device-side address of a page-locked host allocation that is mapped into the
 // device's address space, or null (pageable memory, device memory, unknown).
-const float *mapped_host_ptr(const float *p)
+const float *mapped_host_ptr(const float *p, unsigned align = 16)
 {
     if (!p) return nullptr;
     cudaPointerAttributes a;
@@ -70,7 +70,7 @@ const float *mapped_host_ptr(const float *p)
         return nullptr;
     }
     if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
-    if (((uintptr_t)a.devicePointer & 15u) != 0) return nullptr;  // the row upload moves 16-byte vectors
+    if (((uintptr_t)a.devicePointer & (align - 1)) != 0) return nullptr;  // the row upload moves 16-byte vectors
     return static_cast<const float *>(a.devicePointer);
 }
 
@@ -120,7 +120,7 @@ void free_plan_memory(sddmm_plan_s *p)
     if (p->owns_rows) pool_free(p->d_rows);
     if (p->owns_cols) pool_free(p->d_cols);
     for (void *q : {(void *)p->d_rows_t, (void *)p->d_cols_t, (void *)p->d_perm, (void *)p->d_row_ptr, (void *)p->d_items, (void *)p->d_item_rows,
-                    (void *)p->d_cols_hint, (void *)p->d_used_rows, (void *)p->d_used_cols, (void *)p->d_spmm_scratch,
+                    (void *)p->d_cols_hint, (void *)p->d_col_used, (void *)p->d_used_rows, (void *)p->d_used_cols, (void *)p->d_spmm_scratch,
                     (void *)p->d_Wt, (void *)p->d_Ht, (void *)p->d_W, (void *)p->d_H, (void *)p->d_S, (void *)p->d_P})
         pool_free(q);
     p->dense.release();
@@ -150,6 +150,14 @@ cudaError_t resolve_ms(sddmm_plan_s *p)
     cudaError_t e = cudaSuccess;
     if (p->ms_state == sddmm_plan_s::MS_IN_EVENTS) {
         e = cudaEventElapsedTime(&p->last_ms, h->ev_begin[p->ev_pair], h->ev_end[p->ev_pair]);
+    } else if (p->ms_state == sddmm_plan_s::MS_IN_PIPE) {
+        // kernel time only: the chunks' kernels, not the waits for uploads between them
+        p->last_ms = 0.f;
+        for (int i = 0; i < p->n_pipe && e == cudaSuccess; ++i) {
+            float ms = 0.f;
+            e = cudaEventElapsedTime(&ms, h->pipe_started[i], h->pipe_computed[i]);
+            p->last_ms += ms;
+        }
     } else if (p->ms_state == sddmm_plan_s::MS_IN_CLOCK) {
         unsigned long long t[2] = {0, 0};
         e = cudaMemcpyAsync(t, h->d_clocks + 2 * p->clock, sizeof(t), cudaMemcpyDeviceToHost, h->own_stream);
@@ -255,16 +263,25 @@ cudaError_t ensure_used_cols(sddmm_plan_s *p)
     return e;
 }
 
-// Host-operand pipeline (sddmm_execute with W in host memory): S is cut into chunks of consecutive nonzeros, about 128 MB
+// What the upload of used rows looks at: the row pointer and a mark per column.
+cudaError_t ensure_upload_marks(sddmm_plan_s *p, bool rows, bool cols)
+{
+    cudaError_t e = rows ? ensure_row_ptr(p) : cudaSuccess;
+    if (e == cudaSuccess && cols && !p->d_col_used) {
+        e = dev_alloc(p, &p->d_col_used, (size_t)p->N);
+        if (e == cudaSuccess) e = mark_used_cols(p->d_cols, p->nnz, p->N, p->d_col_used, p->h->stream);
+    }
+    return e;
+}
+
+// Host-operand pipeline (sddmm_execute with W in host memory): S is cut into chunks of consecutive nonzeros, about 32 MB
 // of W rows each.  Rows are sorted, so a chunk needs one contiguous block of W rows, and W rows between two chunks
-// that no nonzero touches are never uploaded.  Here: the first and last row of every chunk and the used-row list.
+// that no nonzero touches are never uploaded.  Here: the first and last row of every chunk.
 cudaError_t ensure_pipe(sddmm_plan_s *p)
 {
     if (p->pipe_ready) return cudaSuccess;
     sddmm_handle_s *h = p->h;
     const int chunks = p->n_pipe;
-    cudaError_t e = ensure_used_rows(p);
-    if (e == cudaSuccess) e = ensure_used_cols(p);
     PickAt at{};
     for (int i = 0; i < chunks; ++i) {
         p->pipe_nnz[i] = (p->nnz * i / chunks) & ~(int64_t)31;
@@ -273,7 +290,7 @@ cudaError_t ensure_pipe(sddmm_plan_s *p)
     }
     p->pipe_nnz[chunks] = p->nnz;
     at.v[2 * chunks - 1] = p->nnz - 1;
-    if (e == cudaSuccess) e = pick_values(p->d_rows, at, 2 * chunks, h->d_words, h->stream);
+    cudaError_t e = pick_values(p->d_rows, at, 2 * chunks, h->d_words, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return e;
     int64_t next_row = 0;  // first row of W no earlier chunk uploads
@@ -281,14 +298,8 @@ cudaError_t ensure_pipe(sddmm_plan_s *p)
         const int64_t first = (int64_t)h->h_words[2 * i], r1 = (int64_t)h->h_words[2 * i + 1] + 1;
         p->pipe_w_begin[i] = first > next_row ? first : next_row;
         p->pipe_w_end[i] = r1 > p->pipe_w_begin[i] ? r1 : p->pipe_w_begin[i];
-        at.v[i] = p->pipe_w_begin[i];
         if (r1 > next_row) next_row = r1;
     }
-    e = rank_values(p->d_used_rows, p->n_used_rows, at, chunks, h->d_words, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return e;
-    for (int i = 0; i < chunks; ++i) p->pipe_list_begin[i] = (int64_t)h->h_words[i];
-    p->pipe_list_begin[chunks] = p->n_used_rows;
     p->pipe_ready = true;
     return cudaSuccess;
 }
@@ -584,8 +595,8 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         }
     }
     // chunks of the host-operand pipeline; what they need is built by the first call with host operands
-    if (p->n_col_tiles == 1 && p->dense.n_cells == 0 && nnz >= (1 << 20)) {
-        const int64_t chunks = std::min<int64_t>((int64_t)sizeof(float) * M * K / (128ll << 20), SDDMM_PIPE_MAX_CHUNKS);
+    if (p->n_col_tiles == 1 && p->dense.n_cells == 0 && nnz >= (1 << 17)) {
+        const int64_t chunks = std::min<int64_t>((int64_t)sizeof(float) * M * K / (32ll << 20), SDDMM_PIPE_MAX_CHUNKS);
         if (chunks >= 2) p->n_pipe = (int)chunks;
     }
     if (more) {
@@ -608,6 +619,7 @@ int sddmm_destroy_plan(sddmm_plan_t p)
     free_plan_memory(p);
     if (p->clock >= 0) p->h->free_clocks.push_back(p->clock);
     for (sddmm_plan_s *&owner : p->h->ev_owner) if (owner == p) owner = nullptr;
+    if (p->h->pipe_owner == p) p->h->pipe_owner = nullptr;
     (void)cudaGetLastError();
     delete p;
     return SDDMM_OK;
@@ -675,16 +687,33 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     float *dP = P;
     const size_t wbytes = sizeof(float) * (size_t)p->M * p->K, hbytes = sizeof(float) * (size_t)p->N * p->K;
     const size_t nbytes = sizeof(float) * (size_t)p->nnz;
-    // W in host memory and a plain ring-kernel plan: upload W (and S) chunk by chunk
-    // and let every chunk's kernel and download run behind the later uploads
     const bool w_t = (flags & SDDMM_FLAG_W_TRANSPOSED) != 0, h_t = (flags & SDDMM_FLAG_H_TRANSPOSED) != 0;
+    // W in host memory and the row path: upload W (and S) chunk by chunk and let every chunk's kernel and download run
+    // behind the later uploads
     const bool pipelined = h->pipeline && p->n_pipe > 0 && !w_dev && !use_gather && !use_panel && !tiled_out && !p->d_perm &&
                            p->dense.n_cells == 0 && !w_t && !h_t;
     if (pipelined) CUDA_TRY(h, ensure_pipe(p));
-    // page-locked, mapped host arrays are read row by row by the GPU: only the rows a nonzero touches travel
-    const float *W_mapped = (pipelined && h->sparse_upload) ? mapped_host_ptr(W) : nullptr;
-    const float *H_mapped = (pipelined && h->sparse_upload && !h_dev) ? mapped_host_ptr(H) : nullptr;
+    // page-locked, mapped host arrays are read by the GPU: one launch for all of them instead of a copy each, and of W and
+    // H only the rows that a nonzero touches travel (short rows all do: reads below 128 bytes waste the link)
+    const float *W_mapped = h->sparse_upload && !w_dev && !w_t ? mapped_host_ptr(W) : nullptr;
+    const float *H_mapped = h->sparse_upload && !h_dev && !h_t ? mapped_host_ptr(H) : nullptr;
+    // a large array with nearly all rows used: the copy engine moves whole arrays at 56 GB/s, the kernel rows at 45 to 50
+    constexpr size_t LARGE = 4 << 20;
+    if (W_mapped && wbytes >= LARGE && p->n_nonempty_rows > p->M * 7 / 8) W_mapped = nullptr;
+    if (H_mapped && hbytes >= LARGE) {
+        int64_t used = 0;  // counted once per plan
+        const int st = sddmm_plan_count_cols(p, &used);
+        if (st != SDDMM_OK) return st;
+        if (used > p->N * 7 / 8) H_mapped = nullptr;
+    }
+    const float *S_mapped = h->sparse_upload && Sval && !s_dev ? mapped_host_ptr(Sval) : nullptr;
+    const bool used_rows_only = p->K >= 32;
+    if (used_rows_only) CUDA_TRY(h, ensure_upload_marks(p, W_mapped != nullptr, H_mapped != nullptr));
+    UploadRows up_w, up_h;
+    up_w.row_bytes = up_h.row_bytes = p->K * (int)sizeof(float);
+    const float *up_s = nullptr;
     p->last_h2d_bytes = p->last_d2h_bytes = 0;
+    p->last_h2d_used_cols = false;
     // K-major operands (the layout make_HTasH builds, util.h:68-73): brought to the device if need be and
     // transposed there into the plan's row-major staging copy
     if (h_t) {
@@ -701,8 +730,12 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     } else if (!h_dev) {
         if (!p->d_H) CUDA_TRY(h, dev_alloc(p, &p->d_H, (size_t)p->N * p->K));
         if (H_mapped) {
-            LAUNCH_TRY(h, launch_upload_rows(H_mapped, p->d_H, p->d_used_cols, p->n_used_cols, p->K, h->upload_ctas, s));
-            p->last_h2d_bytes += (int64_t)sizeof(float) * p->n_used_cols * p->K;
+            up_h.src = reinterpret_cast<const char *>(H_mapped);
+            up_h.dst = reinterpret_cast<char *>(p->d_H);
+            up_h.col_used = used_rows_only ? p->d_col_used : nullptr;
+            up_h.end = p->N;
+            p->last_h2d_used_cols = used_rows_only;
+            if (!used_rows_only) p->last_h2d_bytes += (int64_t)hbytes;
         } else {
             CUDA_TRY(h, cudaMemcpyAsync(p->d_H, H, hbytes, cudaMemcpyHostToDevice, s));
             p->last_h2d_bytes += (int64_t)hbytes;
@@ -722,7 +755,13 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         dW = p->d_W;
     } else if (!w_dev) {
         if (!p->d_W) CUDA_TRY(h, dev_alloc(p, &p->d_W, (size_t)p->M * p->K));
-        if (!pipelined) {
+        if (W_mapped) {
+            up_w.src = reinterpret_cast<const char *>(W_mapped);
+            up_w.dst = reinterpret_cast<char *>(p->d_W);
+            up_w.row_ptr = used_rows_only ? p->d_row_ptr : nullptr;
+            up_w.end = p->M;
+            p->last_h2d_bytes += used_rows_only ? (int64_t)sizeof(float) * p->n_nonempty_rows * p->K : (int64_t)wbytes;
+        } else if (!pipelined) {
             CUDA_TRY(h, cudaMemcpyAsync(p->d_W, W, wbytes, cudaMemcpyHostToDevice, s));
             p->last_h2d_bytes += (int64_t)wbytes;
         }
@@ -730,13 +769,22 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     }
     if (Sval && !s_dev) {
         if (!p->d_S) CUDA_TRY(h, dev_alloc(p, &p->d_S, (size_t)p->nnz));
-        if (!pipelined) CUDA_TRY(h, cudaMemcpyAsync(p->d_S, Sval, nbytes, cudaMemcpyHostToDevice, s));
+        if (S_mapped) up_s = S_mapped;
+        else if (!pipelined) CUDA_TRY(h, cudaMemcpyAsync(p->d_S, Sval, nbytes, cudaMemcpyHostToDevice, s));
         p->last_h2d_bytes += (int64_t)nbytes;
         dS = p->d_S;
     }
+    const bool use_dense = !forced && !tiled_out && p->dense.n_cells > 0;
+    // a call that is one gather launch is timed by the kernel itself, everything else by events
+    const bool one_gather = !use_dense && !use_panel &&
+                            !(ring_supports(p->K) && (use_ring || (!use_gather && ring_preferred(p->N, p->K))));
+    bool p_copy = false;
     if (!p_dev) {
-        if (!p->d_P) CUDA_TRY(h, dev_alloc(p, &p->d_P, (size_t)p->nnz));
-        dP = p->d_P;
+        // a small P is written to mapped host memory by the kernel: its 32-byte stores over PCIe cost less than a copy
+        float *P_mapped = one_gather && !pipelined && h->sparse_upload && nbytes <= (256 << 10) ? const_cast<float *>(mapped_host_ptr(P, 4)) : nullptr;
+        p_copy = !P_mapped;
+        if (p_copy && !p->d_P) CUDA_TRY(h, dev_alloc(p, &p->d_P, (size_t)p->nnz));
+        dP = P_mapped ? P_mapped : p->d_P;
         p->last_d2h_bytes = (int64_t)nbytes;
     }
 
@@ -752,19 +800,23 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
                          : p->K <= 128             ? "ring_small (pipelined chunks)"
                                                    : "ring (pipelined chunks)";
         CUDA_TRY(h, ensure_pipeline(h));
+        if (h->pipe_owner && h->pipe_owner != p && h->pipe_owner->ms_state == sddmm_plan_s::MS_IN_PIPE)
+            CUDA_TRY(h, resolve_ms(h->pipe_owner));
+        h->pipe_owner = p;
         for (int i = 0; i < p->n_pipe; ++i) {
             const int64_t n0 = p->pipe_nnz[i], cnt = p->pipe_nnz[i + 1] - n0;
-            const int64_t r0 = p->pipe_w_begin[i], r1 = p->pipe_w_end[i];
-            if (W_mapped) {
-                const int64_t l0 = p->pipe_list_begin[i], ln = p->pipe_list_begin[i + 1] - l0;
-                LAUNCH_TRY(h, launch_upload_rows(W_mapped, p->d_W, p->d_used_rows + l0, ln, p->K, h->upload_ctas, s));
-                p->last_h2d_bytes += (int64_t)sizeof(float) * ln * p->K;
-            } else if (r1 > r0) {
+            up_w.begin = p->pipe_w_begin[i];
+            up_w.end = W_mapped ? p->pipe_w_end[i] : up_w.begin;
+            if (W_mapped || up_s || (i == 0 && up_h.src))
+                LAUNCH_TRY(h, launch_upload_operands(i == 0 ? up_h : UploadRows(), up_w, up_s ? up_s + n0 : nullptr,
+                                                     up_s ? p->d_S + n0 : nullptr, up_s ? cnt : 0, h->upload_ctas, s));
+            if (!W_mapped && p->pipe_w_end[i] > p->pipe_w_begin[i]) {
+                const int64_t r0 = p->pipe_w_begin[i], r1 = p->pipe_w_end[i];
                 CUDA_TRY(h, cudaMemcpyAsync(p->d_W + r0 * p->K, W + r0 * p->K, sizeof(float) * (size_t)(r1 - r0) * p->K,
                                             cudaMemcpyHostToDevice, s));
                 p->last_h2d_bytes += (int64_t)sizeof(float) * (r1 - r0) * p->K;
             }
-            if (Sval && !s_dev)
+            if (Sval && !s_dev && !up_s)
                 CUDA_TRY(h, cudaMemcpyAsync(p->d_S + n0, Sval + n0, sizeof(float) * (size_t)cnt, cudaMemcpyHostToDevice, s));
             CUDA_TRY(h, cudaEventRecord(h->pipe_uploaded[i], s));
             CUDA_TRY(h, cudaStreamWaitEvent(h->pipe_compute, h->pipe_uploaded[i], 0));
@@ -784,19 +836,11 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         CUDA_TRY(h, cudaStreamWaitEvent(s, h->pipe_joined, 0));
         CUDA_TRY(h, cudaStreamSynchronize(s));
         waited_for(p, s);
-        p->ms_state = sddmm_plan_s::MS_KNOWN;
-        p->last_ms = 0.f;  // kernel time only: the chunks' kernels, not the waits for uploads between them
-        for (int i = 0; i < p->n_pipe; ++i) {
-            float ms = 0.f;
-            CUDA_TRY(h, cudaEventElapsedTime(&ms, h->pipe_started[i], h->pipe_computed[i]));
-            p->last_ms += ms;
-        }
+        p->ms_state = sddmm_plan_s::MS_IN_PIPE;
         return check_device_status(h);
     }
-    const bool use_dense = !forced && !tiled_out && p->dense.n_cells > 0;
-    // a call that is one gather launch is timed by the kernel itself, everything else by events
-    const bool one_gather = !use_dense && !use_panel &&
-                            !(ring_supports(p->K) && (use_ring || (!use_gather && ring_preferred(p->N, p->K))));
+    if (up_w.src || up_h.src || up_s)
+        LAUNCH_TRY(h, launch_upload_operands(up_h, up_w, up_s, p->d_S, up_s ? p->nnz : 0, h->upload_ctas, s));
     CallTimer timer(p, async);
     CUDA_TRY(h, timer.begin(one_gather, s));
     if (use_dense) {
@@ -845,7 +889,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             LAUNCH_TRY(h, launch_rows(p, rows_p, cols_p, perm, dS, dW, dH, dP, 0, p->nnz, use_ring, timer.clk, s));
     }
     CUDA_TRY(h, timer.end(s));
-    if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dP, nbytes, cudaMemcpyDeviceToHost, s));
+    if (p_copy) CUDA_TRY(h, cudaMemcpyAsync(P, dP, nbytes, cudaMemcpyDeviceToHost, s));
     if (async) return SDDMM_OK;
     CUDA_TRY(h, cudaStreamSynchronize(s));
     waited_for(p, s);
@@ -952,7 +996,12 @@ int sddmm_upload_rows(sddmm_handle_t h, const float *host, float *dev, const int
 int sddmm_last_transfer_bytes(sddmm_plan_t p, int64_t *h2d_bytes, int64_t *d2h_bytes)
 {
     if (!p) return SDDMM_INVALID_ARG;
-    if (h2d_bytes) *h2d_bytes = p->last_h2d_bytes;
+    int64_t cols = 0;
+    if (h2d_bytes && p->last_h2d_used_cols) {
+        const int st = sddmm_plan_count_cols(p, &cols);
+        if (st != SDDMM_OK) return st;
+    }
+    if (h2d_bytes) *h2d_bytes = p->last_h2d_bytes + (int64_t)sizeof(float) * cols * p->K;
     if (d2h_bytes) *d2h_bytes = p->last_d2h_bytes;
     return SDDMM_OK;
 }

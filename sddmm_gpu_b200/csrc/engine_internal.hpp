@@ -50,6 +50,7 @@ struct sddmm_handle_s {
     cudaEvent_t pipe_uploaded[SDDMM_PIPE_MAX_CHUNKS] = {};
     cudaEvent_t pipe_started[SDDMM_PIPE_MAX_CHUNKS] = {}, pipe_computed[SDDMM_PIPE_MAX_CHUNKS] = {};  // timing events
     cudaEvent_t pipe_joined = nullptr;
+    sddmm_plan_s *pipe_owner = nullptr;  // whose last call's times the chunk events hold
     bool pipeline = true;  // SDDMM_PIPELINE=0 keeps upload, kernel and download strictly one after the other
     // pipelined calls whose host operands are page-locked and mapped upload only the rows of
     // W and H that a nonzero touches, read by the GPU (SDDMM_SPARSE_UPLOAD=0: whole arrays by cudaMemcpy)
@@ -91,20 +92,20 @@ struct sddmm_plan_s {
     bool pending = false, async_pending = false, async_mixed = false;
     cudaStream_t async_stream = nullptr;
     int clock = -1;              // index of this plan's kernel clock in the handle's array
-    enum { MS_KNOWN, MS_IN_CLOCK, MS_IN_EVENTS } ms_state = MS_KNOWN;  // where the last call's kernel time is
+    enum { MS_KNOWN, MS_IN_CLOCK, MS_IN_EVENTS, MS_IN_PIPE } ms_state = MS_KNOWN;  // where the last call's kernel time is
     int ev_pair = -1;
     // chunks of the host-operand pipeline (0 = not pipelined): nonzeros
     // [pipe_nnz[i], pipe_nnz[i+1]); filled by ensure_pipe
     int n_pipe = 0;
     bool pipe_ready = false;
     int64_t pipe_nnz[SDDMM_PIPE_MAX_CHUNKS + 1] = {};
-    // rows of W chunk i uploads: [pipe_w_begin[i], pipe_w_end[i]) (empty when an earlier chunk brought them),
-    // = entries [pipe_list_begin[i], pipe_list_begin[i+1]) of the used-row list
+    // rows of W chunk i uploads: [pipe_w_begin[i], pipe_w_end[i]) (empty when an earlier chunk brought them)
     int64_t pipe_w_begin[SDDMM_PIPE_MAX_CHUNKS] = {}, pipe_w_end[SDDMM_PIPE_MAX_CHUNKS] = {};
-    int64_t pipe_list_begin[SDDMM_PIPE_MAX_CHUNKS + 1] = {};
+    unsigned char *d_col_used = nullptr;  // marks of the columns that hold a nonzero (row upload of H)
     int32_t *d_used_rows = nullptr, *d_used_cols = nullptr;  // ascending ids of the rows / columns holding a nonzero
     int64_t n_used_rows = 0, n_used_cols = 0;
     int64_t last_h2d_bytes = 0, last_d2h_bytes = 0;  // moved by the last sddmm_execute
+    bool last_h2d_used_cols = false;                 // and the rows of H of the columns that hold a nonzero (counted on request)
     const char *last_kernel = "none";                // kernels the last sddmm_execute launched
     float *d_spmm_scratch = nullptr;  // partial rows of SpMM / fused SDDMM->SpMM, allocated on first use
 };
