@@ -169,7 +169,7 @@ cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const
                                   int *dev_status, cudaStream_t stream);
 
 // SpMM (W null) / fused SDDMM->SpMM (spmm.cu): device arrays, input order.  scratch: spmm_scratch_floats() floats for
-// partial rows; clock as in launch_gather.  K a multiple of 4, at most 1024 (spmm_supports).
+// partial rows, the first spmm_counter_floats() of them zeroed once (every call leaves them zero); clock as in launch_gather.  K a multiple of 4, at most 1024 (spmm_supports).
 struct SpmmCall {
     const int32_t *rows, *cols;
     const int64_t *row_ptr;
@@ -182,6 +182,7 @@ struct SpmmCall {
     unsigned long long *clock;
 };
 bool spmm_supports(int K);
+size_t spmm_counter_floats(int64_t nnz, int K, int sm_count);
 size_t spmm_scratch_floats(int64_t nnz, int K, int sm_count);
 cudaError_t launch_spmm(const SpmmCall &call, int sm_count, int64_t *n_launches, cudaStream_t stream);
 

@@ -1078,8 +1078,10 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     // the class that sddmm_last_kernel_name reports (SDDMM_SPMM_RING=0: never the long-row one)
     bool ring = ring_supports(p->K) && p->nnz >= 65536;
     if (const char *env = std::getenv("SDDMM_SPMM_RING")) ring = ring && std::atoi(env) != 0;
-    if (!p->d_spmm_scratch && p->nnz > 0)
+    if (!p->d_spmm_scratch && p->nnz > 0) {
         CUDA_TRY(h, dev_alloc(p, &p->d_spmm_scratch, spmm_scratch_floats(p->nnz, p->K, h->sm_count)));
+        CUDA_TRY(h, cudaMemsetAsync(p->d_spmm_scratch, 0, sizeof(float) * spmm_counter_floats(p->nnz, p->K, h->sm_count), h->stream));
+    }
     cudaStream_t s = h->stream;
     CallTmp tmp;
     auto stage_in = [&](int slot, const float *src, size_t count, const float **dst) -> cudaError_t {

@@ -17,12 +17,15 @@
 // starts the next one.  Runs are equal shares of the nonzeros whatever the rows look like, so a power-law matrix
 // loads every warp alike, and nothing is built per plan.  A row that crosses a run boundary leaves partial rows in
 // scratch -- tail[q]: run q's part of the row that goes on in run q + 1, head[q]: run q's part of a row that
-// began before it and ends in it -- and spmm_fixup_kernel adds them in run order: no atomics on Y, the result does
-// not depend on scheduling.  Rows of S without nonzeros are zeroed by blocks of their own at the end of the grid.
+// began before it and ends in it.  The run that arrives last at a row (a counter per row) adds the parts in run order:
+// no atomics on Y, the result does not depend on scheduling, and there is no second launch (a fix-up kernel took a third
+// of a call with ten thousand nonzeros).  Parts are added in groups of 16 runs, each by its last run, and the groups by the
+// last of those, so that a row of hundreds of runs does not end in one long chain.  Rows of S without nonzeros are
+// zeroed by blocks of their own at the end of the grid.
 //
 // What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero through L2; used twice in the fused form), hidden
 // by resident warps.  Measured on R-MAT matrices against the row-task and shared-memory-ring kernels this replaces
-// (us): SpMM, 6.0 M nonzeros, 250 K x 250 K: K = 64 755 -> 136;  0.67 M nonzeros: K = 64 379 -> 31;  fused, 16.1 M
+// (us): SpMM, 6.0 M nonzeros, 250 K x 250 K: K = 64 755 -> 125;  0.67 M nonzeros: K = 64 379 -> 29;  fused, 16.1 M
 // nonzeros, 1 M x 1 M: K = 256 2970 -> 1675;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.
 // At K = 64 the gather kernel alone runs at 14.2 TB/s of gathered bytes.
 #include <cuda_runtime.h>
@@ -43,9 +46,7 @@ constexpr int SP_TPB = 256;
 constexpr int SP_NB = 8;         // nonzeros of a set per index step (4 when a set is 4 lanes)
 constexpr int SP_MAX_RUN = 1024;  // bounds the scratch of partial rows
 
-// What a run tells the fix-up (run_row): the row that goes on in the next run, RUN_MIDDLE added when it also began before
-// this run, or RUN_ENDS.
-constexpr int RUN_ENDS = 0x7fffffff, RUN_MIDDLE = (int)0x80000000;
+constexpr unsigned SP_GROUP = 16;  // partial rows that one run adds
 
 // L lanes per nonzero, F pieces per lane, B nonzeros of a set in flight, CTAS resident blocks asked of the compiler.  PF: the
 // W rows of the next step are prefetched into L1.  JOINT: the B dot products are reduced together (fewer shuffles, more
@@ -62,6 +63,12 @@ __device__ __forceinline__ void stg_u64x2(char *p, u64x2 v)
 {
     asm volatile("st.global.cs.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v.a), "l"(v.b) : "memory");
 }
+__device__ __forceinline__ u64x2 ldcg_u64x2(const char *p)  // from L2: written by another SM during this launch
+{
+    u64x2 r;
+    asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(r.a), "=l"(r.b) : "l"(p) : "memory");
+    return r;
+}
 __device__ __forceinline__ unsigned long long pair_of(float x)
 {
     unsigned long long d;
@@ -73,7 +80,7 @@ template <class S>
 __global__ void __launch_bounds__(SP_TPB, S::CTAS)
 spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const float *__restrict__ val,
             const char *__restrict__ W, const char *__restrict__ H, float *__restrict__ P_out, char *__restrict__ Y,
-            char *__restrict__ scratch, int *__restrict__ run_row, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces,
+            char *scratch, unsigned *arrived, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces,
             unsigned run_len, unsigned gather_blocks, unsigned long long *clock)
 {
     constexpr int L = S::L, F = S::F, B = S::B, NB = S::NB, G = S::G;
@@ -126,7 +133,9 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     unsigned j = j0 + il;
     auto at = [&](unsigned x) { return x < nnz ? x : nnz - 1; };
     int cur = __ldg(rows + at(j0));                                // row being summed
-    bool head = j0 > 0 && __ldg(rows + at(j0 - 1)) == cur;         // it began in an earlier run
+    const int row0 = cur;
+    const bool began_before = j0 > 0 && __ldg(rows + at(j0 - 1)) == cur;  // it began in an earlier run
+    bool head = began_before;                                      // and nothing of it has been stored yet
     if (FUSED) load_w((unsigned)cur);
     int r, c;
     float s = 1.f;
@@ -253,79 +262,65 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     if (j0 < nnz) {
         const unsigned end = j0 + run_len;
         const bool goes_on = end < nnz && __ldg(rows + end) == cur;
-        if (lig == 0) run_row[run] = goes_on ? cur | (head ? RUN_MIDDLE : 0) : RUN_ENDS;
         flush(goes_on ? scratch + (size_t)(2 * run + 1) * row_bytes
                       : head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
-    }
-    clock_end(clock);
-}
-
-// Rows that cross a run boundary: Y[row] = tail[first run] + ... + tail[last run - 1] + head[last run].  A set of
-// lanes (1 << log_set, as many as a row has pieces, 32 at most) per run; the row's first run does the row.  Most rows
-// cross one boundary: two loads of run_row, two partial rows, one store.  A row of many runs is left to its whole block.
-__global__ void __launch_bounds__(256)
-spmm_fixup_kernel(const int *__restrict__ run_row, const int64_t *__restrict__ row_ptr, const char *__restrict__ scratch,
-                  char *__restrict__ Y, unsigned n_runs, int pieces, int log_set, unsigned run_len, unsigned long long *clock)
-{
-    constexpr unsigned ALONE = 16;  // partial rows a set adds by itself
-    __shared__ unsigned many[256];  // first runs of the rows with more
-    __shared__ unsigned n_many;
-    __shared__ float4 part[256];
-    const int tid = threadIdx.x;
-    if (tid == 0) n_many = 0;
-    __syncthreads();
-    const size_t row_bytes = (size_t)pieces * 16;
-    auto partial = [&](unsigned q, unsigned last, int piece) {  // run q's part of a row that ends in run `last`
-        return __ldcs(reinterpret_cast<const float4 *>(scratch + (size_t)(2 * q + (q < last ? 1 : 0)) * row_bytes) + piece);
-    };
-    auto add = [](float4 &a, float4 b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
-    auto sum = [&](unsigned q0, unsigned q1, unsigned last, int piece) {  // runs [q0, q1), in order
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        unsigned q = q0;
-        for (; q + 8 <= q1; q += 8) {
-            float4 v[8];
+        // the rows that this run left a part of: the one it began with, the one it ends with
+        const int part_row[2] = {began_before && !head ? row0 : -1, goes_on || head ? cur : -1};
+        if (part_row[0] >= 0 || part_row[1] >= 0) {
+            const unsigned lanes = L == 32 ? FULL : ((1u << (L & 31)) - 1u) << (set * L);
+            auto arrive = [&](unsigned *count) {  // how many came before; everything this set stored is visible first
+                __threadfence();
+                __syncwarp(lanes);
+                unsigned before = 0;
+                if (lig == 0) before = atomicAdd(count, 1u);
+                return __shfl_sync(lanes, before, set * L);
+            };
+#pragma unroll 1
+            for (int k = 0; k < 2; ++k) {
+                if (part_row[k] < 0) continue;
+                const size_t row = (size_t)part_row[k];
+                const unsigned first = (unsigned)row_ptr[row] / run_len, last = (unsigned)(row_ptr[row + 1] - 1) / run_len;
+                auto part = [&](unsigned q) { return scratch + (size_t)(2 * q + (q < last ? 1 : 0)) * row_bytes + lig * 16; };
+                auto add_up = [&](unsigned q0, unsigned q1, unsigned step) {  // y = parts q0, q0 + step, ... <= q1
+                    constexpr int U = F <= 2 ? 4 : F <= 4 ? 2 : 1;
+                    const unsigned long long one = pair_of(1.f);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = partial(q + u, last, piece);
+                    for (int f = 0; f < F; ++f) y[f] = u64x2{0, 0};
+#pragma unroll 1
+                    for (unsigned q = q0; q <= q1; q += U * step) {
+                        u64x2 v[U][F];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) add(acc, v[u]);
-        }
-        for (; q < q1; ++q) add(acc, partial(q, last, piece));
-        return acc;
-    };
-    auto last_run = [&](int row) { return (unsigned)((row_ptr[row + 1] - 1) / run_len); };
-    const unsigned q = (blockIdx.x * 256 + tid) >> log_set;
-    const int lig = tid & ((1 << log_set) - 1);
-    if (q + 1 < n_runs) {
-        const int m0 = __ldg(run_row + q), m1 = __ldg(run_row + q + 1);
-        if (m0 >= 0 && m0 != RUN_ENDS) {
-            const unsigned last = m1 >= 0 ? q + 1 : last_run(m0);
-            if (last - q < ALONE) {
-                for (int p = lig; p < pieces; p += 1 << log_set)
-                    reinterpret_cast<float4 *>(Y + (size_t)m0 * row_bytes)[p] = sum(q, last + 1, last, p);
-            } else if (lig == 0) {
-                many[atomicAdd(&n_many, 1u)] = q;  // (the order of the rows does not matter, each is summed alone)
+                        for (int u = 0; u < U; ++u)
+#pragma unroll
+                            for (int f = 0; f < F; ++f)
+                                v[u][f] = q + u * step <= q1 && (f < F - 1 || last_ok) ? ldcg_u64x2(part(q + u * step) + f * L * 16) : u64x2{0, 0};
+#pragma unroll
+                        for (int u = 0; u < U; ++u)
+#pragma unroll
+                            for (int f = 0; f < F; ++f) {
+                                y[f].a = ffma2(one, v[u][f].a, y[f].a);
+                                y[f].b = ffma2(one, v[u][f].b, y[f].b);
+                            }
+                    }
+                };
+                const unsigned g0 = first + (run - first) / SP_GROUP * SP_GROUP, g1 = min(g0 + SP_GROUP - 1, last);
+                // (a group that is the row's last run only needs no counter, and has none: the next row may begin in that run)
+                if (g1 > g0) {
+                    if (arrive(&arrived[2 * g0]) != g1 - g0) continue;
+                    if (lig == 0) arrived[2 * g0] = 0;  // for the next call
+                    __threadfence();
+                }
+                add_up(g0, g1, 1);
+                if (g0 != first || g1 != last) {
+                    flush(part(g0) - lig * 16);
+                    if (arrive(&arrived[2 * first + 1]) != (last - first) / SP_GROUP) continue;
+                    if (lig == 0) arrived[2 * first + 1] = 0;
+                    __threadfence();
+                    add_up(first, last, SP_GROUP);
+                }
+                flush(Y + row * row_bytes);
             }
         }
-    }
-    __syncthreads();
-    const unsigned n = n_many;
-    // a row of many runs: pieces across the threads, its runs in equal shares over the groups of threads
-    const int width = pieces < 32 ? 1 << log_set : (pieces + 31) / 32 * 32, groups = 256 / width;
-    const int piece = tid % width, group = tid / width;
-    for (unsigned k = 0; k < n; ++k) {
-        const unsigned f = many[k];
-        const int row = run_row[f];
-        const unsigned l = last_run(row), cnt = l - f + 1;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (group < groups && piece < pieces)
-            acc = sum(f + (unsigned)((uint64_t)cnt * group / groups), f + (unsigned)((uint64_t)cnt * (group + 1) / groups), l, piece);
-        part[tid] = acc;
-        __syncthreads();
-        if (group == 0 && piece < pieces) {
-            for (int g = 1; g < groups; ++g) add(acc, part[g * width + piece]);
-            reinterpret_cast<float4 *>(Y + (size_t)row * row_bytes)[piece] = acc;
-        }
-        __syncthreads();
     }
     clock_end(clock);
 }
@@ -333,15 +328,17 @@ spmm_fixup_kernel(const int *__restrict__ run_row, const int64_t *__restrict__ r
 template <class S>
 unsigned run_length(int64_t nnz, int sm_count)
 {
-    // Waves of resident sets against the cost of a run's start and its two partial rows.  Six waves; down to three where
-    // runs would be shorter than 56 nonzeros, up to twelve where they would be longer than 160 (us at 12 / 6 / 3 waves:
-    // fused 16.1 M nonzeros K = 256 1704 / 1775 / 1878; fused 0.9 M K = 256 144 / 130 / 125; SpMM 6 M K = 256 391 / 375).
+    // Waves of resident sets against the cost of a run's two ends.  Six waves; down to three where runs would be shorter
+    // than 80 nonzeros, up to twelve where they would be longer than 160 (us at 12 / 6 / 3 waves: fused 16.1 M nonzeros
+    // K = 256 1704 / 1775 / 1878; fused 0.9 M K = 256 144 / 130 / 125; SpMM 6 M K = 64, 3 waves against 6: 125 / 136).
+    // Below three waves runs of three steps, two where those leave resident sets idle, one where nearly all are
+    // (0.7 M nonzeros K = 64 at 24 / 16: 29.7 / 33.9; 0.3 M at 16 / 8: 17.2 / 23.0; 20 K at 16 / 8: 13.4 / 11.6).
     const int64_t wave = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G;
     int64_t run = nnz / (6 * wave);
-    if (run < 56) run = std::min<int64_t>(56, nnz / (3 * wave));
+    if (run < 80) run = std::min<int64_t>(80, nnz / (3 * wave));
     if (run > 160) run = std::max<int64_t>(160, nnz / (12 * wave));
     run = run / S::NB * S::NB;
-    if (run < 2 * S::NB) run = 2 * S::NB;
+    if (run < 3 * S::NB) run = nnz <= S::NB * wave / 4 ? S::NB : nnz <= S::NB * wave ? 2 * S::NB : 3 * S::NB;
     if (run > SP_MAX_RUN) run = SP_MAX_RUN;
     return (unsigned)run;
 }
@@ -355,21 +352,13 @@ cudaError_t launch_shape(const SpmmCall &a, int sm_count, int64_t *n_launches, c
     const unsigned sets_per_block = SP_TPB / 32 * S::G;
     const unsigned gather_blocks = (n_runs + sets_per_block - 1) / sets_per_block;
     const unsigned zero_blocks = (unsigned)((a.M + SP_TPB - 1) / SP_TPB);
-    char *const scratch = reinterpret_cast<char *>(a.scratch), *const Y = reinterpret_cast<char *>(a.Y);
-    int *const run_row = reinterpret_cast<int *>(a.scratch + (size_t)n_runs * 2 * a.K);
+    // scratch: two counters per run, zero between calls, then the parts
+    unsigned *const arrived = reinterpret_cast<unsigned *>(a.scratch);
+    char *const parts = reinterpret_cast<char *>(a.scratch + spmm_counter_floats(a.nnz, a.K, sm_count));
     spmm_kernel<S><<<gather_blocks + zero_blocks, SP_TPB, 0, stream>>>(
-        a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H), a.P_out, Y, scratch,
-        run_row, a.row_ptr, (unsigned)a.nnz, a.M, pieces, run, gather_blocks, a.clock);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+        a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H), a.P_out,
+        reinterpret_cast<char *>(a.Y), parts, arrived, a.row_ptr, (unsigned)a.nnz, a.M, pieces, run, gather_blocks, a.clock);
     ++*n_launches;
-    if (n_runs < 2) return e;
-    ++*n_launches;
-    int log_set = 0;
-    while (log_set < 5 && (1 << log_set) < pieces) ++log_set;
-    const unsigned per_block = 256u >> log_set;
-    spmm_fixup_kernel<<<(n_runs - 1 + per_block - 1) / per_block, 256, 0, stream>>>(run_row, a.row_ptr, scratch, Y, n_runs, pieces,
-                                                                                  log_set, run, a.clock);
     return cudaGetLastError();
 }
 
@@ -421,12 +410,16 @@ auto with_shape(int K, bool fused, Fn f)
 
 bool spmm_supports(int K) { return K > 0 && K % 4 == 0 && K <= 1024; }
 
-size_t spmm_scratch_floats(int64_t nnz, int K, int sm_count)
+static size_t max_runs(int64_t nnz, int K, int sm_count)  // of either form
 {
-    // enough for either form
     auto run_of = [&](bool fused) { return with_shape(K, fused, [&](auto s) { return run_length<decltype(s)>(nnz, sm_count); }); };
     const unsigned run = std::min(run_of(false), run_of(true));
-    return (size_t)((nnz + run - 1) / run) * (2 * (size_t)K + 1);  // two partial rows and one word per run
+    return (size_t)((nnz + run - 1) / run);
+}
+size_t spmm_counter_floats(int64_t nnz, int K, int sm_count) { return (2 * max_runs(nnz, K, sm_count) + 31) / 32 * 32; }
+size_t spmm_scratch_floats(int64_t nnz, int K, int sm_count)
+{
+    return spmm_counter_floats(nnz, K, sm_count) + max_runs(nnz, K, sm_count) * 2 * (size_t)K;
 }
 
 cudaError_t launch_spmm(const SpmmCall &a, int sm_count, int64_t *n_launches, cudaStream_t stream)

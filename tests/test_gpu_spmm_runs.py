@@ -1,5 +1,6 @@
 """SpMM and the fused form at the run boundaries of csrc/spmm.cu: rows that end exactly where a run ends, that cross one
-boundary, that span a few runs (added by one set of lanes) and hundreds (added by a whole block), stretches of empty rows,
+boundary, that span a few runs, exactly sixteen and seventeen (one and two groups of parts) and hundreds, a row that begins in
+the run where a row of seventeen ends, stretches of empty rows, repeated calls (the counters are left at zero),
 and every lane shape's first and last K.
 
 Tolerance: as tests/test_gpu_spmm.py (1e-4 of the sum of magnitudes per entry of Y, against float64)."""
@@ -24,8 +25,11 @@ def _rows_of_lengths(rng, lengths, N):
 def test_run_boundaries(engine, K):
     rng = np.random.default_rng(K)
     N = 6000
-    # runs are 16 nonzeros at this size for most shapes (8 for K <= 16 and 36 <= K <= 48)
+    # runs are 8 or 16 nonzeros at this size (4 where sets are four lanes)
     lengths = [16, 16, 0, 0, 32, 8, 8, 15, 2, 1, 1, 1, 0, 70, 250, 5000, 3, 0, 0, 0, 16, 129, 6000, 0]
+    lengths = [6, 257, 9, 40, 272, 264, 140] + lengths   # row 1: 17 runs of 16, row 3 begins where it has ended
+    lengths += [(-sum(lengths)) % 16 + 8, 4, 65, 129, 3, 60, 124, 4,
+                8 + 16 * 15, 17 * 16, 5, 2]
     rows, cols = _rows_of_lengths(rng, lengths, N)
     M = len(lengths)
     vals = rng.standard_normal(rows.shape[0]).astype(np.float32)
@@ -44,6 +48,8 @@ def test_run_boundaries(engine, K):
     ref, A = oracle.cpu.spmm_f64(rows, cols, H, M, P64.astype(np.float32))
     _, A_from_p = oracle.cpu.spmm_f64(rows, cols, H, M, A_p)   # an error of 1e-4 A_p in p moves Y by up to that times |H|
     assert np.all(np.abs(Y - ref) <= TOL * (np.maximum(np.abs(ref), A) + A_from_p) + 1e-30)
-    plan.fused(W, H, Y2, vals)
-    assert np.array_equal(Y, Y2)
+    for _ in range(3):
+        Y2.fill(np.nan)
+        plan.fused(W, H, Y2, vals)
+        assert np.array_equal(Y, Y2)
     plan.close()
