@@ -49,8 +49,10 @@ constexpr int SP_MAX_RUN = 1024;  // bounds the scratch of partial rows
 constexpr unsigned SP_GROUP = 16;  // partial rows that one run adds
 
 // L lanes per nonzero, F pieces per lane, B nonzeros of a set in flight, CTAS resident blocks asked of the compiler.  PF: the
-// W rows of the next step are prefetched into L1.  JOINT: the B dot products are reduced together (fewer shuffles, more
-// registers).
+// W rows of the next step are prefetched into L1.  JOINT: the B dot products are reduced together and a block of B that opens
+// no row is summed without the tests for it.  Taken where a nonzero has a whole warp: 3.75 shuffles for each instead of 7 (B =
+// 4; fused, K = 256: 16.1 M nonzeros 1735 -> 1660 us, 6.0 M 567 -> 540; K = 200 583 -> 557), while with several sets in a warp
+// most blocks open a row in one of them (K = 128 871 -> 965).
 template <int L_, int F_, int B_, bool EXACT_, int CTAS_, bool FUSED_ = false, bool PF_ = false, bool JOINT_ = true>
 struct SpmmShape {
     static constexpr int L = L_, F = F_, B = B_, CTAS = CTAS_;
@@ -191,65 +193,101 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             u64x2 h[B][F];
             load_h(b, h);
             float p[B];  // the nonzeros' weights, the same in all lanes of the set
-            if (FUSED && S::JOINT) {
-                // all B products first, so that their reductions overlap: one transposed butterfly, then B broadcasts
-                float acc[B];
-#pragma unroll
-                for (int i = 0; i < B; ++i) {
-                    const int x = b + i;
-                    if (changed & (setmask << x)) {  // uniform over the warp: some set goes on to another row
-                        const int rj = __shfl_sync(FULL, r, x, L);
-                        if ((changed >> (set * L + x)) & 1u) load_w((unsigned)rj);
-                    }
-                    unsigned long long a0 = 0, a1 = 0;
-#pragma unroll
-                    for (int f = 0; f < F; ++f) {
-                        a0 = ffma2(w[f].a, h[i][f].a, a0);
-                        a1 = ffma2(w[f].b, h[i][f].b, a1);
-                    }
-                    acc[i] = fold2(a0) + fold2(a1);
-                }
-                reduce_transposed<L, B>(acc, lig);
-#pragma unroll
-                for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, acc[0], i * (L / B), L) * __shfl_sync(FULL, s, b + i, L);
-#pragma unroll
-                for (int i = 0; i < B; ++i)
-                    if (il == b + i) p_mine = p[i];
-            } else if (FUSED) {
-            } else {
-#pragma unroll
-                for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, s, b + i, L);
-            }
-#pragma unroll
-            for (int i = 0; i < B; ++i) {
-                const int x = b + i;
-                if (changed & (setmask << x)) {
-                    const int rj = __shfl_sync(FULL, r, x, L);
-                    if ((changed >> (set * L + x)) & 1u) {
-                        flush(head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
-                        head = false;
-                        cur = rj;
-                        if (FUSED && !S::JOINT) load_w((unsigned)rj);
-                    }
-                }
-                if (FUSED && !S::JOINT) {
-                    unsigned long long a0 = 0, a1 = 0;
-#pragma unroll
-                    for (int f = 0; f < F; ++f) {
-                        a0 = ffma2(w[f].a, h[i][f].a, a0);
-                        a1 = ffma2(w[f].b, h[i][f].b, a1);
-                    }
-                    float a = fold2(a0) + fold2(a1);
-#pragma unroll
-                    for (int off = L / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
-                    p[i] = a * __shfl_sync(FULL, s, x, L);
-                    if (il == x) p_mine = p[i];
-                }
-                const unsigned long long pp = pair_of(p[i]);
+            const unsigned here = changed >> b;
+            auto opens = [&](int i) { return (here & (setmask << i)) != 0; };  // uniform over the warp: some set goes on to another row
+            auto mine = [&](int i) { return ((here >> (set * L + i)) & 1u) != 0; };
+            auto next_row = [&](int to) {  // the finished row is stored
+                flush(head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
+                head = false;
+                cur = to;
+            };
+            auto add = [&](int i, float weight) {
+                const unsigned long long pp = pair_of(weight);
 #pragma unroll
                 for (int f = 0; f < F; ++f) {
                     y[f].a = ffma2(pp, h[i][f].a, y[f].a);
                     y[f].b = ffma2(pp, h[i][f].b, y[f].b);
+                }
+            };
+            if (FUSED && S::JOINT) {
+                // most blocks of B stay within their rows: one test for the block instead of two for each nonzero
+                const bool stays = (here & (setmask * ((1u << B) - 1u))) == 0;
+                auto dot = [&](int i) {
+                    unsigned long long a = 0;
+#pragma unroll
+                    for (int f = 0; f < F; ++f) {
+                        a = ffma2(w[f].a, h[i][f].a, a);
+                        a = ffma2(w[f].b, h[i][f].b, a);
+                    }
+                    return fold2(a);
+                };
+                // all B products first, so that their reductions overlap: one transposed butterfly leaves product i with the
+                // i-th B-th of the set's lanes, where it is scaled; then B broadcasts
+                float acc[B];
+                if (stays) {
+#pragma unroll
+                    for (int i = 0; i < B; ++i) acc[i] = dot(i);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < B; ++i) {
+                        if (opens(i)) {
+                            const int rj = __shfl_sync(FULL, r, b + i, L);
+                            if (mine(i)) load_w((unsigned)rj);
+                        }
+                        acc[i] = dot(i);
+                    }
+                }
+                reduce_transposed<L, B>(acc, lig);
+                const float scaled = acc[0] * __shfl_sync(FULL, s, b + lig / (L / B), L);
+#pragma unroll
+                for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, scaled, i * (L / B), L);
+                if (stays) {
+#pragma unroll
+                    for (int i = 0; i < B; ++i) add(i, p[i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < B; ++i) {
+                        if (opens(i)) {
+                            const int rj = __shfl_sync(FULL, r, b + i, L);
+                            if (mine(i)) next_row(rj);
+                        }
+                        add(i, p[i]);
+                    }
+                }
+                if (P_out) {
+#pragma unroll
+                    for (int i = 0; i < B; ++i)
+                        if (il == b + i) p_mine = p[i];
+                }
+            } else {
+                if (!FUSED) {
+#pragma unroll
+                    for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, s, b + i, L);
+                }
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    const int x = b + i;
+                    if (opens(i)) {
+                        const int rj = __shfl_sync(FULL, r, x, L);
+                        if (mine(i)) {
+                            next_row(rj);
+                            if (FUSED) load_w((unsigned)rj);
+                        }
+                    }
+                    if (FUSED) {
+                        unsigned long long a0 = 0, a1 = 0;
+#pragma unroll
+                        for (int f = 0; f < F; ++f) {
+                            a0 = ffma2(w[f].a, h[i][f].a, a0);
+                            a1 = ffma2(w[f].b, h[i][f].b, a1);
+                        }
+                        float a = fold2(a0) + fold2(a1);
+#pragma unroll
+                        for (int off = L / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
+                        p[i] = a * __shfl_sync(FULL, s, x, L);
+                        if (il == x) p_mine = p[i];
+                    }
+                    add(i, p[i]);
                 }
             }
         }
@@ -378,8 +416,8 @@ auto with_shape(int K, bool fused, Fn f)
         if (q < 32) return f(SpmmShape<8, 4, 1, false, 3, true, true, false>());
         if (q == 32) return f(SpmmShape<8, 4, 1, true, 4, true, false, false>());
         if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4, true, true, false>());
-        if (q < 64) return f(SpmmShape<32, 2, 2, false, 4, true, true, true>());
-        if (q == 64) return f(SpmmShape<32, 2, 2, true, 4, true, true, true>());
+        if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, true, true, true>());
+        if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, true, true, true>());
         if (q <= 96) return f(SpmmShape<32, 3, 1, false, 4, true, false, false>());
         if (q <= 128) return f(SpmmShape<32, 4, 1, false, 4, true, false, false>());
         if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3, true, false, false>());
