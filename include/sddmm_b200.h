@@ -160,8 +160,8 @@ SDDMM_API int sddmm_execute(sddmm_plan_t p, const float *W, const float *H,
  *                        the fly (Sval NULL: unscaled) -- P never goes to memory and every H row
  *                        is gathered once for both uses; P_out != NULL also stores P (input order).
  * K a multiple of 4 up to 1024 (SDDMM_K_UNSUPPORTED otherwise).  Pointers host or device (host
- * arrays are staged for the call); flags: 0 or SDDMM_FLAG_ASYNC (device pointers only).  Rows
- * are processed whole by one warp, long rows in pieces that are added in a fixed order: the
+ * arrays are staged for the call); flags: 0 or SDDMM_FLAG_ASYNC (device pointers only).  The
+ * nonzeros are cut into equal runs; the parts of a row of S that spans runs are added in run order: the
  * result does not depend on scheduling.  Works on the plan's input order (column tiles of the
  * plan are not used).  sddmm_last_kernel_ms() reports the kernels' time.
  */
