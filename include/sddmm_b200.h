@@ -275,7 +275,7 @@ typedef struct {
     int64_t device_bytes;   /* device memory the plan owns                     */
     float plan_ms;          /* device time of the binning pass                 */
     int32_t reserved0;
-    int64_t n_dense_cells;  /* 128 x 64 cells handed to the dense-cell kernel  */
+    int64_t n_dense_cells;  /* 128 x 64 cells that are dense enough for the dense-cell kernel; calls use it if nnz * K >= 2^26 */
     int64_t n_dense_nnz;    /* nonzeros inside them                            */
     int64_t n_hub_cols;     /* columns marked for L2 residency (ring kernel)   */
 } sddmm_plan_info;

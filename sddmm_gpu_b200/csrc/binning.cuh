@@ -113,6 +113,8 @@ struct DensePlan {
     int64_t n_dense_rows = 0, n_dense_cols = 0;
     void release();
 };
+// a cell is dense if it is a quarter full; cells are used if they hold half of S
+constexpr float DENSE_MIN_FILL = 0.25f, DENSE_MIN_SHARE = 0.5f;
 cudaError_t build_dense_cells(const int32_t *d_rows, const int32_t *d_cols, const int64_t *d_row_ptr, int64_t nnz,
                               int64_t M, int64_t N, float min_density, float min_share, DensePlan *out,
                               cudaStream_t stream);

@@ -570,14 +570,19 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     // Locally dense matrices (many nonzeros per row): cells that are at least a
     // quarter full go to the dense-cell kernel, if they hold half of S or more
     // (below that the second launch and the permuted remainder cost more than they save).
-    // SDDMM_DENSE_CELLS=0 switches the classification off.
+    // Below 2^26 multiplications the gather kernel is as fast or faster, and the plan need not be classified (us per call, band +
+    // global masks, gather / cells: 0.36 M nonzeros, K = 64 11 / 18;  0.9 M, K = 64 17 / 19;  1.1 M, K = 64 21 / 21;  1.9 M, K = 32
+    // 22 / 21;  1.6 M, K = 64 28 / 19;  0.9 M, K = 128 34 / 26;  planned, called and closed: 0.36 M, K = 64 42 / 365).
+    // SDDMM_DENSE_CELLS=0 switches the classification off, 1 takes it at every size.
     {
         const char *env = std::getenv("SDDMM_DENSE_CELLS");
-        const bool enabled = !(env && std::atoi(env) == 0);
-        if (enabled && p->n_col_tiles == 1 && p->n_nonempty_rows > 0 && nnz / p->n_nonempty_rows >= 32) {
+        const bool enabled = !(env && std::atoi(env) == 0), always = env && std::atoi(env) == 1;
+        const bool candidate = enabled && p->n_col_tiles == 1 && p->n_nonempty_rows > 0 && nnz / p->n_nonempty_rows >= 32;
+        p->cells_uncounted = candidate && !always && nnz * K < (1ll << 26);
+        if (candidate && !p->cells_uncounted) {
             PLAN_TRY(begin_more());
             PLAN_TRY(ensure_row_ptr(p));
-            PLAN_TRY(build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, nnz, M, N, 0.25f, 0.5f, &p->dense, s));
+            PLAN_TRY(build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, nnz, M, N, DENSE_MIN_FILL, DENSE_MIN_SHARE, &p->dense, s));
             if (p->dense.n_cells > 0)
                 p->device_bytes += (int64_t)(sizeof(DenseCell) * p->dense.n_cells + 6 * p->dense.n_dense_nnz + 17 * DENSE_CELL_ROWS * p->dense.n_cells +
                                              12 * p->dense.n_sparse);
@@ -1225,6 +1230,16 @@ int sddmm_plan_get_info(sddmm_plan_t p, sddmm_plan_info *info)
     PoolScope scope(p->h->pool, p->h->stream);
     CUDA_TRY(p->h, ensure_items(p));
     CUDA_TRY(p->h, ensure_hints(p));
+    if (p->cells_uncounted) {  // cells that no call uses: only counted
+        DensePlan cells;
+        CUDA_TRY(p->h, ensure_row_ptr(p));
+        const cudaError_t e = build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, p->nnz, p->M, p->N, DENSE_MIN_FILL, DENSE_MIN_SHARE, &cells, p->h->stream);
+        p->counted_cells = cells.n_cells;
+        p->counted_cell_nnz = cells.n_dense_nnz;
+        cells.release();
+        CUDA_TRY(p->h, e);
+        p->cells_uncounted = false;
+    }
     info->M = p->M; info->N = p->N; info->nnz = p->nnz; info->K = p->K;
     info->panel_rows = p->cfg.panel_rows;
     info->col_tile = p->col_tile;
@@ -1234,8 +1249,8 @@ int sddmm_plan_get_info(sddmm_plan_t p, sddmm_plan_info *info)
     info->n_nonempty_cols = p->n_nonempty_cols;
     info->device_bytes = p->device_bytes;
     info->plan_ms = p->plan_ms;
-    info->n_dense_cells = p->dense.n_cells;
-    info->n_dense_nnz = p->dense.n_dense_nnz;
+    info->n_dense_cells = p->dense.n_cells + p->counted_cells;
+    info->n_dense_nnz = p->dense.n_dense_nnz + p->counted_cell_nnz;
     info->n_hub_cols = p->n_hub_cols;
     return SDDMM_OK;
 }

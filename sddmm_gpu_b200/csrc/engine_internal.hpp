@@ -80,6 +80,8 @@ struct sddmm_plan_s {
     bool hints_built = false;
     // dense cells + row-sorted remainder (single-tile plans of locally dense matrices)
     DensePlan dense;
+    bool cells_uncounted = false;  // too little work for them: the cells are counted when the plan's info is asked for
+    int64_t counted_cells = 0, counted_cell_nnz = 0;
     int64_t n_hub_cols = 0;
     int64_t n_item_rows = 0;
     int64_t n_nonempty_rows = 0, n_nonempty_cols = -1;

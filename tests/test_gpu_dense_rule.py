@@ -1,0 +1,53 @@
+"""When a locally dense matrix goes through the dense-cell kernel (from nnz * K = 2^26 on), and that kernel at small sizes.
+
+Tolerance: tests/helpers.py (1e-4 of max(|ref|, sum of magnitudes) per nonzero, against the CPU oracle)."""
+import numpy as np
+import pytest
+
+from helpers import assert_parity
+from sddmm_gpu_b200 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(h, p, rows, cols, vals):
+    plan = h.plan_coo(p["M"], p["N"], rows, cols, p["W"].shape[1])
+    P = np.full(rows.shape[0], np.nan, np.float32)
+    plan.execute(p["W"], p["H"], P, vals)
+    name, info = plan.last_kernel_name(), plan.info()
+    again = np.full(rows.shape[0], np.nan, np.float32)
+    plan.execute(p["W"], p["H"], again, vals)    # the same kernel whether or not the cells have been counted meanwhile
+    assert plan.last_kernel_name() == name and np.array_equal(P, again)
+    plan.close()
+    assert_parity(P, rows, cols, p["W"], p["H"], vals)
+    return name, info
+
+
+@pytest.mark.parametrize("K", [256, 512])
+def test_line_between_the_kernels(engine, K):
+    p = synth.to_numpy(synth.attention_mask(M=1100, half_width=96, n_global=7, K=K, device="cpu"))
+    rows, cols = p["rows"], p["cols"]
+    work = rows.shape[0] * K
+    name, info = _run(engine, p, rows, cols, None)
+    assert (work >= 1 << 26) == (K == 512)
+    assert name.startswith("dense") == (K == 512)
+    assert info.n_dense_cells > 0 and 0 < info.n_dense_nnz <= info.nnz
+
+
+@pytest.mark.parametrize("M,half_width,n_global", [(300, 64, 0), (1100, 96, 7), (4096, 96, 20)])
+@pytest.mark.parametrize("mode", ["2", "1", "0"])
+@pytest.mark.parametrize("K", [16, 36, 64, 100, 256])
+def test_dense_cells_at_small_sizes(monkeypatch, K, mode, M, half_width, n_global):
+    # a CTA with one cell, with none, with several; chunks of K that are full, ragged, single
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")
+    monkeypatch.setenv("SDDMM_DENSE_TENSOR", mode)
+    h = api.Handle(0)
+    p = synth.to_numpy(synth.attention_mask(M=M, half_width=half_width, n_global=n_global, K=K, device="cpu"))
+    rng = np.random.default_rng(K)
+    rows, cols = p["rows"], p["cols"]
+    vals = rng.standard_normal(rows.shape[0]).astype(np.float32)
+    order = np.lexsort((rng.random(rows.shape[0]), rows))    # columns in random order inside each row: per-nonzero lists
+    for c, v in ((cols, vals), (cols, None), (cols[order], vals[order])):
+        name, info = _run(h, p, rows, c, v)
+        assert name.startswith("dense") and info.n_dense_cells > 0
+    h.close()
