@@ -21,7 +21,7 @@
 //               commits them to the stage's "empty" barrier; after a cell's last
 //               chunk it commits to the accumulator's "full" barrier;
 //   warps 9-24  epilogue: read the finished block from TMEM (tcgen05.ld, a quarter row per
-//               thread), release the accumulator (two of them alternate), park the
+//               thread), release the accumulator (one of four), park the
 //               block in shared memory and let the cell's nonzeros pick their entries.
 //
 // Shared-memory operand layout (K-major, 128-byte swizzle): a tile of R rows x 32 k is R lines of
@@ -68,7 +68,8 @@ constexpr int TC_SMEM_BYTES = STAGES * STAGE_BYTES + CT_BYTES;  // 182,272 bytes
 constexpr int N_PRODUCERS = 256, N_EPILOGUE = 512;
 constexpr int MMA_WARP = N_PRODUCERS / 32, EPI_WARP0 = MMA_WARP + 1;
 constexpr int TC_THREADS = N_PRODUCERS + 32 + N_EPILOGUE;  // 800
-constexpr uint32_t TMEM_COLS = 2 * DC;  // two accumulators
+constexpr unsigned N_ACC = 4;              // accumulators: the tensor core runs up to so many cells ahead of the epilogue
+constexpr uint32_t TMEM_COLS = N_ACC * DC;  // 256
 constexpr uint32_t LBO = 16, SBO = 8 * KC * 4;  // leading offset unused by swizzled K-major tiles; 8 rows of 128 bytes
 // What the epilogue needs to know about a cell before its product is there: fetched into shared memory two
 // cells ahead.
@@ -149,7 +150,7 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     float *Ct = reinterpret_cast<float *>(smem + STAGES * STAGE_BYTES);
-    __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[N_ACC], acc_empty[N_ACC];
     __shared__ MetaSlot meta[META_SLOTS];
     __shared__ uint32_t tmem_holder;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -159,7 +160,7 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
             mbar_init(&full_bar[s], N_PRODUCERS / 32);  // one arrival per producer warp, after all its lanes' stores
             mbar_init(&empty_bar[s], 1);           // one tcgen05.commit
         }
-        for (int b = 0; b < 2; ++b) {
+        for (unsigned b = 0; b < N_ACC; ++b) {
             mbar_init(&acc_full[b], 1);            // one tcgen05.commit
             mbar_init(&acc_empty[b], N_EPILOGUE / 32);  // one arrival per epilogue warp, after its tcgen05.ld
         }
@@ -266,7 +267,7 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
         // ---------------- MMA issue: the whole warp walks the loop, lane 0 issues ----------------
         unsigned g = 0, n_acc = 0;
         for (int i = 0; i < my_cells && ok; ++i) {
-            const unsigned b = n_acc & 1u, use = n_acc >> 1;
+            const unsigned b = n_acc % N_ACC, use = n_acc / N_ACC;
             // the epilogue has read this accumulator
             if (!wait_bar(&acc_empty[b], (use & 1u) ^ 1u)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -371,8 +372,11 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
             fetch_meta(i + 2);
             float n_lo[8], n_hi[8];
             load_s(i + 1, n_lo, n_hi);
-            const unsigned b = n_acc & 1u;
-            ok = epilogue_all(wait_bar(&acc_full[b], (n_acc >> 1) & 1u));
+            const unsigned b = n_acc % N_ACC;
+            // One warp polls, the barrier holds the others: polls take shared-memory bandwidth from the tensor core (all sixteen
+            // polling, without a sleep in between, 235 us; all with it and two accumulators 191; as here 185: 65,536-token
+            // mask, K = 64).
+            ok = epilogue_all(ew != 0 || wait_bar(&acc_full[b], (n_acc / N_ACC) & 1u));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             {
