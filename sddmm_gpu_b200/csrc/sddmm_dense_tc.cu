@@ -21,7 +21,7 @@
 //               commits them to the stage's "empty" barrier; after a cell's last
 //               chunk it commits to the accumulator's "full" barrier;
 //   warps 9-24  epilogue: read the finished block from TMEM (tcgen05.ld, a quarter row per
-//               thread), release the accumulator (one of four), park the
+//               thread), release the accumulator (one of eight), park the
 //               block in shared memory and let the cell's nonzeros pick their entries.
 //
 // Shared-memory operand layout (K-major, 128-byte swizzle): a tile of R rows x 32 k is R lines of
@@ -68,8 +68,10 @@ constexpr int TC_SMEM_BYTES = STAGES * STAGE_BYTES + CT_BYTES;  // 182,272 bytes
 constexpr int N_PRODUCERS = 256, N_EPILOGUE = 512;
 constexpr int MMA_WARP = N_PRODUCERS / 32, EPI_WARP0 = MMA_WARP + 1;
 constexpr int TC_THREADS = N_PRODUCERS + 32 + N_EPILOGUE;  // 800
-constexpr unsigned N_ACC = 4;              // accumulators: the tensor core runs up to so many cells ahead of the epilogue
-constexpr uint32_t TMEM_COLS = N_ACC * DC;  // 256
+// Accumulators: the tensor core runs up to so many cells ahead of the epilogue, which evens out what a cell takes in either (65,536-token
+// mask, K = 64: two 189 us, four 185, eight 180.5; K = 128 266, 260, 255).  All of tensor memory: no second CTA fits an SM anyway.
+constexpr unsigned N_ACC = 8;
+constexpr uint32_t TMEM_COLS = N_ACC * DC;  // 512
 constexpr uint32_t LBO = 16, SBO = 8 * KC * 4;  // leading offset unused by swizzled K-major tiles; 8 rows of 128 bytes
 // What the epilogue needs to know about a cell before its product is there: fetched into shared memory two
 // cells ahead.
@@ -374,8 +376,8 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
             load_s(i + 1, n_lo, n_hi);
             const unsigned b = n_acc % N_ACC;
             // One warp polls, the barrier holds the others: polls take shared-memory bandwidth from the tensor core (all sixteen
-            // polling, without a sleep in between, 235 us; all with it and two accumulators 191; as here 185: 65,536-token
-            // mask, K = 64).
+            // polling, without a sleep in between, 235 us; all with it 191, one 189, with two accumulators: 65,536-token mask,
+            // K = 64).
             ok = epilogue_all(ew != 0 || wait_bar(&acc_full[b], (n_acc / N_ACC) & 1u));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
