@@ -88,9 +88,10 @@ PanelConfig choose_panel_config(int K, int panel_rows_hint, int sm_count, size_t
 
 // Gather kernel (sddmm_gather.cu): any K % 4 == 0, no plan data needed; the default path.  perm as in launch_panel.
 // clock: two device words that receive the kernel's start and end (clock_begin / clock_end), or null.
+// beside (with perm only): may run beside the kernel before it in the stream, once that has signalled it; it ends no earlier.
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                           const float *W, const float *H, float *P, int64_t nnz, int K, int sm_count,
-                          unsigned long long *clock, cudaStream_t stream);
+                          unsigned long long *clock, cudaStream_t stream, bool beside = false);
 // The same over operands stored in bfloat16 (rows of 2K bytes): K = 256, 512 or 1024.
 bool gather_bf16_supports(int K);
 cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,

@@ -117,8 +117,8 @@ namespace sddmm {
 constexpr int N_KERNEL_CLOCKS = 1024;
 
 // SDDMM over nonzeros in the plan's processing order, [first, first + count): the ring kernel when it is the faster one
-// for this plan (or forced), else the gather kernel.
+// for this plan (or forced), else the gather kernel (beside: see launch_gather).
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
-                        unsigned long long *clock, cudaStream_t stream);
+                        unsigned long long *clock, cudaStream_t stream, bool beside = false);
 }  // namespace sddmm

@@ -178,6 +178,8 @@ sddmm_dense_tc_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_holder;
+    // every block runs: the gather kernel of the remaining nonzeros may start beside this one
+    if (tid == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int n_chunks = (K + KC - 1) / KC;
     bool ok = true;
     // The cells of this CTA: every gridDim.x-th of the list; cell_of(i) is the i-th of them.

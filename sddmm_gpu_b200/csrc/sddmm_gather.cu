@@ -33,6 +33,10 @@ using namespace dev;
 namespace {
 
 constexpr int GA_TPB = 256;
+// Launched beside the kernel before it in the stream (the remainder of a matrix with dense cells): the persistent block of the dense-cell
+// kernel leaves an SM 7,900 registers, room for two warps of any shape here (32 to 128 threads measure alike).  65,536-token mask, 0.3 M of
+// 44 M nonzeros left over, K = 64: 180 us after the cells, 168 beside them; 12,777 tokens 37 -> 29.6.
+constexpr int GA_TPB_BESIDE = 64;
 
 // L lanes per nonzero, F 16-byte pieces per lane, B nonzeros of a set in flight, RB nonzeros per reduction, CTAS
 // resident blocks per SM asked of the compiler.  EXACT: the L * F pieces are the row (no predicate on the last one).
@@ -96,7 +100,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
     clock_begin(clock);
     constexpr int L = S::L, F = S::F, B = S::B, RB = S::RB, NB = S::NB, G = S::G;
     const int lane = threadIdx.x & 31, lig = lane & (L - 1), set = lane / L;
-    const unsigned warp0 = ((blockIdx.x * GA_TPB + threadIdx.x) >> 5) * (G * run_len);  // first nonzero of this warp
+    const unsigned warp0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (G * run_len);  // first nonzero of this warp
     if (warp0 >= nnz) return;
     const unsigned row_bytes = (unsigned)pieces * 16u;
     const char *H_lane = H + lig * 16, *W_lane = W + lig * 16;
@@ -143,6 +147,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
                 for (unsigned o = 0; o < row_bytes; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(wp + o));
             }
         }
+        if (HAS_PERM && sval) s = __ldg(sval + dst);
         float res = 0.f;
 #pragma unroll
         for (int h0 = 0; h0 < NB; h0 += RB) {
@@ -174,12 +179,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
             if (RB == NB || il / RB == h0 / RB) res = t;
         }
         if (lig < NB && j < nnz) {
-            if (HAS_PERM) {
-                if (sval) res *= __ldg(sval + dst);
-                P[dst] = res;
-            } else {
-                P[j] = res * s;
-            }
+            P[HAS_PERM ? (unsigned)dst : j] = res * s;
         }
         j += NB;
         r = rn;
@@ -187,6 +187,8 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
         s = sn;
         dst = dn;
     }
+    // (launched beside the kernel before it: that one is done when this one is)
+    if (HAS_PERM && blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     clock_end(clock);
 }
 
@@ -234,7 +236,8 @@ sddmm_gather_long_kernel(const int32_t *__restrict__ rows, const int32_t *__rest
 
 template <class S, bool HAS_PERM>
 cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                           const void *H, float *P, unsigned nnz, int pieces, int sm_count, unsigned long long *clock, cudaStream_t stream)
+                           const void *H, float *P, unsigned nnz, int pieces, int sm_count, unsigned long long *clock, bool beside,
+                           cudaStream_t stream)
 {
     // only the last piece of a lane is predicated: the ones before it have to lie inside the row
     if (pieces > S::L * S::F || pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
@@ -243,8 +246,21 @@ cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32
     const unsigned resident = (unsigned)sm_count * S::CTAS * (GA_TPB / 32) * S::G;  // sets
     unsigned run = nnz / resident / S::NB * S::NB;
     run = run < (unsigned)S::NB ? (unsigned)S::NB : run > most ? most : run;
-    const unsigned per_block = run * S::G * (GA_TPB / 32);
+    const unsigned tpb = beside ? GA_TPB_BESIDE : GA_TPB, per_block = run * S::G * (tpb / 32);
     const unsigned blocks = (unsigned)(((uint64_t)nnz + per_block - 1) / per_block);
+    if (HAS_PERM && beside) {
+        cudaLaunchAttribute attr = {};
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(tpb);
+        cfg.stream = stream;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, sddmm_gather_kernel<S, HAS_PERM>, rows, cols, perm, sval, static_cast<const char *>(W),
+                                  static_cast<const char *>(H), P, nnz, pieces, run, clock);
+    }
     sddmm_gather_kernel<S, HAS_PERM><<<blocks, GA_TPB, 0, stream>>>(rows, cols, perm, sval, static_cast<const char *>(W),
                                                                     static_cast<const char *>(H), P, nnz, pieces, run, clock);
     return cudaGetLastError();
@@ -252,10 +268,11 @@ cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32
 
 template <class S>
 cudaError_t launch_shape(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                         const void *H, float *P, unsigned nnz, int pieces, int sm_count, unsigned long long *clock, cudaStream_t stream)
+                         const void *H, float *P, unsigned nnz, int pieces, int sm_count, unsigned long long *clock, bool beside,
+                         cudaStream_t stream)
 {
-    return perm ? launch_shape_p<S, true>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, clock, stream)
-                : launch_shape_p<S, false>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, clock, stream);
+    return perm ? launch_shape_p<S, true>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, clock, beside, stream)
+                : launch_shape_p<S, false>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, clock, false, stream);
 }
 
 }  // namespace
@@ -264,7 +281,7 @@ cudaError_t launch_shape(const int32_t *rows, const int32_t *cols, const int32_t
 // are busy and large enough that F pieces of W and B * F of H stay in few registers.  Every line is the best of a sweep
 // over (L, B, RB, prefetch, resident blocks) at a K of its range on the matrices named at the top of this file.
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const float *W,
-                          const float *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream)
+                          const float *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream, bool beside)
 {
     constexpr int64_t SLICE = 1ll << 30;  // the kernels count nonzeros in 32 bits
     for (int64_t j0 = 0; j0 < nnz; j0 += SLICE) {
@@ -275,7 +292,7 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
         const int q = K / 4;
         cudaError_t e;
 #define GA_GO(L, F, B, RB, EXACT, PF, CTAS) \
-    e = launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS>>(r, c, p, s, W, H, out, n, q, sm_count, clock, stream)
+    e = launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS>>(r, c, p, s, W, H, out, n, q, sm_count, clock, beside && j0 == 0, stream)
         if (q <= 4) GA_GO(4, 1, 4, 4, false, false, 6);
         else if (q < 8) GA_GO(8, 1, 4, 4, false, false, 6);
         else if (q == 8) GA_GO(8, 1, 4, 4, true, false, 6);
@@ -319,7 +336,7 @@ cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const i
     if (nnz > INT32_MAX) return cudaErrorInvalidValue;  // plans hold fewer
     const unsigned n = (unsigned)nnz;
 #define GA_GO(L, F, B, PF, CTAS) \
-    return launch_shape<GatherShape<L, F, B, 8, true, PF, CTAS, true>>(rows, cols, perm, sval, W, H, P, n, K / 8, sm_count, clock, stream)
+    return launch_shape<GatherShape<L, F, B, 8, true, PF, CTAS, true>>(rows, cols, perm, sval, W, H, P, n, K / 8, sm_count, clock, false, stream)
     switch (K) {
     case 256: GA_GO(16, 2, 2, false, 5);
     case 512: GA_GO(16, 4, 1, true, 4);

@@ -51,3 +51,29 @@ def test_dense_cells_at_small_sizes(monkeypatch, K, mode, M, half_width, n_globa
         name, info = _run(h, p, rows, c, v)
         assert name.startswith("dense") and info.n_dense_cells > 0
     h.close()
+
+
+@pytest.mark.parametrize("K,half_width,n_global", [(64, 96, 6), (100, 40, 60), (512, 70, 3)])
+def test_remainder_beside_the_cells(engine, K, half_width, n_global):
+    # the remainder runs beside the dense cells: what follows on the stream sees all of P, and the next call overwrites it
+    # only after that
+    import torch
+    p = synth.attention_mask(M=8192, half_width=half_width, n_global=n_global, K=K, device="cuda")
+    plan = engine.plan_coo(p["M"], p["N"], p["rows"], p["cols"], K)
+    info = plan.info()
+    assert 0 < info.n_dense_nnz < info.nnz
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        P = torch.empty(info.nnz, device="cuda")
+        seen = []
+        for _ in range(6):
+            P.fill_(float("nan"))
+            plan.execute(p["W"], p["H"], P, p["vals"], api.FLAG_ASYNC)
+            seen.append(P.clone())
+    stream.synchronize()
+    assert plan.last_kernel_name().startswith("dense_tc+")
+    q = synth.to_numpy(p)
+    assert_parity(seen[0].cpu().numpy(), q["rows"], q["cols"], q["W"], q["H"], q["vals"])
+    assert all(torch.equal(seen[0], s) for s in seen[1:])
+    plan.close()
