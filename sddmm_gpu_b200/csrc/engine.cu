@@ -570,9 +570,10 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     // Locally dense matrices (many nonzeros per row): cells that are at least a
     // quarter full go to the dense-cell kernel, if they hold half of S or more
     // (below that the second launch and the permuted remainder cost more than they save).
-    // Below 2^26 multiplications the gather kernel is as fast or faster, and the plan need not be classified (us per call, band +
-    // global masks, gather / cells: 0.36 M nonzeros, K = 64 11 / 18;  0.9 M, K = 64 17 / 19;  1.1 M, K = 64 21 / 21;  1.9 M, K = 32
-    // 22 / 21;  1.6 M, K = 64 28 / 19;  0.9 M, K = 128 34 / 26;  planned, called and closed: 0.36 M, K = 64 42 / 365).
+    // Below 2^26 multiplications the cells save little or nothing, and the classification costs a plan 300 us that a pattern
+    // of that size, planned for a call or a few, does not earn back (us per call, band + global masks, gather / cells: 0.36 M nonzeros,
+    // K = 64 11 / 12;  0.9 M, K = 32 13 / 13, K = 64 18 / 13;  1.1 M, K = 32 16 / 16, K = 64 22 / 17;  1.6 M, K = 64 28 / 13;
+    // 1.9 M, K = 64 33 / 19;  planned, called and closed: 0.36 M, K = 64 42 / 365).
     // SDDMM_DENSE_CELLS=0 switches the classification off, 1 takes it at every size.
     {
         const char *env = std::getenv("SDDMM_DENSE_CELLS");
