@@ -134,12 +134,17 @@ __device__ __forceinline__ bool epilogue_all(bool mine)
 __device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync 1, 512;" ::: "memory"); }
 
 // A warp waits for a barrier phase: lane 0 polls (32 lanes polling one word cost 32 accesses of the shared-memory
-// pipe per poll), the others take its answer; __shfl_sync orders the warp's memory accesses behind the wait.
+// pipe per poll), the others take its answer; __syncwarp orders the warp's memory accesses behind the wait.  The polling
+// loop is a call: inlined at five places it took instruction cache and registers from the roles (with the vote in place
+// of a shuffle, 65,536-token mask: K = 64 168.5 -> 166, K = 128 245 -> 239.5 us).
+__device__ __noinline__ bool wait_polling(uint64_t *bar, unsigned parity) { return mbar_wait_bounded(bar, parity); }
 __device__ __forceinline__ bool wait_bar(uint64_t *bar, unsigned parity)
 {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = (mbar_try_wait(bar, parity) || mbar_wait_bounded(bar, parity)) ? 1 : 0;
-    return __shfl_sync(FULL, ok, 0) != 0;
+    bool ok = true;
+    if ((threadIdx.x & 31) == 0) ok = mbar_try_wait(bar, parity) || wait_polling(bar, parity);
+    ok = __all_sync(FULL, ok);
+    __syncwarp();
+    return ok;
 }
 
 __global__ void __launch_bounds__(TC_THREADS, 1)
