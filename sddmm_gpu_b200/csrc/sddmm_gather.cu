@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "device_utils.cuh"
+#include "gather_index.hpp"
 
 namespace sddmm {
 
@@ -32,7 +33,7 @@ using namespace dev;
 
 namespace {
 
-constexpr int GA_TPB = 256;
+constexpr int GA_TPB = GATHER_TPB;
 // Launched beside the kernel before it in the stream (the remainder of a matrix with dense cells): the persistent block of the dense-cell
 // kernel leaves an SM 7,900 registers, room for two warps of any shape here (32 to 128 threads measure alike).  65,536-token mask, 0.3 M of
 // 44 M nonzeros left over, K = 64: 180 us after the cells, 168 beside them; 12,777 tokens 37 -> 29.6.
@@ -100,7 +101,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
     clock_begin(clock);
     constexpr int L = S::L, F = S::F, B = S::B, RB = S::RB, NB = S::NB, G = S::G;
     const int lane = threadIdx.x & 31, lig = lane & (L - 1), set = lane / L;
-    const unsigned warp0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (G * run_len);  // first nonzero of this warp
+    const unsigned warp0 = gather_warp(blockIdx.x, blockDim.x, threadIdx.x) * (G * run_len);  // first nonzero of this warp
     if (warp0 >= nnz) return;
     const unsigned row_bytes = (unsigned)pieces * 16u;
     const char *H_lane = H + lig * 16, *W_lane = W + lig * 16;
@@ -202,7 +203,7 @@ sddmm_gather_long_kernel(const int32_t *__restrict__ rows, const int32_t *__rest
     clock_begin(clock);
     constexpr int U = 4;
     const int lane = threadIdx.x & 31;
-    const unsigned j = (blockIdx.x * GA_TPB + threadIdx.x) >> 5;
+    const unsigned j = gather_warp(blockIdx.x, GA_TPB, threadIdx.x);
     if (j >= nnz) return;
     const char *wp = W + (size_t)(unsigned)__ldg(rows + j) * pieces * 16 + lane * 16;
     const char *hp = H + (size_t)(unsigned)__ldg(cols + j) * pieces * 16 + lane * 16;
@@ -283,9 +284,8 @@ cudaError_t launch_shape(const int32_t *rows, const int32_t *cols, const int32_t
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const float *W,
                           const float *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream, bool beside)
 {
-    constexpr int64_t SLICE = 1ll << 30;  // the kernels count nonzeros in 32 bits
-    for (int64_t j0 = 0; j0 < nnz; j0 += SLICE) {
-        const unsigned n = (unsigned)(nnz - j0 < SLICE ? nnz - j0 : SLICE);
+    for (int64_t j0 = 0; j0 < nnz; j0 += GATHER_SLICE) {
+        const unsigned n = (unsigned)(nnz - j0 < GATHER_SLICE ? nnz - j0 : GATHER_SLICE);
         const int32_t *r = rows + j0, *c = cols + j0, *p = perm ? perm + j0 : nullptr;
         const float *s = sval && !perm ? sval + j0 : sval;
         float *out = perm ? P : P + j0;
@@ -314,7 +314,7 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
         else if (q <= 224) GA_GO(32, 7, 1, 8, false, false, 3);
         else if (q <= 256) GA_GO(32, 8, 1, 8, false, false, 3);
         else {
-            const unsigned blocks = (n + GA_TPB / 32 - 1) / (GA_TPB / 32);
+            const unsigned blocks = gather_long_blocks(n);
             if (p) sddmm_gather_long_kernel<true><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock);
             else sddmm_gather_long_kernel<false><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock);
             e = cudaGetLastError();

@@ -61,3 +61,32 @@ def test_kernel_time_of_small_calls(engine):
     assert plans[1][0].last_kernel_ms() == times[1]
     for plan, _, _ in plans:
         plan.close()
+
+
+def _all_of_P(engine, M, N, nnz, K):
+    """A call of nnz nonzeros with small whole-number operands (every product and sum exact): P against W H^T, everywhere.
+    Returns the plan's kernel time and the whole call's, in ms."""
+    g = torch.Generator(device="cuda").manual_seed(nnz % 1009)
+    j = torch.arange(nnz, device="cuda")
+    rows, cols = (j * M // nnz).to(torch.int32), (j % N).to(torch.int32)
+    del j
+    W, H = (torch.randint(-2, 3, (n, K), generator=g, device="cuda").float() for n in (M, N))
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    P = torch.full((nnz,), float("nan"), device="cuda")
+    t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    t0.record()
+    plan.execute(W, H, P)
+    t1.record()
+    torch.cuda.synchronize()
+    ms = plan.last_kernel_ms()
+    plan.close()
+    table = (W.double() @ H.double().T).float()
+    for a in range(0, nnz, 1 << 27):
+        b = min(nnz, a + (1 << 27))
+        assert torch.equal(P[a:b], table[rows[a:b].long(), cols[a:b].long()]), (a, b)
+    return ms, t0.elapsed_time(t1)
+
+
+def test_long_rows_beyond_two_to_the_27_nonzeros(engine):
+    # K > 1024: a warp per nonzero, 2^32 threads at 2^27 nonzeros
+    _all_of_P(engine, 512, 509, (1 << 27) + 12345, 1028)

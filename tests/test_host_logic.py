@@ -340,3 +340,22 @@ def test_host_code_under_address_and_ub_sanitizers(tmp_path):
                          env=dict(os.environ, ASAN_OPTIONS="detect_leaks=1:abort_on_error=0", UBSAN_OPTIONS="print_stacktrace=1"))
     assert run.returncode == 0, run.stdout[-3000:] + run.stderr[-3000:]
     assert "FAILED" not in run.stdout and run.stdout.count("ok:") >= 40
+
+
+def _run_cpp(tmp_path, name, *flags):
+    """tests/c_abi/<name>.cpp, compiled with g++ against csrc/ and run."""
+    import shutil
+    import subprocess
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no compiler")
+    exe = str(tmp_path / name)
+    build = subprocess.run([cxx, "-std=c++17", "-Wall", "-O1", "-I", os.path.join(ROOT, "sddmm_gpu_b200", "csrc"),
+                            os.path.join(ROOT, "tests", "c_abi", name + ".cpp"), "-o", exe, *flags], capture_output=True, text=True)
+    assert build.returncode == 0, build.stderr
+    run = subprocess.run([exe], capture_output=True, text=True)
+    assert run.returncode == 0 and "FAILED" not in run.stdout, run.stdout + run.stderr
+
+
+def test_gather_launch_arithmetic_past_2_to_the_32_threads(tmp_path):
+    _run_cpp(tmp_path, "gather_index")
