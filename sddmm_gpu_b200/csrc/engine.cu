@@ -534,7 +534,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     }
     if (nnz > 0) {
         PLAN_TRY(scan_coo(p->d_rows, p->d_cols, nnz, M, N, h->d_plan_words, h->d_words, s));
-        PLAN_TRY(cudaStreamSynchronize(s));
+        PLAN_TRY(h->pool.wait(s));
         const unsigned long long unsorted = h->h_words[0], oob = h->h_words[1];
         if (!(flags & SDDMM_PLAN_SKIP_VALIDATION) && (unsorted != ULLONG_MAX || oob != ULLONG_MAX)) {
             char buf[160];
@@ -607,13 +607,12 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     }
     if (more) {
         PLAN_TRY(cudaEventRecord(h->ev_plan[1], s));
-        PLAN_TRY(cudaEventSynchronize(h->ev_plan[1]));
+        PLAN_TRY(h->pool.wait(s));
         float ms = 0.f;
         PLAN_TRY(cudaEventElapsedTime(&ms, h->ev_plan[0], h->ev_plan[1]));
         p->plan_ms += ms;
     }
 #undef PLAN_TRY
-    h->pool.settle(s);
     *out = p;
     return SDDMM_OK;
 }

@@ -4,7 +4,7 @@
 // The pool belongs to one handle and is used by one host thread at a time, like the handle.  It keeps at most LIMIT bytes
 // that nobody uses; more go back to CUDA at once, all of it when the handle is destroyed or an allocation fails.  A
 // block given back while work on a stream may still touch it carries that stream and is handed out again only to work
-// on the same stream, until settle() says that the stream has been waited for.
+// on the same stream, until wait() has waited for that stream.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -67,11 +67,14 @@ public:
         kept_ += it->second;
         free_.emplace(it->second, Block{ptr, stream, busy, ++clock_});
     }
-    // the stream has been waited for: what was given back on it is idle
-    void settle(cudaStream_t s)
+    // Waits for the stream; what was given back on it is idle then.
+    cudaError_t wait(cudaStream_t s)
     {
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return e;
         for (auto &f : free_)
             if (f.second.stream == s) f.second.busy = false;
+        return cudaSuccess;
     }
     void release()
     {

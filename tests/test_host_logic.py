@@ -342,6 +342,14 @@ def test_host_code_under_address_and_ub_sanitizers(tmp_path):
     assert "FAILED" not in run.stdout and run.stdout.count("ok:") >= 40
 
 
+def _nvcc():
+    import shutil
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no CUDA toolkit")
+    return os.path.realpath(nvcc)
+
+
 def _run_cpp(tmp_path, name, *flags):
     """tests/c_abi/<name>.cpp, compiled with g++ against csrc/ and run."""
     import shutil
@@ -359,3 +367,8 @@ def _run_cpp(tmp_path, name, *flags):
 
 def test_gather_launch_arithmetic_past_2_to_the_32_threads(tmp_path):
     _run_cpp(tmp_path, "gather_index")
+
+
+def test_memory_pool_hands_out_only_what_has_been_waited_for(tmp_path):
+    nvcc = _nvcc()
+    _run_cpp(tmp_path, "pool", "-I", os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include"))
