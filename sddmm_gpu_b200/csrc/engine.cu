@@ -237,13 +237,40 @@ const char *rows_class_name(const sddmm_plan_s *p, bool panel, bool ring)
     return p->K <= 128 ? "ring_small" : "ring";
 }
 
+// Plan data that is built when a call first needs it.  It is built on the handle's own stream, whose pattern is complete
+// since planning, and waited for: calls of the plan on any stream find it complete.  The calling thread may be capturing a
+// stream meanwhile; allocating and waiting for another stream are allowed then in the relaxed mode only.
+template <class Fn>
+cudaError_t build_now(sddmm_handle_s *h, Fn build)
+{
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    {
+        PoolScope scope(h->pool, h->own_stream);
+        e = build(h->own_stream);
+        const cudaError_t w = h->pool.wait(h->own_stream);  // after an error too: its temporaries have gone back to the pool
+        if (e == cudaSuccess) e = w;
+    }
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    return e;
+}
+
 // Row pointer over all rows (empty rows included).
+cudaError_t build_plan_row_ptr(sddmm_plan_s *p, cudaStream_t s)
+{
+    int64_t *row_ptr = nullptr;
+    cudaError_t e = dev_alloc(p, &row_ptr, (size_t)p->M + 1);
+    if (e != cudaSuccess) return e;
+    e = build_row_ptr(p->d_rows, p->nnz, p->M, row_ptr, s);
+    if (e == cudaSuccess) p->d_row_ptr = row_ptr;
+    else pool_free(row_ptr);
+    return e;
+}
 cudaError_t ensure_row_ptr(sddmm_plan_s *p)
 {
     if (p->d_row_ptr) return cudaSuccess;
-    cudaError_t e = dev_alloc(p, &p->d_row_ptr, (size_t)p->M + 1);
-    if (e == cudaSuccess) e = build_row_ptr(p->d_rows, p->nnz, p->M, p->d_row_ptr, p->h->stream);
-    return e;
+    return build_now(p->h, [&](cudaStream_t s) { return build_plan_row_ptr(p, s); });
 }
 
 // The rows of W (0) or H (1) that are read at all.
@@ -251,14 +278,15 @@ cudaError_t ensure_used_rows(sddmm_plan_s *p)
 {
     if (p->d_used_rows || p->nnz == 0) return cudaSuccess;
     cudaError_t e = ensure_row_ptr(p);
-    if (e == cudaSuccess) e = build_used_row_list(p->d_row_ptr, p->M, &p->d_used_rows, &p->n_used_rows, p->h->stream);
+    if (e != cudaSuccess) return e;
+    e = build_now(p->h, [&](cudaStream_t s) { return build_used_row_list(p->d_row_ptr, p->M, &p->d_used_rows, &p->n_used_rows, s); });
     p->device_bytes += (int64_t)sizeof(int32_t) * p->n_used_rows;
     return e;
 }
 cudaError_t ensure_used_cols(sddmm_plan_s *p)
 {
     if (p->d_used_cols || p->nnz == 0) return cudaSuccess;
-    cudaError_t e = build_used_col_list(p->d_cols, p->nnz, p->N, &p->d_used_cols, &p->n_used_cols, p->h->stream);
+    const cudaError_t e = build_now(p->h, [&](cudaStream_t s) { return build_used_col_list(p->d_cols, p->nnz, p->N, &p->d_used_cols, &p->n_used_cols, s); });
     p->device_bytes += (int64_t)sizeof(int32_t) * p->n_used_cols;
     return e;
 }
@@ -267,11 +295,16 @@ cudaError_t ensure_used_cols(sddmm_plan_s *p)
 cudaError_t ensure_upload_marks(sddmm_plan_s *p, bool rows, bool cols)
 {
     cudaError_t e = rows ? ensure_row_ptr(p) : cudaSuccess;
-    if (e == cudaSuccess && cols && !p->d_col_used) {
-        e = dev_alloc(p, &p->d_col_used, (size_t)p->N);
-        if (e == cudaSuccess) e = mark_used_cols(p->d_cols, p->nnz, p->N, p->d_col_used, p->h->stream);
-    }
-    return e;
+    if (e != cudaSuccess || !cols || p->d_col_used) return e;
+    return build_now(p->h, [&](cudaStream_t s) {
+        unsigned char *used = nullptr;
+        cudaError_t e = dev_alloc(p, &used, (size_t)p->N);
+        if (e != cudaSuccess) return e;
+        e = mark_used_cols(p->d_cols, p->nnz, p->N, used, s);
+        if (e == cudaSuccess) p->d_col_used = used;
+        else pool_free(used);
+        return e;
+    });
 }
 
 // Host-operand pipeline (sddmm_execute with W in host memory): S is cut into chunks of consecutive nonzeros, about 32 MB
@@ -290,8 +323,7 @@ cudaError_t ensure_pipe(sddmm_plan_s *p)
     }
     p->pipe_nnz[chunks] = p->nnz;
     at.v[2 * chunks - 1] = p->nnz - 1;
-    cudaError_t e = pick_values(p->d_rows, at, 2 * chunks, h->d_words, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    const cudaError_t e = build_now(h, [&](cudaStream_t s) { return pick_values(p->d_rows, at, 2 * chunks, h->d_words, s); });
     if (e != cudaSuccess) return e;
     int64_t next_row = 0;  // first row of W no earlier chunk uploads
     for (int i = 0; i < chunks; ++i) {
@@ -310,8 +342,10 @@ cudaError_t ensure_items(sddmm_plan_s *p)
     if (p->n_items >= 0) return cudaSuccess;
     const bool tiled = p->d_perm != nullptr;
     int64_t n = 0;
-    cudaError_t e = build_work_items(tiled ? p->d_rows_t : p->d_rows, tiled ? p->d_cols_t : p->d_cols, p->nnz, p->cfg.panel_rows,
-                                     p->col_tile, p->cfg.item_nnz, &p->d_items, &n, &p->d_item_rows, &p->n_item_rows, p->h->stream);
+    const cudaError_t e = build_now(p->h, [&](cudaStream_t s) {
+        return build_work_items(tiled ? p->d_rows_t : p->d_rows, tiled ? p->d_cols_t : p->d_cols, p->nnz, p->cfg.panel_rows, p->col_tile,
+                                p->cfg.item_nnz, &p->d_items, &n, &p->d_item_rows, &p->n_item_rows, s);
+    });
     if (e != cudaSuccess) return e;
     p->n_items = n;
     p->device_bytes += (int64_t)(sizeof(WorkItem) * (size_t)n + sizeof(int32_t) * (size_t)p->n_item_rows);
@@ -319,20 +353,28 @@ cudaError_t ensure_items(sddmm_plan_s *p)
 }
 
 // Hub-column marks for the ring kernel, when H is too large to live in L2 as a whole.
-cudaError_t ensure_hints(sddmm_plan_s *p)
+cudaError_t build_hints(sddmm_plan_s *p, cudaStream_t s)
 {
-    if (p->hints_built) return cudaSuccess;
     const int64_t row_bytes = (int64_t)p->K * 4;
     if (p->nnz > 0 && rows_path_supports(p->K) && p->hub_budget > 0 && p->N * row_bytes > p->hub_budget) {
-        cudaError_t e = dev_alloc(p, &p->d_cols_hint, (size_t)p->nnz);
-        int thr = 0;
-        if (e == cudaSuccess)
-            e = build_hub_column_hints(p->d_perm ? p->d_cols_t : p->d_cols, p->nnz, p->N, row_bytes, p->hub_budget, p->d_cols_hint,
-                                       &p->n_hub_cols, &thr, p->h->stream);
+        int32_t *marked = nullptr;
+        cudaError_t e = dev_alloc(p, &marked, (size_t)p->nnz);
         if (e != cudaSuccess) return e;
+        int thr = 0;
+        e = build_hub_column_hints(p->d_perm ? p->d_cols_t : p->d_cols, p->nnz, p->N, row_bytes, p->hub_budget, marked, &p->n_hub_cols, &thr, s);
+        if (e != cudaSuccess) {
+            pool_free(marked);
+            return e;
+        }
+        p->d_cols_hint = marked;
     }
     p->hints_built = true;
     return cudaSuccess;
+}
+cudaError_t ensure_hints(sddmm_plan_s *p)
+{
+    if (p->hints_built) return cudaSuccess;
+    return build_now(p->h, [&](cudaStream_t s) { return build_hints(p, s); });
 }
 
 }  // namespace
@@ -582,7 +624,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         p->cells_uncounted = candidate && !always && nnz * K < (1ll << 26);
         if (candidate && !p->cells_uncounted) {
             PLAN_TRY(begin_more());
-            PLAN_TRY(ensure_row_ptr(p));
+            PLAN_TRY(build_plan_row_ptr(p, s));
             PLAN_TRY(build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, nnz, M, N, DENSE_MIN_FILL, DENSE_MIN_SHARE, &p->dense, s));
             if (p->dense.n_cells > 0)
                 p->device_bytes += (int64_t)(sizeof(DenseCell) * p->dense.n_cells + 6 * p->dense.n_dense_nnz + 17 * DENSE_CELL_ROWS * p->dense.n_cells +
@@ -597,7 +639,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         p->hub_budget = budget_mb > 0 ? budget_mb * (1ll << 20) : 0;
         if (ring_preferred(N, K)) {
             PLAN_TRY(begin_more());
-            PLAN_TRY(ensure_hints(p));
+            PLAN_TRY(build_hints(p, s));
         }
     }
     // chunks of the host-operand pipeline; what they need is built by the first call with host operands
@@ -1071,6 +1113,21 @@ int sddmm_check_result(sddmm_plan_t p, const float *W, const float *H, const flo
 
 namespace {
 
+// Partial rows of SpMM and the counters before them, which every call leaves at zero.
+cudaError_t ensure_spmm_scratch(sddmm_plan_s *p)
+{
+    if (p->d_spmm_scratch || p->nnz == 0) return cudaSuccess;
+    return build_now(p->h, [&](cudaStream_t s) {
+        float *scratch = nullptr;
+        cudaError_t e = dev_alloc(p, &scratch, spmm_scratch_floats(p->nnz, p->K, p->h->sm_count));
+        if (e != cudaSuccess) return e;
+        e = cudaMemsetAsync(scratch, 0, sizeof(float) * spmm_counter_floats(p->nnz, p->K, p->h->sm_count), s);
+        if (e == cudaSuccess) p->d_spmm_scratch = scratch;
+        else pool_free(scratch);
+        return e;
+    });
+}
+
 // Y = P H (fused: P = S o (W H^T) on the fly).  Host arrays are staged for the call.
 int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const float *pval, float *P_out, float *Y,
              uint32_t flags)
@@ -1084,10 +1141,8 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     // the class that sddmm_last_kernel_name reports (SDDMM_SPMM_RING=0: never the long-row one)
     bool ring = ring_supports(p->K) && p->nnz >= 65536;
     if (const char *env = std::getenv("SDDMM_SPMM_RING")) ring = ring && std::atoi(env) != 0;
-    if (!p->d_spmm_scratch && p->nnz > 0) {
-        CUDA_TRY(h, dev_alloc(p, &p->d_spmm_scratch, spmm_scratch_floats(p->nnz, p->K, h->sm_count)));
-        CUDA_TRY(h, cudaMemsetAsync(p->d_spmm_scratch, 0, sizeof(float) * spmm_counter_floats(p->nnz, p->K, h->sm_count), h->stream));
-    }
+    CUDA_TRY(h, ensure_row_ptr(p));
+    CUDA_TRY(h, ensure_spmm_scratch(p));
     cudaStream_t s = h->stream;
     CallTmp tmp;
     auto stage_in = [&](int slot, const float *src, size_t count, const float **dst) -> cudaError_t {
@@ -1120,7 +1175,6 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
     CallTimer timer(p, async);
     mark_pending(p, async, s);
-    CUDA_TRY(h, ensure_row_ptr(p));
     CUDA_TRY(h, timer.begin(p->M > 0, s));
     SpmmCall call{p->d_rows, p->d_cols, p->d_row_ptr, dV, fused ? dW : nullptr, dH, dP, dY, p->d_spmm_scratch, p->M, p->nnz, p->K,
                   timer.clk};

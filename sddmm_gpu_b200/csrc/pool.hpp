@@ -111,13 +111,20 @@ private:
 // The pool that pool_alloc / pool_free use on this thread while a PoolScope lives; without one they are cudaMalloc / cudaFree.
 DevicePool *&current_pool();
 struct PoolScope {
-    DevicePool *before;
-    PoolScope(DevicePool &p, cudaStream_t s) : before(current_pool())
+    DevicePool *const before, &pool;
+    const cudaStream_t stream_before;
+    PoolScope(DevicePool &p, cudaStream_t s) : before(current_pool()), pool(p), stream_before(p.stream)
     {
         current_pool() = &p;
         p.stream = s;
     }
-    ~PoolScope() { current_pool() = before; }
+    ~PoolScope()
+    {
+        pool.stream = stream_before;
+        current_pool() = before;
+    }
+    PoolScope(const PoolScope &) = delete;
+    PoolScope &operator=(const PoolScope &) = delete;
 };
 cudaError_t pool_alloc(void **ptr, size_t bytes);
 void pool_free(void *ptr);  // after the last use on the call's stream has been enqueued

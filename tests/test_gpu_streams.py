@@ -1,0 +1,95 @@
+"""Plans used from several streams and under stream capture.
+
+What a plan builds when a call first needs it (row pointer, scratch of SpMM, hub marks, work items) has to be complete for the
+calls that follow on other streams, and may be built while a stream is captured.  Results are compared bit for bit with
+the same calls made one after the other."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import assert_parity, random_coo
+from sddmm_gpu_b200 import api
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(M, N, nnz, K, seed=0):
+    rng = np.random.default_rng(seed)
+    rows, cols = random_coo(rng, M, N, nnz, empty_rows=[0, 7, M - 1], hub_row=5)
+    vals = rng.standard_normal(rows.shape[0]).astype(np.float32)
+    W, H = (rng.standard_normal((n, K)).astype(np.float32) for n in (M, N))
+    return [torch.from_numpy(a).cuda() for a in (rows, cols, vals, W, H)]
+
+
+def _keep_busy():
+    """Work on the current stream that takes some tens of milliseconds."""
+    a = torch.randn(8192, 8192, device="cuda")
+    for _ in range(40):
+        a = a @ a * 1e-4
+    return a
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_first_spmm_on_a_busy_stream_second_on_another(engine, fused):
+    M, N, K = 4000, 3000, 64
+    rows, cols, vals, W, H = _problem(M, N, 200_000, K)
+
+    def call(plan, Y, flags=0):
+        plan.fused(W, H, Y, vals, None, flags) if fused else plan.spmm(H, Y, vals, flags)
+
+    reference = torch.full((M, K), float("nan"), device="cuda")
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    call(plan, reference)
+    plan.close()
+    A, B = torch.cuda.Stream(), torch.cuda.Stream()
+    Y = [torch.full((M, K), float("nan"), device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    with torch.cuda.stream(A):
+        busy = _keep_busy()
+        call(plan, Y[0], api.FLAG_ASYNC)
+    with torch.cuda.stream(B):
+        assert plan.export_row_ptr()[-1] == rows.shape[0]
+    A.synchronize()     # the scratch of the two calls is the plan's
+    with torch.cuda.stream(B):
+        call(plan, Y[1], api.FLAG_ASYNC)
+    torch.cuda.synchronize()
+    assert torch.equal(Y[0], reference) and torch.equal(Y[1], reference)
+    plan.close()
+    del busy
+
+
+@pytest.mark.parametrize("what", ["ring", "panel", "gather", "default", "bf16_ring", "spmm", "fused"])
+def test_first_call_of_a_plan_may_be_captured(engine, what, monkeypatch):
+    monkeypatch.setenv("SDDMM_L2_HUB_MB", "1")     # the ring kernel's hub marks are wanted at this size
+    M, N, K = 3000, 2500, 256
+    rows, cols, vals, W, H = _problem(M, N, 150_000, K)
+    Wb, Hb = W.to(torch.bfloat16), H.to(torch.bfloat16)
+    flags = {"ring": api.FLAG_KERNEL_RING, "panel": api.FLAG_KERNEL_PANEL, "gather": api.FLAG_KERNEL_GATHER, "default": 0,
+             "bf16_ring": api.FLAG_KERNEL_RING | api.FLAG_OPERANDS_BF16}
+
+    def call(plan, out, extra=0):
+        if what == "spmm":
+            plan.spmm(H, out, vals, extra)
+        elif what == "fused":
+            plan.fused(W, H, out, vals, None, extra)
+        else:
+            plan.execute(*((Wb, Hb) if what == "bf16_ring" else (W, H)), out, vals, flags[what] | extra)
+
+    shape = (M, K) if what in ("spmm", "fused") else (rows.shape[0],)
+    expect, out = (torch.full(shape, float("nan"), device="cuda") for _ in range(2))
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    call(plan, expect)
+    plan.close()
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(plan, out, api.FLAG_ASYNC)
+    assert bool(torch.isnan(out).all())            # captured, not run
+    for _ in range(3):
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, expect)
+    del graph
+    plan.close()
