@@ -164,6 +164,9 @@ SDDMM_API int sddmm_execute(sddmm_plan_t p, const float *W, const float *H,
  * nonzeros are cut into equal runs; the parts of a row of S that spans runs are added in run order: the
  * result does not depend on scheduling.  Works on the plan's input order (column tiles of the
  * plan are not used).  sddmm_last_kernel_ms() reports the kernels' time.
+ * The parts lie in scratch that belongs to the plan: calls of one plan on different streams run one after the
+ * other (the engine orders them).  Replays of a captured call are the caller's to order: they must not overlap another call or
+ * replay of the same plan.
  */
 SDDMM_API int sddmm_spmm_execute(sddmm_plan_t p, const float *Pval, const float *H, float *Y, uint32_t flags);
 SDDMM_API int sddmm_fused_execute(sddmm_plan_t p, const float *W, const float *H, const float *Sval,

@@ -665,6 +665,7 @@ int sddmm_destroy_plan(sddmm_plan_t p)
     cudaSetDevice(p->h->device);
     free_plan_memory(p);
     if (p->clock >= 0) p->h->free_clocks.push_back(p->clock);
+    if (p->spmm_done) cudaEventDestroy(p->spmm_done);
     for (sddmm_plan_s *&owner : p->h->ev_owner) if (owner == p) owner = nullptr;
     if (p->h->pipe_owner == p) p->h->pipe_owner = nullptr;
     (void)cudaGetLastError();
@@ -1128,6 +1129,23 @@ cudaError_t ensure_spmm_scratch(sddmm_plan_s *p)
     });
 }
 
+// The scratch is the plan's: a call on another stream starts behind the one before it.  (A captured call does not: what its
+// replays overlap is decided where they are launched.)
+cudaError_t spmm_behind_last(sddmm_plan_s *p, bool captured, cudaStream_t s)
+{
+    return p->spmm_running && !captured && p->spmm_stream != s ? cudaStreamWaitEvent(s, p->spmm_done, 0) : cudaSuccess;
+}
+cudaError_t spmm_enqueued(sddmm_plan_s *p, bool captured, cudaStream_t s)
+{
+    if (captured) return cudaSuccess;
+    cudaError_t e = p->spmm_done ? cudaSuccess : cudaEventCreateWithFlags(&p->spmm_done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(p->spmm_done, s);
+    if (e != cudaSuccess) return e;
+    p->spmm_running = true;
+    p->spmm_stream = s;
+    return cudaSuccess;
+}
+
 // Y = P H (fused: P = S o (W H^T) on the fly).  Host arrays are staged for the call.
 int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const float *pval, float *P_out, float *Y,
              uint32_t flags)
@@ -1141,6 +1159,9 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     // the class that sddmm_last_kernel_name reports (SDDMM_SPMM_RING=0: never the long-row one)
     bool ring = ring_supports(p->K) && p->nnz >= 65536;
     if (const char *env = std::getenv("SDDMM_SPMM_RING")) ring = ring && std::atoi(env) != 0;
+    const bool y_dev = is_device_ptr(Y), p_dev = P_out ? is_device_ptr(P_out) : true;
+    auto on_host = [](const float *a) { return a && !is_device_ptr(a); };
+    if ((flags & SDDMM_FLAG_ASYNC) && (!y_dev || !p_dev || on_host(W) || on_host(H) || on_host(pval))) return SDDMM_INVALID_ARG;
     CUDA_TRY(h, ensure_row_ptr(p));
     CUDA_TRY(h, ensure_spmm_scratch(p));
     cudaStream_t s = h->stream;
@@ -1158,8 +1179,6 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     CUDA_TRY(h, stage_in(1, H, nk, &dH));
     CUDA_TRY(h, stage_in(2, pval, nz, &dV));
     float *dY = Y, *dP = P_out;
-    const bool y_dev = is_device_ptr(Y), p_dev = P_out ? is_device_ptr(P_out) : true;
-    if ((flags & SDDMM_FLAG_ASYNC) && (!y_dev || !p_dev || tmp.p[0] || tmp.p[1] || tmp.p[2])) return SDDMM_INVALID_ARG;
     if (!y_dev) {
         CUDA_TRY(h, pool_alloc(&tmp.p[3], sizeof(float) * (mk ? mk : 1)));
         dY = (float *)tmp.p[3];
@@ -1175,6 +1194,10 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
     CallTimer timer(p, async);
     mark_pending(p, async, s);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (async) CUDA_TRY(h, cudaStreamIsCapturing(s, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    CUDA_TRY(h, spmm_behind_last(p, captured, s));
     CUDA_TRY(h, timer.begin(p->M > 0, s));
     SpmmCall call{p->d_rows, p->d_cols, p->d_row_ptr, dV, fused ? dW : nullptr, dH, dP, dY, p->d_spmm_scratch, p->M, p->nnz, p->K,
                   timer.clk};
@@ -1183,8 +1206,12 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     p->last_kernel = ring ? (fused ? "fused_sddmm_spmm_ring" : "spmm_ring") : (fused ? "fused_sddmm_spmm" : "spmm");
     if (!y_dev) CUDA_TRY(h, cudaMemcpyAsync(Y, dY, sizeof(float) * mk, cudaMemcpyDeviceToHost, s));
     if (P_out && !p_dev) CUDA_TRY(h, cudaMemcpyAsync(P_out, dP, sizeof(float) * nz, cudaMemcpyDeviceToHost, s));
-    if (async) return SDDMM_OK;
+    if (async) {
+        CUDA_TRY(h, spmm_enqueued(p, captured, s));
+        return SDDMM_OK;
+    }
     CUDA_TRY(h, cudaStreamSynchronize(s));
+    p->spmm_running = false;  // (this call was behind all of them)
     waited_for(p, s);
     timer.done();
     return check_device_status(h);

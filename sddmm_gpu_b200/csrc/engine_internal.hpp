@@ -110,6 +110,10 @@ struct sddmm_plan_s {
     bool last_h2d_used_cols = false;                 // and the rows of H of the columns that hold a nonzero (counted on request)
     const char *last_kernel = "none";                // kernels the last sddmm_execute launched
     float *d_spmm_scratch = nullptr;  // partial rows of SpMM / fused SDDMM->SpMM, allocated on first use
+    // end of the last asynchronous call that uses the scratch, while nothing has waited for it, and its stream
+    cudaEvent_t spmm_done = nullptr;
+    bool spmm_running = false;
+    cudaStream_t spmm_stream = nullptr;
 };
 
 

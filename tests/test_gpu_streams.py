@@ -50,7 +50,6 @@ def test_first_spmm_on_a_busy_stream_second_on_another(engine, fused):
         call(plan, Y[0], api.FLAG_ASYNC)
     with torch.cuda.stream(B):
         assert plan.export_row_ptr()[-1] == rows.shape[0]
-    A.synchronize()     # the scratch of the two calls is the plan's
     with torch.cuda.stream(B):
         call(plan, Y[1], api.FLAG_ASYNC)
     torch.cuda.synchronize()
@@ -92,4 +91,31 @@ def test_first_call_of_a_plan_may_be_captured(engine, what, monkeypatch):
         torch.cuda.synchronize()
         assert torch.equal(out, expect)
     del graph
+    plan.close()
+
+
+def test_overlapping_spmm_calls_of_one_plan(engine):
+    """Asynchronous calls alternating over three streams, rows of many partial sums: the scratch and its counters are the
+    plan's, so the calls run one after the other; and the calls after them find the counters at zero."""
+    M, N, K = 3000, 2500, 128
+    rows, cols, vals, W, H = _problem(M, N, 400_000, K, seed=3)
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    expect = [torch.full((M, K), float("nan"), device="cuda") for _ in range(2)]
+    plan.spmm(H, expect[0], vals)
+    plan.fused(W, H, expect[1], vals)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    out = [torch.full((M, K), float("nan"), device="cuda") for _ in range(24)]
+    torch.cuda.synchronize()
+    for i, Y in enumerate(out):
+        with torch.cuda.stream(streams[i % 3]):
+            plan.fused(W, H, Y, vals, None, api.FLAG_ASYNC) if i % 2 else plan.spmm(H, Y, vals, api.FLAG_ASYNC)
+    late = torch.full((M, K), float("nan"), device="cuda")
+    plan.spmm(H, late, vals)                       # waits, behind all of them
+    assert torch.equal(late, expect[0])
+    torch.cuda.synchronize()
+    for i, Y in enumerate(out):
+        assert torch.equal(Y, expect[i % 2]), i
+    with pytest.raises(api.SddmmError) as e:       # host arrays need the call to wait
+        plan.spmm(np.zeros((N, K), np.float32), late, vals, api.FLAG_ASYNC)
+    assert e.value.status == api.INVALID_ARG
     plan.close()
