@@ -1016,6 +1016,8 @@ int sddmm_plan_used_lines(sddmm_plan_t p, int which, const int32_t **d_ids, int6
         *d_ids = p->d_used_cols;
         *n = p->n_used_cols;
     }
+    // whoever reads the list does so on streams that the plan never hears of: destroying it waits for the device
+    p->pending = p->async_pending = p->async_mixed = true;
     return SDDMM_OK;
 }
 

@@ -119,3 +119,36 @@ def test_overlapping_spmm_calls_of_one_plan(engine):
         plan.spmm(np.zeros((N, K), np.float32), late, vals, api.FLAG_ASYNC)
     assert e.value.status == api.INVALID_ARG
     plan.close()
+
+
+def test_plan_destroyed_behind_a_queued_row_upload(engine):
+    """The list of used rows belongs to the plan and is read by uploads on any stream: destroying the plan waits for them, and
+    the memory of the list goes to the next plan only then."""
+    M, N, K = 60000, 500, 32
+    rng = np.random.default_rng(2)
+    rows = np.sort(rng.choice(np.arange(0, M, 2), 40_000)).astype(np.int32)      # odd rows stay empty
+    cols = rng.integers(0, N, rows.size).astype(np.int32)
+    rows_d, cols_d = torch.from_numpy(rows).cuda(), torch.from_numpy(cols).cuda()
+    host = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float32)).pin_memory()
+    dev = torch.zeros((M, K), device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    plan = engine.plan_coo(M, N, rows_d, cols_d, K)
+    ids, n = plan.used_lines(0)
+    with torch.cuda.stream(side):
+        busy = _keep_busy()
+    engine.upload_rows(host, dev, ids, n, K, side.cuda_stream)
+    plan.close()
+    assert side.query()                            # the upload is done, the list was free to go
+    others = []
+    for _ in range(4):                             # plans that take memory of that size and write to it
+        q = engine.plan_coo(M, N, rows_d, cols_d, K)
+        q.used_lines(0)
+        others.append(q)
+    torch.cuda.synchronize()
+    expect = np.zeros((M, K), np.float32)
+    expect[rows] = host.numpy()[rows]
+    assert np.array_equal(dev.cpu().numpy(), expect)
+    for q in others:
+        q.close()
+    del busy
