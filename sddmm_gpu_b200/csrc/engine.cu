@@ -1116,13 +1116,16 @@ int sddmm_check_result(sddmm_plan_t p, const float *W, const float *H, const flo
 
 namespace {
 
-// Partial rows of SpMM and the counters before them, which every call leaves at zero.
-cudaError_t ensure_spmm_scratch(sddmm_plan_s *p)
+// What SpMM needs of the plan: the row pointer, and scratch for partial rows behind their counters, which every call leaves at
+// zero.
+cudaError_t ensure_spmm_data(sddmm_plan_s *p)
 {
-    if (p->d_spmm_scratch || p->nnz == 0) return cudaSuccess;
+    if (p->d_row_ptr && (p->d_spmm_scratch || p->nnz == 0)) return cudaSuccess;
     return build_now(p->h, [&](cudaStream_t s) {
+        cudaError_t e = p->d_row_ptr ? cudaSuccess : build_plan_row_ptr(p, s);
+        if (e != cudaSuccess || p->d_spmm_scratch || p->nnz == 0) return e;
         float *scratch = nullptr;
-        cudaError_t e = dev_alloc(p, &scratch, spmm_scratch_floats(p->nnz, p->K, p->h->sm_count));
+        e = dev_alloc(p, &scratch, spmm_scratch_floats(p->nnz, p->K, p->h->sm_count));
         if (e != cudaSuccess) return e;
         e = cudaMemsetAsync(scratch, 0, sizeof(float) * spmm_counter_floats(p->nnz, p->K, p->h->sm_count), s);
         if (e == cudaSuccess) p->d_spmm_scratch = scratch;
@@ -1131,21 +1134,30 @@ cudaError_t ensure_spmm_scratch(sddmm_plan_s *p)
     });
 }
 
-// The scratch is the plan's: a call on another stream starts behind the one before it.  (A captured call does not: what its
-// replays overlap is decided where they are launched.)
-cudaError_t spmm_behind_last(sddmm_plan_s *p, bool captured, cudaStream_t s)
+// The scratch is the plan's, so a call on another stream starts behind the one before it.  A plan whose calls stay on one
+// stream keeps no event for that (one behind every call costs 2 us of a call of 24): the first change of stream waits for
+// the device, the later ones for the event.  A captured call waits for nothing: what its replays overlap is decided where they
+// are launched.
+cudaError_t spmm_behind_last(sddmm_plan_s *p, cudaStream_t s, bool *captured)
 {
-    return p->spmm_running && !captured && p->spmm_stream != s ? cudaStreamWaitEvent(s, p->spmm_done, 0) : cudaSuccess;
+    *captured = false;
+    if (!p->spmm_running || (p->spmm_stream == s && !p->spmm_event_kept)) return cudaSuccess;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    *captured = capture != cudaStreamCaptureStatusNone;
+    if (e != cudaSuccess || *captured || p->spmm_stream == s) return e;
+    if (p->spmm_event_kept) return cudaStreamWaitEvent(s, p->spmm_done, 0);
+    e = cudaEventCreateWithFlags(&p->spmm_done, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+    p->spmm_event_kept = true;
+    return cudaDeviceSynchronize();
 }
-cudaError_t spmm_enqueued(sddmm_plan_s *p, bool captured, cudaStream_t s)
+cudaError_t spmm_enqueued(sddmm_plan_s *p, cudaStream_t s, bool captured)
 {
     if (captured) return cudaSuccess;
-    cudaError_t e = p->spmm_done ? cudaSuccess : cudaEventCreateWithFlags(&p->spmm_done, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventRecord(p->spmm_done, s);
-    if (e != cudaSuccess) return e;
     p->spmm_running = true;
     p->spmm_stream = s;
-    return cudaSuccess;
+    return p->spmm_event_kept ? cudaEventRecord(p->spmm_done, s) : cudaSuccess;
 }
 
 // Y = P H (fused: P = S o (W H^T) on the fly).  Host arrays are staged for the call.
@@ -1164,8 +1176,7 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     const bool y_dev = is_device_ptr(Y), p_dev = P_out ? is_device_ptr(P_out) : true;
     auto on_host = [](const float *a) { return a && !is_device_ptr(a); };
     if ((flags & SDDMM_FLAG_ASYNC) && (!y_dev || !p_dev || on_host(W) || on_host(H) || on_host(pval))) return SDDMM_INVALID_ARG;
-    CUDA_TRY(h, ensure_row_ptr(p));
-    CUDA_TRY(h, ensure_spmm_scratch(p));
+    CUDA_TRY(h, ensure_spmm_data(p));
     cudaStream_t s = h->stream;
     CallTmp tmp;
     auto stage_in = [&](int slot, const float *src, size_t count, const float **dst) -> cudaError_t {
@@ -1196,10 +1207,8 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
     CallTimer timer(p, async);
     mark_pending(p, async, s);
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (async) CUDA_TRY(h, cudaStreamIsCapturing(s, &capture));
-    const bool captured = capture != cudaStreamCaptureStatusNone;
-    CUDA_TRY(h, spmm_behind_last(p, captured, s));
+    bool captured = false;
+    CUDA_TRY(h, spmm_behind_last(p, s, &captured));
     CUDA_TRY(h, timer.begin(p->M > 0, s));
     SpmmCall call{p->d_rows, p->d_cols, p->d_row_ptr, dV, fused ? dW : nullptr, dH, dP, dY, p->d_spmm_scratch, p->M, p->nnz, p->K,
                   timer.clk};
@@ -1209,7 +1218,7 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     if (!y_dev) CUDA_TRY(h, cudaMemcpyAsync(Y, dY, sizeof(float) * mk, cudaMemcpyDeviceToHost, s));
     if (P_out && !p_dev) CUDA_TRY(h, cudaMemcpyAsync(P_out, dP, sizeof(float) * nz, cudaMemcpyDeviceToHost, s));
     if (async) {
-        CUDA_TRY(h, spmm_enqueued(p, captured, s));
+        CUDA_TRY(h, spmm_enqueued(p, s, captured));
         return SDDMM_OK;
     }
     CUDA_TRY(h, cudaStreamSynchronize(s));

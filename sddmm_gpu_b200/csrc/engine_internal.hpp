@@ -110,10 +110,11 @@ struct sddmm_plan_s {
     bool last_h2d_used_cols = false;                 // and the rows of H of the columns that hold a nonzero (counted on request)
     const char *last_kernel = "none";                // kernels the last sddmm_execute launched
     float *d_spmm_scratch = nullptr;  // partial rows of SpMM / fused SDDMM->SpMM, allocated on first use
-    // end of the last asynchronous call that uses the scratch, while nothing has waited for it, and its stream
-    cudaEvent_t spmm_done = nullptr;
-    bool spmm_running = false;
+    // An asynchronous call that uses the scratch and that nothing has waited for: its stream, and once a plan's calls have been
+    // seen on more than one stream (spmm_event_kept) the event at its end.
+    bool spmm_running = false, spmm_event_kept = false;
     cudaStream_t spmm_stream = nullptr;
+    cudaEvent_t spmm_done = nullptr;
 };
 
 
