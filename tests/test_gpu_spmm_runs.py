@@ -53,3 +53,32 @@ def test_run_boundaries(engine, K):
         plan.fused(W, H, Y2, vals)
         assert np.array_equal(Y, Y2)
     plan.close()
+
+
+@pytest.mark.parametrize("K", [4, 32, 36, 64, 96, 100, 128, 192, 252, 256, 384, 512, 640, 1024])
+def test_last_nonzero_infinite(engine, K):
+    # positive operands: the last row is +Inf everywhere, all other rows are finite; the matrix ends inside a step of every
+    # shape, and inside a warp's last sets
+    rng = np.random.default_rng(K)
+    M, N = 40, 50
+    for nnz in (1, 3, 5, 121, 1001):
+        cells = np.sort(rng.choice((M - 1) * N, nnz - 1, replace=False))
+        rows, cols = np.append(cells // N, M - 1).astype(np.int32), np.append(cells % N, 3).astype(np.int32)
+        W, H = rng.random((M, K), dtype=np.float32) + 1, rng.random((N, K), dtype=np.float32) + 1
+        vals = rng.random(nnz, dtype=np.float32) + 1
+        infinite = vals.copy()
+        infinite[-1] = np.inf
+        W_inf = W.copy()
+        W_inf[-1, K // 2] = np.inf
+        plan = engine.plan_coo(M, N, rows, cols, K)
+        for call, weights in ((lambda Y: plan.spmm(H, Y, infinite), vals),
+                              (lambda Y: plan.fused(W, H, Y, infinite), None), (lambda Y: plan.fused(W_inf, H, Y, vals), None)):
+            Y = np.full((M, K), np.nan, np.float32)
+            call(Y)
+            assert np.all(Y[-1] == np.inf)
+            if weights is None:
+                weights = oracle.cpu.sddmm_coo_f64(rows, cols, W, H, vals)[0].astype(np.float32)
+            ref, A = oracle.cpu.spmm_f64(rows[:-1], cols[:-1], H, M, weights[:-1])
+            # all terms are positive: an error of 1e-4 in each weight is one of 1e-4 in the sum
+            assert np.all(np.abs(Y[:-1] - ref[:-1]) <= 2 * TOL * A[:-1])
+        plan.close()
