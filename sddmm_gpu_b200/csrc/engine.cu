@@ -269,7 +269,11 @@ cudaError_t build_plan_row_ptr(sddmm_plan_s *p, cudaStream_t s)
 }
 cudaError_t ensure_row_ptr(sddmm_plan_s *p)
 {
-    if (p->d_row_ptr) return cudaSuccess;
+    if (p->d_row_ptr) {
+        const cudaError_t e = p->row_ptr_unwaited ? cudaDeviceSynchronize() : cudaSuccess;
+        if (e == cudaSuccess) p->row_ptr_unwaited = false;
+        return e;
+    }
     return build_now(p->h, [&](cudaStream_t s) { return build_plan_row_ptr(p, s); });
 }
 
@@ -1117,21 +1121,31 @@ int sddmm_check_result(sddmm_plan_t p, const float *W, const float *H, const flo
 namespace {
 
 // What SpMM needs of the plan: the row pointer, and scratch for partial rows behind their counters, which every call leaves at
-// zero.
-cudaError_t ensure_spmm_data(sddmm_plan_s *p)
+// zero.  Enqueued in front of the first call, as part of it: what orders the later calls behind that one (spmm_behind_last)
+// orders them behind this too, and a pattern that is planned for one call does not wait for it (20 us of 65).  Under capture it is
+// built at once.
+cudaError_t ensure_spmm_data(sddmm_plan_s *p, cudaStream_t s)
 {
     if (p->d_row_ptr && (p->d_spmm_scratch || p->nnz == 0)) return cudaSuccess;
-    return build_now(p->h, [&](cudaStream_t s) {
-        cudaError_t e = p->d_row_ptr ? cudaSuccess : build_plan_row_ptr(p, s);
+    auto build = [&](cudaStream_t on) {
+        cudaError_t e = p->d_row_ptr ? cudaSuccess : build_plan_row_ptr(p, on);
         if (e != cudaSuccess || p->d_spmm_scratch || p->nnz == 0) return e;
         float *scratch = nullptr;
         e = dev_alloc(p, &scratch, spmm_scratch_floats(p->nnz, p->K, p->h->sm_count));
         if (e != cudaSuccess) return e;
-        e = cudaMemsetAsync(scratch, 0, sizeof(float) * spmm_counter_floats(p->nnz, p->K, p->h->sm_count), s);
+        e = cudaMemsetAsync(scratch, 0, sizeof(float) * spmm_counter_floats(p->nnz, p->K, p->h->sm_count), on);
         if (e == cudaSuccess) p->d_spmm_scratch = scratch;
         else pool_free(scratch);
         return e;
-    });
+    };
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    if (e != cudaSuccess) return e;
+    if (capture != cudaStreamCaptureStatusNone) return build_now(p->h, build);
+    p->row_ptr_unwaited = p->row_ptr_unwaited || !p->d_row_ptr;
+    p->spmm_running = true;
+    p->spmm_stream = s;
+    return build(s);
 }
 
 // The scratch is the plan's, so a call on another stream starts behind the one before it.  A plan whose calls stay on one
@@ -1141,11 +1155,12 @@ cudaError_t ensure_spmm_data(sddmm_plan_s *p)
 cudaError_t spmm_behind_last(sddmm_plan_s *p, cudaStream_t s, bool *captured)
 {
     *captured = false;
-    if (!p->spmm_running || (p->spmm_stream == s && !p->spmm_event_kept)) return cudaSuccess;
+    const bool other = p->spmm_running && p->spmm_stream != s;
+    if (!other && !p->spmm_event_kept) return cudaSuccess;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(s, &capture);
-    *captured = capture != cudaStreamCaptureStatusNone;
-    if (e != cudaSuccess || *captured || p->spmm_stream == s) return e;
+    *captured = capture != cudaStreamCaptureStatusNone;  // (an event recorded under capture could not be waited for)
+    if (e != cudaSuccess || *captured || !other) return e;
     if (p->spmm_event_kept) return cudaStreamWaitEvent(s, p->spmm_done, 0);
     e = cudaEventCreateWithFlags(&p->spmm_done, cudaEventDisableTiming);
     if (e != cudaSuccess) return e;
@@ -1176,8 +1191,12 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     const bool y_dev = is_device_ptr(Y), p_dev = P_out ? is_device_ptr(P_out) : true;
     auto on_host = [](const float *a) { return a && !is_device_ptr(a); };
     if ((flags & SDDMM_FLAG_ASYNC) && (!y_dev || !p_dev || on_host(W) || on_host(H) || on_host(pval))) return SDDMM_INVALID_ARG;
-    CUDA_TRY(h, ensure_spmm_data(p));
+    const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
     cudaStream_t s = h->stream;
+    mark_pending(p, async, s);
+    bool captured = false;
+    CUDA_TRY(h, spmm_behind_last(p, s, &captured));
+    CUDA_TRY(h, ensure_spmm_data(p, s));
     CallTmp tmp;
     auto stage_in = [&](int slot, const float *src, size_t count, const float **dst) -> cudaError_t {
         if (!src || is_device_ptr(src)) { *dst = src; return cudaSuccess; }
@@ -1204,11 +1223,7 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
         h->last_error = "W, H and Y must be 16-byte aligned on the device";
         return SDDMM_INVALID_ARG;
     }
-    const bool async = (flags & SDDMM_FLAG_ASYNC) != 0;
     CallTimer timer(p, async);
-    mark_pending(p, async, s);
-    bool captured = false;
-    CUDA_TRY(h, spmm_behind_last(p, s, &captured));
     CUDA_TRY(h, timer.begin(p->M > 0, s));
     SpmmCall call{p->d_rows, p->d_cols, p->d_row_ptr, dV, fused ? dW : nullptr, dH, dP, dY, p->d_spmm_scratch, p->M, p->nnz, p->K,
                   timer.clk};
@@ -1222,7 +1237,7 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
         return SDDMM_OK;
     }
     CUDA_TRY(h, cudaStreamSynchronize(s));
-    p->spmm_running = false;  // (this call was behind all of them)
+    p->spmm_running = p->row_ptr_unwaited = false;  // (this call was behind all of them)
     waited_for(p, s);
     timer.done();
     return check_device_status(h);

@@ -113,6 +113,7 @@ struct sddmm_plan_s {
     // An asynchronous call that uses the scratch and that nothing has waited for: its stream, and once a plan's calls have been
     // seen on more than one stream (spmm_event_kept) the event at its end.
     bool spmm_running = false, spmm_event_kept = false;
+    bool row_ptr_unwaited = false;  // d_row_ptr was enqueued by such a call
     cudaStream_t spmm_stream = nullptr;
     cudaEvent_t spmm_done = nullptr;
 };

@@ -115,6 +115,19 @@ def test_overlapping_spmm_calls_of_one_plan(engine):
     torch.cuda.synchronize()
     for i, Y in enumerate(out):
         assert torch.equal(Y, expect[i % 2]), i
+    # a captured call between them, and its replays in order with the others
+    graph, Y = torch.cuda.CUDAGraph(), torch.full((M, K), float("nan"), device="cuda")
+    with torch.cuda.graph(graph):
+        plan.spmm(H, Y, vals, api.FLAG_ASYNC)
+    for i in range(4):
+        Y.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(Y, expect[0])
+        with torch.cuda.stream(streams[i % 3]):
+            plan.fused(W, H, out[i], vals, None, api.FLAG_ASYNC)
+        torch.cuda.synchronize()
+        assert torch.equal(out[i], expect[1])
     with pytest.raises(api.SddmmError) as e:       # host arrays need the call to wait
         plan.spmm(np.zeros((N, K), np.float32), late, vals, api.FLAG_ASYNC)
     assert e.value.status == api.INVALID_ARG
