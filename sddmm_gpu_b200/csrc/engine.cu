@@ -107,7 +107,7 @@ void mark_pending(sddmm_plan_s *p, bool async, cudaStream_t s)
 void waited_for(sddmm_plan_s *p, cudaStream_t s)
 {
     if (p->async_mixed || (p->async_pending && p->async_stream != s)) return;
-    p->pending = p->async_pending = false;
+    p->pending = p->async_pending = p->setup_unwaited = false;
 }
 
 // Gives the plan's memory back to the handle's pool.  Work that was enqueued and not waited for may still use it: wait
@@ -267,13 +267,17 @@ cudaError_t build_plan_row_ptr(sddmm_plan_s *p, cudaStream_t s)
     else pool_free(row_ptr);
     return e;
 }
+// Set-up that a call enqueued in front of itself, and that nothing has waited for since, has to be complete for another call.
+cudaError_t wait_for_setup(sddmm_plan_s *p)
+{
+    if (!p->setup_unwaited) return cudaSuccess;
+    const cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) p->setup_unwaited = false;
+    return e;
+}
 cudaError_t ensure_row_ptr(sddmm_plan_s *p)
 {
-    if (p->d_row_ptr) {
-        const cudaError_t e = p->row_ptr_unwaited ? cudaDeviceSynchronize() : cudaSuccess;
-        if (e == cudaSuccess) p->row_ptr_unwaited = false;
-        return e;
-    }
+    if (p->d_row_ptr) return wait_for_setup(p);
     return build_now(p->h, [&](cudaStream_t s) { return build_plan_row_ptr(p, s); });
 }
 
@@ -295,20 +299,25 @@ cudaError_t ensure_used_cols(sddmm_plan_s *p)
     return e;
 }
 
-// What the upload of used rows looks at: the row pointer and a mark per column.
-cudaError_t ensure_upload_marks(sddmm_plan_s *p, bool rows, bool cols)
+// What the upload of used rows looks at: the row pointer and a mark per column.  Enqueued in front of the call, which waits
+// for all of it.
+cudaError_t ensure_upload_marks(sddmm_plan_s *p, bool rows, bool cols, cudaStream_t s)
 {
-    cudaError_t e = rows ? ensure_row_ptr(p) : cudaSuccess;
-    if (e != cudaSuccess || !cols || p->d_col_used) return e;
-    return build_now(p->h, [&](cudaStream_t s) {
-        unsigned char *used = nullptr;
-        cudaError_t e = dev_alloc(p, &used, (size_t)p->N);
-        if (e != cudaSuccess) return e;
-        e = mark_used_cols(p->d_cols, p->nnz, p->N, used, s);
-        if (e == cudaSuccess) p->d_col_used = used;
-        else pool_free(used);
-        return e;
-    });
+    cudaError_t e = wait_for_setup(p);
+    rows = rows && !p->d_row_ptr;
+    cols = cols && !p->d_col_used;
+    if (e != cudaSuccess || (!rows && !cols)) return e;
+    p->setup_unwaited = true;
+    mark_pending(p, true, s);
+    if (rows) e = build_plan_row_ptr(p, s);
+    if (e != cudaSuccess || !cols) return e;
+    unsigned char *used = nullptr;
+    e = dev_alloc(p, &used, (size_t)p->N);
+    if (e != cudaSuccess) return e;
+    e = mark_used_cols(p->d_cols, p->nnz, p->N, used, s);
+    if (e == cudaSuccess) p->d_col_used = used;
+    else pool_free(used);
+    return e;
 }
 
 // Host-operand pipeline (sddmm_execute with W in host memory): S is cut into chunks of consecutive nonzeros, about 32 MB
@@ -760,7 +769,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     }
     const float *S_mapped = h->sparse_upload && Sval && !s_dev ? mapped_host_ptr(Sval) : nullptr;
     const bool used_rows_only = p->K >= 32;
-    if (used_rows_only) CUDA_TRY(h, ensure_upload_marks(p, W_mapped != nullptr, H_mapped != nullptr));
+    if (used_rows_only) CUDA_TRY(h, ensure_upload_marks(p, W_mapped != nullptr, H_mapped != nullptr, s));
     UploadRows up_w, up_h;
     up_w.row_bytes = up_h.row_bytes = p->K * (int)sizeof(float);
     const float *up_s = nullptr;
@@ -1142,7 +1151,8 @@ cudaError_t ensure_spmm_data(sddmm_plan_s *p, cudaStream_t s)
     const cudaError_t e = cudaStreamIsCapturing(s, &capture);
     if (e != cudaSuccess) return e;
     if (capture != cudaStreamCaptureStatusNone) return build_now(p->h, build);
-    p->row_ptr_unwaited = p->row_ptr_unwaited || !p->d_row_ptr;
+    p->setup_unwaited = p->setup_unwaited || !p->d_row_ptr;
+    mark_pending(p, true, s);
     p->spmm_running = true;
     p->spmm_stream = s;
     return build(s);
@@ -1237,7 +1247,7 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
         return SDDMM_OK;
     }
     CUDA_TRY(h, cudaStreamSynchronize(s));
-    p->spmm_running = p->row_ptr_unwaited = false;  // (this call was behind all of them)
+    p->spmm_running = false;  // (this call was behind all of them)
     waited_for(p, s);
     timer.done();
     return check_device_status(h);

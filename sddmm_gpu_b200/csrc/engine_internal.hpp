@@ -103,6 +103,7 @@ struct sddmm_plan_s {
     int64_t pipe_nnz[SDDMM_PIPE_MAX_CHUNKS + 1] = {};
     // rows of W chunk i uploads: [pipe_w_begin[i], pipe_w_end[i]) (empty when an earlier chunk brought them)
     int64_t pipe_w_begin[SDDMM_PIPE_MAX_CHUNKS] = {}, pipe_w_end[SDDMM_PIPE_MAX_CHUNKS] = {};
+    bool setup_unwaited = false;  // the row pointer or the marks were enqueued by a call that nothing has waited for
     unsigned char *d_col_used = nullptr;  // marks of the columns that hold a nonzero (row upload of H)
     int32_t *d_used_rows = nullptr, *d_used_cols = nullptr;  // ascending ids of the rows / columns holding a nonzero
     int64_t n_used_rows = 0, n_used_cols = 0;
@@ -113,7 +114,6 @@ struct sddmm_plan_s {
     // An asynchronous call that uses the scratch and that nothing has waited for: its stream, and once a plan's calls have been
     // seen on more than one stream (spmm_event_kept) the event at its end.
     bool spmm_running = false, spmm_event_kept = false;
-    bool row_ptr_unwaited = false;  // d_row_ptr was enqueued by such a call
     cudaStream_t spmm_stream = nullptr;
     cudaEvent_t spmm_done = nullptr;
 };
