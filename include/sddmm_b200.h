@@ -62,7 +62,7 @@ enum {
                                           (HiPC18/src/sddmm.cu:32) */
 
 /* ---- plan flags ---------------------------------------------------------- */
-#define SDDMM_PLAN_SKIP_VALIDATION 0x1u /* trust sortedness and bounds (the reference checks neither) */
+#define SDDMM_PLAN_SKIP_VALIDATION 0x1u /* trust sortedness and bounds (the reference checks neither).  sddmm_execute() works on nonzeros in any order; what goes by whole rows of S (SpMM, the fused form, the row pointer, the used rows) answers SDDMM_UNSORTED_INPUT for unsorted ones */
 #define SDDMM_PLAN_DEVICE_INDICES  0x2u /* rows/cols are device pointers on the handle's device */
 #define SDDMM_PLAN_FORCE_H_CHUNKS  0x4u /* sddmm_dist_plan_coo: build and use the column-bucketed form even with a single rank (exercises the overlapped execute on one GPU; the broadcasts are no-ops) */
 

@@ -74,6 +74,13 @@ const float *mapped_host_ptr(const float *p, unsigned align = 16)
     return static_cast<const float *>(a.devicePointer);
 }
 
+// Behind SDDMM_PLAN_SKIP_VALIDATION: what works on whole rows has no row pointer to go by.
+int needs_sorted(sddmm_handle_s *h)
+{
+    h->last_error = "the plan's nonzeros are not sorted by row";
+    return SDDMM_UNSORTED_INPUT;
+}
+
 int check_k(int K)
 {
     if (K <= 0 || (K % 4) != 0 || K > SDDMM_MAX_K) return SDDMM_K_UNSUPPORTED;
@@ -598,6 +605,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
             h->last_error = buf;
             return drop(oob != ULLONG_MAX ? SDDMM_INDEX_OUT_OF_RANGE : SDDMM_UNSORTED_INPUT);
         }
+        p->sorted = unsorted == ULLONG_MAX;
         p->n_nonempty_rows = (int64_t)h->h_words[2];
         p->plan_ms = (float)((double)h->h_words[3] * 1e-6);
     }
@@ -633,7 +641,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     {
         const char *env = std::getenv("SDDMM_DENSE_CELLS");
         const bool enabled = !(env && std::atoi(env) == 0), always = env && std::atoi(env) == 1;
-        const bool candidate = enabled && p->n_col_tiles == 1 && p->n_nonempty_rows > 0 && nnz / p->n_nonempty_rows >= 32;
+        const bool candidate = enabled && p->sorted && p->n_col_tiles == 1 && p->n_nonempty_rows > 0 && nnz / p->n_nonempty_rows >= 32;
         p->cells_uncounted = candidate && !always && nnz * K < (1ll << 26);
         if (candidate && !p->cells_uncounted) {
             PLAN_TRY(begin_more());
@@ -656,7 +664,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         }
     }
     // chunks of the host-operand pipeline; what they need is built by the first call with host operands
-    if (p->n_col_tiles == 1 && p->dense.n_cells == 0 && nnz >= (1 << 17)) {
+    if (p->sorted && p->n_col_tiles == 1 && p->dense.n_cells == 0 && nnz >= (1 << 17)) {
         const int64_t chunks = std::min<int64_t>((int64_t)sizeof(float) * M * K / (32ll << 20), SDDMM_PIPE_MAX_CHUNKS);
         if (chunks >= 2) p->n_pipe = (int)chunks;
     }
@@ -756,7 +764,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (pipelined) CUDA_TRY(h, ensure_pipe(p));
     // page-locked, mapped host arrays are read by the GPU: one launch for all of them instead of a copy each, and of W and
     // H only the rows that a nonzero touches travel (short rows all do: reads below 128 bytes waste the link)
-    const float *W_mapped = h->sparse_upload && !w_dev && !w_t ? mapped_host_ptr(W) : nullptr;
+    const float *W_mapped = h->sparse_upload && p->sorted && !w_dev && !w_t ? mapped_host_ptr(W) : nullptr;
     const float *H_mapped = h->sparse_upload && !h_dev && !h_t ? mapped_host_ptr(H) : nullptr;
     // a large array with nearly all rows used: the copy engine moves whole arrays at 56 GB/s, the kernel rows at 45 to 50
     constexpr size_t LARGE = 4 << 20;
@@ -1018,6 +1026,7 @@ int sddmm_plan_used_lines(sddmm_plan_t p, int which, const int32_t **d_ids, int6
     *d_ids = nullptr;
     *n = 0;
     if (p->nnz == 0) return SDDMM_OK;
+    if (which == 0 && !p->sorted) return needs_sorted(h);
     CUDA_TRY(h, cudaSetDevice(h->device));
     PoolScope scope(h->pool, h->stream);
     if (which == 0) {
@@ -1193,6 +1202,7 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     if (!spmm_supports(p->K)) return SDDMM_K_UNSUPPORTED;
     if (!H || !Y || (fused && !W)) return SDDMM_INVALID_ARG;
     if (flags & ~(uint32_t)SDDMM_FLAG_ASYNC) return SDDMM_INVALID_ARG;
+    if (!p->sorted) return needs_sorted(h);
     CUDA_TRY(h, cudaSetDevice(h->device));
     PoolScope scope(h->pool, h->stream);
     // the class that sddmm_last_kernel_name reports (SDDMM_SPMM_RING=0: never the long-row one)
@@ -1392,6 +1402,7 @@ int sddmm_plan_export_row_ptr(sddmm_plan_t p, int64_t *row_ptr)
 {
     if (!p || !row_ptr) return SDDMM_INVALID_ARG;
     sddmm_handle_s *h = p->h;
+    if (!p->sorted) return needs_sorted(h);
     CUDA_TRY(h, cudaSetDevice(h->device));
     PoolScope scope(h->pool, h->stream);
     CUDA_TRY(h, ensure_row_ptr(p));

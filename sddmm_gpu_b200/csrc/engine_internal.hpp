@@ -63,6 +63,7 @@ struct sddmm_plan_s {
     sddmm_handle_s *h = nullptr;
     int64_t M = 0, N = 0, nnz = 0;
     int K = 0;
+    bool sorted = true;   // by row; false only behind SDDMM_PLAN_SKIP_VALIDATION, and then nothing may look at the row pointer
     int col_tile = 0;     // == N (clamped) when there is a single column tile
     int n_col_tiles = 1;
     PanelConfig cfg{};

@@ -77,3 +77,33 @@ def test_remainder_beside_the_cells(engine, K, half_width, n_global):
     assert_parity(seen[0].cpu().numpy(), q["rows"], q["cols"], q["W"], q["H"], q["vals"])
     assert all(torch.equal(seen[0], s) for s in seen[1:])
     plan.close()
+
+
+@pytest.mark.parametrize("where", ["pageable", "pinned", "device"])
+def test_unsorted_rows_behind_skipped_validation(engine, where, monkeypatch):
+    # blocks of full rows in descending order, long rows and enough work for dense cells: only sddmm_execute, which looks at a
+    # nonzero at a time, takes them, and goes by no row pointer
+    import torch
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")
+    M, N, K = 700, 300, 64
+    rng = np.random.default_rng(4)
+    rows = np.repeat(np.arange(M - 1, -1, -1), 200).astype(np.int32)
+    cols = np.concatenate([np.sort(rng.choice(N, 200, replace=False)) for _ in range(M)]).astype(np.int32)
+    vals = rng.standard_normal(rows.size).astype(np.float32)
+    W, H = (rng.standard_normal((n, K)).astype(np.float32) for n in (M, N))
+    plan = engine.plan_coo(M, N, rows, cols, K, flags=api.PLAN_SKIP_VALIDATION)
+    P = np.full(rows.size, np.nan, np.float32)
+    args = [torch.from_numpy(a) for a in (W, H, P, vals)]
+    if where == "pinned":
+        args = [a.pin_memory() for a in args]
+    elif where == "device":
+        args = [a.cuda() for a in args]
+    plan.execute(*args)
+    assert_parity(args[2].cpu().numpy(), rows, cols, W, H, vals)
+    Y = np.zeros((M, K), np.float32)
+    for refused in (lambda: plan.spmm(H, Y, vals), lambda: plan.fused(W, H, Y, vals), lambda: plan.used_lines(0), plan.export_row_ptr):
+        with pytest.raises(api.SddmmError) as e:
+            refused()
+        assert e.value.status == api.UNSORTED_INPUT
+    assert plan.used_lines(1)[1] == np.unique(cols).size
+    plan.close()
