@@ -653,12 +653,14 @@ def main():
         plan.execute(l_W, H, P, l_vals, kflag | api.FLAG_ASYNC)
     barrier()
     evs = [torch.cuda.Event(enable_timing=True) for _ in range(args.steps + 1)]
+    launches_timed = handle.kernel_launches()
     with ClockSampler(local_rank) as clocks:
         evs[0].record()
         for i in range(args.steps):
             plan.execute(l_W, H, P, l_vals, kflag | api.FLAG_ASYNC)
             evs[i + 1].record()
         barrier()
+    launches_timed = handle.kernel_launches() - launches_timed
     step_ms = [evs[i].elapsed_time(evs[i + 1]) for i in range(args.steps)]
     total_ms = evs[0].elapsed_time(evs[-1])
     t = torch.tensor([total_ms], device=device, dtype=torch.float64)
@@ -672,7 +674,7 @@ def main():
     ms_per_step = total_ms_max / args.steps
     value = 2.0 * nnz * K / (ms_per_step * 1e-3) / 1e9
 
-    kernel_name = plan.last_kernel_name()   # what actually ran: ring, ring_small, panel, gather, dense_*+...
+    kernel_name = plan.last_kernel_name()   # what actually ran: gather, ring, panel, dense_*[+...]
     # ---- roofline of the dominant kernel (this rank's launch) -------------------
     peak, peak_kind = hbm_peak()
     alg_bytes = synth.algorithmic_bytes(row_end - row_begin, b - a, K, m_nz_local, n_nz_local)
@@ -850,11 +852,10 @@ def main():
                        "dense_cells": info.n_dense_cells, "dense_cell_nnz": info.n_dense_nnz,
                        "hub_columns": info.n_hub_cols},
             "roofline": roofline, "cpu_baseline": cpu_baseline, "e2e": e2e, "parity": parity, "h_broadcast": bcast,
-            # counted by the library: kernels launched by sddmm_execute / sddmm_upload_rows on this rank from the
-            # first warm-up step to the end of the end-to-end steps (timed steps: one SDDMM kernel each, two when
-            # the plan split S into dense cells and a remainder)
+            # counted by the library: kernels launched by sddmm_execute / sddmm_upload_rows on this rank, from the
+            # first warm-up step to the end of the end-to-end steps, and within the timed steps
             "gpu_launches": launches_main,
-            "gpu_launches_timed_steps": args.steps * (2 if (info.n_dense_cells > 0 and args.kernel == "auto") else 1),
+            "gpu_launches_timed_steps": launches_timed,
             "clocks": clocks.summary(),
         }
         if also is not None:

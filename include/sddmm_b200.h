@@ -179,12 +179,10 @@ SDDMM_API int sddmm_fused_execute(sddmm_plan_t p, const float *W, const float *H
  * uploads between them are not counted. */
 SDDMM_API int sddmm_last_kernel_ms(sddmm_plan_t p, float *ms);
 
-/* Which path the last sddmm_execute() on this plan took (static storage): "ring" (K = 256, 512,
- * 1024), "ring_small" (K = 32, 64, 128), "panel" (any other K, or fewer than 65,536 nonzeros), "htile" (K = 128, 256, 512 and few columns),
- * "dense_tc+ring_small", ... by default; "ring", "ring_small", "panel" or "gather" when forced by a flag.
- * The names stand for classes of K and size, not for kernel functions: by default the row classes run on the
- * gather kernel, and on the rings where H is far larger than L2.  The reference has one
- * kernel, comp_kernel_COO (HiPC18/src/kernel.h:2), and nothing to report. */
+/* The kernels that the last call on this plan launched (static storage): "gather", "ring", "panel";
+ * "dense_tc", "dense_mma_sync" or "dense_fma" where dense cells hold all of S, with "+gather" or "+ring" behind it where
+ * nonzeros remain; " (bf16 operands)" or " (pipelined chunks)" behind the name; "spmm", "fused_sddmm_spmm".
+ * "none" before the first call.  The reference has one kernel, comp_kernel_COO (HiPC18/src/kernel.h:2), and nothing to report. */
 SDDMM_API const char *sddmm_last_kernel_name(sddmm_plan_t p);
 
 /* Number of kernels sddmm_execute() and sddmm_upload_rows() have launched through this
@@ -272,15 +270,15 @@ typedef struct {
     int32_t panel_rows;     /* rows of W per staged panel actually used        */
     int32_t col_tile;       /* column-tile width actually used (N if single)   */
     int32_t n_col_tiles;
-    int64_t n_work_items;
+    int64_t n_work_items;   /* of the row-panel kernel: 0 until a call has forced it */
     int64_t n_nonempty_rows;
     int64_t n_nonempty_cols; /* -1 unless computed (sddmm_plan_count_cols)     */
     int64_t device_bytes;   /* device memory the plan owns                     */
     float plan_ms;          /* device time of the binning pass                 */
     int32_t reserved0;
-    int64_t n_dense_cells;  /* 128 x 64 cells that are dense enough for the dense-cell kernel; calls use it if nnz * K >= 2^26 */
+    int64_t n_dense_cells;  /* 128 x 64 cells handed to the dense-cell kernel (none below nnz * K = 2^26) */
     int64_t n_dense_nnz;    /* nonzeros inside them                            */
-    int64_t n_hub_cols;     /* columns marked for L2 residency (ring kernel)   */
+    int64_t n_hub_cols;     /* columns marked for L2 residency: 0 unless the ring kernel runs by default or a call has forced it */
 } sddmm_plan_info;
 SDDMM_API int sddmm_plan_get_info(sddmm_plan_t p, sddmm_plan_info *info);
 

@@ -230,20 +230,6 @@ int check_device_status(sddmm_handle_s *h)
     return SDDMM_OK;
 }
 
-// What sddmm_last_kernel_name reports for a call on the row path: the class of its K and size.  The names are part of the
-// interface and outlived the kernels they were taken from; "panel" by default means K outside the list of
-// SDDMM_FLAG_KERNEL_RING or fewer than 65,536 nonzeros.
-const char *rows_class_name(const sddmm_plan_s *p, bool panel, bool ring)
-{
-    if (panel || !rows_path_supports(p->K) || (!ring && p->nnz < 65536)) return "panel";
-    if (!ring && p->n_col_tiles == 1 && (p->K == 128 || p->K == 256 || p->K == 512)) {
-        // few columns and many nonzeros per column: H is at most 64 blocks of 192 KB, a block has 8 nonzeros per row and SM
-        const int64_t block = 196608 / (p->K * 4);
-        if ((p->N + block - 1) / block <= 64 && p->nnz / p->h->sm_count >= 8 * block) return "htile";
-    }
-    return p->K <= 128 ? "ring_small" : "ring";
-}
-
 // Plan data that is built when a call first needs it.  It is built on the handle's own stream, whose pattern is complete
 // since planning, and waited for: calls of the plan on any stream find it complete.  The calling thread may be capturing a
 // stream meanwhile; allocating and waiting for another stream are allowed then in the relaxed mode only.
@@ -376,7 +362,7 @@ cudaError_t ensure_items(sddmm_plan_s *p)
 cudaError_t build_hints(sddmm_plan_s *p, cudaStream_t s)
 {
     const int64_t row_bytes = (int64_t)p->K * 4;
-    if (p->nnz > 0 && rows_path_supports(p->K) && p->hub_budget > 0 && p->N * row_bytes > p->hub_budget) {
+    if (p->nnz > 0 && ring_supports(p->K) && p->hub_budget > 0 && p->N * row_bytes > p->hub_budget) {
         int32_t *marked = nullptr;
         cudaError_t e = dev_alloc(p, &marked, (size_t)p->nnz);
         if (e != cudaSuccess) return e;
@@ -401,6 +387,11 @@ cudaError_t ensure_hints(sddmm_plan_s *p)
 
 namespace sddmm {
 
+bool rows_on_ring(const sddmm_plan_s *p, bool force_ring)
+{
+    return ring_supports(p->K) && (force_ring || ring_preferred(p->N, p->K));
+}
+
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
                         unsigned long long *clock, cudaStream_t stream, bool beside)
@@ -414,7 +405,7 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
         P += first;
         if (sval) sval += first;
     }
-    if (ring_supports(p->K) && (force_ring || ring_preferred(p->N, p->K))) {
+    if (rows_on_ring(p, force_ring)) {
         // the marks are in the plan's processing order: not for the dense-cell remainder
         const bool hinted = p->d_cols_hint && cols == (p->d_perm ? p->d_cols_t : p->d_cols);
         return launch_ring(rows, (hinted ? p->d_cols_hint : cols) + first, perm, sval, W, H, P, count, p->K, hinted, h->sm_count,
@@ -642,8 +633,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         const char *env = std::getenv("SDDMM_DENSE_CELLS");
         const bool enabled = !(env && std::atoi(env) == 0), always = env && std::atoi(env) == 1;
         const bool candidate = enabled && p->sorted && p->n_col_tiles == 1 && p->n_nonempty_rows > 0 && nnz / p->n_nonempty_rows >= 32;
-        p->cells_uncounted = candidate && !always && nnz * K < (1ll << 26);
-        if (candidate && !p->cells_uncounted) {
+        if (candidate && (always || nnz * K >= (1ll << 26))) {
             PLAN_TRY(begin_more());
             PLAN_TRY(build_plan_row_ptr(p, s));
             PLAN_TRY(build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, nnz, M, N, DENSE_MIN_FILL, DENSE_MIN_SHARE, &p->dense, s));
@@ -736,7 +726,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         // rows of half the bytes: the same line between the two kernels as for fp32 rows of K / 2
         const bool gather = gather_bf16_supports(p->K) && !(flags & SDDMM_FLAG_KERNEL_RING) && !ring_preferred(p->N / 2, p->K);
         if (!gather) CUDA_TRY(h, ensure_hints(p));
-        p->last_kernel = "ring (bf16 operands)";
+        p->last_kernel = gather ? "gather (bf16 operands)" : "ring (bf16 operands)";
         p->last_h2d_bytes = p->last_d2h_bytes = 0;
         CallTimer timer(p, async);
         CUDA_TRY(h, timer.begin(gather, s));
@@ -845,8 +835,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     }
     const bool use_dense = !forced && !tiled_out && p->dense.n_cells > 0;
     // a call that is one gather launch is timed by the kernel itself, everything else by events
-    const bool one_gather = !use_dense && !use_panel &&
-                            !(ring_supports(p->K) && (use_ring || (!use_gather && ring_preferred(p->N, p->K))));
+    const bool one_gather = !use_dense && !use_panel && (use_gather || !rows_on_ring(p, use_ring));
     bool p_copy = false;
     if (!p_dev) {
         // a small P is written to mapped host memory by the kernel: its 32-byte stores over PCIe cost less than a copy
@@ -865,9 +854,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (use_panel) CUDA_TRY(h, ensure_items(p));
     if (use_ring && ring_supports(p->K)) CUDA_TRY(h, ensure_hints(p));
     if (pipelined) {
-        p->last_kernel = !rows_path_supports(p->K) ? "panel (pipelined chunks)"
-                         : p->K <= 128             ? "ring_small (pipelined chunks)"
-                                                   : "ring (pipelined chunks)";
+        p->last_kernel = rows_on_ring(p, use_ring) ? "ring (pipelined chunks)" : "gather (pipelined chunks)";
         CUDA_TRY(h, ensure_pipeline(h));
         if (h->pipe_owner && h->pipe_owner != p && h->pipe_owner->ms_state == sddmm_plan_s::MS_IN_PIPE)
             CUDA_TRY(h, resolve_ms(h->pipe_owner));
@@ -915,11 +902,10 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (use_dense) {
         // locally dense plan: dense cells as small dense products, the rest gathered
         {
-            static const char *const names[3][4] = {
-                {"dense_fma", "dense_fma+panel", "dense_fma+ring_small", "dense_fma+ring"},
-                {"dense_mma_sync", "dense_mma_sync+panel", "dense_mma_sync+ring_small", "dense_mma_sync+ring"},
-                {"dense_tc", "dense_tc+panel", "dense_tc+ring_small", "dense_tc+ring"}};
-            p->last_kernel = names[h->dense_mode][p->dense.n_sparse == 0 ? 0 : !rows_path_supports(p->K) ? 1 : p->K <= 128 ? 2 : 3];
+            static const char *const names[3][3] = {{"dense_fma", "dense_fma+gather", "dense_fma+ring"},
+                                                    {"dense_mma_sync", "dense_mma_sync+gather", "dense_mma_sync+ring"},
+                                                    {"dense_tc", "dense_tc+gather", "dense_tc+ring"}};
+            p->last_kernel = names[h->dense_mode][p->dense.n_sparse == 0 ? 0 : rows_on_ring(p, false) ? 2 : 1];
         }
         if (h->dense_mode == 2)
             LAUNCH_TRY(h, launch_dense_cells_tc(p->dense.cells, p->dense.n_cells, p->dense.idx, p->dense.rc, p->dense.row_mask,
@@ -951,7 +937,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             h->last_error = "SDDMM_FLAG_TILED_ORDER with S values is not supported on a multi-tile plan";
             return SDDMM_INVALID_ARG;
         }
-        p->last_kernel = rows_class_name(p, use_panel, use_ring);
+        p->last_kernel = use_panel ? "panel" : rows_on_ring(p, use_ring) ? "ring" : "gather";
         if (use_panel)
             LAUNCH_TRY(h, launch_panel(p->d_items, p->n_items, p->d_item_rows, rows_p, cols_p, perm, dS, dW, dH, dP, p->K,
                                      p->cfg, h->sm_count, h->d_status, s));
@@ -1205,9 +1191,6 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
     if (!p->sorted) return needs_sorted(h);
     CUDA_TRY(h, cudaSetDevice(h->device));
     PoolScope scope(h->pool, h->stream);
-    // the class that sddmm_last_kernel_name reports (SDDMM_SPMM_RING=0: never the long-row one)
-    bool ring = ring_supports(p->K) && p->nnz >= 65536;
-    if (const char *env = std::getenv("SDDMM_SPMM_RING")) ring = ring && std::atoi(env) != 0;
     const bool y_dev = is_device_ptr(Y), p_dev = P_out ? is_device_ptr(P_out) : true;
     auto on_host = [](const float *a) { return a && !is_device_ptr(a); };
     if ((flags & SDDMM_FLAG_ASYNC) && (!y_dev || !p_dev || on_host(W) || on_host(H) || on_host(pval))) return SDDMM_INVALID_ARG;
@@ -1249,7 +1232,7 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
                   timer.clk};
     CUDA_TRY(h, launch_spmm(call, h->sm_count, &h->n_launches, s));
     CUDA_TRY(h, timer.end(s));
-    p->last_kernel = ring ? (fused ? "fused_sddmm_spmm_ring" : "spmm_ring") : (fused ? "fused_sddmm_spmm" : "spmm");
+    p->last_kernel = fused ? "fused_sddmm_spmm" : "spmm";
     if (!y_dev) CUDA_TRY(h, cudaMemcpyAsync(Y, dY, sizeof(float) * mk, cudaMemcpyDeviceToHost, s));
     if (P_out && !p_dev) CUDA_TRY(h, cudaMemcpyAsync(P_out, dP, sizeof(float) * nz, cudaMemcpyDeviceToHost, s));
     if (async) {
@@ -1354,31 +1337,17 @@ int sddmm_selftest_wait_timeout(sddmm_handle_t h)
 int sddmm_plan_get_info(sddmm_plan_t p, sddmm_plan_info *info)
 {
     if (!p || !info) return SDDMM_INVALID_ARG;
-    CUDA_TRY(p->h, cudaSetDevice(p->h->device));
-    PoolScope scope(p->h->pool, p->h->stream);
-    CUDA_TRY(p->h, ensure_items(p));
-    CUDA_TRY(p->h, ensure_hints(p));
-    if (p->cells_uncounted) {  // cells that no call uses: only counted
-        DensePlan cells;
-        CUDA_TRY(p->h, ensure_row_ptr(p));
-        const cudaError_t e = build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, p->nnz, p->M, p->N, DENSE_MIN_FILL, DENSE_MIN_SHARE, &cells, p->h->stream);
-        p->counted_cells = cells.n_cells;
-        p->counted_cell_nnz = cells.n_dense_nnz;
-        cells.release();
-        CUDA_TRY(p->h, e);
-        p->cells_uncounted = false;
-    }
     info->M = p->M; info->N = p->N; info->nnz = p->nnz; info->K = p->K;
     info->panel_rows = p->cfg.panel_rows;
     info->col_tile = p->col_tile;
     info->n_col_tiles = p->n_col_tiles;
-    info->n_work_items = p->n_items;
+    info->n_work_items = p->n_items < 0 ? 0 : p->n_items;
     info->n_nonempty_rows = p->n_nonempty_rows;
     info->n_nonempty_cols = p->n_nonempty_cols;
     info->device_bytes = p->device_bytes;
     info->plan_ms = p->plan_ms;
-    info->n_dense_cells = p->dense.n_cells + p->counted_cells;
-    info->n_dense_nnz = p->dense.n_dense_nnz + p->counted_cell_nnz;
+    info->n_dense_cells = p->dense.n_cells;
+    info->n_dense_nnz = p->dense.n_dense_nnz;
     info->n_hub_cols = p->n_hub_cols;
     return SDDMM_OK;
 }

@@ -81,8 +81,6 @@ struct sddmm_plan_s {
     bool hints_built = false;
     // dense cells + row-sorted remainder (single-tile plans of locally dense matrices)
     DensePlan dense;
-    bool cells_uncounted = false;  // too little work for them: the cells are counted when the plan's info is asked for
-    int64_t counted_cells = 0, counted_cell_nnz = 0;
     int64_t n_hub_cols = 0;
     int64_t n_item_rows = 0;
     int64_t n_nonempty_rows = 0, n_nonempty_cols = -1;
@@ -123,8 +121,10 @@ struct sddmm_plan_s {
 namespace sddmm {
 constexpr int N_KERNEL_CLOCKS = 1024;
 
-// SDDMM over nonzeros in the plan's processing order, [first, first + count): the ring kernel when it is the faster one
-// for this plan (or forced), else the gather kernel (beside: see launch_gather).
+// Whether launch_rows takes the ring kernel: it is the faster one for this plan, or forced.
+bool rows_on_ring(const sddmm_plan_s *p, bool force_ring);
+// SDDMM over nonzeros in the plan's processing order, [first, first + count): the ring kernel (rows_on_ring) or the gather
+// kernel (beside: see launch_gather).
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
                         unsigned long long *clock, cudaStream_t stream, bool beside = false);

@@ -28,8 +28,14 @@ def run_plan(engine, M, N, rows, cols, W, H, vals=None, flags=0, panel_rows=0, c
     P = np.full(rows.shape[0], np.nan, np.float32)
     plan.execute(W, H, P, vals, flags)
     info = plan.info()
+    info.kernel = plan.last_kernel_name()
     plan.close()
     return P, info
+
+
+def ran_by(kernel, K):
+    """What a forced kernel's name is for this K: the ring flag stands for the row path, whose rings take long rows only."""
+    return "gather" if kernel == "ring" and K not in LONG_ROW_K else kernel
 
 
 def test_hand_computable(engine):
@@ -58,7 +64,8 @@ def test_every_k(engine, kernel, K):
     vals = rng.standard_normal(rows.shape[0]).astype(np.float32)
     W = rng.standard_normal((M, K)).astype(np.float32)
     H = rng.standard_normal((N, K)).astype(np.float32)
-    P, _ = run_plan(engine, M, N, rows, cols, W, H, vals, KERNELS[kernel])
+    P, info = run_plan(engine, M, N, rows, cols, W, H, vals, KERNELS[kernel])
+    assert info.kernel == ran_by(kernel, K)
     assert_parity(P, rows, cols, W, H, vals)
     P, _ = run_plan(engine, M, N, rows, cols, W, H, None, KERNELS[kernel])
     assert_parity(P, rows, cols, W, H, None)
@@ -67,7 +74,7 @@ def test_every_k(engine, kernel, K):
 @pytest.mark.parametrize("kernel", list(KERNELS))
 def test_structure_edge_cases(engine, kernel):
     rng = np.random.default_rng(7)
-    K = 128 if kernel == "ring" else 32
+    K = 256 if kernel == "ring" else 32
     flag = KERNELS[kernel]
     cases = []
     # nnz = 1, M = 1, N = 1, max column index, one row holding everything
@@ -85,6 +92,7 @@ def test_structure_edge_cases(engine, kernel):
         W = rng.random((M, K), dtype=np.float32)
         H = rng.random((N, K), dtype=np.float32)
         P, info = run_plan(engine, M, N, rows, cols, W, H, None, flag)
+        assert info.kernel == kernel
         assert_parity(P, rows, cols, W, H)
         assert info.n_nonempty_rows == np.unique(rows).size
 
@@ -208,7 +216,7 @@ def test_calls_follow_torch_current_stream_without_manual_sync():
         ref = oracle.cpu.sddmm_coo(q["rows"], q["cols"], q["W"], q["H"], q["vals"])
         assert_parity(P.cpu().numpy(), q["rows"], q["cols"], q["W"], q["H"], q["vals"])
         assert abs(got_total - float(ref.astype(np.float64).sum())) <= 1e-3 * float(np.abs(ref).sum())
-        assert plan.last_kernel_name() == "ring"
+        assert plan.last_kernel_name() == "gather"
         # the device-side float64 self-check agrees, and notices a damaged result
         worst, n, bad = plan.check_result(p["W"], p["H"], P, p["vals"])
         assert n == rows.shape[0] and bad == 0 and worst <= 1e-4
@@ -243,7 +251,7 @@ def test_benchmark_configs(engine, name, kernel):
     P, info = run_plan(engine, p["M"], p["N"], p["rows"], p["cols"], p["W"], p["H"], p["vals"], KERNELS[kernel],
                        p["panel_rows"], p["col_tile"])
     assert_parity(P, p["rows"], p["cols"], p["W"], p["H"], p["vals"])
-    assert info.nnz == p["rows"].shape[0]
+    assert info.nnz == p["rows"].shape[0] and info.kernel == ran_by(kernel, p["K"])
 
 
 @pytest.mark.parametrize("K", LONG_ROW_K)
@@ -259,7 +267,8 @@ def test_long_row_ring_shapes(engine, K):
         W = rng.standard_normal((M, K)).astype(np.float32)
         H = rng.standard_normal((N, K)).astype(np.float32)
         for sv in (vals, None):
-            P, _ = run_plan(engine, M, N, rows, cols, W, H, sv, KERNELS["ring"], 0, col_tile)
+            P, info = run_plan(engine, M, N, rows, cols, W, H, sv, KERNELS["ring"], 0, col_tile)
+            assert info.kernel == "ring"
             assert_parity(P, rows, cols, W, H, sv)
 
 
@@ -364,7 +373,7 @@ def test_cli_prints_reference_lines_and_matches_oracle(tmp_path):
         assert res.returncode == 0, res.stderr
         import json
         rep = json.load(open(tmp_path / "r.json"))
-        assert rep["kernel"] == "panel" and rep["gpus"] == 1 and rep["host_cores"] >= 1   # 3000 nonzeros: the panel kernel
+        assert rep["kernel"] == "gather" and rep["gpus"] == 1 and rep["host_cores"] >= 1
         assert rep["check"]["ran"] and rep["check"]["n"] == rows.shape[0] and rep["check"]["bad"] == 0
         assert rep["check"]["max_scaled_err"] <= 1e-4
         n_cols_used = np.unique(cols).size
@@ -414,20 +423,23 @@ def test_cli_prints_reference_lines_and_matches_oracle(tmp_path):
 # ---- dense cells: locally dense matrices split into dense blocks + gathered remainder ----
 
 @pytest.mark.parametrize("K", [16, 64, 100, 256])
-def test_dense_cell_path(engine, K):
+def test_dense_cell_path(engine, K, monkeypatch):
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")     # below the size from which cells are taken by default
     p = synth.to_numpy(synth.attention_mask(M=1100, half_width=96, n_global=7, K=K, device="cpu"))
     rng = np.random.default_rng(K)
     vals = rng.standard_normal(p["rows"].shape[0]).astype(np.float32)
     for sv in (vals, None):
         P, info = run_plan(engine, p["M"], p["N"], p["rows"], p["cols"], p["W"], p["H"], sv, 0)
-        assert info.n_dense_cells > 0 and 0 < info.n_dense_nnz <= info.nnz
+        assert info.n_dense_cells > 0 and 0 < info.n_dense_nnz <= info.nnz and info.kernel.startswith("dense_tc")
         assert_parity(P, p["rows"], p["cols"], p["W"], p["H"], sv)
     # a forced kernel bypasses the split and must agree
-    P2, _ = run_plan(engine, p["M"], p["N"], p["rows"], p["cols"], p["W"], p["H"], vals, api.FLAG_KERNEL_GATHER)
+    P2, info = run_plan(engine, p["M"], p["N"], p["rows"], p["cols"], p["W"], p["H"], vals, api.FLAG_KERNEL_GATHER)
+    assert info.kernel == "gather"
     assert_parity(P2, p["rows"], p["cols"], p["W"], p["H"], vals)
 
 
-def test_dense_cells_cover_everything_or_nothing(engine):
+def test_dense_cells_cover_everything_or_nothing(engine, monkeypatch):
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")
     # fully dense small matrix: the full cells are dense, the thin edge cells fall to the remainder
     M, N, K = 200, 130, 32
     rows = np.repeat(np.arange(M), N).astype(np.int32)
@@ -436,14 +448,14 @@ def test_dense_cells_cover_everything_or_nothing(engine):
     W = rng.standard_normal((M, K)).astype(np.float32)
     H = rng.standard_normal((N, K)).astype(np.float32)
     P, info = run_plan(engine, M, N, rows, cols, W, H, None, 0)
-    assert info.n_dense_cells >= 2 and 128 * 128 <= info.n_dense_nnz < rows.shape[0]
+    assert info.n_dense_cells >= 2 and 128 * 128 <= info.n_dense_nnz < rows.shape[0] and info.kernel == "dense_tc+gather"
     assert_parity(P, rows, cols, W, H)
     # sparse matrix with long rows but no dense cell: classification declines
     rows, cols = random_coo(rng, 64, 60000, 64 * 40)
     W = rng.standard_normal((64, K)).astype(np.float32)
     H = rng.standard_normal((60000, K)).astype(np.float32)
     P, info = run_plan(engine, 64, 60000, rows, cols, W, H, None, 0)
-    assert info.n_dense_cells == 0
+    assert info.n_dense_cells == 0 and info.kernel == "gather"
     assert_parity(P, rows, cols, W, H)
 
 
@@ -455,24 +467,21 @@ def test_benchmark_configs_default_path(engine, name):
     assert_parity(P, p["rows"], p["cols"], p["W"], p["H"], p["vals"])
 
 
-@pytest.mark.parametrize("runs", ["0", "1"])
 @pytest.mark.parametrize("K", [16, 36, 64])
-def test_dense_cell_forms(engine, K, runs, monkeypatch):
-    # K <= 64: the general form of the tcgen05 dense-cell kernel and the one that keeps a row block's W tile in shared
-    # memory across consecutive cells, on a band + global rows / columns mask (compacted and regular cells, runs of
-    # several cells and of one)
-    monkeypatch.setenv("SDDMM_DENSE_RUNS", runs)
+def test_dense_cell_classes(engine, K, monkeypatch):
+    # compacted and regular cells of a band + global rows / columns mask
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")
     p = _scaled(synth.attention_mask, M=4096, half_width=96, n_global=20, K=K)
     P, info = run_plan(engine, p["M"], p["N"], p["rows"], p["cols"], p["W"], p["H"], p["vals"], 0)
-    assert info.n_dense_nnz > 0
+    assert info.n_dense_nnz > 0 and info.kernel == "dense_tc+gather"
     assert_parity(P, p["rows"], p["cols"], p["W"], p["H"], p["vals"])
 
 
 @pytest.mark.parametrize("K", [128, 256, 512])
 @pytest.mark.parametrize("N", [150, 777, 1500])
-def test_column_tile_kernel(engine, K, N, monkeypatch):
-    # few columns, many nonzeros per column: tiles of H in shared memory (one tile, a ragged last tile, eight tiles
-    # at K = 256); the dense-cell split is switched off so that the 42 % dense case takes this path as well
+def test_few_columns(engine, K, N, monkeypatch):
+    # few columns, many nonzeros per column; the dense-cell split is switched off so that the 42 % dense case takes the row
+    # path as well
     monkeypatch.setenv("SDDMM_DENSE_CELLS", "0")
     rng = np.random.default_rng(K + N)
     M = 8000
@@ -483,11 +492,11 @@ def test_column_tile_kernel(engine, K, N, monkeypatch):
     plan = engine.plan_coo(M, N, rows, cols, K)
     P = np.full(rows.shape[0], np.nan, np.float32)
     plan.execute(W, H, P, vals, 0)
-    assert plan.last_kernel_name() == "htile"
+    assert plan.last_kernel_name() == "gather"
     assert_parity(P, rows, cols, W, H, vals)
     P2 = np.full(rows.shape[0], np.nan, np.float32)
-    plan.execute(W, H, P2, None, api.FLAG_KERNEL_RING)    # the forced ring kernel on the same plan, S = 1
-    assert plan.last_kernel_name().startswith("ring")
+    plan.execute(W, H, P2, None, api.FLAG_KERNEL_RING)    # the row path forced on the same plan, S = 1
+    assert plan.last_kernel_name() == ran_by("ring", K)
     assert_parity(P2, rows, cols, W, H, None)
     plan.close()
 
@@ -508,7 +517,7 @@ def test_bounded_wait_reports_timeout_and_handle_survives(engine):
 
 # ---- hub-column L2 hints (bit 31 of the plan's column copy) --------------------
 
-@pytest.mark.parametrize("K", [32, 128, 256, 1024])
+@pytest.mark.parametrize("K", LONG_ROW_K)
 def test_hub_column_hints_do_not_change_results(engine, K, monkeypatch):
     # force the marks on a small matrix (the default only marks when H exceeds 64 MB): results must be
     # those of the unmarked plan bit for bit, and the oracle's within tolerance
@@ -517,9 +526,8 @@ def test_hub_column_hints_do_not_change_results(engine, K, monkeypatch):
     P0, info0 = run_plan(engine, p["M"], p["N"], p["rows"], p["cols"], p["W"], p["H"], p["vals"], api.FLAG_KERNEL_RING)
     monkeypatch.setenv("SDDMM_L2_HUB_MB", "1")
     P1, info1 = run_plan(engine, p["M"], p["N"], p["rows"], p["cols"], p["W"], p["H"], p["vals"], api.FLAG_KERNEL_RING)
-    assert info0.n_hub_cols == 0
-    if p["N"] * K * 4 > (1 << 20):
-        assert info1.n_hub_cols > 0
+    assert info0.kernel == info1.kernel == "ring"
+    assert info0.n_hub_cols == 0 and info1.n_hub_cols > 0
     assert np.array_equal(P0, P1)
     assert_parity(P1, p["rows"], p["cols"], p["W"], p["H"], p["vals"])
 
@@ -546,9 +554,12 @@ def test_bf16_operand_storage(engine, K):
         for sv in (vals, None):
             P = torch.full((rows.shape[0],), float("nan"), device="cuda")
             dS = None if sv is None else torch.from_numpy(sv).cuda()
-            plan.execute(W16, H16, P, dS, api.FLAG_OPERANDS_BF16)
-            assert plan.last_kernel_name() == "ring (bf16 operands)"
-            assert_parity(P.cpu().numpy(), rows, cols, Wr, Hr, sv)
+            # (the ring flag by itself is for K of the fp32 row path; 2048 is on the rings anyway)
+            for flag, name in ((0, "gather"), (api.FLAG_KERNEL_RING, "ring")) if K <= 1024 else ((0, "ring"),):
+                P.fill_(float("nan"))
+                plan.execute(W16, H16, P, dS, api.FLAG_OPERANDS_BF16 | flag)
+                assert plan.last_kernel_name() == name + " (bf16 operands)"
+                assert_parity(P.cpu().numpy(), rows, cols, Wr, Hr, sv)
         plan.close()
     # other K, host arrays or a second kernel flag are refused
     plan = engine.plan_coo(M, N, rows, cols, 128)
@@ -655,20 +666,21 @@ def test_gpu_coo_sort_equals_host_sort(engine, transpose):
     assert np.array_equal(vd.cpu().numpy(), ref[4])
 
 
-def test_dense_cells_with_columns_unsorted_inside_rows(engine):
+def test_dense_cells_with_columns_unsorted_inside_rows(engine, monkeypatch):
     # row-sorted input whose columns are shuffled inside every row: dense cells cannot use their row-mask
     # form (a row's nonzeros are not in column order) and take the per-nonzero lists; results must not change
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")
     p = synth.to_numpy(synth.attention_mask(M=900, half_width=80, n_global=5, K=64, device="cpu"))
     rng = np.random.default_rng(5)
     rows, cols = p["rows"].copy(), p["cols"].copy()
     vals = rng.standard_normal(rows.shape[0]).astype(np.float32)
     P_sorted, info = run_plan(engine, p["M"], p["N"], rows, cols, p["W"], p["H"], vals)
-    assert info.n_dense_cells > 0
+    assert info.n_dense_cells > 0 and info.kernel.startswith("dense_tc")
     order = np.lexsort((rng.random(rows.shape[0]), rows))                    # random order inside each row
     r2, c2, v2 = rows[order], cols[order], vals[order]
     assert np.array_equal(r2, rows) and not np.array_equal(c2, cols)
     P_shuffled, info2 = run_plan(engine, p["M"], p["N"], r2, c2, p["W"], p["H"], v2)
-    assert info2.n_dense_cells > 0
+    assert info2.n_dense_cells > 0 and info2.kernel.startswith("dense_tc")
     assert_parity(P_shuffled, r2, c2, p["W"], p["H"], v2)
     inv = np.empty_like(order)
     inv[order] = np.arange(order.size)
@@ -712,6 +724,7 @@ def test_transposed_operands(engine, K):
 def test_dense_cell_variants(monkeypatch, K, mode):
     # 2 = tcgen05 / tensor memory (the default), 1 = mma.sync, 0 = fp32 FMA
     monkeypatch.setenv("SDDMM_DENSE_TENSOR", mode)
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")
     h = api.Handle(0)
     p = synth.to_numpy(synth.attention_mask(M=1100, half_width=96, n_global=7, K=K, device="cpu"))
     rng = np.random.default_rng(K)
@@ -719,6 +732,7 @@ def test_dense_cell_variants(monkeypatch, K, mode):
     for sv in (vals, None):
         P, info = run_plan(h, p["M"], p["N"], p["rows"], p["cols"], p["W"], p["H"], sv, 0)
         assert info.n_dense_cells > 0 and 0 < info.n_dense_nnz <= info.nnz
+        assert info.kernel.startswith({"2": "dense_tc", "1": "dense_mma_sync", "0": "dense_fma"}[mode])
         assert_parity(P, p["rows"], p["cols"], p["W"], p["H"], sv)
     # a plan reused for several calls: tensor memory is allocated and released by every launch
     plan = h.plan_coo(p["M"], p["N"], p["rows"], p["cols"], K)

@@ -60,11 +60,9 @@ def test_spmm_and_fused_every_k(engine, K):
 
 
 @pytest.mark.parametrize("K", [256, 512, 1024])
-def test_ring_form_for_long_rows(engine, K, monkeypatch):
-    """K = 256, 512, 1024 and 65,536 nonzeros or more run on the shared-memory rings over padded row groups:
-    empty rows at both ends and in the middle (written as zeros), rows of 1 .. B+1 nonzeros (padding), one row
-    holding every column (cut into pieces and summed by the fix-up kernel); against the oracle, and against
-    the register-staged kernel (SDDMM_SPMM_RING=0)."""
+def test_long_rows(engine, K):
+    """120,000 nonzeros at K = 256, 512, 1024: empty rows at both ends and in the middle (written as zeros), rows of 1 to 5
+    nonzeros, one row holding every column (cut into runs whose parts are added); against the oracle."""
     rng = np.random.default_rng(7 * K)
     M, N = 900, 700
     rows, cols = random_coo(rng, M, N, 120_000, empty_rows=[0, 1, 2, 450, 451, 898, 899], hub_row=17)
@@ -80,7 +78,7 @@ def test_ring_form_for_long_rows(engine, K, monkeypatch):
     plan = engine.plan_coo(M, N, rows, cols, K)
     Y = np.full((M, K), np.nan, np.float32)
     plan.spmm(H, Y, vals)
-    assert plan.last_kernel_name() == "spmm_ring"
+    assert plan.last_kernel_name() == "spmm"
     _check_y(Y, rows, cols, H, M, vals)
     P_ref = oracle.cpu.sddmm_coo(rows, cols, W, H, vals)
     P64, A_p = oracle.cpu.sddmm_coo_f64(rows, cols, W, H, vals)
@@ -88,20 +86,13 @@ def test_ring_form_for_long_rows(engine, K, monkeypatch):
     Yf = np.full((M, K), np.nan, np.float32)
     P_out = np.full(rows.shape[0], np.nan, np.float32)
     plan.fused(W, H, Yf, vals, P_out)
-    assert plan.last_kernel_name() == "fused_sddmm_spmm_ring"
+    assert plan.last_kernel_name() == "fused_sddmm_spmm"
     assert np.all(np.abs(P_out.astype(np.float64) - P64) <= TOL * np.maximum(np.abs(P64), A_p))
     _check_y(Yf, rows, cols, H, M, P_ref, A_extra=A_from_p)
     Yu = np.full((M, K), np.nan, np.float32)
     plan.fused(W, H, Yu, None)                       # unscaled
     _check_y(Yu, rows, cols, H, M, oracle.cpu.sddmm_coo(rows, cols, W, H), A_extra=oracle.cpu.spmm_f64(
         rows, cols, H, M, oracle.cpu.sddmm_coo_f64(rows, cols, W, H)[1])[1])
-    plan.close()
-    monkeypatch.setenv("SDDMM_SPMM_RING", "0")
-    plan = engine.plan_coo(M, N, rows, cols, K)
-    Y2 = np.full((M, K), np.nan, np.float32)
-    plan.fused(W, H, Y2, vals)
-    assert plan.last_kernel_name() == "fused_sddmm_spmm"
-    _check_y(Y2, rows, cols, H, M, P_ref, A_extra=A_from_p)
     plan.close()
 
 
