@@ -172,11 +172,13 @@ SDDMM_API int sddmm_spmm_execute(sddmm_plan_t p, const float *Pval, const float 
 SDDMM_API int sddmm_fused_execute(sddmm_plan_t p, const float *W, const float *H, const float *Sval,
                                   float *P_out, float *Y, uint32_t flags);
 
-/* Milliseconds of the kernels of the last synchronous sddmm_execute(), measured
- * with CUDA events on the compute stream -- the region the reference times and
- * prints as "Time for SDDMM with K = ..." (sddmm.cu:93,109-114).  For a pipelined
- * call (see sddmm_execute) it is the sum over the chunks' kernels; the waits for
- * uploads between them are not counted. */
+/* Milliseconds of the kernels of the last synchronous sddmm_execute(), sddmm_spmm_execute() or
+ * sddmm_fused_execute() -- the region the reference times and prints as "Time for SDDMM with K = ..."
+ * (sddmm.cu:93,109-114); -1 behind an asynchronous call.  A call that is one launch of the gather or SpMM
+ * kernel is timed by the kernel itself (nanosecond timer of the GPU: first block's start to last block's
+ * end), which leaves out the launch; every other call by CUDA events around its kernels, which add
+ * some microseconds.  For a pipelined call (see sddmm_execute) it is the sum over the chunks'
+ * kernels; the waits for uploads between them are not counted. */
 SDDMM_API int sddmm_last_kernel_ms(sddmm_plan_t p, float *ms);
 
 /* The kernels that the last call on this plan launched (static storage): "gather", "ring", "panel";

@@ -136,16 +136,19 @@ __device__ __forceinline__ void report_timeout(int *dev_status)
     *reinterpret_cast<volatile int *>(dev_status) = (int)DEV_MBARRIER_TIMEOUT;
     __threadfence_system();
 }
-// Kernel time of a synchronous call, from the nanosecond timer (32 ns steps): clock[0] = start of block 0, clock[1] =
-// the latest end of a block (time only grows, so the word is never cleared).  Two events around the launch cost 5 us
-// of a small call; this costs nothing measurable.  clock null: nothing.
+// Kernel time of a synchronous call, from the nanosecond timer: clock[0] = start of block 0, clock[1] = the latest end of a
+// block, when its last warp is done (time only grows, so the word is never cleared).  Two events around the launch
+// cost 5 us of a small call; this costs nothing measurable.  clock null: nothing.  Every thread of the block that has
+// not left the kernel calls clock_end.
 __device__ __forceinline__ void clock_begin(unsigned long long *clock)
 {
     if (clock && threadIdx.x == 0 && blockIdx.x == 0) clock[0] = globaltimer_ns();
 }
 __device__ __forceinline__ void clock_end(unsigned long long *clock)
 {
-    if (clock && threadIdx.x == 0) atomicMax(clock + 1, globaltimer_ns());
+    if (!clock) return;
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(clock + 1, globaltimer_ns());
 }
 // Wall-clock budget of one bounded wait.  The poll count alone says little about
 // time (every try_wait may block for a hardware-defined slice before it answers),

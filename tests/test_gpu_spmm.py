@@ -96,6 +96,28 @@ def test_long_rows(engine, K):
     plan.close()
 
 
+def test_kernel_time_lasts_until_the_last_warp(engine):
+    # one row in thousands of runs: whichever warp arrives last adds up the parts, while the first warp of its block has long
+    # ended.  The kernel's time has to cover that: it agrees with events around the call but for the launch.
+    N, K = 1 << 19, 512
+    cols = torch.arange(N, device="cuda", dtype=torch.int32)
+    H = torch.ones((N, K), device="cuda")
+    plan = engine.plan_coo(1, N, torch.zeros_like(cols), cols, K)
+    Y = torch.zeros((1, K), device="cuda")
+    for _ in range(3):
+        plan.spmm(H, Y)
+    for _ in range(5):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        e[0].record()
+        plan.spmm(H, Y)
+        e[1].record()
+        torch.cuda.synchronize()
+        around = e[0].elapsed_time(e[1])
+        assert around - 0.05 <= plan.last_kernel_ms() <= around
+    assert bool((Y == N).all())
+    plan.close()
+
+
 def test_spmm_unsupported_k_and_empty(engine):
     rows, cols = np.array([0, 1], np.int32), np.array([1, 0], np.int32)
     plan = engine.plan_coo(2, 2, rows, cols, 2048)
