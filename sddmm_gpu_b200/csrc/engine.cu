@@ -17,6 +17,7 @@
 
 #include "binning.cuh"
 #include "common.cuh"
+#include "gather_index.hpp"
 #include "sddmm_b200.h"
 
 using namespace sddmm;
@@ -901,7 +902,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (up_w.src || up_h.src || up_s)
         LAUNCH_TRY(h, launch_upload_operands(up_h, up_w, up_s, p->d_S, up_s ? p->nnz : 0, h->upload_ctas, s));
     CallTimer timer(p, async);
-    CUDA_TRY(h, timer.begin(one_gather, s));
+    CUDA_TRY(h, timer.begin(one_gather && p->nnz <= GATHER_SLICE, s));
     if (use_dense) {
         // locally dense plan: dense cells as small dense products, the rest gathered
         {

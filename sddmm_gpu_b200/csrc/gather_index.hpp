@@ -11,7 +11,8 @@
 namespace sddmm {
 
 constexpr unsigned GATHER_TPB = 256;
-// Nonzeros of one launch: the kernels count them in 32 bits.
+// Nonzeros of one launch: the kernels count them in 32 bits.  (The kernel clock times one launch, so longer calls are timed by
+// events.)
 constexpr int64_t GATHER_SLICE = 1ll << 30;
 
 // Number of a warp within its launch.  Not (block * threads per block + thread) / 32: a launch with a warp per nonzero has 2^32

@@ -91,3 +91,10 @@ def test_long_rows_beyond_two_to_the_27_nonzeros(engine, monkeypatch):
     # K > 1024: a warp per nonzero, 2^32 threads at 2^27 nonzeros
     monkeypatch.setenv("SDDMM_DENSE_CELLS", "0")   # every cell of these few rows and columns is full
     _all_of_P(engine, 512, 509, (1 << 27) + 12345, 1028)
+
+
+def test_kernel_time_covers_all_launches(engine, monkeypatch):
+    # more than 2^30 nonzeros go out in two launches
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "0")
+    ms, around = _all_of_P(engine, 512, 509, (1 << 30) + 54321, 4)
+    assert 0.9 * around <= ms <= around
