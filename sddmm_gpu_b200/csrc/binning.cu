@@ -16,20 +16,20 @@
 
 namespace sddmm {
 
-DevicePool *&current_pool()
+PoolScope *&PoolScope::current()
 {
-    static thread_local DevicePool *pool = nullptr;
-    return pool;
+    static thread_local PoolScope *scope = nullptr;
+    return scope;
 }
 cudaError_t pool_alloc(void **ptr, size_t bytes)
 {
-    if (DevicePool *p = current_pool()) return p->alloc(ptr, bytes);
+    if (PoolScope *at = PoolScope::current()) return at->pool.alloc(ptr, bytes, at->stream);
     return cudaMalloc(ptr, bytes);
 }
 void pool_free(void *ptr)
 {
     if (!ptr) return;
-    if (DevicePool *p = current_pool()) p->free(ptr, true);
+    if (PoolScope *at = PoolScope::current()) at->pool.free(ptr, at->stream, true);
     else cudaFree(ptr);
 }
 

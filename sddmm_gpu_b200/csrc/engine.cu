@@ -192,6 +192,7 @@ struct CallTimer {
     {
         if (async) return cudaSuccess;
         sddmm_handle_s *h = p->h;
+        std::lock_guard<std::mutex> hold(h->owners);
         if (kernel_has_clock && p->clock < 0 && !h->free_clocks.empty()) {
             p->clock = h->free_clocks.back();
             h->free_clocks.pop_back();
@@ -679,10 +680,13 @@ int sddmm_destroy_plan(sddmm_plan_t p)
     if (!p) return SDDMM_OK;
     cudaSetDevice(p->h->device);
     free_plan_memory(p);
-    if (p->clock >= 0) p->h->free_clocks.push_back(p->clock);
     if (p->spmm_done) cudaEventDestroy(p->spmm_done);
-    for (sddmm_plan_s *&owner : p->h->ev_owner) if (owner == p) owner = nullptr;
-    if (p->h->pipe_owner == p) p->h->pipe_owner = nullptr;
+    {
+        std::lock_guard<std::mutex> hold(p->h->owners);
+        if (p->clock >= 0) p->h->free_clocks.push_back(p->clock);
+        for (sddmm_plan_s *&owner : p->h->ev_owner) if (owner == p) owner = nullptr;
+        if (p->h->pipe_owner == p) p->h->pipe_owner = nullptr;
+    }
     (void)cudaGetLastError();
     delete p;
     return SDDMM_OK;
@@ -860,9 +864,12 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (pipelined) {
         p->last_kernel = rows_on_ring(p, use_ring) ? "ring (pipelined chunks)" : "gather (pipelined chunks)";
         CUDA_TRY(h, ensure_pipeline(h));
-        if (h->pipe_owner && h->pipe_owner != p && h->pipe_owner->ms_state == sddmm_plan_s::MS_IN_PIPE)
-            CUDA_TRY(h, resolve_ms(h->pipe_owner));
-        h->pipe_owner = p;
+        {
+            std::lock_guard<std::mutex> hold(h->owners);
+            if (h->pipe_owner && h->pipe_owner != p && h->pipe_owner->ms_state == sddmm_plan_s::MS_IN_PIPE)
+                CUDA_TRY(h, resolve_ms(h->pipe_owner));
+            h->pipe_owner = p;
+        }
         for (int i = 0; i < p->n_pipe; ++i) {
             const int64_t n0 = p->pipe_nnz[i], cnt = p->pipe_nnz[i + 1] - n0;
             up_w.begin = p->pipe_w_begin[i];

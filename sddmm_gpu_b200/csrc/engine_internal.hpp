@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -25,6 +26,8 @@ struct sddmm_handle_s {
     size_t smem_optin = 0;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
+    // guards free_clocks and the owners of events, which a plan that another thread destroys leaves
+    std::mutex owners;
     // event pairs around the kernels of synchronous calls that no kernel clock times, taken in turn; a plan's time is
     // read from its pair when it is asked for, or before another plan takes the pair
     cudaEvent_t ev_begin[SDDMM_EVENT_PAIRS] = {}, ev_end[SDDMM_EVENT_PAIRS] = {};

@@ -1,8 +1,9 @@
 // Device memory that plans and calls give back is kept by the handle for the next ones: cudaMalloc and cudaFree of a few
 // megabytes cost up to 1.5 ms a pair and wait for the whole device, more than planning a small matrix.
 //
-// The pool belongs to one handle and is used by one host thread at a time, like the handle.  It keeps at most LIMIT bytes
-// that nobody uses; more go back to CUDA at once, all of it when the handle is destroyed or an allocation fails.  A
+// The pool belongs to one handle.  The handle is used by one host thread at a time, but its plans may be destroyed by others
+// (a garbage collector's), so the pool locks.  It keeps at most LIMIT bytes that nobody uses; more go back to CUDA at
+// once, all of it when the handle is trimmed or destroyed or an allocation fails.  A
 // block given back while work on a stream may still touch it carries that stream and is handed out again only to work
 // on the same stream, until wait() has waited for that stream.
 #pragma once
@@ -10,6 +11,8 @@
 
 #include <cstddef>
 #include <map>
+#include <mutex>
+#include <new>
 #include <unordered_map>
 
 namespace sddmm {
@@ -17,11 +20,12 @@ namespace sddmm {
 class DevicePool {
 public:
     static constexpr size_t LIMIT = 2ull << 30;
-    cudaStream_t stream = nullptr;  // the stream of the current call
 
     ~DevicePool() { release(); }
-    cudaError_t alloc(void **ptr, size_t bytes)
+    // for work on the stream
+    cudaError_t alloc(void **ptr, size_t bytes, cudaStream_t stream)
     {
+        std::lock_guard<std::mutex> hold(lock_);
         const size_t n = rounded(bytes);
         // a quarter more than asked for at most, so that a small request does not take a large block away
         for (auto it = free_.lower_bound(n); it != free_.end() && it->first <= n + n / 4; ++it) {
@@ -34,20 +38,27 @@ public:
         cudaError_t e = cudaMalloc(ptr, n);
         if (e == cudaErrorMemoryAllocation && kept_ > 0) {
             (void)cudaGetLastError();
-            release();
+            release_all();
             e = cudaMalloc(ptr, n);
         }
         if (e != cudaSuccess) {
             *ptr = nullptr;
             return e;
         }
-        size_.emplace(*ptr, n);
+        try {
+            size_[*ptr] = n;
+        } catch (const std::bad_alloc &) {
+            cudaFree(*ptr);
+            *ptr = nullptr;
+            return cudaErrorMemoryAllocation;
+        }
         return cudaSuccess;
     }
-    // busy: work enqueued on the current stream may still use the block
-    void free(void *ptr, bool busy)
+    // busy: work enqueued on the stream may still use the block
+    void free(void *ptr, cudaStream_t stream, bool busy)
     {
         if (!ptr) return;
+        std::lock_guard<std::mutex> hold(lock_);
         auto it = size_.find(ptr);
         if (it == size_.end() || it->second > LIMIT / 2) {
             if (it != size_.end()) size_.erase(it);
@@ -64,19 +75,39 @@ public:
             cudaFree(old->second.ptr);
             free_.erase(old);
         }
-        kept_ += it->second;
-        free_.emplace(it->second, Block{ptr, stream, busy, ++clock_});
+        try {
+            free_.emplace(it->second, Block{ptr, stream, busy, ++clock_});
+            kept_ += it->second;
+        } catch (const std::bad_alloc &) {
+            size_.erase(it);
+            cudaFree(ptr);
+        }
     }
     // Waits for the stream; what was given back on it is idle then.
     cudaError_t wait(cudaStream_t s)
     {
+        // only what was given back before the wait began: another thread may give more back meanwhile
+        unsigned long long before;
+        {
+            std::lock_guard<std::mutex> hold(lock_);
+            before = clock_;
+        }
         const cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return e;
+        std::lock_guard<std::mutex> hold(lock_);
         for (auto &f : free_)
-            if (f.second.stream == s) f.second.busy = false;
+            if (f.second.stream == s && f.second.since <= before) f.second.busy = false;
         return cudaSuccess;
     }
+    // everything that nobody uses goes back to CUDA
     void release()
+    {
+        std::lock_guard<std::mutex> hold(lock_);
+        release_all();
+    }
+
+private:
+    void release_all()
     {
         for (auto &f : free_) {
             size_.erase(f.second.ptr);
@@ -86,7 +117,6 @@ public:
         kept_ = 0;
     }
 
-private:
     struct Block {
         void *ptr;
         cudaStream_t stream;
@@ -97,6 +127,7 @@ private:
     std::unordered_map<void *, size_t> size_;  // every block taken from CUDA and not given back to it
     size_t kept_ = 0;
     unsigned long long clock_ = 0;
+    std::mutex lock_;
 
     // sizes with three bits of mantissa, so that similar requests share blocks
     static size_t rounded(size_t n)
@@ -108,23 +139,17 @@ private:
     }
 };
 
-// The pool that pool_alloc / pool_free use on this thread while a PoolScope lives; without one they are cudaMalloc / cudaFree.
-DevicePool *&current_pool();
+// The pool and stream that pool_alloc / pool_free use on this thread while a PoolScope lives; without one they are cudaMalloc /
+// cudaFree.
 struct PoolScope {
-    DevicePool *const before, &pool;
-    const cudaStream_t stream_before;
-    PoolScope(DevicePool &p, cudaStream_t s) : before(current_pool()), pool(p), stream_before(p.stream)
-    {
-        current_pool() = &p;
-        p.stream = s;
-    }
-    ~PoolScope()
-    {
-        pool.stream = stream_before;
-        current_pool() = before;
-    }
+    DevicePool &pool;
+    const cudaStream_t stream;
+    PoolScope *const before;
+    PoolScope(DevicePool &p, cudaStream_t s) : pool(p), stream(s), before(current()) { current() = this; }
+    ~PoolScope() { current() = before; }
     PoolScope(const PoolScope &) = delete;
     PoolScope &operator=(const PoolScope &) = delete;
+    static PoolScope *&current();
 };
 cudaError_t pool_alloc(void **ptr, size_t bytes);
 void pool_free(void *ptr);  // after the last use on the call's stream has been enqueued

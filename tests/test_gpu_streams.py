@@ -165,3 +165,39 @@ def test_plan_destroyed_behind_a_queued_row_upload(engine):
     for q in others:
         q.close()
     del busy
+
+
+def test_plans_destroyed_by_another_thread(engine):
+    """A garbage collector may destroy plans from any thread while the handle works: what they give back (memory, kernel clocks,
+    event pairs) is shared."""
+    import threading
+    M, N, K = 2000, 1500, 64
+    rows, cols, vals, W, H = _problem(M, N, 60_000, K)
+    expect = torch.full((rows.shape[0],), float("nan"), device="cuda")
+    Y = torch.full((M, K), float("nan"), device="cuda")
+    plans = []
+    for i in range(60):
+        p = engine.plan_coo(M, N, rows, cols, K)
+        p.execute(W, H, expect, vals)                                     # holds a clock
+        if i % 2:
+            p.execute(W, H, expect, vals, api.FLAG_KERNEL_PANEL)          # holds an event pair
+        p.spmm(H, Y, vals)
+        plans.append(p)
+    keep = engine.plan_coo(M, N, rows, cols, K)
+    keep.execute(W, H, expect, vals)
+    worker = threading.Thread(target=lambda: [p.close() for p in plans])
+    worker.start()
+    for _ in range(200):
+        out = torch.full((rows.shape[0],), float("nan"), device="cuda")
+        engine.sddmm_coo(M, N, rows, cols, W, H, K, out, vals)
+        assert torch.equal(out, expect)
+        again = engine.plan_coo(M, N, rows, cols, K)
+        again.execute(W, H, out, vals)
+        assert torch.equal(out, expect) and 0 < again.last_kernel_ms() < 10
+        again.close()
+        if not worker.is_alive():
+            break
+    worker.join()
+    keep.execute(W, H, out, vals)
+    assert torch.equal(out, expect)
+    keep.close()

@@ -371,4 +371,4 @@ def test_gather_launch_arithmetic_past_2_to_the_32_threads(tmp_path):
 
 def test_memory_pool_hands_out_only_what_has_been_waited_for(tmp_path):
     nvcc = _nvcc()
-    _run_cpp(tmp_path, "pool", "-I", os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include"))
+    _run_cpp(tmp_path, "pool", "-pthread", "-fsanitize=thread", "-g", "-I", os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include"))
