@@ -27,4 +27,7 @@ SDDMM_HD unsigned gather_long_blocks(unsigned nnz)
     return (unsigned)(((uint64_t)nnz + GATHER_TPB / 32 - 1) / (GATHER_TPB / 32));
 }
 
+// First of the blocks that can be the last to run, of a grid of which `resident` blocks run at a time.
+SDDMM_HD unsigned last_wave(unsigned blocks, unsigned resident) { return blocks > resident ? blocks - resident : 0; }
+
 }  // namespace sddmm

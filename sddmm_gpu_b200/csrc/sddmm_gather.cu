@@ -96,7 +96,7 @@ template <class S, bool HAS_PERM>
 __global__ void __launch_bounds__(GA_TPB, S::CTAS)
 sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
                     const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
-                    float *__restrict__ P, unsigned nnz, int pieces, unsigned run_len, unsigned long long *clock)
+                    float *__restrict__ P, unsigned nnz, int pieces, unsigned run_len, unsigned long long *clock, unsigned meet_from)
 {
     clock_begin(clock);
     constexpr int L = S::L, F = S::F, B = S::B, RB = S::RB, NB = S::NB, G = S::G;
@@ -190,7 +190,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
     }
     // (launched beside the kernel before it: that one is done when this one is)
     if (HAS_PERM && blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
-    clock_end(clock);
+    clock_end(clock, meet_from);
 }
 
 // Rows of more than 256 pieces (K > 1024): a warp per nonzero, both rows in passes of 32 pieces, W through L1.
@@ -198,7 +198,7 @@ template <bool HAS_PERM>
 __global__ void __launch_bounds__(GA_TPB)
 sddmm_gather_long_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
                          const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
-                         float *__restrict__ P, unsigned nnz, int pieces, unsigned long long *clock)
+                         float *__restrict__ P, unsigned nnz, int pieces, unsigned long long *clock, unsigned meet_from)
 {
     clock_begin(clock);
     constexpr int U = 4;
@@ -232,7 +232,7 @@ sddmm_gather_long_kernel(const int32_t *__restrict__ rows, const int32_t *__rest
         if (sval) a *= __ldg(sval + dst);
         P[dst] = a;
     }
-    clock_end(clock);
+    clock_end(clock, meet_from);
 }
 
 template <class S, bool HAS_PERM>
@@ -249,6 +249,7 @@ cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32
     run = run < (unsigned)S::NB ? (unsigned)S::NB : run > most ? most : run;
     const unsigned tpb = beside ? GA_TPB_BESIDE : GA_TPB, per_block = run * S::G * (tpb / 32);
     const unsigned blocks = (unsigned)(((uint64_t)nnz + per_block - 1) / per_block);
+    const unsigned meet_from = last_wave(blocks, (unsigned)sm_count * S::CTAS);
     if (HAS_PERM && beside) {
         cudaLaunchAttribute attr = {};
         attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -260,10 +261,10 @@ cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         return cudaLaunchKernelEx(&cfg, sddmm_gather_kernel<S, HAS_PERM>, rows, cols, perm, sval, static_cast<const char *>(W),
-                                  static_cast<const char *>(H), P, nnz, pieces, run, clock);
+                                  static_cast<const char *>(H), P, nnz, pieces, run, clock, meet_from);
     }
     sddmm_gather_kernel<S, HAS_PERM><<<blocks, GA_TPB, 0, stream>>>(rows, cols, perm, sval, static_cast<const char *>(W),
-                                                                    static_cast<const char *>(H), P, nnz, pieces, run, clock);
+                                                                    static_cast<const char *>(H), P, nnz, pieces, run, clock, meet_from);
     return cudaGetLastError();
 }
 
@@ -314,9 +315,9 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
         else if (q <= 224) GA_GO(32, 7, 1, 8, false, false, 3);
         else if (q <= 256) GA_GO(32, 8, 1, 8, false, false, 3);
         else {
-            const unsigned blocks = gather_long_blocks(n);
-            if (p) sddmm_gather_long_kernel<true><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock);
-            else sddmm_gather_long_kernel<false><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock);
+            const unsigned blocks = gather_long_blocks(n), meet_from = last_wave(blocks, (unsigned)sm_count * 8);
+            if (p) sddmm_gather_long_kernel<true><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock, meet_from);
+            else sddmm_gather_long_kernel<false><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock, meet_from);
             e = cudaGetLastError();
         }
 #undef GA_GO

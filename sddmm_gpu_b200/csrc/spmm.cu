@@ -35,6 +35,7 @@
 
 #include "common.cuh"
 #include "device_utils.cuh"
+#include "gather_index.hpp"
 
 namespace sddmm {
 
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(SP_TPB, S::CTAS)
 spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const float *__restrict__ val,
             const char *__restrict__ W, const char *__restrict__ H, float *__restrict__ P_out, char *__restrict__ Y,
             char *scratch, unsigned *arrived, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces,
-            unsigned run_len, unsigned gather_blocks, unsigned long long *clock)
+            unsigned run_len, unsigned gather_blocks, unsigned long long *clock, unsigned meet_from)
 {
     constexpr int L = S::L, F = S::F, B = S::B, NB = S::NB, G = S::G;
     constexpr bool FUSED = S::FUSED;
@@ -100,7 +101,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             empty &= empty - 1;
             for (int q = lane; q < pieces; q += 32) stg_u64x2(out + q * 16, u64x2{0, 0});
         }
-        clock_end(clock);
+        if (clock && threadIdx.x == 0) clock_note(clock);
         return;
     }
     const int lig = lane & (L - 1), set = lane / L;
@@ -365,12 +366,15 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                     if (lig == 0) arrived[2 * first + 1] = 0;
                     __threadfence();
                     add_up(first, last, SP_GROUP);
+                    flush(Y + row * row_bytes);
+                    if (clock && lig == 0) clock_note(clock);  // (a row of many runs: this may outlast every block that starts later)
+                    continue;
                 }
                 flush(Y + row * row_bytes);
             }
         }
     }
-    clock_end(clock);
+    clock_end(clock, meet_from);
 }
 
 template <class S>
@@ -405,7 +409,7 @@ cudaError_t launch_shape(const SpmmCall &a, int sm_count, int64_t *n_launches, c
     char *const parts = reinterpret_cast<char *>(a.scratch + spmm_counter_floats(a.nnz, a.K, sm_count));
     spmm_kernel<S><<<gather_blocks + zero_blocks, SP_TPB, 0, stream>>>(
         a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H), a.P_out,
-        reinterpret_cast<char *>(a.Y), parts, arrived, a.row_ptr, (unsigned)a.nnz, a.M, pieces, run, gather_blocks, a.clock);
+        reinterpret_cast<char *>(a.Y), parts, arrived, a.row_ptr, (unsigned)a.nnz, a.M, pieces, run, gather_blocks, a.clock, last_wave(gather_blocks, (unsigned)sm_count * S::CTAS));
     ++*n_launches;
     return cudaGetLastError();
 }
