@@ -100,7 +100,7 @@ struct sddmm_plan_s {
     int ev_pair = -1;
     // chunks of the host-operand pipeline (0 = not pipelined): nonzeros
     // [pipe_nnz[i], pipe_nnz[i+1]); filled by ensure_pipe
-    int n_pipe = 0;
+    int n_pipe = 0, pipe_step = 1;  // chunks; chunks that the last call took together
     bool pipe_ready = false;
     int64_t pipe_nnz[SDDMM_PIPE_MAX_CHUNKS + 1] = {};
     // rows of W chunk i uploads: [pipe_w_begin[i], pipe_w_end[i]) (empty when an earlier chunk brought them)

@@ -66,3 +66,24 @@ def test_chunked_call_keeps_its_kernel_time(engine):
     assert all(t > 0 for t in times) and times == [plan.last_kernel_ms() for plan in plans]
     for plan in plans:
         plan.close()
+
+
+def test_chunks_taken_together_for_a_pageable_result(engine):
+    # 168 MB of W are five chunks; with P in pageable memory four of them go together, then the last one
+    rng = np.random.default_rng(1)
+    M, N, K = 656_000, 300, 64
+    rows = np.sort(rng.integers(0, M, 150_003)).astype(np.int32)
+    cols = rng.integers(0, N, rows.size).astype(np.int32)
+    W, H = (rng.standard_normal((n, K)).astype(np.float32) for n in (M, N))
+    vals = rng.standard_normal(rows.size).astype(np.float32)
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    Wp = _pinned(W)
+    for operand in (W, Wp, W):
+        P = np.full(rows.size, np.nan, np.float32)
+        plan.execute(operand, H, P, vals)
+        assert plan.last_kernel_name() == "gather (pipelined chunks)" and plan.last_kernel_ms() > 0
+        assert_parity(P, rows, cols, W, H, vals)
+        Pp = torch.full((rows.size,), float("nan")).pin_memory()       # chunk by chunk
+        plan.execute(operand, H, Pp, vals)
+        assert plan.last_kernel_ms() > 0 and np.array_equal(Pp.numpy(), P)
+    plan.close()
