@@ -80,6 +80,13 @@ SDDMM_API const char *sddmm_status_string(int status);
 SDDMM_API int sddmm_create(sddmm_handle_t *out, int device);
 SDDMM_API int sddmm_destroy(sddmm_handle_t h);
 
+/*
+ * Device memory that closed plans and finished calls give back stays with the handle for the next
+ * ones, up to 2 GB (the reference allocates and frees on every call, sddmm.cu:38-73,147-150).  Other
+ * allocators in the process cannot see it: this gives all of it back to CUDA.  Waits for the device.
+ */
+SDDMM_API int sddmm_trim(sddmm_handle_t h);
+
 /* Text of the last CUDA / parse error seen through this handle ("" if none). */
 SDDMM_API const char *sddmm_last_error(sddmm_handle_t h);
 

@@ -33,7 +33,7 @@ PLAN_FORCE_H_CHUNKS = 0x4
 
 EXPORTED_SYMBOLS = [
     "sddmm_status_string", "sddmm_create", "sddmm_destroy", "sddmm_last_error", "sddmm_set_stream",
-    "sddmm_plan_coo", "sddmm_destroy_plan", "sddmm_execute", "sddmm_last_kernel_ms", "sddmm_last_transfer_bytes", "sddmm_plan_used_lines", "sddmm_upload_rows", "sddmm_coo",
+    "sddmm_trim", "sddmm_plan_coo", "sddmm_destroy_plan", "sddmm_execute", "sddmm_last_kernel_ms", "sddmm_last_transfer_bytes", "sddmm_plan_used_lines", "sddmm_upload_rows", "sddmm_coo",
     "sddmm_selftest_wait_timeout", "sddmm_plan_get_info", "sddmm_plan_count_cols", "sddmm_count_cols_noalloc", "sddmm_plan_export_row_ptr",
     "sddmm_plan_export_tiling", "sddmm_partition_rows", "sddmm_partition_rows_weighted", "sddmm_mtx_open", "sddmm_mtx_read",
     "sddmm_spmm_execute", "sddmm_fused_execute", "sddmm_last_kernel_name", "sddmm_kernel_launches", "sddmm_sync", "sddmm_check_result", "sddmm_selftest_optin_cache",
@@ -87,6 +87,7 @@ def lib():
     L.sddmm_destroy_plan.argtypes = [vp]
     L.sddmm_execute.argtypes = [vp, vp, vp, vp, vp, u32]
     L.sddmm_last_kernel_ms.argtypes = [vp, C.POINTER(C.c_float)]
+    L.sddmm_trim.argtypes = [vp]
     L.sddmm_last_kernel_name.restype = C.c_char_p
     L.sddmm_last_kernel_name.argtypes = [vp]
     L.sddmm_spmm_execute.argtypes = [vp, vp, vp, vp, u32]
@@ -250,6 +251,10 @@ class Handle:
     def _check(self, st):
         if st != OK:
             raise SddmmError(st, self.last_error())
+
+    def trim(self):
+        """Give the device memory that the handle keeps for its next plans and calls (up to 2 GB) back to CUDA."""
+        self._check(lib().sddmm_trim(self._h))
 
     def selftest_wait_timeout(self):
         """Status of a wait that is made to run out (expected: DEVICE_TIMEOUT)."""

@@ -530,6 +530,14 @@ int sddmm_destroy(sddmm_handle_t h)
     return SDDMM_OK;
 }
 
+int sddmm_trim(sddmm_handle_t h)
+{
+    if (!h) return SDDMM_INVALID_ARG;
+    CUDA_TRY(h, cudaSetDevice(h->device));
+    h->pool.release();
+    return SDDMM_OK;
+}
+
 const char *sddmm_last_error(sddmm_handle_t h) { return h ? h->last_error.c_str() : ""; }
 
 int sddmm_set_stream(sddmm_handle_t h, void *cuda_stream)

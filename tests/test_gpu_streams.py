@@ -201,3 +201,22 @@ def test_plans_destroyed_by_another_thread(engine):
     keep.execute(W, H, out, vals)
     assert torch.equal(out, expect)
     keep.close()
+
+
+def test_trim_gives_the_kept_memory_back():
+    h = api.Handle(0)
+    M, N, K = 40_000, 30_000, 256
+    rows, cols, vals, W, H = _problem(M, N, 300_000, K)
+    out = torch.zeros(rows.shape[0], device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    Wh, Hh = W.cpu(), H.cpu()
+    for _ in range(3):
+        h.sddmm_coo(M, N, rows, cols, Wh, Hh, K, out, vals)        # 72 MB of operands staged
+    assert before - torch.cuda.mem_get_info()[0] >= 60 << 20
+    h.trim()
+    assert before - torch.cuda.mem_get_info()[0] < 20 << 20
+    expect = out.clone()
+    h.sddmm_coo(M, N, rows, cols, W, H, K, out, vals)
+    assert torch.equal(out, expect)
+    h.close()
