@@ -2,7 +2,8 @@
 // Replaces the host driver sddmm_GPU of the reference (HiPC18/src/sddmm.cu:32-151):
 // device memory for the pattern is owned by a reusable plan instead of being
 // allocated and freed per call, errors come back as status codes instead of
-// assert(), and there is exactly one kernel launch per execute.
+// assert(), and an execute with device operands is one kernel launch (two where S
+// has dense cells and a remainder).
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -637,11 +638,14 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
     // Locally dense matrices (many nonzeros per row): cells that are at least a
     // quarter full go to the dense-cell kernel, if they hold half of S or more
     // (below that the second launch and the permuted remainder cost more than they save).
-    // Below 2^26 multiplications the cells save little or nothing, and the classification costs a plan 300 us that a pattern
-    // of that size, planned for a call or a few, does not earn back (us per call, band + global masks, gather / cells: 0.36 M nonzeros,
-    // K = 64 11 / 12;  0.9 M, K = 32 13 / 13, K = 64 18 / 13;  1.1 M, K = 32 16 / 16, K = 64 22 / 17;  1.6 M, K = 64 28 / 13;
-    // 1.9 M, K = 64 33 / 19;  planned, called and closed: 0.36 M, K = 64 42 / 365).
-    // SDDMM_DENSE_CELLS=0 switches the classification off, 1 takes it at every size.
+    // From 2^26 multiplications on.  The line is a compromise between the call and the plan, to which the classification adds
+    // 300 us.  Up to 2^25.2 the cells save a call nothing; from there to the line 1 to 6 us of 14 to 20, which a mask pays that
+    // is kept for more than some fifty calls; above it 6 us and more.  (us per call, band + global masks, gather / cells:
+    // 2^24.3 multiplications: 0.33 M nonzeros, K = 64 10.4 / 10.7;  2^25.1: 0.57 M, K = 64 12.4 / 11.6, 1.1 M, K = 32 14.5 / 13.9,
+    // 0.14 M, K = 256 12.5 / 16.4;  2^25.3: 0.33 M, K = 128 15.5 / 13.0, 0.67 M, K = 64 14.4 / 12.4;  2^25.7: 0.57 M, K = 96 16.5 /
+    // 12.4, 1.7 M, K = 32 18.6 / 14.3;  2^25.9: 0.67 M, K = 96 20.4 / 14.4;  2^26.1: 0.57 M, K = 128 22.4 / 13.3, 2.2 M, K = 32
+    // 22.7 / 16.5, 0.14 M, K = 512 22.7 / 22.7;  planned, called and closed: 0.36 M, K = 64 42 / 365.)
+    // SDDMM_DENSE_CELLS=0 switches the classification off, 1 takes it at every size: the choice for a mask of that size that is kept.
     {
         const char *env = std::getenv("SDDMM_DENSE_CELLS");
         const bool enabled = !(env && std::atoi(env) == 0), always = env && std::atoi(env) == 1;
