@@ -24,9 +24,10 @@
 // zeroed by blocks of their own at the end of the grid.
 //
 // What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero through L2; used twice in the fused form), hidden
-// by resident warps.  Measured on R-MAT matrices against the row-task and shared-memory-ring kernels this replaces
+// by resident warps.  The fused form at K = 256 reaches neither bound (16.1 M nonzeros: 7.1 GB through DRAM at 4.5 TB/s, 13.4 TB/s read at
+// the L2 slices): between two blocks of B rows a set reduces, broadcasts and adds with nothing in flight.  Measured on R-MAT matrices against the row-task and shared-memory-ring kernels this replaces
 // (us): SpMM, 6.0 M nonzeros, 250 K x 250 K: K = 64 755 -> 125;  0.67 M nonzeros: K = 64 379 -> 29;  fused, 16.1 M
-// nonzeros, 1 M x 1 M: K = 256 2970 -> 1675;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.
+// nonzeros, 1 M x 1 M: K = 256 2970 -> 1720 to 1785;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.
 // At K = 64 the gather kernel alone runs at 14.2 TB/s of gathered bytes.
 #include <cuda_runtime.h>
 #include <stdint.h>
