@@ -809,7 +809,7 @@ __global__ void fill_dense_kernel(const Key *__restrict__ keys_s, const int32_t 
             DenseCell dcell;
             dcell.row0 = row0;
             dcell.col0 = col0;
-            dcell.offset = dense_off[ci];
+            dcell.slot = dense_off[ci];  // of its nonzeros in the lists, until the forms are known
             dcell.count = cell_start[ci + 1] - start;
             dcell.cls = cls;
             cells[dense_slot[ci]] = dcell;
@@ -836,8 +836,8 @@ __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const i
         }
         __syncthreads();
         const DenseCell dc = cells[cell];
-        const int32_t *ci = idx + dc.offset;
-        const uint16_t *cr = rc + dc.offset;
+        const int32_t *ci = idx + dc.slot;
+        const uint16_t *cr = rc + dc.slot;
         unsigned long long *mk = row_mask + cell * DENSE_CELL_ROWS;
         for (int t = threadIdx.x; t < dc.count; t += blockDim.x) {
             const unsigned code = cr[t];
@@ -848,6 +848,7 @@ __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const i
                 first[r] = ci[t];
             } else {
                 if ((int)(prev & 255u) >= c) bad = 1;
+                if (ci[t] - ci[t - 1] != c - (int)(prev & 255u)) forms = 0;
                 if (ci[t] != ci[t - 1] + 1) {
                     if (atomicAdd(&gaps[r], 1) > 0) bad = 1;
                     split[r] = c;
@@ -864,7 +865,6 @@ __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const i
             row_base[cell * DENSE_CELL_ROWS + r] = make_int2(first[r], second[r] - before);
             const int c0 = m ? __ffsll(m) - 1 : 0, n = __popcll(m);
             row_span[cell * DENSE_CELL_ROWS + r] = (uint32_t)c0 | (uint32_t)n << 8 | (uint32_t)s << 16;
-            if (s < DENSE_CELL_COLS || (m && (m >> c0) != (n < 64 ? (1ull << n) - 1ull : ~0ull))) forms = 0;
         }
         __syncthreads();
         if (threadIdx.x == 0 && !bad) {
@@ -872,6 +872,71 @@ __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const i
             atomicAdd(n_mask_cells, 1ull);
         }
         __syncthreads();
+    }
+}
+
+// Tables of the cells that are not in row-mask form (one CTA per cell, grid-stride); DenseCell::slot becomes the number of the
+// table.  table arrives filled with -1.  Of several nonzeros of one row and column the first is entered, the others go to
+// the remainder.  words[0]: tables, words[1]: nonzeros that went; both arrive 0.
+__global__ void cell_tables_kernel(DenseCell *cells, int64_t n_cells, const int32_t *__restrict__ idx, const uint16_t *__restrict__ rc,
+                                   int32_t *table, unsigned char *is_dense, unsigned long long *words)
+{
+    __shared__ unsigned long long slot;
+    for (int64_t cell = blockIdx.x; cell < n_cells; cell += gridDim.x) {
+        const DenseCell dc = cells[cell];
+        if (dc.cls & CELL_MASKED) continue;  // the same for the whole block
+        if (threadIdx.x == 0) slot = atomicAdd(words, 1ull);
+        __syncthreads();
+        unsigned *t = reinterpret_cast<unsigned *>(table) + slot * (DENSE_CELL_ROWS * DENSE_CELL_COLS);
+        auto entry = [&](int i) {
+            const unsigned code = rc[dc.slot + i];
+            return t + (code >> 8) * DENSE_CELL_COLS + (code & 255u);
+        };
+        for (int i = threadIdx.x; i < dc.count; i += blockDim.x) atomicMin(entry(i), (unsigned)idx[dc.slot + i]);
+        __threadfence_block();
+        __syncthreads();
+        unsigned long long gone = 0;
+        for (int i = threadIdx.x; i < dc.count; i += blockDim.x) {
+            const unsigned mine = (unsigned)idx[dc.slot + i];
+            if (atomicMin(entry(i), 0xffffffffu) != mine) {
+                is_dense[mine] = 0;
+                ++gone;
+            }
+        }
+        if (gone) atomicAdd(words + 1, gone);
+        if (threadIdx.x == 0) cells[cell].slot = (int64_t)slot;
+        __syncthreads();
+    }
+}
+
+// Cells are in the order of (class, row0, col0): a unit begins at every second cell of the same rows.
+struct UnitHead {
+    const DenseCell *cells;
+    __device__ __forceinline__ bool operator()(int c) const
+    {
+        const int cls = cells[c].cls & 0xff, row0 = cells[c].row0;
+        int lo = 0, hi = c;  // first cell of these rows
+        while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2, k = cells[mid].cls & 0xff;
+            if (k < cls || (k == cls && cells[mid].row0 < row0)) lo = mid + 1;
+            else hi = mid;
+        }
+        return ((c - lo) & 1) == 0;
+    }
+};
+__global__ void unit_fill_kernel(const DenseCell *__restrict__ cells, const int32_t *__restrict__ heads, int n_cells, int n_units, DenseUnit *units)
+{
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x) {
+        const int c = heads[u], n = (u + 1 < n_units ? heads[u + 1] : n_cells) - c;
+        DenseUnit d = {};
+        d.n = n;
+        d.row0 = cells[c].row0;
+        for (int k = 0; k < n; ++k) {
+            d.number[k] = cells[c + k].cls & CELL_MASKED ? c + k : (int32_t)cells[c + k].slot;
+            d.col0[k] = cells[c + k].col0;
+            d.cls[k] = cells[c + k].cls;
+        }
+        units[u] = d;
     }
 }
 
@@ -884,12 +949,12 @@ struct NotDense {
 
 void DensePlan::release()
 {
-    pool_free(cells); pool_free(idx); pool_free(rc); pool_free(rows_s); pool_free(cols_s); pool_free(perm_s);
+    pool_free(cells); pool_free(units); pool_free(table); pool_free(rows_s); pool_free(cols_s); pool_free(perm_s);
     pool_free(dense_rows); pool_free(dense_cols); pool_free(row_mask); pool_free(row_base); pool_free(row_span);
-    cells = nullptr; idx = nullptr; rc = nullptr; rows_s = cols_s = perm_s = nullptr;
+    cells = nullptr; units = nullptr; table = nullptr; rows_s = cols_s = perm_s = nullptr;
     dense_rows = dense_cols = nullptr;
     row_mask = nullptr; row_base = nullptr; row_span = nullptr;
-    n_cells = n_dense_nnz = n_sparse = n_dense_rows = n_dense_cols = n_mask_cells = 0;
+    n_cells = n_dense_nnz = n_sparse = n_dense_rows = n_dense_cols = n_units = n_table_cells = 0;
 }
 
 // Key: of a cell; 32 bits wherever they are enough (the sort moves two thirds of the bytes).
@@ -1020,14 +1085,16 @@ static cudaError_t build_dense_cells_k(const int32_t *d_rows, const int32_t *d_c
     // 4. the dense arrays and the remainder
     auto body = [&]() -> cudaError_t {
         CK(pool_alloc(&out->cells, (size_t)n_dense_cells));
-        CK(pool_alloc(&out->idx, (size_t)n_dense_nnz));
-        CK(pool_alloc(&out->rc, (size_t)n_dense_nnz));
+        Scratch lists;  // idx: input index of every dense-cell nonzero, grouped by cell, row-major inside; rc: (row - row0) << 8 | (col - col0)
+        CK(lists.reserve((size_t)n_dense_nnz * 6));
+        int32_t *idx = (int32_t *)lists.ptr;
+        uint16_t *rc = (uint16_t *)(idx + n_dense_nnz);
         Scratch flags;
         CK(flags.reserve((size_t)nnz));
         CK(cudaMemsetAsync(flags.ptr, 0, (size_t)nnz, stream));
         fill_dense_kernel<<<grid_for(nnz), TPB, 0, stream>>>(k_s, i_s, cellid, cell_start, dense_flag, dense_slot, dense_off,
                                                             d_rows, d_cols, row_vid, col_vid, nnz, geo, out->cells,
-                                                            out->idx, out->rc, (unsigned char *)flags.ptr);
+                                                            idx, rc, (unsigned char *)flags.ptr);
         CK(cudaGetLastError());
         // row-mask form of the cells that allow it
         {
@@ -1040,13 +1107,44 @@ static cudaError_t build_dense_cells_k(const int32_t *d_rows, const int32_t *d_c
             CK(cnt.reserve(sizeof(unsigned long long)));
             CK(cudaMemsetAsync(cnt.ptr, 0, sizeof(unsigned long long), stream));
             cell_row_masks_kernel<<<grid_for((int64_t)n_dense_cells * TPB), TPB, 0, stream>>>(
-                out->cells, n_dense_cells, out->idx, out->rc, out->row_mask, out->row_base,
+                out->cells, n_dense_cells, idx, rc, out->row_mask, out->row_base,
                 out->row_span, (unsigned long long *)cnt.ptr);
             CK(cudaGetLastError());
             unsigned long long n_mask = 0;
             CK(cudaMemcpyAsync(&n_mask, cnt.ptr, sizeof(n_mask), cudaMemcpyDeviceToHost, stream));
             CK(cudaStreamSynchronize(stream));
-            out->n_mask_cells = (int64_t)n_mask;
+            out->n_table_cells = n_dense_cells - (int64_t)n_mask;
+        }
+        if (out->n_table_cells > 0) {
+            const size_t entries = (size_t)out->n_table_cells * DENSE_CELL_ROWS * DENSE_CELL_COLS;
+            CK(pool_alloc(&out->table, entries));
+            CK(cudaMemsetAsync(out->table, 0xff, sizeof(int32_t) * entries, stream));
+            Scratch words;
+            CK(words.reserve(2 * sizeof(unsigned long long)));
+            CK(cudaMemsetAsync(words.ptr, 0, 2 * sizeof(unsigned long long), stream));
+            cell_tables_kernel<<<grid_for((int64_t)n_dense_cells * TPB), TPB, 0, stream>>>(out->cells, n_dense_cells, idx, rc, out->table,
+                                                                                          (unsigned char *)flags.ptr, (unsigned long long *)words.ptr);
+            CK(cudaGetLastError());
+            unsigned long long gone = 0;
+            CK(cudaMemcpyAsync(&gone, (unsigned long long *)words.ptr + 1, sizeof(gone), cudaMemcpyDeviceToHost, stream));
+            CK(cudaStreamSynchronize(stream));
+            n_dense_nnz -= (int64_t)gone;
+        }
+        // units of one or two cells
+        {
+            Scratch heads;
+            CK(heads.reserve(sizeof(int32_t) * (size_t)n_dense_cells));
+            tb = 0;
+            CK(cub::DeviceSelect::If(nullptr, tb, counting, (int32_t *)heads.ptr, d_n_sel, n_dense_cells, UnitHead{out->cells}, stream));
+            CK(tmp.reserve(tb));
+            CK(cub::DeviceSelect::If(tmp.ptr, tb, counting, (int32_t *)heads.ptr, d_n_sel, n_dense_cells, UnitHead{out->cells}, stream));
+            int n_units = 0;
+            CK(cudaMemcpyAsync(&n_units, d_n_sel, sizeof(int), cudaMemcpyDeviceToHost, stream));
+            CK(cudaStreamSynchronize(stream));
+            CK(pool_alloc(&out->units, (size_t)n_units));
+            unit_fill_kernel<<<grid_for(n_units), TPB, 0, stream>>>(out->cells, (const int32_t *)heads.ptr, n_dense_cells, n_units, out->units);
+            CK(cudaGetLastError());
+            out->n_units = n_units;
         }
         const int64_t n_sparse = nnz - n_dense_nnz;
         if (n_sparse > 0) {

@@ -94,18 +94,21 @@ cudaError_t build_hub_column_hints(const int32_t *d_cols_p, int64_t nnz, int64_t
 struct DensePlan {
     DenseCell *cells = nullptr;   // one descriptor per dense cell
     int64_t n_cells = 0;
-    int32_t *idx = nullptr;       // input index of every dense-cell nonzero, grouped by cell, row-major inside
-    uint16_t *rc = nullptr;       // (row - row0) << 8 | (col - col0)
+    // Cells of the same rows in twos (consecutive ones, from the first cell of those rows on; the last one may be alone).
+    DenseUnit *units = nullptr;
+    int64_t n_units = 0;
     // Row-mask form of a cell (DenseCell::cls bit 8 set): per cell row a 64-bit column mask and the input positions of
     // its nonzeros as at most two runs: the nonzero in column c sits at popc(mask below c) past row_base.x, or past
     // row_base.y from column row_span >> 16 on (64: one run; the lower bytes of row_span: first column and number).  Valid for cells in which the nonzeros of every row have
     // ascending columns and at most one gap in their input positions: cells of the regular grid (the gap is a nonzero
     // that went to a compacted full column) and cells of compacted columns (the gap is the band between them) of a
-    // (row, col)-sorted input; such a cell's nonzeros need no per-nonzero list.
+    // (row, col)-sorted input.  All other cells are in table form: the input position of every entry of the cell, -1 where S
+    // holds nothing.  (A second nonzero of the same row and column is not in its cell then but in the remainder.)
     unsigned long long *row_mask = nullptr;  // [n_cells][DENSE_CELL_ROWS]
     int2 *row_base = nullptr;                // [n_cells][DENSE_CELL_ROWS]
     uint32_t *row_span = nullptr;            // [n_cells][DENSE_CELL_ROWS]
-    int64_t n_mask_cells = 0;
+    int32_t *table = nullptr;                // [n_table_cells][DENSE_CELL_ROWS][DENSE_CELL_COLS]
+    int64_t n_table_cells = 0;
     int64_t n_dense_nnz = 0;
     int32_t *rows_s = nullptr, *cols_s = nullptr, *perm_s = nullptr;  // remainder: indices and input positions
     int64_t n_sparse = 0;

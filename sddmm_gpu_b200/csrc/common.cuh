@@ -25,21 +25,27 @@ struct WorkItem {
 };
 
 // A dense cell of S: rows [row0, row0 + DENSE_CELL_ROWS) x columns [col0, col0 +
-// DENSE_CELL_COLS) (clipped), whose `count` nonzeros start at `offset` in the
-// plan's dense arrays.  cls 0: row0 indexes the list of compacted full rows;
+// DENSE_CELL_COLS) (clipped).  cls 0: row0 indexes the list of compacted full rows;
 // cls 1: col0 indexes the list of compacted full columns; cls 2: both are
 // plain matrix coordinates.
 constexpr int DENSE_CELL_ROWS = 128;
 constexpr int DENSE_CELL_COLS = 64;
 // Forms of a cell in DenseCell::cls, above the class: CELL_MASKED = the row-mask form (see DensePlan); CELL_RUNS = of those, a
-// cell in which every row is one run of columns at consecutive input positions.
+// cell in which the input position of every row's nonzeros is their column plus a number of the row (columns may be missing: those
+// that are in another cell); neither = the table form, the cell's input positions are table number `slot` of the plan.
 constexpr int CELL_MASKED = 0x100, CELL_RUNS = 0x200;
 struct DenseCell {
-    int64_t offset;
+    int64_t slot;
     int32_t row0, col0;
     int32_t count;
     int32_t cls;
 };
+// One or two cells of the same rows: a product of the tcgen05 kernel.  number: of the cell or, in table form, of its table.
+struct DenseUnit {
+    int32_t number[2], n;
+    int32_t row0, col0[2], cls[2];
+};
+struct DensePlan;
 
 // The opt-in to more than 48 KB of dynamic shared memory (cudaFuncSetAttribute) is a
 // property of a kernel ON ONE DEVICE: a process that drives several GPUs must make it
@@ -153,21 +159,14 @@ cudaError_t launch_ring_bf16(const int32_t *rows, const int32_t *cols, const int
 
 // Dense-cell kernel: every dense cell is computed as the 128 x 64 block
 // W[rows] * H[cols]^T -- fp32 FMAs, or (tensor) 3xTF32 on the tensor cores -- then
-// the cell's nonzeros pick their entries: P[idx[i]] = block[rc[i]] (* sval[idx[i]]).
-// Cells whose cls has bit 8 set are in row-mask form (row_mask / row_base, see DensePlan) and
-// do not read idx / rc.
-cudaError_t launch_dense_cells(const DenseCell *cells, int64_t n_cells, const int32_t *idx, const uint16_t *rc,
-                               const unsigned long long *row_mask, const int2 *row_base, const uint32_t *row_span, const int32_t *dense_rows, int64_t n_dense_rows, const int32_t *dense_cols,
-                               int64_t n_dense_cols, const float *sval, const float *W, const float *H, float *P,
+// the cell's nonzeros pick their entries: P[i] = block[r][c] (* sval[i]) for the nonzero at input position i.
+cudaError_t launch_dense_cells(const DensePlan &d, const float *sval, const float *W, const float *H, float *P,
                                int64_t M, int64_t N, int K, bool tensor, int sm_count, cudaStream_t stream);
 
 // The same dense cells on tcgen05: MMAs issued by one thread from shared-memory descriptors, accumulator in
 // tensor memory (3xTF32).  dev_status receives DEV_MBARRIER_TIMEOUT if a bounded wait gives up.
-cudaError_t launch_dense_cells_tc(const DenseCell *cells, int64_t n_cells, const int32_t *idx, const uint16_t *rc,
-                                  const unsigned long long *row_mask, const int2 *row_base, const uint32_t *row_span, const int32_t *dense_rows,
-                                  int64_t n_dense_rows, const int32_t *dense_cols, int64_t n_dense_cols, const float *sval,
-                                  const float *W, const float *H, float *P, int64_t M, int64_t N, int K, int sm_count,
-                                  int *dev_status, cudaStream_t stream);
+cudaError_t launch_dense_cells_tc(const DensePlan &d, const float *sval, const float *W, const float *H, float *P, int64_t M, int64_t N,
+                                  int K, int sm_count, int *dev_status, cudaStream_t stream);
 
 // SpMM (W null) / fused SDDMM->SpMM (spmm.cu): device arrays, input order.  scratch: spmm_scratch_floats() floats for
 // partial rows, the first spmm_counter_floats() of them zeroed once (every call leaves them zero); clock as in launch_gather.  K a multiple of 4, at most 1024 (spmm_supports).

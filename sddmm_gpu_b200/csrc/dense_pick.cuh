@@ -9,9 +9,9 @@
 
 namespace sddmm {
 
-template <int NT = 256>
+template <int NT = 256>  // divides a quarter of the cell's entries
 __device__ __forceinline__ void pick_block(const float *Ct, int stride, const DenseCell &dc, bool masked, int64_t cell,
-                                           int tid, const int32_t *__restrict__ idx, const uint16_t *__restrict__ rc,
+                                           int tid, const int32_t *__restrict__ table,
                                            const unsigned long long *__restrict__ row_mask,
                                            const int2 *__restrict__ row_base, const uint32_t *__restrict__ row_span, const float *__restrict__ sval,
                                            float *__restrict__ P)
@@ -58,33 +58,22 @@ __device__ __forceinline__ void pick_block(const float *Ct, int stride, const De
             }
         }
     } else {
-        // per-nonzero lists: input index and (row, column) inside the cell
-        const int32_t *cidx = idx + dc.offset;
-        const uint16_t *crc = rc + dc.offset;
-        int i = tid;
-        for (; i + 3 * NT < dc.count; i += 4 * NT) {  // four independent nonzeros per thread and trip
-            unsigned code[4];
+        // table form: the input position of every entry
+        const int32_t *t = table + dc.slot * (DENSE_CELL_ROWS * DENSE_CELL_COLS);
+        for (int i = tid; i < DENSE_CELL_ROWS * DENSE_CELL_COLS; i += 4 * NT) {  // four independent entries per thread and trip
             int32_t o[4];
             float v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                code[u] = __ldcs(crc + i + u * NT);
-                o[u] = __ldcs(cidx + i + u * NT);
-            }
+            for (int u = 0; u < 4; ++u) o[u] = __ldg(t + i + u * NT);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                v[u] = Ct[(code[u] >> 8) * stride + (code[u] & 255u)];
-                if (sval) v[u] *= __ldg(sval + o[u]);
+                const int e = i + u * NT;
+                v[u] = Ct[e / DENSE_CELL_COLS * stride + e % DENSE_CELL_COLS];
+                if (sval && o[u] >= 0) v[u] *= __ldg(sval + o[u]);
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) P[o[u]] = v[u];
-        }
-        for (; i < dc.count; i += NT) {
-            const unsigned code = crc[i];
-            const int32_t o = cidx[i];
-            float v = Ct[(code >> 8) * stride + (code & 255u)];
-            if (sval) v *= __ldg(sval + o);
-            P[o] = v;
+            for (int u = 0; u < 4; ++u)
+                if (o[u] >= 0) P[o[u]] = v[u];
         }
     }
 }

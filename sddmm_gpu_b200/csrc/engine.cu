@@ -655,8 +655,8 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
             PLAN_TRY(build_plan_row_ptr(p, s));
             PLAN_TRY(build_dense_cells(p->d_rows, p->d_cols, p->d_row_ptr, nnz, M, N, DENSE_MIN_FILL, DENSE_MIN_SHARE, &p->dense, s));
             if (p->dense.n_cells > 0)
-                p->device_bytes += (int64_t)(sizeof(DenseCell) * p->dense.n_cells + 6 * p->dense.n_dense_nnz + 17 * DENSE_CELL_ROWS * p->dense.n_cells +
-                                             12 * p->dense.n_sparse);
+                p->device_bytes += (int64_t)((sizeof(DenseCell) + 20 * DENSE_CELL_ROWS) * p->dense.n_cells + sizeof(DenseUnit) * p->dense.n_units +
+                                             sizeof(int32_t) * DENSE_CELL_ROWS * DENSE_CELL_COLS * p->dense.n_table_cells + 12 * p->dense.n_sparse);
         }
     }
     // Hub-column marks are for the ring kernel: now if it will run by default, else if it is forced.
@@ -936,15 +936,9 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             p->last_kernel = names[h->dense_mode][p->dense.n_sparse == 0 ? 0 : rows_on_ring(p, false) ? 2 : 1];
         }
         if (h->dense_mode == 2)
-            LAUNCH_TRY(h, launch_dense_cells_tc(p->dense.cells, p->dense.n_cells, p->dense.idx, p->dense.rc, p->dense.row_mask,
-                                              p->dense.row_base, p->dense.row_span, p->dense.dense_rows, p->dense.n_dense_rows,
-                                              p->dense.dense_cols, p->dense.n_dense_cols, dS, dW, dH, dP, p->M, p->N, p->K,
-                                              h->sm_count, h->d_status, s));
+            LAUNCH_TRY(h, launch_dense_cells_tc(p->dense, dS, dW, dH, dP, p->M, p->N, p->K, h->sm_count, h->d_status, s));
         else
-            LAUNCH_TRY(h, launch_dense_cells(p->dense.cells, p->dense.n_cells, p->dense.idx, p->dense.rc, p->dense.row_mask,
-                                           p->dense.row_base, p->dense.row_span, p->dense.dense_rows, p->dense.n_dense_rows,
-                                           p->dense.dense_cols, p->dense.n_dense_cols, dS, dW, dH, dP, p->M, p->N, p->K,
-                                           h->dense_mode == 1, h->sm_count, s));
+            LAUNCH_TRY(h, launch_dense_cells(p->dense, dS, dW, dH, dP, p->M, p->N, p->K, h->dense_mode == 1, h->sm_count, s));
         // the remainder runs beside the cells (other entries of P; 12 us of 180 on a 65,536-token mask when it ran after them)
         if (p->dense.n_sparse > 0)
             LAUNCH_TRY(h, launch_rows(p, p->dense.rows_s, p->dense.cols_s, p->dense.perm_s, dS, dW, dH, dP, 0, p->dense.n_sparse,

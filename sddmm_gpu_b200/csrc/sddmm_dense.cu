@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "binning.cuh"
 #include "common.cuh"
 #include "dense_pick.cuh"
 
@@ -81,8 +82,8 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
 // TENSOR = true : 3xTF32 on the tensor cores (mma.sync m16n8k8), warp tile 32 x 32.
 template <bool TENSOR>
 __global__ void __launch_bounds__(256, 3)
-sddmm_dense_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, const int32_t *__restrict__ idx,
-                   const uint16_t *__restrict__ rc, const unsigned long long *__restrict__ row_mask,
+sddmm_dense_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, const int32_t *__restrict__ table,
+                   const unsigned long long *__restrict__ row_mask,
                    const int2 *__restrict__ row_base, const uint32_t *__restrict__ row_span, const int32_t *__restrict__ dense_rows, int64_t n_dense_rows,
                    const int32_t *__restrict__ dense_cols, int64_t n_dense_cols, const float *__restrict__ sval,
                    const float *__restrict__ W, const float *__restrict__ H, float *__restrict__ P, int64_t M,
@@ -102,7 +103,7 @@ sddmm_dense_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, const i
 
     for (int64_t cell = blockIdx.x; cell < n_cells; cell += gridDim.x) {
         DenseCell dc = cells[cell];
-        const bool masked = (dc.cls & CELL_MASKED) != 0;  // row-mask form: no per-nonzero list
+        const bool masked = (dc.cls & CELL_MASKED) != 0;  // row-mask form, else table form
         dc.cls &= 0xff;
         float acc[8][4];  // FMA path: [row i][col j]; tensor path: [m-tile*4 + n-tile][fragment register]
 #pragma unroll
@@ -207,19 +208,17 @@ sddmm_dense_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, const i
                 for (int j = 0; j < 4; ++j) Ct[(ty + 16 * i) * CT_STRIDE + tx + 16 * j] = acc[i][j];
         }
         __syncthreads();
-        pick_block(Ct, CT_STRIDE, dc, masked, cell, tid, idx, rc, row_mask, row_base, row_span, sval, P);
+        pick_block(Ct, CT_STRIDE, dc, masked, cell, tid, table, row_mask, row_base, row_span, sval, P);
         __syncthreads();  // the block is overwritten by the next cell's staging
     }
 }
 
 }  // namespace
 
-cudaError_t launch_dense_cells(const DenseCell *cells, int64_t n_cells, const int32_t *idx, const uint16_t *rc,
-                               const unsigned long long *row_mask, const int2 *row_base, const uint32_t *row_span, const int32_t *dense_rows, int64_t n_dense_rows, const int32_t *dense_cols,
-                               int64_t n_dense_cols, const float *sval, const float *W, const float *H, float *P,
+cudaError_t launch_dense_cells(const DensePlan &d, const float *sval, const float *W, const float *H, float *P,
                                int64_t M, int64_t N, int K, bool tensor, int sm_count, cudaStream_t stream)
 {
-    if (n_cells == 0) return cudaSuccess;
+    if (d.n_cells == 0) return cudaSuccess;
     const size_t smem = sizeof(float) * SMEM_FLOATS;
     static SmemOptinCache optin_fma, optin_tensor;  // per device
     {
@@ -228,15 +227,10 @@ cudaError_t launch_dense_cells(const DenseCell *cells, int64_t n_cells, const in
         if (e != cudaSuccess) return e;
     }
     int64_t blocks = (int64_t)sm_count * 3;
-    if (blocks > n_cells) blocks = n_cells;
-    if (tensor)
-        sddmm_dense_kernel<true><<<(unsigned)blocks, 256, smem, stream>>>(cells, n_cells, idx, rc, row_mask, row_base, row_span,
-                                                                          dense_rows, n_dense_rows, dense_cols,
-                                                                          n_dense_cols, sval, W, H, P, M, N, K);
-    else
-        sddmm_dense_kernel<false><<<(unsigned)blocks, 256, smem, stream>>>(cells, n_cells, idx, rc, row_mask, row_base, row_span,
-                                                                           dense_rows, n_dense_rows, dense_cols,
-                                                                           n_dense_cols, sval, W, H, P, M, N, K);
+    if (blocks > d.n_cells) blocks = d.n_cells;
+    auto kern = tensor ? sddmm_dense_kernel<true> : sddmm_dense_kernel<false>;
+    kern<<<(unsigned)blocks, 256, smem, stream>>>(d.cells, d.n_cells, d.table, d.row_mask, d.row_base, d.row_span, d.dense_rows,
+                                                  d.n_dense_rows, d.dense_cols, d.n_dense_cols, sval, W, H, P, M, N, K);
     return cudaGetLastError();
 }
 

@@ -54,6 +54,31 @@ def test_dense_cells_at_small_sizes(monkeypatch, K, mode, M, half_width, n_globa
     h.close()
 
 
+@pytest.mark.parametrize("mode", ["2", "1", "0"])
+@pytest.mark.parametrize("M,N,fill", [(128, 64, 1.0), (200, 64 * 3, 0.5), (390, 64 * 5 + 3, 0.3), (1300, 64, 0.9)])
+def test_cells_with_several_nonzeros_in_one_place(monkeypatch, mode, M, N, fill):
+    # one cell, an odd number of cells in a row of cells (a unit of one), units of rows that end in the cell; and rows in which some
+    # columns come twice or three times: of those a cell holds one, the others are in the remainder
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")
+    monkeypatch.setenv("SDDMM_DENSE_TENSOR", mode)
+    h = api.Handle(0)
+    rng = np.random.default_rng(M)
+    K = 72
+    W, H = (rng.standard_normal((n, K)).astype(np.float32) for n in (M, N))
+    cells = rng.random((M, N)) < fill
+    for extra in (0, M // 2):
+        rows, cols = np.nonzero(cells)
+        again = rng.integers(0, rows.size, extra)
+        again = np.concatenate([again, again[: extra // 3]])
+        rows, cols = np.concatenate([rows, rows[again]]), np.concatenate([cols, cols[again]])
+        order = np.lexsort((cols, rows))
+        rows, cols = rows[order].astype(np.int32), cols[order].astype(np.int32)
+        vals = rng.standard_normal(rows.size).astype(np.float32)
+        name, info = _run(h, dict(M=M, N=N, W=W, H=H), rows, cols, vals)
+        assert name.startswith("dense") and 0 < info.n_dense_nnz <= rows.size - again.size
+    h.close()
+
+
 @pytest.mark.parametrize("K,half_width,n_global", [(64, 96, 6), (100, 40, 60), (512, 70, 3)])
 def test_remainder_beside_the_cells(engine, K, half_width, n_global):
     # the remainder runs beside the dense cells: what follows on the stream sees all of P, and the next call overwrites it
