@@ -95,13 +95,20 @@ PanelConfig choose_panel_config(int K, int panel_rows_hint, int sm_count, size_t
 // Gather kernel (sddmm_gather.cu): any K % 4 == 0, no plan data needed; the default path.  perm as in launch_panel.
 // clock: two device words that receive the kernel's start and end (clock_begin / clock_end), or null.
 // beside (with perm only): may run beside the kernel before it in the stream, once that has signalled it; it ends no earlier.
+// passes: the columns of W and H that a launch multiplies (without perm; with it there is one).  Every pass but the first adds to P.
+struct GatherPasses {
+    int n, floats;  // launches, columns of each (the last one may have fewer)
+};
+// What is best for an H of N rows; one pass where S values and P share memory.
+GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, const float *P);
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
-                          const float *W, const float *H, float *P, int64_t nnz, int K, int sm_count,
+                          const float *W, const float *H, float *P, int64_t nnz, int K, GatherPasses passes, int sm_count,
                           unsigned long long *clock, cudaStream_t stream, bool beside = false);
 // The same over operands stored in bfloat16 (rows of 2K bytes): K = 256, 512 or 1024.
 bool gather_bf16_supports(int K);
+GatherPasses gather_passes_bf16(int64_t nnz, int64_t N, int K, const float *sval, const float *P);
 cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                               const void *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream);
+                               const void *H, float *P, int64_t nnz, int64_t N, int K, int sm_count, unsigned long long *clock, cudaStream_t stream);
 
 // Row-panel kernel: persistent CTAs walk the work items; the W rows an item
 // touches (item_rows lists them) are staged into shared memory with bulk

@@ -393,9 +393,9 @@ cudaError_t ensure_hints(sddmm_plan_s *p)
 
 namespace sddmm {
 
-bool rows_on_ring(const sddmm_plan_s *p, bool force_ring)
+bool rows_on_ring(const sddmm_plan_s *p, bool force_ring, bool permuted)
 {
-    return ring_supports(p->K) && (force_ring || ring_preferred(p->N, p->K));
+    return ring_supports(p->K) && (force_ring || (permuted && ring_preferred(p->N, p->K)));
 }
 
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
@@ -411,13 +411,15 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
         P += first;
         if (sval) sval += first;
     }
-    if (rows_on_ring(p, force_ring)) {
+    if (rows_on_ring(p, force_ring, perm != nullptr)) {
         // the marks are in the plan's processing order: not for the dense-cell remainder
         const bool hinted = p->d_cols_hint && cols == (p->d_perm ? p->d_cols_t : p->d_cols);
         return launch_ring(rows, (hinted ? p->d_cols_hint : cols) + first, perm, sval, W, H, P, count, p->K, hinted, h->sm_count,
                            h->d_work_counter, h->d_status, stream);
     }
-    return launch_gather(rows, cols + first, perm, sval, W, H, P, count, p->K, h->sm_count, clock, stream, beside);
+    const GatherPasses passes = gather_passes(count, p->N, p->K, sval, P);
+    if (!perm) h->n_launches += passes.n - 1;
+    return launch_gather(rows, cols + first, perm, sval, W, H, P, count, p->K, passes, h->sm_count, clock, stream, beside);
 }
 
 }  // namespace sddmm
@@ -665,7 +667,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
         int64_t budget_mb = 64;  // best of a 16..128 MB sweep on the scale-22 R-MAT matrix at K = 256
         if (const char *env = std::getenv("SDDMM_L2_HUB_MB")) budget_mb = std::atoll(env);
         p->hub_budget = budget_mb > 0 ? budget_mb * (1ll << 20) : 0;
-        if (ring_preferred(N, K)) {
+        if (p->d_perm && ring_preferred(N, K)) {
             PLAN_TRY(begin_more());
             PLAN_TRY(build_hints(p, s));
         }
@@ -729,7 +731,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     mark_pending(p, async, s);
 
     if (flags & SDDMM_FLAG_OPERANDS_BF16) {
-        // W and H hold bfloat16: the TMA rings over rows of 2K bytes, products and sums in fp32.  Opt-in and
+        // W and H hold bfloat16: rows of 2K bytes, products and sums in fp32.  Opt-in and
         // outside the fp32 tolerance contract; device arrays only, no other layout or kernel flag.
         if (!ring_bf16_supports(p->K)) return SDDMM_K_UNSUPPORTED;
         if (!all_dev || (flags & ~(uint32_t)(SDDMM_FLAG_OPERANDS_BF16 | SDDMM_FLAG_ASYNC | SDDMM_FLAG_KERNEL_RING))) {
@@ -744,14 +746,16 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         const int32_t *rows_p = tiled ? p->d_rows_t : p->d_rows, *cols_p = tiled ? p->d_cols_t : p->d_cols;
         const int32_t *perm_p = tiled ? p->d_perm : nullptr;
         // rows of half the bytes: the same line between the two kernels as for fp32 rows of K / 2
-        const bool gather = gather_bf16_supports(p->K) && !(flags & SDDMM_FLAG_KERNEL_RING) && !ring_preferred(p->N / 2, p->K);
+        const bool gather = gather_bf16_supports(p->K) && !(flags & SDDMM_FLAG_KERNEL_RING) && !(tiled && ring_preferred(p->N / 2, p->K));
+        const int passes = gather && !tiled ? gather_passes_bf16(p->nnz, p->N, p->K, Sval, P).n : 1;
         if (!gather) CUDA_TRY(h, ensure_hints(p));
         p->last_kernel = gather ? "gather (bf16 operands)" : "ring (bf16 operands)";
         p->last_h2d_bytes = p->last_d2h_bytes = 0;
         CallTimer timer(p, async);
-        CUDA_TRY(h, timer.begin(gather, s));
+        CUDA_TRY(h, timer.begin(gather && passes == 1, s));
+        h->n_launches += passes - 1;
         if (gather)
-            LAUNCH_TRY(h, launch_gather_bf16(rows_p, cols_p, perm_p, Sval, W, H, P, p->nnz, p->K, h->sm_count, timer.clk, s));
+            LAUNCH_TRY(h, launch_gather_bf16(rows_p, cols_p, perm_p, Sval, W, H, P, p->nnz, p->N, p->K, h->sm_count, timer.clk, s));
         else
             LAUNCH_TRY(h, launch_ring_bf16(rows_p, p->d_cols_hint ? p->d_cols_hint : cols_p, perm_p, Sval, W, H, P, p->nnz, p->K,
                                            p->d_cols_hint != nullptr, h->sm_count, h->d_work_counter, h->d_status, s));
@@ -855,7 +859,8 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     }
     const bool use_dense = !forced && !tiled_out && p->dense.n_cells > 0;
     // a call that is one gather launch is timed by the kernel itself, everything else by events
-    const bool one_gather = !use_dense && !use_panel && (use_gather || !rows_on_ring(p, use_ring));
+    const bool one_gather = !use_dense && !use_panel && (use_gather || !rows_on_ring(p, use_ring, p->d_perm && !tiled_out)) &&
+                            (p->d_perm || use_gather || gather_passes(p->nnz, p->N, p->K, dS, P).n == 1);
     bool p_copy = false;
     if (!p_dev) {
         // a small P is written to mapped host memory by the kernel: its 32-byte stores over PCIe cost less than a copy
@@ -874,7 +879,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     if (use_panel) CUDA_TRY(h, ensure_items(p));
     if (use_ring && ring_supports(p->K)) CUDA_TRY(h, ensure_hints(p));
     if (pipelined) {
-        p->last_kernel = rows_on_ring(p, use_ring) ? "ring (pipelined chunks)" : "gather (pipelined chunks)";
+        p->last_kernel = rows_on_ring(p, use_ring, false) ? "ring (pipelined chunks)" : "gather (pipelined chunks)";
         CUDA_TRY(h, ensure_pipeline(h));
         {
             std::lock_guard<std::mutex> hold(h->owners);
@@ -933,7 +938,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             static const char *const names[3][3] = {{"dense_fma", "dense_fma+gather", "dense_fma+ring"},
                                                     {"dense_mma_sync", "dense_mma_sync+gather", "dense_mma_sync+ring"},
                                                     {"dense_tc", "dense_tc+gather", "dense_tc+ring"}};
-            p->last_kernel = names[h->dense_mode][p->dense.n_sparse == 0 ? 0 : rows_on_ring(p, false) ? 2 : 1];
+            p->last_kernel = names[h->dense_mode][p->dense.n_sparse == 0 ? 0 : rows_on_ring(p, false, true) ? 2 : 1];
         }
         if (h->dense_mode == 2)
             LAUNCH_TRY(h, launch_dense_cells_tc(p->dense, dS, dW, dH, dP, p->M, p->N, p->K, h->sm_count, h->d_status, s));
@@ -945,7 +950,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
                                       false, nullptr, s, h->dense_mode == 2));
     } else if (use_gather) {
         p->last_kernel = "gather";
-        LAUNCH_TRY(h, launch_gather(p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, p->nnz, p->K, h->sm_count, timer.clk, s));
+        LAUNCH_TRY(h, launch_gather(p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, p->nnz, p->K, {1, p->K}, h->sm_count, timer.clk, s));
     } else {
         const bool tiled = p->d_perm != nullptr;
         const int32_t *rows_p = tiled ? p->d_rows_t : p->d_rows;
@@ -959,7 +964,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             h->last_error = "SDDMM_FLAG_TILED_ORDER with S values is not supported on a multi-tile plan";
             return SDDMM_INVALID_ARG;
         }
-        p->last_kernel = use_panel ? "panel" : rows_on_ring(p, use_ring) ? "ring" : "gather";
+        p->last_kernel = use_panel ? "panel" : rows_on_ring(p, use_ring, perm != nullptr) ? "ring" : "gather";
         if (use_panel)
             LAUNCH_TRY(h, launch_panel(p->d_items, p->n_items, p->d_item_rows, rows_p, cols_p, perm, dS, dW, dH, dP, p->K,
                                      p->cfg, h->sm_count, h->d_status, s));
@@ -1340,7 +1345,7 @@ int sddmm_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const int32_t
         dp = (float *)tmp.p[5];
     }
     CUDA_TRY(h, launch_gather((const int32_t *)dr, (const int32_t *)dc, nullptr, (const float *)ds, (const float *)dw,
-                              (const float *)dh, dp, nnz, K, h->sm_count, nullptr, s));
+                              (const float *)dh, dp, nnz, K, gather_passes(nnz, N, K, (const float *)ds, dp), h->sm_count, nullptr, s));
     if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dp, sizeof(float) * nnz, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
     return SDDMM_OK;

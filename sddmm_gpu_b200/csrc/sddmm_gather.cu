@@ -90,20 +90,24 @@ struct WShare {
     }
 };
 
-// pieces: 16-byte pieces of a row.  run_len: nonzeros of a set, a multiple of S::NB.  perm (HAS_PERM): the result of
-// nonzero j goes to P[perm[j]] and is scaled by sval[perm[j]].
-template <class S, bool HAS_PERM>
+// What becomes of a dot product: stored (STORE); stored through perm, the result of nonzero j to P[perm[j]], scaled by
+// sval[perm[j]] (PERM); or added to what P holds, the product over earlier columns of the operands (ADD): by a reduction that
+// nothing waits for, or, with `finish`, read, added and scaled.
+enum GatherMode { STORE, PERM, ADD };
+
+// pieces: 16-byte pieces of a row that are multiplied.  row_bytes: from one row to the next.  run_len: nonzeros of a set, a multiple of S::NB.
+template <class S, GatherMode MODE>
 __global__ void __launch_bounds__(GA_TPB, S::CTAS)
 sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
                     const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
-                    float *__restrict__ P, unsigned nnz, int pieces, unsigned run_len, unsigned long long *clock, unsigned meet_from)
+                    float *__restrict__ P, unsigned nnz, int pieces, unsigned row_bytes, bool finish, unsigned run_len, unsigned long long *clock, unsigned meet_from)
 {
     clock_begin(clock);
+    constexpr bool HAS_PERM = MODE == PERM;
     constexpr int L = S::L, F = S::F, B = S::B, RB = S::RB, NB = S::NB, G = S::G;
     const int lane = threadIdx.x & 31, lig = lane & (L - 1), set = lane / L;
     const unsigned warp0 = gather_warp(blockIdx.x, blockDim.x, threadIdx.x) * (G * run_len);  // first nonzero of this warp
     if (warp0 >= nnz) return;
-    const unsigned row_bytes = (unsigned)pieces * 16u;
     const char *H_lane = H + lig * 16, *W_lane = W + lig * 16;
     const bool last_ok = S::EXACT || lig + (F - 1) * L < pieces;
     unsigned setmask = 0;  // lane 0 of every set
@@ -145,10 +149,13 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
             if (lig == 0) b2 = cur;
             if (rn != b2 && lig < NB) {
                 const char *wp = W + (size_t)(unsigned)rn * row_bytes;
-                for (unsigned o = 0; o < row_bytes; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(wp + o));
+                for (unsigned o = 0; o < (unsigned)pieces * 16u; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(wp + o));
             }
         }
         if (HAS_PERM && sval) s = __ldg(sval + dst);
+        float sum = 0.f;
+        // (volatile: it is to be under way while the rows of H are, not waited for at the end of the step)
+        if (MODE == ADD && finish && lig < NB) asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(sum) : "l"(P + at(j)));
         float res = 0.f;
 #pragma unroll
         for (int h0 = 0; h0 < NB; h0 += RB) {
@@ -180,7 +187,8 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
             if (RB == NB || il / RB == h0 / RB) res = t;
         }
         if (lig < NB && j < nnz) {
-            P[HAS_PERM ? (unsigned)dst : j] = res * s;
+            if (MODE == ADD && !finish) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(P + j), "f"(res) : "memory");
+            else P[HAS_PERM ? (unsigned)dst : j] = (MODE == ADD ? sum + res : res) * s;
         }
         j += NB;
         r = rn;
@@ -239,93 +247,149 @@ sddmm_gather_long_kernel(const int32_t *__restrict__ rows, const int32_t *__rest
     clock_end(clock, meet_from);
 }
 
-template <class S, bool HAS_PERM>
-cudaError_t launch_shape_p(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                           const void *H, float *P, unsigned nnz, int pieces, int sm_count, unsigned long long *clock, bool beside,
-                           cudaStream_t stream)
+struct GatherCall {
+    const int32_t *rows, *cols, *perm;
+    const float *sval;
+    const char *W, *H;
+    float *P;
+    unsigned nnz;
+    int pieces;
+    unsigned row_bytes;
+    bool add, finish;  // to P (perm null), and for the last time
+    int sm_count;
+    unsigned long long *clock;
+    bool beside;
+    cudaStream_t stream;
+};
+
+template <class S, GatherMode MODE>
+cudaError_t launch_mode(const GatherCall &c)
 {
     // only the last piece of a lane is predicated: the ones before it have to lie inside the row
-    if (pieces > S::L * S::F || pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
+    if (c.pieces > S::L * S::F || c.pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
     // A set's share: 16 nonzeros (32 when a warp is one or two sets), less when the warps would not fill the SMs.
     constexpr unsigned most = S::L >= 16 ? 32 : 16;
-    const unsigned resident = (unsigned)sm_count * S::CTAS * (GA_TPB / 32) * S::G;  // sets
-    unsigned run = nnz / resident / S::NB * S::NB;
+    const unsigned resident = (unsigned)c.sm_count * S::CTAS * (GA_TPB / 32) * S::G;  // sets
+    unsigned run = c.nnz / resident / S::NB * S::NB;
     run = run < (unsigned)S::NB ? (unsigned)S::NB : run > most ? most : run;
-    const unsigned tpb = beside ? GA_TPB_BESIDE : GA_TPB, per_block = run * S::G * (tpb / 32);
-    const unsigned blocks = (unsigned)(((uint64_t)nnz + per_block - 1) / per_block);
-    const unsigned meet_from = last_wave(blocks, (unsigned)sm_count * S::CTAS);
-    if (HAS_PERM && beside) {
-        cudaLaunchAttribute attr = {};
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(tpb);
-        cfg.stream = stream;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, sddmm_gather_kernel<S, HAS_PERM>, rows, cols, perm, sval, static_cast<const char *>(W),
-                                  static_cast<const char *>(H), P, nnz, pieces, run, clock, meet_from);
-    }
-    sddmm_gather_kernel<S, HAS_PERM><<<blocks, GA_TPB, 0, stream>>>(rows, cols, perm, sval, static_cast<const char *>(W),
-                                                                    static_cast<const char *>(H), P, nnz, pieces, run, clock, meet_from);
-    return cudaGetLastError();
+    const unsigned tpb = c.beside ? GA_TPB_BESIDE : GA_TPB, per_block = run * S::G * (tpb / 32);
+    const unsigned blocks = (unsigned)(((uint64_t)c.nnz + per_block - 1) / per_block);
+    const unsigned meet_from = last_wave(blocks, (unsigned)c.sm_count * S::CTAS);
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(tpb);
+    cfg.stream = c.stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = c.beside ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, sddmm_gather_kernel<S, MODE>, c.rows, c.cols, c.perm, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.row_bytes,
+                              c.finish, run, c.clock, meet_from);
 }
 
 template <class S>
-cudaError_t launch_shape(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                         const void *H, float *P, unsigned nnz, int pieces, int sm_count, unsigned long long *clock, bool beside,
-                         cudaStream_t stream)
+cudaError_t launch_shape(const GatherCall &c)
 {
-    return perm ? launch_shape_p<S, true>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, clock, beside, stream)
-                : launch_shape_p<S, false>(rows, cols, perm, sval, W, H, P, nnz, pieces, sm_count, clock, false, stream);
+    return c.perm ? launch_mode<S, PERM>(c) : c.add ? launch_mode<S, ADD>(c) : launch_mode<S, STORE>(c);
+}
+
+// The shape for `pieces` pieces of a row: L * (F - 1) < pieces <= L * F, L small enough that a set's lanes
+// are busy and large enough that F pieces of W and B * F of H stay in few registers.  Every line is the best of a sweep
+// over (L, B, RB, prefetch, resident blocks) at a K of its range on the matrices named at the top of this file.
+cudaError_t launch_pieces(const GatherCall &c)
+{
+    const int q = c.pieces;
+#define GA_GO(L, F, B, RB, EXACT, PF, CTAS) return launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS>>(c)
+    if (q <= 4) GA_GO(4, 1, 4, 4, false, false, 6);
+    if (q < 8) GA_GO(8, 1, 4, 4, false, false, 6);
+    if (q == 8) GA_GO(8, 1, 4, 4, true, false, 6);
+    if (q <= 12) GA_GO(4, 3, 2, 4, false, true, 4);
+    if (q < 16) GA_GO(8, 2, 4, 4, false, true, 4);
+    if (q == 16) GA_GO(8, 2, 4, 4, true, true, 4);
+    if (q <= 24) GA_GO(8, 3, 2, 8, false, true, 4);
+    if (q < 32) GA_GO(16, 2, 2, 8, false, true, 5);
+    if (q == 32) GA_GO(16, 2, 2, 8, true, false, 5);
+    if (q <= 48) GA_GO(16, 3, 2, 8, false, true, 4);
+    if (q < 64) GA_GO(16, 4, 1, 8, false, true, 4);
+    if (q == 64) GA_GO(32, 2, 2, 8, true, false, 5);
+    if (q <= 80) GA_GO(16, 5, 1, 8, false, true, 4);
+    if (q <= 96) GA_GO(16, 6, 1, 8, false, false, 4);
+    if (q < 128) GA_GO(32, 4, 2, 8, false, true, 3);
+    if (q == 128) GA_GO(32, 4, 2, 8, true, true, 3);
+    if (q <= 160) GA_GO(32, 5, 1, 8, false, false, 4);
+    if (q <= 192) GA_GO(32, 6, 1, 8, false, false, 4);
+    if (q <= 224) GA_GO(32, 7, 1, 8, false, false, 3);
+    if (q <= 256) GA_GO(32, 8, 1, 8, false, false, 3);
+#undef GA_GO
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-// The shape for a row of K floats: L * (F - 1) < K / 4 <= L * F, L small enough that a set's lanes
-// are busy and large enough that F pieces of W and B * F of H stay in few registers.  Every line is the best of a sweep
-// over (L, B, RB, prefetch, resident blocks) at a K of its range on the matrices named at the top of this file.
-cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const float *W,
-                          const float *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream, bool beside)
+// Long rows in passes over their columns.  A pass multiplies `floats` columns of every row; its part of H is so much smaller that more
+// of the gathers hit L2, and it runs on one of the shapes that take few registers.  Against that a pass costs the indices again and a
+// sum in P that is written and read: 16 bytes a nonzero.  Sustained us, one pass -> passes of 64 / 96 / 192 (R-MAT unless said):
+//   K = 256: 4.2 M rows of H, 97 M nonzeros 9330 (the ring kernel) -> 8340 / - / -, another GPU 8922 (one pass of this kernel) -> 8552 /
+//   8669 / 8877; 50 M nonzeros 4740 -> 4676 / 4687 / 4757; 25 M 2421 -> 2514 / 2448 / 2502; 3 M rows, 36 M 3078 -> 3168 / 3111 / 3127;
+//   1.5 M rows, 18 M 1409 -> 1532 / 1438 / 1454; K = 300, 1.5 M rows 1803 -> 2163 / 2016 / 1904
+//   K = 384: 20 K rows 44 -> 74 / 63 / 47; 300 K 515 -> 587 / 506 / 494; 1.5 M 2578 -> 2224 / 2112 / 2114; 4.2 M 16233 -> 13008 / 12806 / 13466
+//   K = 512: 300 K rows 607 -> 773 / 666 / 635; 700 K 1245 -> 1381 / 1253 / 1214; 1.5 M 3052 -> 3053 / 2894 / 2830
+//   K = 768: 100 K rows, 1.2 M nonzeros 255 -> 392 / 295 / 255; 200 K, uniform, 2 M 972 -> 712 / 646 / 770; 150 K, uniform, 0.3 M 197 -> 228
+//   / 190 / 217; 700 K, 8.4 M 2356 -> 2081 / 1836 / 1822; 1.5 M, 18 M 5688 -> 4545 / 4267 / 4212
+//   K = 1028: 20 K rows, 0.24 M 105 -> 205 / 143 / 134; 100 K, 1.2 M 548 -> 551 / 426 / 384; 1 M, 12 M 6685 -> 4807 / 4261 / 4189
+GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, const float *P)
 {
-    for (int64_t j0 = 0; j0 < nnz; j0 += GATHER_SLICE) {
-        const unsigned n = (unsigned)(nnz - j0 < GATHER_SLICE ? nnz - j0 : GATHER_SLICE);
-        const int32_t *r = rows + j0, *c = cols + j0, *p = perm ? perm + j0 : nullptr;
-        const float *s = sval && !perm ? sval + j0 : sval;
-        float *out = perm ? P : P + j0;
-        const int q = K / 4;
-        cudaError_t e;
-#define GA_GO(L, F, B, RB, EXACT, PF, CTAS) \
-    e = launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS>>(r, c, p, s, W, H, out, n, q, sm_count, clock, beside && j0 == 0, stream)
-        if (q <= 4) GA_GO(4, 1, 4, 4, false, false, 6);
-        else if (q < 8) GA_GO(8, 1, 4, 4, false, false, 6);
-        else if (q == 8) GA_GO(8, 1, 4, 4, true, false, 6);
-        else if (q <= 12) GA_GO(4, 3, 2, 4, false, true, 4);
-        else if (q < 16) GA_GO(8, 2, 4, 4, false, true, 4);
-        else if (q == 16) GA_GO(8, 2, 4, 4, true, true, 4);
-        else if (q <= 24) GA_GO(8, 3, 2, 8, false, true, 4);
-        else if (q < 32) GA_GO(16, 2, 2, 8, false, true, 5);
-        else if (q == 32) GA_GO(16, 2, 2, 8, true, false, 5);
-        else if (q <= 48) GA_GO(16, 3, 2, 8, false, true, 4);
-        else if (q < 64) GA_GO(16, 4, 1, 8, false, true, 4);
-        else if (q == 64) GA_GO(32, 2, 2, 8, true, false, 5);
-        else if (q <= 80) GA_GO(16, 5, 1, 8, false, true, 4);
-        else if (q <= 96) GA_GO(16, 6, 1, 8, false, false, 4);
-        else if (q < 128) GA_GO(32, 4, 2, 8, false, true, 3);
-        else if (q == 128) GA_GO(32, 4, 2, 8, true, true, 3);
-        else if (q <= 160) GA_GO(32, 5, 1, 8, false, false, 4);
-        else if (q <= 192) GA_GO(32, 6, 1, 8, false, false, 4);
-        else if (q <= 224) GA_GO(32, 7, 1, 8, false, false, 3);
-        else if (q <= 256) GA_GO(32, 8, 1, 8, false, false, 3);
-        else {
-            const unsigned blocks = gather_long_blocks(n), meet_from = last_wave(blocks, (unsigned)sm_count * 8);
-            if (p) sddmm_gather_long_kernel<true><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock, meet_from);
-            else sddmm_gather_long_kernel<false><<<blocks, GA_TPB, 0, stream>>>(r, c, p, s, (const char *)W, (const char *)H, out, n, q, clock, meet_from);
-            e = cudaGetLastError();
+    const GatherPasses whole = {1, K};
+    if (sval && sval < P + nnz && P < sval + nnz) return whole;  // the first pass would overwrite S values that the last one needs
+    const int64_t h_bytes = N * K * 4;
+    int floats = K;
+    if (K > 320) {
+        // (the shape for 512 floats is the one that holds its own longest)
+        if (nnz >= 1000000 && h_bytes >= (K > 480 && K <= 512 ? 1000000000 : 400000000)) floats = N > 2000000 ? 96 : 192;
+    } else if (K > 192 && h_bytes >= 4000000000 && nnz >= 16 * N) {
+        floats = 64;
+    }
+    return floats < K ? GatherPasses{(K + floats - 1) / floats, floats} : whole;
+}
+
+cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const float *W,
+                          const float *H, float *P, int64_t nnz, int K, GatherPasses passes, int sm_count, unsigned long long *clock,
+                          cudaStream_t stream, bool beside)
+{
+    if (perm) passes = {1, K};
+    for (int pass = 0; pass < passes.n; ++pass) {
+        const int k0 = pass * passes.floats, width = K - k0 < passes.floats ? K - k0 : passes.floats;
+        for (int64_t j0 = 0; j0 < nnz; j0 += GATHER_SLICE) {
+            GatherCall c;
+            c.nnz = (unsigned)(nnz - j0 < GATHER_SLICE ? nnz - j0 : GATHER_SLICE);
+            c.rows = rows + j0;
+            c.cols = cols + j0;
+            c.perm = perm ? perm + j0 : nullptr;
+            c.sval = sval && !perm ? sval + j0 : sval;
+            if (pass < passes.n - 1) c.sval = nullptr;  // the sum is scaled
+            c.W = reinterpret_cast<const char *>(W + k0);
+            c.H = reinterpret_cast<const char *>(H + k0);
+            c.P = perm ? P : P + j0;
+            c.pieces = width / 4;
+            c.row_bytes = (unsigned)K * 4u;
+            c.add = pass > 0;
+            c.finish = pass == passes.n - 1;
+            c.sm_count = sm_count;
+            c.clock = clock;
+            c.beside = beside && j0 == 0;
+            c.stream = stream;
+            cudaError_t e;
+            if (c.pieces <= 256) {
+                e = launch_pieces(c);
+            } else {
+                const unsigned blocks = gather_long_blocks(c.nnz), meet_from = last_wave(blocks, (unsigned)sm_count * 8);
+                if (perm) sddmm_gather_long_kernel<true><<<blocks, GA_TPB, 0, stream>>>(c.rows, c.cols, c.perm, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, clock, meet_from);
+                else sddmm_gather_long_kernel<false><<<blocks, GA_TPB, 0, stream>>>(c.rows, c.cols, c.perm, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, clock, meet_from);
+                e = cudaGetLastError();
+            }
+            if (e != cudaSuccess) return e;
         }
-#undef GA_GO
-        if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
@@ -334,21 +398,33 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
 // mixed-precision FMA (fewer registers: five resident blocks instead of four); K = 512: 1378 -> 1190.
 bool gather_bf16_supports(int K) { return K == 256 || K == 512 || K == 1024; }
 
+// Passes of 256 values, sustained us, the ring kernel / one pass / these: K = 1024, 0.3 M rows of H - / 544 / 583, 0.7 M 1394 / 1406 / 1405, 1 M 2775 / 2747 /
+// 2600, 1.5 M 4320 / 4466 / 4119;  K = 512, 1.5 M 2036 / 2047 / 2038, 4.2 M 9298 / 9264 / 8920;  K = 256, 4.2 M 4864 / 4218 / -.
+GatherPasses gather_passes_bf16(int64_t nnz, int64_t N, int K, const float *sval, const float *P)
+{
+    const GatherPasses whole = {1, K};
+    if (sval && sval < P + nnz && P < sval + nnz) return whole;
+    return N * K * 2 >= (K >= 1024 ? 1900000000 : 4000000000) && K > 256 ? GatherPasses{K / 256, 256} : whole;
+}
+
 cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,
-                               const void *H, float *P, int64_t nnz, int K, int sm_count, unsigned long long *clock, cudaStream_t stream)
+                               const void *H, float *P, int64_t nnz, int64_t N, int K, int sm_count, unsigned long long *clock, cudaStream_t stream)
 {
     if (nnz == 0) return cudaSuccess;
     if (nnz > INT32_MAX) return cudaErrorInvalidValue;  // plans hold fewer
-    const unsigned n = (unsigned)nnz;
-#define GA_GO(L, F, B, PF, CTAS) \
-    return launch_shape<GatherShape<L, F, B, 8, true, PF, CTAS, true>>(rows, cols, perm, sval, W, H, P, n, K / 8, sm_count, clock, false, stream)
-    switch (K) {
-    case 256: GA_GO(16, 2, 2, false, 5);
-    case 512: GA_GO(16, 4, 1, true, 4);
-    case 1024: GA_GO(32, 4, 2, true, 3);
-    default: return cudaErrorInvalidValue;
+    GatherPasses p = gather_passes_bf16(nnz, N, K, sval, P);
+    if (perm) p = {1, K};
+    for (int pass = 0; pass < p.n; ++pass) {
+        GatherCall c = {rows, cols, perm, pass < p.n - 1 ? nullptr : sval, static_cast<const char *>(W) + 2 * pass * p.floats,
+                        static_cast<const char *>(H) + 2 * pass * p.floats, P, (unsigned)nnz, p.floats / 8, (unsigned)K * 2u, pass > 0,
+                        pass == p.n - 1, sm_count, clock, false, stream};
+        cudaError_t e = cudaErrorInvalidValue;
+        if (p.floats == 256) e = launch_shape<GatherShape<16, 2, 2, 8, true, false, 5, true>>(c);
+        else if (p.floats == 512) e = launch_shape<GatherShape<16, 4, 1, 8, true, true, 4, true>>(c);
+        else if (p.floats == 1024) e = launch_shape<GatherShape<32, 4, 2, 8, true, true, 3, true>>(c);
+        if (e != cudaSuccess) return e;
     }
-#undef GA_GO
+    return cudaSuccess;
 }
 
 }  // namespace sddmm

@@ -27,9 +27,11 @@
 // memory, L1/L2) only when the row changes -- one group ahead, right after the
 // previous group's FMAs.
 //
-// Used for K = 256, 512 and 1024 (C = 2, 4, 8) when H is far larger than L2 (ring_preferred): there most gathers
-// come from DRAM, whose latency the deep rings hide better than the gather kernel's resident warps, and the copies
-// carry the plan's hub-column hints.  Everything else is the gather kernel's (sddmm_gather.cu).
+// Used for K = 256, 512 and 1024 (C = 2, 4, 8) where the nonzeros come through a permutation (column tiles, the buckets of a broadcast H) and H is
+// far larger than L2 (ring_preferred): there most gathers
+// come from DRAM, whose latency the deep rings hide, and the copies
+// carry the plan's hub-column hints; and for bfloat16 rows of K = 2048.  Everything else is the gather kernel's (sddmm_gather.cu), which
+// in its passes over part of the columns is ahead of the rings at every size (97 M nonzeros, 4.2 M rows of H, K = 256: 9330 -> 8340 us).
 #include <cuda_runtime.h>
 #include <stdint.h>
 

@@ -98,3 +98,50 @@ def test_kernel_time_covers_all_launches(engine, monkeypatch):
     monkeypatch.setenv("SDDMM_DENSE_CELLS", "0")
     ms, around = _all_of_P(engine, 512, 509, (1 << 30) + 54321, 4)
     assert 0.9 * around <= ms <= around
+
+
+@pytest.mark.parametrize("K,N,bf16", [(324, 310_000, False), (388, 2_100_000, False), (512, 489_000, False), (772, 131_000, False),
+                                      (1028, 98_000, False), (1024, 930_000, True)])
+def test_long_rows_in_passes(engine, K, N, bf16):
+    # large H, long rows: passes over part of the columns, the later ones adding to P.  The last pass narrower than the others, rows of
+    # one and of many nonzeros, a nonzero count that ends inside a step; against fp64 on the GPU and against the call in one pass
+    M, nnz = 20_011, 1_000_003
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda") ** 2 // M).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H = (torch.randn((n, K), generator=g, device="cuda") for n in (M, N))
+    vals = torch.randn(nnz, generator=g, device="cuda")
+    flag = 0
+    if bf16:
+        W, H, flag = W.bfloat16(), H.bfloat16(), api.FLAG_OPERANDS_BF16
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    ref, mag = torch.empty(nnz, device="cuda", dtype=torch.float64), torch.empty(nnz, device="cuda", dtype=torch.float64)
+    for a in range(0, nnz, 50_000):
+        i = slice(a, min(nnz, a + 50_000))
+        t = W[rows[i].long()].double() * H[cols[i].long()].double()
+        ref[i], mag[i] = t.sum(1), t.abs().sum(1)
+    n0 = engine.kernel_launches()
+    for S in (None, vals):
+        P = torch.full((nnz,), float("nan"), device="cuda")
+        plan.execute(W, H, P, S, flag)
+        s = 1.0 if S is None else S.double()
+        # K products and sums in fp32, and one more rounding for S
+        assert bool(((P.double() - ref * s).abs() <= (K + 2) * 2.0 ** -24 * (mag * s).abs()).all())
+        assert plan.last_kernel_ms() > 0
+    assert engine.kernel_launches() - n0 >= 4      # passes, not one launch each
+    # S and P in one array: the S values have to outlive the first pass
+    both = vals.clone()
+    plan.execute(W, H, both, both, flag)
+    assert bool(((both.double() - ref * vals.double()).abs() <= (K + 2) * 2.0 ** -24 * (mag * vals.double()).abs()).all())
+    # not finite: in one row of H, and in one S value
+    c = int(cols[5])
+    H[c, K - 1] = float("inf")
+    vals[9] = float("nan")
+    plan.execute(W, H, P, vals, flag)
+    want = torch.isfinite(vals) & (cols != c)
+    assert torch.equal(torch.isfinite(P), want)
+    if not bf16:
+        whole = torch.empty_like(P)
+        plan.execute(W, H, whole, vals, api.FLAG_KERNEL_GATHER)
+        assert torch.equal(torch.isfinite(whole), want)
+    plan.close()
