@@ -184,13 +184,14 @@ struct SpmmCall {
     const float *W, *H;
     float *P_out;      // fused: receives P, or null
     float *Y, *scratch;
-    int64_t M, nnz;
+    int64_t M, N, nnz;
     int K;
     unsigned long long *clock;
 };
 bool spmm_supports(int K);
-size_t spmm_counter_floats(int64_t nnz, int K, int sm_count);
-size_t spmm_scratch_floats(int64_t nnz, int K, int sm_count);
+size_t spmm_counter_floats(int64_t nnz, int64_t N, int K, int sm_count);
+size_t spmm_scratch_floats(int64_t nnz, int64_t N, int K, int sm_count);
+int spmm_passes(int64_t nnz, int64_t N, int K);  // launches of an SpMM
 cudaError_t launch_spmm(const SpmmCall &call, int sm_count, int64_t *n_launches, cudaStream_t stream);
 
 // float64 recomputation of every stride-th nonzero on the device (see check.cu).

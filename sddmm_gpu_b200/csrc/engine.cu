@@ -1162,9 +1162,9 @@ cudaError_t ensure_spmm_data(sddmm_plan_s *p, cudaStream_t s)
         cudaError_t e = p->d_row_ptr ? cudaSuccess : build_plan_row_ptr(p, on);
         if (e != cudaSuccess || p->d_spmm_scratch || p->nnz == 0) return e;
         float *scratch = nullptr;
-        e = dev_alloc(p, &scratch, spmm_scratch_floats(p->nnz, p->K, p->h->sm_count));
+        e = dev_alloc(p, &scratch, spmm_scratch_floats(p->nnz, p->N, p->K, p->h->sm_count));
         if (e != cudaSuccess) return e;
-        e = cudaMemsetAsync(scratch, 0, sizeof(float) * spmm_counter_floats(p->nnz, p->K, p->h->sm_count), on);
+        e = cudaMemsetAsync(scratch, 0, sizeof(float) * spmm_counter_floats(p->nnz, p->N, p->K, p->h->sm_count), on);
         if (e == cudaSuccess) p->d_spmm_scratch = scratch;
         else pool_free(scratch);
         return e;
@@ -1254,8 +1254,8 @@ int run_spmm(sddmm_plan_s *p, bool fused, const float *W, const float *H, const 
         return SDDMM_INVALID_ARG;
     }
     CallTimer timer(p, async);
-    CUDA_TRY(h, timer.begin(p->M > 0, s));
-    SpmmCall call{p->d_rows, p->d_cols, p->d_row_ptr, dV, fused ? dW : nullptr, dH, dP, dY, p->d_spmm_scratch, p->M, p->nnz, p->K,
+    CUDA_TRY(h, timer.begin(p->M > 0 && (fused || spmm_passes(p->nnz, p->N, p->K) == 1), s));
+    SpmmCall call{p->d_rows, p->d_cols, p->d_row_ptr, dV, fused ? dW : nullptr, dH, dP, dY, p->d_spmm_scratch, p->M, p->N, p->nnz, p->K,
                   timer.clk};
     CUDA_TRY(h, launch_spmm(call, h->sm_count, &h->n_launches, s));
     CUDA_TRY(h, timer.end(s));

@@ -90,20 +90,21 @@ struct WShare {
     }
 };
 
-// What becomes of a dot product: stored (STORE); stored through perm, the result of nonzero j to P[perm[j]], scaled by
-// sval[perm[j]] (PERM); or added to what P holds, the product over earlier columns of the operands (ADD): by a reduction that
-// nothing waits for, or, with `finish`, read, added and scaled.
-enum GatherMode { STORE, PERM, ADD };
+// What is multiplied and what becomes of a dot product: whole rows, the product stored (STORE) or stored through perm, the result of nonzero
+// j to P[perm[j]], scaled by sval[perm[j]] (PERM); or one pass over some columns of rows that are `pitch` bytes apart (PASS): stored by
+// the first pass, added to P by the later ones -- by a reduction that nothing waits for, or, in the last pass (`finish`), read, added and scaled.
+enum GatherMode { STORE, PERM, PASS };
 
-// pieces: 16-byte pieces of a row that are multiplied.  row_bytes: from one row to the next.  run_len: nonzeros of a set, a multiple of S::NB.
+// pieces: 16-byte pieces of a row that are multiplied.  run_len: nonzeros of a set, a multiple of S::NB.
 template <class S, GatherMode MODE>
 __global__ void __launch_bounds__(GA_TPB, S::CTAS)
 sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
                     const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
-                    float *__restrict__ P, unsigned nnz, int pieces, unsigned row_bytes, bool finish, unsigned run_len, unsigned long long *clock, unsigned meet_from)
+                    float *__restrict__ P, unsigned nnz, int pieces, unsigned pitch, bool add, bool finish, unsigned run_len, unsigned long long *clock, unsigned meet_from)
 {
     clock_begin(clock);
     constexpr bool HAS_PERM = MODE == PERM;
+    const unsigned row_bytes = MODE == PASS ? pitch : (unsigned)pieces * 16u;  // from one row to the next
     constexpr int L = S::L, F = S::F, B = S::B, RB = S::RB, NB = S::NB, G = S::G;
     const int lane = threadIdx.x & 31, lig = lane & (L - 1), set = lane / L;
     const unsigned warp0 = gather_warp(blockIdx.x, blockDim.x, threadIdx.x) * (G * run_len);  // first nonzero of this warp
@@ -155,7 +156,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
         if (HAS_PERM && sval) s = __ldg(sval + dst);
         float sum = 0.f;
         // (volatile: it is to be under way while the rows of H are, not waited for at the end of the step)
-        if (MODE == ADD && finish && lig < NB) asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(sum) : "l"(P + at(j)));
+        if (MODE == PASS && add && finish && lig < NB) asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(sum) : "l"(P + at(j)));
         float res = 0.f;
 #pragma unroll
         for (int h0 = 0; h0 < NB; h0 += RB) {
@@ -187,8 +188,8 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
             if (RB == NB || il / RB == h0 / RB) res = t;
         }
         if (lig < NB && j < nnz) {
-            if (MODE == ADD && !finish) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(P + j), "f"(res) : "memory");
-            else P[HAS_PERM ? (unsigned)dst : j] = (MODE == ADD ? sum + res : res) * s;
+            if (MODE == PASS && add && !finish) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(P + j), "f"(res) : "memory");
+            else P[HAS_PERM ? (unsigned)dst : j] = (MODE == PASS ? sum + res : res) * s;
         }
         j += NB;
         r = rn;
@@ -254,8 +255,9 @@ struct GatherCall {
     float *P;
     unsigned nnz;
     int pieces;
-    unsigned row_bytes;
-    bool add, finish;  // to P (perm null), and for the last time
+    bool pass;         // one of several passes (perm null)
+    unsigned pitch;
+    bool add, finish;
     int sm_count;
     unsigned long long *clock;
     bool beside;
@@ -284,14 +286,14 @@ cudaError_t launch_mode(const GatherCall &c)
     cfg.stream = c.stream;
     cfg.attrs = &attr;
     cfg.numAttrs = c.beside ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, sddmm_gather_kernel<S, MODE>, c.rows, c.cols, c.perm, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.row_bytes,
+    return cudaLaunchKernelEx(&cfg, sddmm_gather_kernel<S, MODE>, c.rows, c.cols, c.perm, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.pitch, c.add,
                               c.finish, run, c.clock, meet_from);
 }
 
 template <class S>
 cudaError_t launch_shape(const GatherCall &c)
 {
-    return c.perm ? launch_mode<S, PERM>(c) : c.add ? launch_mode<S, ADD>(c) : launch_mode<S, STORE>(c);
+    return c.perm ? launch_mode<S, PERM>(c) : c.pass ? launch_mode<S, PASS>(c) : launch_mode<S, STORE>(c);
 }
 
 // The shape for `pieces` pieces of a row: L * (F - 1) < pieces <= L * F, L small enough that a set's lanes
@@ -372,7 +374,8 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
             c.H = reinterpret_cast<const char *>(H + k0);
             c.P = perm ? P : P + j0;
             c.pieces = width / 4;
-            c.row_bytes = (unsigned)K * 4u;
+            c.pass = passes.n > 1;
+            c.pitch = (unsigned)K * 4u;
             c.add = pass > 0;
             c.finish = pass == passes.n - 1;
             c.sm_count = sm_count;
@@ -416,7 +419,7 @@ cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const i
     if (perm) p = {1, K};
     for (int pass = 0; pass < p.n; ++pass) {
         GatherCall c = {rows, cols, perm, pass < p.n - 1 ? nullptr : sval, static_cast<const char *>(W) + 2 * pass * p.floats,
-                        static_cast<const char *>(H) + 2 * pass * p.floats, P, (unsigned)nnz, p.floats / 8, (unsigned)K * 2u, pass > 0,
+                        static_cast<const char *>(H) + 2 * pass * p.floats, P, (unsigned)nnz, p.floats / 8, p.n > 1, (unsigned)K * 2u, pass > 0,
                         pass == p.n - 1, sm_count, clock, false, stream};
         cudaError_t e = cudaErrorInvalidValue;
         if (p.floats == 256) e = launch_shape<GatherShape<16, 2, 2, 8, true, false, 5, true>>(c);

@@ -84,14 +84,16 @@ template <class S>
 __global__ void __launch_bounds__(SP_TPB, S::CTAS)
 spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const float *__restrict__ val,
             const char *__restrict__ W, const char *__restrict__ H, float *__restrict__ P_out, char *__restrict__ Y,
-            char *scratch, unsigned *arrived, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces,
+            char *scratch, unsigned *arrived, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces, unsigned pitch,
             unsigned run_len, unsigned gather_blocks, unsigned long long *clock, unsigned meet_from)
 {
     constexpr int L = S::L, F = S::F, B = S::B, NB = S::NB, G = S::G;
     constexpr bool FUSED = S::FUSED;
+    // From one row to the next.  (The fused form multiplies whole rows and holds one value less: with a second one it spills, 1707 -> 1801 us
+    // at K = 256, 16.1 M nonzeros.)
+    const unsigned row_bytes = !FUSED ? pitch : (unsigned)pieces * 16u;
     clock_begin(clock);
     const int lane = threadIdx.x & 31;
-    const unsigned row_bytes = (unsigned)pieces * 16u;
     if (blockIdx.x >= gather_blocks) {
         // 32 rows of S per warp: those without nonzeros are written as zeros
         const int64_t r0 = ((int64_t)(blockIdx.x - gather_blocks) * (SP_TPB / 32) + (threadIdx.x >> 5)) * 32;
@@ -142,11 +144,9 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     // after is not stored.  (Each where it costs nothing measurable.  fused, 16.1 M nonzeros, K = 256, us: without either 1646,
     // zero weights 1683, a row of its own 1638; 6.0 M, K = 512: 1088 / 1095 / 1142; SpMM, 6.0 M, K = 128: 224 / 224 / 229.)
     constexpr bool PAD = FUSED && S::JOINT;
-    const unsigned padding = j0 < nnz ? nnz : 0xffffffffu;
-    int cur = __ldg(rows + at(j0));                                // row being summed
-    const int row0 = cur;
-    const bool began_before = j0 > 0 && __ldg(rows + at(j0 - 1)) == cur;  // it began in an earlier run
-    bool head = began_before;                                      // and nothing of it has been stored yet
+    int cur = __ldg(rows + at(j0));                                // row being summed: that of the nonzero before this step
+    auto began_before = [&](int row) { return j0 > 0 && __ldg(rows + at(j0 - 1)) == row; };  // it began in an earlier run
+    bool head = began_before(cur);                                 // and nothing of it has been stored yet
     if (FUSED) load_w((unsigned)cur);
     int r, c;
     float s = 1.f;
@@ -156,7 +156,6 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         c = __ldg(cols + a);
         if (val) s = __ldg(val + a);
     }
-    int last = cur;  // row of the nonzero before this step
 #pragma unroll 1
     for (unsigned step = run_len / NB; step > 0; --step) {
         int rn = 0, cn = 0;
@@ -168,14 +167,14 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             if (val) sn = __ldg(val + a);
         }
         int before = __shfl_up_sync(FULL, r, 1, L);
-        if (lig == 0) before = last;
-        const unsigned changed = __ballot_sync(FULL, (r != before || (PAD && j == padding)) && lig < NB);
+        if (lig == 0) before = cur;
+        const unsigned changed = __ballot_sync(FULL, (r != before || (PAD && j == nnz && (G == 1 || j0 < nnz))) && lig < NB);
         const bool full = __all_sync(FULL, j < nnz);
         if (!FUSED && !full && j >= nnz) s = 0.f;
-        last = __shfl_sync(FULL, r, NB - 1, L);
         if (FUSED && S::PF && step > 1) {
             // the W rows that the next step opens, into L1
             int b2 = __shfl_up_sync(FULL, rn, 1, L);
+            const int last = __shfl_sync(FULL, r, NB - 1, L);
             if (lig == 0) b2 = last;
             if (rn != b2 && lig < NB) {
                 const char *wp = W + (size_t)(unsigned)rn * row_bytes;
@@ -308,14 +307,15 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         c = cn;
         s = sn;
     }
-    if (j0 < nnz) {
+    if (G == 1 || j0 < nnz) {
         const unsigned end = j0 + run_len;
         const bool goes_on = end < nnz && __ldg(rows + end) == cur;
         if (!PAD || end <= nnz)  // (else it was stored when the padding opened)
             flush(goes_on ? scratch + (size_t)(2 * run + 1) * row_bytes
                           : head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
         // the rows that this run left a part of: the one it began with, the one it ends with
-        const int part_row[2] = {began_before && !head ? row0 : -1, goes_on || head ? cur : -1};
+        const int row0 = __ldg(rows + j0);  // (read again: kept from the start it is a register more in the loop, where the shapes spill)
+        const int part_row[2] = {!head && began_before(row0) ? row0 : -1, goes_on || head ? cur : -1};
         if (part_row[0] >= 0 || part_row[1] >= 0) {
             const unsigned lanes = L == 32 ? FULL : ((1u << (L & 31)) - 1u) << (set * L);
             auto arrive = [&](unsigned *count) {  // how many came before; everything this set stored is visible first
@@ -397,9 +397,9 @@ unsigned run_length(int64_t nnz, int sm_count)
 }
 
 template <class S>
-cudaError_t launch_shape(const SpmmCall &a, int sm_count, int64_t *n_launches, cudaStream_t stream)
+cudaError_t launch_shape(const SpmmCall &a, int k0, int width, int sm_count, int64_t *n_launches, cudaStream_t stream)
 {
-    const int pieces = a.K / 4;
+    const int pieces = width / 4;
     if (pieces > S::L * S::F || pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
     const unsigned run = run_length<S>(a.nnz, sm_count), n_runs = (unsigned)((a.nnz + run - 1) / run);
     const unsigned sets_per_block = SP_TPB / 32 * S::G;
@@ -407,10 +407,10 @@ cudaError_t launch_shape(const SpmmCall &a, int sm_count, int64_t *n_launches, c
     const unsigned zero_blocks = (unsigned)((a.M + SP_TPB - 1) / SP_TPB);
     // scratch: two counters per run, zero between calls, then the parts
     unsigned *const arrived = reinterpret_cast<unsigned *>(a.scratch);
-    char *const parts = reinterpret_cast<char *>(a.scratch + spmm_counter_floats(a.nnz, a.K, sm_count));
+    char *const parts = reinterpret_cast<char *>(a.scratch + spmm_counter_floats(a.nnz, a.N, a.K, sm_count));
     spmm_kernel<S><<<gather_blocks + zero_blocks, SP_TPB, 0, stream>>>(
-        a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H), a.P_out,
-        reinterpret_cast<char *>(a.Y), parts, arrived, a.row_ptr, (unsigned)a.nnz, a.M, pieces, run, gather_blocks, a.clock, last_wave(gather_blocks, (unsigned)sm_count * S::CTAS));
+        a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H + k0), a.P_out,
+        reinterpret_cast<char *>(a.Y + k0), parts, arrived, a.row_ptr, (unsigned)a.nnz, a.M, pieces, (unsigned)a.K * 4u, run, gather_blocks, a.clock, last_wave(gather_blocks, (unsigned)sm_count * S::CTAS));
     ++*n_launches;
     return cudaGetLastError();
 }
@@ -461,24 +461,48 @@ auto with_shape(int K, bool fused, Fn f)
 
 }  // namespace
 
+// SpMM of long rows with a large H in passes of 192 columns (of H and of Y; the fused form needs whole rows).  More gathers of a pass hit L2,
+// and the shapes for more columns hold so many registers that few warps are resident.  Sustained us, one pass / these: K = 384, 0.3 M rows
+// of H 573 / 570, 0.7 M 1166 / 1062, 1 M 2163 / 1975; K = 512, 0.3 M 734 / 782, 0.7 M 1449 / 1453, 1 M 2806 / 2678, 1.5 M 4516 / 4181; K = 256, 1.5 M 2096 / 2138.
+static int pass_floats(int64_t nnz, int64_t N, int K)
+{
+    const int64_t h_bytes = N * K * 4;
+    return K > 320 && nnz >= 1000000 && h_bytes >= (K > 480 && K <= 512 ? 1700000000 : 900000000) ? 192 : K;
+}
+
+int spmm_passes(int64_t nnz, int64_t N, int K)
+{
+    const int w = pass_floats(nnz, N, K);
+    return (K + w - 1) / w;
+}
+
 bool spmm_supports(int K) { return K > 0 && K % 4 == 0 && K <= 1024; }
 
-static size_t max_runs(int64_t nnz, int K, int sm_count)  // of either form
+static size_t max_runs(int64_t nnz, int64_t N, int K, int sm_count)  // of either form and of every pass
 {
-    auto run_of = [&](bool fused) { return with_shape(K, fused, [&](auto s) { return run_length<decltype(s)>(nnz, sm_count); }); };
-    const unsigned run = std::min(run_of(false), run_of(true));
+    auto run_of = [&](int width, bool fused) { return with_shape(width, fused, [&](auto s) { return run_length<decltype(s)>(nnz, sm_count); }); };
+    unsigned run = std::min(run_of(K, false), run_of(K, true));
+    const int w = pass_floats(nnz, N, K);
+    if (w < K) run = std::min(run, run_of(w, false));
+    if (K % w) run = std::min(run, run_of(K % w, false));
     return (size_t)((nnz + run - 1) / run);
 }
-size_t spmm_counter_floats(int64_t nnz, int K, int sm_count) { return (2 * max_runs(nnz, K, sm_count) + 31) / 32 * 32; }
-size_t spmm_scratch_floats(int64_t nnz, int K, int sm_count)
+size_t spmm_counter_floats(int64_t nnz, int64_t N, int K, int sm_count) { return (2 * max_runs(nnz, N, K, sm_count) + 31) / 32 * 32; }
+size_t spmm_scratch_floats(int64_t nnz, int64_t N, int K, int sm_count)
 {
-    return spmm_counter_floats(nnz, K, sm_count) + max_runs(nnz, K, sm_count) * 2 * (size_t)K;
+    return spmm_counter_floats(nnz, N, K, sm_count) + max_runs(nnz, N, K, sm_count) * 2 * (size_t)K;
 }
 
 cudaError_t launch_spmm(const SpmmCall &a, int sm_count, int64_t *n_launches, cudaStream_t stream)
 {
     if (a.M == 0) return cudaSuccess;
-    return with_shape(a.K, a.W != nullptr, [&](auto s) { return launch_shape<decltype(s)>(a, sm_count, n_launches, stream); });
+    const int w = a.W ? a.K : pass_floats(a.nnz, a.N, a.K);
+    for (int k0 = 0; k0 < a.K; k0 += w) {
+        const int width = std::min(w, a.K - k0);
+        const cudaError_t e = with_shape(width, a.W != nullptr, [&](auto s) { return launch_shape<decltype(s)>(a, k0, width, sm_count, n_launches, stream); });
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace sddmm

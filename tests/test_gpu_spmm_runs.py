@@ -82,3 +82,33 @@ def test_last_nonzero_infinite(engine, K):
             # all terms are positive: an error of 1e-4 in each weight is one of 1e-4 in the sum
             assert np.all(np.abs(Y[:-1] - ref[:-1]) <= 2 * TOL * A[:-1])
         plan.close()
+
+
+@pytest.mark.parametrize("K,N", [(388, 581_000), (512, 831_000), (900, 251_000)])
+def test_long_rows_in_passes(engine, K, N):
+    # a large H, long rows: passes over part of the columns (the last one of 4, 128 and 132), a row of many runs, rows without nonzeros
+    import torch
+    M, nnz = 7_013, 1_000_003
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = (torch.rand(nnz, generator=g, device="cuda") ** 3 * M).to(torch.int64).clamp_(max=M - 1)
+    rows = torch.sort(torch.where(rows % 7 == 3, 0, rows)).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    H, vals = torch.randn((N, K), generator=g, device="cuda"), torch.randn(nnz, generator=g, device="cuda")
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    for pv in (vals, None):
+        n0 = engine.kernel_launches()
+        Y = torch.full((M, K), float("nan"), device="cuda")
+        plan.spmm(H, Y, pv)
+        assert plan.last_kernel_ms() > 0 and engine.kernel_launches() - n0 == -(-K // 192)
+        ref, A = (torch.zeros((M, K), device="cuda", dtype=torch.float64) for _ in range(2))
+        for a in range(0, nnz, 100_000):
+            t = H[cols[a:a + 100_000].long()].double()
+            if pv is not None:
+                t *= pv[a:a + 100_000, None].double()
+            ref.index_add_(0, rows[a:a + 100_000].long(), t)
+            A.index_add_(0, rows[a:a + 100_000].long(), t.abs())
+        assert bool(((Y.double() - ref).abs() <= TOL * A).all())
+        again = torch.full((M, K), float("nan"), device="cuda")
+        plan.spmm(H, again, pv)
+        assert torch.equal(Y, again)
+    plan.close()
