@@ -269,11 +269,16 @@ cudaError_t launch_mode(const GatherCall &c)
 {
     // only the last piece of a lane is predicated: the ones before it have to lie inside the row
     if (c.pieces > S::L * S::F || c.pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
-    // A set's share: 16 nonzeros (32 when a warp is one or two sets), less when the warps would not fill the SMs.
-    constexpr unsigned most = S::L >= 16 ? 32 : 16;
-    const unsigned resident = (unsigned)c.sm_count * S::CTAS * (GA_TPB / 32) * S::G;  // sets
-    unsigned run = c.nnz / resident / S::NB * S::NB;
-    run = run < (unsigned)S::NB ? (unsigned)S::NB : run > most ? most : run;
+    // A set's run.  A long one spreads what a run costs at its ends and keeps the W row over more nonzeros; the last wave of blocks, which
+    // may be nearly empty, lasts as long as a run.  So by the nonzeros that there are for a resident set (us at runs of 8 / 16 / 32):
+    // below 40: K = 32, 1.0 M nonzeros 18.6 / 21.1 / 27.3;  K = 64, 0.4 M 12.4 / 14.4 / 14.4, 0.7 M 19.6 / 20.7 / 24.0;  K = 128, 0.24 M 12.4 / 14.4 /
+    // 14.2, 0.4 M, planned, called and closed 49.6 / 50.1 / 55.3;  K = 256, 0.18 M 18.0 / 17.5 / 19.2;  K = 512, 0.12 M 24.2 / 24.4 / 28.0;
+    // from there on: K = 64, 1.6 M 51.8 / 48.5 / 51.8, 4.0 M 88.3 / 77.9 / 79.0;  K = 128, 1.0 M 43.1 / 41.0 / 44.4, 2.0 M 74.0 / 67.6 / 69.9;
+    // K = 300, 1.0 M 79.9 / 76.0 / 84.9;  K = 256, 0.7 M 53.6 / 49.9 / 51.7, documents x words, 0.75 M 56.7 / 50.0 / 47.8;
+    // two sets to a warp, from 256 on: K = 192, 2.5 M 122 / 109.5 / 108.6;  K = 300, 2.5 M 179 / 177 / 168;  K = 100, 4.1 M 149 / 130 / 125.
+    const unsigned resident = (unsigned)c.sm_count * S::CTAS * (GA_TPB / 32) * S::G, share = c.nnz / resident;  // sets; nonzeros for each
+    unsigned run = share < 40 ? 8 : S::L == 32 || (S::L == 16 && share >= 256) ? 32 : 16;
+    if (share < 8) run = S::NB;
     const unsigned tpb = c.beside ? GA_TPB_BESIDE : GA_TPB, per_block = run * S::G * (tpb / 32);
     const unsigned blocks = (unsigned)(((uint64_t)c.nnz + per_block - 1) / per_block);
     const unsigned meet_from = last_wave(blocks, (unsigned)c.sm_count * S::CTAS);
