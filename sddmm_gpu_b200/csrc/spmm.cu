@@ -27,7 +27,8 @@
 // by resident warps.  The fused form at K = 256 reaches neither bound (16.1 M nonzeros: 7.1 GB through DRAM at 4.5 TB/s, 13.4 TB/s read at
 // the L2 slices): between two blocks of B rows a set reduces, broadcasts and adds with nothing in flight.  Measured on R-MAT matrices against the row-task and shared-memory-ring kernels this replaces
 // (us): SpMM, 6.0 M nonzeros, 250 K x 250 K: K = 64 755 -> 125;  0.67 M nonzeros: K = 64 379 -> 29;  fused, 16.1 M
-// nonzeros, 1 M x 1 M: K = 256 2970 -> 1720 to 1785;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.
+// nonzeros, 1 M x 1 M: K = 256 2970 -> 1720 to 1785;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.  With runs that fill whole waves
+// since then: SpMM, 6.0 M, K = 64 128 -> 117;  16.1 M, K = 256 1346 -> 1270;  0.75 M documents x words, K = 256 58 -> 43.
 // At K = 64 the gather kernel alone runs at 14.2 TB/s of gathered bytes.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -77,6 +78,19 @@ __device__ __forceinline__ unsigned long long pair_of(float x)
 {
     unsigned long long d;
     asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+    return d;
+}
+
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 
@@ -218,9 +232,26 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                     y[f].b = ffma2(pp, h[i][f].b, y[f].b);
                 }
             };
+            // B nonzeros of one row are summed before they are added to it: a long row's chain of roundings is a B-th as long, which is what
+            // lets runs be as long as they are (SpMM, 6.0 M nonzeros, K = 64, against 64 bits: runs of 80 one by one 1.4e-7 to 1.6e-7, runs of 320
+            // 2.6e-7, in blocks of four 1.4e-7).
+            auto add_block = [&]() {
+#pragma unroll
+                for (int f = 0; f < F; ++f) {
+                    unsigned long long pp = pair_of(p[0]), ta = mul2(pp, h[0][f].a), tb = mul2(pp, h[0][f].b);
+#pragma unroll
+                    for (int i = 1; i < B; ++i) {
+                        pp = pair_of(p[i]);
+                        ta = ffma2(pp, h[i][f].a, ta);
+                        tb = ffma2(pp, h[i][f].b, tb);
+                    }
+                    y[f].a = add2(y[f].a, ta);
+                    y[f].b = add2(y[f].b, tb);
+                }
+            };
+            // most blocks of B stay within their rows: one test for the block instead of two for each nonzero
+            const bool stays = (here & (setmask * ((1u << B) - 1u))) == 0;
             if (FUSED && S::JOINT) {
-                // most blocks of B stay within their rows: one test for the block instead of two for each nonzero
-                const bool stays = (here & (setmask * ((1u << B) - 1u))) == 0;
                 auto dot = [&](int i) {
                     unsigned long long a = 0;
 #pragma unroll
@@ -251,8 +282,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 #pragma unroll
                 for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, scaled, i * (L / B), L);
                 if (stays) {
-#pragma unroll
-                    for (int i = 0; i < B; ++i) add(i, p[i]);
+                    add_block();
                 } else {
 #pragma unroll
                     for (int i = 0; i < B; ++i) {
@@ -272,6 +302,31 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                 if (!FUSED) {
 #pragma unroll
                     for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, s, b + i, L);
+                    if (B > 1 && stays) {
+                        add_block();
+                        continue;
+                    }
+                }
+                auto weight = [&](int i) {  // fused: of nonzero i of the block
+                    const int x = b + i;
+                    unsigned long long a0 = 0, a1 = 0;
+#pragma unroll
+                    for (int f = 0; f < F; ++f) {
+                        a0 = ffma2(w[f].a, h[i][f].a, a0);
+                        a1 = ffma2(w[f].b, h[i][f].b, a1);
+                    }
+                    float a = fold2(a0) + fold2(a1);
+#pragma unroll
+                    for (int off = L / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
+                    p[i] = a * __shfl_sync(FULL, s, x, L);
+                    if (!full && j - il + x >= nnz) p[i] = 0.f;
+                    if (il == x) p_mine = p[i];
+                };
+                if (FUSED && B > 1 && stays) {
+#pragma unroll
+                    for (int i = 0; i < B; ++i) weight(i);
+                    add_block();
+                    continue;
                 }
 #pragma unroll
                 for (int i = 0; i < B; ++i) {
@@ -283,20 +338,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                             if (FUSED) load_w((unsigned)rj);
                         }
                     }
-                    if (FUSED) {
-                        unsigned long long a0 = 0, a1 = 0;
-#pragma unroll
-                        for (int f = 0; f < F; ++f) {
-                            a0 = ffma2(w[f].a, h[i][f].a, a0);
-                            a1 = ffma2(w[f].b, h[i][f].b, a1);
-                        }
-                        float a = fold2(a0) + fold2(a1);
-#pragma unroll
-                        for (int off = L / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
-                        p[i] = a * __shfl_sync(FULL, s, x, L);
-                        if (!full && j - il + x >= nnz) p[i] = 0.f;
-                        if (il == x) p_mine = p[i];
-                    }
+                    if (FUSED) weight(i);
                     add(i, p[i]);
                 }
             }
@@ -378,22 +420,27 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     clock_end(clock, meet_from);
 }
 
+// Runs are cut so that they fill whole waves of resident sets: a wave lasts as long as its runs, and a last one that is nearly empty as
+// long as a full one (SpMM, K = 64, 6.0 M nonzeros, us: 2.0 waves 117, 2.5 waves 127, 2.8 waves 121, 4.0 waves 124).  How many: each
+// run pays for its two ends (partial rows, the dependent loads it starts with), so few; but rows of a power-law matrix make some
+// runs slower than others, the fused form more than SpMM, and long runs spread a wave over more rows of H than L2 holds.  Sustained us at
+// 1 / 2 / 3 / 4 / 5 / 8 waves (s: nonzeros for a resident set; in brackets: runs of 80 to 160 nonzeros, whatever the waves):
+//   SpMM: s = 37, K = 64 24 / 29 / 33 / 33 / 45 / 45 (29);  40, documents x words 23 / 29 / 33 / 33 / 44 / 43 (29);  118, K = 256 52 / 56 / 62 / 64 / 69 / 80 (64);
+//     253, uniform, K = 256 133 / 139 / 146 / 153 / 161 / 176 (160);  317, K = 64 114 / 117 / 121 / 124 / 127 / 141 (124);  577, K = 100 143 / 142 / 143 / 147 / 151 / 169 (180);
+//     849, K = 64 330 / 320 / 320 / 335 / 329 / 345 (354);  1351, K = 200 674 / 550 / 579 / 569 / 556 / 576 (594);  2252, K = 300 - / - / 863 / 877 / 887 / 894 (929)
+//   fused: s = 53, uniform, K = 128 71 / 80 / 93 / 94 / 95 / 111 (92);  63, K = 128 72 / 77 / 83 / 91 / 91 / 123 (83);  148, K = 256 89 / 86 / 84 / 86 / 88 / 93 (87);
+//     211, K = 128 232 / 219 / 224 / 229 / 238 / 246 (235);  310, attention, K = 64 129 / 132 / 141 / 142 / 144 / 152 (142);  422, K = 64 280 / 260 / 252 / 254 / 259 / 267 (262);
+//     845, K = 512 857 / 798 / 808 / 790 / 780 / 792 (806);  1689, K = 200 925 / 852 / 826 / 818 / 806 / 795 (798);  3396, K = 256 at 5 / 8 / 12 waves 1727 / 1649 / 1652 (1656)
 template <class S>
 unsigned run_length(int64_t nnz, int sm_count)
 {
-    // Waves of resident sets against the cost of a run's two ends.  Six waves; down to three where runs would be shorter
-    // than 80 nonzeros, up to twelve where they would be longer than 160 (us at 12 / 6 / 3 waves: fused 16.1 M nonzeros
-    // K = 256 1704 / 1775 / 1878; fused 0.9 M K = 256 144 / 130 / 125; SpMM 6 M K = 64, 3 waves against 6: 125 / 136).
-    // Below three waves runs of three steps, two where those leave resident sets idle, one where nearly all are
-    // (0.7 M nonzeros K = 64 at 24 / 16: 29.7 / 33.9; 0.3 M at 16 / 8: 17.2 / 23.0; 20 K at 16 / 8: 13.4 / 11.6).
-    const int64_t wave = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G;
-    int64_t run = nnz / (6 * wave);
-    if (run < 80) run = std::min<int64_t>(80, nnz / (3 * wave));
-    if (run > 160) run = std::max<int64_t>(160, nnz / (12 * wave));
-    run = run / S::NB * S::NB;
-    if (run < 3 * S::NB) run = nnz <= S::NB * wave / 4 ? S::NB : nnz <= S::NB * wave ? 2 * S::NB : 3 * S::NB;
-    if (run > SP_MAX_RUN) run = SP_MAX_RUN;
-    return (unsigned)run;
+    const int64_t wave = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G, s = nnz / wave + 1;
+    // (one nonzero at a time, B = 1, the roundings of a long row are as many as the run is long: no longer runs than 80 to 160)
+    const int64_t waves = S::B == 1 ? (s <= 480 ? (s + 79) / 80 : s <= 1920 ? (s + 159) / 160 : 12)
+                          : S::FUSED ? (s <= 120 ? 1 : s <= 330 ? 2 : s > 1500 ? (s + 299) / 300 : (s + 169) / 170)
+                                     : s <= 340 ? 1 : std::max<int64_t>(2, (s + 759) / 760);
+    const int64_t run = (nnz / (waves * wave) + S::NB) / S::NB * S::NB;  // rounded up: one run less than a wave, not one more
+    return (unsigned)std::min<int64_t>(run, SP_MAX_RUN);
 }
 
 template <class S>
@@ -430,7 +477,7 @@ auto with_shape(int K, bool fused, Fn f)
         if (q <= 24) return f(SpmmShape<8, 3, 2, false, 3, true, true, false>());
         if (q < 32) return f(SpmmShape<8, 4, 1, false, 3, true, true, false>());
         if (q == 32) return f(SpmmShape<8, 4, 1, true, 4, true, false, false>());
-        if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4, true, true, false>());
+        if (q <= 48) return f(SpmmShape<16, 3, 1, false, 4, true, true, false>());
         if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, true, true, true>());
         if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, true, true, true>());
         if (q <= 96) return f(SpmmShape<32, 3, 1, false, 4, true, false, false>());
@@ -443,14 +490,14 @@ auto with_shape(int K, bool fused, Fn f)
     if (q <= 4) return f(SpmmShape<4, 1, 4, false, 4>());
     if (q <= 8) return f(SpmmShape<8, 1, 4, false, 4>());
     if (q <= 12) return f(SpmmShape<4, 3, 2, false, 4>());
-    if (q < 16) return f(SpmmShape<8, 2, 4, false, 4>());
+    if (q < 16) return f(SpmmShape<8, 2, 4, false, 3>());
     if (q == 16) return f(SpmmShape<8, 2, 4, true, 4>());
     if (q <= 24) return f(SpmmShape<8, 3, 2, false, 4>());
-    if (q < 32) return f(SpmmShape<16, 2, 4, false, 4>());
+    if (q < 32) return f(SpmmShape<16, 2, 4, false, 3>());
     if (q == 32) return f(SpmmShape<16, 2, 4, true, 4>());
     if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4>());
     if (q < 64) return f(SpmmShape<32, 2, 2, false, 5>());
-    if (q == 64) return f(SpmmShape<32, 2, 2, true, 5>());
+    if (q == 64) return f(SpmmShape<32, 2, 4, true, 4>());
     if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3>());
     if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3>());
     if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3>());
