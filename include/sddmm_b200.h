@@ -124,7 +124,7 @@ SDDMM_API int sddmm_destroy_plan(sddmm_plan_t p);
 /*
  * Replaces the W/H uploads, cudaMemset, launch loop and result download of
  * sddmm_GPU (HiPC18/src/sddmm.cu:53,71-73,93-119) and the kernel comp_kernel_COO
- * (HiPC18/src/kernel.h:2-52) -- one launch, no K-slicing.
+ * (HiPC18/src/kernel.h:2-52) -- one launch; long rows of a large H in a few, each over part of the columns.
  *
  *   W, H, P : host or device pointers (detected); host buffers go
  *             through plan-owned device staging inside the call.  With W in
@@ -287,7 +287,7 @@ typedef struct {
     int32_t reserved0;
     int64_t n_dense_cells;  /* 128 x 64 cells handed to the dense-cell kernel (none below nnz * K = 2^26) */
     int64_t n_dense_nnz;    /* nonzeros inside them                            */
-    int64_t n_hub_cols;     /* columns marked for L2 residency: 0 unless the ring kernel runs by default or a call has forced it */
+    int64_t n_hub_cols;     /* columns marked for L2 residency: 0 unless the plan is column-tiled with a large H or a call has forced the ring kernel */
 } sddmm_plan_info;
 SDDMM_API int sddmm_plan_get_info(sddmm_plan_t p, sddmm_plan_info *info);
 

@@ -661,7 +661,7 @@ int sddmm_plan_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const in
                                              sizeof(int32_t) * DENSE_CELL_ROWS * DENSE_CELL_COLS * p->dense.n_table_cells + 12 * p->dense.n_sparse);
         }
     }
-    // Hub-column marks are for the ring kernel: now if it will run by default, else if it is forced.
+    // Hub-column marks are for the ring kernel: now if the order is permuted and it will run by default, else if it is forced.
     // SDDMM_L2_HUB_MB overrides the share of L2 set aside for hub rows (0 = off).
     {
         int64_t budget_mb = 64;  // best of a 16..128 MB sweep on the scale-22 R-MAT matrix at K = 256
