@@ -859,8 +859,9 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     }
     const bool use_dense = !forced && !tiled_out && p->dense.n_cells > 0;
     // a call that is one gather launch is timed by the kernel itself, everything else by events
-    const bool one_gather = !use_dense && !use_panel && (use_gather || !rows_on_ring(p, use_ring, p->d_perm && !tiled_out)) &&
-                            (p->d_perm || use_gather || gather_passes(p->nnz, p->N, p->K, dS, P).n == 1);
+    const bool permuted = p->d_perm && !tiled_out;
+    const bool one_gather = !use_dense && !use_panel && (use_gather || !rows_on_ring(p, use_ring, permuted)) &&
+                            (permuted || use_gather || gather_passes(p->nnz, p->N, p->K, dS, P).n == 1);
     bool p_copy = false;
     if (!p_dev) {
         // a small P is written to mapped host memory by the kernel: its 32-byte stores over PCIe cost less than a copy

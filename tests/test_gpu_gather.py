@@ -145,3 +145,29 @@ def test_long_rows_in_passes(engine, K, N, bf16):
         plan.execute(W, H, whole, vals, api.FLAG_KERNEL_GATHER)
         assert torch.equal(torch.isfinite(whole), want)
     plan.close()
+
+
+def test_tiled_order_in_passes(engine):
+    # a column-tiled plan asked for its own order has no permutation: passes as in input order, timed as a whole
+    K, M, N, nnz, tile = 768, 60_013, 150_011, 4_000_003, 70_000
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H = (torch.randint(-2, 3, (n, K), generator=g, device="cuda").float() for n in (M, N))   # every product and sum exact
+    plan = engine.plan_coo(M, N, rows, cols, K, 0, tile)
+    P = torch.full((nnz,), float("nan"), device="cuda")
+    for _ in range(2):
+        n0 = engine.kernel_launches()
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        plan.execute(W, H, P, None, api.FLAG_TILED_ORDER)
+        t1.record()
+        torch.cuda.synchronize()
+        assert engine.kernel_launches() - n0 == 4
+    # the four passes take milliseconds, of which a launch and a wait are tens of microseconds
+    assert 0.9 * t0.elapsed_time(t1) <= plan.last_kernel_ms() <= t0.elapsed_time(t1)
+    order = torch.argsort(cols // tile, stable=True)
+    for a in range(0, nnz, 200_000):
+        i = order[a:a + 200_000]
+        assert torch.equal(P[a:a + 200_000], (W[rows[i].long()] * H[cols[i].long()]).sum(1)), a
+    plan.close()
