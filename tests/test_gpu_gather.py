@@ -171,3 +171,28 @@ def test_tiled_order_in_passes(engine):
         i = order[a:a + 200_000]
         assert torch.equal(P[a:a + 200_000], (W[rows[i].long()] * H[cols[i].long()]).sum(1)), a
     plan.close()
+
+
+@pytest.mark.parametrize("K,N,bf16", [(580, 180_000, False), (1024, 930_000, True)])
+def test_subnormal_sums_in_passes(engine, K, N, bf16):
+    # products that are multiples of 2^-142 and whose sums stay below 2^-126: exact in fp32 as long as no pass makes zeros of them
+    M, nnz = 20_011, 1_000_003
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H = (torch.randint(-2, 3, (n, K), generator=g, device="cuda").float() * 2.0 ** -71 for n in (M, N))
+    flag = 0
+    if bf16:
+        W, H, flag = W.bfloat16(), H.bfloat16(), api.FLAG_OPERANDS_BF16
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    S = torch.full((nnz,), 2.0 ** 100, device="cuda")
+    n0 = engine.kernel_launches()
+    P, scaled = (torch.full((nnz,), float("nan"), device="cuda") for _ in range(2))
+    plan.execute(W, H, P, None, flag)
+    plan.execute(W, H, scaled, S, flag)
+    assert engine.kernel_launches() - n0 == 2 * 4      # three later passes, two of them between the first and the last
+    for a in range(0, nnz, 200_000):
+        i = slice(a, a + 200_000)
+        ref = (W[rows[i].long()].double() * H[cols[i].long()].double()).sum(1)
+        assert torch.equal(P[i].double(), ref) and torch.equal(scaled[i].double(), ref * 2.0 ** 100)
+    plan.close()
