@@ -435,10 +435,20 @@ template <class S>
 unsigned run_length(int64_t nnz, int sm_count)
 {
     const int64_t wave = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G, s = nnz / wave + 1;
-    // (one nonzero at a time, B = 1, the roundings of a long row are as many as the run is long: no longer runs than 80 to 160)
-    const int64_t waves = S::B == 1 ? (s <= 480 ? (s + 79) / 80 : s <= 1920 ? (s + 159) / 160 : 12)
-                          : S::FUSED ? (s <= 120 ? 1 : s <= 330 ? 2 : s > 1500 ? (s + 299) / 300 : (s + 169) / 170)
-                                     : s <= 340 ? 1 : std::max<int64_t>(2, (s + 759) / 760);
+    int64_t waves;
+    if (S::B == 1) {
+        // One nonzero at a time: a row that fills a run has as many roundings one after the other as the run is long.  24 nonzeros and up to a
+        // third of a set's share, 80 and up to a sixth, 160 and up to a twelfth.
+        waves = s <= 240 ? std::min<int64_t>(3, (s + 23) / 24) : s <= 480 ? (s + 79) / 80 : std::min<int64_t>(12, std::max<int64_t>(6, (s + 159) / 160));
+    } else {
+        // B at a time (add_block): a B-th of the roundings.  At most as many as where one at a time is added, and 80 up to 1,920 nonzeros.
+        // (Error over the sum of magnitudes, rms of all entries; one at a time / the waves of the table alone / with this limit.
+        // K = 200, 8 M nonzeros, rows of 700: 9.9e-8 / 2.8e-7 / 9.0e-8;  K = 64, 28 M: 9.9e-8 / 2.0e-7 / 9.3e-8.)
+        const int64_t chain = s < 240 ? std::max<int64_t>(24, s / 3) : std::max<int64_t>(80, s / 24);
+        waves = S::FUSED ? (s <= 120 ? 1 : s <= 330 ? 2 : s > 1500 ? (s + 299) / 300 : (s + 169) / 170)
+                         : s <= 340 ? 1 : std::max<int64_t>(2, (s + 759) / 760);
+        waves = std::max(waves, (s + S::B * chain - 1) / (S::B * chain));
+    }
     const int64_t run = (nnz / (waves * wave) + S::NB) / S::NB * S::NB;  // rounded up: one run less than a wave, not one more
     return (unsigned)std::min<int64_t>(run, SP_MAX_RUN);
 }

@@ -112,3 +112,26 @@ def test_long_rows_in_passes(engine, K, N):
         plan.spmm(H, again, pv)
         assert torch.equal(Y, again)
     plan.close()
+
+
+@pytest.mark.parametrize("K,M,n,block,chain", [(200, 11_400, 700, 2, 80), (64, 40_000, 700, 4, 80), (576, 3_550, 80, 1, 32)])
+def test_rounding_of_long_rows(engine, K, M, n, block, chain):
+    # Rows of n positive terms, all of them as large on average.  A run adds at most `chain` times to a row's sum one after the other, `block`
+    # nonzeros at a time, so the row is p = n / (chain block) such chains.  With an error of 2^-24 / sqrt(3) rms for every rounding, relative to the
+    # partial sum: chain / 3 p from the chains, p / 3 from adding them up, 1 for the products.
+    import torch
+    N = 20_000
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.arange(M, device="cuda", dtype=torch.int32).repeat_interleave(n)
+    cols = torch.randint(0, N, (M, n), generator=g, device="cuda").sort(dim=1).values
+    H, vals = torch.rand((N, K), generator=g, device="cuda"), torch.rand((M, n), generator=g, device="cuda")
+    plan = engine.plan_coo(M, N, rows, cols.flatten().to(torch.int32), K)
+    Y = torch.full((M, K), float("nan"), device="cuda")
+    plan.spmm(H, Y, vals.flatten())
+    plan.close()
+    square = 0.0
+    for a in range(0, M, 200):
+        ref = torch.einsum("mn,mnk->mk", vals[a:a + 200].double(), H[cols[a:a + 200]].double())
+        square += float(((Y[a:a + 200].double() - ref) / ref).square().sum())
+    p = n / (chain * block)
+    assert (square / (M * K)) ** 0.5 <= 2.0 ** -24 / 3 ** 0.5 * (chain / (3 * p) + p / 3 + 1) ** 0.5
