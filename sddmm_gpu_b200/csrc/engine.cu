@@ -404,6 +404,8 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
 {
     sddmm_handle_s *h = p->h;
     p->pending = true;  // (sddmm_execute clears it again when it waits)
+    // the split of the whole matrix: a chunk of it is summed in the order that the whole would be
+    const GatherPasses passes = gather_passes(p->nnz, p->N, p->K, sval, P);
     rows += first;
     if (perm) {
         perm += first;
@@ -417,7 +419,6 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
         return launch_ring(rows, (hinted ? p->d_cols_hint : cols) + first, perm, sval, W, H, P, count, p->K, hinted, h->sm_count,
                            h->d_work_counter, h->d_status, stream);
     }
-    const GatherPasses passes = gather_passes(count, p->N, p->K, sval, P);
     if (!perm) h->n_launches += passes.n - 1;
     return launch_gather(rows, cols + first, perm, sval, W, H, P, count, p->K, passes, h->sm_count, clock, stream, beside);
 }

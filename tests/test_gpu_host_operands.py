@@ -87,3 +87,22 @@ def test_chunks_taken_together_for_a_pageable_result(engine):
         plan.execute(operand, H, Pp, vals)
         assert plan.last_kernel_ms() > 0 and np.array_equal(Pp.numpy(), P)
     plan.close()
+
+
+def test_chunks_are_split_as_the_whole(engine):
+    # 77 MB of W in two chunks of 0.6 M nonzeros, of a matrix of 1.2 M that is multiplied in two passes over the columns: the chunks as well,
+    # so that P has the same bits wherever W is
+    M, N, K, nnz = 50_003, 300_007, 384, 1_200_007
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H = (torch.randn((n, K), generator=g, device="cuda") for n in (M, N))
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    P, P_host = torch.full((nnz,), float("nan"), device="cuda"), torch.full((nnz,), float("nan")).pin_memory()
+    n0 = engine.kernel_launches()
+    plan.execute(W, H, P)
+    assert engine.kernel_launches() - n0 == 2
+    plan.execute(W.cpu().pin_memory(), H, P_host)
+    assert plan.last_kernel_name() == "gather (pipelined chunks)" and plan.last_kernel_ms() > 0
+    assert torch.equal(P.cpu(), P_host)
+    plan.close()
