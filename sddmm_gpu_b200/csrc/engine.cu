@@ -417,7 +417,7 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
         // the marks are in the plan's processing order: not for the dense-cell remainder
         const bool hinted = p->d_cols_hint && cols == (p->d_perm ? p->d_cols_t : p->d_cols);
         return launch_ring(rows, (hinted ? p->d_cols_hint : cols) + first, perm, sval, W, H, P, count, p->K, hinted, h->sm_count,
-                           h->d_work_counter, h->d_status, stream);
+                           h->work_counter(), h->d_status, stream);
     }
     if (!perm) h->n_launches += passes.n - 1;
     return launch_gather(rows, cols + first, perm, sval, W, H, P, count, p->K, passes, h->sm_count, clock, stream, beside);
@@ -477,7 +477,7 @@ int sddmm_create(sddmm_handle_t *out, int device)
     }
     if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_clocks, 2 * sizeof(unsigned long long) * N_KERNEL_CLOCKS);
     if (e == cudaSuccess) e = cudaMemset(h->d_clocks, 0, 2 * sizeof(unsigned long long) * N_KERNEL_CLOCKS);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_work_counter, sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_work_counters, sizeof(unsigned long long) * SDDMM_WORK_COUNTERS);
     // mapped host memory: the status word, and at 64 bytes the words that plan-time kernels answer in
     if (e == cudaSuccess) e = cudaHostAlloc((void **)&h->h_status, 64 + sizeof(unsigned long long) * PICK_MAX, cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&h->d_status, h->h_status, 0);
@@ -521,7 +521,7 @@ int sddmm_destroy(sddmm_handle_t h)
     if (h->d_plan_words) cudaFree(h->d_plan_words);
     for (cudaEvent_t e : h->ev_plan) if (e) cudaEventDestroy(e);
     h->pool.release();
-    if (h->d_work_counter) cudaFree(h->d_work_counter);
+    if (h->d_work_counters) cudaFree(h->d_work_counters);
     if (h->h_status) cudaFreeHost(h->h_status);
     if (h->pipe_compute) cudaStreamDestroy(h->pipe_compute);
     if (h->pipe_download) cudaStreamDestroy(h->pipe_download);
@@ -759,7 +759,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             LAUNCH_TRY(h, launch_gather_bf16(rows_p, cols_p, perm_p, Sval, W, H, P, p->nnz, p->N, p->K, h->sm_count, timer.clk, s));
         else
             LAUNCH_TRY(h, launch_ring_bf16(rows_p, p->d_cols_hint ? p->d_cols_hint : cols_p, perm_p, Sval, W, H, P, p->nnz, p->K,
-                                           p->d_cols_hint != nullptr, h->sm_count, h->d_work_counter, h->d_status, s));
+                                           p->d_cols_hint != nullptr, h->sm_count, h->work_counter(), h->d_status, s));
         CUDA_TRY(h, timer.end(s));
         if (async) return SDDMM_OK;
         CUDA_TRY(h, cudaStreamSynchronize(s));

@@ -19,6 +19,7 @@ using namespace sddmm;
 #define SDDMM_PIPE_MAX_CHUNKS 16
 
 #define SDDMM_EVENT_PAIRS 8
+#define SDDMM_WORK_COUNTERS 1024
 
 struct sddmm_handle_s {
     int device = 0;
@@ -35,7 +36,10 @@ struct sddmm_handle_s {
     int next_pair = 0;
     int *h_status = nullptr;  // status word of bounded waits, in mapped host memory
     int *d_status = nullptr;  // its device address
-    unsigned long long *d_work_counter = nullptr;  // dynamic work distribution of the ring kernel
+    // dynamic work distribution of the ring kernel: a counter for each launch, taken in turn, since launches on other streams may overlap
+    unsigned long long *d_work_counters = nullptr;
+    unsigned next_work_counter = 0;
+    unsigned long long *work_counter() { return d_work_counters + next_work_counter++ % SDDMM_WORK_COUNTERS; }
     // kernel clocks (two words each) of plans whose last synchronous call was a single gather launch
     unsigned long long *d_clocks = nullptr;
     unsigned long long *d_plan_words = nullptr;                          // of scan_coo

@@ -134,6 +134,34 @@ def test_overlapping_spmm_calls_of_one_plan(engine):
     plan.close()
 
 
+def test_overlapping_ring_calls(engine):
+    """Asynchronous calls on two streams through the kernel whose warps take their share of the work from a counter: a large one
+    is under way when a small one begins."""
+    K, N = 256, 60_000
+    g = torch.Generator(device="cuda").manual_seed(0)
+    plans, calls = [], []
+    for M, nnz in ((50_000, 12_000_000), (3_000, 40_000)):
+        rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+        cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+        W, H = (torch.randn((n, K), generator=g, device="cuda") for n in (M, N))
+        plan, expect = engine.plan_coo(M, N, rows, cols, K), torch.empty(nnz, device="cuda")
+        plan.execute(W, H, expect, None, api.FLAG_KERNEL_RING)
+        plans.append((plan, rows, cols))
+        calls.append((plan, W, H, expect))
+    streams = [torch.cuda.Stream() for _ in calls]
+    for _ in range(3):
+        out = [torch.full_like(expect, float("nan")) for _, _, _, expect in calls]
+        torch.cuda.synchronize()
+        for stream, (plan, W, H, _), P in zip(streams, calls, out):
+            with torch.cuda.stream(stream):
+                plan.execute(W, H, P, None, api.FLAG_ASYNC | api.FLAG_KERNEL_RING)
+        torch.cuda.synchronize()
+        for P, (_, _, _, expect) in zip(out, calls):
+            assert torch.equal(P, expect)
+    for plan, _, _ in plans:
+        plan.close()
+
+
 def test_plan_destroyed_behind_a_queued_row_upload(engine):
     """The list of used rows belongs to the plan and is read by uploads on any stream: destroying the plan waits for them, and
     the memory of the list goes to the next plan only then."""
