@@ -152,6 +152,7 @@ bool ring_supports(int K);
 inline bool rows_path_supports(int K) { return K == 32 || K == 64 || K == 128 || K == 256 || K == 512 || K == 1024; }
 // Whether the ring kernel is the faster one for an H of N rows (see sddmm_ring.cu).
 bool ring_preferred(int64_t N, int K);
+bool ring_few(int64_t nnz, int row_bytes);  // ... also where the nonzeros are in input order
 // cols_hinted: bit 31 of every column index marks a hub column (see build_hub_column_hints).
 cudaError_t launch_ring(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t nnz, int K, bool cols_hinted, int sm_count,

@@ -395,7 +395,7 @@ namespace sddmm {
 
 bool rows_on_ring(const sddmm_plan_s *p, bool force_ring, bool permuted)
 {
-    return ring_supports(p->K) && (force_ring || (permuted && ring_preferred(p->N, p->K)));
+    return ring_supports(p->K) && (force_ring || (ring_preferred(p->N, p->K) && (permuted || ring_few(p->nnz, p->K * 4))));
 }
 
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,

@@ -342,8 +342,9 @@ cudaError_t launch_pieces(const GatherCall &c)
 //   K = 512: 300 K rows 607 -> 773 / 666 / 635; 700 K 1245 -> 1381 / 1253 / 1214; 1.5 M 3052 -> 3053 / 2894 / 2830
 //   K = 768: 100 K rows, 1.2 M nonzeros 255 -> 392 / 295 / 255; 200 K, uniform, 2 M 972 -> 712 / 646 / 770; 150 K, uniform, 0.3 M 197 -> 228
 //   / 190 / 217; 700 K, 8.4 M 2356 -> 2081 / 1836 / 1822; 1.5 M, 18 M 5688 -> 4545 / 4267 / 4212
-//   few nonzeros, H of 1.8 to 2 GB, one pass -> passes of 192: 0.95 M, K = 512 192 -> 191, K = 768 314 -> 270, K = 1024 439 -> 358; 0.6 M, K = 384 108 -> 104;
-//   0.4 M, K = 512 102 -> 106, K = 768 153 -> 147, K = 1024 207 -> 195
+//   few nonzeros, H of 1.6 and of 3.2 GB, one pass -> passes of 192 (K = 512 and 1024: see ring_few), all columns alike; R-MAT:
+//   K = 384: 0.25 M 90 -> 91, 90 -> 92, 60 -> 63, 70 -> 71; 0.5 M 156 -> 153, 158 -> 156, 105 -> 105, 125 -> 124; 1 M 271 -> 253, 277 -> 262, 182 -> 172, 213 -> 202
+//   K = 768: 0.25 M 167 -> 179, 169 -> 183, 107 -> 113, 126 -> 125; 0.5 M 296 -> 293, 300 -> 307, 187 -> 180, 223 -> 211; 1 M 522 -> 474, 531 -> 507, 327 -> 292, 387 -> 343
 //   K = 1028: 20 K rows, 0.24 M 105 -> 205 / 143 / 134; 100 K, 1.2 M 548 -> 551 / 426 / 384; 1 M, 12 M 6685 -> 4807 / 4261 / 4189
 GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, const float *P)
 {
@@ -353,7 +354,7 @@ GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, con
     int floats = K;
     if (K > 320) {
         // (the shape for 512 floats is the one that holds its own longest)
-        if (nnz >= (h_bytes >= 1500000000 ? 250000 : 1000000) && h_bytes >= (K > 480 && K <= 512 ? 1000000000 : 400000000)) floats = N > 2000000 ? 96 : 192;
+        if (nnz >= (h_bytes >= 1500000000 ? 500000 : 1000000) && h_bytes >= (K > 480 && K <= 512 ? 1000000000 : 400000000)) floats = N > 2000000 ? 96 : 192;
     } else if (K > 192 && h_bytes >= 4000000000 && nnz >= 16 * N) {
         floats = 64;
     }

@@ -27,11 +27,11 @@
 // memory, L1/L2) only when the row changes -- one group ahead, right after the
 // previous group's FMAs.
 //
-// Used for K = 256, 512 and 1024 (C = 2, 4, 8) where the nonzeros come through a permutation (column tiles, the buckets of a broadcast H) and H is
-// far larger than L2 (ring_preferred): there most gathers
-// come from DRAM, whose latency the deep rings hide, and the copies
-// carry the plan's hub-column hints; and for bfloat16 rows of K = 2048.  Everything else is the gather kernel's (sddmm_gather.cu), which
-// in its passes over part of the columns is ahead of the rings at every size (97 M nonzeros, 4.2 M rows of H, K = 256: 9330 -> 8340 us).
+// Used for K = 256, 512 and 1024 (C = 2, 4, 8) where H is far larger than L2 and the nonzeros come through a permutation (column tiles, the
+// buckets of a broadcast H; ring_preferred) or are few (ring_few): there most gathers come from DRAM, whose latency the deep rings hide; under a
+// permutation the copies carry the plan's hub-column hints.  And for bfloat16 rows of K = 2048.  Everything else is the gather kernel's
+// (sddmm_gather.cu), which from a million nonzeros on is ahead in its passes over part of the columns (97 M nonzeros, 4.2 M rows of H, K = 256:
+// 9330 -> 8340 us).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -372,6 +372,15 @@ bool ring_supports(int K) { return K == 256 || K == 512 || K == 1024; }
 // K = 256: 0.27 GB 0.28 / 0.37, 1.1 GB 1.15 / 1.25, 2.6 GB 1.95 / 1.90, 4.3 GB 8.7 / 8.3;
 // K = 512: 0.5 GB 0.52 / 0.60, 1.1 GB 1.27 / 1.31, 2.1 GB 2.40 / 2.28;  K = 1024: 4.3 GB 6.2 / 5.0.
 bool ring_preferred(int64_t N, int K) { return ring_supports(K) && N * K * 4 >= (3ll << 29); }
+// Nonzeros in input order, by what they bring from such an H: too few for passes of the gather kernel to pay, too many for what the rings cost at
+// the start, and rows so long that the gather kernel holds few of them in flight (us, gather kernel in one pass / in passes / rings without hub
+// marks; H of 1.6 and of 3.2 GB, all columns alike; R-MAT):
+// K = 512: 0.1 M nonzeros 53.5 / 69.7 / 54.7, 35.9 / 51.6 / 36.7;  0.25 M 125 / 123 / 109, 127 / 126 / 110, 84 / 83 / 73, 103 / 94 / 83;  0.5 M 195 / 202 / 190,
+//   197 / 209 / 195, 133 / 136 / 130, 165 / 159 / 149;  1 M 334 / 333 / 341, 340 / 350 / 349, 225 / 222 / 230, 277 / 258 / 269;
+// K = 1024: 0.02 M 29.9 / 61.5 / 29.9;  0.1 M 111 / 135 / 105, 68 / 92 / 63;  0.25 M 233 / 236 / 211, 146 / 150 / 131;  0.5 M 388 / 380 / 370, 395 / 408 / 375, 249 / 238 /
+//   234, 296 / 273 / 276;  1 M 704 / 614 / 663, 715 / 671 / 676, 450 / 377 / 423;
+// K = 256 (1 KB) 0.1 M 31.1 / - / 32.9, 0.4 M 87 / - / 87, 1 M 171 / - / 183.
+bool ring_few(int64_t nnz, int row_bytes) { return row_bytes >= 2048 && nnz * row_bytes >= (1ll << 28) && nnz < 1000000; }
 
 cudaError_t launch_ring(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t nnz, int K, bool cols_hinted, int sm_count,

@@ -196,3 +196,30 @@ def test_subnormal_sums_in_passes(engine, K, N, bf16):
         ref = (W[rows[i].long()].double() * H[cols[i].long()].double()).sum(1)
         assert torch.equal(P[i].double(), ref) and torch.equal(scaled[i].double(), ref * 2.0 ** 100)
     plan.close()
+
+
+def _sampled_pattern(M, N, nnz, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    return rows, torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+
+
+@pytest.mark.parametrize("K,N,edges", [(512, 790_000, (131_071, 131_073, 999_999)), (1024, 394_000, (65_535, 65_539, 999_999))])
+def test_few_nonzeros_of_a_large_H(engine, K, N, edges):
+    # rows of 2 KB and more of an H of 1.6 GB: from 256 MB of rows to a million nonzeros the ring kernel, on whole rows, as the gather kernel below
+    M = 20_011
+    W, H = (torch.randint(-2, 3, (n, K), device="cuda").float() for n in (M, N))   # every product and sum exact
+    for nnz, kernel in zip(edges, ("gather", "ring", "ring")):
+        rows, cols = _sampled_pattern(M, N, nnz, nnz)
+        S = torch.randint(-3, 4, (nnz,), device="cuda").float()
+        plan = engine.plan_coo(M, N, rows, cols, K)
+        n0 = engine.kernel_launches()
+        P, inside = torch.full((nnz,), float("nan"), device="cuda"), S.clone()
+        plan.execute(W, H, P, S)
+        assert plan.last_kernel_name() == kernel and engine.kernel_launches() - n0 == 1 and plan.last_kernel_ms() > 0
+        plan.execute(W, H, inside, inside)     # S and P in one array
+        for a in range(0, nnz, 100_000):
+            i = slice(a, a + 100_000)
+            assert torch.equal(P[i], (W[rows[i].long()] * H[cols[i].long()]).sum(1) * S[i]), a
+        assert torch.equal(P, inside)
+        plan.close()
