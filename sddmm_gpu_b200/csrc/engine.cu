@@ -747,9 +747,10 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
         const int32_t *rows_p = tiled ? p->d_rows_t : p->d_rows, *cols_p = tiled ? p->d_cols_t : p->d_cols;
         const int32_t *perm_p = tiled ? p->d_perm : nullptr;
         // rows of half the bytes: the same line between the two kernels as for fp32 rows of K / 2
-        const bool gather = gather_bf16_supports(p->K) && !(flags & SDDMM_FLAG_KERNEL_RING) && !(tiled && ring_preferred(p->N / 2, p->K));
+        const bool few = !tiled && !(flags & SDDMM_FLAG_KERNEL_RING) && ring_few(p->nnz, p->K * 2);
+        const bool gather = gather_bf16_supports(p->K) && !(flags & SDDMM_FLAG_KERNEL_RING) && !(ring_preferred(p->N / 2, p->K) && (tiled || few));
         const int passes = gather && !tiled ? gather_passes_bf16(p->nnz, p->N, p->K, Sval, P).n : 1;
-        if (!gather) CUDA_TRY(h, ensure_hints(p));
+        if (!gather && !few) CUDA_TRY(h, ensure_hints(p));
         p->last_kernel = gather ? "gather (bf16 operands)" : "ring (bf16 operands)";
         p->last_h2d_bytes = p->last_d2h_bytes = 0;
         CallTimer timer(p, async);

@@ -408,11 +408,15 @@ bool gather_bf16_supports(int K) { return K == 256 || K == 512 || K == 1024; }
 
 // Passes of 256 values, sustained us, the ring kernel / one pass / these: K = 1024, 0.3 M rows of H - / 544 / 583, 0.7 M 1394 / 1406 / 1405, 1 M 2775 / 2747 /
 // 2600, 1.5 M 4320 / 4466 / 4119;  K = 512, 1.5 M 2036 / 2047 / 2038, 4.2 M 9298 / 9264 / 8920;  K = 256, 4.2 M 4864 / 4218 / -.
+// From a million nonzeros and one for each row of H on; K = 1024 below a million on the rings (ring_few).  All columns alike, R-MAT: K = 512, H of 4.3 GB, 0.3 M nonzeros 68 / 66 / 78,
+// 60 / 55 / 66; 1 M 179 / 177 / 188, 161 / 164 / 162; 3 M 490 / 488 / 483, 412 / 422 / 393;  K = 1024, 2.1 GB, 0.02 M 18.5 / 16.4 / 41; 0.3 M 128 / 136 / 154,
+// 88 / 101 / 110; 1 M 345 / 337 / 349, 239 / 243 / 253; 3 M 934 / 896 / 872, 628 / 611 / 598;  4.3 GB, 1 M 351 / 342 / 368, 274 / 294 / 285; 3 M 953 / 913 / 934,
+// 706 / 718 / 683.
 GatherPasses gather_passes_bf16(int64_t nnz, int64_t N, int K, const float *sval, const float *P)
 {
     const GatherPasses whole = {1, K};
     if (sval && sval < P + nnz && P < sval + nnz) return whole;
-    return N * K * 2 >= (K >= 1024 ? 1900000000 : 4000000000) && K > 256 ? GatherPasses{K / 256, 256} : whole;
+    return nnz >= 1000000 && nnz >= N && N * K * 2 >= (K >= 1024 ? 1900000000 : 4000000000) && K > 256 ? GatherPasses{K / 256, 256} : whole;
 }
 
 cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval, const void *W,

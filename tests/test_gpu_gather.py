@@ -223,3 +223,19 @@ def test_few_nonzeros_of_a_large_H(engine, K, N, edges):
             assert torch.equal(P[i], (W[rows[i].long()] * H[cols[i].long()]).sum(1) * S[i]), a
         assert torch.equal(P, inside)
         plan.close()
+
+
+def test_few_nonzeros_of_a_large_bf16_H(engine):
+    # whole rows through the gather kernel and through the ring kernel, one launch each; four passes from a million nonzeros on
+    M, N, K = 20_011, 930_000, 1024
+    W, H = (torch.randint(-2, 3, (n, K), device="cuda").bfloat16() for n in (M, N))   # every product and sum exact
+    for nnz, kernel, launches in ((20_001, "gather", 1), (131_073, "ring", 1), (999_999, "ring", 1), (1_000_001, "gather", 4)):
+        rows, cols = _sampled_pattern(M, N, nnz, nnz)
+        plan = engine.plan_coo(M, N, rows, cols, K)
+        P, n0 = torch.full((nnz,), float("nan"), device="cuda"), engine.kernel_launches()
+        plan.execute(W, H, P, None, api.FLAG_OPERANDS_BF16)
+        assert plan.last_kernel_name() == kernel + " (bf16 operands)" and engine.kernel_launches() - n0 == launches
+        for a in range(0, nnz, 100_000):
+            i = slice(a, a + 100_000)
+            assert torch.equal(P[i], (W[rows[i].long()].float() * H[cols[i].long()].float()).sum(1)), a
+        plan.close()
