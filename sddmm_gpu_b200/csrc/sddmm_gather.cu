@@ -346,6 +346,18 @@ cudaError_t launch_pieces(const GatherCall &c)
 //   K = 384: 0.25 M 90 -> 91, 90 -> 92, 60 -> 63, 70 -> 71; 0.5 M 156 -> 153, 158 -> 156, 105 -> 105, 125 -> 124; 1 M 271 -> 253, 277 -> 262, 182 -> 172, 213 -> 202
 //   K = 768: 0.25 M 167 -> 179, 169 -> 183, 107 -> 113, 126 -> 125; 0.5 M 296 -> 293, 300 -> 307, 187 -> 180, 223 -> 211; 1 M 522 -> 474, 531 -> 507, 327 -> 292, 387 -> 343
 //   K = 1028: 20 K rows, 0.24 M 105 -> 205 / 143 / 134; 100 K, 1.2 M 548 -> 551 / 426 / 384; 1 M, 12 M 6685 -> 4807 / 4261 / 4189
+// Where rows are no multiple of 128 bytes, neighbouring passes touch the same lines: a pass of 192 then costs a sixth more, and a last one
+// of a few columns as much as a third of that (12 nonzeros a row; one pass -> 192, all columns alike, R-MAT).  It still pays up to 384 columns, and
+// from 640 on, where one pass runs on few warps:
+//   K = 324, H of 1.3 GB 2890 -> 2861, 1564 -> 1378;  3 GB 6826 -> 6879, 4172 -> 3598;   K = 392 2543 -> 2920, 1406 -> 1333;  6023 -> 7054, 3604 -> 3449
+//   K = 452 2541 -> 2785, 1358 -> 1293;  6020 -> 6836, 3542 -> 3345;   K = 584 2490 -> 2755, 1273 -> 1237;  5904 -> 6799, 3417 -> 3225
+//   K = 644 2705 -> 2674, 1453 -> 1237;  6384 -> 6683, 3908 -> 3122;   K = 780 2490 -> 2659, 1343 -> 1216;  5891 -> 6715, 3501 -> 3087;  0.6 GB 1092 -> 1008, 540 -> 536
+//   K = 900 2707 -> 2523, 1546 -> 1188;  6366 -> 6463, 4013 -> 2995;   K = 1060 2677 -> 2451, 1930 -> 1168;  6394 -> 6364, 4817 -> 2919
+// and with rows that are: K = 352 2662 -> 2425, 1445 -> 1221;  6265 -> 5880, 3785 -> 3085;   K = 416 2420 -> 2474, 1341 -> 1196;  5738 -> 5979, 3474 -> 3074
+//   K = 512 2380 -> 2305, 1223 -> 1129;  5642 -> 5673, 3254 -> 2885;   K = 640 2382 -> 2261, 1162 -> 1098;  5647 -> 5624, 3334 -> 2793
+// 193 to 320 columns, 16 nonzeros a row, one pass -> 64: K = 256, 4.3 GB 10612 -> 10663, 6403 -> 5979;  8.2 GB 20431 -> 21017, 12972 -> 12923;  16 GB 40877 -> 43462,
+//   28282 -> 27961;   K = 320, 4.5 GB 11657 -> 11535, 6863 -> 6515;   K = 224, 4.1 GB 10898 -> 11299, 6617 -> 6412;   K = 196 12237 -> 16677, 7471 -> 8135;
+//   K = 260 12684 -> 17282, 7300 -> 8052;   K = 300 14697 -> 19795, 8501 -> 9396
 GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, const float *P)
 {
     const GatherPasses whole = {1, K};
@@ -353,9 +365,12 @@ GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, con
     const int64_t h_bytes = N * K * 4;
     int floats = K;
     if (K > 320) {
-        // (the shape for 512 floats is the one that holds its own longest)
-        if (nnz >= (h_bytes >= 1500000000 ? 500000 : 1000000) && h_bytes >= (K > 480 && K <= 512 ? 1000000000 : 400000000)) floats = N > 2000000 ? 96 : 192;
-    } else if (K > 192 && h_bytes >= 4000000000 && nnz >= 16 * N) {
+        const bool lines = K % 32 == 0;
+        const bool pays = lines || K <= 384 || K > 1024 || (K > 640 && (K % 192 >= 32 || h_bytes < 1000000000));
+        // (the shapes for 512 and 640 floats are the ones that hold their own longest)
+        if (pays && nnz >= (h_bytes >= 1500000000 ? 500000 : 1000000) && h_bytes >= (K > 480 && K <= 640 ? 1000000000 : 400000000))
+            floats = lines && N > 2000000 ? 96 : 192;
+    } else if (K > 192 && K % 64 == 0 && h_bytes >= 4000000000 && h_bytes < 8000000000 && nnz >= 16 * N) {
         floats = 64;
     }
     return floats < K ? GatherPasses{(K + floats - 1) / floats, floats} : whole;
