@@ -99,8 +99,8 @@ PanelConfig choose_panel_config(int K, int panel_rows_hint, int sm_count, size_t
 struct GatherPasses {
     int n, floats;  // launches, columns of each (the last one may have fewer)
 };
-// What is best for an H of N rows; one pass where S values and P share memory.
-GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, const float *P);
+// What is best for an H of N rows; one pass where S values and P share memory.  tiled: the nonzeros are in the order of column tiles.
+GatherPasses gather_passes(int64_t nnz, int64_t N, int K, bool tiled, const float *sval, const float *P);
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                           const float *W, const float *H, float *P, int64_t nnz, int K, GatherPasses passes, int sm_count,
                           unsigned long long *clock, cudaStream_t stream, bool beside = false);

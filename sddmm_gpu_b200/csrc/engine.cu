@@ -405,7 +405,7 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
     sddmm_handle_s *h = p->h;
     p->pending = true;  // (sddmm_execute clears it again when it waits)
     // the split of the whole matrix: a chunk of it is summed in the order that the whole would be
-    const GatherPasses passes = gather_passes(p->nnz, p->N, p->K, sval, P);
+    const GatherPasses passes = gather_passes(p->nnz, p->N, p->K, p->d_perm && !perm, sval, P);
     rows += first;
     if (perm) {
         perm += first;
@@ -863,7 +863,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     // a call that is one gather launch is timed by the kernel itself, everything else by events
     const bool permuted = p->d_perm && !tiled_out;
     const bool one_gather = !use_dense && !use_panel && (use_gather || !rows_on_ring(p, use_ring, permuted)) &&
-                            (permuted || use_gather || gather_passes(p->nnz, p->N, p->K, dS, P).n == 1);
+                            (permuted || use_gather || gather_passes(p->nnz, p->N, p->K, p->d_perm != nullptr, dS, P).n == 1);
     bool p_copy = false;
     if (!p_dev) {
         // a small P is written to mapped host memory by the kernel: its 32-byte stores over PCIe cost less than a copy
@@ -1348,7 +1348,7 @@ int sddmm_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const int32_t
         dp = (float *)tmp.p[5];
     }
     CUDA_TRY(h, launch_gather((const int32_t *)dr, (const int32_t *)dc, nullptr, (const float *)ds, (const float *)dw,
-                              (const float *)dh, dp, nnz, K, gather_passes(nnz, N, K, (const float *)ds, dp), h->sm_count, nullptr, s));
+                              (const float *)dh, dp, nnz, K, gather_passes(nnz, N, K, false, (const float *)ds, dp), h->sm_count, nullptr, s));
     if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dp, sizeof(float) * nnz, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
     return SDDMM_OK;

@@ -358,7 +358,9 @@ cudaError_t launch_pieces(const GatherCall &c)
 // 193 to 320 columns, 16 nonzeros a row, one pass -> 64: K = 256, 4.3 GB 10612 -> 10663, 6403 -> 5979;  8.2 GB 20431 -> 21017, 12972 -> 12923;  16 GB 40877 -> 43462,
 //   28282 -> 27961;   K = 320, 4.5 GB 11657 -> 11535, 6863 -> 6515;   K = 224, 4.1 GB 10898 -> 11299, 6617 -> 6412;   K = 196 12237 -> 16677, 7471 -> 8135;
 //   K = 260 12684 -> 17282, 7300 -> 8052;   K = 300 14697 -> 19795, 8501 -> 9396
-GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, const float *P)
+// In the order of column tiles a tile's rows of H stay in L2 as they are: K = 256, 67 M nonzeros, tiles of 65,536 columns, R-MAT 5470 -> 6932.  Longer rows gain
+// all the same (their rows of W are read again for every tile): K = 512, 18 M, tiles of 32,768, one pass -> 192 10656 -> 8919, 3129 -> 3082.
+GatherPasses gather_passes(int64_t nnz, int64_t N, int K, bool tiled, const float *sval, const float *P)
 {
     const GatherPasses whole = {1, K};
     if (sval && sval < P + nnz && P < sval + nnz) return whole;  // the first pass would overwrite S values that the last one needs
@@ -370,7 +372,7 @@ GatherPasses gather_passes(int64_t nnz, int64_t N, int K, const float *sval, con
         // (the shapes for 512 and 640 floats are the ones that hold their own longest)
         if (pays && nnz >= (h_bytes >= 1500000000 ? 500000 : 1000000) && h_bytes >= (K > 480 && K <= 640 ? 1000000000 : 400000000))
             floats = lines && N > 2000000 ? 96 : 192;
-    } else if (K > 192 && K % 64 == 0 && h_bytes >= 4000000000 && h_bytes < 8000000000 && nnz >= 16 * N) {
+    } else if (K > 192 && K % 64 == 0 && !tiled && h_bytes >= 4000000000 && h_bytes < 8000000000 && nnz >= 16 * N) {
         floats = 64;
     }
     return floats < K ? GatherPasses{(K + floats - 1) / floats, floats} : whole;

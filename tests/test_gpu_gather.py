@@ -258,3 +258,20 @@ def test_passes_by_the_lines_of_a_row(engine, K, N, nnz, passes):
         assert torch.equal(P[i], (W[rows[i].long()] * H[cols[i].long()]).sum(1)), a
     assert not torch.isnan(P).any()
     plan.close()
+
+
+def test_tiled_order_of_a_large_H(engine):
+    # K = 256 and an H that input order multiplies in four passes: whole rows in the order of column tiles
+    K, M, N = 256, 20_011, 3_910_001
+    nnz = 16 * N + 5
+    rows, cols = _sampled_pattern(M, N, nnz, K)
+    W, H = (torch.randint(-2, 3, (n, K), device="cuda").float() for n in (M, N))   # every product and sum exact
+    plan = engine.plan_coo(M, N, rows, cols, K, 0, 1_000_000)
+    order = torch.argsort(cols // 1_000_000, stable=True)
+    P, n0 = torch.full((nnz,), float("nan"), device="cuda"), engine.kernel_launches()
+    plan.execute(W, H, P, None, api.FLAG_TILED_ORDER)
+    assert plan.last_kernel_name() == "gather" and engine.kernel_launches() - n0 == 1 and not torch.isnan(P).any()
+    plan.close()
+    for a in range(0, nnz, 6_300_000):
+        i = order[a:a + 6_300_000:63]
+        assert torch.equal(P[a:a + 6_300_000:63], (W[rows[i].long()] * H[cols[i].long()]).sum(1)), a
