@@ -521,10 +521,16 @@ auto with_shape(int K, bool fused, Fn f)
 // SpMM of long rows with a large H in passes of 192 columns (of H and of Y; the fused form needs whole rows).  More gathers of a pass hit L2,
 // and the shapes for more columns hold so many registers that few warps are resident.  Sustained us, one pass / these: K = 384, 0.3 M rows
 // of H 573 / 570, 0.7 M 1166 / 1062, 1 M 2163 / 1975; K = 512, 0.3 M 734 / 782, 0.7 M 1449 / 1453, 1 M 2806 / 2678, 1.5 M 4516 / 4181; K = 256, 1.5 M 2096 / 2138.
+// Rows of whole 128-byte lines, and no narrow last pass: neighbouring passes touch the same lines otherwise (one pass / these, all columns alike, R-MAT: K = 352,
+// 1.8 GB of H 3451 / 3447, 2110 / 2025;  K = 324 3715 / 4062, 2312 / 2353;  K = 388 3608 / 4350, 2168 / 2427;  K = 416 3378 / 3586, 1961 / 2012;  K = 544 3505 / 3372,
+// 2146 / 1896;  K = 608 3453 / 3468, 2058 / 1932;  K = 644 3563 / 3931, 2130 / 2123;  K = 704 3389 / 3291, 2029 / 1799;  K = 772 3596 / 4001, 2203 / 2132).  Above 768
+// columns, where a row whole runs on very few warps, also other rows of an H that is not too large (K = 900, 1.0 GB 1940 / 1891, 1111 / 1089; 1.8 GB 3545 / 3733, 2178 / 1993;
+// K = 1020 1907 / 1806, 1075 / 1043; 3488 / 3656, 2139 / 1973).
 static int pass_floats(int64_t nnz, int64_t N, int K)
 {
     const int64_t h_bytes = N * K * 4;
-    return K > 320 && nnz >= 1000000 && h_bytes >= (K > 480 && K <= 512 ? 1700000000 : 900000000) ? 192 : K;
+    const bool pays = K % 32 == 0 ? K % 192 == 0 || K % 192 >= 64 || K > 512 : K > 768 && h_bytes < 1500000000;
+    return K > 320 && pays && nnz >= 1000000 && h_bytes >= (K > 480 && K <= 512 ? 1700000000 : 900000000) ? 192 : K;
 }
 
 int spmm_passes(int64_t nnz, int64_t N, int K)

@@ -84,9 +84,9 @@ def test_last_nonzero_infinite(engine, K):
         plan.close()
 
 
-@pytest.mark.parametrize("K,N", [(388, 581_000), (512, 831_000), (900, 251_000)])
+@pytest.mark.parametrize("K,N", [(448, 503_000), (512, 831_000), (900, 251_000)])
 def test_long_rows_in_passes(engine, K, N):
-    # a large H, long rows: passes over part of the columns (the last one of 4, 128 and 132), a row of many runs, rows without nonzeros
+    # a large H, long rows: passes over part of the columns (the last one of 64, 128 and 132), a row of many runs, rows without nonzeros
     import torch
     M, nnz = 7_013, 1_000_003
     g = torch.Generator(device="cuda").manual_seed(K)
@@ -135,3 +135,24 @@ def test_rounding_of_long_rows(engine, K, M, n, block, chain):
         square += float(((Y[a:a + 200].double() - ref) / ref).square().sum())
     p = n / (chain * block)
     assert (square / (M * K)) ** 0.5 <= 2.0 ** -24 / 3 ** 0.5 * (chain / (3 * p) + p / 3 + 1) ** 0.5
+
+
+@pytest.mark.parametrize("K,N", [(388, 590_000), (416, 545_000), (644, 354_000), (900, 420_000)])
+def test_long_rows_whole(engine, K, N):
+    # rows that are no multiple of 128 bytes, or whose last pass would be narrow: one launch, however large H is
+    import torch
+    M, nnz = 7_013, 1_000_003
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    H, vals = (torch.randint(-2, 3, n, generator=g, device="cuda").float() for n in ((N, K), (nnz,)))   # every product and sum exact
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    Y, n0 = torch.full((M, K), float("nan"), device="cuda"), engine.kernel_launches()
+    plan.spmm(H, Y, vals)
+    assert engine.kernel_launches() - n0 == 1
+    plan.close()
+    ref = torch.zeros((M, K), device="cuda")
+    for a in range(0, nnz, 100_000):
+        i = slice(a, a + 100_000)
+        ref.index_add_(0, rows[i].long(), vals[i, None] * H[cols[i].long()])
+    assert torch.equal(Y, ref)
