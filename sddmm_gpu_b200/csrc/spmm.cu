@@ -506,7 +506,9 @@ auto with_shape(int K, bool fused, Fn f)
     if (q < 32) return f(SpmmShape<16, 2, 4, false, 3>());
     if (q == 32) return f(SpmmShape<16, 2, 4, true, 4>());
     if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4>());
-    if (q < 64) return f(SpmmShape<32, 2, 2, false, 5>());
+    // (two at a time with five resident blocks spill; us, those one nonzero at a time / with block sums / this: 0.75 M nonzeros, K = 200 63 / 59 / 49; 4.0 M 270 / 289 / 253;
+    // 16 M 1146 / 1232 / 1133; all columns alike, 4.0 M 470 / 464 / 421;  K = 252, 4.0 M 320 / 338 / 293)
+    if (q < 64) return f(SpmmShape<32, 2, 4, false, 3>());
     if (q == 64) return f(SpmmShape<32, 2, 4, true, 4>());
     if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3>());
     if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3>());

@@ -114,7 +114,7 @@ def test_long_rows_in_passes(engine, K, N):
     plan.close()
 
 
-@pytest.mark.parametrize("K,M,n,block,chain", [(200, 11_400, 700, 2, 80), (64, 40_000, 700, 4, 80), (576, 3_550, 80, 1, 32)])
+@pytest.mark.parametrize("K,M,n,block,chain", [(192, 11_400, 700, 2, 80), (200, 11_400, 700, 4, 80), (64, 40_000, 700, 4, 80), (576, 3_550, 80, 1, 32)])
 def test_rounding_of_long_rows(engine, K, M, n, block, chain):
     # Rows of n positive terms, all of them as large on average.  A run adds at most `chain` times to a row's sum one after the other, `block`
     # nonzeros at a time, so the row is p = n / (chain block) such chains.  With an error of 2^-24 / sqrt(3) rms for every rounding, relative to the
