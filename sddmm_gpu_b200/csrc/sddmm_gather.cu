@@ -92,8 +92,9 @@ struct WShare {
 
 // What is multiplied and what becomes of a dot product: whole rows, the product stored (STORE) or stored through perm, the result of nonzero
 // j to P[perm[j]], scaled by sval[perm[j]] (PERM); or one pass over some columns of rows that are `pitch` bytes apart (PASS): stored by
-// the first pass, added to P by the later ones (`add`), scaled by the last.  The sum is read, added to and stored: every entry has one writer, and
-// red.global.add.f32 would make zeros of subnormal sums, which one pass keeps.
+// the first pass, added to P by the later ones (`add`) -- by a reduction that nothing waits for, or, in the last pass (`finish`), read, added and scaled.
+// red.global.add.f32 makes zeros of subnormal numbers, P's own among them.  Beside a part of 2^-100 and more that is less than its rounding; a smaller part is
+// read, added and stored (every entry has one writer), a part that is zero is not added.  (All parts that way: graph of 97 M nonzeros, K = 256 8.6 -> 9.05 ms.)
 enum GatherMode { STORE, PERM, PASS };
 
 // pieces: 16-byte pieces of a row that are multiplied.  run_len: nonzeros of a set, a multiple of S::NB.
@@ -101,7 +102,7 @@ template <class S, GatherMode MODE>
 __global__ void __launch_bounds__(GA_TPB, S::CTAS)
 sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const int32_t *__restrict__ perm,
                     const float *__restrict__ sval, const char *__restrict__ W, const char *__restrict__ H,
-                    float *__restrict__ P, unsigned nnz, int pieces, unsigned pitch, bool add, unsigned run_len, unsigned long long *clock, unsigned meet_from)
+                    float *__restrict__ P, unsigned nnz, int pieces, unsigned pitch, bool add, bool finish, unsigned run_len, unsigned long long *clock, unsigned meet_from)
 {
     clock_begin(clock);
     constexpr bool HAS_PERM = MODE == PERM;
@@ -157,7 +158,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
         if (HAS_PERM && sval) s = __ldg(sval + dst);
         float sum = 0.f;
         // (volatile: it is to be under way while the rows of H are, not waited for at the end of the step)
-        if (MODE == PASS && add && lig < NB) asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(sum) : "l"(P + at(j)));
+        if (MODE == PASS && add && finish && lig < NB) asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(sum) : "l"(P + at(j)));
         float res = 0.f;
 #pragma unroll
         for (int h0 = 0; h0 < NB; h0 += RB) {
@@ -188,7 +189,17 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
             const float t = RB == L ? acc[0] : __shfl_sync(FULL, acc[0], (lig & (RB - 1)) * (L / RB), L);
             if (RB == NB || il / RB == h0 / RB) res = t;
         }
-        if (lig < NB && j < nnz) P[HAS_PERM ? (unsigned)dst : j] = (MODE == PASS ? sum + res : res) * s;
+        if (lig < NB && j < nnz) {
+            if (MODE == PASS && add && !finish) {
+                // (all of it predicated: with a branch around the rare addition 97 M nonzeros took 8.74 ms in place of 8.52)
+                const unsigned small = fabsf(res) < 0x1p-100f;
+                asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %2, 0;\n\t@p red.global.add.f32 [%0], %1;\n\t}" ::"l"(P + j), "f"(res), "r"(small) : "memory");
+                asm volatile("{\n\t.reg .pred p;\n\t.reg .f32 t;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.f32 t, [%0];\n\t@p add.rn.f32 t, t, %1;\n\t@p st.global.f32 [%0], t;\n\t}" ::"l"(P + j),
+                             "f"(res), "r"((unsigned)(small && res != 0.f)) : "memory");
+            } else {
+                P[HAS_PERM ? (unsigned)dst : j] = (MODE == PASS ? sum + res : res) * s;
+            }
+        }
         j += NB;
         r = rn;
         c = cn;
@@ -255,7 +266,7 @@ struct GatherCall {
     int pieces;
     bool pass;         // one of several passes (perm null)
     unsigned pitch;
-    bool add;
+    bool add, finish;
     int sm_count;
     unsigned long long *clock;
     bool beside;
@@ -289,8 +300,8 @@ cudaError_t launch_mode(const GatherCall &c)
     cfg.stream = c.stream;
     cfg.attrs = &attr;
     cfg.numAttrs = c.beside ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, sddmm_gather_kernel<S, MODE>, c.rows, c.cols, c.perm, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.pitch, c.add, run,
-                              c.clock, meet_from);
+    return cudaLaunchKernelEx(&cfg, sddmm_gather_kernel<S, MODE>, c.rows, c.cols, c.perm, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.pitch, c.add,
+                              c.finish, run, c.clock, meet_from);
 }
 
 template <class S>
@@ -400,6 +411,7 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
             c.pass = passes.n > 1;
             c.pitch = (unsigned)K * 4u;
             c.add = pass > 0;
+            c.finish = pass == passes.n - 1;
             c.sm_count = sm_count;
             c.clock = clock;
             c.beside = beside && j0 == 0;
@@ -446,7 +458,7 @@ cudaError_t launch_gather_bf16(const int32_t *rows, const int32_t *cols, const i
     for (int pass = 0; pass < p.n; ++pass) {
         GatherCall c = {rows, cols, perm, pass < p.n - 1 ? nullptr : sval, static_cast<const char *>(W) + 2 * pass * p.floats,
                         static_cast<const char *>(H) + 2 * pass * p.floats, P, (unsigned)nnz, p.floats / 8, p.n > 1, (unsigned)K * 2u, pass > 0,
-                        sm_count, clock, false, stream};
+                        pass == p.n - 1, sm_count, clock, false, stream};
         cudaError_t e = cudaErrorInvalidValue;
         if (p.floats == 256) e = launch_shape<GatherShape<16, 2, 2, 8, true, false, 5, true>>(c);
         else if (p.floats == 512) e = launch_shape<GatherShape<16, 4, 1, 8, true, true, 4, true>>(c);

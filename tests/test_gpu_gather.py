@@ -275,3 +275,29 @@ def test_tiled_order_of_a_large_H(engine):
     for a in range(0, nnz, 6_300_000):
         i = order[a:a + 6_300_000:63]
         assert torch.equal(P[a:a + 6_300_000:63], (W[rows[i].long()] * H[cols[i].long()]).sum(1)), a
+
+
+@pytest.mark.parametrize("K,N,width,bf16", [(768, 131_000, 192, False), (1024, 930_000, 256, True)])
+def test_parts_of_all_sizes_in_passes(engine, K, N, width, bf16):
+    # the parts that the passes add: zero, subnormal, either side of the line between the two ways of adding, and ordinary, in every order.  Each part is exact, so the
+    # sum is off by three roundings; where all parts are subnormal by none at all (the bound is below the smallest number then)
+    M, nnz, blocks = 20_011, 1_000_003, K // width
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H = (torch.randint(-2, 3, (n, K), generator=g, device="cuda").float() for n in (M, N))
+    size = torch.tensor([0.0, 2.0 ** -70, 2.0 ** -50, 2.0 ** -40, 2.0 ** -38, 2.0 ** -30, 1.0], device="cuda")
+    W = (W.view(M, blocks, width) * size[torch.randint(0, 7, (M, blocks, 1), generator=g, device="cuda")]).view(M, K)
+    H *= 2.0 ** -70
+    flag = 0
+    if bf16:
+        W, H, flag = W.bfloat16(), H.bfloat16(), api.FLAG_OPERANDS_BF16
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    P, n0 = torch.full((nnz,), float("nan"), device="cuda"), engine.kernel_launches()
+    plan.execute(W, H, P, None, flag)
+    assert engine.kernel_launches() - n0 == blocks
+    plan.close()
+    for a in range(0, nnz, 200_000):
+        i = slice(a, a + 200_000)
+        parts = (W[rows[i].long()].double() * H[cols[i].long()].double()).view(-1, blocks, width).sum(2)
+        assert bool(((P[i].double() - parts.sum(1)).abs() <= 4 * 2.0 ** -24 * parts.abs().sum(1)).all()), a
