@@ -817,17 +817,17 @@ __global__ void fill_dense_kernel(const Key *__restrict__ keys_s, const int32_t 
     }
 }
 // Row masks and run positions of every dense cell (one CTA per cell, grid-stride), and whether the cell qualifies for
-// the row-mask form: inside every row the list entries (input order) have ascending columns and their input indices are
-// consecutive but for one gap at most.  row_mask arrives zeroed.
+// the row-mask form: inside every row the list entries (input order) have ascending columns, and either their input indices are
+// consecutive but for one gap at most or index and column go up together (any number of columns may be in other cells then).  row_mask arrives zeroed.
 __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const int32_t *__restrict__ idx,
                                       const uint16_t *__restrict__ rc, unsigned long long *row_mask, int2 *row_base,
                                       uint32_t *row_span, unsigned long long *n_mask_cells)
 {
-    __shared__ int bad, forms;
+    __shared__ int unordered, gapped, forms;
     __shared__ int gaps[DENSE_CELL_ROWS], first[DENSE_CELL_ROWS], split[DENSE_CELL_ROWS], second[DENSE_CELL_ROWS];
     for (int64_t cell = blockIdx.x; cell < n_cells; cell += gridDim.x) {
         if (threadIdx.x == 0) {
-            bad = 0;
+            unordered = gapped = 0;
             forms = CELL_RUNS;
         }
         for (int r = threadIdx.x; r < DENSE_CELL_ROWS; r += blockDim.x) {
@@ -847,10 +847,10 @@ __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const i
             if (t == 0 || (prev >> 8) != (unsigned)r) {
                 first[r] = ci[t];
             } else {
-                if ((int)(prev & 255u) >= c) bad = 1;
+                if ((int)(prev & 255u) >= c) unordered = 1;
                 if (ci[t] - ci[t - 1] != c - (int)(prev & 255u)) forms = 0;
                 if (ci[t] != ci[t - 1] + 1) {
-                    if (atomicAdd(&gaps[r], 1) > 0) bad = 1;
+                    if (atomicAdd(&gaps[r], 1) > 0) gapped = 1;
                     split[r] = c;
                     second[r] = ci[t];
                 }
@@ -867,7 +867,7 @@ __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const i
             row_span[cell * DENSE_CELL_ROWS + r] = (uint32_t)c0 | (uint32_t)n << 8 | (uint32_t)s << 16;
         }
         __syncthreads();
-        if (threadIdx.x == 0 && !bad) {
+        if (threadIdx.x == 0 && !unordered && (forms || !gapped)) {
             cells[cell].cls = dc.cls | CELL_MASKED | forms;
             atomicAdd(n_mask_cells, 1ull);
         }

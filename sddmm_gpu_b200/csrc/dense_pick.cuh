@@ -10,7 +10,7 @@
 namespace sddmm {
 
 template <int NT = 256>  // divides a quarter of the cell's entries
-__device__ __forceinline__ void pick_block(const float *Ct, int stride, const DenseCell &dc, bool masked, int64_t cell,
+__device__ __forceinline__ void pick_block(const float *Ct, int stride, const DenseCell &dc, bool masked, bool runs, int64_t cell,
                                            int tid, const int32_t *__restrict__ table,
                                            const unsigned long long *__restrict__ row_mask,
                                            const int2 *__restrict__ row_base, const uint32_t *__restrict__ row_span, const float *__restrict__ sval,
@@ -19,7 +19,7 @@ __device__ __forceinline__ void pick_block(const float *Ct, int stride, const De
     if (masked) {
         // Row r of the cell holds the columns of mask[r]; in column order its nonzeros are one or two runs of
         // consecutive input positions: the one in column c sits at popc(mask[r] below bit c) past base[r].x, or past
-        // base[r].y from column span[r] >> 16 on.  A warp takes four rows at a time, lane l the columns l and l + 32: the S
+        // base[r].y from column span[r] >> 16 on; or (runs) as far past base[r].x as it is past the row's first column, span[r] & 255.  A warp takes four rows at a time, lane l the columns l and l + 32: the S
         // loads and the P stores of a row are a few contiguous runs.
         const unsigned long long *cm = row_mask + cell * DENSE_CELL_ROWS;
         const int2 *cb = row_base + cell * DENSE_CELL_ROWS;
@@ -29,14 +29,16 @@ __device__ __forceinline__ void pick_block(const float *Ct, int stride, const De
         for (int r0 = warp * 4; r0 < DENSE_CELL_ROWS; r0 += NT / 8) {
             unsigned lo[4], hi[4];
             int2 base[4];
-            int split[4];
+            int split[4], c0[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const unsigned long long m = __ldg(cm + r0 + u);
                 lo[u] = (unsigned)m;
                 hi[u] = (unsigned)(m >> 32);
                 base[u] = __ldg(cb + r0 + u);
-                split[u] = (int)(__ldg(cs + r0 + u) >> 16);
+                const uint32_t span = __ldg(cs + r0 + u);
+                split[u] = (int)(span >> 16);
+                c0[u] = (int)(span & 255u);
             }
             float s_lo[4], s_hi[4];
             int32_t p_lo[4], p_hi[4];
@@ -44,6 +46,10 @@ __device__ __forceinline__ void pick_block(const float *Ct, int stride, const De
             for (int u = 0; u < 4; ++u) {
                 p_lo[u] = (lane < split[u] ? base[u].x : base[u].y) + __popc(lo[u] & below);
                 p_hi[u] = (lane + 32 < split[u] ? base[u].x : base[u].y) + __popc(lo[u]) + __popc(hi[u] & below);
+                if (runs) {
+                    p_lo[u] = base[u].x + lane - c0[u];
+                    p_hi[u] = p_lo[u] + 32;
+                }
                 s_lo[u] = s_hi[u] = 1.f;
                 if (sval) {
                     if ((lo[u] >> lane) & 1u) s_lo[u] = __ldcs(sval + p_lo[u]);

@@ -103,7 +103,7 @@ sddmm_dense_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, const i
 
     for (int64_t cell = blockIdx.x; cell < n_cells; cell += gridDim.x) {
         DenseCell dc = cells[cell];
-        const bool masked = (dc.cls & CELL_MASKED) != 0;  // row-mask form, else table form
+        const bool masked = (dc.cls & CELL_MASKED) != 0, runs = (dc.cls & CELL_RUNS) != 0;  // row-mask form, else table form
         dc.cls &= 0xff;
         float acc[8][4];  // FMA path: [row i][col j]; tensor path: [m-tile*4 + n-tile][fragment register]
 #pragma unroll
@@ -208,7 +208,7 @@ sddmm_dense_kernel(const DenseCell *__restrict__ cells, int64_t n_cells, const i
                 for (int j = 0; j < 4; ++j) Ct[(ty + 16 * i) * CT_STRIDE + tx + 16 * j] = acc[i][j];
         }
         __syncthreads();
-        pick_block(Ct, CT_STRIDE, dc, masked, cell, tid, table, row_mask, row_base, row_span, sval, P);
+        pick_block(Ct, CT_STRIDE, dc, masked, runs, cell, tid, table, row_mask, row_base, row_span, sval, P);
         __syncthreads();  // the block is overwritten by the next cell's staging
     }
 }

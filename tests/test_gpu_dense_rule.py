@@ -79,6 +79,36 @@ def test_cells_with_several_nonzeros_in_one_place(monkeypatch, mode, M, N, fill)
     h.close()
 
 
+@pytest.mark.parametrize("mode", ["2", "1", "0"])
+@pytest.mark.parametrize("M,half_width,full", [(1300, 128, (300, 310)), (700, 64, (0, 5, 9, 130, 135, 140, 699)), (600, 96, (100, 101, 120, 121, 122, 180))])
+def test_cells_with_columns_in_other_cells(monkeypatch, mode, M, half_width, full):
+    # a band and a few full columns: the full ones are taken out of the band's cells, whose rows then have several gaps in their input positions.  Position and column
+    # go up together all the same, so none of them needs a table (32 KB); the full columns, fewer than a quarter of a cell, are in the remainder
+    import torch
+    monkeypatch.setenv("SDDMM_DENSE_CELLS", "1")
+    monkeypatch.setenv("SDDMM_DENSE_TENSOR", mode)
+    h = api.Handle(0)
+    K = 40
+    at = torch.arange(M, device="cuda")
+    cells = (at[:, None] - at).abs() <= half_width
+    cells[:, list(full)] = True
+    rows, cols = (a.to(torch.int32).contiguous() for a in cells.nonzero().T)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    W, H = (torch.randint(-2, 3, (M, K), generator=g, device="cuda").float() for _ in range(2))   # every product and sum exact
+    S = torch.randint(-3, 4, rows.shape, generator=g, device="cuda").float()
+    plan = h.plan_coo(M, M, rows, cols, K)
+    info = plan.info()
+    assert info.n_dense_cells > 0 and info.nnz - info.n_dense_nnz >= len(full) * M // 2
+    assert info.device_bytes < (24 + 2560 + 32) * info.n_dense_cells + 12 * (info.nnz - info.n_dense_nnz) + 8 * (M + 1) + 32768
+    ref = (W @ H.T)[rows.long(), cols.long()]
+    for v in (S, None):
+        P = torch.full(rows.shape, float("nan"), device="cuda")
+        plan.execute(W, H, P, v)
+        assert plan.last_kernel_name().startswith("dense") and torch.equal(P, ref if v is None else ref * v)
+    plan.close()
+    h.close()
+
+
 @pytest.mark.parametrize("K,half_width,n_global", [(64, 96, 6), (100, 40, 60), (512, 70, 3)])
 def test_remainder_beside_the_cells(engine, K, half_width, n_global):
     # the remainder runs beside the dense cells: what follows on the stream sees all of P, and the next call overwrites it
