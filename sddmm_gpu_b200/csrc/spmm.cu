@@ -437,9 +437,9 @@ unsigned run_length(int64_t nnz, int sm_count)
     const int64_t wave = (int64_t)sm_count * S::CTAS * (SP_TPB / 32) * S::G, s = nnz / wave + 1;
     int64_t waves;
     if (S::B == 1) {
-        // One nonzero at a time: a row that fills a run has as many roundings one after the other as the run is long.  24 nonzeros and up to a
+        // One nonzero at a time: a row that fills a run has as many roundings one after the other as the run is long.  32 nonzeros and up to a
         // third of a set's share, 80 and up to a sixth, 160 and up to a twelfth.
-        waves = s <= 240 ? std::min<int64_t>(3, (s + 23) / 24) : s <= 480 ? (s + 79) / 80 : std::min<int64_t>(12, std::max<int64_t>(6, (s + 159) / 160));
+        waves = s <= 32 ? 1 : s <= 64 ? 2 : s <= 240 ? 3 : s <= 480 ? (s + 79) / 80 : std::min<int64_t>(12, std::max<int64_t>(6, (s + 159) / 160));
     } else {
         // B at a time (add_block): a B-th of the roundings.  At most as many as where one at a time is added, and 80 up to 1,920 nonzeros.
         // (Error over the sum of magnitudes, rms of all entries; one at a time / the waves of the table alone / with this limit.
@@ -449,7 +449,13 @@ unsigned run_length(int64_t nnz, int sm_count)
                          : s <= 340 ? 1 : std::max<int64_t>(2, (s + 759) / 760);
         waves = std::max(waves, (s + S::B * chain - 1) / (S::B * chain));
     }
-    const int64_t run = (nnz / (waves * wave) + S::NB) / S::NB * S::NB;  // rounded up: one run less than a wave, not one more
+    int64_t run = (nnz / (waves * wave) + S::NB) / S::NB * S::NB;  // rounded up: one run less than a wave, not one more
+    // Fewer, longer runs where they would be very short (us at runs of 8 / 16 / 24, SpMM: s = 3, K = 128 10.5 / 11.0 / 11.9, K = 512 12.0 / 10.3 / 12.0;  s = 6, K = 192 14.8 / 14.3 / 15.3,
+    // K = 512 15.8 / 14.3 / 12.3;  s = 8, K = 128 13.8 / 12.3 / 14.3, K = 192 16.0 / 14.4 / 16.4;  s = 10, K = 256 15.5 / 12.5 / 12.3, K = 512 18.4 / 15.0 / 16.4;  s = 14, K = 64 20.6 / 16.4 / 16.5,
+    // K = 300 19.0 / 16.8 / 15.1, K = 512 22.5 / 19.0 / 16.4;  fused: s = 6, K = 64 14.2 / 14.7 / 16.4, K = 256 12.4 / 13.6 / 16.4, K = 512 20.5 / 19.5 / 22.3;  s = 14, K = 64 22.6 / 18.4 / 20.5,
+    // K = 512 31.0 / 24.5 / 25.9).
+    if (!S::FUSED && s > 4) run = std::max<int64_t>(run, (s > 12 ? 3 : 2) * S::NB);
+    if (S::FUSED && S::F >= 4 && s > 5) run = std::max<int64_t>(run, 2 * S::NB);
     return (unsigned)std::min<int64_t>(run, SP_MAX_RUN);
 }
 
