@@ -863,8 +863,8 @@ __global__ void cell_row_masks_kernel(DenseCell *cells, int64_t n_cells, const i
             const int s = split[r];
             const int before = s < DENSE_CELL_COLS ? __popcll(m & ((1ull << s) - 1ull)) : 0;
             row_base[cell * DENSE_CELL_ROWS + r] = make_int2(first[r], second[r] - before);
-            const int c0 = m ? __ffsll(m) - 1 : 0, n = __popcll(m);
-            row_span[cell * DENSE_CELL_ROWS + r] = (uint32_t)c0 | (uint32_t)n << 8 | (uint32_t)s << 16;
+            const int c0 = m ? __ffsll(m) - 1 : 0;
+            row_span[cell * DENSE_CELL_ROWS + r] = (uint32_t)c0 | (uint32_t)s << 16;
         }
         __syncthreads();
         if (threadIdx.x == 0 && !unordered && (forms || !gapped)) {
