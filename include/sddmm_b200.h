@@ -287,7 +287,7 @@ typedef struct {
     int32_t reserved0;
     int64_t n_dense_cells;  /* 128 x 64 cells handed to the dense-cell kernel (none below nnz * K = 2^26) */
     int64_t n_dense_nnz;    /* nonzeros inside them                            */
-    int64_t n_hub_cols;     /* columns marked for L2 residency: 0 unless the plan is column-tiled with a large H or a call has forced the ring kernel */
+    int64_t n_hub_cols;     /* columns marked for L2 residency: 0 unless the plan is column-tiled with a large H, a call has forced the ring kernel, or bfloat16 rows of K = 2048 ran on it */
 } sddmm_plan_info;
 SDDMM_API int sddmm_plan_get_info(sddmm_plan_t p, sddmm_plan_info *info);
 

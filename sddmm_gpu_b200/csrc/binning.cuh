@@ -94,7 +94,8 @@ cudaError_t build_hub_column_hints(const int32_t *d_cols_p, int64_t nnz, int64_t
 struct DensePlan {
     DenseCell *cells = nullptr;   // one descriptor per dense cell
     int64_t n_cells = 0;
-    // Cells of the same rows in twos (consecutive ones, from the first cell of those rows on; the last one may be alone).
+    // Cells of the same rows in twos (consecutive ones, from the first cell of those rows on; the last one may be alone).  Also where each could
+    // have an SM to itself (masks of K = 128, 77 to 145 cells, in twos / one by one, us: 1,211 tokens 16.3 / 16.3, 2,000 18.4 / 22.1, 3,000 15.3 / 17.5).
     DenseUnit *units = nullptr;
     int64_t n_units = 0;
     // Row-mask form of a cell (DenseCell::cls bit 8 set): per cell row a 64-bit column mask and the input positions of

@@ -14,8 +14,8 @@
 // 0.59 ms at 24 warps with two, 0.64 ms at 16 warps with four).  No shared memory: all of it is L1, which serves the
 // hub columns of a power-law matrix, and nothing is issued beyond the load, the packed FMAs (two per instruction) and
 // 1/8 of a butterfly -- 9 warp instructions per nonzero at K = 128 where the shared-memory ring needed 34.  Grids are
-// not persistent: a warp's share is 16 or 32 nonzeros per set, the hardware's block scheduler evens out the rest, and
-// there is no work counter to clear before the launch.
+// not persistent: a warp's share is 8, 16 or 32 nonzeros per set (4 where sets of four lanes are many), the hardware's block scheduler
+// evens out the rest, and there is no work counter to clear before the launch.
 //
 // Measured against the shared-memory ring and panel kernels (R-MAT, 16.1 M nonzeros, 1 M x 1 M, and 4.1 M nonzeros,
 // 300 K x 250 K; us before -> after):  K = 32: 250 -> 185, K = 64: 480 -> 296, K = 128: 832 -> 540, K = 256: 1250 ->

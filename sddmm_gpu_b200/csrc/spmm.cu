@@ -424,7 +424,8 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 // long as a full one (SpMM, K = 64, 6.0 M nonzeros, us: 2.0 waves 117, 2.5 waves 127, 2.8 waves 121, 4.0 waves 124).  How many: each
 // run pays for its two ends (partial rows, the dependent loads it starts with), so few; but rows of a power-law matrix make some
 // runs slower than others, the fused form more than SpMM, and long runs spread a wave over more rows of H than L2 holds.  Sustained us at
-// 1 / 2 / 3 / 4 / 5 / 8 waves (s: nonzeros for a resident set; in brackets: runs of 80 to 160 nonzeros, whatever the waves):
+// 1 / 2 / 3 / 4 / 5 / 8 waves (s: nonzeros for a resident set; in brackets: runs of 80 to 160 nonzeros, whatever the waves, one added at a time;
+// K = 200 and 300: two at a time):
 //   SpMM: s = 37, K = 64 24 / 29 / 33 / 33 / 45 / 45 (29);  40, documents x words 23 / 29 / 33 / 33 / 44 / 43 (29);  118, K = 256 52 / 56 / 62 / 64 / 69 / 80 (64);
 //     253, uniform, K = 256 133 / 139 / 146 / 153 / 161 / 176 (160);  317, K = 64 114 / 117 / 121 / 124 / 127 / 141 (124);  577, K = 100 143 / 142 / 143 / 147 / 151 / 169 (180);
 //     849, K = 64 330 / 320 / 320 / 335 / 329 / 345 (354);  1351, K = 200 674 / 550 / 579 / 569 / 556 / 576 (594);  2252, K = 300 - / - / 863 / 877 / 887 / 894 (929)
@@ -442,8 +443,9 @@ unsigned run_length(int64_t nnz, int sm_count)
         waves = s <= 32 ? 1 : s <= 64 ? 2 : s <= 240 ? 3 : s <= 480 ? (s + 79) / 80 : std::min<int64_t>(12, std::max<int64_t>(6, (s + 159) / 160));
     } else {
         // B at a time (add_block): a B-th of the roundings.  At most as many as where one at a time is added, and 80 up to 1,920 nonzeros.
-        // (Error over the sum of magnitudes, rms of all entries; one at a time / the waves of the table alone / with this limit.
-        // K = 200, 8 M nonzeros, rows of 700: 9.9e-8 / 2.8e-7 / 9.0e-8;  K = 64, 28 M: 9.9e-8 / 2.0e-7 / 9.3e-8.)
+        // (Relative error of sums of positive terms, rms of all entries, one at a time / the waves of the table alone / with this limit: 8 M nonzeros, rows of
+        // 700, K = 192 8.4e-8 / 1.4e-7 / 7.1e-8, K = 200 9.7e-8 / 2.0e-7 / 9.1e-8;  28 M, K = 64 9.8e-8 / 1.5e-7 / 8.6e-8;  and of one at a time, 0.28 M, rows of 80,
+        // K = 576 5.5e-8 / 1.4e-7 / 6.2e-8.  It costs up to 5 % of the time: K = 192, 4 M 216 -> 220 us, K = 384 446 -> 460, K = 512, 3 M 439 -> 460; K = 40 79 -> 88.)
         const int64_t chain = s < 240 ? std::max<int64_t>(24, s / 3) : std::max<int64_t>(80, s / 24);
         waves = S::FUSED ? (s <= 120 ? 1 : s <= 330 ? 2 : s > 1500 ? (s + 299) / 300 : (s + 169) / 170)
                          : s <= 340 ? 1 : std::max<int64_t>(2, (s + 759) / 760);
