@@ -15,20 +15,21 @@
 // at a time, lane l holding the 16-byte pieces l, l + L, ... of the H row, of the Y row being summed and (fused) of the
 // W row; B nonzeros of H are in flight per set.  When the row of S changes the set stores the finished row of Y and
 // starts the next one.  Runs are equal shares of the nonzeros whatever the rows look like, so a power-law matrix
-// loads every warp alike, and nothing is built per plan.  A row that crosses a run boundary leaves partial rows in
-// scratch -- tail[q]: run q's part of the row that goes on in run q + 1, head[q]: run q's part of a row that
-// began before it and ends in it.  The run that arrives last at a row (a counter per row) adds the parts in run order:
-// no atomics on Y, the result does not depend on scheduling, and there is no second launch (a fix-up kernel took a third
-// of a call with ten thousand nonzeros).  Parts are added in groups of 16 runs, each by its last run, and the groups by the
-// last of those, so that a row of hundreds of runs does not end in one long chain.  Rows of S without nonzeros are
-// zeroed by blocks of their own at the end of the grid.
+// loads every warp alike, and nothing is built per plan.
 //
-// What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero through L2; used twice in the fused form), hidden
-// by resident warps.  The fused form at K = 256 reaches neither bound (16.1 M nonzeros: 7.1 GB through DRAM at 4.5 TB/s, 13.4 TB/s read at
-// the L2 slices): between two blocks of B rows a set reduces, broadcasts and adds with nothing in flight.  Measured on R-MAT matrices against the row-task and shared-memory-ring kernels this replaces
-// (us): SpMM, 6.0 M nonzeros, 250 K x 250 K: K = 64 755 -> 125;  0.67 M nonzeros: K = 64 379 -> 29;  fused, 16.1 M
-// nonzeros, 1 M x 1 M: K = 256 2970 -> 1720 to 1785;  3.8 M nonzeros: K = 64 1205 -> 139;  30.8 M nonzeros: K = 512 8110 -> 7010.  With runs that fill whole waves
-// since then: SpMM, 6.0 M, K = 64 128 -> 117;  16.1 M, K = 256 1346 -> 1270;  0.75 M documents x words, K = 256 58 -> 43.
+// A row that crosses a run boundary is in parts: what the run in which it ends has of it (its head) and what the runs before that one have (their tails).  The runs of a
+// block follow one another, so a block adds up its own parts: tails go to shared memory, heads to Y for the time being, and behind a barrier the run in which a row ends
+// adds the tails before it, in order.  Only the row that a block begins with and the one that goes on behind it concern other blocks.  Their parts
+// go to scratch -- 2 b: block b's part of a row that ends in it, 2 b + 1: of one that goes on -- and the block that arrives last at a row (a counter per row) adds them
+// up in order: no atomics on Y, the result does not depend on scheduling, and there is no second launch (a fix-up kernel took a third of a call with ten thousand
+// nonzeros).  Parts are added in groups of 16 blocks, each by its last block, and the groups by the last of those, so that a row of hundreds of blocks does not end in one long
+// chain.  With a fence, a counter and two reads of the row pointer at both ends of every run, a run's ends took some 8 us, what 40 nonzeros at K = 64 take (us, then / now:
+// SpMM, 0.2 M nonzeros, K = 64, 128 14.4 / 12.3, 17.0 / 14.4;  1.2 M, K = 64, 128 31.0 / 26.6, 47 / 41;  6.0 M, K = 64 114 / 100;  fused, 30 K nonzeros, K = 64 12.2 / 9.2;
+// 0.2 M, K = 128 24.5 / 20.5;  1.2 M, K = 128 75 / 62;  1.5 M, columns alike, K = 32 39 / 29).  Rows of S without nonzeros are zeroed by blocks of their own at the end of the grid.
+//
+// What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero from L2, some 65 bytes a clock and SM at most; used twice in the fused form), hidden
+// by resident warps: SpMM takes 46 bytes a clock at K = 64, 67 at K = 256.  The fused form at K = 256 reaches neither bound:
+// between two blocks of B rows a set reduces, broadcasts and adds with nothing in flight.
 // At K = 64 the gather kernel alone runs at 14.2 TB/s of gathered bytes.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -47,26 +48,35 @@ namespace {
 
 constexpr int SP_TPB = 256;
 constexpr int SP_NB = 8;         // nonzeros of a set per index step (4 when a set is 4 lanes)
-constexpr int SP_MAX_RUN = 1024;  // bounds the scratch of partial rows
+constexpr int SP_MAX_RUN = 1024;
 
-constexpr unsigned SP_GROUP = 16;  // partial rows that one run adds
+constexpr unsigned SP_GROUP = 16;  // parts that one block adds
 
 // L lanes per nonzero, F pieces per lane, B nonzeros of a set in flight, CTAS resident blocks asked of the compiler.  PF: the
 // W rows of the next step are prefetched into L1.  JOINT: the B dot products are reduced together and a block of B that opens
-// no row is summed without the tests for it.  Taken where a nonzero has a whole warp: 3.75 shuffles for each instead of 7 (B =
-// 4; fused, K = 256: 16.1 M nonzeros 1735 -> 1660 us, 6.0 M 567 -> 540; K = 200 583 -> 557), while with several sets in a warp
-// most blocks open a row in one of them (K = 128 871 -> 965).
-template <int L_, int F_, int B_, bool EXACT_, int CTAS_, bool FUSED_ = false, bool PF_ = false, bool JOINT_ = true>
+// no row is summed without the tests for it.  Taken where a nonzero has a whole warp or a set few pieces, while with several sets in a warp
+// most blocks open a row in one of them (K = 128 871 -> 965).  FAR: tails in scratch instead of shared memory, which is L1 that four blocks of SpMM with a warp for a nonzero miss (6.0 M nonzeros, K = 256: 348 / 330 us, 338
+// with no shared memory and the run ends of before; K = 512 722 / 726).
+template <int L_, int F_, int B_, bool EXACT_, int CTAS_, bool FUSED_ = false, bool PF_ = false, bool JOINT_ = true, bool FAR_ = false>
 struct SpmmShape {
     static constexpr int L = L_, F = F_, B = B_, CTAS = CTAS_;
-    static constexpr bool EXACT = EXACT_, FUSED = FUSED_, PF = PF_, JOINT = JOINT_;
+    static constexpr bool EXACT = EXACT_, FUSED = FUSED_, PF = PF_, JOINT = JOINT_, FAR = FAR_;
     static constexpr int NB = L < SP_NB ? L : SP_NB, G = 32 / L;
+    static constexpr int SETS = SP_TPB / 32 * G;         // of a block
+    static constexpr int TAIL_BYTES = FAR ? 0 : SP_TPB * F * 16;  // a row for each of them
     static_assert(NB % B == 0, "step geometry");
+    static_assert(!FAR || L == 32, "FAR_SETS");
 };
 
 __device__ __forceinline__ void stg_u64x2(char *p, u64x2 v)
 {
     asm volatile("st.global.cs.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v.a), "l"(v.b) : "memory");
+}
+__device__ __forceinline__ u64x2 lds_u64x2(uint32_t p)
+{
+    u64x2 r;
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(r.a), "=l"(r.b) : "r"(p) : "memory");
+    return r;
 }
 __device__ __forceinline__ u64x2 ldcg_u64x2(const char *p)  // from L2: written by another SM during this launch
 {
@@ -101,8 +111,11 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             char *scratch, unsigned *arrived, const int64_t *__restrict__ row_ptr, unsigned nnz, int64_t M, int pieces, unsigned pitch,
             unsigned run_len, unsigned gather_blocks, unsigned long long *clock, unsigned meet_from)
 {
-    constexpr int L = S::L, F = S::F, B = S::B, NB = S::NB, G = S::G;
+    constexpr int L = S::L, F = S::F, B = S::B, NB = S::NB, G = S::G, T = S::SETS;
     constexpr bool FUSED = S::FUSED;
+    extern __shared__ __align__(16) char tails[];  // what the sets have of rows that go on behind their runs, a piece for each lane
+    __shared__ int first_row[T];
+    __shared__ unsigned openers[2];  // the sets whose tail is the beginning of its row, a bit each
     // From one row to the next.  (The fused form multiplies whole rows and holds one value less: with a second one it spills, 1707 -> 1801 us
     // at K = 256, 16.1 M nonzeros.)
     const unsigned row_bytes = !FUSED ? pitch : (unsigned)pieces * 16u;
@@ -124,6 +137,8 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     const int lig = lane & (L - 1), set = lane / L;
     const unsigned warp = (blockIdx.x * SP_TPB + threadIdx.x) >> 5;
     const unsigned run = warp * G + set;
+    if (threadIdx.x < 2) openers[threadIdx.x] = 0;
+    __syncthreads();
     if (warp * G * run_len >= nnz) return;
     const unsigned j0 = run * run_len;
     const char *H_lane = H + lig * 16, *W_lane = W + lig * 16;
@@ -149,8 +164,6 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             y[f] = u64x2{0, 0};
         }
     };
-    const int il = lig & (NB - 1);
-    unsigned j = j0 + il;
     auto at = [&](unsigned x) { return x < nnz ? x : nnz - 1; };
     // Past the end of the matrix a run sees the last nonzero again and again.  Its H row is replaced by zeros there, but a weight
     // that is not finite would make NaN of them.  So the weight is zero as well; or, where several weights are reduced together
@@ -161,7 +174,51 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     int cur = __ldg(rows + at(j0));                                // row being summed: that of the nonzero before this step
     auto began_before = [&](int row) { return j0 > 0 && __ldg(rows + at(j0 - 1)) == row; };  // it began in an earlier run
     bool head = began_before(cur);                                 // and nothing of it has been stored yet
+    const bool enters = head;
+    const int my_set = (threadIdx.x >> 5) * G + set;
+    if (lig == 0) first_row[my_set] = cur;
     if (FUSED) load_w((unsigned)cur);
+    auto next_row = [&](int to) {  // the finished row is stored (one that began before this run for now: see below)
+        flush(Y + (size_t)(unsigned)cur * row_bytes);
+        head = false;
+        cur = to;
+    };
+    auto add = [&](float weight, const u64x2 (&h)[F]) {
+        const unsigned long long pp = pair_of(weight);
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            y[f].a = ffma2(pp, h[f].a, y[f].a);
+            y[f].b = ffma2(pp, h[f].b, y[f].b);
+        }
+    };
+    // B nonzeros of one row are summed before they are added to it: a long row's chain of roundings is a B-th as long, which is what
+    // lets runs be as long as they are (SpMM, 6.0 M nonzeros, K = 64, against 64 bits: runs of 80 one by one 1.4e-7 to 1.6e-7, runs of 320
+    // 2.6e-7, in blocks of four 1.4e-7).
+    auto add_block = [&](const float (&p)[B], const u64x2 (&h)[B][F]) {
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            unsigned long long pp = pair_of(p[0]), ta = mul2(pp, h[0][f].a), tb = mul2(pp, h[0][f].b);
+#pragma unroll
+            for (int i = 1; i < B; ++i) {
+                pp = pair_of(p[i]);
+                ta = ffma2(pp, h[i][f].a, ta);
+                tb = ffma2(pp, h[i][f].b, tb);
+            }
+            y[f].a = add2(y[f].a, ta);
+            y[f].b = add2(y[f].b, tb);
+        }
+    };
+    auto dot = [&](const u64x2 (&h)[F]) {
+        unsigned long long a = 0;
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            a = ffma2(w[f].a, h[f].a, a);
+            a = ffma2(w[f].b, h[f].b, a);
+        }
+        return fold2(a);
+    };
+    const int il = lig & (NB - 1);
+    unsigned j = j0 + il;
     int r, c;
     float s = 1.f;
     {
@@ -219,54 +276,15 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             const unsigned here = changed >> b;
             auto opens = [&](int i) { return (here & (setmask << i)) != 0; };  // uniform over the warp: some set goes on to another row
             auto mine = [&](int i) { return ((here >> (set * L + i)) & 1u) != 0; };
-            auto next_row = [&](int to) {  // the finished row is stored
-                flush(head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
-                head = false;
-                cur = to;
-            };
-            auto add = [&](int i, float weight) {
-                const unsigned long long pp = pair_of(weight);
-#pragma unroll
-                for (int f = 0; f < F; ++f) {
-                    y[f].a = ffma2(pp, h[i][f].a, y[f].a);
-                    y[f].b = ffma2(pp, h[i][f].b, y[f].b);
-                }
-            };
-            // B nonzeros of one row are summed before they are added to it: a long row's chain of roundings is a B-th as long, which is what
-            // lets runs be as long as they are (SpMM, 6.0 M nonzeros, K = 64, against 64 bits: runs of 80 one by one 1.4e-7 to 1.6e-7, runs of 320
-            // 2.6e-7, in blocks of four 1.4e-7).
-            auto add_block = [&]() {
-#pragma unroll
-                for (int f = 0; f < F; ++f) {
-                    unsigned long long pp = pair_of(p[0]), ta = mul2(pp, h[0][f].a), tb = mul2(pp, h[0][f].b);
-#pragma unroll
-                    for (int i = 1; i < B; ++i) {
-                        pp = pair_of(p[i]);
-                        ta = ffma2(pp, h[i][f].a, ta);
-                        tb = ffma2(pp, h[i][f].b, tb);
-                    }
-                    y[f].a = add2(y[f].a, ta);
-                    y[f].b = add2(y[f].b, tb);
-                }
-            };
             // most blocks of B stay within their rows: one test for the block instead of two for each nonzero
             const bool stays = (here & (setmask * ((1u << B) - 1u))) == 0;
             if (FUSED && S::JOINT) {
-                auto dot = [&](int i) {
-                    unsigned long long a = 0;
-#pragma unroll
-                    for (int f = 0; f < F; ++f) {
-                        a = ffma2(w[f].a, h[i][f].a, a);
-                        a = ffma2(w[f].b, h[i][f].b, a);
-                    }
-                    return fold2(a);
-                };
                 // all B products first, so that their reductions overlap: one transposed butterfly leaves product i with the
                 // i-th B-th of the set's lanes, where it is scaled; then B broadcasts
                 float acc[B];
                 if (stays) {
 #pragma unroll
-                    for (int i = 0; i < B; ++i) acc[i] = dot(i);
+                    for (int i = 0; i < B; ++i) acc[i] = dot(h[i]);
                 } else {
 #pragma unroll
                     for (int i = 0; i < B; ++i) {
@@ -274,7 +292,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                             const int rj = __shfl_sync(FULL, r, b + i, L);
                             if (mine(i)) load_w((unsigned)rj);
                         }
-                        acc[i] = dot(i);
+                        acc[i] = dot(h[i]);
                     }
                 }
                 reduce_transposed<L, B>(acc, lig);
@@ -282,7 +300,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 #pragma unroll
                 for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, scaled, i * (L / B), L);
                 if (stays) {
-                    add_block();
+                    add_block(p, h);
                 } else {
 #pragma unroll
                     for (int i = 0; i < B; ++i) {
@@ -290,7 +308,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                             const int rj = __shfl_sync(FULL, r, b + i, L);
                             if (mine(i)) next_row(rj);
                         }
-                        add(i, p[i]);
+                        add(p[i], h[i]);
                     }
                 }
                 if (P_out) {
@@ -303,7 +321,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 #pragma unroll
                     for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, s, b + i, L);
                     if (B > 1 && stays) {
-                        add_block();
+                        add_block(p, h);
                         continue;
                     }
                 }
@@ -325,7 +343,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                 if (FUSED && B > 1 && stays) {
 #pragma unroll
                     for (int i = 0; i < B; ++i) weight(i);
-                    add_block();
+                    add_block(p, h);
                     continue;
                 }
 #pragma unroll
@@ -339,7 +357,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                         }
                     }
                     if (FUSED) weight(i);
-                    add(i, p[i]);
+                    add(p[i], h[i]);
                 }
             }
         }
@@ -349,89 +367,151 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         c = cn;
         s = sn;
     }
+    auto far_tail_of = [&](int q) { return scratch + (size_t)(2 * gather_blocks + blockIdx.x * T + q) * row_bytes + lig * 16; };
+    auto tail_of = [&](int q) { return smem_u32(tails) + q / G * (F * 512) + (q % G * L + lig) * 16; };
+    bool goes_on = false;
     if (G == 1 || j0 < nnz) {
         const unsigned end = j0 + run_len;
-        const bool goes_on = end < nnz && __ldg(rows + end) == cur;
-        if (!PAD || end <= nnz)  // (else it was stored when the padding opened)
-            flush(goes_on ? scratch + (size_t)(2 * run + 1) * row_bytes
-                          : head ? scratch + (size_t)(2 * run) * row_bytes : Y + (size_t)(unsigned)cur * row_bytes);
-        // the rows that this run left a part of: the one it began with, the one it ends with
-        const int row0 = __ldg(rows + j0);  // (read again: kept from the start it is a register more in the loop, where the shapes spill)
-        const int part_row[2] = {!head && began_before(row0) ? row0 : -1, goes_on || head ? cur : -1};
-        if (part_row[0] >= 0 || part_row[1] >= 0) {
-            const unsigned lanes = L == 32 ? FULL : ((1u << (L & 31)) - 1u) << (set * L);
-            auto arrive = [&](unsigned *count) {  // how many came before; everything this set stored is visible first
-                __threadfence();
-                __syncwarp(lanes);
-                unsigned before = 0;
-                if (lig == 0) before = atomicAdd(count, 1u);
-                return __shfl_sync(lanes, before, set * L);
-            };
-#pragma unroll 1
-            for (int k = 0; k < 2; ++k) {
-                if (part_row[k] < 0) continue;
-                const size_t row = (size_t)part_row[k];
-                const unsigned first = (unsigned)row_ptr[row] / run_len, last = (unsigned)(row_ptr[row + 1] - 1) / run_len;
-                auto part = [&](unsigned q) { return scratch + (size_t)(2 * q + (q < last ? 1 : 0)) * row_bytes + lig * 16; };
-                auto add_up = [&](unsigned q0, unsigned q1, unsigned step) {  // y = parts q0, q0 + step, ... <= q1
-                    constexpr int U = F <= 2 ? 4 : F <= 4 ? 2 : 1;
-                    const unsigned long long one = pair_of(1.f);
+        goes_on = end < nnz && __ldg(rows + end) == cur;
+        if (goes_on) {
+            if constexpr (S::FAR) {
+                flush(far_tail_of(my_set) - lig * 16);
+            } else {
 #pragma unroll
-                    for (int f = 0; f < F; ++f) y[f] = u64x2{0, 0};
-#pragma unroll 1
-                    for (unsigned q = q0; q <= q1; q += U * step) {
-                        u64x2 v[U][F];
-#pragma unroll
-                        for (int u = 0; u < U; ++u)
-#pragma unroll
-                            for (int f = 0; f < F; ++f)
-                                v[u][f] = q + u * step <= q1 && (f < F - 1 || last_ok) ? ldcg_u64x2(part(q + u * step) + f * L * 16) : u64x2{0, 0};
-#pragma unroll
-                        for (int u = 0; u < U; ++u)
-#pragma unroll
-                            for (int f = 0; f < F; ++f) {
-                                y[f].a = ffma2(one, v[u][f].a, y[f].a);
-                                y[f].b = ffma2(one, v[u][f].b, y[f].b);
-                            }
-                    }
-                };
-                const unsigned g0 = first + (run - first) / SP_GROUP * SP_GROUP, g1 = min(g0 + SP_GROUP - 1, last);
-                // (a group that is the row's last run only needs no counter, and has none: the next row may begin in that run)
-                if (g1 > g0) {
-                    if (arrive(&arrived[2 * g0]) != g1 - g0) continue;
-                    if (lig == 0) arrived[2 * g0] = 0;  // for the next call
-                    __threadfence();
-                }
-                add_up(g0, g1, 1);
-                if (g0 != first || g1 != last) {
-                    flush(part(g0) - lig * 16);
-                    if (arrive(&arrived[2 * first + 1]) != (last - first) / SP_GROUP) continue;
-                    if (lig == 0) arrived[2 * first + 1] = 0;
-                    __threadfence();
-                    add_up(first, last, SP_GROUP);
-                    flush(Y + row * row_bytes);
-                    if (clock && lig == 0) clock_note(clock);  // (a row of many runs: this may outlast every block that starts later)
-                    continue;
-                }
-                flush(Y + row * row_bytes);
+                for (int f = 0; f < F; ++f)
+                    asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(tail_of(my_set) + f * 512), "l"(y[f].a), "l"(y[f].b) : "memory");
             }
+            if (!head && lig == 0) atomicOr(&openers[my_set / 32], 1u << (my_set & 31));
+        } else if (!PAD || end <= nnz) {  // (else it was stored when the padding opened)
+            flush(Y + (size_t)(unsigned)cur * row_bytes);
+            head = false;
         }
+    }
+    __syncthreads();
+    // y += the tails of the sets before set `to` that belong to the row at hand, in their order; whether the row began in this block
+    auto add_tails = [&](int to) {
+        unsigned long long before = openers[0];
+        if (T > 32) before |= (unsigned long long)openers[1] << 32;
+        if (to < 64) before &= (1ull << to) - 1;
+        const int from = before ? 63 - __clzll((long long)before) : 0;
+        constexpr int U = F <= 2 ? 4 : F <= 4 ? 2 : 1;  // sums side by side
+        u64x2 sum[U][F];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int f = 0; f < F; ++f) sum[u][f] = u64x2{0, 0};
+#pragma unroll 1
+        for (int q = from; q < to; q += U) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (q + u < to) {
+#pragma unroll
+                    for (int f = 0; f < F; ++f) {
+                        const u64x2 v = !S::FAR ? lds_u64x2(tail_of(q + u) + f * 512)
+                                                : f < F - 1 || last_ok ? ldcg_u64x2(far_tail_of(q + u) + f * L * 16) : u64x2{0, 0};
+                        sum[u][f].a = add2(sum[u][f].a, v.a);
+                        sum[u][f].b = add2(sum[u][f].b, v.b);
+                    }
+                }
+        }
+#pragma unroll
+        for (int u = U / 2; u >= 1; u /= 2)
+#pragma unroll
+            for (int v = 0; v < u; ++v)
+#pragma unroll
+                for (int f = 0; f < F; ++f) {
+                    sum[v][f].a = add2(sum[v][f].a, sum[v + u][f].a);
+                    sum[v][f].b = add2(sum[v][f].b, sum[v + u][f].b);
+                }
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            y[f].a = add2(y[f].a, sum[0][f].a);
+            y[f].b = add2(y[f].b, sum[0][f].b);
+        }
+        return before != 0;
+    };
+    // The row in y is one of several blocks': its part goes to scratch -- part 2 b of block b: the row ends there, 2 b + 1: it goes on -- and the block that
+    // arrives last adds the parts up.
+    const unsigned lanes = L == 32 ? FULL : ((1u << (L & 31)) - 1u) << (set * L);
+    auto hand_over = [&](size_t row) {
+        auto arrive = [&](unsigned *count) {  // how many came before; everything this set stored is visible first
+            __threadfence();
+            __syncwarp(lanes);
+            unsigned before = 0;
+            if (lig == 0) before = atomicAdd(count, 1u);
+            return __shfl_sync(lanes, before, set * L);
+        };
+        const unsigned per_block = T * run_len, me = blockIdx.x;
+        const unsigned first = (unsigned)row_ptr[row] / per_block, last = (unsigned)(row_ptr[row + 1] - 1) / per_block;
+        auto part = [&](unsigned q) { return scratch + (size_t)(2 * q + (q < last ? 1 : 0)) * row_bytes + lig * 16; };
+        auto add_up = [&](unsigned q0, unsigned q1, unsigned step) {  // y = parts q0, q0 + step, ... <= q1
+            constexpr int U = F <= 2 ? 4 : F <= 4 ? 2 : 1;
+#pragma unroll
+            for (int f = 0; f < F; ++f) y[f] = u64x2{0, 0};
+#pragma unroll 1
+            for (unsigned q = q0; q <= q1; q += U * step) {
+                u64x2 v[U][F];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int f = 0; f < F; ++f)
+                        v[u][f] = q + u * step <= q1 && (f < F - 1 || last_ok) ? ldcg_u64x2(part(q + u * step) + f * L * 16) : u64x2{0, 0};
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int f = 0; f < F; ++f) {
+                        y[f].a = add2(y[f].a, v[u][f].a);
+                        y[f].b = add2(y[f].b, v[u][f].b);
+                    }
+            }
+        };
+        flush(part(me) - lig * 16);
+        const unsigned g0 = first + (me - first) / SP_GROUP * SP_GROUP, g1 = min(g0 + SP_GROUP - 1, last);
+        // (a group that is the row's last block only needs no counter, and has none: the next row may begin in that block)
+        if (g1 > g0) {
+            if (arrive(&arrived[2 * g0]) != g1 - g0) return;
+            if (lig == 0) arrived[2 * g0] = 0;  // for the next call
+            __threadfence();
+        }
+        add_up(g0, g1, 1);
+        if (g0 != first || g1 != last) {
+            flush(part(g0) - lig * 16);
+            if (arrive(&arrived[2 * first + 1]) != (last - first) / SP_GROUP) return;
+            if (lig == 0) arrived[2 * first + 1] = 0;
+            __threadfence();
+            add_up(first, last, SP_GROUP);
+        }
+        flush(Y + row * row_bytes);
+        if (clock && lig == 0) clock_note(clock);  // (a row of many blocks: this may outlast every block that starts later)
+    };
+    if (enters && !head) {  // a row that began before this run has ended in it
+        const size_t row = (size_t)(unsigned)first_row[my_set];
+#pragma unroll
+        for (int f = 0; f < F; ++f)
+            y[f] = f < F - 1 || last_ok ? ldcg_u64x2(Y + row * row_bytes + (f * L + lig) * 16) : u64x2{0, 0};
+        if (add_tails(my_set)) flush(Y + row * row_bytes);
+        else hand_over(row);
+    }
+    if (goes_on && my_set == T - 1) {
+#pragma unroll
+        for (int f = 0; f < F; ++f) y[f] = u64x2{0, 0};
+        (void)add_tails(T);
+        hand_over((size_t)(unsigned)cur);
     }
     clock_end(clock, meet_from);
 }
 
 // Runs are cut so that they fill whole waves of resident sets: a wave lasts as long as its runs, and a last one that is nearly empty as
 // long as a full one (SpMM, K = 64, 6.0 M nonzeros, us: 2.0 waves 117, 2.5 waves 127, 2.8 waves 121, 4.0 waves 124).  How many: each
-// run pays for its two ends (partial rows, the dependent loads it starts with), so few; but rows of a power-law matrix make some
-// runs slower than others, the fused form more than SpMM, and long runs spread a wave over more rows of H than L2 holds.  Sustained us at
-// 1 / 2 / 3 / 4 / 5 / 8 waves (s: nonzeros for a resident set; in brackets: runs of 80 to 160 nonzeros, whatever the waves, one added at a time;
-// K = 200 and 300: two at a time):
-//   SpMM: s = 37, K = 64 24 / 29 / 33 / 33 / 45 / 45 (29);  40, documents x words 23 / 29 / 33 / 33 / 44 / 43 (29);  118, K = 256 52 / 56 / 62 / 64 / 69 / 80 (64);
-//     253, uniform, K = 256 133 / 139 / 146 / 153 / 161 / 176 (160);  317, K = 64 114 / 117 / 121 / 124 / 127 / 141 (124);  577, K = 100 143 / 142 / 143 / 147 / 151 / 169 (180);
-//     849, K = 64 330 / 320 / 320 / 335 / 329 / 345 (354);  1351, K = 200 674 / 550 / 579 / 569 / 556 / 576 (594);  2252, K = 300 - / - / 863 / 877 / 887 / 894 (929)
-//   fused: s = 53, uniform, K = 128 71 / 80 / 93 / 94 / 95 / 111 (92);  63, K = 128 72 / 77 / 83 / 91 / 91 / 123 (83);  148, K = 256 89 / 86 / 84 / 86 / 88 / 93 (87);
-//     211, K = 128 232 / 219 / 224 / 229 / 238 / 246 (235);  310, attention, K = 64 129 / 132 / 141 / 142 / 144 / 152 (142);  422, K = 64 280 / 260 / 252 / 254 / 259 / 267 (262);
-//     845, K = 512 857 / 798 / 808 / 790 / 780 / 792 (806);  1689, K = 200 925 / 852 / 826 / 818 / 806 / 795 (798);  3396, K = 256 at 5 / 8 / 12 waves 1727 / 1649 / 1652 (1656)
+// run pays for its two ends, so few; but rows of a power-law matrix make some
+// runs slower than others, the fused form more than SpMM, and long runs spread a wave over more rows of H than L2 holds.  us at
+// 1 / 2 / 3 / 4 / 6 / 8 waves (s: nonzeros for a resident set):
+//   SpMM, K = 64: s = 11 12.3 / 15.5 / 15.5 / 15.4 / 15.4 / 15.5;  62 28 / 31 / 32 / 35 / 35 / 45;  80, columns alike 31 / 35 / 39 / 39 / 42 / 43;  317 114 / 113 / 117 / 117 / 122 / 123
+//   (before blocks added up their own parts: 118, K = 256 52 / 56 / 62 / 64 / - / 80;  577, K = 100 143 / 142 / 143 / 147 / - / 169;  1351, K = 200 674 / 550 / 579 / 569 / - / 576)
+//   fused, sets of eight lanes: s = 11, K = 64 14.5 / 16.9 / 17.0 / 17.0;  62 41 / 40 / 41 / 43 / 43 / 55;  80, columns alike 45 / 47 / 51 / 53 / 56 / 56;  254, K = 32 - / 133 / 132 / 119 / 121 / -;
+//     317, K = 64 205 / 186 / 180 / 177 / 173 / 175;  317, K = 128 - / - / - / 268 / - / 266;  849, K = 128 at 4 / 6 / 8 786 / 761 / 776
+//   fused, a warp for a nonzero (before blocks added up their own parts): 148, K = 256 89 / 86 / 84 / 86 / - / 93;  845, K = 512 857 / 798 / 808 / 790 / - / 792;  1689, K = 200 925 / 852 / 826 / 818 / - / 795;
+//     3396, K = 256 at 5 / 8 / 12 waves 1727 / 1649 / 1652
 template <class S>
 unsigned run_length(int64_t nnz, int sm_count)
 {
@@ -447,7 +527,8 @@ unsigned run_length(int64_t nnz, int sm_count)
         // 700, K = 192 8.4e-8 / 1.4e-7 / 7.1e-8, K = 200 9.7e-8 / 2.0e-7 / 9.1e-8;  28 M, K = 64 9.8e-8 / 1.5e-7 / 8.6e-8;  and of one at a time, 0.28 M, rows of 80,
         // K = 576 5.5e-8 / 1.4e-7 / 6.2e-8.  It costs up to 5 % of the time: K = 192, 4 M 216 -> 220 us, K = 384 446 -> 460, K = 512, 3 M 439 -> 460; K = 40 79 -> 88.)
         const int64_t chain = s < 240 ? std::max<int64_t>(24, s / 3) : std::max<int64_t>(80, s / 24);
-        waves = S::FUSED ? (s <= 120 ? 1 : s <= 330 ? 2 : s > 1500 ? (s + 299) / 300 : (s + 169) / 170)
+        waves = S::FUSED && S::L == 32 ? (s <= 120 ? 1 : s <= 330 ? 2 : s > 1500 ? (s + 299) / 300 : (s + 169) / 170)
+              : S::FUSED ? (s <= 120 ? 1 : s <= 240 ? 2 : std::max<int64_t>(std::min<int64_t>(12, (s + 79) / 80), (s + 299) / 300))
                          : s <= 340 ? 1 : std::max<int64_t>(2, (s + 759) / 760);
         waves = std::max(waves, (s + S::B * chain - 1) / (S::B * chain));
     }
@@ -466,14 +547,19 @@ cudaError_t launch_shape(const SpmmCall &a, int k0, int width, int sm_count, int
 {
     const int pieces = width / 4;
     if (pieces > S::L * S::F || pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
-    const unsigned run = run_length<S>(a.nnz, sm_count), n_runs = (unsigned)((a.nnz + run - 1) / run);
-    const unsigned sets_per_block = SP_TPB / 32 * S::G;
-    const unsigned gather_blocks = (n_runs + sets_per_block - 1) / sets_per_block;
+    const unsigned run = run_length<S>(a.nnz, sm_count), per_block = S::SETS * run;
+    const unsigned gather_blocks = (unsigned)((a.nnz + per_block - 1) / per_block);
     const unsigned zero_blocks = (unsigned)((a.M + SP_TPB - 1) / SP_TPB);
     // scratch: two counters per run, zero between calls, then the parts
     unsigned *const arrived = reinterpret_cast<unsigned *>(a.scratch);
     char *const parts = reinterpret_cast<char *>(a.scratch + spmm_counter_floats(a.nnz, a.N, a.K, sm_count));
-    spmm_kernel<S><<<gather_blocks + zero_blocks, SP_TPB, 0, stream>>>(
+    constexpr int smem = S::TAIL_BYTES;
+    if (smem > 32 * 1024) {
+        static SmemOptinCache optin;  // per device
+        const cudaError_t e = optin_dynamic_smem(spmm_kernel<S>, smem, optin);
+        if (e != cudaSuccess) return e;
+    }
+    spmm_kernel<S><<<gather_blocks + zero_blocks, SP_TPB, smem, stream>>>(
         a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H + k0), a.P_out,
         reinterpret_cast<char *>(a.Y + k0), parts, arrived, a.row_ptr, (unsigned)a.nnz, a.M, pieces, (unsigned)a.K * 4u, run, gather_blocks, a.clock, last_wave(gather_blocks, (unsigned)sm_count * S::CTAS));
     ++*n_launches;
@@ -481,23 +567,28 @@ cudaError_t launch_shape(const SpmmCall &a, int k0, int width, int sm_count, int
 }
 
 // Calls f with the shape for K (L * (F - 1) < K / 4 <= L * F).  The fused form holds the W row as well and wants fewer
-// nonzeros in flight; every line is the best of a sweep over (L, B, prefetch, joint reduction, resident blocks).
+// nonzeros in flight; every line is the best of a sweep over (L, B, prefetch, joint reduction, resident blocks).  The fused ones against the lines before them, us,
+// 6.0 M / 1.2 M nonzeros: K = 32, sets of 8 x 1, two at a time 170 / 35, this 118 / 31;  K = 96, 8 x 3, two at a time 241 / 57, this 211 / 47;  K = 160, 16 x 3 391 / 92, this 334 / 79;
+// K = 320, a warp 696 / 151, this 637 / 133.  SpMM, K = 200, three blocks / this: 6.0 M 355 / 300, 1.5 M, columns alike 101 / 82.
 template <class Fn>
 auto with_shape(int K, bool fused, Fn f)
 {
     const int q = K / 4;
     if (fused) {
         if (q <= 4) return f(SpmmShape<4, 1, 2, false, 4, true, true, false>());
-        if (q <= 8) return f(SpmmShape<8, 1, 2, false, 4, true, true, false>());
+        if (q < 8) return f(SpmmShape<8, 1, 4, false, 5, true, true, true>());
+        if (q == 8) return f(SpmmShape<8, 1, 4, true, 5, true, true, true>());
         if (q <= 12) return f(SpmmShape<4, 3, 2, false, 4, true, true, false>());
         if (q < 16) return f(SpmmShape<8, 2, 2, false, 4, true, true, false>());
         if (q == 16) return f(SpmmShape<8, 2, 2, true, 4, true, true, false>());
-        if (q <= 24) return f(SpmmShape<8, 3, 2, false, 3, true, true, false>());
+        if (q <= 24) return f(SpmmShape<8, 3, 1, false, 4, true, true, false>());
         if (q < 32) return f(SpmmShape<8, 4, 1, false, 3, true, true, false>());
         if (q == 32) return f(SpmmShape<8, 4, 1, true, 4, true, false, false>());
+        if (q <= 40) return f(SpmmShape<8, 5, 1, false, 3, true, true, false>());
         if (q <= 48) return f(SpmmShape<16, 3, 1, false, 4, true, true, false>());
         if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, true, true, true>());
         if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, true, true, true>());
+        if (q <= 80) return f(SpmmShape<16, 5, 1, false, 3, true, true, false>());
         if (q <= 96) return f(SpmmShape<32, 3, 1, false, 4, true, false, false>());
         if (q <= 128) return f(SpmmShape<32, 4, 1, false, 4, true, false, false>());
         if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3, true, false, false>());
@@ -514,10 +605,8 @@ auto with_shape(int K, bool fused, Fn f)
     if (q < 32) return f(SpmmShape<16, 2, 4, false, 3>());
     if (q == 32) return f(SpmmShape<16, 2, 4, true, 4>());
     if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4>());
-    // (two at a time with five resident blocks spill; us, those one nonzero at a time / with block sums / this: 0.75 M nonzeros, K = 200 63 / 59 / 49; 4.0 M 270 / 289 / 253;
-    // 16 M 1146 / 1232 / 1133; all columns alike, 4.0 M 470 / 464 / 421;  K = 252, 4.0 M 320 / 338 / 293)
-    if (q < 64) return f(SpmmShape<32, 2, 4, false, 3>());
-    if (q == 64) return f(SpmmShape<32, 2, 4, true, 4>());
+    if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, false, false, true, true>());
+    if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, false, false, true, true>());
     if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3>());
     if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3>());
     if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3>());
@@ -551,19 +640,26 @@ int spmm_passes(int64_t nnz, int64_t N, int K)
 
 bool spmm_supports(int K) { return K > 0 && K % 4 == 0 && K <= 1024; }
 
-static size_t max_runs(int64_t nnz, int64_t N, int K, int sm_count)  // of either form and of every pass
+constexpr size_t FAR_SETS = SP_TPB / 32;  // whose tails a block may leave in scratch (FAR)
+// Blocks of runs, the most of either form and of every pass.
+static size_t max_blocks(int64_t nnz, int64_t N, int K, int sm_count)
 {
-    auto run_of = [&](int width, bool fused) { return with_shape(width, fused, [&](auto s) { return run_length<decltype(s)>(nnz, sm_count); }); };
-    unsigned run = std::min(run_of(K, false), run_of(K, true));
+    auto blocks = [&](int width, bool fused) {
+        return with_shape(width, fused, [&](auto s) {
+            const size_t per_block = (size_t)decltype(s)::SETS * run_length<decltype(s)>(nnz, sm_count);
+            return ((size_t)nnz + per_block - 1) / per_block;
+        });
+    };
+    size_t n = std::max(blocks(K, false), blocks(K, true));
     const int w = pass_floats(nnz, N, K);
-    if (w < K) run = std::min(run, run_of(w, false));
-    if (K % w) run = std::min(run, run_of(K % w, false));
-    return (size_t)((nnz + run - 1) / run);
+    if (w < K) n = std::max(n, blocks(w, false));
+    if (K % w) n = std::max(n, blocks(K % w, false));
+    return n;
 }
-size_t spmm_counter_floats(int64_t nnz, int64_t N, int K, int sm_count) { return (2 * max_runs(nnz, N, K, sm_count) + 31) / 32 * 32; }
+size_t spmm_counter_floats(int64_t nnz, int64_t N, int K, int sm_count) { return (2 * max_blocks(nnz, N, K, sm_count) + 31) / 32 * 32; }
 size_t spmm_scratch_floats(int64_t nnz, int64_t N, int K, int sm_count)
 {
-    return spmm_counter_floats(nnz, N, K, sm_count) + max_runs(nnz, N, K, sm_count) * 2 * (size_t)K;
+    return spmm_counter_floats(nnz, N, K, sm_count) + max_blocks(nnz, N, K, sm_count) * (2 + FAR_SETS) * (size_t)K;
 }
 
 cudaError_t launch_spmm(const SpmmCall &a, int sm_count, int64_t *n_launches, cudaStream_t stream)

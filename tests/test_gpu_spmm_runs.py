@@ -1,6 +1,6 @@
 """SpMM and the fused form at the run boundaries of csrc/spmm.cu: rows that end exactly where a run ends, that cross one
-boundary, that span a few runs, exactly sixteen and seventeen (one and two groups of parts) and hundreds, a row that begins in
-the run where a row of seventeen ends, stretches of empty rows, repeated calls (the counters are left at zero),
+boundary, that span a few runs, exactly sixteen and seventeen and hundreds, a row that begins in
+the run where a row of seventeen ends, the same with blocks of runs (one and two groups of parts), stretches of empty rows, repeated calls (the counters are left at zero),
 and every lane shape's first and last K.
 
 Tolerance: as tests/test_gpu_spmm.py (1e-4 of the sum of magnitudes per entry of Y, against float64)."""
@@ -52,6 +52,33 @@ def test_run_boundaries(engine, K):
         Y2.fill(np.nan)
         plan.fused(W, H, Y2, vals)
         assert np.array_equal(Y, Y2)
+    plan.close()
+
+
+@pytest.mark.parametrize("K", [16, 32, 64, 96, 160, 192, 200, 256, 320, 384, 512, 768, 1024])
+def test_block_boundaries(engine, K):
+    # A block holds 8 to 64 runs of 8, 16 or 24 nonzeros.  Rows that begin and end at multiples of 8 and 64 and one beside them, rows of a block and of
+    # 16 and 17 blocks, many short rows in a run, rows that a block has only the end of; small whole numbers, so that every sum is exact.
+    rng = np.random.default_rng(K)
+    N = 17 * 1536 + 9
+    lengths = [64, 64, 1, 63, 8, 56, 512, 7, 1, 504, 512 + 1, 511, 0, 1024, 8, 8, 48] + [1] * 32 + [2] * 16 + [16 * 64, 17 * 64, 16 * 192, 17 * 192, 16 * 512, 17 * 512 - 1, 1, 17 * 1536, 5, 3]
+    lengths += [int(n) for n in rng.choice([8, 16, 24, 64, 128, 192, 256, 384, 512, 768], 60)]
+    rows, cols = _rows_of_lengths(rng, lengths, N)
+    M = len(lengths)
+    vals = rng.integers(-1, 2, rows.shape[0]).astype(np.float32)
+    W, H = rng.integers(-1, 2, (M, K)).astype(np.float32), rng.integers(-1, 2, (N, K)).astype(np.float32)
+    P = np.einsum("ij,ij->i", W[rows], H[cols]) * vals   # at most K
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    for weights, call in ((vals, lambda Y, p: plan.spmm(H, Y, vals)), (P, lambda Y, p: plan.fused(W, H, Y, vals, p))):
+        ref, ends = np.zeros((M, K)), np.concatenate([[0], np.cumsum(lengths)])
+        for r in range(M):
+            ref[r] = weights[ends[r]:ends[r + 1]].astype(np.float64) @ H[cols[ends[r]:ends[r + 1]]]
+        assert np.abs(ref).max() < 2 ** 20   # (random signs: partial sums are far from 2^24)
+        for _ in range(2):   # (the counters are left at zero)
+            Y, p = np.full((M, K), np.nan, np.float32), np.full(rows.shape[0], np.nan, np.float32)
+            call(Y, p)
+            assert np.array_equal(Y, ref.astype(np.float32))
+            assert weights is vals or np.array_equal(p, P)
     plan.close()
 
 
