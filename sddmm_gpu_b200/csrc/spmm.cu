@@ -28,13 +28,16 @@
 // 0.2 M, K = 128 24.5 / 20.5;  1.2 M, K = 128 75 / 62;  1.5 M, columns alike, K = 32 39 / 29).  Rows of S without nonzeros are zeroed by blocks of their own at the end of the grid.
 //
 // What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero from L2, some 65 bytes a clock and SM at most; used twice in the fused form), hidden
-// by resident warps: SpMM takes 46 bytes a clock at K = 64, 67 at K = 256.  The fused form at K = 256 reaches neither bound:
-// between two blocks of B rows a set reduces, broadcasts and adds with nothing in flight.
+// by resident warps: SpMM takes 46 bytes a clock at K = 64, 67 at K = 256.  The fused form also computes: a block of B nonzeros is reduced, spread
+// and added with nothing of its warp in flight (6.0 M nonzeros, K = 256: 1,180 clocks of 2,220 wait for memory), and more warps or more rows in flight do not fit the
+// registers.  Measured and not kept: rows of H through a ring of shared memory by 16-byte or bulk copies (the ring takes what L1 gave: 16.1 M, K = 256, 1407 with a ring of 64 KB a block while L1 had 32 KB, 2180
+// with 9 KB; bulk copies 1617 - 2490), H rows of the next block in registers (two nonzeros a block, 1571).
 // At K = 64 the gather kernel alone runs at 14.2 TB/s of gathered bytes.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "device_utils.cuh"
@@ -55,18 +58,39 @@ constexpr unsigned SP_GROUP = 16;  // parts that one block adds
 // L lanes per nonzero, F pieces per lane, B nonzeros of a set in flight, CTAS resident blocks asked of the compiler.  PF: the
 // W rows of the next step are prefetched into L1.  JOINT: the B dot products are reduced together and a block of B that opens
 // no row is summed without the tests for it.  Taken where a nonzero has a whole warp or a set few pieces, while with several sets in a warp
-// most blocks open a row in one of them (K = 128 871 -> 965).  FAR: tails in scratch instead of shared memory, which is L1 that four blocks of SpMM with a warp for a nonzero miss (6.0 M nonzeros, K = 256: 348 / 330 us, 338
+// most blocks open a row in one of them (K = 128 871 -> 965).  STAGED (a warp for a nonzero): rows, columns and S values of 32 nonzeros in shared memory, see the
+// kernel.  FAR: tails in scratch instead of shared memory, which is L1 that four blocks of SpMM with a warp for a nonzero miss (6.0 M nonzeros, K = 256: 348 / 330 us, 338
 // with no shared memory and the run ends of before; K = 512 722 / 726).
-template <int L_, int F_, int B_, bool EXACT_, int CTAS_, bool FUSED_ = false, bool PF_ = false, bool JOINT_ = true, bool FAR_ = false>
+template <int L_, int F_, int B_, bool EXACT_, int CTAS_, bool FUSED_ = false, bool PF_ = false, bool JOINT_ = true, bool STAGED_ = false, bool FAR_ = false>
 struct SpmmShape {
     static constexpr int L = L_, F = F_, B = B_, CTAS = CTAS_;
-    static constexpr bool EXACT = EXACT_, FUSED = FUSED_, PF = PF_, JOINT = JOINT_, FAR = FAR_;
+    static constexpr bool EXACT = EXACT_, FUSED = FUSED_, PF = PF_, JOINT = JOINT_, STAGED = STAGED_, FAR = FAR_;
     static constexpr int NB = L < SP_NB ? L : SP_NB, G = 32 / L;
     static constexpr int SETS = SP_TPB / 32 * G;         // of a block
     static constexpr int TAIL_BYTES = FAR ? 0 : SP_TPB * F * 16;  // a row for each of them
     static_assert(NB % B == 0, "step geometry");
     static_assert(!FAR || L == 32, "FAR_SETS");
+    static_assert(!STAGED || (FUSED && JOINT && L == 32), "staged: a warp for a nonzero");
 };
+
+// STAGED: what a warp knows of the 32 nonzeros at hand.
+struct Staged {
+    int32_t row[32], col[32];
+    float val[32], p[32];  // p: the weights
+};
+template <int B> struct Vec;
+template <> struct Vec<1> { using I = int; using V = float; };
+template <> struct Vec<2> { using I = int2; using V = float2; };
+template <> struct Vec<4> { using I = int4; using V = float4; };
+template <int B, class T>
+__device__ __forceinline__ void lds_vec(T (&out)[B], const T *p)
+{
+    using X = typename std::conditional<std::is_same<T, float>::value, typename Vec<B>::V, typename Vec<B>::I>::type;
+    const X v = *reinterpret_cast<const X *>(p);
+    if constexpr (B == 1) out[0] = v;
+    if constexpr (B >= 2) out[0] = v.x, out[1] = v.y;
+    if constexpr (B == 4) out[2] = v.z, out[3] = v.w;
+}
 
 __device__ __forceinline__ void stg_u64x2(char *p, u64x2 v)
 {
@@ -116,6 +140,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     extern __shared__ __align__(16) char tails[];  // what the sets have of rows that go on behind their runs, a piece for each lane
     __shared__ int first_row[T];
     __shared__ unsigned openers[2];  // the sets whose tail is the beginning of its row, a bit each
+    __shared__ __align__(16) Staged staged[S::STAGED ? SP_TPB / 32 : 1];
     // From one row to the next.  (The fused form multiplies whole rows and holds one value less: with a second one it spills, 1707 -> 1801 us
     // at K = 256, 16.1 M nonzeros.)
     const unsigned row_bytes = !FUSED ? pitch : (unsigned)pieces * 16u;
@@ -217,155 +242,233 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         }
         return fold2(a);
     };
-    const int il = lig & (NB - 1);
-    unsigned j = j0 + il;
-    int r, c;
-    float s = 1.f;
-    {
-        const unsigned a = at(j);
-        r = __ldg(rows + a);
-        c = __ldg(cols + a);
-        if (val) s = __ldg(val + a);
-    }
-#pragma unroll 1
-    for (unsigned step = run_len / NB; step > 0; --step) {
-        int rn = 0, cn = 0;
+    if constexpr (S::STAGED) {
+        // Rows, columns and S values of 32 nonzeros lie in shared memory, from where a block of B takes its columns and its weights by one
+        // load each that all lanes share.  With a shuffle for each they take as much of the load/store pipe as half of the loads of H, and registers that make the loop
+        // spill.  us, so / this: 16.1 M nonzeros, K = 256 1598 / 1455 (sustained 1776 / 1571);  6.0 M, K = 200, 256, 384, 512 528 / 456, 528 / 475, 800 / 732, 990 / 915;
+        // 0.2 M, K = 256, 512 28.9 / 26.7, 48 / 45;  1.2 M, K = 768 344 / 297;  but K = 640, 1024 259 / 264, 395 / 404.
+        Staged &st = staged[threadIdx.x >> 5];
+        int rn, cn;
         float sn = 1.f;
-        if (step > 1) {
-            const unsigned a = at(j + NB);
+        auto fetch = [&](unsigned done) {  // the nonzeros from `done` of the run on
+            const unsigned a = at(j0 + done + lane);
             rn = __ldg(rows + a);
             cn = __ldg(cols + a);
             if (val) sn = __ldg(val + a);
-        }
-        int before = __shfl_up_sync(FULL, r, 1, L);
-        if (lig == 0) before = cur;
-        const unsigned changed = __ballot_sync(FULL, (r != before || (PAD && j == nnz && (G == 1 || j0 < nnz))) && lig < NB);
-        const bool full = __all_sync(FULL, j < nnz);
-        if (!FUSED && !full && j >= nnz) s = 0.f;
-        if (FUSED && S::PF && step > 1) {
-            // the W rows that the next step opens, into L1
-            int b2 = __shfl_up_sync(FULL, rn, 1, L);
-            const int last = __shfl_sync(FULL, r, NB - 1, L);
-            if (lig == 0) b2 = last;
-            if (rn != b2 && lig < NB) {
+        };
+        fetch(0);
+#pragma unroll 1
+        for (unsigned done = 0; done < run_len; done += 32) {
+            st.row[lane] = rn;
+            st.col[lane] = cn;
+            st.val[lane] = sn;
+            int before = __shfl_up_sync(FULL, rn, 1);
+            if (lane == 0) before = cur;
+            const unsigned changed = __ballot_sync(FULL, rn != before || j0 + done + lane == nnz);  // (the padding opens a row)
+            __syncwarp();
+            if (S::PF && lane >= B && (changed >> lane) & 1u) {
+                // the W rows that these nonzeros open, into L1
                 const char *wp = W + (size_t)(unsigned)rn * row_bytes;
                 for (unsigned o = 0; o < row_bytes; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(wp + o));
             }
-        }
-        float p_mine = 0.f;
-        auto load_h = [&](int b, u64x2 (&h)[B][F]) {
+            if (done + 32 < run_len) fetch(done + 32);
+            const int n = min(run_len - done, 32u);
+#pragma unroll 1
+            for (int b = 0; b < n; b += B) {
+                int c[B];
+                lds_vec<B>(c, &st.col[b]);
+                u64x2 h[B][F];
 #pragma unroll
-            for (int i = 0; i < B; ++i) {
-                const unsigned cj = (unsigned)__shfl_sync(FULL, c, b + i, L);
-                const char *hp = H_lane + (size_t)cj * row_bytes;
-                if (full) {
+                for (int i = 0; i < B; ++i) {
+                    const char *hp = H_lane + (size_t)(unsigned)c[i] * row_bytes;
 #pragma unroll
                     for (int f = 0; f < F; ++f) h[i][f] = f < F - 1 || last_ok ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
-                } else {  // the end of the matrix
-                    const bool ok = j - il + b + i < nnz;
-#pragma unroll
-                    for (int f = 0; f < F; ++f) h[i][f] = ok && (f < F - 1 || last_ok) ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
                 }
-            }
-        };
-#pragma unroll
-        for (int b = 0; b < NB; b += B) {
-            u64x2 h[B][F];
-            load_h(b, h);
-            float p[B];  // the nonzeros' weights, the same in all lanes of the set
-            const unsigned here = changed >> b;
-            auto opens = [&](int i) { return (here & (setmask << i)) != 0; };  // uniform over the warp: some set goes on to another row
-            auto mine = [&](int i) { return ((here >> (set * L + i)) & 1u) != 0; };
-            // most blocks of B stay within their rows: one test for the block instead of two for each nonzero
-            const bool stays = (here & (setmask * ((1u << B) - 1u))) == 0;
-            if (FUSED && S::JOINT) {
-                // all B products first, so that their reductions overlap: one transposed butterfly leaves product i with the
-                // i-th B-th of the set's lanes, where it is scaled; then B broadcasts
-                float acc[B];
-                if (stays) {
+                const unsigned here = (changed >> b) & ((1u << B) - 1u);
+                float acc[B], p[B];
+                if (here == 0) {
 #pragma unroll
                     for (int i = 0; i < B; ++i) acc[i] = dot(h[i]);
                 } else {
 #pragma unroll
                     for (int i = 0; i < B; ++i) {
-                        if (opens(i)) {
-                            const int rj = __shfl_sync(FULL, r, b + i, L);
-                            if (mine(i)) load_w((unsigned)rj);
-                        }
+                        if (here >> i & 1u) load_w((unsigned)st.row[b + i]);
                         acc[i] = dot(h[i]);
                     }
                 }
                 reduce_transposed<L, B>(acc, lig);
-                const float scaled = acc[0] * __shfl_sync(FULL, s, b + lig / (L / B), L);
-#pragma unroll
-                for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, scaled, i * (L / B), L);
-                if (stays) {
+                const int mine = b + lane / (L / B);
+                const float scaled = acc[0] * st.val[mine];
+                if (lane % (L / B) == 0) st.p[mine] = scaled;
+                __syncwarp();
+                lds_vec<B>(p, &st.p[b]);
+                if (here == 0) {
                     add_block(p, h);
                 } else {
 #pragma unroll
                     for (int i = 0; i < B; ++i) {
-                        if (opens(i)) {
-                            const int rj = __shfl_sync(FULL, r, b + i, L);
-                            if (mine(i)) next_row(rj);
-                        }
+                        if (here >> i & 1u) next_row(st.row[b + i]);
                         add(p[i], h[i]);
                     }
                 }
-                if (P_out) {
-#pragma unroll
-                    for (int i = 0; i < B; ++i)
-                        if (il == b + i) p_mine = p[i];
+            }
+            __syncwarp();
+            if (P_out) {
+                if (lane < n && j0 + done + lane < nnz) P_out[j0 + done + lane] = st.p[lane];
+                __syncwarp();
+            }
+        }
+    } else {
+        const int il = lig & (NB - 1);
+        unsigned j = j0 + il;
+        int r, c;
+        float s = 1.f;
+        {
+            const unsigned a = at(j);
+            r = __ldg(rows + a);
+            c = __ldg(cols + a);
+            if (val) s = __ldg(val + a);
+        }
+#pragma unroll 1
+        for (unsigned step = run_len / NB; step > 0; --step) {
+            int rn = 0, cn = 0;
+            float sn = 1.f;
+            if (step > 1) {
+                const unsigned a = at(j + NB);
+                rn = __ldg(rows + a);
+                cn = __ldg(cols + a);
+                if (val) sn = __ldg(val + a);
+            }
+            int before = __shfl_up_sync(FULL, r, 1, L);
+            if (lig == 0) before = cur;
+            const unsigned changed = __ballot_sync(FULL, (r != before || (PAD && j == nnz && (G == 1 || j0 < nnz))) && lig < NB);
+            const bool full = __all_sync(FULL, j < nnz);
+            if (!FUSED && !full && j >= nnz) s = 0.f;
+            if (FUSED && S::PF && step > 1) {
+                // the W rows that the next step opens, into L1
+                int b2 = __shfl_up_sync(FULL, rn, 1, L);
+                const int last = __shfl_sync(FULL, r, NB - 1, L);
+                if (lig == 0) b2 = last;
+                if (rn != b2 && lig < NB) {
+                    const char *wp = W + (size_t)(unsigned)rn * row_bytes;
+                    for (unsigned o = 0; o < row_bytes; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(wp + o));
                 }
-            } else {
-                if (!FUSED) {
+            }
+            float p_mine = 0.f;
+            auto load_h = [&](int b, u64x2 (&h)[B][F]) {
 #pragma unroll
-                    for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, s, b + i, L);
-                    if (B > 1 && stays) {
+                for (int i = 0; i < B; ++i) {
+                    const unsigned cj = (unsigned)__shfl_sync(FULL, c, b + i, L);
+                    const char *hp = H_lane + (size_t)cj * row_bytes;
+                    if (full) {
+#pragma unroll
+                        for (int f = 0; f < F; ++f) h[i][f] = f < F - 1 || last_ok ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
+                    } else {  // the end of the matrix
+                        const bool ok = j - il + b + i < nnz;
+#pragma unroll
+                        for (int f = 0; f < F; ++f) h[i][f] = ok && (f < F - 1 || last_ok) ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
+                    }
+                }
+            };
+#pragma unroll
+            for (int b = 0; b < NB; b += B) {
+                u64x2 h[B][F];
+                load_h(b, h);
+                float p[B];  // the nonzeros' weights, the same in all lanes of the set
+                const unsigned here = changed >> b;
+                auto opens = [&](int i) { return (here & (setmask << i)) != 0; };  // uniform over the warp: some set goes on to another row
+                auto mine = [&](int i) { return ((here >> (set * L + i)) & 1u) != 0; };
+                // most blocks of B stay within their rows: one test for the block instead of two for each nonzero
+                const bool stays = (here & (setmask * ((1u << B) - 1u))) == 0;
+                if (FUSED && S::JOINT) {
+                    // all B products first, so that their reductions overlap: one transposed butterfly leaves product i with the
+                    // i-th B-th of the set's lanes, where it is scaled; then B broadcasts
+                    float acc[B];
+                    if (stays) {
+#pragma unroll
+                        for (int i = 0; i < B; ++i) acc[i] = dot(h[i]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < B; ++i) {
+                            if (opens(i)) {
+                                const int rj = __shfl_sync(FULL, r, b + i, L);
+                                if (mine(i)) load_w((unsigned)rj);
+                            }
+                            acc[i] = dot(h[i]);
+                        }
+                    }
+                    reduce_transposed<L, B>(acc, lig);
+                    const float scaled = acc[0] * __shfl_sync(FULL, s, b + lig / (L / B), L);
+#pragma unroll
+                    for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, scaled, i * (L / B), L);
+                    if (stays) {
+                        add_block(p, h);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < B; ++i) {
+                            if (opens(i)) {
+                                const int rj = __shfl_sync(FULL, r, b + i, L);
+                                if (mine(i)) next_row(rj);
+                            }
+                            add(p[i], h[i]);
+                        }
+                    }
+                    if (P_out) {
+#pragma unroll
+                        for (int i = 0; i < B; ++i)
+                            if (il == b + i) p_mine = p[i];
+                    }
+                } else {
+                    if (!FUSED) {
+#pragma unroll
+                        for (int i = 0; i < B; ++i) p[i] = __shfl_sync(FULL, s, b + i, L);
+                        if (B > 1 && stays) {
+                            add_block(p, h);
+                            continue;
+                        }
+                    }
+                    auto weight = [&](int i) {  // fused: of nonzero i of the block
+                        const int x = b + i;
+                        unsigned long long a0 = 0, a1 = 0;
+#pragma unroll
+                        for (int f = 0; f < F; ++f) {
+                            a0 = ffma2(w[f].a, h[i][f].a, a0);
+                            a1 = ffma2(w[f].b, h[i][f].b, a1);
+                        }
+                        float a = fold2(a0) + fold2(a1);
+#pragma unroll
+                        for (int off = L / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
+                        p[i] = a * __shfl_sync(FULL, s, x, L);
+                        if (!full && j - il + x >= nnz) p[i] = 0.f;
+                        if (il == x) p_mine = p[i];
+                    };
+                    if (FUSED && B > 1 && stays) {
+#pragma unroll
+                        for (int i = 0; i < B; ++i) weight(i);
                         add_block(p, h);
                         continue;
                     }
-                }
-                auto weight = [&](int i) {  // fused: of nonzero i of the block
-                    const int x = b + i;
-                    unsigned long long a0 = 0, a1 = 0;
 #pragma unroll
-                    for (int f = 0; f < F; ++f) {
-                        a0 = ffma2(w[f].a, h[i][f].a, a0);
-                        a1 = ffma2(w[f].b, h[i][f].b, a1);
-                    }
-                    float a = fold2(a0) + fold2(a1);
-#pragma unroll
-                    for (int off = L / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(FULL, a, off);
-                    p[i] = a * __shfl_sync(FULL, s, x, L);
-                    if (!full && j - il + x >= nnz) p[i] = 0.f;
-                    if (il == x) p_mine = p[i];
-                };
-                if (FUSED && B > 1 && stays) {
-#pragma unroll
-                    for (int i = 0; i < B; ++i) weight(i);
-                    add_block(p, h);
-                    continue;
-                }
-#pragma unroll
-                for (int i = 0; i < B; ++i) {
-                    const int x = b + i;
-                    if (opens(i)) {
-                        const int rj = __shfl_sync(FULL, r, x, L);
-                        if (mine(i)) {
-                            next_row(rj);
-                            if (FUSED) load_w((unsigned)rj);
+                    for (int i = 0; i < B; ++i) {
+                        const int x = b + i;
+                        if (opens(i)) {
+                            const int rj = __shfl_sync(FULL, r, x, L);
+                            if (mine(i)) {
+                                next_row(rj);
+                                if (FUSED) load_w((unsigned)rj);
+                            }
                         }
+                        if (FUSED) weight(i);
+                        add(p[i], h[i]);
                     }
-                    if (FUSED) weight(i);
-                    add(p[i], h[i]);
                 }
             }
+            if (FUSED && P_out && lig < NB && j < nnz) P_out[j] = p_mine;
+            j += NB;
+            r = rn;
+            c = cn;
+            s = sn;
         }
-        if (FUSED && P_out && lig < NB && j < nnz) P_out[j] = p_mine;
-        j += NB;
-        r = rn;
-        c = cn;
-        s = sn;
     }
     auto far_tail_of = [&](int q) { return scratch + (size_t)(2 * gather_blocks + blockIdx.x * T + q) * row_bytes + lig * 16; };
     auto tail_of = [&](int q) { return smem_u32(tails) + q / G * (F * 512) + (q % G * L + lig) * 16; };
@@ -510,8 +613,8 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 //   (before blocks added up their own parts: 118, K = 256 52 / 56 / 62 / 64 / - / 80;  577, K = 100 143 / 142 / 143 / 147 / - / 169;  1351, K = 200 674 / 550 / 579 / 569 / - / 576)
 //   fused, sets of eight lanes: s = 11, K = 64 14.5 / 16.9 / 17.0 / 17.0;  62 41 / 40 / 41 / 43 / 43 / 55;  80, columns alike 45 / 47 / 51 / 53 / 56 / 56;  254, K = 32 - / 133 / 132 / 119 / 121 / -;
 //     317, K = 64 205 / 186 / 180 / 177 / 173 / 175;  317, K = 128 - / - / - / 268 / - / 266;  849, K = 128 at 4 / 6 / 8 786 / 761 / 776
-//   fused, a warp for a nonzero (before blocks added up their own parts): 148, K = 256 89 / 86 / 84 / 86 / - / 93;  845, K = 512 857 / 798 / 808 / 790 / - / 792;  1689, K = 200 925 / 852 / 826 / 818 / - / 795;
-//     3396, K = 256 at 5 / 8 / 12 waves 1727 / 1649 / 1652
+//   fused, a warp for a nonzero, K = 256: s = 58 27 / 27 / 29 / - / - / 41;  330 163 / 129 / 125 / - / - / 116;  422, columns alike - / 146 / 151 / - / 166 / -;  1689 at 5 / 6 / 8 / 12 / 20 533 / 500 / 499 /
+//     494 / 499;  4531 at 12 / 16 1492 / 1478
 template <class S>
 unsigned run_length(int64_t nnz, int sm_count)
 {
@@ -586,13 +689,12 @@ auto with_shape(int K, bool fused, Fn f)
         if (q == 32) return f(SpmmShape<8, 4, 1, true, 4, true, false, false>());
         if (q <= 40) return f(SpmmShape<8, 5, 1, false, 3, true, true, false>());
         if (q <= 48) return f(SpmmShape<16, 3, 1, false, 4, true, true, false>());
-        if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, true, true, true>());
-        if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, true, true, true>());
+        if (q <= 64) return f(SpmmShape<32, 2, 4, false, 3, true, true, true, true>());
         if (q <= 80) return f(SpmmShape<16, 5, 1, false, 3, true, true, false>());
-        if (q <= 96) return f(SpmmShape<32, 3, 1, false, 4, true, false, false>());
-        if (q <= 128) return f(SpmmShape<32, 4, 1, false, 4, true, false, false>());
+        if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3, true, true, true, true>());
+        if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3, true, false, true, true>());
         if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3, true, false, false>());
-        if (q <= 192) return f(SpmmShape<32, 6, 1, false, 2, true, false, false>());
+        if (q <= 192) return f(SpmmShape<32, 6, 2, false, 2, true, false, true, true>());
         if (q <= 224) return f(SpmmShape<32, 7, 1, false, 2, true, false, false>());
         return f(SpmmShape<32, 8, 1, false, 2, true, false, false>());
     }
@@ -605,8 +707,8 @@ auto with_shape(int K, bool fused, Fn f)
     if (q < 32) return f(SpmmShape<16, 2, 4, false, 3>());
     if (q == 32) return f(SpmmShape<16, 2, 4, true, 4>());
     if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4>());
-    if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, false, false, true, true>());
-    if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, false, false, true, true>());
+    if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, false, false, true, false, true>());
+    if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, false, false, true, false, true>());
     if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3>());
     if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3>());
     if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3>());
