@@ -97,7 +97,8 @@ PanelConfig choose_panel_config(int K, int panel_rows_hint, int sm_count, size_t
 // beside (with perm only): may run beside the kernel before it in the stream, once that has signalled it; it ends no earlier.
 // passes: the columns of W and H that a launch multiplies (without perm; with it there is one).  Every pass but the first adds to P.
 struct GatherPasses {
-    int n, floats;  // launches, columns of each (the last one may have fewer)
+    int n, floats;           // launches, columns of each (the last one may have fewer)
+    bool few_lanes = false;  // the shape with fewer lanes for a nonzero, where there are two
 };
 // What is best for an H of N rows; one pass where S values and P share memory.  tiled: the nonzeros are in the order of column tiles.
 GatherPasses gather_passes(int64_t nnz, int64_t N, int K, bool tiled, const float *sval, const float *P);

@@ -405,7 +405,8 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
     sddmm_handle_s *h = p->h;
     p->pending = true;  // (sddmm_execute clears it again when it waits)
     // the split of the whole matrix: a chunk of it is summed in the order that the whole would be
-    const GatherPasses passes = gather_passes(p->nnz, p->N, p->K, p->d_perm && !perm, sval, P);
+    const int64_t whole = rows == p->dense.rows_s ? p->dense.n_sparse : p->nnz;
+    const GatherPasses passes = gather_passes(whole, p->N, p->K, p->d_perm && !perm, sval, P);
     rows += first;
     if (perm) {
         perm += first;

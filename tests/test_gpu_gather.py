@@ -39,6 +39,34 @@ def test_gather_shapes(engine, K):
         assert_parity(P, rows, cols, W, H, vals)
 
 
+@pytest.mark.parametrize("K,N", [(100, 20_000), (124, 16_130), (124, 16_128), (64, 20_000), (60, 20_000)])
+def test_many_nonzeros_of_a_large_h(engine, K, N):
+    # from a million nonzeros and 8 MB of H on rows of 100 to 124 columns have a shape of their own (16,128 rows are below); the chunks of a call with host
+    # operands are summed as the whole.  Small whole numbers: every product and sum is exact.
+    M, nnz = 200_003, 1_000_003
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H, S = (torch.randint(-2, 3, n, generator=g, device="cuda").float() for n in ((M, K), (N, K), (nnz,)))
+    ref = torch.cat([torch.einsum("nk,nk->n", W[rows[i:i + 100_000].long()], H[cols[i:i + 100_000].long()]) for i in range(0, nnz, 100_000)])
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    tiled = engine.plan_coo(M, N, rows, cols, K, 0, N // 3)
+    for p, sv, flags in ((plan, S, 0), (plan, None, 0), (plan, S, api.FLAG_KERNEL_GATHER), (tiled, S, 0)):
+        P = torch.full((nnz,), float("nan"), device="cuda")
+        p.execute(W, H, P, sv, flags)
+        assert torch.equal(P, ref if sv is None else ref * sv)
+    P = torch.full((nnz,), float("nan"), device="cuda")
+    engine.sddmm_coo(M, N, rows, cols, W, H, K, P, S)
+    assert torch.equal(P, ref * S)
+    W, H = torch.randn((M, K), generator=g, device="cuda"), torch.randn((N, K), generator=g, device="cuda")
+    plan.execute(W, H, P, S)
+    on_host = [a.cpu().pin_memory() for a in (W, H, S, torch.zeros(nnz))]
+    plan.execute(on_host[0], on_host[1], on_host[3], on_host[2])
+    assert torch.equal(P.cpu(), on_host[3])
+    plan.close()
+    tiled.close()
+
+
 def test_kernel_time_of_small_calls(engine):
     # timed by the kernel's own clock; each plan keeps its own time, also when calls of other plans lie between, and an
     # asynchronous call has none
