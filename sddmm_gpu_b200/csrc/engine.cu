@@ -406,7 +406,8 @@ cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *col
     p->pending = true;  // (sddmm_execute clears it again when it waits)
     // the split of the whole matrix: a chunk of it is summed in the order that the whole would be
     const int64_t whole = rows == p->dense.rows_s ? p->dense.n_sparse : p->nnz;
-    const GatherPasses passes = gather_passes(whole, p->N, p->K, p->d_perm && !perm, sval, P);
+    GatherPasses passes = gather_passes(whole, p->N, p->K, p->d_perm && !perm, sval, P);
+    passes.awaited = clock != nullptr;
     rows += first;
     if (perm) {
         perm += first;
@@ -1348,8 +1349,10 @@ int sddmm_coo(sddmm_handle_t h, int64_t M, int64_t N, int64_t nnz, const int32_t
         CUDA_TRY(h, pool_alloc(&tmp.p[5], sizeof(float) * nnz));
         dp = (float *)tmp.p[5];
     }
+    GatherPasses passes = gather_passes(nnz, N, K, false, (const float *)ds, dp);
+    passes.awaited = true;
     CUDA_TRY(h, launch_gather((const int32_t *)dr, (const int32_t *)dc, nullptr, (const float *)ds, (const float *)dw,
-                              (const float *)dh, dp, nnz, K, gather_passes(nnz, N, K, false, (const float *)ds, dp), h->sm_count, nullptr, s));
+                              (const float *)dh, dp, nnz, K, passes, h->sm_count, nullptr, s));
     if (!p_dev) CUDA_TRY(h, cudaMemcpyAsync(P, dp, sizeof(float) * nnz, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(h, cudaStreamSynchronize(s));
     return SDDMM_OK;

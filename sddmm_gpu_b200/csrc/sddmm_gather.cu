@@ -38,6 +38,7 @@ constexpr int GA_TPB = GATHER_TPB;
 // kernel leaves an SM 7,900 registers, room for two warps of any shape here (32 to 128 threads measure alike).  65,536-token mask, 0.3 M of
 // 44 M nonzeros left over, K = 64: 180 us after the cells, 168 beside them; 12,777 tokens 37 -> 29.6.
 constexpr int GA_TPB_BESIDE = 64;
+constexpr int FEW_EACH = 2;  // nonzeros of a set (sddmm_gather_few_kernel)
 
 // L lanes per nonzero, F 16-byte pieces per lane, B nonzeros of a set in flight, RB nonzeros per reduction, CTAS
 // resident blocks per SM asked of the compiler.  EXACT: the L * F pieces are the row (no predicate on the last one).
@@ -211,6 +212,54 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
     clock_end(clock, meet_from);
 }
 
+// Few nonzeros, two for each set: every row of W and of H is asked for at once, where the kernel above waits for an H row after the other and for the W row of every row of S
+// that a step opens.  The sums are the same, bit for bit: the same pieces to the same lanes, reduced in the same order.  What bounds it: three latencies, indices, rows, the wait
+// for the call.  Synchronous calls, us, above / this: uniform, 16,777 nonzeros, K = 32 14.2 / 13.3, K = 64 14.5 / 13.6, K = 128 14.4 / 14.1;  4,000, K = 32, 128, 512 14.2 / 13.1, 14.0 /
+// 13.6, 14.3 / 14.1;  40,000, K = 64 14.5 / 14.0;  R-MAT, 70,000, K = 32 14.7 / 14.2.  One or four for each set: 13.3, 13.7 and 13.6, 14.1 in the first two.
+template <class S>
+__global__ void __launch_bounds__(GA_TPB)
+sddmm_gather_few_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const float *__restrict__ sval,
+                        const char *__restrict__ W, const char *__restrict__ H, float *__restrict__ P, unsigned nnz, int pieces,
+                        unsigned long long *clock, unsigned meet_from)
+{
+    clock_begin(clock);
+    constexpr int L = S::L, F = S::F, G = S::G, U = FEW_EACH;
+    const int lane = threadIdx.x & 31, lig = lane & (L - 1), set = lane / L;
+    const unsigned first = gather_warp(blockIdx.x, GA_TPB, threadIdx.x) * (G * U);  // nonzero u of a set: first + u G + set
+    if (first >= nnz) return;
+    const unsigned row_bytes = (unsigned)pieces * 16u;
+    const char *H_lane = H + lig * 16, *W_lane = W + lig * 16;
+    const bool last_ok = S::EXACT || lig + (F - 1) * L < pieces;
+    unsigned r[U], c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const unsigned j = first + u * G + set, a = j < nnz ? j : nnz - 1;
+        r[u] = (unsigned)__ldg(rows + a);
+        c[u] = (unsigned)__ldg(cols + a);
+    }
+    // what this lane stores, if anything
+    const unsigned mine = first + lig / (L / U) * G + set;
+    const bool stores = lig % (L / U) == 0 && mine < nnz;
+    float s = 1.f;
+    if (stores && sval) s = __ldg(sval + mine);
+    u64x2 h[U][F];
+    WShare<S> w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const char *hp = H_lane + (size_t)c[u] * row_bytes;
+#pragma unroll
+        for (int f = 0; f < F; ++f) h[u][f] = f < F - 1 || last_ok ? ldg_u64x2(hp + f * L * 16) : u64x2{0, 0};
+        w[u].clear();
+        w[u].load(W_lane + (size_t)r[u] * row_bytes, last_ok);
+    }
+    float acc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc[u] = w[u].dot(h[u]);
+    reduce_transposed<L, U>(acc, lig);
+    if (stores) P[mine] = acc[0] * s;
+    clock_end(clock, meet_from);
+}
+
 // Rows of more than 256 pieces (K > 1024): a warp per nonzero, both rows in passes of 32 pieces.  The W row is read again for
 // every nonzero, from L1: 9 TB/s of H rows on 1.9 M nonzeros of an R-MAT matrix, beside as much of W.
 // Against the row-panel kernel, which stages W in shared memory (us, panel / this): R-MAT, 0.23 M nonzeros, K = 1028 460 / 100,
@@ -271,14 +320,31 @@ struct GatherCall {
     unsigned long long *clock;
     bool beside;
     cudaStream_t stream;
-    bool few_lanes = false;
+    bool few_lanes = false, awaited = false;
 };
+
+template <class S>
+cudaError_t launch_few(const GatherCall &c)
+{
+    const unsigned per_block = GA_TPB / S::L * FEW_EACH, blocks = (c.nnz + per_block - 1) / per_block;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(GA_TPB);
+    cfg.stream = c.stream;
+    return cudaLaunchKernelEx(&cfg, sddmm_gather_few_kernel<S>, c.rows, c.cols, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.clock,
+                              last_wave(blocks, (unsigned)c.sm_count * 3));
+}
 
 template <class S, GatherMode MODE>
 cudaError_t launch_mode(const GatherCall &c)
 {
     // only the last piece of a lane is predicated: the ones before it have to lie inside the row
     if (c.pieces > S::L * S::F || c.pieces <= S::L * (S::F - 1)) return cudaErrorInvalidValue;
+    // Up to 10 MB of H rows a call is a few latencies long, which count where it is waited for.  (Above it W rows that are read again for every nonzero cost more: synchronous calls
+    // of 80,000 nonzeros, uniform, K = 64 15.3 / 15.0, K = 128 16.3 / 16.9;  40,000, K = 128 14.8 / 15.1, K = 256 16.0 / 16.7;  150,000, R-MAT, K = 32 15.2 / 15.3.  Asynchronous calls one
+    // after the other take what the host needs to launch them, and that is more with the shorter kernel: 16,777 nonzeros, K = 32, 64 5.0 / 5.5, of 2.9 / 1.7, 3.0 / 1.9 on the GPU.)
+    if constexpr (MODE == STORE && S::F <= 4)
+        if (c.awaited && (uint64_t)c.nnz * (unsigned)c.pieces * 16u <= 10000000) return launch_few<S>(c);
     // A set's run.  A long one spreads what a run costs at its ends and keeps the W row over more nonzeros; the last wave of blocks, which
     // may be nearly empty, lasts as long as a run.  So by the nonzeros that there are for a resident set (us at runs of 8 / 16 / 32):
     // below 40: K = 32, 1.0 M nonzeros 18.6 / 21.1 / 27.3;  K = 64, 0.4 M 12.4 / 14.4 / 14.4, 0.7 M 19.6 / 20.7 / 24.0;  K = 128, 0.24 M 12.4 / 14.4 /
@@ -426,6 +492,7 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
             c.beside = beside && j0 == 0;
             c.stream = stream;
             c.few_lanes = passes.few_lanes;
+            c.awaited = passes.awaited;
             cudaError_t e;
             if (c.pieces <= 256) {
                 e = launch_pieces(c);

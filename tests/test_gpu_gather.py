@@ -39,6 +39,35 @@ def test_gather_shapes(engine, K):
         assert_parity(P, rows, cols, W, H, vals)
 
 
+@pytest.mark.parametrize("K", [4, 16, 28, 32, 44, 48, 60, 64, 96, 100, 128, 160, 192, 200, 256, 300, 380, 384, 500, 512])
+def test_few_nonzeros_as_many(engine, K):
+    # calls of at most 10 MB of H rows that are waited for have a kernel of their own: the same bits as the same nonzeros at the front of a call that is larger
+    M, N = 900, 1100
+    most = 10_000_000 // (4 * K)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    nnz = most + 5000
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H, S = (torch.randn(n, generator=g, device="cuda") for n in ((M, K), (N, K), (nnz,)))
+    W[M // 2, 1], H[3, 0], S[1] = float("inf"), float("nan"), float("-inf")
+    many = {}
+    for sv in (S, None):
+        many[sv is None] = torch.full((nnz,), 7.0, device="cuda")
+        plan = engine.plan_coo(M, N, rows, cols, K)
+        plan.execute(W, H, many[sv is None], sv)
+        plan.close()
+    for n in (1, 2, 3, 9, 63, 65, 1000, most - 1, most, most + 1):
+        plan = engine.plan_coo(M, N, rows[:n], cols[:n], K)
+        for sv in (S, None):
+            P = torch.full((n + 1,), 7.0, device="cuda")
+            plan.execute(W, H, P[:n], None if sv is None else sv[:n])
+            assert torch.equal(P[:n].view(torch.int32), many[sv is None][:n].view(torch.int32)) and float(P[n]) == 7.0
+            assert plan.last_kernel_ms() > 0
+            engine.sddmm_coo(M, N, rows[:n], cols[:n], W, H, K, P[:n], None if sv is None else sv[:n])
+            assert torch.equal(P[:n].view(torch.int32), many[sv is None][:n].view(torch.int32)) and float(P[n]) == 7.0
+        plan.close()
+
+
 @pytest.mark.parametrize("K,N", [(100, 20_000), (124, 16_130), (124, 16_128), (64, 20_000), (60, 20_000)])
 def test_many_nonzeros_of_a_large_h(engine, K, N):
     # from a million nonzeros and 8 MB of H on rows of 100 to 124 columns have a shape of their own (16,128 rows are below); the chunks of a call with host
