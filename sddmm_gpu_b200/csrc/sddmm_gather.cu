@@ -391,6 +391,10 @@ cudaError_t launch_pieces(const GatherCall &c)
     if (q < 8) GA_GO(8, 1, 4, 8, false, false, 6);
     if (q == 8) GA_GO(8, 1, 4, 8, true, false, 6);
     if (q <= 12) GA_GO(4, 3, 2, 4, false, true, 4);
+    // Up to two waves of blocks a block's own time counts: four rows at a time (same bits; synchronous calls, us, two / four: K = 64 0.22 M nonzeros 18.9 / 18.1, 0.25 M 19.3 / 18.7,
+    // 0.3 M 19.9 / 19.3, 0.4 M 21.3 / 21.1, a row of W for each of 0.07 M 15.7 / 15.3;  but 0.15 M 15.9 / 16.1, 0.205 M 17.6 / 18.2, 0.6 M 25.0 / 25.0, asynchronous 14.9 / 15.6).
+    const unsigned share = c.nnz / ((unsigned)c.sm_count * 5 * (GA_TPB / 32) * 4);
+    if (q > 12 && q <= 16 && !c.pass && share < 20) GA_GO(8, 2, 4, 8, false, false, 4);
     if (q < 16) GA_GO(8, 2, 2, 8, false, true, 5);
     if (q == 16 && c.pass) return launch_mode<GatherShape<8, 2, 4, 4, true, true, 4>, PASS>(c);
     if (q == 16) return c.perm ? launch_mode<GatherShape<8, 2, 2, 8, true, false, 5>, PERM>(c) : launch_mode<GatherShape<8, 2, 2, 8, true, false, 5>, STORE>(c);

@@ -68,6 +68,23 @@ def test_few_nonzeros_as_many(engine, K):
         plan.close()
 
 
+@pytest.mark.parametrize("K", [52, 60, 64])
+def test_two_waves_as_many(engine, K):
+    # up to 473,600 nonzeros of 148 SMs take four rows at a time: the same bits as the front of a call that takes two
+    M, N, nnz = 9_001, 7_001, 600_000
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H, S = (torch.randn(n, generator=g, device="cuda") for n in ((M, K), (N, K), (nnz,)))
+    P = {}
+    for n in (nnz, 50_001, 213_119, 300_001, 473_599, 473_600):
+        plan = engine.plan_coo(M, N, rows[:n], cols[:n], K)
+        P[n] = torch.full((n + 1,), 7.0, device="cuda")
+        plan.execute(W, H, P[n][:n], S[:n])
+        plan.close()
+        assert torch.equal(P[n][:n], P[nnz][:n]) and float(P[n][n]) == 7.0
+
+
 @pytest.mark.parametrize("K,N", [(100, 20_000), (124, 16_130), (124, 16_128), (64, 20_000), (60, 20_000)])
 def test_many_nonzeros_of_a_large_h(engine, K, N):
     # from a million nonzeros and 8 MB of H on rows of 100 to 124 columns have a shape of their own (16,128 rows are below); the chunks of a call with host
