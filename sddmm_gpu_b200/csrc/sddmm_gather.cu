@@ -42,9 +42,13 @@ constexpr int FEW_EACH = 2;  // nonzeros of a set (sddmm_gather_few_kernel)
 
 // L lanes per nonzero, F 16-byte pieces per lane, B nonzeros of a set in flight, RB nonzeros per reduction, CTAS
 // resident blocks per SM asked of the compiler.  EXACT: the L * F pieces are the row (no predicate on the last one).
-// PF: the W rows of the next step are prefetched into L1.  BF16: W and H hold bfloat16 (a piece is 8 values).
-template <int L_, int F_, int B_, int RB_, bool EXACT_, bool PF_, int CTAS_, bool BF16_ = false>
+// PF: the W rows of the next step are prefetched into L1.  BF16: W and H hold bfloat16 (a piece is 8 values).  STAGED: the columns of a step come from shared memory, two
+// loads for 8, in place of a shuffle each: where a nonzero is six pieces of a lane or more (one in flight) that is faster, else slower (us, shuffles / this: K = 1024 0.75 M nonzeros,
+// documents x words 163 / 141, 0.2 M 59.6 / 53.2, 0.6 M 159 / 151;  K = 768 106 / 101, 46.3 / 44.3, 112 / 109;  K = 384 62.0 / 59.8, 1.6 M 148 / 146;  but K = 896, 1.6 M 320 / 344,
+// K = 256, 16.1 M 1080 / 1177, K = 128 520 / 642).
+template <int L_, int F_, int B_, int RB_, bool EXACT_, bool PF_, int CTAS_, bool BF16_ = false, bool STAGED_ = false>
 struct GatherShape {
+    static constexpr bool STAGED = STAGED_;
     static constexpr int L = L_, F = F_, B = B_, RB = RB_, CTAS = CTAS_;
     static constexpr bool EXACT = EXACT_, PF = PF_, BF16 = BF16_;
     static constexpr int NB = L < 8 ? L : 8;  // nonzeros of a set per step
@@ -118,6 +122,8 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
 #pragma unroll
     for (int g = 0; g < G; ++g) setmask |= 1u << (g * L);
 
+    __shared__ __align__(16) int step_cols[S::STAGED ? GA_TPB / 32 : 1][S::STAGED ? G * NB : 1];
+    int *const my_cols = step_cols[S::STAGED ? threadIdx.x >> 5 : 0] + (S::STAGED ? set * NB : 0);
     WShare<S> w;
     w.clear();
     const int il = lig & (NB - 1);  // lanes >= NB of a set mirror a nonzero
@@ -161,6 +167,21 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
         // (volatile: it is to be under way while the rows of H are, not waited for at the end of the step)
         if (MODE == PASS && add && finish && lig < NB) asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(sum) : "l"(P + at(j)));
         float res = 0.f;
+        int cs[NB];
+        if constexpr (S::STAGED) {
+            static_assert(NB == 8, "two loads of four");
+            __syncwarp();
+            if (lig < NB) my_cols[lig] = c;
+            __syncwarp();
+#pragma unroll
+            for (int x = 0; x < NB; x += 4) {
+                const int4 t = *reinterpret_cast<const int4 *>(my_cols + x);
+                cs[x] = t.x;
+                cs[x + 1] = t.y;
+                cs[x + 2] = t.z;
+                cs[x + 3] = t.w;
+            }
+        }
 #pragma unroll
         for (int h0 = 0; h0 < NB; h0 += RB) {
             float acc[RB];
@@ -169,7 +190,7 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
                 u64x2 h[B][F];
 #pragma unroll
                 for (int i = 0; i < B; ++i) {
-                    const unsigned cj = (unsigned)__shfl_sync(FULL, c, h0 + b + i, L);
+                    const unsigned cj = S::STAGED ? (unsigned)cs[h0 + b + i] : (unsigned)__shfl_sync(FULL, c, h0 + b + i, L);
                     const char *hp = H_lane + (size_t)cj * row_bytes;
 #pragma unroll
                     for (int f = 0; f < F; ++f)
@@ -353,7 +374,9 @@ cudaError_t launch_mode(const GatherCall &c)
     // K = 300, 1.0 M 79.9 / 76.0 / 84.9;  K = 256, 0.7 M 53.6 / 49.9 / 51.7, documents x words, 0.75 M 56.7 / 50.0 / 47.8;
     // two sets to a warp, from 256 on: K = 192, 2.5 M 122 / 109.5 / 108.6;  K = 300, 2.5 M 179 / 177 / 168;  K = 100, 4.1 M 149 / 130 / 125.
     const unsigned resident = (unsigned)c.sm_count * S::CTAS * (GA_TPB / 32) * S::G, share = c.nnz / resident;  // sets; nonzeros for each
-    unsigned run = share < 40 ? 8 : S::L == 32 || (S::L == 16 && share >= 256) ? 32 : 16;
+    // a nonzero to a warp, 40 to 95 nonzeros for each (runs of 16 / 32): K = 256, 0.4 M 24.5 / 25.4, K = 512, 0.2 M 26.8 / 29.9, 0.22 M 24.8 / 28.7;  from there on: K = 256, 0.75 M 39.2 / 38.0,
+    // K = 512, 0.6 M 74.0 / 72.2.
+    unsigned run = share < 40 ? 8 : (S::L == 32 && (S::F > 4 || share >= 96)) || (S::L == 16 && share >= 256) ? 32 : 16;
     if (share < 8) run = S::NB;
     const unsigned tpb = c.beside ? GA_TPB_BESIDE : GA_TPB, per_block = run * S::G * (tpb / 32);
     const unsigned blocks = (unsigned)(((uint64_t)c.nnz + per_block - 1) / per_block);
@@ -409,13 +432,17 @@ cudaError_t launch_pieces(const GatherCall &c)
     if (q < 64) GA_GO(16, 4, 1, 8, false, true, 4);
     if (q == 64) GA_GO(32, 2, 2, 8, true, false, 5);
     if (q <= 80) GA_GO(16, 5, 1, 8, false, true, 4);
-    if (q <= 96) GA_GO(16, 6, 1, 8, false, false, 4);
+#define GA_STAGED(L, F, B, RB, EXACT, PF, CTAS) return launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS, false, true>>(c)
+    if (q <= 96) GA_STAGED(16, 6, 1, 8, false, false, 4);
     if (q < 128) GA_GO(32, 4, 2, 8, false, true, 3);
-    if (q == 128) GA_GO(32, 4, 2, 8, true, true, 3);
+    // (two at a time on three blocks / this, us: 0.75 M nonzeros, documents x words 69.9 / 65.8, 0.6 M 75.6 / 72.2, 1.6 M 182.4 / 179.9, 0.2 M 27.0 / 26.8)
+    if (q == 128) GA_GO(32, 4, 1, 8, true, false, 4);
     if (q <= 160) GA_GO(32, 5, 1, 8, false, false, 4);
-    if (q <= 192) GA_GO(32, 6, 1, 8, false, false, 4);
+    if (q == 192) GA_STAGED(32, 6, 1, 8, true, false, 4);  // (0.75 M nonzeros 104.6 / 100.9)
+    if (q <= 192) GA_STAGED(32, 6, 1, 8, false, false, 4);
     if (q <= 224) GA_GO(32, 7, 1, 8, false, false, 3);
-    if (q <= 256) GA_GO(32, 8, 1, 8, false, false, 3);
+    if (q <= 256) GA_STAGED(32, 8, 1, 8, false, false, 3);
+#undef GA_STAGED
 #undef GA_GO
     return cudaErrorInvalidValue;
 }
