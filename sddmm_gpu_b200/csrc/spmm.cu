@@ -674,7 +674,7 @@ cudaError_t launch_shape(const SpmmCall &a, int k0, int width, int sm_count, int
 // 6.0 M / 1.2 M nonzeros: K = 32, sets of 8 x 1, two at a time 170 / 35, this 118 / 31;  K = 96, 8 x 3, two at a time 241 / 57, this 211 / 47;  K = 160, 16 x 3 391 / 92, this 334 / 79;
 // K = 320, a warp 696 / 151, this 637 / 133.  SpMM, K = 200, three blocks / this: 6.0 M 355 / 300, 1.5 M, columns alike 101 / 82.
 template <class Fn>
-auto with_shape(int K, bool fused, Fn f)
+auto with_shape(int K, bool fused, int64_t nnz, Fn f)
 {
     const int q = K / 4;
     if (fused) {
@@ -707,6 +707,10 @@ auto with_shape(int K, bool fused, Fn f)
     if (q < 32) return f(SpmmShape<16, 2, 4, false, 3>());
     if (q == 32) return f(SpmmShape<16, 2, 4, true, 4>());
     if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4>());
+    // (few nonzeros: a block fewer, tails in shared memory; us, this / the lines below: K = 200 0.26 M 24.6 / 26.5, documents x words, 0.75 M 43.6 / 45.3;  1.2 M 72.3 / 66.1, 1.5 M, columns alike 101 /
+    // 81;  K = 256 0.2 M 18.6 / 20.5, 0.26 M 26.9 / 28.7;  0.3 M 24.6 / 23.7, 0.6 M 41.3 / 40.8, 1.2 M 79.5 / 69.4)
+    if (q > 48 && q < 64 && nnz < 1000000) return f(SpmmShape<32, 2, 4, false, 3>());
+    if (q == 64 && nnz < 300000) return f(SpmmShape<32, 2, 4, true, 3>());
     if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, false, false, true, false, true>());
     if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, false, false, true, false, true>());
     if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3>());
@@ -747,7 +751,7 @@ constexpr size_t FAR_SETS = SP_TPB / 32;  // whose tails a block may leave in sc
 static size_t max_blocks(int64_t nnz, int64_t N, int K, int sm_count)
 {
     auto blocks = [&](int width, bool fused) {
-        return with_shape(width, fused, [&](auto s) {
+        return with_shape(width, fused, nnz, [&](auto s) {
             const size_t per_block = (size_t)decltype(s)::SETS * run_length<decltype(s)>(nnz, sm_count);
             return ((size_t)nnz + per_block - 1) / per_block;
         });
@@ -770,7 +774,7 @@ cudaError_t launch_spmm(const SpmmCall &a, int sm_count, int64_t *n_launches, cu
     const int w = a.W ? a.K : pass_floats(a.nnz, a.N, a.K);
     for (int k0 = 0; k0 < a.K; k0 += w) {
         const int width = std::min(w, a.K - k0);
-        const cudaError_t e = with_shape(width, a.W != nullptr, [&](auto s) { return launch_shape<decltype(s)>(a, k0, width, sm_count, n_launches, stream); });
+        const cudaError_t e = with_shape(width, a.W != nullptr, a.nnz, [&](auto s) { return launch_shape<decltype(s)>(a, k0, width, sm_count, n_launches, stream); });
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

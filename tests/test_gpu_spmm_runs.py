@@ -55,6 +55,29 @@ def test_run_boundaries(engine, K):
     plan.close()
 
 
+@pytest.mark.parametrize("K", [196, 200, 252, 256])
+def test_tails_in_scratch(engine, K):
+    # a million nonzeros (K = 256: 300,000) and more leave the tails of runs in scratch; whole numbers: exact sums, on both sides of the lines
+    import torch
+    N, M = 5_003, 60_001
+    g = torch.Generator(device="cuda").manual_seed(K)
+    H = torch.randint(-1, 2, (N, K), generator=g, device="cuda").float()
+    for nnz in (299_999, 300_000, 999_999, 1_000_000, 1_300_007):
+        rows = torch.sort((torch.rand(nnz, generator=g, device="cuda") ** 4 * M).to(torch.int32).clamp_(max=M - 1)).values   # rows of many blocks and of a few nonzeros, and none
+        cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+        vals = torch.randint(-1, 2, (nnz,), generator=g, device="cuda").float()
+        plan = engine.plan_coo(M, N, rows, cols, K)
+        for pv in (vals, None):
+            Y = torch.full((M, K), float("nan"), device="cuda")
+            plan.spmm(H, Y, pv)
+            ref = torch.zeros((M, K), device="cuda", dtype=torch.float64)
+            for a in range(0, nnz, 200_000):
+                part = H[cols[a:a + 200_000].long()].double()
+                ref.index_add_(0, rows[a:a + 200_000].long(), part if pv is None else part * pv[a:a + 200_000, None].double())
+            assert float(ref.abs().max()) < 2 ** 22 and torch.equal(Y.double(), ref)
+        plan.close()
+
+
 @pytest.mark.parametrize("K", [16, 32, 64, 96, 160, 192, 200, 256, 320, 384, 512, 768, 1024])
 def test_block_boundaries(engine, K):
     # A block holds 8 to 64 runs of 8, 16 or 24 nonzeros.  Rows that begin and end at multiples of 8 and 64 and one beside them, rows of a block and of
