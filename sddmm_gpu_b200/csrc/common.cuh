@@ -99,6 +99,7 @@ PanelConfig choose_panel_config(int K, int panel_rows_hint, int sm_count, size_t
 struct GatherPasses {
     int n, floats;           // launches, columns of each (the last one may have fewer)
     bool few_lanes = false;  // the shape with fewer lanes for a nonzero, where there are two
+    bool large_h = false;    // most rows of H come from DRAM
     bool awaited = false;    // by the host, as soon as it has been launched
 };
 // What is best for an H of N rows; one pass where S values and P share memory.  tiled: the nonzeros are in the order of column tiles.

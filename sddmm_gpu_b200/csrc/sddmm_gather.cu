@@ -341,7 +341,7 @@ struct GatherCall {
     unsigned long long *clock;
     bool beside;
     cudaStream_t stream;
-    bool few_lanes = false, awaited = false;
+    bool few_lanes = false, large_h = false, awaited = false;
 };
 
 template <class S>
@@ -410,7 +410,8 @@ cudaError_t launch_pieces(const GatherCall &c)
     if (q <= 4) GA_GO(4, 1, 4, 4, false, false, 6);
     // Up to 16 pieces all eight sums of a step are reduced together, eight shuffles for 8 instead of ten; with 48 registers more blocks are resident.  us, four at
     // a time / this: K = 64 16.1 M nonzeros 285.7 / 279.9, 6.0 M 107.1 / 102.3, 1.5 M, columns alike 30.7 / 28.7, 0.2 M 9.0 / 8.2;  K = 56 6.0 M 110.1 / 103.8;  K = 32 6.0 M 72.4 /
-    // 70.4, 1.6 M 22.4 / 20.9, documents x words, 0.7 M 12.0 / 10.5.  Passes of 64 columns keep four at a time (97 M nonzeros, K = 256 7729 / 8641).
+    // 70.4, 1.6 M 22.4 / 20.9, documents x words, 0.7 M 12.0 / 10.5.  Passes of 64 columns, and rows of 52 to 64 of an H that is mostly read from DRAM, keep
+    // four at a time (97 M nonzeros, 4.2 M rows of H: K = 256 7729 / 8641, K = 64 1805 / 1845; 1 M rows: above).
     if (q < 8) GA_GO(8, 1, 4, 8, false, false, 6);
     if (q == 8) GA_GO(8, 1, 4, 8, true, false, 6);
     if (q <= 12) GA_GO(4, 3, 2, 4, false, true, 4);
@@ -418,13 +419,15 @@ cudaError_t launch_pieces(const GatherCall &c)
     // 0.3 M 19.9 / 19.3, 0.4 M 21.3 / 21.1, a row of W for each of 0.07 M 15.7 / 15.3;  but 0.15 M 15.9 / 16.1, 0.205 M 17.6 / 18.2, 0.6 M 25.0 / 25.0, asynchronous 14.9 / 15.6).
     const unsigned share = c.nnz / ((unsigned)c.sm_count * 5 * (GA_TPB / 32) * 4);
     if (q > 12 && q <= 16 && !c.pass && share < 20) GA_GO(8, 2, 4, 8, false, false, 4);
+    if (q < 16 && c.large_h) GA_GO(8, 2, 4, 4, false, true, 4);
     if (q < 16) GA_GO(8, 2, 2, 8, false, true, 5);
-    if (q == 16 && c.pass) return launch_mode<GatherShape<8, 2, 4, 4, true, true, 4>, PASS>(c);
-    if (q == 16) return c.perm ? launch_mode<GatherShape<8, 2, 2, 8, true, false, 5>, PERM>(c) : launch_mode<GatherShape<8, 2, 2, 8, true, false, 5>, STORE>(c);
+    if (q == 16 && (c.pass || c.large_h)) GA_GO(8, 2, 4, 4, true, true, 4);
+    if (q == 16) GA_GO(8, 2, 2, 8, true, false, 5);
     if (q <= 24) GA_GO(8, 3, 2, 8, false, true, 4);
     // Here sixteen lanes take two pieces each, 25 to 31 of the 32, or eight lanes four.  Eight lanes need fewer shuffles, but a wave of them is more nonzeros, and fewer warps: for
     // many nonzeros of an H that L1 holds little of (gather_passes).  K = 100, us, sixteen / eight: 6.0 M nonzeros 175.6 / 168.0, 4.1 M 126.6 / 121.5, 1.6 M 53.7 / 51.7, 1.5 M, columns
-    // alike 51.4 / 47.4;  but 0.2 M 11.5 / 14.3, documents x words 0.75 M, 4,000 words 1.8 M 27.0 / 28.7, 59.9 / 61.7.
+    // alike 51.4 / 47.4;  but 0.2 M 11.5 / 14.3, documents x words 0.75 M, 4,000 words 1.8 M 27.0 / 28.7, 59.9 / 61.7, and
+    // 97 M of an H of 1.7 GB 3690 / 3863.
     if (q < 32 && c.few_lanes) GA_GO(8, 4, 1, 8, false, true, 4);
     if (q < 32) GA_GO(16, 2, 2, 8, false, true, 5);
     if (q == 32) GA_GO(16, 2, 2, 8, true, false, 5);
@@ -480,7 +483,7 @@ cudaError_t launch_pieces(const GatherCall &c)
 GatherPasses gather_passes(int64_t nnz, int64_t N, int K, bool tiled, const float *sval, const float *P)
 {
     const int64_t h_bytes = N * K * 4;
-    const GatherPasses whole = {1, K, nnz >= 1000000 && h_bytes >= 8000000};
+    const GatherPasses whole = {1, K, nnz >= 1000000 && h_bytes >= 8000000 && h_bytes < 300000000, h_bytes >= 500000000};
     if (sval && sval < P + nnz && P < sval + nnz) return whole;  // the first pass would overwrite S values that the last one needs
     int floats = K;
     if (K > 320) {
@@ -499,7 +502,7 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
                           const float *H, float *P, int64_t nnz, int K, GatherPasses passes, int sm_count, unsigned long long *clock,
                           cudaStream_t stream, bool beside)
 {
-    if (perm) passes = {1, K, passes.few_lanes};
+    if (perm) passes = {1, K, passes.few_lanes, passes.large_h};
     for (int pass = 0; pass < passes.n; ++pass) {
         const int k0 = pass * passes.floats, width = K - k0 < passes.floats ? K - k0 : passes.floats;
         for (int64_t j0 = 0; j0 < nnz; j0 += GATHER_SLICE) {
@@ -523,6 +526,7 @@ cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_
             c.beside = beside && j0 == 0;
             c.stream = stream;
             c.few_lanes = passes.few_lanes;
+            c.large_h = passes.large_h;
             c.awaited = passes.awaited;
             cudaError_t e;
             if (c.pieces <= 256) {
