@@ -353,7 +353,7 @@ cudaError_t launch_few(const GatherCall &c)
     cfg.blockDim = dim3(GA_TPB);
     cfg.stream = c.stream;
     return cudaLaunchKernelEx(&cfg, sddmm_gather_few_kernel<S>, c.rows, c.cols, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.clock,
-                              last_wave(blocks, (unsigned)c.sm_count * 3));
+                              last_wave(blocks, (unsigned)c.sm_count * (2048 / GA_TPB)));
 }
 
 template <class S, GatherMode MODE>
