@@ -27,8 +27,8 @@
 // SpMM, 0.2 M nonzeros, K = 64, 128 14.4 / 12.3, 17.0 / 14.4;  1.2 M, K = 64, 128 31.0 / 26.6, 47 / 41;  6.0 M, K = 64 114 / 100;  fused, 30 K nonzeros, K = 64 12.2 / 9.2;
 // 0.2 M, K = 128 24.5 / 20.5;  1.2 M, K = 128 75 / 62;  1.5 M, columns alike, K = 32 39 / 29).  Rows of S without nonzeros are zeroed by blocks of their own at the end of the grid.
 //
-// What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero from L2, some 65 bytes a clock and SM at most; used twice in the fused form), hidden
-// by resident warps: SpMM takes 46 bytes a clock at K = 64, 67 at K = 256.  The fused form also computes: a block of B nonzeros is reduced, spread
+// What bounds it: the gathers, as in SDDMM (4K bytes of H per nonzero from L2, some 65 to 70 bytes a clock and SM at most; used twice in the fused form), hidden
+// by resident warps: SpMM takes 59 bytes a clock at K = 64, 70 at K = 256 (6.0 M nonzeros).  The fused form also computes: a block of B nonzeros is reduced, spread
 // and added with nothing of its warp in flight (6.0 M nonzeros, K = 256: 1,180 clocks of 2,220 wait for memory), and more warps or more rows in flight do not fit the
 // registers.  Measured and not kept: rows of H through a ring of shared memory by 16-byte or bulk copies (the ring takes what L1 gave: 16.1 M, K = 256, 1407 with a ring of 64 KB a block while L1 had 32 KB, 2180
 // with 9 KB; bulk copies 1617 - 2490), H rows of the next block in registers (two nonzeros a block, 1571).
