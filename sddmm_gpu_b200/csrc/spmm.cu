@@ -624,6 +624,8 @@ unsigned run_length(int64_t nnz, int sm_count)
         // One nonzero at a time: a row that fills a run has as many roundings one after the other as the run is long.  32 nonzeros and up to a
         // third of a set's share, 80 and up to a sixth, 160 and up to a twelfth.
         waves = s <= 32 ? 1 : s <= 64 ? 2 : s <= 240 ? 3 : s <= 480 ? (s + 79) / 80 : std::min<int64_t>(12, std::max<int64_t>(6, (s + 159) / 160));
+        // (the fused form of 68 to 96 columns took two at a time before it had this shape: runs of two thirds leave its sums no less exact)
+        if (S::FUSED && S::L == 8 && S::F == 3 && s > 32) waves = (waves * 3 + 1) / 2;
     } else {
         // B at a time (add_block): a B-th of the roundings.  At most as many as where one at a time is added, and 80 up to 1,920 nonzeros.
         // (Relative error of sums of positive terms, rms of all entries, one at a time / the waves of the table alone / with this limit: 8 M nonzeros, rows of
