@@ -233,14 +233,17 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             y[f].b = add2(y[f].b, tb);
         }
     };
+    // Two sums from three pieces on: one sum of six terms and more loses more to rounding (operands of both signs, rms: K = 384 8.19e-8 / 8.03e-8, K = 512 8.62e-8 / 8.29e-8,
+    // K = 768 9.39e-8 / 8.76e-8).
     auto dot = [&](const u64x2 (&h)[F]) {
-        unsigned long long a = 0;
+        unsigned long long a = 0, b = 0;
 #pragma unroll
         for (int f = 0; f < F; ++f) {
             a = ffma2(w[f].a, h[f].a, a);
-            a = ffma2(w[f].b, h[f].b, a);
+            if constexpr (F > 2) b = ffma2(w[f].b, h[f].b, b);
+            else a = ffma2(w[f].b, h[f].b, a);
         }
-        return fold2(a);
+        return F > 2 ? fold2(a) + fold2(b) : fold2(a);
     };
     if constexpr (S::STAGED) {
         // Rows, columns and S values of 32 nonzeros lie in shared memory, from where a block of B takes its columns and its weights by one

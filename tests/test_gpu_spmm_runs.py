@@ -134,6 +134,23 @@ def test_last_nonzero_infinite(engine, K):
         plan.close()
 
 
+@pytest.mark.parametrize("K", [388, 512, 644, 768])
+def test_weights_of_fused_as_sddmm(engine, K):
+    # the same lanes hold the same pieces as in the gather kernel at these K, two sums a lane: P comes out with the same bits
+    import torch
+    M, N, nnz = 900, 1_100, 30_001
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    W, H, S = (torch.randn(n, generator=g, device="cuda") for n in ((M, K), (N, K), (nnz,)))
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    P, P_fused, Y = torch.empty(nnz, device="cuda"), torch.full((nnz,), float("nan"), device="cuda"), torch.empty((M, K), device="cuda")
+    plan.execute(W, H, P, S)
+    plan.fused(W, H, Y, S, P_fused)
+    plan.close()
+    assert torch.equal(P, P_fused)
+
+
 @pytest.mark.parametrize("K,N", [(448, 503_000), (512, 831_000), (900, 251_000)])
 def test_long_rows_in_passes(engine, K, N):
     # a large H, long rows: passes over part of the columns (the last one of 64, 128 and 132), a row of many runs, rows without nonzeros
