@@ -166,6 +166,8 @@ SDDMM_API int sddmm_execute(sddmm_plan_t p, const float *W, const float *H,
  *   sddmm_fused_execute: the same with Pval[i] = (sum_t W[r,t] H[col_i,t]) * Sval[i] computed on
  *                        the fly (Sval NULL: unscaled) -- P never goes to memory and every H row
  *                        is gathered once for both uses; P_out != NULL also stores P (input order).
+ * Y may be W itself in sddmm_fused_execute (an update of W in place): each row of W is used up
+ * before the row of Y is stored.  Apart from that Y must not overlap what the call reads.
  * K a multiple of 4 up to 1024 (SDDMM_K_UNSUPPORTED otherwise).  Pointers host or device (host
  * arrays are staged for the call); flags: 0 or SDDMM_FLAG_ASYNC (device pointers only).  The
  * nonzeros are cut into equal runs; the parts of a row of S that spans runs are added in run order: the

@@ -19,7 +19,8 @@
 //
 // A row that crosses a run boundary is in parts: what the run in which it ends has of it (its head) and what the runs before that one have (their tails).  The runs of a
 // block follow one another, so a block adds up its own parts: tails go to shared memory, heads to Y for the time being, and behind a barrier the run in which a row ends
-// adds the tails before it, in order.  Only the row that a block begins with and the one that goes on behind it concern other blocks.  Their parts
+// adds the tails before it, in order.  (Y of the fused form may be W: each row of W is used up before its row of Y is stored.  Heads go to scratch then, ON_W, since other runs may
+// still read the row of W.  Heads in scratch for all calls: 1 to 10 % slower, K = 32 10 %, K = 256 3 %, since what picks the address sits in the loop.)  Only the row that a block begins with and the one that goes on behind it concern other blocks.  Their parts
 // go to scratch -- 2 b: block b's part of a row that ends in it, 2 b + 1: of one that goes on -- and the block that arrives last at a row (a counter per row) adds them
 // up in order: no atomics on Y, the result does not depend on scheduling, and there is no second launch (a fix-up kernel took a third of a call with ten thousand
 // nonzeros).  Parts are added in groups of 16 blocks, each by its last block, and the groups by the last of those, so that a row of hundreds of blocks does not end in one long
@@ -69,7 +70,8 @@ struct SpmmShape {
     static constexpr int SETS = SP_TPB / 32 * G;         // of a block
     static constexpr int TAIL_BYTES = FAR ? 0 : SP_TPB * F * 16;  // a row for each of them
     static_assert(NB % B == 0, "step geometry");
-    static_assert(!FAR || L == 32, "FAR_SETS");
+    static_assert(!FAR || !FUSED, "a set has one row in scratch");
+    static constexpr int SLOTS = FUSED || FAR ? SETS : 0;  // rows of a block's sets in scratch: heads of the fused form (ON_W), tails of FAR
     static_assert(!STAGED || (FUSED && JOINT && L == 32), "staged: a warp for a nonzero");
 };
 
@@ -128,7 +130,7 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
     return d;
 }
 
-template <class S>
+template <class S, bool ON_W>
 __global__ void __launch_bounds__(SP_TPB, S::CTAS)
 spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const float *__restrict__ val,
             const char *__restrict__ W, const char *__restrict__ H, float *__restrict__ P_out, char *__restrict__ Y,
@@ -196,6 +198,12 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     // after is not stored.  (Each where it costs nothing measurable.  fused, 16.1 M nonzeros, K = 256, us: without either 1646,
     // zero weights 1683, a row of its own 1638; 6.0 M, K = 512: 1088 / 1095 / 1142; SpMM, 6.0 M, K = 128: 224 / 224 / 229.)
     constexpr bool PAD = FUSED && S::JOINT;
+    // A row for each set, behind the blocks' parts.  (The block is read again each time: an address that waits in registers all through the loop makes shapes spill.)
+    auto slot_of = [&](int q) {
+        unsigned block;
+        asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block));
+        return scratch + (size_t)(2 * gather_blocks + block * T + q) * row_bytes;
+    };
     int cur = __ldg(rows + at(j0));                                // row being summed: that of the nonzero before this step
     auto began_before = [&](int row) { return j0 > 0 && __ldg(rows + at(j0 - 1)) == row; };  // it began in an earlier run
     bool head = began_before(cur);                                 // and nothing of it has been stored yet
@@ -203,9 +211,14 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     const int my_set = (threadIdx.x >> 5) * G + set;
     if (lig == 0) first_row[my_set] = cur;
     if (FUSED) load_w((unsigned)cur);
-    auto next_row = [&](int to) {  // the finished row is stored (one that began before this run for now: see below)
-        flush(Y + (size_t)(unsigned)cur * row_bytes);
+    auto store_row = [&] {  // the finished row; the head of one that began before this run for now
+        char *out = Y + (size_t)(unsigned)cur * row_bytes;
+        if (ON_W && head) out = slot_of(my_set);
+        flush(out);
         head = false;
+    };
+    auto next_row = [&](int to) {
+        store_row();
         cur = to;
     };
     auto add = [&](float weight, const u64x2 (&h)[F]) {
@@ -473,7 +486,6 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             s = sn;
         }
     }
-    auto far_tail_of = [&](int q) { return scratch + (size_t)(2 * gather_blocks + blockIdx.x * T + q) * row_bytes + lig * 16; };
     auto tail_of = [&](int q) { return smem_u32(tails) + q / G * (F * 512) + (q % G * L + lig) * 16; };
     bool goes_on = false;
     if (G == 1 || j0 < nnz) {
@@ -481,7 +493,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         goes_on = end < nnz && __ldg(rows + end) == cur;
         if (goes_on) {
             if constexpr (S::FAR) {
-                flush(far_tail_of(my_set) - lig * 16);
+                flush(slot_of(my_set));
             } else {
 #pragma unroll
                 for (int f = 0; f < F; ++f)
@@ -489,8 +501,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
             }
             if (!head && lig == 0) atomicOr(&openers[my_set / 32], 1u << (my_set & 31));
         } else if (!PAD || end <= nnz) {  // (else it was stored when the padding opened)
-            flush(Y + (size_t)(unsigned)cur * row_bytes);
-            head = false;
+            store_row();
         }
     }
     __syncthreads();
@@ -514,7 +525,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 #pragma unroll
                     for (int f = 0; f < F; ++f) {
                         const u64x2 v = !S::FAR ? lds_u64x2(tail_of(q + u) + f * 512)
-                                                : f < F - 1 || last_ok ? ldcg_u64x2(far_tail_of(q + u) + f * L * 16) : u64x2{0, 0};
+                                                : f < F - 1 || last_ok ? ldcg_u64x2(slot_of(q + u) + (f * L + lig) * 16) : u64x2{0, 0};
                         sum[u][f].a = add2(sum[u][f].a, v.a);
                         sum[u][f].b = add2(sum[u][f].b, v.b);
                     }
@@ -592,9 +603,10 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
     };
     if (enters && !head) {  // a row that began before this run has ended in it
         const size_t row = (size_t)(unsigned)first_row[my_set];
+        const char *const mine = (ON_W ? slot_of(my_set) : Y + row * row_bytes) + lig * 16;
 #pragma unroll
         for (int f = 0; f < F; ++f)
-            y[f] = f < F - 1 || last_ok ? ldcg_u64x2(Y + row * row_bytes + (f * L + lig) * 16) : u64x2{0, 0};
+            y[f] = f < F - 1 || last_ok ? ldcg_u64x2(mine + f * L * 16) : u64x2{0, 0};
         if (add_tails(my_set)) flush(Y + row * row_bytes);
         else hand_over(row);
     }
@@ -664,12 +676,16 @@ cudaError_t launch_shape(const SpmmCall &a, int k0, int width, int sm_count, int
     constexpr int smem = S::TAIL_BYTES;
     if (smem > 32 * 1024) {
         static SmemOptinCache optin;  // per device
-        const cudaError_t e = optin_dynamic_smem(spmm_kernel<S>, smem, optin);
+        const cudaError_t e = optin_dynamic_smem(spmm_kernel<S, false>, smem, optin);
         if (e != cudaSuccess) return e;
     }
-    spmm_kernel<S><<<gather_blocks + zero_blocks, SP_TPB, smem, stream>>>(
-        a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H + k0), a.P_out,
-        reinterpret_cast<char *>(a.Y + k0), parts, arrived, a.row_ptr, (unsigned)a.nnz, a.M, pieces, (unsigned)a.K * 4u, run, gather_blocks, a.clock, last_wave(gather_blocks, (unsigned)sm_count * S::CTAS));
+    auto launch = [&](auto kernel) {
+        kernel<<<gather_blocks + zero_blocks, SP_TPB, smem, stream>>>(
+            a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H + k0), a.P_out,
+            reinterpret_cast<char *>(a.Y + k0), parts, arrived, a.row_ptr, (unsigned)a.nnz, a.M, pieces, (unsigned)a.K * 4u, run, gather_blocks, a.clock, last_wave(gather_blocks, (unsigned)sm_count * S::CTAS));
+    };
+    if (S::FUSED && a.Y < a.W + a.M * a.K && a.W < a.Y + a.M * a.K) launch(spmm_kernel<S, S::FUSED>);
+    else launch(spmm_kernel<S, false>);
     ++*n_launches;
     return cudaGetLastError();
 }
@@ -751,26 +767,29 @@ int spmm_passes(int64_t nnz, int64_t N, int K)
 
 bool spmm_supports(int K) { return K > 0 && K % 4 == 0 && K <= 1024; }
 
-constexpr size_t FAR_SETS = SP_TPB / 32;  // whose tails a block may leave in scratch (FAR)
-// Blocks of runs, the most of either form and of every pass.
-static size_t max_blocks(int64_t nnz, int64_t N, int K, int sm_count)
+// The largest f(shape, blocks of runs) of either form and of every pass.
+template <class Fn>
+static size_t largest(int64_t nnz, int64_t N, int K, int sm_count, Fn f)
 {
-    auto blocks = [&](int width, bool fused) {
+    auto of = [&](int width, bool fused) {
         return with_shape(width, fused, nnz, [&](auto s) {
             const size_t per_block = (size_t)decltype(s)::SETS * run_length<decltype(s)>(nnz, sm_count);
-            return ((size_t)nnz + per_block - 1) / per_block;
+            return f(s, ((size_t)nnz + per_block - 1) / per_block);
         });
     };
-    size_t n = std::max(blocks(K, false), blocks(K, true));
+    size_t n = std::max(of(K, false), of(K, true));
     const int w = pass_floats(nnz, N, K);
-    if (w < K) n = std::max(n, blocks(w, false));
-    if (K % w) n = std::max(n, blocks(K % w, false));
+    if (w < K) n = std::max(n, of(w, false));
+    if (K % w) n = std::max(n, of(K % w, false));
     return n;
 }
-size_t spmm_counter_floats(int64_t nnz, int64_t N, int K, int sm_count) { return (2 * max_blocks(nnz, N, K, sm_count) + 31) / 32 * 32; }
+size_t spmm_counter_floats(int64_t nnz, int64_t N, int K, int sm_count)
+{
+    return (2 * largest(nnz, N, K, sm_count, [](auto, size_t blocks) { return blocks; }) + 31) / 32 * 32;
+}
 size_t spmm_scratch_floats(int64_t nnz, int64_t N, int K, int sm_count)
 {
-    return spmm_counter_floats(nnz, N, K, sm_count) + max_blocks(nnz, N, K, sm_count) * (2 + FAR_SETS) * (size_t)K;
+    return spmm_counter_floats(nnz, N, K, sm_count) + largest(nnz, N, K, sm_count, [](auto s, size_t blocks) { return blocks * (2 + decltype(s)::SLOTS); }) * (size_t)K;
 }
 
 cudaError_t launch_spmm(const SpmmCall &a, int sm_count, int64_t *n_launches, cudaStream_t stream)

@@ -134,6 +134,29 @@ def test_last_nonzero_infinite(engine, K):
         plan.close()
 
 
+@pytest.mark.parametrize("K", [4, 16, 20, 32, 36, 48, 60, 64, 68, 96, 100, 128, 160, 192, 200, 256, 320, 384, 512, 640, 768, 896, 1024])
+def test_fused_on_w(engine, K):
+    # Y on the memory of W: rows of a few nonzeros and of many blocks, at the borders of runs, the same bits as with Y elsewhere
+    import torch
+    M, N = 3_001, 2_003
+    g = torch.Generator(device="cuda").manual_seed(K)
+    for nnz in (2_999, 60_007, 400_009):
+        rows = torch.sort((torch.rand(nnz, generator=g, device="cuda") ** 4 * M).to(torch.int32).clamp_(max=M - 1)).values   # (and rows without any)
+        cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+        W, H, S = (torch.randn(n, generator=g, device="cuda") for n in ((M, K), (N, K), (nnz,)))
+        plan = engine.plan_coo(M, N, rows, cols, K)
+        Y, P = torch.full((M, K), float("nan"), device="cuda"), torch.full((nnz,), float("nan"), device="cuda")
+        plan.fused(W, H, Y, S, P)
+        for _ in range(3):
+            WY, P2 = W.clone(), torch.full((nnz,), float("nan"), device="cuda")
+            plan.fused(WY, H, WY, S, P2)
+            assert torch.equal(WY, Y) and torch.equal(P2, P)
+            WY = W.clone()
+            plan.fused(WY, H, WY, S)
+            assert torch.equal(WY, Y)
+        plan.close()
+
+
 @pytest.mark.parametrize("K", [388, 512, 644, 768])
 def test_weights_of_fused_as_sddmm(engine, K):
     # the same lanes hold the same pieces as in the gather kernel at these K, two sums a lane: P comes out with the same bits
