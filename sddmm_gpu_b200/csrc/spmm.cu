@@ -23,7 +23,7 @@
 // still read the row of W.  Heads in scratch for all calls: 1 to 10 % slower, K = 32 10 %, K = 256 3 %, since what picks the address sits in the loop.)  Only the row that a block begins with and the one that goes on behind it concern other blocks.  Their parts
 // go to scratch -- 2 b: block b's part of a row that ends in it, 2 b + 1: of one that goes on -- and the block that arrives last at a row (a counter per row) adds them
 // up in order: no atomics on Y, the result does not depend on scheduling, and there is no second launch (a fix-up kernel took a third of a call with ten thousand
-// nonzeros).  Parts are added in groups of 16 blocks, each by its last block, and the groups by the last of those, so that a row of hundreds of blocks does not end in one long
+// nonzeros).  Parts are added in groups of 16 or 8 blocks, each by its last block, and the groups by the last of those, so that a row of hundreds of blocks does not end in one long
 // chain.  With a fence, a counter and two reads of the row pointer at both ends of every run, a run's ends took some 8 us, what 40 nonzeros at K = 64 take (us, then / now:
 // SpMM, 0.2 M nonzeros, K = 64, 128 14.4 / 12.3, 17.0 / 14.4;  1.2 M, K = 64, 128 31.0 / 26.6, 47 / 41;  6.0 M, K = 64 114 / 100;  fused, 30 K nonzeros, K = 64 12.2 / 9.2;
 // 0.2 M, K = 128 24.5 / 20.5;  1.2 M, K = 128 75 / 62;  1.5 M, columns alike, K = 32 39 / 29).  Rows of S without nonzeros are zeroed by blocks of their own at the end of the grid.
@@ -54,7 +54,7 @@ constexpr int SP_TPB = 256;
 constexpr int SP_NB = 8;         // nonzeros of a set per index step (4 when a set is 4 lanes)
 constexpr int SP_MAX_RUN = 1024;
 
-constexpr unsigned SP_GROUP = 16;  // parts that one block adds
+constexpr int TAILS = 8;         // tails of a block's runs that are added before they go to the row
 
 // L lanes per nonzero, F pieces per lane, B nonzeros of a set in flight, CTAS resident blocks asked of the compiler.  PF: the
 // W rows of the next step are prefetched into L1.  JOINT: the B dot products are reduced together and a block of B that opens
@@ -139,6 +139,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 {
     constexpr int L = S::L, F = S::F, B = S::B, NB = S::NB, G = S::G, T = S::SETS;
     constexpr bool FUSED = S::FUSED;
+    constexpr unsigned GROUP = T == 8 && (F == 5 || F == 6) ? 8 : 16;  // parts that one block adds, at most eight times one after the other where a block is few sets
     extern __shared__ __align__(16) char tails[];  // what the sets have of rows that go on behind their runs, a piece for each lane
     __shared__ int first_row[T];
     __shared__ unsigned openers[2];  // the sets whose tail is the beginning of its row, a bit each
@@ -505,45 +506,39 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         }
     }
     __syncthreads();
-    // y += the tails of the sets before set `to` that belong to the row at hand, in their order; whether the row began in this block
+    // y += the tails of the sets before set `to` that belong to the row at hand, in their order; whether the row began in this block.  Eight are added before they go to the row: a
+    // block of sets of eight lanes may have 31, of four 63, and one by one they lose more to rounding than the runs do.  (Relative rms error against 64 bits, one by one or in two sums / so:
+    // documents x words, 0.75 M nonzeros, fused, K = 160 6.6e-8 / 5.3e-8, K = 48 5.7e-8 / 4.9e-8, SpMM, K = 48 5.5e-8 / 4.6e-8.  Two or four sums side by side hold more registers: fused, K = 48,
+    // six matrices 5 to 12 % slower.)
     auto add_tails = [&](int to) {
         unsigned long long before = openers[0];
         if (T > 32) before |= (unsigned long long)openers[1] << 32;
         if (to < 64) before &= (1ull << to) - 1;
         const int from = before ? 63 - __clzll((long long)before) : 0;
-        constexpr int U = F <= 2 ? 4 : F <= 4 ? 2 : 1;  // sums side by side
-        u64x2 sum[U][F];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int f = 0; f < F; ++f) sum[u][f] = u64x2{0, 0};
+        constexpr int AHEAD = FUSED ? 1 : 4;  // (the fused form has fewer registers to spare: K = 128 4 6 % slower)
+        auto tail = [&](int q, int f) {
+            return !S::FAR ? lds_u64x2(tail_of(q) + f * 512) : f < F - 1 || last_ok ? ldcg_u64x2(slot_of(q) + (f * L + lig) * 16) : u64x2{0, 0};
+        };
 #pragma unroll 1
-        for (int q = from; q < to; q += U) {
+        for (int q0 = from; q0 < to; q0 += TAILS) {
+            u64x2 sum[F];
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (q + u < to) {
-#pragma unroll
-                    for (int f = 0; f < F; ++f) {
-                        const u64x2 v = !S::FAR ? lds_u64x2(tail_of(q + u) + f * 512)
-                                                : f < F - 1 || last_ok ? ldcg_u64x2(slot_of(q + u) + (f * L + lig) * 16) : u64x2{0, 0};
-                        sum[u][f].a = add2(sum[u][f].a, v.a);
-                        sum[u][f].b = add2(sum[u][f].b, v.b);
-                    }
-                }
-        }
-#pragma unroll
-        for (int u = U / 2; u >= 1; u /= 2)
-#pragma unroll
-            for (int v = 0; v < u; ++v)
+            for (int f = 0; f < F; ++f) sum[f] = tail(q0, f);
+            const int q1 = min(q0 + TAILS, to);
+#pragma unroll AHEAD
+            for (int q = q0 + 1; q < q1; ++q) {
 #pragma unroll
                 for (int f = 0; f < F; ++f) {
-                    sum[v][f].a = add2(sum[v][f].a, sum[v + u][f].a);
-                    sum[v][f].b = add2(sum[v][f].b, sum[v + u][f].b);
+                    const u64x2 v = tail(q, f);
+                    sum[f].a = add2(sum[f].a, v.a);
+                    sum[f].b = add2(sum[f].b, v.b);
                 }
+            }
 #pragma unroll
-        for (int f = 0; f < F; ++f) {
-            y[f].a = add2(y[f].a, sum[0][f].a);
-            y[f].b = add2(y[f].b, sum[0][f].b);
+            for (int f = 0; f < F; ++f) {
+                y[f].a = add2(y[f].a, sum[f].a);
+                y[f].b = add2(y[f].b, sum[f].b);
+            }
         }
         return before != 0;
     };
@@ -562,7 +557,7 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         const unsigned first = (unsigned)row_ptr[row] / per_block, last = (unsigned)(row_ptr[row + 1] - 1) / per_block;
         auto part = [&](unsigned q) { return scratch + (size_t)(2 * q + (q < last ? 1 : 0)) * row_bytes + lig * 16; };
         auto add_up = [&](unsigned q0, unsigned q1, unsigned step) {  // y = parts q0, q0 + step, ... <= q1
-            constexpr int U = F <= 2 ? 4 : F <= 4 ? 2 : 1;
+            constexpr int U = F <= 2 ? 4 : F <= 4 || F > 6 ? 2 : 1;  // (two of five or six pieces spill)
 #pragma unroll
             for (int f = 0; f < F; ++f) y[f] = u64x2{0, 0};
 #pragma unroll 1
@@ -574,16 +569,23 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
                     for (int f = 0; f < F; ++f)
                         v[u][f] = q + u * step <= q1 && (f < F - 1 || last_ok) ? ldcg_u64x2(part(q + u * step) + f * L * 16) : u64x2{0, 0};
 #pragma unroll
-                for (int u = 0; u < U; ++u)
+                for (int u = U / 2; u >= 1; u /= 2)
 #pragma unroll
-                    for (int f = 0; f < F; ++f) {
-                        y[f].a = add2(y[f].a, v[u][f].a);
-                        y[f].b = add2(y[f].b, v[u][f].b);
-                    }
+                    for (int x = 0; x < u; ++x)
+#pragma unroll
+                        for (int f = 0; f < F; ++f) {
+                            v[x][f].a = add2(v[x][f].a, v[x + u][f].a);
+                            v[x][f].b = add2(v[x][f].b, v[x + u][f].b);
+                        }
+#pragma unroll
+                for (int f = 0; f < F; ++f) {
+                    y[f].a = add2(y[f].a, v[0][f].a);
+                    y[f].b = add2(y[f].b, v[0][f].b);
+                }
             }
         };
         flush(part(me) - lig * 16);
-        const unsigned g0 = first + (me - first) / SP_GROUP * SP_GROUP, g1 = min(g0 + SP_GROUP - 1, last);
+        const unsigned g0 = first + (me - first) / GROUP * GROUP, g1 = min(g0 + GROUP - 1, last);
         // (a group that is the row's last block only needs no counter, and has none: the next row may begin in that block)
         if (g1 > g0) {
             if (arrive(&arrived[2 * g0]) != g1 - g0) return;
@@ -593,10 +595,10 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
         add_up(g0, g1, 1);
         if (g0 != first || g1 != last) {
             flush(part(g0) - lig * 16);
-            if (arrive(&arrived[2 * first + 1]) != (last - first) / SP_GROUP) return;
+            if (arrive(&arrived[2 * first + 1]) != (last - first) / GROUP) return;
             if (lig == 0) arrived[2 * first + 1] = 0;
             __threadfence();
-            add_up(first, last, SP_GROUP);
+            add_up(first, last, GROUP);
         }
         flush(Y + row * row_bytes);
         if (clock && lig == 0) clock_note(clock);  // (a row of many blocks: this may outlast every block that starts later)

@@ -227,6 +227,35 @@ def test_rounding_of_long_rows(engine, K, M, n, block, chain):
     assert (square / (M * K)) ** 0.5 <= 2.0 ** -24 / 3 ** 0.5 * (chain / (3 * p) + p / 3 + 1) ** 0.5
 
 
+@pytest.mark.parametrize("fused,K,M,n,block,chain", [(False, 48, 550, 700, 2, 6), (True, 48, 550, 700, 2, 6), (True, 160, 550, 700, 1, 24)])
+def test_rounding_of_parts(engine, fused, K, M, n, block, chain):
+    # As above, the fused form too (W picks a column of ones of H: the weights are S).  The p parts of a row are added eight at a time and the sums of eight one after the other, and a row
+    # goes over to the next block: 1 more.  A rounding is 2^-24 / sqrt(3) rms of the power of two below the sum; over all places between two powers of two, by their logarithm, that is
+    # sqrt(0.54) of it relative to the sum.  (Parts one after the other, 29 and 31 of them: 1.1 to 1.3 times these bounds.)
+    import torch
+    N = 20_000
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.arange(M, device="cuda", dtype=torch.int32).repeat_interleave(n)
+    cols = torch.randint(0, N, (M, n), generator=g, device="cuda").sort(dim=1).values
+    H, vals = torch.rand((N, K), generator=g, device="cuda"), torch.rand((M, n), generator=g, device="cuda")
+    plan = engine.plan_coo(M, N, rows, cols.flatten().to(torch.int32), K)
+    Y = torch.full((M, K), float("nan"), device="cuda")
+    if fused:
+        W = torch.zeros((M, K), device="cuda")
+        H[:, 0], W[:, 0] = 1, 1
+        plan.fused(W, H, Y, vals.flatten())
+    else:
+        plan.spmm(H, Y, vals.flatten())
+    plan.close()
+    square = 0.0
+    for a in range(0, M, 200):
+        ref = torch.einsum("mn,mnk->mk", vals[a:a + 200].double(), H[cols[a:a + 200]].double())
+        square += float(((Y[a:a + 200].double() - ref) / ref).square().sum())
+    p = n / (chain * block)
+    parts = p / 3 if p <= 8 else 64 / (3 * p) + p / 24
+    assert square / (M * K) <= 2.0 ** -48 / 3 * 0.54 * (chain / (3 * p) + parts + 2)
+
+
 @pytest.mark.parametrize("K,N", [(388, 590_000), (416, 545_000), (644, 354_000), (900, 420_000)])
 def test_long_rows_whole(engine, K, N):
     # rows that are no multiple of 128 bytes, or whose last pass would be narrow: one launch, however large H is
