@@ -38,6 +38,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "common.cuh"
@@ -60,10 +61,11 @@ constexpr int TAILS = 8;         // tails of a block's runs that are added befor
 // W rows of the next step are prefetched into L1.  JOINT: the B dot products are reduced together and a block of B that opens
 // no row is summed without the tests for it.  Taken where a nonzero has a whole warp or a set few pieces, while with several sets in a warp
 // most blocks open a row in one of them (K = 128 871 -> 965).  STAGED (a warp for a nonzero): rows, columns and S values of 32 nonzeros in shared memory, see the
-// kernel.  FAR: tails in scratch instead of shared memory, which is L1 that four blocks of SpMM with a warp for a nonzero miss (6.0 M nonzeros, K = 256: 348 / 330 us, 338
+// kernel.  LIMIT: a shape that rounds as much as this one may (run_length).  FAR: tails in scratch instead of shared memory, which is L1 that four blocks of SpMM with a warp for a nonzero miss (6.0 M nonzeros, K = 256: 348 / 330 us, 338
 // with no shared memory and the run ends of before; K = 512 722 / 726).
-template <int L_, int F_, int B_, bool EXACT_, int CTAS_, bool FUSED_ = false, bool PF_ = false, bool JOINT_ = true, bool STAGED_ = false, bool FAR_ = false>
+template <int L_, int F_, int B_, bool EXACT_, int CTAS_, bool FUSED_ = false, bool PF_ = false, bool JOINT_ = true, bool STAGED_ = false, bool FAR_ = false, class LIMIT_ = void>
 struct SpmmShape {
+    using LIMIT = LIMIT_;
     static constexpr int L = L_, F = F_, B = B_, CTAS = CTAS_;
     static constexpr bool EXACT = EXACT_, FUSED = FUSED_, PF = PF_, JOINT = JOINT_, STAGED = STAGED_, FAR = FAR_;
     static constexpr int NB = L < SP_NB ? L : SP_NB, G = 32 / L;
@@ -641,8 +643,6 @@ unsigned run_length(int64_t nnz, int sm_count)
         // One nonzero at a time: a row that fills a run has as many roundings one after the other as the run is long.  32 nonzeros and up to a
         // third of a set's share, 80 and up to a sixth, 160 and up to a twelfth.
         waves = s <= 32 ? 1 : s <= 64 ? 2 : s <= 240 ? 3 : s <= 480 ? (s + 79) / 80 : std::min<int64_t>(12, std::max<int64_t>(6, (s + 159) / 160));
-        // (the fused form of 68 to 96 columns took two at a time before it had this shape: runs of two thirds leave its sums no less exact)
-        if (S::FUSED && S::L == 8 && S::F == 3 && s > 32) waves = (waves * 3 + 1) / 2;
     } else {
         // B at a time (add_block): a B-th of the roundings.  At most as many as where one at a time is added, and 80 up to 1,920 nonzeros.
         // (Relative error of sums of positive terms, rms of all entries, one at a time / the waves of the table alone / with this limit: 8 M nonzeros, rows of
@@ -654,14 +654,24 @@ unsigned run_length(int64_t nnz, int sm_count)
                          : s <= 340 ? 1 : std::max<int64_t>(2, (s + 759) / 760);
         waves = std::max(waves, (s + S::B * chain - 1) / (S::B * chain));
     }
-    int64_t run = (nnz / (waves * wave) + S::NB) / S::NB * S::NB;  // rounded up: one run less than a wave, not one more
     // Fewer, longer runs where they would be very short (us at runs of 8 / 16 / 24, SpMM: s = 3, K = 128 10.5 / 11.0 / 11.9, K = 512 12.0 / 10.3 / 12.0;  s = 6, K = 192 14.8 / 14.3 / 15.3,
     // K = 512 15.8 / 14.3 / 12.3;  s = 8, K = 128 13.8 / 12.3 / 14.3, K = 192 16.0 / 14.4 / 16.4;  s = 10, K = 256 15.5 / 12.5 / 12.3, K = 512 18.4 / 15.0 / 16.4;  s = 14, K = 64 20.6 / 16.4 / 16.5,
     // K = 300 19.0 / 16.8 / 15.1, K = 512 22.5 / 19.0 / 16.4;  fused: s = 6, K = 64 14.2 / 14.7 / 16.4, K = 256 12.4 / 13.6 / 16.4, K = 512 20.5 / 19.5 / 22.3;  s = 14, K = 64 22.6 / 18.4 / 20.5,
     // K = 512 31.0 / 24.5 / 25.9).
-    if (!S::FUSED && s > 4) run = std::max<int64_t>(run, (s > 12 ? 3 : 2) * S::NB);
-    if (S::FUSED && S::F >= 4 && s > 5) run = std::max<int64_t>(run, 2 * S::NB);
-    return (unsigned)std::min<int64_t>(run, SP_MAX_RUN);
+    int64_t least = S::NB, most = SP_MAX_RUN;
+    if (!S::FUSED && s > 4) least = (s > 12 ? 3 : 2) * S::NB;
+    if (S::FUSED && S::F >= 4 && s > 5) least = 2 * S::NB;
+    // The share s of a set, and with it the table, depends on how many sets are resident and on how many nonzeros they take at a time.  A shape with another of either than the one that the
+    // roundings were measured with (LIMIT) has runs no longer than that one's.  A run of n nonzeros adds n / B times to a row's sum, one after the other, and a long row loses a third of
+    // that to rounding, in squares and for the run's part of it: n^2 / B counts.  More waves then, not runs that end in the middle of one (fused, K = 256, 0.2 M nonzeros on three
+    // resident blocks, runs of 48 32.4 us, of 32 28.2).  Rows of 700 positive terms, squares of the relative error in 2^-48 / 3, by the table alone / so: fused, K = 256, 6.5 M nonzeros
+    // 4.7 / 3.2, K = 512, 2.0 M 4.1 / 2.9, SpMM, K = 200, 1.4 M 6.0 / 3.1.
+    if constexpr (!std::is_void<typename S::LIMIT>::value)
+        most = std::max<int64_t>(S::NB, (int64_t)(run_length<typename S::LIMIT>(nnz, sm_count) * std::sqrt((double)S::B / S::LIMIT::B) + S::NB / 2) / S::NB * S::NB);
+    least = std::min(least, most);
+    auto cut = [&] { return std::max(least, (nnz / (waves * wave) + S::NB) / S::NB * S::NB); };  // rounded up: one run less than a wave, not one more
+    while (cut() > most && cut() > S::NB) ++waves;
+    return (unsigned)std::min(cut(), most);
 }
 
 template <class S>
@@ -693,31 +703,33 @@ cudaError_t launch_shape(const SpmmCall &a, int k0, int width, int sm_count, int
 }
 
 // Calls f with the shape for K (L * (F - 1) < K / 4 <= L * F).  The fused form holds the W row as well and wants fewer
-// nonzeros in flight; every line is the best of a sweep over (L, B, prefetch, joint reduction, resident blocks).  The fused ones against the lines before them, us,
-// 6.0 M / 1.2 M nonzeros: K = 32, sets of 8 x 1, two at a time 170 / 35, this 118 / 31;  K = 96, 8 x 3, two at a time 241 / 57, this 211 / 47;  K = 160, 16 x 3 391 / 92, this 334 / 79;
-// K = 320, a warp 696 / 151, this 637 / 133.  SpMM, K = 200, three blocks / this: 6.0 M 355 / 300, 1.5 M, columns alike 101 / 82.
+// nonzeros in flight; every line is the best of a sweep over (L, B, prefetch, joint reduction, resident blocks).  The fused ones against the LIMIT lines that they took the place of, us,
+// 6.0 M / 1.2 M nonzeros: K = 32 161 / 37, this 130 / 32;  K = 160 411 / 98, this 330 / 78;  K = 320 780 / 168, this 628 / 131;  K = 256 531 / 127, this 474 / 114;  K = 512 996 / 212, this
+// 941 / 206.  SpMM, K = 200, three blocks / this: 6.0 M 357 / 301, 1.35 M 83 / 77, 1.5 M, columns alike 103 / 86.  Not taken, since short rows lose more to rounding: fused, K = 96, one at a time
+// (239 / 57 -> 218 / 50, but rows of 100, 30 M nonzeros, squares of the relative error in 2^-48 / 3 7.6 -> 11.0), K = 32, four at a time (130 / 32 -> 120 / 31; rows of 15, 1.5 M
+// 5.39e-8 -> 5.48e-8).
 template <class Fn>
 auto with_shape(int K, bool fused, int64_t nnz, Fn f)
 {
     const int q = K / 4;
     if (fused) {
         if (q <= 4) return f(SpmmShape<4, 1, 2, false, 4, true, true, false>());
-        if (q < 8) return f(SpmmShape<8, 1, 4, false, 5, true, true, true>());
-        if (q == 8) return f(SpmmShape<8, 1, 4, true, 5, true, true, true>());
+        if (q < 8) return f(SpmmShape<8, 1, 2, false, 5, true, true, true, false, false, SpmmShape<8, 1, 2, false, 4, true>>());
+        if (q == 8) return f(SpmmShape<8, 1, 2, true, 5, true, true, true, false, false, SpmmShape<8, 1, 2, false, 4, true>>());
         if (q <= 12) return f(SpmmShape<4, 3, 2, false, 4, true, true, false>());
         if (q < 16) return f(SpmmShape<8, 2, 2, false, 4, true, true, false>());
         if (q == 16) return f(SpmmShape<8, 2, 2, true, 4, true, true, false>());
-        if (q <= 24) return f(SpmmShape<8, 3, 1, false, 4, true, true, false>());
+        if (q <= 24) return f(SpmmShape<8, 3, 2, false, 3, true, true, false>());
         if (q < 32) return f(SpmmShape<8, 4, 1, false, 3, true, true, false>());
         if (q == 32) return f(SpmmShape<8, 4, 1, true, 4, true, false, false>());
-        if (q <= 40) return f(SpmmShape<8, 5, 1, false, 3, true, true, false>());
+        if (q <= 40) return f(SpmmShape<8, 5, 1, false, 3, true, true, false, false, false, SpmmShape<16, 3, 1, false, 4, true>>());
         if (q <= 48) return f(SpmmShape<16, 3, 1, false, 4, true, true, false>());
-        if (q <= 64) return f(SpmmShape<32, 2, 4, false, 3, true, true, true, true>());
-        if (q <= 80) return f(SpmmShape<16, 5, 1, false, 3, true, true, false>());
-        if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3, true, true, true, true>());
-        if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3, true, false, true, true>());
+        if (q <= 64) return f(SpmmShape<32, 2, 4, false, 3, true, true, true, true, false, SpmmShape<32, 2, 4, false, 4, true>>());
+        if (q <= 80) return f(SpmmShape<16, 5, 1, false, 3, true, true, false, false, false, SpmmShape<32, 3, 1, false, 4, true>>());
+        if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3, true, true, true, true, false, SpmmShape<32, 3, 1, false, 4, true>>());
+        if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3, true, false, true, true, false, SpmmShape<32, 4, 1, false, 4, true>>());
         if (q <= 160) return f(SpmmShape<32, 5, 1, false, 3, true, false, false>());
-        if (q <= 192) return f(SpmmShape<32, 6, 2, false, 2, true, false, true, true>());
+        if (q <= 192) return f(SpmmShape<32, 6, 2, false, 2, true, false, true, true, false, SpmmShape<32, 6, 1, false, 2, true>>());
         if (q <= 224) return f(SpmmShape<32, 7, 1, false, 2, true, false, false>());
         return f(SpmmShape<32, 8, 1, false, 2, true, false, false>());
     }
@@ -730,11 +742,12 @@ auto with_shape(int K, bool fused, int64_t nnz, Fn f)
     if (q < 32) return f(SpmmShape<16, 2, 4, false, 3>());
     if (q == 32) return f(SpmmShape<16, 2, 4, true, 4>());
     if (q <= 48) return f(SpmmShape<16, 3, 2, false, 4>());
-    // (few nonzeros: a block fewer, tails in shared memory; us, this / the lines below: K = 200 0.26 M 24.6 / 26.5, documents x words, 0.75 M 43.6 / 45.3;  1.2 M 72.3 / 66.1, 1.5 M, columns alike 101 /
-    // 81;  K = 256 0.2 M 18.6 / 20.5, 0.26 M 26.9 / 28.7;  0.3 M 24.6 / 23.7, 0.6 M 41.3 / 40.8, 1.2 M 79.5 / 69.4)
+    // (few nonzeros, tails in shared memory; us, this / the lines below: K = 200, a block fewer, 0.26 M 24.6 / 26.5, documents x words, 0.75 M 43.6 / 45.3, but 1.2 M 73 / 68;  K = 256, three blocks / four /
+    // four and tails in scratch: 60 K 10.4 / 12.3 / -, 79 K 12.4 / 14.4 / 14.4, 70 K 12.3 / 12.3 / 14.4, 0.1 M 18.2 / 14.0 / -, 0.2 M 21 / 20.3 / 20.6, 0.28 M 30.5 / 25.1 / 24.7)
     if (q > 48 && q < 64 && nnz < 1000000) return f(SpmmShape<32, 2, 4, false, 3>());
-    if (q == 64 && nnz < 300000) return f(SpmmShape<32, 2, 4, true, 3>());
-    if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, false, false, true, false, true>());
+    if (q == 64 && nnz < 85000) return f(SpmmShape<32, 2, 4, true, 3, false, false, true, false, false, SpmmShape<32, 2, 4, true, 4>>());
+    if (q == 64 && nnz < 300000) return f(SpmmShape<32, 2, 4, true, 4>());
+    if (q < 64) return f(SpmmShape<32, 2, 4, false, 4, false, false, true, false, true, SpmmShape<32, 2, 4, false, 3>>());
     if (q == 64) return f(SpmmShape<32, 2, 4, true, 4, false, false, true, false, true>());
     if (q <= 96) return f(SpmmShape<32, 3, 2, false, 3>());
     if (q <= 128) return f(SpmmShape<32, 4, 2, false, 3>());
