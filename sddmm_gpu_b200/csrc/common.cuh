@@ -100,7 +100,7 @@ struct GatherPasses {
     int n, floats;           // launches, columns of each (the last one may have fewer)
     bool few_lanes = false;  // the shape with fewer lanes for a nonzero, where there are two
     bool large_h = false;    // most rows of H come from DRAM
-    bool awaited = false;    // by the host, as soon as it has been launched
+    bool awaited = false;    // by the host, as soon as it has been launched, with P in the GPU's memory
 };
 // What is best for an H of N rows; one pass where S values and P share memory.  tiled: the nonzeros are in the order of column tiles.
 GatherPasses gather_passes(int64_t nnz, int64_t N, int K, bool tiled, const float *sval, const float *P);

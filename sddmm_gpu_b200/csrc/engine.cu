@@ -400,14 +400,14 @@ bool rows_on_ring(const sddmm_plan_s *p, bool force_ring, bool permuted)
 
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
-                        unsigned long long *clock, cudaStream_t stream, bool beside)
+                        unsigned long long *clock, cudaStream_t stream, bool beside, bool awaited)
 {
     sddmm_handle_s *h = p->h;
     p->pending = true;  // (sddmm_execute clears it again when it waits)
     // the split of the whole matrix: a chunk of it is summed in the order that the whole would be
     const int64_t whole = rows == p->dense.rows_s ? p->dense.n_sparse : p->nnz;
     GatherPasses passes = gather_passes(whole, p->N, p->K, p->d_perm && !perm, sval, P);
-    passes.awaited = clock != nullptr;
+    passes.awaited = awaited;
     rows += first;
     if (perm) {
         perm += first;
@@ -867,10 +867,12 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
     const bool one_gather = !use_dense && !use_panel && (use_gather || !rows_on_ring(p, use_ring, permuted)) &&
                             (permuted || use_gather || gather_passes(p->nnz, p->N, p->K, p->d_perm != nullptr, dS, P).n == 1);
     bool p_copy = false;
+    bool awaited = !async;  // the kernel for few nonzeros stores in smaller pieces, which counts over PCIe (mapped P, us, before / with it: K = 32, 30,000 nonzeros 18.8 / 20.4, K = 128, 16,777 18.7 / 21.1)
     if (!p_dev) {
         // a small P is written to mapped host memory by the kernel: its 32-byte stores over PCIe cost less than a copy
         float *P_mapped = one_gather && !pipelined && h->sparse_upload && nbytes <= (256 << 10) ? const_cast<float *>(mapped_host_ptr(P, 4)) : nullptr;
         p_copy = !P_mapped;
+        awaited &= p_copy;
         if (p_copy && !p->d_P) CUDA_TRY(h, dev_alloc(p, &p->d_P, (size_t)p->nnz));
         dP = P_mapped ? P_mapped : p->d_P;
         p->last_d2h_bytes = (int64_t)nbytes;
@@ -974,7 +976,7 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
             LAUNCH_TRY(h, launch_panel(p->d_items, p->n_items, p->d_item_rows, rows_p, cols_p, perm, dS, dW, dH, dP, p->K,
                                      p->cfg, h->sm_count, h->d_status, s));
         else
-            LAUNCH_TRY(h, launch_rows(p, rows_p, cols_p, perm, dS, dW, dH, dP, 0, p->nnz, use_ring, timer.clk, s));
+            LAUNCH_TRY(h, launch_rows(p, rows_p, cols_p, perm, dS, dW, dH, dP, 0, p->nnz, use_ring, timer.clk, s, false, awaited));
     }
     CUDA_TRY(h, timer.end(s));
     if (p_copy) CUDA_TRY(h, cudaMemcpyAsync(P, dP, nbytes, cudaMemcpyDeviceToHost, s));

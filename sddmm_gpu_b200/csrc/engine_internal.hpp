@@ -131,8 +131,8 @@ constexpr int N_KERNEL_CLOCKS = 1024;
 // Whether launch_rows takes the ring kernel: it is the faster one for this plan, or forced.  permuted: perm is given.
 bool rows_on_ring(const sddmm_plan_s *p, bool force_ring, bool permuted);
 // SDDMM over nonzeros in the plan's processing order, [first, first + count): the ring kernel (rows_on_ring) or the gather
-// kernel in as many passes as are best (beside: see launch_gather).  Launches beyond the first are counted here.
+// kernel in as many passes as are best (beside: see launch_gather; awaited: see GatherPasses).  Launches beyond the first are counted here.
 cudaError_t launch_rows(sddmm_plan_s *p, const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,
                         const float *W, const float *H, float *P, int64_t first, int64_t count, bool force_ring,
-                        unsigned long long *clock, cudaStream_t stream, bool beside = false);
+                        unsigned long long *clock, cudaStream_t stream, bool beside = false, bool awaited = false);
 }  // namespace sddmm
