@@ -102,6 +102,8 @@ struct GatherPasses {
     bool large_h = false;    // most rows of H come from DRAM
     bool awaited = false;    // by the host, as soon as it has been launched, with P in the GPU's memory
 };
+// One pass over whole rows of an H of N rows.
+GatherPasses gather_whole(int64_t nnz, int64_t N, int K);
 // What is best for an H of N rows; one pass where S values and P share memory.  tiled: the nonzeros are in the order of column tiles.
 GatherPasses gather_passes(int64_t nnz, int64_t N, int K, bool tiled, const float *sval, const float *P);
 cudaError_t launch_gather(const int32_t *rows, const int32_t *cols, const int32_t *perm, const float *sval,

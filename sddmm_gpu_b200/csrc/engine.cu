@@ -957,7 +957,9 @@ int sddmm_execute(sddmm_plan_t p, const float *W, const float *H, const float *S
                                       false, nullptr, s, h->dense_mode == 2));
     } else if (use_gather) {
         p->last_kernel = "gather";
-        LAUNCH_TRY(h, launch_gather(p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, p->nnz, p->K, {1, p->K}, h->sm_count, timer.clk, s));
+        GatherPasses whole = gather_whole(p->nnz, p->N, p->K);
+        whole.awaited = awaited;
+        LAUNCH_TRY(h, launch_gather(p->d_rows, p->d_cols, nullptr, dS, dW, dH, dP, p->nnz, p->K, whole, h->sm_count, timer.clk, s));
     } else {
         const bool tiled = p->d_perm != nullptr;
         const int32_t *rows_p = tiled ? p->d_rows_t : p->d_rows;

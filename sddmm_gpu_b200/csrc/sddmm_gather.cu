@@ -452,6 +452,13 @@ cudaError_t launch_pieces(const GatherCall &c)
 
 }  // namespace
 
+// (where the lines lie: launch_pieces)
+GatherPasses gather_whole(int64_t nnz, int64_t N, int K)
+{
+    const int64_t h_bytes = N * K * 4;
+    return {1, K, nnz >= 1000000 && h_bytes >= 8000000 && h_bytes < 300000000, h_bytes >= 500000000};
+}
+
 // Long rows in passes over their columns.  A pass multiplies `floats` columns of every row; its part of H is so much smaller that more
 // of the gathers hit L2, and it runs on one of the shapes that take few registers.  Against that a pass costs the indices again and a
 // sum in P that is written and read: 16 bytes a nonzero.  Sustained us, one pass -> passes of 64 / 96 / 192 (R-MAT unless said):
@@ -483,7 +490,7 @@ cudaError_t launch_pieces(const GatherCall &c)
 GatherPasses gather_passes(int64_t nnz, int64_t N, int K, bool tiled, const float *sval, const float *P)
 {
     const int64_t h_bytes = N * K * 4;
-    const GatherPasses whole = {1, K, nnz >= 1000000 && h_bytes >= 8000000 && h_bytes < 300000000, h_bytes >= 500000000};
+    const GatherPasses whole = gather_whole(nnz, N, K);
     if (sval && sval < P + nnz && P < sval + nnz) return whole;  // the first pass would overwrite S values that the last one needs
     int floats = K;
     if (K > 320) {

@@ -109,6 +109,9 @@ def test_many_nonzeros_of_a_large_h(engine, K, N):
     on_host = [a.cpu().pin_memory() for a in (W, H, S, torch.zeros(nnz))]
     plan.execute(on_host[0], on_host[1], on_host[3], on_host[2])
     assert torch.equal(P.cpu(), on_host[3])
+    forced = torch.full((nnz,), float("nan"), device="cuda")
+    plan.execute(W, H, forced, S, api.FLAG_KERNEL_GATHER)   # the same shape
+    assert torch.equal(P, forced)
     plan.close()
     tiled.close()
 
