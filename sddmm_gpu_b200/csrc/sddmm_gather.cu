@@ -410,16 +410,21 @@ cudaError_t launch_pieces(const GatherCall &c)
     if (q <= 4) GA_GO(4, 1, 4, 4, false, false, 6);
     // Up to 16 pieces all eight sums of a step are reduced together, eight shuffles for 8 instead of ten; with 48 registers more blocks are resident.  us, four at
     // a time / this: K = 64 16.1 M nonzeros 285.7 / 279.9, 6.0 M 107.1 / 102.3, 1.5 M, columns alike 30.7 / 28.7, 0.2 M 9.0 / 8.2;  K = 56 6.0 M 110.1 / 103.8;  K = 32 6.0 M 72.4 /
-    // 70.4, 1.6 M 22.4 / 20.9, documents x words, 0.7 M 12.0 / 10.5.  Passes of 64 columns, and rows of 52 to 64 of an H that is mostly read from DRAM, keep
+    // 70.4, 1.6 M 22.4 / 20.9, documents x words, 0.7 M 12.0 / 10.5.  Passes, and rows of 52 to 64 columns of an H that is mostly read from DRAM, keep
     // four at a time (97 M nonzeros, 4.2 M rows of H: K = 256 7729 / 8641, K = 64 1805 / 1845; 1 M rows: above).
     if (q < 8) GA_GO(8, 1, 4, 8, false, false, 6);
     if (q == 8) GA_GO(8, 1, 4, 8, true, false, 6);
     if (q <= 12) GA_GO(4, 3, 2, 4, false, true, 4);
-    // Up to two waves of blocks a block's own time counts: four rows at a time (same bits; synchronous calls, us, two / four: K = 64 0.22 M nonzeros 18.9 / 18.1, 0.25 M 19.3 / 18.7,
-    // 0.3 M 19.9 / 19.3, 0.4 M 21.3 / 21.1, a row of W for each of 0.07 M 15.7 / 15.3;  but 0.15 M 15.9 / 16.1, 0.205 M 17.6 / 18.2, 0.6 M 25.0 / 25.0, asynchronous 14.9 / 15.6).
-    const unsigned share = c.nnz / ((unsigned)c.sm_count * 5 * (GA_TPB / 32) * 4);
-    if (q > 12 && q <= 16 && !c.pass && share < 20) GA_GO(8, 2, 4, 8, false, false, 4);
-    if (q < 16 && c.large_h) GA_GO(8, 2, 4, 4, false, true, 4);
+    // Where two or three waves of blocks are all, their number counts and a block's own time: four rows at a time on four resident blocks where that takes no more waves than two on five (a tenth
+    // of a wave more is lost in the ends of the one before).  Same bits; us, two / four, and where the host waits: K = 64, uniform, 0.15 M nonzeros 6.2 / 6.6 (16.2 / 16.4), 0.175 M 6.4 / 8.2
+    // (16.5 / 18.1), 0.26 M 10.3 / 10.3 (19.5 / 19.1), 0.3 M 10.3 / 10.3 (19.7 / 19.4), 0.35 M 10.3 / 12.3 (20.2 / 21.8), 0.45 M 12.9 / 12.3 (23.0 / 22.7);  K = 52, R-MAT, 0.205 M 8.2 / 9.7 (17.8 / 18.7).
+    auto waves = [&](unsigned per_block, unsigned ctas, unsigned slack) {
+        const unsigned blocks = c.nnz / per_block + 1, wave = (unsigned)c.sm_count * ctas;
+        return (blocks - (blocks > slack ? slack : 0) + wave - 1) / wave;
+    };
+    const unsigned at_four = waves(256, 4, 0);
+    if (q > 12 && q <= 16 && !c.pass && at_four > 1 && at_four <= 3 && at_four == waves(256, 5, (unsigned)c.sm_count / 2)) GA_GO(8, 2, 4, 8, false, false, 4);
+    if (q < 16 && (c.pass || c.large_h)) GA_GO(8, 2, 4, 4, false, true, 4);
     if (q < 16) GA_GO(8, 2, 2, 8, false, true, 5);
     if (q == 16 && (c.pass || c.large_h)) GA_GO(8, 2, 4, 4, true, true, 4);
     if (q == 16) GA_GO(8, 2, 2, 8, true, false, 5);
@@ -438,7 +443,10 @@ cudaError_t launch_pieces(const GatherCall &c)
 #define GA_STAGED(L, F, B, RB, EXACT, PF, CTAS) return launch_shape<GatherShape<L, F, B, RB, EXACT, PF, CTAS, false, true>>(c)
     if (q <= 96) GA_STAGED(16, 6, 1, 8, false, false, 4);
     if (q < 128) GA_GO(32, 4, 2, 8, false, true, 3);
-    // (two at a time on three blocks / this, us: 0.75 M nonzeros, documents x words 69.9 / 65.8, 0.6 M 75.6 / 72.2, 1.6 M 182.4 / 179.9, 0.2 M 27.0 / 26.8)
+    // (two at a time on three blocks / this, us: 0.75 M nonzeros, documents x words 69.9 / 65.8, 0.6 M 75.6 / 72.2, 1.6 M 182.4 / 179.9, 0.2 M 27.0 / 26.8, 32 K, uniform 10.3 / 8.2, 60 K 14.3 / 13.0;
+    // two at a time where that takes no more waves, from the second on: 50 K 11.1 / 12.3, 78 K 15.3 / 16.4, documents x words, 50 K 8.5 / 10.3)
+    const unsigned at_one = waves(64, 4, 0);
+    if (q == 128 && at_one > 1 && at_one <= 3 && at_one == waves(64, 3, 0)) GA_GO(32, 4, 2, 8, true, true, 3);
     if (q == 128) GA_GO(32, 4, 1, 8, true, false, 4);
     if (q <= 160) GA_GO(32, 5, 1, 8, false, false, 4);
     if (q == 192) GA_STAGED(32, 6, 1, 8, true, false, 4);  // (0.75 M nonzeros 104.6 / 100.9)

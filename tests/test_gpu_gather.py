@@ -68,16 +68,17 @@ def test_few_nonzeros_as_many(engine, K):
         plan.close()
 
 
-@pytest.mark.parametrize("K", [52, 60, 64])
-def test_two_waves_as_many(engine, K):
-    # up to 473,600 nonzeros of 148 SMs take four rows at a time: the same bits as the front of a call that takes two
+@pytest.mark.parametrize("K", [52, 60, 64, 512])
+def test_few_waves_as_many(engine, K):
+    # 52 to 64 columns: from 208,384 to 303,103 nonzeros of 148 SMs and from 397,824 to 454,655 take four rows at a time, K = 512: from 37,888 to 56,831 and from 75,776
+    # to 85,247 two: the same bits as the front of a call of many
     M, N, nnz = 9_001, 7_001, 600_000
     g = torch.Generator(device="cuda").manual_seed(K)
     rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
     cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
     W, H, S = (torch.randn(n, generator=g, device="cuda") for n in ((M, K), (N, K), (nnz,)))
     P = {}
-    for n in (nnz, 50_001, 213_119, 300_001, 473_599, 473_600):
+    for n in (nnz, 37_887, 37_888, 50_001, 56_831, 56_832, 75_776, 85_248, 151_552, 208_383, 208_384, 303_103, 303_104, 397_823, 397_824, 454_655, 454_656):
         plan = engine.plan_coo(M, N, rows[:n], cols[:n], K)
         P[n] = torch.full((n + 1,), 7.0, device="cuda")
         plan.execute(W, H, P[n][:n], S[:n])
