@@ -4,14 +4,15 @@
 // time: lane l of the set holds the 16-byte pieces l, l + L, ... (F of them) of the W row and of the H row, so one
 // load instruction of a set covers L * 16 consecutive bytes of one row.  H rows are loaded straight into registers, B
 // nonzeros ahead of their use; the W row stays in registers until the row of S changes.  Rows, columns and S values of
-// a step (8 nonzeros per set) are loaded one step ahead, one nonzero per lane, and spread by shuffles; the 8 partial
+// a step (8 nonzeros per set) are loaded one step ahead, one nonzero per lane, and spread by shuffles (STAGED: columns through shared memory); the 8 partial
 // sums of a lane are reduced by one transposed butterfly, after which lane l stores nonzero l of the set.
 //
 // What bounds it.  Every nonzero brings one row of H from L2 (or L1, or DRAM) to its SM: 4K bytes, 16.7 TB/s at most
 // over all SMs (a bare copy loop).  Latency is hidden by warps, not by a pipeline inside the warp: few registers per
 // thread and many resident warps (24 to 48 per SM, __launch_bounds__ below) move more bytes than deeper batches with
 // fewer warps (K = 128, 16.1 M nonzeros of an R-MAT matrix: 0.53 ms at 40 warps with one nonzero in flight per set,
-// 0.59 ms at 24 warps with two, 0.64 ms at 16 warps with four).  No shared memory: all of it is L1, which serves the
+// 0.59 ms at 24 warps with two, 0.64 ms at 16 warps with four).  Next to no shared memory (32 or 64 bytes a warp for
+// the columns of a step, K = 324 to 384, 644 to 768 and 900 to 1024): the rest is L1, which serves the
 // hub columns of a power-law matrix, and nothing is issued beyond the load, the packed FMAs (two per instruction) and
 // 1/8 of a butterfly -- 9 warp instructions per nonzero at K = 128 where the shared-memory ring needed 34.  Grids are
 // not persistent: a warp's share is 8, 16 or 32 nonzeros per set (4 where sets of four lanes are many), the hardware's block scheduler
@@ -233,18 +234,20 @@ sddmm_gather_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict_
     clock_end(clock, meet_from);
 }
 
-// Few nonzeros, two for each set: every row of W and of H is asked for at once, where the kernel above waits for an H row after the other and for the W row of every row of S
-// that a step opens.  The sums are the same, bit for bit: the same pieces to the same lanes, reduced in the same order.  What bounds it: three latencies, indices, rows, the wait
+// Few nonzeros, two for each set: rows of W and of H are asked for together, where the kernel above waits for an H row after the other and for the W row of every row of S
+// that a step opens.  (All four rows of a set at once at F = 1; from F = 2 on the compiler keeps 32 to 40 registers and the second nonzero's rows follow the first's.)  The sums are
+// the same, bit for bit: the same pieces to the same lanes, reduced in the same order.  What bounds it: three latencies, indices, rows, the wait
 // for the call.  Synchronous calls, us, above / this: uniform, 16,777 nonzeros, K = 32 14.2 / 13.3, K = 64 14.5 / 13.6, K = 128 14.4 / 14.1;  4,000, K = 32, 128, 512 14.2 / 13.1, 14.0 /
 // 13.6, 14.3 / 14.1;  40,000, K = 64 14.5 / 14.0;  R-MAT, 70,000, K = 32 14.7 / 14.2.  One or four for each set: 13.3, 13.7 and 13.6, 14.1 in the first two.
-template <class S>
+template <int L, int F, bool EXACT>
 __global__ void __launch_bounds__(GA_TPB)
 sddmm_gather_few_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, const float *__restrict__ sval,
                         const char *__restrict__ W, const char *__restrict__ H, float *__restrict__ P, unsigned nnz, int pieces,
                         unsigned long long *clock, unsigned meet_from)
 {
     clock_begin(clock);
-    constexpr int L = S::L, F = S::F, G = S::G, U = FEW_EACH;
+    using S = GatherShape<L, F, 1, 1, EXACT, false, 1>;
+    constexpr int G = S::G, U = FEW_EACH;
     const int lane = threadIdx.x & 31, lig = lane & (L - 1), set = lane / L;
     const unsigned first = gather_warp(blockIdx.x, GA_TPB, threadIdx.x) * (G * U);  // nonzero u of a set: first + u G + set
     if (first >= nnz) return;
@@ -352,7 +355,7 @@ cudaError_t launch_few(const GatherCall &c)
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(GA_TPB);
     cfg.stream = c.stream;
-    return cudaLaunchKernelEx(&cfg, sddmm_gather_few_kernel<S>, c.rows, c.cols, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.clock,
+    return cudaLaunchKernelEx(&cfg, sddmm_gather_few_kernel<S::L, S::F, S::EXACT>, c.rows, c.cols, c.sval, c.W, c.H, c.P, c.nnz, c.pieces, c.clock,
                               last_wave(blocks, (unsigned)c.sm_count * (2048 / GA_TPB)));
 }
 
@@ -364,7 +367,8 @@ cudaError_t launch_mode(const GatherCall &c)
     // Up to 10 MB of H rows a call is a few latencies long, which count where it is waited for.  (Above it W rows that are read again for every nonzero cost more: synchronous calls
     // of 80,000 nonzeros, uniform, K = 64 15.3 / 15.0, K = 128 16.3 / 16.9;  40,000, K = 128 14.8 / 15.1, K = 256 16.0 / 16.7;  150,000, R-MAT, K = 32 15.2 / 15.3.  Asynchronous calls one
     // after the other take what the host needs to launch them, and that is more with the shorter kernel: 16,777 nonzeros, K = 32, 64 5.0 / 5.5, of 2.9 / 1.7, 3.0 / 1.9 on the GPU.)
-    if constexpr (MODE == STORE && S::F <= 4)
+    // (the shape of eight lanes and four pieces is taken from a million nonzeros on, and no call with bfloat16 operands asks)
+    if constexpr (MODE == STORE && S::F <= 4 && !(S::L == 8 && S::F == 4) && !S::BF16)
         if (c.awaited && (uint64_t)c.nnz * (unsigned)c.pieces * 16u <= 10000000) return launch_few<S>(c);
     // A set's run.  A long one spreads what a run costs at its ends and keeps the W row over more nonzeros; the last wave of blocks, which
     // may be nearly empty, lasts as long as a run.  So by the nonzeros that there are for a resident set (us at runs of 8 / 16 / 32):

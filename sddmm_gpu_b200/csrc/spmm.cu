@@ -74,7 +74,7 @@ struct SpmmShape {
     static_assert(NB % B == 0, "step geometry");
     static_assert(!FAR || !FUSED, "a set has one row in scratch");
     static constexpr int SLOTS = FUSED || FAR ? SETS : 0;  // rows of a block's sets in scratch: heads of the fused form (ON_W), tails of FAR
-    static_assert(!STAGED || (FUSED && JOINT && L == 32), "staged: a warp for a nonzero");
+    static_assert(!STAGED || (FUSED && JOINT && L == 32 && B > 1), "staged: a warp for a nonzero");
 };
 
 // STAGED: what a warp knows of the 32 nonzeros at hand.
@@ -83,7 +83,6 @@ struct Staged {
     float val[32], p[32];  // p: the weights
 };
 template <int B> struct Vec;
-template <> struct Vec<1> { using I = int; using V = float; };
 template <> struct Vec<2> { using I = int2; using V = float2; };
 template <> struct Vec<4> { using I = int4; using V = float4; };
 template <int B, class T>
@@ -91,8 +90,7 @@ __device__ __forceinline__ void lds_vec(T (&out)[B], const T *p)
 {
     using X = typename std::conditional<std::is_same<T, float>::value, typename Vec<B>::V, typename Vec<B>::I>::type;
     const X v = *reinterpret_cast<const X *>(p);
-    if constexpr (B == 1) out[0] = v;
-    if constexpr (B >= 2) out[0] = v.x, out[1] = v.y;
+    out[0] = v.x, out[1] = v.y;
     if constexpr (B == 4) out[2] = v.z, out[3] = v.w;
 }
 
@@ -682,15 +680,11 @@ cudaError_t launch_shape(const SpmmCall &a, int k0, int width, int sm_count, int
     const unsigned run = run_length<S>(a.nnz, sm_count), per_block = S::SETS * run;
     const unsigned gather_blocks = (unsigned)((a.nnz + per_block - 1) / per_block);
     const unsigned zero_blocks = (unsigned)((a.M + SP_TPB - 1) / SP_TPB);
-    // scratch: two counters per run, zero between calls, then the parts
+    // scratch: two counters per block, zero between calls, then the parts, then a row for each set (SLOTS)
     unsigned *const arrived = reinterpret_cast<unsigned *>(a.scratch);
     char *const parts = reinterpret_cast<char *>(a.scratch + spmm_counter_floats(a.nnz, a.N, a.K, sm_count));
     constexpr int smem = S::TAIL_BYTES;
-    if (smem > 32 * 1024) {
-        static SmemOptinCache optin;  // per device
-        const cudaError_t e = optin_dynamic_smem(spmm_kernel<S, false>, smem, optin);
-        if (e != cudaSuccess) return e;
-    }
+    static_assert(smem + sizeof(Staged) * (SP_TPB / 32) + 512 <= 48 * 1024, "without opt-in");
     auto launch = [&](auto kernel) {
         kernel<<<gather_blocks + zero_blocks, SP_TPB, smem, stream>>>(
             a.rows, a.cols, a.val, reinterpret_cast<const char *>(a.W), reinterpret_cast<const char *>(a.H + k0), a.P_out,

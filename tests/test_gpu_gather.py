@@ -117,6 +117,24 @@ def test_many_nonzeros_of_a_large_h(engine, K, N):
     tiled.close()
 
 
+@pytest.mark.parametrize("K,N", [(52, 2_403_847), (60, 2_083_334), (64, 1_953_125), (64, 1_953_124)])
+def test_rows_of_a_very_large_h(engine, K, N):
+    # 52 to 64 columns of an H of 500 MB and more (the last N is below) have the shape of the passes; whole numbers: every product and sum is exact
+    M, nnz = 50_021, 600_011
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rows = torch.sort(torch.randint(0, M, (nnz,), generator=g, device="cuda")).values.to(torch.int32)
+    cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    cols[-1] = N - 1
+    W, H, S = (torch.randint(-2, 3, n, generator=g, device="cuda").float() for n in ((M, K), (N, K), (nnz,)))
+    ref = torch.cat([torch.einsum("nk,nk->n", W[rows[i:i + 100_000].long()], H[cols[i:i + 100_000].long()]) for i in range(0, nnz, 100_000)]) * S
+    plan = engine.plan_coo(M, N, rows, cols, K)
+    for flags in (0, api.FLAG_KERNEL_GATHER):
+        P = torch.full((nnz + 1,), 7.0, device="cuda")
+        plan.execute(W, H, P[:nnz], S, flags)
+        assert torch.equal(P[:nnz], ref) and float(P[nnz]) == 7.0
+    plan.close()
+
+
 def test_kernel_time_of_small_calls(engine):
     # timed by the kernel's own clock; each plan keeps its own time, also when calls of other plans lie between, and an
     # asynchronous call has none

@@ -80,7 +80,7 @@ def test_tails_in_scratch(engine, K):
 
 @pytest.mark.parametrize("K", [16, 32, 64, 96, 160, 192, 200, 256, 320, 384, 512, 768, 1024])
 def test_block_boundaries(engine, K):
-    # A block holds 8 to 64 runs of 8, 16 or 24 nonzeros.  Rows that begin and end at multiples of 8 and 64 and one beside them, rows of a block and of
+    # A block holds 8 to 64 runs of 8, 16 or 24 nonzeros (K = 16: of 4).  Rows that begin and end at multiples of 8 and 64 and one beside them, rows of a block and of
     # 16 and 17 blocks, many short rows in a run, rows that a block has only the end of; small whole numbers, so that every sum is exact.
     rng = np.random.default_rng(K)
     N = 17 * 1536 + 9
