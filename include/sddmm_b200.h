@@ -170,7 +170,7 @@ SDDMM_API int sddmm_execute(sddmm_plan_t p, const float *W, const float *H,
  * before the row of Y is stored.  Apart from that Y must not overlap what the call reads.
  * K a multiple of 4 up to 1024 (SDDMM_K_UNSUPPORTED otherwise).  Pointers host or device (host
  * arrays are staged for the call); flags: 0 or SDDMM_FLAG_ASYNC (device pointers only).  The
- * nonzeros are cut into equal runs; the parts of a row of S that spans runs are added in run order: the
+ * nonzeros are cut into equal runs; the parts of a row of S that spans runs are added in a fixed order: the
  * result does not depend on scheduling.  Works on the plan's input order (column tiles of the
  * plan are not used).  sddmm_last_kernel_ms() reports the kernels' time.
  * The parts lie in scratch that belongs to the plan: calls of one plan on different streams run one after the

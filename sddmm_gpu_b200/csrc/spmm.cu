@@ -626,12 +626,13 @@ spmm_kernel(const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, 
 // run pays for its two ends, so few; but rows of a power-law matrix make some
 // runs slower than others, the fused form more than SpMM, and long runs spread a wave over more rows of H than L2 holds.  us at
 // 1 / 2 / 3 / 4 / 6 / 8 waves (s: nonzeros for a resident set):
-//   SpMM, K = 64: s = 11 12.3 / 15.5 / 15.5 / 15.4 / 15.4 / 15.5;  62 28 / 31 / 32 / 35 / 35 / 45;  80, columns alike 31 / 35 / 39 / 39 / 42 / 43;  317 114 / 113 / 117 / 117 / 122 / 123
-//   (before blocks added up their own parts: 118, K = 256 52 / 56 / 62 / 64 / - / 80;  577, K = 100 143 / 142 / 143 / 147 / - / 169;  1351, K = 200 674 / 550 / 579 / 569 / - / 576)
-//   fused, sets of eight lanes: s = 11, K = 64 14.5 / 16.9 / 17.0 / 17.0;  62 41 / 40 / 41 / 43 / 43 / 55;  80, columns alike 45 / 47 / 51 / 53 / 56 / 56;  254, K = 32 - / 133 / 132 / 119 / 121 / -;
-//     317, K = 64 205 / 186 / 180 / 177 / 173 / 175;  317, K = 128 - / - / - / 268 / - / 266;  849, K = 128 at 4 / 6 / 8 786 / 761 / 776
-//   fused, a warp for a nonzero, K = 256: s = 58 27 / 27 / 29 / - / - / 41;  330 163 / 129 / 125 / - / - / 116;  422, columns alike - / 146 / 151 / - / 166 / -;  1689 at 5 / 6 / 8 / 12 / 20 533 / 500 / 499 /
-//     494 / 499;  4531 at 12 / 16 1492 / 1478
+//   SpMM, K = 64: s = 14 12.6 / 12.4 / 12.5 / 12.5 / 12.5 / 12.5 (runs of 24 at least);  80, columns alike 28.8 / 31.6 / 35.4 / 37.2 / 37.2 / 37.3;  317 100 / 99.5 / 101 / 102 / 107 / 112
+//   K = 256: 127 40.9 / 43.9 / 46.1 / 50.4 / 54.5 / 54.6;  K = 100: 577 137 / 135 / 136 / 138 / 143 / 148, 845 183 / 181 / 181 / 183 / 186 / 192;  K = 200: 1267 295 / 295 / 297 / 299 / 302 / 308
+//   fused, sets of eight lanes, K = 64: s = 14 14.4 / 17.2 / 17.2 / 17.2 / 17.2 / 17.2;  80, columns alike 41.7 / 43.8 / 49.0 / 50.5 / 52.8 / 52.8;  317 194 / 179 / 174 / 172 / 168 / 169
+//   K = 128: 72 75 / 74 / 74 / 74 / 79 / 79;  317 303 / 279 / 276 / 273 / 271 / 270
+//   fused, a warp for a nonzero, K = 256: s = 58 26.7 / 26.9 / 28.7 / 30.6 / 30.6 / 39.6;  330 133 / 116 / 113 / 110 / 110 / 111;  423, columns alike 138 / 145 / 150 / 158 / 165 / 168;
+//   1690 528 / 530 / 514 / 517 / 475 / 473;  4531 at 12 / 16 1492 / 1478
+// (SpMM: what asks for more than two are roundings.)
 template <class S>
 unsigned run_length(int64_t nnz, int sm_count)
 {
