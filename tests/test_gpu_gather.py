@@ -78,7 +78,7 @@ def test_few_waves_as_many(engine, K):
     cols = torch.randint(0, N, (nnz,), generator=g, device="cuda", dtype=torch.int32)
     W, H, S = (torch.randn(n, generator=g, device="cuda") for n in ((M, K), (N, K), (nnz,)))
     P = {}
-    for n in (nnz, 37_887, 37_888, 50_001, 56_831, 56_832, 75_776, 85_248, 151_552, 208_383, 208_384, 303_103, 303_104, 397_823, 397_824, 454_655, 454_656):
+    for n in (nnz, 37_887, 37_888, 50_001, 56_831, 56_832, 75_776, 85_248, 151_552, 208_383, 208_384, 213_119, 300_001, 303_103, 303_104, 397_823, 397_824, 454_655, 454_656, 473_599, 473_600):
         plan = engine.plan_coo(M, N, rows[:n], cols[:n], K)
         P[n] = torch.full((n + 1,), 7.0, device="cuda")
         plan.execute(W, H, P[n][:n], S[:n])
